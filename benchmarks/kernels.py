@@ -43,7 +43,7 @@ def main():
     ap.add_argument("--split", action="store_true",
                     help="only compare products with and without sharing the last round of tiles along the depth")
     ap.add_argument("--tilings", action="store_true",
-                    help="only compare the three GEMM tilings (128-row, CTA pair, tall) on a few shapes")
+                    help="only compare the two GEMM tilings (128-row, CTA pair) on a few shapes")
     args = ap.parse_args()
     from moe_distributed_training_b200.ops import cuda_ops as ops
     peaks = {}
@@ -92,7 +92,7 @@ def main():
                           (4096, 4096, 4096)]:
             x, w = torch.randn(M, K, device=dev, dtype=bf) * 0.1, torch.randn(N, K, device=dev, dtype=bf) * 0.1
             out = torch.empty(M, N, device=dev, dtype=bf)
-            for name, policy in (("tile128", 0), ("pair", 2), ("tall", 4)):
+            for name, policy in (("tile128", 0), ("pair", 2)):
                 prev = ops.ext.gemm_set_pair_policy(policy)
                 report(f"gemm_nt_{M}x{N}x{K}_{name}", timeit(lambda: ops.mm_nt(x, w, out=out), flush=flush), flops=2.0 * M * N * K)
                 ops.ext.gemm_set_pair_policy(prev)

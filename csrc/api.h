@@ -62,8 +62,8 @@ long long mdt_skinny_launch_count(void);
 int mdt_skinny_mm(const void* x, const void* A, void* y, int M, int K, int r, long long ldx, long long lda,
                   int a_is_kr, float alpha, cudaStream_t s);
 // Kernel for 256-wide tiles: 0 the 128-row kernel, 1 / 2 the CTA-pair (cta_group::2) kernel where the shape fills
-// 256-row tiles / always, 3 / 4 the tall single-CTA 256 x 256 kernel where it fills / always; returns the previous
-// policy (policy < 0 only reads it).
+// 256-row tiles / always, 3 / 4 the same where 256-row tiles win by a margin / always, 5 (default) the one that the
+// measured model finds faster; returns the previous policy (policy < 0 only reads it).
 int mdt_gemm_set_pair_policy(int policy);
 // CTA pairs resident at once on this device (0 until the pair kernel has been launched)
 int mdt_gemm_max_pairs(void);
@@ -71,7 +71,7 @@ int mdt_gemm_max_pairs(void);
 // capacity; 0 = unknown.  Only guides the choice of tile shape.
 void mdt_gemm_rows_hint(long long rows);
 // The tiling mdt_gemm would pick for `d` under `policy` (see mdt_gemm_set_pair_policy) with that rows hint on a GPU with
-// `num_sms` SMs: 0 = 128-row tiles, 1 = CTA pair, 2 = tall.  Reads only M, N, K, K_l, G, mode, dual, c_fp32, accumulate,
+// `num_sms` SMs: 0 = 128-row tiles, otherwise CTA-pair tiles (2 under policies 3 to 5).  Reads only M, N, K, K_l, G, mode, dual, c_fp32, accumulate,
 // capacity_rows and whether offsets is set; needs no GPU.
 int mdt_gemm_choose_tiling(const MdtGemmDesc* d, int policy, long long rows_hint, int num_sms);
 // Sharing of the last, partly filled round of 128-row tiles by all SMs along the depth (partial sums through an fp32

@@ -171,6 +171,24 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// True in one lane of a converged warp.  The producer and MMA roles run as whole warps and elect a lane only around
+// the issuing instructions: the compiler then keeps descriptors, addresses and loop state in uniform registers, which
+// tcgen05 and TMA instructions read directly (a role that runs under `if (lane == 0)` moves every operand across for
+// each instruction).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(pred));
+  return pred != 0;
+}
+// wait_parity for a whole warp: every lane waits, and all lanes leave together with the same answer
+__device__ __forceinline__ bool wait_parity_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, wait_parity(bar, parity, abort_flag));
+}
+
 // Shared-memory matrix descriptor, 128-byte swizzle, tile base 1024-byte aligned.
 //   K-major  operand: rows of 128 bytes, 8-row groups 1024 bytes apart  -> lbo = 16 (unused), sbo = 1024
 //   MN-major operand: 64-element column chunks `lbo` bytes apart, 8 K-rows per 1024 bytes -> sbo = 1024

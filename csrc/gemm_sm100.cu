@@ -14,8 +14,8 @@
 // mode that computes gate and up projections in one 256-wide MMA and applies SwiGLU in the
 // epilogue, alpha scaling and accumulation into C (gradient accumulation), fp32 or bf16 C.
 //
-// Role layout of a 192-thread CTA: warp 0 = TMA producer, warp 1 = MMA issuer (owns TMEM),
-// warps 2-5 = epilogue (each owns one 32-lane quarter of TMEM).
+// Role layout of a 320-thread CTA: warp 0 = TMA producer, warp 1 = MMA issuer (owns TMEM), warps 2-9 = epilogue
+// (a warp reads the 32-lane quarter warp % 4 of TMEM; two warps share a quarter, half of the columns each).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -39,7 +39,8 @@ namespace mdt {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int A_BYTES = BM * BK * 2;
-constexpr int GEMM_THREADS = 192;
+constexpr int GEMM_THREADS = 320;
+constexpr int SPLIT_COUNTERS = 12;   // of a shared tile: 8 parts (row quarter x column half), 4 row quarters
 
 struct GemmParams {
   CUtensorMap tmA, tmB, tmB2;        // main depth segment (tmB2: second B matrix of the dual mode)
@@ -96,46 +97,77 @@ __device__ __forceinline__ bool gemm_dead(const GemmParams& p) {
   return p.status != nullptr && (p.tile_ready != nullptr || p.row_dest_rank != nullptr) && *reinterpret_cast<const volatile int*>(p.status) != 0;
 }
 
-struct Tile {
-  int g, m0, n0, krow0, num_kb, num_kb_l;
-};
+// Order of the output tiles.  A persistent grid works on a window of consecutive tiles at a time; what that window
+// reads should stay in L2.  Tiles therefore go through panels of at most 2048 rows (16 blocks of 128 or 8 of 256),
+// m fastest inside a panel, then n: 148 CTAs then share about 2048 rows of A and 9 column blocks of B.  With m fastest
+// over all rows, a window of the expert products (18 400 rows x K 14336) streamed the whole 530 MB of A once per column
+// block, 1.0-1.2 PFLOP/s instead of the 1.4 that the same kernel reaches when the window fits.  Row groups are
+// enumerated one after the other for the same reason: a window then holds one expert's weights.
+constexpr int PANEL_ROWS = 2048;
+__host__ __device__ __forceinline__ void panel_order(int r, int m_blocks, int n_blocks, int panel, int& m, int& n) {
+  const int first = r / (panel * n_blocks) * panel;
+  const int width = m_blocks - first < panel ? m_blocks - first : panel;
+  const int q = r - first * n_blocks;
+  m = first + q % width;
+  n = q / width;
+}
 
-// Maps a linear tile index to its coordinates; returns false past the last tile.  (Also callable on the host, where
-// a unit test enumerates the tiles of random problems and checks that they cover every block exactly once.)
-template <int BN_OUT>
-__host__ __device__ __forceinline__ bool get_tile(const GemmParams& p, int t, Tile& o) {
+struct Tile {
+  int g, m0, n0, krow0, num_kb, num_kb_l, second_ok;
+};
+typedef Tile PairTile;
+
+// Maps a linear tile index to its coordinates, for tiles of ROWS rows (128, or 256 for the CTA pair); returns false past
+// the last tile.  In the grouped-rows mode a 256-row tile never straddles two groups: a group with an odd number of
+// 128-row blocks ends with a tile whose second half is idle (second_ok = 0).  (Also callable on the host, where a unit
+// test enumerates the tiles of random problems and checks that they cover every block exactly once.)
+template <int BN_OUT, int ROWS>
+__host__ __device__ __forceinline__ bool locate_tile(const GemmParams& p, int t, Tile& o) {
   const int n_blocks = (p.N + BN_OUT - 1) / BN_OUT;
+  int m, n;
   o.num_kb_l = (p.K_l + BK - 1) / BK;
-  if (p.mode == 2) {
-    const int m_blocks = (p.M + BM - 1) / BM;
-    const int per_group = m_blocks * n_blocks;
-    if (t >= per_group * p.G) return false;
-    o.g = t / per_group;
-    int r = t - o.g * per_group;
-    o.m0 = (r % m_blocks) * BM;
-    o.n0 = (r / m_blocks) * BN_OUT;
-    int k_begin = 0, k_end = p.K;
-    if (p.offsets != nullptr) { k_begin = p.offsets[o.g]; k_end = p.offsets[o.g + 1]; }
-    o.krow0 = k_begin;
-    o.num_kb = (k_end - k_begin + BK - 1) / BK;
-    return true;
-  }
-  int rows = p.M;
-  if (p.mode == 1) rows = p.offsets[p.G];
-  const int m_blocks = (rows + BM - 1) / BM;
-  if (t >= m_blocks * n_blocks) return false;
-  o.m0 = (t % m_blocks) * BM;
-  o.n0 = (t / m_blocks) * BN_OUT;
-  o.g = 0;
-  if (p.mode == 1) {
-    int g = 0;
-    while (g + 1 < p.G && p.offsets[g + 1] <= o.m0) ++g;
-    o.g = g;
-  }
+  o.second_ok = 1;
   o.krow0 = 0;
   o.num_kb = (p.K + BK - 1) / BK;
+  if (p.mode == 1) {
+    for (int g = 0; g < p.G; ++g) {
+      const int begin = p.offsets[g], end = p.offsets[g + 1];
+      const int m_blocks = (end - begin + ROWS - 1) / ROWS;
+      if (t < m_blocks * n_blocks) {
+        panel_order(t, m_blocks, n_blocks, PANEL_ROWS / ROWS, m, n);
+        o.g = g;
+        o.m0 = begin + m * ROWS;
+        o.n0 = n * BN_OUT;
+        if (ROWS > BM) o.second_ok = (o.m0 + BM < end) ? 1 : 0;
+        return true;
+      }
+      t -= m_blocks * n_blocks;
+    }
+    return false;
+  }
+  const int m_blocks = (p.M + ROWS - 1) / ROWS;
+  const int per_group = m_blocks * n_blocks;
+  o.g = 0;
+  if (p.mode == 2) {
+    if (t >= per_group * p.G) return false;
+    o.g = t / per_group;
+    t -= o.g * per_group;
+    if (p.offsets != nullptr) {
+      o.krow0 = p.offsets[o.g];
+      o.num_kb = (p.offsets[o.g + 1] - o.krow0 + BK - 1) / BK;
+    }
+  } else if (t >= per_group) {
+    return false;
+  }
+  panel_order(t, m_blocks, n_blocks, PANEL_ROWS / ROWS, m, n);
+  o.m0 = m * ROWS;
+  o.n0 = n * BN_OUT;
   return true;
 }
+template <int BN_OUT>
+__host__ __device__ __forceinline__ bool get_tile(const GemmParams& p, int t, Tile& o) { return locate_tile<BN_OUT, BM>(p, t, o); }
+template <int BN_OUT>
+__host__ __device__ __forceinline__ bool get_pair_tile(const GemmParams& p, int t, PairTile& o) { return locate_tile<BN_OUT, 2 * BM>(p, t, o); }
 
 // One unit of work of a CTA: a whole output tile, or a piece [kb0, kb1) of the depth of a tile that several CTAs share.
 struct Work {
@@ -235,6 +267,207 @@ __device__ __forceinline__ void store8(void* C, long long idx, const float (&v0)
   }
 }
 
+// ---- epilogue: eight warps, warp -> (32-row quarter of the tile = its TMEM lanes, half of the tile's columns) ----------
+// bf16 results leave through a 4 KB stage per warp, 32 rows x 64 columns: a lane holds one row of the accumulator, so
+// storing from registers would write 16 bytes to each of 32 rows per instruction.  From the stage a warp writes whole
+// 128-byte lines, four rows per instruction.  What is added to the result (C itself when accumulating, or the residual)
+// comes in the same way, the first chunk fetched before the warp waits for the accumulator and the next one while the
+// first is processed, so that the latency passes under other work.  Weight gradients of one micro-batch
+// (3 k blocks per 128 x 256 tile of an 8 x 14336 x 4096 matrix, read and written) are bound by exactly this traffic:
+// 1400 us with per-row accesses by four warps.
+// 16-byte slots are XOR-swizzled by the row, so that row-wise and line-wise accesses are both free of bank conflicts.
+constexpr int EPI_WARPS = 8;
+constexpr int EPI_STAGE_BYTES = 32 * 128;
+__device__ __forceinline__ uint4* epi_slot(uint8_t* stage, int row, int slot) {
+  return reinterpret_cast<uint4*>(stage + row * 128 + ((slot ^ (row & 7)) << 4));
+}
+// the 64-column chunk at `col` of the matrix whose rows start at `mine` (one per lane), line-wise: 8 x 16 bytes per lane
+// (`safe`: an address that may be read instead of one that is out of range, so that the loads need no branches)
+__device__ __forceinline__ void epi_fetch(uint4 (&v)[8], unsigned long long mine, unsigned row_ok, int lane, int col, int N, const void* safe) {
+  const int c = col + (lane & 7) * 8;
+  const uint4* src[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = i * 4 + (lane >> 3);
+    const unsigned long long ptr = __shfl_sync(0xffffffffu, mine, row);
+    src[i] = ((row_ok >> row) & 1u) && c < N ? reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(ptr) + c)
+                                             : reinterpret_cast<const uint4*>(safe);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[i].x), "=r"(v[i].y), "=r"(v[i].z), "=r"(v[i].w) : "l"(src[i]));
+}
+__device__ __forceinline__ void epi_stage_in(uint8_t* stage, const uint4 (&v)[8], int lane) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) *epi_slot(stage, i * 4 + (lane >> 3), lane & 7) = v[i];
+  __syncwarp();
+}
+// this lane's row, columns [32 * part, 32 * part + 32) of the chunk; ADD: plus what the stage holds there
+template <bool ADD>
+__device__ __forceinline__ void epi_stage_row(uint8_t* stage, const float (&v)[32], int part, int lane) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint4* slot = epi_slot(stage, lane, part * 4 + j);
+    float f[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = v[j * 8 + i];
+    if (ADD) {
+      const uint4 old = *slot;
+      const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&old);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { const float2 t = __bfloat1622float2(o2[i]); f[2 * i] += t.x; f[2 * i + 1] += t.y; }
+    }
+    uint4 out;
+    __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&out);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    *slot = out;
+  }
+}
+__device__ __forceinline__ void epi_flush(uint8_t* stage, unsigned long long mine, unsigned row_ok, int lane, int col, int N) {
+  __syncwarp();
+  const int c = col + (lane & 7) * 8;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int row = i * 4 + (lane >> 3);
+    const unsigned long long ptr = __shfl_sync(0xffffffffu, mine, row);
+    const uint4 val = *epi_slot(stage, row, lane & 7);
+    if (((row_ok >> row) & 1u) && c < N) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(ptr) + c) = val;
+  }
+  __syncwarp();
+}
+// The row of C (or of a peer's buffer) that a lane of an epilogue warp owns.
+struct EpiRow { void* C; long long base; bool ok; int dest; };
+__device__ __forceinline__ EpiRow epi_row(const GemmParams& p, int g, int row, bool row_ok) {
+  EpiRow r;
+  r.base = (p.mode == 2 ? (long long)g * p.c_group_stride : 0) + (long long)row * p.ldc;
+  r.C = p.C;
+  r.dest = -1;
+  r.ok = row_ok;
+  if (p.row_dest_rank != nullptr) {          // result rows go straight into peers' buffers
+    r.dest = row_ok ? p.row_dest_rank[row] : -1;
+    const int drow = row_ok ? p.row_dest_row[row] : -1;
+    if (r.dest >= p.num_peers || drow < 0) r.dest = -1;
+    r.ok = r.dest >= 0;
+    if (r.ok) { r.C = reinterpret_cast<void*>(p.peer_out[r.dest]); r.base = (long long)drow * p.ldc; }
+  }
+  return r;
+}
+// publish a warp's delivered rows: one count per (row, column tile) and destination
+__device__ __forceinline__ void epi_publish(const GemmParams& p, int dest, int lane) {
+  __threadfence_system();
+  __syncwarp();
+  for (int d = 0; d < p.num_peers; ++d) {
+    const unsigned m = __ballot_sync(0xffffffffu, dest == d);
+    if (lane == 0 && m != 0) red_add_release_sys(reinterpret_cast<unsigned*>(p.peer_arrive[d]), __popc(m));
+  }
+}
+// a tile without any depth (an empty group of a weight gradient): zeros unless accumulating
+template <int COLS>
+__device__ __forceinline__ void epi_zero(const GemmParams& p, const EpiRow& r, bool row_ok, int col0) {
+  if (p.accumulate || !row_ok) return;
+  const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int c = 0; c < COLS; c += 8)
+    if (col0 + c < p.N) store8(p.C, r.base + col0 + c, z, p.c_fp32, 0);
+}
+
+// One warp's part of a tile: COLS = BN / 2 accumulator columns from TMEM column `taddr` on (dual: COLS / 2 outputs, the
+// up accumulators being 2 * COLS / 2 = BN / 2 columns further).  `wait` is called once, before the first TMEM load.
+template <int BN, class Wait>
+__device__ __forceinline__ bool epi_tile(const GemmParams& p, uint8_t* stage, uint32_t tacc, int half, int lane, int n0, const EpiRow& r, Wait wait) {
+  const bool fast = !p.c_fp32 && !(p.accumulate && p.R != nullptr);
+  const unsigned row_ok = __ballot_sync(0xffffffffu, r.ok);
+  const unsigned long long mine = reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16*>(r.C) + r.base);
+  if (p.dual) {
+    constexpr int OUT = BN / 4;                   // output columns of this warp
+    if (!wait()) return false;
+    const int n_mats = p.store_gate_up ? 3 : 1;
+#pragma unroll 1
+    for (int c = 0; c < OUT; c += 64) {
+      const int col = n0 + half * OUT + c;
+      if (col >= p.N) break;
+#pragma unroll 1
+      for (int mat = 0; mat < n_mats; ++mat) {    // h, gate, up
+#pragma unroll 1
+        for (int part = 0; part < (OUT < 64 ? 1 : 2); ++part) {
+          const uint32_t ta = tacc + half * OUT + c + part * 32;
+          uint32_t r0[32], r1[32];                // gate and up; or only the one that is stored
+          float v[32];
+          tmem_ld_32x32(mat == 2 ? ta + BN / 2 : ta, r0);
+          if (mat == 0) {
+            tmem_ld_32x32(ta + BN / 2, r1);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float g = __uint_as_float(r0[i]);
+              v[i] = g / (1.0f + __expf(-g)) * __uint_as_float(r1[i]);
+            }
+          } else {
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r0[i]);
+          }
+          epi_stage_row<false>(stage, v, part, lane);
+        }
+        const void* out = mat == 0 ? p.C : (mat == 1 ? p.C2 : p.C3);
+        epi_flush(stage, reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(out) + r.base), row_ok, lane, col, min(p.N, n0 + (half + 1) * OUT));
+      }
+    }
+    return true;
+  }
+  constexpr int CHUNKS = BN / 128;                // 64-column chunks of this warp
+  const int col0 = n0 + half * (BN / 2);
+  const bool add = fast && (p.accumulate || p.R != nullptr);
+  const unsigned long long src = p.accumulate ? mine : reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(p.R) + r.base);
+  uint4 pre[8];                                   // (two chunks' worth of registers would spill, and serialise the loads)
+  if (add) epi_fetch(pre, src, row_ok, lane, col0, p.N, p.accumulate ? p.C : p.R);
+  if (!wait()) return false;
+#pragma unroll 1
+  for (int ch = 0; ch < CHUNKS; ++ch) {
+    const int col = col0 + ch * 64;
+    if (col >= p.N) break;
+    if (add) {
+      epi_stage_in(stage, pre, lane);
+      if (ch + 1 < CHUNKS) epi_fetch(pre, src, row_ok, lane, col + 64, p.N, p.accumulate ? p.C : p.R);
+    }
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+      uint32_t acc[32];
+      float v[32];
+      tmem_ld_32x32(tacc + half * (BN / 2) + ch * 64 + part * 32, acc);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]) * p.alpha;
+      if (add) {
+        epi_stage_row<true>(stage, v, part, lane);
+      } else if (fast) {
+        epi_stage_row<false>(stage, v, part, lane);
+      } else if (r.ok) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const int cc = col + part * 32 + w * 8;
+          if (cc < p.N) {
+            float o[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = v[w * 8 + i];
+            store8(r.C, r.base + cc, o, p.c_fp32, p.accumulate, p.R);
+          }
+        }
+      }
+      __syncwarp();   // the next TMEM load is warp-aligned
+    }
+    if (fast) epi_flush(stage, mine, row_ok, lane, col, p.N);
+  }
+  return true;
+}
+
+// Descriptor of a 64-deep operand tile in shared memory, and its step per 16 k (in descriptor units of 16 bytes; the
+// address field never carries out of its 14 bits, shared memory being smaller than 256 KB).
+__device__ __forceinline__ uint64_t operand_desc(uint32_t addr, int mn_major) {
+  return mn_major ? make_smem_desc(addr, 8192, 1024) : make_smem_desc(addr, 16, 1024);
+}
+__device__ __forceinline__ uint32_t operand_kstep(int mn_major) { return mn_major ? 2048 >> 4 : 32 >> 4; }
+
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
   constexpr int B_BYTES = BN * BK * 2;
@@ -249,13 +482,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  // [accumulator buffer][row quarter]: column halves whose rows have been delivered to peers.  A buffer's two halves
+  // count the same tile: a warp reaches the buffer's next tile only after both have released the accumulator.
+  unsigned* rows_done = reinterpret_cast<unsigned*>(tmem_slot + 2);
+  uint8_t* epi_stage = smem + STAGES * STAGE_BYTES + 256;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BN_OUT = p.dual ? BN / 2 : BN;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 4); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], EPI_WARPS); }
+    for (int i = 0; i < 8; ++i) rows_done[i] = 0;
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -270,12 +508,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
     if (p.status != nullptr) atomicCAS(p.status, 0, code);
   };
 
-  const bool dead = gemm_dead(p);
+  const bool dead = __any_sync(0xffffffffu, gemm_dead(p));
   if (dead) {
     // nothing to do; fall through to the common exit
-  } else if (warp == 0 && lane == 0) {
+  } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    prefetch_tensormap(&p.tmA); prefetch_tensormap(&p.tmB);
+    if (elect_one()) { prefetch_tensormap(&p.tmA); prefetch_tensormap(&p.tmB); }
     uint32_t it = 0;
     Work w;
     bool ok = true;
@@ -285,21 +523,20 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
       if (p.tile_ready != nullptr) {
         // rows of this tile are stored by peer GPUs: wait for them, then order the TMA reads after the acquire
         const int ti = t.m0 / BM;
-        if (!wait_ge(p.tile_ready + ti, (unsigned)p.tile_expected[ti], p.peer_wait_ns)) { fail(ST_TIMEOUT_PEER); ok = false; break; }
+        if (!__all_sync(0xffffffffu, wait_ge(p.tile_ready + ti, (unsigned)p.tile_expected[ti], p.peer_wait_ns))) { fail(ST_TIMEOUT_PEER); ok = false; break; }
         fence_proxy_async_all();
       }
       if (p.mode != 2 && total_kb > 0 && (p.rdy_b.ready != nullptr || p.rdy_b2.ready != nullptr || p.rdy_bl.ready != nullptr)) {
         // the weight operand is part of a buffer that an all-gather on another stream is still filling
-        if (!wait_b_tile(p, t.g, t.n0, BN_OUT)) { fail(ST_TIMEOUT_PEER); ok = false; break; }
+        if (!__all_sync(0xffffffffu, wait_b_tile(p, t.g, t.n0, BN_OUT))) { fail(ST_TIMEOUT_PEER); ok = false; break; }
         fence_proxy_async_all();
       }
       for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!wait_parity(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
+        if (!wait_parity_warp(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
         uint8_t* sA = smem + s * STAGE_BYTES;
         uint8_t* sB = sA + A_BYTES;
-        mbar_expect_tx(&full_bar[s], STAGE_BYTES);
         const bool lora = kb >= t.num_kb;
         const int kk = (lora ? kb - t.num_kb : kb) * BK;
         const CUtensorMap* mA = lora ? &p.tmA_l : &p.tmA;
@@ -308,29 +545,32 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
         const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
         const int krow = (lora ? 0 : t.krow0) + kk;
         const int zB = (p.mode == 2) ? 0 : t.g;
-        if (a_mn == 0) {
-          tma_load_2d(sA, mA, &full_bar[s], kk, t.m0);
-        } else {
-          tma_load_2d(sA, mA, &full_bar[s], t.m0, krow);
-          tma_load_2d(sA + 8192, mA, &full_bar[s], t.m0 + 64, krow);
-        }
-        if (b_mn == 0) {
-          if (p.dual) {
-            tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
-            tma_load_3d(sB + B_BYTES / 2, mB2, &full_bar[s], kk, t.n0, zB);
+        if (elect_one()) {
+          mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+          if (a_mn == 0) {
+            tma_load_2d(sA, mA, &full_bar[s], kk, t.m0);
           } else {
-            tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
+            tma_load_2d(sA, mA, &full_bar[s], t.m0, krow);
+            tma_load_2d(sA + 8192, mA, &full_bar[s], t.m0 + 64, krow);
           }
-        } else {
-          if (p.dual) {
-#pragma unroll
-            for (int c = 0; c < BN / 128; ++c) {
-              tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
-              tma_load_3d(sB + B_BYTES / 2 + c * 8192, mB2, &full_bar[s], t.n0 + 64 * c, krow, zB);
+          if (b_mn == 0) {
+            if (p.dual) {
+              tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
+              tma_load_3d(sB + B_BYTES / 2, mB2, &full_bar[s], kk, t.n0, zB);
+            } else {
+              tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
             }
           } else {
+            if (p.dual) {
 #pragma unroll
-            for (int c = 0; c < BN / 64; ++c) tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
+              for (int c = 0; c < BN / 128; ++c) {
+                tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
+                tma_load_3d(sB + B_BYTES / 2 + c * 8192, mB2, &full_bar[s], t.n0 + 64 * c, krow, zB);
+              }
+            } else {
+#pragma unroll
+              for (int c = 0; c < BN / 64; ++c) tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
+            }
           }
         }
       }
@@ -341,7 +581,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
         while (!mbar_try_wait(&full_bar[s], 0) && !mbar_try_wait(&full_bar[s], 1) && global_timer_ns() - t0 < 1000000ull) {}
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     uint32_t it = 0, acc_it = 0;
     Work w;
@@ -352,184 +592,124 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
       if (total_kb == 0) continue;
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
-      if (!wait_parity(&tempty_bar[buf], aph ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
+      if (!wait_parity_warp(&tempty_bar[buf], aph ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + buf * BN;
       for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!wait_parity(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
+        if (!wait_parity_warp(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
         tc_fence_after();
         const bool lora = kb >= t.num_kb;
         const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
         const uint32_t idesc = make_idesc_bf16(BM, BN, a_mn, b_mn);
         const uint32_t sA = smem_u32(smem + s * STAGE_BYTES);
-        const uint32_t sB = sA + A_BYTES;
+        const uint64_t da = operand_desc(sA, a_mn), db = operand_desc(sA + A_BYTES, b_mn);
+        const uint32_t ka = operand_kstep(a_mn), kbs = operand_kstep(b_mn);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t da = a_mn ? make_smem_desc(sA + k * 2048, 8192, 1024) : make_smem_desc(sA + k * 32, 16, 1024);
-          const uint64_t db = b_mn ? make_smem_desc(sB + k * 2048, 8192, 1024) : make_smem_desc(sB + k * 32, 16, 1024);
-          umma_bf16(d_tmem, da, db, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16(d_tmem, da + k * ka, db + k * kbs, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+          umma_commit(&empty_bar[s]);   // frees the stage when these MMAs have read it
         }
-        umma_commit(&empty_bar[s]);   // frees the stage when these MMAs have read it
       }
       if (!ok) break;
-      umma_commit(&tfull_bar[buf]);   // accumulator complete
+      if (elect_one()) umma_commit(&tfull_bar[buf]);   // accumulator complete
       ++acc_it;
     }
   } else if (warp >= 2) {
     // ------------------------------------------------------------------ epilogue
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint8_t* stage = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
     uint32_t acc_it = 0;
     Work w;
     for (int wi = 0; (p.dual ? get_work<BN / 2>(p, blockIdx.x, gridDim.x, wi, w) : get_work<BN>(p, blockIdx.x, gridDim.x, wi, w)); ++wi) {
       const Tile& t = w.t;
-      const int total_kb = w.kb1 - w.kb0;
       const int row = t.m0 + q * 32 + lane;
-      const int row_limit = (p.mode == 1) ? p.offsets[p.G] : p.M;
-      const bool row_ok = row < row_limit;
-      long long base = (p.mode == 2 ? (long long)t.g * p.c_group_stride : 0) + (long long)row * p.ldc;
-      void* Cout = p.C;
-      int dest = -1;
-      bool store_ok = row_ok;
-      if (p.row_dest_rank != nullptr) {          // result rows go straight into peers' buffers
-        dest = row_ok ? p.row_dest_rank[row] : -1;
-        const int drow = row_ok ? p.row_dest_row[row] : -1;
-        if (dest >= p.num_peers || drow < 0) dest = -1;
-        store_ok = dest >= 0;
-        if (store_ok) { Cout = reinterpret_cast<void*>(p.peer_out[dest]); base = (long long)drow * p.ldc; }
-      }
-      if (total_kb == 0) {
-        if (!p.accumulate && row_ok) {
-          float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-          for (int c = 0; c < BN_OUT; c += 8)
-            if (t.n0 + c < p.N) store8(p.C, base + t.n0 + c, z, p.c_fp32, 0);
-        }
+      const bool row_ok = row < ((p.mode == 1) ? p.offsets[p.G] : p.M);
+      const EpiRow r = epi_row(p, t.g, row, row_ok);
+      if (w.kb1 == w.kb0) {
+        if (p.dual) epi_zero<BN / 4>(p, r, row_ok, t.n0 + half * (BN / 4));
+        else epi_zero<BN / 2>(p, r, row_ok, t.n0 + half * (BN / 2));
         continue;
       }
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
-      if (!wait_parity(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
-      __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-      if (p.dual) {
+      auto wait = [&]() {
+        if (!wait_parity(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
+        __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
+        tc_fence_after();
+        return true;
+      };
+      const uint32_t tacc = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
+      bool publish = p.row_dest_rank != nullptr;
+      if (w.split >= 0) {
+        // A piece of a shared tile: add the partial sums into the tile's fp32 workspace (four columns of a row at a time,
+        // rows adjacent, so that a warp's reduction covers 512 contiguous bytes), release the accumulator, count this
+        // warp in, and if it is the last of the contributors to its part, read the sums back and finish that part.
+        // Each (32-row quarter, column half) has its own counter, so no warp ever has to meet another one of its CTA.
+        if (!wait()) break;
+        float4* ws = reinterpret_cast<float4*>(p.sk_ws) + (long long)w.split * (BM * BN / 4) + half * (BN / 8) * BM + (q * 32 + lane);
 #pragma unroll 1
         for (int c = 0; c < BN / 2; c += 32) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(taddr + c, rg);
-          tmem_ld_32x32(taddr + BN / 2 + c, ru);
-          tmem_ld_wait();
-          if (row_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float h[8], gg[8], uu[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  gg[i] = __uint_as_float(rg[v * 8 + i]);
-                  uu[i] = __uint_as_float(ru[v * 8 + i]);
-                  h[i] = gg[i] / (1.0f + __expf(-gg[i])) * uu[i];
-                }
-                store8(p.C, base + col, h, 0, 0);
-                if (p.store_gate_up) { store8(p.C2, base + col, gg, 0, 0); store8(p.C3, base + col, uu, 0, 0); }
-              }
-            }
-          }
-          __syncwarp();   // the next TMEM load is warp-aligned
-        }
-      } else if (w.split >= 0) {
-        // A piece of a shared tile: add the partial sums into the tile's fp32 workspace (column-major inside the tile,
-        // so that the 32 rows of a warp are 128 contiguous bytes), release the accumulator, count this CTA in, and
-        // if it is the last one of the tile's contributors, read the sums back and finish the tile.
-        float* ws = p.sk_ws + (long long)w.split * (BM * BN) + (q * 32 + lane);
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c, r);
+          uint32_t acc[32];
+          tmem_ld_32x32(tacc + half * (BN / 2) + c, acc);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) atomicAdd(ws + (c + i) * BM, __uint_as_float(r[i]));
+          for (int i = 0; i < 32; i += 4)
+            red_add_v4_f32(reinterpret_cast<float*>(ws + (c + i) / 4 * BM), __uint_as_float(acc[i]), __uint_as_float(acc[i + 1]),
+                           __uint_as_float(acc[i + 2]), __uint_as_float(acc[i + 3]));
           __syncwarp();
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         ++acc_it;
-        // Each 32-row quarter of the tile has its own counter, so a warp never has to meet the other warps of its CTA:
-        // the warp that arrives last at its quarter finishes that quarter.
         __threadfence();
         __syncwarp();
+        unsigned* ctr = p.sk_ctr + w.split * SPLIT_COUNTERS;
         unsigned before = 0;
-        if (lane == 0) before = atomicAdd(p.sk_ctr + w.split * 4 + q, 1u);
+        if (lane == 0) before = atomicAdd(ctr + q * 2 + half, 1u);
         before = __shfl_sync(0xffffffffu, before, 0);
-        const bool last = before == (unsigned)w.contributors - 1u;
-        if (!last) continue;
+        if (before != (unsigned)w.contributors - 1u) continue;
         __threadfence();
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          float acc[32];
+        for (int c = 0; c < BN / 2; c += 8) {
+          float o[8];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) { acc[i] = __ldcg(ws + (c + i) * BM); __stcg(ws + (c + i) * BM, 0.f); }   // leave the workspace clean
-          if (store_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = acc[v * 8 + i] * p.alpha;
-                store8(Cout, base + col, o, p.c_fp32, p.accumulate, p.R);
-              }
-            }
+          for (int i = 0; i < 8; i += 4) {
+            float4* src = ws + (c + i) / 4 * BM;
+            const float4 v = __ldcg(src);
+            __stcg(src, make_float4(0.f, 0.f, 0.f, 0.f));   // leave the workspace clean
+            o[i] = v.x * p.alpha; o[i + 1] = v.y * p.alpha; o[i + 2] = v.z * p.alpha; o[i + 3] = v.w * p.alpha;
           }
+          const int col = t.n0 + half * (BN / 2) + c;
+          if (r.ok && col < p.N) store8(r.C, r.base + col, o, p.c_fp32, p.accumulate, p.R);
         }
         __syncwarp();
-        if (lane == 0) p.sk_ctr[w.split * 4 + q] = 0;
-        if (p.row_dest_rank != nullptr) {
+        if (lane == 0) ctr[q * 2 + half] = 0;
+        if (publish) {          // by the half that finishes second
           __threadfence_system();
           __syncwarp();
-          for (int d = 0; d < p.num_peers; ++d) {
-            const unsigned m = __ballot_sync(0xffffffffu, dest == d);
-            if (lane == 0 && m != 0) red_add_release_sys(reinterpret_cast<unsigned*>(p.peer_arrive[d]), __popc(m));
-          }
+          if (lane == 0) { before = atomicAdd(ctr + 8 + q, 1u); if (before == 1u) ctr[8 + q] = 0; }
+          before = __shfl_sync(0xffffffffu, before, 0);
+          if (before == 1u) epi_publish(p, r.dest, lane);
         }
         continue;
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c, r);
-          tmem_ld_wait();
-          if (store_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[v * 8 + i]) * p.alpha;
-                store8(Cout, base + col, o, p.c_fp32, p.accumulate, p.R);
-              }
-            }
-          }
-          __syncwarp();   // the next TMEM load is warp-aligned
-        }
+      }
+      if (!epi_tile<BN>(p, stage, tacc, half, lane, t.n0, r, wait)) break;
+      if (publish) {            // by the half that finishes second (before the accumulator is released, see rows_done)
+        __threadfence_system();
+        __syncwarp();
+        unsigned before = 0;
+        if (lane == 0) before = atomicAdd(&rows_done[buf * 4 + q], 1u);
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if (before & 1u) epi_publish(p, r.dest, lane);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[buf]);
       ++acc_it;
-      if (p.row_dest_rank != nullptr) {
-        // publish this warp's rows: one count per (row, column tile) and destination
-        __threadfence_system();
-        __syncwarp();
-        for (int d = 0; d < p.num_peers; ++d) {
-          const unsigned m = __ballot_sync(0xffffffffu, dest == d);
-          if (lane == 0 && m != 0) red_add_release_sys(reinterpret_cast<unsigned*>(p.peer_arrive[d]), __popc(m));
-        }
-      }
     }
   }
 
@@ -542,73 +722,24 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
 // CTA-pair variant (cta_group::2).  Two CTAs of a cluster share one 256 x 256 MMA tile: each CTA loads its own
 // 128 rows of A and half of B's 256 columns (in the dual mode: the leader the gate matrix, its peer the up
 // matrix), the leader's MMA thread reads both CTAs' shared memory, and each CTA's TMEM receives the accumulators
-// of its own 128 rows.  Per CTA and 64-deep k block that is 32 KB of operands instead of 48 KB, which is what
-// bounds the single-CTA kernel, and the ring holds 7 stages instead of 4.
+// of its own 128 rows.  Per CTA and 64-deep k block that is 32 KB of operands instead of 48 KB.  What bounds the
+// single-CTA kernel is the ~64 bytes per clock that an SM takes in (0.38 us for 48 KB; with the MMAs left out it runs
+// no faster), and a 256 x 256 tile in one CTA is bound by shared memory (64 KB written, 96 KB read by the MMAs per k
+// block).  The pair needs 64 KB of either for 512 clocks of MMA.  8192^3: 1634 TFLOP/s (128-row kernel 1390, torch's
+// library call 1670); 9200 x 4096 x 4096: 183 us, 1684 TFLOP/s (before: 212 us).  Its roles run as whole warps: with a
+// single lane in the loops (922 us at 8192^3) the issue of the MMAs was the limit.
 //   full_bar[s]   (leader's is used): the leader's producer arrives and announces both CTAs' TMA bytes
 //   empty_bar[s]  (one per CTA)     : arrives by the leader's commit, delivered to both CTAs
 //   tfull_bar[b]  (one per CTA)     : same, when a tile's accumulators are complete
-//   tempty_bar[b] (leader's is used): 8 arrivals, the 4 epilogue warps of each CTA
+//   tempty_bar[b] (leader's is used): 16 arrivals, the 8 epilogue warps of each CTA
 // Every load lands in the shared memory of the CTA that issued it.
 // ---------------------------------------------------------------------------------------------
 constexpr int PAIR_BN = 256;
-constexpr int PAIR_STAGES = 7;
+constexpr int PAIR_STAGES = 6;
 constexpr int PAIR_B_BYTES = 128 * BK * 2;
 constexpr int PAIR_STAGE_BYTES = A_BYTES + PAIR_B_BYTES;
-static_assert(PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256 <= 227 * 1024, "pair kernel: stages + barriers exceed the shared memory of a CTA");
-
-struct PairTile {
-  int g, m0, n0, krow0, num_kb, num_kb_l, second_ok;
-};
-
-// Pair tiles cover 256 rows.  In the grouped-rows mode a pair never straddles two groups: a group with an odd
-// number of 128-row blocks ends with a pair whose second half is idle (second_ok = 0).
-template <int BN_OUT>
-__host__ __device__ __forceinline__ bool get_pair_tile(const GemmParams& p, int t, PairTile& o) {
-  const int n_blocks = (p.N + BN_OUT - 1) / BN_OUT;
-  o.num_kb_l = (p.K_l + BK - 1) / BK;
-  o.second_ok = 1;
-  if (p.mode == 2) {
-    const int m_pairs = (p.M + 2 * BM - 1) / (2 * BM);
-    const int per_group = m_pairs * n_blocks;
-    if (t >= per_group * p.G) return false;
-    o.g = t / per_group;
-    const int r = t - o.g * per_group;
-    o.m0 = (r % m_pairs) * 2 * BM;
-    o.n0 = (r / m_pairs) * BN_OUT;
-    int k_begin = 0, k_end = p.K;
-    if (p.offsets != nullptr) { k_begin = p.offsets[o.g]; k_end = p.offsets[o.g + 1]; }
-    o.krow0 = k_begin;
-    o.num_kb = (k_end - k_begin + BK - 1) / BK;
-    return true;
-  }
-  o.krow0 = 0;
-  o.num_kb = (p.K + BK - 1) / BK;
-  if (p.mode == 0) {
-    const int m_pairs = (p.M + 2 * BM - 1) / (2 * BM);
-    if (t >= m_pairs * n_blocks) return false;
-    o.g = 0;
-    o.m0 = (t % m_pairs) * 2 * BM;
-    o.n0 = (t / m_pairs) * BN_OUT;
-    return true;
-  }
-  int total = 0;
-  for (int g = 0; g < p.G; ++g) total += ((p.offsets[g + 1] - p.offsets[g]) / BM + 1) / 2;
-  if (total == 0 || t >= total * n_blocks) return false;
-  int mp = t % total;
-  o.n0 = (t / total) * BN_OUT;
-  for (int g = 0; g < p.G; ++g) {
-    const int begin = p.offsets[g], end = p.offsets[g + 1];
-    const int pairs = ((end - begin) / BM + 1) / 2;
-    if (mp < pairs) {
-      o.g = g;
-      o.m0 = begin + mp * 2 * BM;
-      o.second_ok = (o.m0 + BM < end) ? 1 : 0;
-      return true;
-    }
-    mp -= pairs;
-  }
-  return false;
-}
+constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES;
+static_assert(PAIR_SMEM <= 227 * 1024, "pair kernel: stages + barriers + epilogue stages exceed the shared memory of a CTA");
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_pair_kernel(const __grid_constant__ GemmParams p) {
   constexpr int STAGES = PAIR_STAGES;
@@ -624,6 +755,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   uint64_t* tempty_bar = tfull_bar + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  unsigned* rows_done = reinterpret_cast<unsigned*>(tmem_slot + 2);   // as in the 128-row kernel
+  uint8_t* epi_stage = smem + STAGES * PAIR_STAGE_BYTES + 256;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta_rank = cluster_ctarank();          // 0 = leader
@@ -632,7 +765,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * EPI_WARPS); }
+    for (int i = 0; i < 8; ++i) rows_done[i] = 0;
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -647,12 +781,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     if (p.status != nullptr) atomicCAS(p.status, 0, code);
   };
 
-  const bool dead = gemm_dead(p);   // the same in both CTAs of the pair: the word never returns to zero while kernels run
+  const bool dead = __any_sync(0xffffffffu, gemm_dead(p));   // the same in both CTAs of the pair: the word never returns to zero while kernels run
   if (dead) {
     // nothing to do; fall through to the common exit
-  } else if (warp == 0 && lane == 0) {
+  } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (one per CTA)
-    prefetch_tensormap(&p.tmA); prefetch_tensormap(&p.tmB);
+    if (elect_one()) { prefetch_tensormap(&p.tmA); prefetch_tensormap(&p.tmB); }
     uint32_t it = 0;
     PairTile t;
     bool ok = true;
@@ -662,17 +796,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
       const bool half_ok = cta_rank == 0 || t.second_ok;
       if (p.tile_ready != nullptr && half_ok && total_kb > 0) {
         const int ti = my_m0 / BM;
-        if (!wait_ge(p.tile_ready + ti, (unsigned)p.tile_expected[ti], p.peer_wait_ns)) { fail(ST_TIMEOUT_PEER); ok = false; break; }
+        if (!__all_sync(0xffffffffu, wait_ge(p.tile_ready + ti, (unsigned)p.tile_expected[ti], p.peer_wait_ns))) { fail(ST_TIMEOUT_PEER); ok = false; break; }
         fence_proxy_async_all();
       }
       if (p.mode != 2 && total_kb > 0 && (p.rdy_b.ready != nullptr || p.rdy_b2.ready != nullptr || p.rdy_bl.ready != nullptr)) {
-        if (!wait_b_tile(p, t.g, t.n0, BN_OUT)) { fail(ST_TIMEOUT_PEER); ok = false; break; }
+        if (!__all_sync(0xffffffffu, wait_b_tile(p, t.g, t.n0, BN_OUT))) { fail(ST_TIMEOUT_PEER); ok = false; break; }
         fence_proxy_async_all();
       }
       for (int kb = 0; kb < total_kb; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!wait_parity(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
+        if (!wait_parity_warp(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
         uint8_t* sA = smem + s * PAIR_STAGE_BYTES;
         uint8_t* sB = sA + A_BYTES;
         // Only the leader arrives, announcing both CTAs' bytes: a cluster-scope arrive from the peer would put a
@@ -680,28 +814,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
         // leader's announcement (the transaction count goes negative for a moment; the phase cannot complete
         // before the leader's arrival).
         const uint32_t bar = mapa_shared(smem_u32(&full_bar[s]), 0);
-        if (cta_rank == 0) mbar_expect_tx(&full_bar[s], 2 * PAIR_STAGE_BYTES);
         const bool lora = kb >= t.num_kb;
         const int kk = (lora ? kb - t.num_kb : kb) * BK;
         const CUtensorMap* mA = lora ? &p.tmA_l : &p.tmA;
         const CUtensorMap* mB = lora ? &p.tmB_l : &p.tmB;
         const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
         const int krow = (lora ? 0 : t.krow0) + kk;
-        if (a_mn == 0) {
-          tma_load_2d_pair(sA, mA, bar, kk, my_m0);
-        } else {
-          tma_load_2d_pair(sA, mA, bar, my_m0, krow);
-          tma_load_2d_pair(sA + 8192, mA, bar, my_m0 + 64, krow);
-        }
         const int zB = (p.mode == 2) ? 0 : t.g;
         // this CTA's half of B: columns n0 + 128*rank, or in the dual mode the gate (leader) / up (peer) matrix
         if (p.dual && cta_rank == 1) mB = lora ? &p.tmB2_l : &p.tmB2;
         const int my_n0 = p.dual ? t.n0 : t.n0 + (int)cta_rank * 128;
-        if (b_mn == 0) {
-          tma_load_3d_pair(sB, mB, bar, kk, my_n0, zB);
-        } else {
-          tma_load_3d_pair(sB, mB, bar, my_n0, krow, zB);
-          tma_load_3d_pair(sB + 8192, mB, bar, my_n0 + 64, krow, zB);
+        if (elect_one()) {
+          if (cta_rank == 0) mbar_expect_tx(&full_bar[s], 2 * PAIR_STAGE_BYTES);
+          if (a_mn == 0) {
+            tma_load_2d_pair(sA, mA, bar, kk, my_m0);
+          } else {
+            tma_load_2d_pair(sA, mA, bar, my_m0, krow);
+            tma_load_2d_pair(sA + 8192, mA, bar, my_m0 + 64, krow);
+          }
+          if (b_mn == 0) {
+            tma_load_3d_pair(sB, mB, bar, kk, my_n0, zB);
+          } else {
+            tma_load_3d_pair(sB, mB, bar, my_n0, krow, zB);
+            tma_load_3d_pair(sB + 8192, mB, bar, my_n0 + 64, krow, zB);
+          }
         }
       }
     }
@@ -709,7 +845,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
       const uint64_t t0 = global_timer_ns();
       while (global_timer_ns() - t0 < 2000000ull) {}
     }
-  } else if (warp == 1 && lane == 0 && cta_rank == 0) {
+  } else if (warp == 1 && cta_rank == 0) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     uint32_t it = 0, acc_it = 0;
     PairTile t;
@@ -719,127 +855,68 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
       if (total_kb == 0) continue;
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
-      if (!wait_parity(&tempty_bar[buf], aph ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
+      if (!wait_parity_warp(&tempty_bar[buf], aph ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + buf * BN;
       for (int kb = 0; kb < total_kb; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
-        if (!wait_parity(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
+        if (!wait_parity_warp(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
         tc_fence_after();
         const bool lora = kb >= t.num_kb;
         const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
         const uint32_t idesc = make_idesc_bf16(2 * BM, BN, a_mn, b_mn);
         const uint32_t sA = smem_u32(smem + s * PAIR_STAGE_BYTES);
-        const uint32_t sB = sA + A_BYTES;
+        const uint64_t da = operand_desc(sA, a_mn), db = operand_desc(sA + A_BYTES, b_mn);
+        const uint32_t ka = operand_kstep(a_mn), kbs = operand_kstep(b_mn);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t da = a_mn ? make_smem_desc(sA + k * 2048, 8192, 1024) : make_smem_desc(sA + k * 32, 16, 1024);
-          const uint64_t db = b_mn ? make_smem_desc(sB + k * 2048, 8192, 1024) : make_smem_desc(sB + k * 32, 16, 1024);
-          umma_bf16_pair(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16_pair(d_tmem, da + k * ka, db + k * kbs, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty_bar[s], 3);   // frees the stage in both CTAs
         }
-        umma_commit_pair(&empty_bar[s], 3);   // frees the stage in both CTAs
       }
       if (!ok) break;
-      umma_commit_pair(&tfull_bar[buf], 3);   // accumulators complete, in both CTAs
+      if (elect_one()) umma_commit_pair(&tfull_bar[buf], 3);   // accumulators complete, in both CTAs
       ++acc_it;
     }
   } else if (warp >= 2) {
     // ------------------------------------------------------------------ epilogue (both CTAs, own 128 rows)
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint8_t* stage = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
     uint32_t acc_it = 0;
     PairTile t;
     for (int tile = pair_id; (p.dual ? get_pair_tile<BN / 2>(p, tile, t) : get_pair_tile<BN>(p, tile, t)); tile += num_pairs) {
       const int total_kb = t.num_kb + (t.num_kb > 0 || p.mode != 2 ? t.num_kb_l : 0);
-      const bool half_ok = cta_rank == 0 || t.second_ok;
       const int row = t.m0 + (int)cta_rank * BM + q * 32 + lane;
-      const int row_limit = (p.mode == 1) ? p.offsets[p.G] : p.M;
-      const bool row_ok = half_ok && row < row_limit;
-      long long base = (p.mode == 2 ? (long long)t.g * p.c_group_stride : 0) + (long long)row * p.ldc;
-      void* Cout = p.C;
-      int dest = -1;
-      bool store_ok = row_ok;
-      if (p.row_dest_rank != nullptr) {          // result rows go straight into peers' buffers
-        dest = row_ok ? p.row_dest_rank[row] : -1;
-        const int drow = row_ok ? p.row_dest_row[row] : -1;
-        if (dest >= p.num_peers || drow < 0) dest = -1;
-        store_ok = dest >= 0;
-        if (store_ok) { Cout = reinterpret_cast<void*>(p.peer_out[dest]); base = (long long)drow * p.ldc; }
-      }
+      const bool row_ok = (cta_rank == 0 || t.second_ok) && row < ((p.mode == 1) ? p.offsets[p.G] : p.M);
+      const EpiRow r = epi_row(p, t.g, row, row_ok);
       if (total_kb == 0) {
-        if (!p.accumulate && row_ok) {
-          float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-          for (int c = 0; c < BN_OUT; c += 8)
-            if (t.n0 + c < p.N) store8(p.C, base + t.n0 + c, z, p.c_fp32, 0);
-        }
+        if (p.dual) epi_zero<BN / 4>(p, r, row_ok, t.n0 + half * (BN / 4));
+        else epi_zero<BN / 2>(p, r, row_ok, t.n0 + half * (BN / 2));
         continue;
       }
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
-      if (!wait_parity(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
-      __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-      if (p.dual) {
-#pragma unroll 1
-        for (int c = 0; c < BN / 2; c += 32) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(taddr + c, rg);
-          tmem_ld_32x32(taddr + BN / 2 + c, ru);
-          tmem_ld_wait();
-          if (row_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float h[8], gg[8], uu[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  gg[i] = __uint_as_float(rg[v * 8 + i]);
-                  uu[i] = __uint_as_float(ru[v * 8 + i]);
-                  h[i] = gg[i] / (1.0f + __expf(-gg[i])) * uu[i];
-                }
-                store8(p.C, base + col, h, 0, 0);
-                if (p.store_gate_up) { store8(p.C2, base + col, gg, 0, 0); store8(p.C3, base + col, uu, 0, 0); }
-              }
-            }
-          }
-          __syncwarp();   // the next TMEM load is warp-aligned
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c, r);
-          tmem_ld_wait();
-          if (store_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[v * 8 + i]) * p.alpha;
-                store8(Cout, base + col, o, p.c_fp32, p.accumulate, p.R);
-              }
-            }
-          }
-          __syncwarp();   // the next TMEM load is warp-aligned
-        }
+      auto wait = [&]() {
+        if (!wait_parity(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
+        __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
+        tc_fence_after();
+        return true;
+      };
+      if (!epi_tile<BN>(p, stage, tmem_base + buf * BN + ((uint32_t)(q * 32) << 16), half, lane, t.n0, r, wait)) break;
+      if (p.row_dest_rank != nullptr) {            // by the half that finishes second (see the 128-row kernel)
+        __threadfence_system();
+        __syncwarp();
+        unsigned before = 0;
+        if (lane == 0) before = atomicAdd(&rows_done[buf * 4 + q], 1u);
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if (before & 1u) epi_publish(p, r.dest, lane);
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
       ++acc_it;
-      if (p.row_dest_rank != nullptr) {
-        // publish this warp's rows: one count per (row, column tile) and destination
-        __threadfence_system();
-        __syncwarp();
-        for (int d = 0; d < p.num_peers; ++d) {
-          const unsigned m = __ballot_sync(0xffffffffu, dest == d);
-          if (lane == 0 && m != 0) red_add_release_sys(reinterpret_cast<unsigned*>(p.peer_arrive[d]), __popc(m));
-        }
-      }
     }
   }
 
@@ -848,340 +925,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   tc_fence_before();
   cluster_sync_all();
   if (warp == 1) { tc_fence_after(); tmem_dealloc_pair(tmem_base, TMEM_COLS); }
-}
-
-// ---------------------------------------------------------------------------------------------
-// Tall variant: one CTA computes a 256 x 256 tile as two 128-row MMAs that share the B operand.  Per 64-deep
-// k block the CTA takes in 64 KB for 256 x 256 x 64 MACs, i.e. 32 KB per 128 x 256 x 64, against 48 KB in the
-// 128 x 256 kernel, whose k blocks arrive more slowly than its MMAs retire them.  The two accumulators fill
-// all 512 TMEM columns, so the epilogue of a tile does not overlap the next tile's MMAs (its loads do); eight
-// epilogue warps (two per TMEM lane quarter, one per 128-row half) keep that phase short.
-// Roles of the 320 threads: warp 0 = TMA producer, warp 1 = MMA issuer (owns TMEM), warps 2-9 = epilogue.
-// ---------------------------------------------------------------------------------------------
-// Coalesced bf16 store of one 32-row x 32-column block held as one row per lane: the warp transposes it through a
-// 2 KB shared-memory stage (16-byte slots, XOR-swizzled so that both passes are conflict-free) and then writes
-// 64 contiguous bytes per row, eight rows per instruction, instead of 16 bytes to each of 32 rows.
-// row_ptr[i] / bit i of ok_mask describe row i*8 + lane/4, the row this lane stores in pass i.
-__device__ __forceinline__ void store32_coalesced(uint8_t* stage, const float (&v)[32], int lane, const unsigned long long (&row_ptr)[4],
-                                                  unsigned ok_mask, int col0, int N) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    uint4 out;
-    __nv_bfloat162* q = reinterpret_cast<__nv_bfloat162*>(&out);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) q[i] = __floats2bfloat162_rn(v[j * 8 + 2 * i], v[j * 8 + 2 * i + 1]);
-    *reinterpret_cast<uint4*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = out;
-  }
-  __syncwarp();
-  const int j = lane & 3;
-  const int col = col0 + j * 8;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = i * 8 + (lane >> 2);
-    const uint4 val = *reinterpret_cast<const uint4*>(stage + row * 64 + ((j ^ ((row >> 1) & 3)) << 4));
-    if (((ok_mask >> i) & 1u) && col < N)
-      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(row_ptr[i]) + col) = val;
-  }
-  __syncwarp();
-}
-
-constexpr int TALL_THREADS = 320;
-constexpr int TALL_STAGES = 3;
-constexpr int TALL_BN = 256;
-constexpr int TALL_STAGE_BYTES = 2 * A_BYTES + TALL_BN * BK * 2;
-static_assert(TALL_STAGES * TALL_STAGE_BYTES + 1024 + 256 + 8 * 2048 <= 227 * 1024, "tall kernel: stages + barriers + store stage exceed the shared memory of a CTA");
-static_assert(TALL_THREADS == 32 * (2 + 8), "tall kernel: producer, MMA issuer and eight epilogue warps");
-
-__global__ void __launch_bounds__(TALL_THREADS, 1) gemm_sm100_tall_kernel(const __grid_constant__ GemmParams p) {
-  constexpr int STAGES = TALL_STAGES;
-  constexpr int BN = TALL_BN;
-  constexpr int B_BYTES = BN * BK * 2;
-  constexpr uint32_t TMEM_COLS = 2 * BN;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * TALL_STAGE_BYTES);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* tfull_bar = empty_bar + STAGES;
-  uint64_t* tempty_bar = tfull_bar + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  uint8_t* store_stage = smem + STAGES * TALL_STAGE_BYTES + 256;   // 8 epilogue warps x 2 KB
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int BN_OUT = p.dual ? BN / 2 : BN;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(tfull_bar, 1);
-    mbar_init(tempty_bar, 8);
-    *abort_flag = 0;
-    fence_barrier_init();
-  }
-  if (warp == 1) { tmem_alloc(tmem_slot, TMEM_COLS); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-
-  auto fail = [&](int code) {
-    *abort_flag = 1;
-    if (p.status != nullptr) atomicCAS(p.status, 0, code);
-  };
-
-  const bool dead = gemm_dead(p);
-  if (dead) {
-    // nothing to do; fall through to the common exit
-  } else if (warp == 0 && lane == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    prefetch_tensormap(&p.tmA); prefetch_tensormap(&p.tmB);
-    uint32_t it = 0;
-    PairTile t;
-    bool ok = true;
-    for (int tile = blockIdx.x; ok && (p.dual ? get_pair_tile<BN / 2>(p, tile, t) : get_pair_tile<BN>(p, tile, t)); tile += gridDim.x) {
-      const int total_kb = t.num_kb + (t.num_kb > 0 || p.mode != 2 ? t.num_kb_l : 0);
-      if (p.tile_ready != nullptr && total_kb > 0) {
-        for (int h = 0; h < (t.second_ok ? 2 : 1) && ok; ++h) {
-          const int ti = t.m0 / BM + h;
-          if (!wait_ge(p.tile_ready + ti, (unsigned)p.tile_expected[ti], p.peer_wait_ns)) { fail(ST_TIMEOUT_PEER); ok = false; }
-        }
-        if (!ok) break;
-        fence_proxy_async_all();
-      }
-      if (p.mode != 2 && total_kb > 0 && (p.rdy_b.ready != nullptr || p.rdy_b2.ready != nullptr || p.rdy_bl.ready != nullptr)) {
-        if (!wait_b_tile(p, t.g, t.n0, BN_OUT)) { fail(ST_TIMEOUT_PEER); ok = false; break; }
-        fence_proxy_async_all();
-      }
-      for (int kb = 0; kb < total_kb; ++kb, ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        if (!wait_parity(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
-        uint8_t* sA = smem + s * TALL_STAGE_BYTES;
-        uint8_t* sB = sA + 2 * A_BYTES;
-        mbar_expect_tx(&full_bar[s], TALL_STAGE_BYTES);
-        const bool lora = kb >= t.num_kb;
-        const int kk = (lora ? kb - t.num_kb : kb) * BK;
-        const CUtensorMap* mA = lora ? &p.tmA_l : &p.tmA;
-        const CUtensorMap* mB = lora ? &p.tmB_l : &p.tmB;
-        const CUtensorMap* mB2 = lora ? &p.tmB2_l : &p.tmB2;
-        const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
-        const int krow = (lora ? 0 : t.krow0) + kk;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int m0 = t.m0 + h * BM;
-          if (a_mn == 0) {
-            tma_load_2d(sA + h * A_BYTES, mA, &full_bar[s], kk, m0);
-          } else {
-            tma_load_2d(sA + h * A_BYTES, mA, &full_bar[s], m0, krow);
-            tma_load_2d(sA + h * A_BYTES + 8192, mA, &full_bar[s], m0 + 64, krow);
-          }
-        }
-        const int zB = (p.mode == 2) ? 0 : t.g;
-        if (b_mn == 0) {
-          if (p.dual) {
-            tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
-            tma_load_3d(sB + B_BYTES / 2, mB2, &full_bar[s], kk, t.n0, zB);
-          } else {
-            tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
-            tma_load_3d(sB + B_BYTES / 2, mB, &full_bar[s], kk, t.n0 + 128, zB);
-          }
-        } else {
-          if (p.dual) {
-#pragma unroll
-            for (int c = 0; c < BN / 128; ++c) {
-              tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
-              tma_load_3d(sB + B_BYTES / 2 + c * 8192, mB2, &full_bar[s], t.n0 + 64 * c, krow, zB);
-            }
-          } else {
-#pragma unroll
-            for (int c = 0; c < BN / 64; ++c) tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
-          }
-        }
-      }
-    }
-    if (!ok) {  // give copies already in flight a bounded time to land before the CTA exits
-      for (int s = 0; s < STAGES; ++s) {
-        uint64_t t0 = global_timer_ns();
-        while (!mbar_try_wait(&full_bar[s], 0) && !mbar_try_wait(&full_bar[s], 1) && global_timer_ns() - t0 < 1000000ull) {}
-      }
-    }
-  } else if (warp == 1 && lane == 0) {
-    // ------------------------------------------------------------------ MMA issuer
-    uint32_t it = 0, acc_it = 0;
-    PairTile t;
-    bool ok = true;
-    for (int tile = blockIdx.x; ok && (p.dual ? get_pair_tile<BN / 2>(p, tile, t) : get_pair_tile<BN>(p, tile, t)); tile += gridDim.x) {
-      const int total_kb = t.num_kb + (t.num_kb > 0 || p.mode != 2 ? t.num_kb_l : 0);
-      if (total_kb == 0) continue;
-      if (!wait_parity(tempty_bar, (acc_it & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
-      tc_fence_after();
-      for (int kb = 0; kb < total_kb; ++kb, ++it) {
-        const int s = it % STAGES;
-        const uint32_t ph = (it / STAGES) & 1;
-        if (!wait_parity(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
-        tc_fence_after();
-        const bool lora = kb >= t.num_kb;
-        const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
-        const uint32_t idesc = make_idesc_bf16(BM, BN, a_mn, b_mn);
-        const uint32_t sA = smem_u32(smem + s * TALL_STAGE_BYTES);
-        const uint32_t sB = sA + 2 * A_BYTES;
-#pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t db = b_mn ? make_smem_desc(sB + k * 2048, 8192, 1024) : make_smem_desc(sB + k * 32, 16, 1024);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint32_t a0 = sA + h * A_BYTES;
-            const uint64_t da = a_mn ? make_smem_desc(a0 + k * 2048, 8192, 1024) : make_smem_desc(a0 + k * 32, 16, 1024);
-            umma_bf16(tmem_base + h * BN, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          }
-        }
-        umma_commit(&empty_bar[s]);   // frees the stage when these MMAs have read it
-      }
-      if (!ok) break;
-      umma_commit(tfull_bar);         // both accumulators complete
-      ++acc_it;
-    }
-  } else if (warp >= 2) {
-    // ------------------------------------------------------------------ epilogue: warp -> (lane quarter, row half)
-    const int q = warp & 3;
-    const int h = (warp - 2) >> 2;
-    uint32_t acc_it = 0;
-    PairTile t;
-    for (int tile = blockIdx.x; (p.dual ? get_pair_tile<BN / 2>(p, tile, t) : get_pair_tile<BN>(p, tile, t)); tile += gridDim.x) {
-      const int total_kb = t.num_kb + (t.num_kb > 0 || p.mode != 2 ? t.num_kb_l : 0);
-      const bool half_ok = h == 0 || t.second_ok;
-      const int row = t.m0 + h * BM + q * 32 + lane;
-      const int row_limit = (p.mode == 1) ? p.offsets[p.G] : p.M;
-      const bool row_ok = half_ok && row < row_limit;
-      long long base = (p.mode == 2 ? (long long)t.g * p.c_group_stride : 0) + (long long)row * p.ldc;
-      void* Cout = p.C;
-      int dest = -1;
-      bool store_ok = row_ok;
-      if (p.row_dest_rank != nullptr) {          // result rows go straight into peers' buffers
-        dest = row_ok ? p.row_dest_rank[row] : -1;
-        const int drow = row_ok ? p.row_dest_row[row] : -1;
-        if (dest >= p.num_peers || drow < 0) dest = -1;
-        store_ok = dest >= 0;
-        if (store_ok) { Cout = reinterpret_cast<void*>(p.peer_out[dest]); base = (long long)drow * p.ldc; }
-      }
-      if (total_kb == 0) {
-        if (!p.accumulate && row_ok) {
-          float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-          for (int c = 0; c < BN_OUT; c += 8)
-            if (t.n0 + c < p.N) store8(p.C, base + t.n0 + c, z, p.c_fp32, 0);
-        }
-        continue;
-      }
-      if (!wait_parity(tfull_bar, acc_it & 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
-      __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + h * BN + ((uint32_t)(q * 32) << 16);
-      // bf16 results without accumulation go out through the coalescing stage; the row this lane stores in pass i
-      // is row i*8 + lane/4 of the warp's 32, whose address and validity come from the lane that owns it
-      const bool fast = !p.c_fp32 && !p.accumulate && p.R == nullptr;
-      uint8_t* stage = store_stage + (warp - 2) * 2048;
-      unsigned long long rptr[4] = {0, 0, 0, 0};
-      unsigned okm = 0;
-      if (fast) {
-        const unsigned long long mine = reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16*>(Cout) + base);
-        const int okv = (p.dual ? row_ok : store_ok) ? 1 : 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int src = i * 8 + (lane >> 2);
-          rptr[i] = __shfl_sync(0xffffffffu, mine, src);
-          okm |= (unsigned)(__shfl_sync(0xffffffffu, okv, src) & 1) << i;
-        }
-      }
-      if (p.dual) {
-        const long long d2 = reinterpret_cast<const char*>(p.C2) - reinterpret_cast<const char*>(p.C);
-        const long long d3 = reinterpret_cast<const char*>(p.C3) - reinterpret_cast<const char*>(p.C);
-#pragma unroll 1
-        for (int c = 0; c < BN / 2; c += 32) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(taddr + c, rg);
-          tmem_ld_32x32(taddr + BN / 2 + c, ru);
-          tmem_ld_wait();
-          if (fast) {
-            float hh[32], gg[32], uu[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              gg[i] = __uint_as_float(rg[i]);
-              uu[i] = __uint_as_float(ru[i]);
-              hh[i] = gg[i] / (1.0f + __expf(-gg[i])) * uu[i];
-            }
-            store32_coalesced(stage, hh, lane, rptr, okm, t.n0 + c, p.N);
-            if (p.store_gate_up) {
-              unsigned long long r2[4], r3[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) { r2[i] = rptr[i] + d2; r3[i] = rptr[i] + d3; }
-              store32_coalesced(stage, gg, lane, r2, okm, t.n0 + c, p.N);
-              store32_coalesced(stage, uu, lane, r3, okm, t.n0 + c, p.N);
-            }
-          } else if (row_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float hh[8], gg[8], uu[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                  gg[i] = __uint_as_float(rg[v * 8 + i]);
-                  uu[i] = __uint_as_float(ru[v * 8 + i]);
-                  hh[i] = gg[i] / (1.0f + __expf(-gg[i])) * uu[i];
-                }
-                store8(p.C, base + col, hh, 0, 0);
-                if (p.store_gate_up) { store8(p.C2, base + col, gg, 0, 0); store8(p.C3, base + col, uu, 0, 0); }
-              }
-            }
-          }
-          __syncwarp();   // the next TMEM load is warp-aligned
-        }
-      } else {
-#pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c, r);
-          tmem_ld_wait();
-          if (fast) {
-            float o[32];
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __uint_as_float(r[i]) * p.alpha;
-            store32_coalesced(stage, o, lane, rptr, okm, t.n0 + c, p.N);
-          } else if (store_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              const int col = t.n0 + c + v * 8;
-              if (col < p.N) {
-                float o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[v * 8 + i]) * p.alpha;
-                store8(Cout, base + col, o, p.c_fp32, p.accumulate, p.R);
-              }
-            }
-          }
-          __syncwarp();   // the next TMEM load is warp-aligned
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tempty_bar);
-      ++acc_it;
-      if (p.row_dest_rank != nullptr) {
-        // publish this warp's rows: one count per (row, column tile) and destination
-        __threadfence_system();
-        __syncwarp();
-        for (int d = 0; d < p.num_peers; ++d) {
-          const unsigned m = __ballot_sync(0xffffffffu, dest == d);
-          if (lane == 0 && m != 0) red_add_release_sys(reinterpret_cast<unsigned*>(p.peer_arrive[d]), __popc(m));
-        }
-      }
-    }
-  }
-
-  __syncwarp();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1274,7 +1017,7 @@ static bool split_workspace(cudaStream_t stream, SplitWorkspace* out) {
   if (it == g_split_ws.end()) {
     if (g_split_ws.size() >= 64) return false;          // more streams than expected: those products run unsplit
     SplitWorkspace w{nullptr, nullptr};
-    const size_t ws_bytes = (size_t)g_num_sms * BM * 256 * sizeof(float), ctr_bytes = (size_t)g_num_sms * 4 * sizeof(unsigned);
+    const size_t ws_bytes = (size_t)g_num_sms * BM * 256 * sizeof(float), ctr_bytes = (size_t)g_num_sms * SPLIT_COUNTERS * sizeof(unsigned);
     if (cudaMalloc(&w.ws, ws_bytes) != cudaSuccess) { cudaGetLastError(); return false; }
     if (cudaMalloc(&w.ctr, ctr_bytes) != cudaSuccess) { cudaGetLastError(); cudaFree(w.ws); return false; }
     cudaMemset(w.ws, 0, ws_bytes);
@@ -1287,7 +1030,8 @@ static bool split_workspace(cudaStream_t stream, SplitWorkspace* out) {
 
 template <int BN, int STAGES>
 static cudaError_t launch(const GemmParams& p, int grid, cudaStream_t stream) {
-  constexpr int smem = STAGES * (A_BYTES + BN * BK * 2) + 1024 + 256;
+  constexpr int smem = STAGES * (A_BYTES + BN * BK * 2) + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES;
+  static_assert(smem <= 227 * 1024, "stages + barriers + epilogue stages exceed the shared memory of a CTA");
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_sm100_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1299,26 +1043,13 @@ static cudaError_t launch(const GemmParams& p, int grid, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-static cudaError_t launch_tall(const GemmParams& p, int grid, cudaStream_t stream) {
-  constexpr int smem = TALL_STAGES * TALL_STAGE_BYTES + 1024 + 256 + 8 * 2048;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_tall_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  gemm_sm100_tall_kernel<<<grid, TALL_THREADS, smem, stream>>>(p);
-  ++g_launches;
-  return cudaGetLastError();
-}
-
 // Number of CTA pairs that can be resident at once (pairs never span GPCs, so this can be below SMs / 2); the
 // persistent grid is sized to it because tiles are assigned to pairs statically.
 static int g_max_pairs = 0;
 static int g_pair_cap = 0;   // optional upper bound set through mdt_gemm_set_pair_cap (0 = none)
 
 static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream_t stream) {
-  constexpr int smem = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256;
+  constexpr int smem = PAIR_SMEM;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_sm100_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -1346,20 +1077,65 @@ static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream
 static thread_local long long t_rows_hint = 0;
 
 // Which kernel takes the 256-wide tiles: 0 = the 128-row kernel always, 1 = the CTA-pair kernel where the shape
-// fills 256-row tiles, 2 = the CTA-pair kernel always (tests), 3 = the tall kernel where the shape fills
-// several waves of 256-row tiles (default), 4 = the tall kernel always (tests).  Initial value from MDT_GEMM_PAIR;
-// mdt_gemm_set_pair_policy() changes it.
+// fills 256-row tiles, 2 and 4 = the CTA-pair kernel always, 3 = the CTA-pair kernel where 256-row tiles win by a margin
+// even with an exposed epilogue, 5 = whichever is faster by the measured model (default).  Initial value from
+// MDT_GEMM_PAIR; mdt_gemm_set_pair_policy() changes it.
+constexpr int MAX_POLICY = 5;
 static int g_pair_policy = -1;
 static int pair_policy() {
   if (g_pair_policy < 0) {
     const char* e = getenv("MDT_GEMM_PAIR");
-    g_pair_policy = (e != nullptr && e[0] >= '0' && e[0] <= '4') ? e[0] - '0' : 3;
+    g_pair_policy = (e != nullptr && e[0] >= '0' && e[0] <= '0' + MAX_POLICY) ? e[0] - '0' : MAX_POLICY;
   }
   return g_pair_policy;
 }
 
-// Which kernel runs a product: 0 = 128-row tiles, 1 = CTA pair, 2 = tall 256 x 256 tiles.  Pure arithmetic on the
-// descriptor (no CUDA call), so that it can be examined without a GPU.
+// The default rule: rounds x time per round of either kernel, microseconds, as measured on B200.
+//   128-row kernel: 0.48 per 64-deep k block and CTA (bound by the 48 KB it brings in) + 1 per tile
+//   pair kernel:    0.34 per k block and pair (32 KB per CTA; near the tensor core's 0.27) + 2 per tile
+//   a tile takes at least its epilogue: 3.4 / 3.1, and 2.3 more where C is read as well
+//   weights arrive at no more than 5.6 TB/s, so below that the two are the same and the smaller tiles stay
+// E.g. gate/up of 8 experts, 4096 -> 14336: 400 tokens 342 against 387, 800 tokens 467 / 439, 2000 tokens 929 / 846, 9200
+// tokens 3058 / 2853; dense 9200 x 4096 x 4096 249 / 183; dense 1152 x 4096 x 4096 (144 or 80 tiles) 40 / 52.
+static bool pair_is_faster(const MdtGemmDesc* d, long long thread_rows_hint, int num_sms, int bn_out) {
+  const int G = d->G < 1 ? 1 : d->G;
+  const double pairs = num_sms / 2;
+  double rows = d->mode == 1 ? (double)d->capacity_rows : (double)d->M;
+  double depth = (double)d->K;
+  if (d->mode == 1) {
+    // row groups padded to 128: the capacity leaves 127 rows of padding for each; a hint says what to expect instead
+    rows = rows - 127.0 * G > G ? rows - 127.0 * G : G;
+    if (thread_rows_hint > 0 && (double)thread_rows_hint < rows) rows = (double)thread_rows_hint;
+  }
+  if (d->mode == 2 && d->offsets != nullptr) {
+    double n = (double)d->capacity_rows;
+    if (thread_rows_hint > 0 && (double)thread_rows_hint < n) n = (double)thread_rows_hint;
+    depth = n / G;
+  }
+  const double nb = (double)((d->N + bn_out - 1) / bn_out) * (d->mode == 2 ? G : 1);
+  double m1 = ceil(rows / BM), m2 = ceil(rows / (2 * BM));
+  if (d->mode == 1) {   // the last block of a group is half full on average
+    m1 = fmax(rows / BM + 0.5 * G, (double)G);
+    m2 = fmax(rows / (2 * BM) + 0.5 * G, (double)G);
+  }
+  const double kb = ceil(depth / BK) + ceil((double)d->K_l / BK);
+  const double more = d->accumulate ? 2.3 : 0.0;
+  const double e1 = m1 * nb / num_sms, e2 = m2 * nb / pairs;
+  // rounds: whole ones where the row count is known
+  double r1 = d->mode == 1 ? fmax(1.0, e1 + 0.3) : ceil(e1), r2 = d->mode == 1 ? fmax(1.0, e2 + 0.3) : ceil(e2);
+  double extra1 = 0.0;
+  if (split_enabled() && d->mode != 2 && !d->dual && e1 > 1.0 && e1 - floor(e1) < 0.875 && kb >= 8.0) {   // shared last round
+    r1 = e1 + (d->mode == 1 ? 0.38 : 0.08);
+    extra1 = 15.0;
+  }
+  const double weights = d->mode == 2 ? 0.0 : (double)d->K * d->N * G * (d->dual ? 4.0 : 2.0) / 5.6e6;
+  const double t1 = fmax(r1 * fmax(kb * 0.48 + 1.0, 3.4 + more) + extra1, weights);
+  const double t2 = fmax(r2 * fmax(kb * 0.34 + 2.0, 3.1 + more), weights);
+  return t2 < 0.97 * t1;
+}
+
+// Which kernel runs a product: 0 = 128-row tiles, otherwise the CTA pair (1: policies 1 and 2, 2: policies 3 to 5).
+// Pure arithmetic on the descriptor (no CUDA call), so that it can be examined without a GPU.
 static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows_hint, int num_sms) {
   const int G = d->G < 1 ? 1 : d->G;
   const int BN = (d->dual || d->N > 128) ? 256 : 128;
@@ -1371,14 +1147,11 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
   const bool fills = rows_hint >= 2 * BM && (d->mode != 1 || rows_hint >= (long long)G * 4 * BM);
   if (policy == 2 || (policy == 1 && fills)) return 1;
   if (policy == 4) return 2;
+  if (policy == 5) return pair_is_faster(d, thread_rows_hint, num_sms, bn_out) ? 2 : 0;
   if (policy != 3) return 0;
-  // The tall kernel retires k blocks faster (0.70 us per 256 x 256 x 64 against 0.47 us per 128 x 256 x 64, i.e.
-  // 1.3x per flop) but exposes its epilogue (~5 us per tile, ~14 with the SwiGLU epilogue) and halves the number
-  // of tiles, which changes how full the last wave is.  Where the row count is known (dense and depth-grouped
-  // products, and row-grouped ones whose caller gave the expected rows of a capacity-sized buffer) the two are
-  // compared by waves x time per tile; the typical win at one micro-batch's ~1300 expert rows is a product with
-  // 4096 output columns whose 160 tiles would need a second, almost empty wave.  Without a row count only
-  // products of >= 2048 rows and >= 3 waves of 128-row tiles take the tall kernel.
+  // Policy 3 weighs 256-row tiles as if they had no second accumulator (0.70 us per k block of a tile whose epilogue, ~5 us
+  // or ~14 with SwiGLU, is not hidden) and wants 10 % in return; without a row count it takes them for products of
+  // >= 2048 rows and >= 3 waves of 128-row tiles only.
   long long r = rows_hint;
   const bool hinted = d->mode == 1 && thread_rows_hint > 0;
   if (hinted && thread_rows_hint < r) r = thread_rows_hint;
@@ -1388,7 +1161,7 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
   const double nb = (double)((d->N + bn_out - 1) / bn_out) * (d->mode == 2 ? G : 1);
   const double depth = (d->mode == 2 && d->offsets != nullptr) ? (double)grouped_depth / G : (double)d->K;
   const double kb = ceil(depth / BK) + ceil((double)d->K_l / BK);
-  bool tall;
+  bool wide;
   if (d->mode != 1 || hinted) {
     const double sms = num_sms;
     const double slow_epilogue = (!d->c_fp32 && !d->accumulate) ? 0.0 : 6.0;   // the uncoalesced epilogue costs more
@@ -1401,11 +1174,11 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
     }
     const double t1 = rounds * (fmax(kb * 0.47, 2.0) + 1.0);
     const double t2 = ceil(ceil(blocks / 2 + (d->mode == 1 ? 0.25 * G : 0.0)) * nb / sms) * (kb * 0.70 + 5.0 + (d->dual ? 9.0 : 0.0) + slow_epilogue);
-    tall = r >= 2 * BM && kb >= 32.0 && t2 < 0.9 * t1;
+    wide = r >= 2 * BM && kb >= 32.0 && t2 < 0.9 * t1;
   } else {
-    tall = r >= 16 * BM && ceil(blocks) * nb >= 3.0 * num_sms && kb >= 32.0;
+    wide = r >= 16 * BM && ceil(blocks) * nb >= 3.0 * num_sms && kb >= 32.0;
   }
-  return tall ? 2 : 0;
+  return wide ? 2 : 0;
 }
 
 }  // namespace mdt
@@ -1424,7 +1197,7 @@ extern "C" int mdt_gemm_set_split(int on) {
 }
 extern "C" int mdt_gemm_set_pair_policy(int policy) {
   const int old = mdt::pair_policy();
-  if (policy >= 0 && policy <= 4) mdt::g_pair_policy = policy;
+  if (policy >= 0 && policy <= mdt::MAX_POLICY) mdt::g_pair_policy = policy;
   return old;
 }
 
@@ -1462,8 +1235,8 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   const int BN = (p.dual || p.N > 128) ? 256 : 128;
   const int bn_out = p.dual ? BN / 2 : BN;
   const int tiling = choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms);
-  const bool pair = tiling == 1, tall = tiling == 2;
-  const bool half_box = pair || tall;   // these kernels load B in 128-row boxes
+  const bool pair = tiling != 0;
+  const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
   int rc = 0;
   // A: [a_rows, a_cols] row-major, a_cols contiguous.  K-major: rows = M, cols = K.  MN-major: rows = depth, cols = M.
   rc |= make_map(&p.tmA, d->A, d->a_cols, d->a_rows, 1, d->lda, 0, 64, d->a_mn ? 64 : BM, 2);
@@ -1482,12 +1255,6 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   long long rows = (p.mode == 1) ? d->capacity_rows : p.M;
   long long tiles = ((rows + BM - 1) / BM) * ((p.N + bn_out - 1) / bn_out) * (p.mode == 2 ? p.G : 1);
   int grid = (int)(tiles < g_num_sms ? (tiles < 1 ? 1 : tiles) : g_num_sms);
-  if (tall) {
-    long long t256 = ((rows + 2 * BM - 1) / (2 * BM) + (p.mode == 1 ? p.G : 0)) * ((p.N + bn_out - 1) / bn_out) * (p.mode == 2 ? p.G : 1);
-    const int g = (int)(t256 < 1 ? 1 : (t256 > g_num_sms ? g_num_sms : t256));
-    cudaError_t e3 = launch_tall(p, g, stream);
-    return e3 == cudaSuccess ? 0 : -100 - (int)e3;
-  }
   if (pair) {
     long long pairs = ((rows + 2 * BM - 1) / (2 * BM) + (p.mode == 1 ? p.G : 0)) * ((p.N + bn_out - 1) / bn_out) * (p.mode == 2 ? p.G : 1);
     const int np = (int)(pairs < 1 ? 1 : (pairs > g_num_sms ? g_num_sms : pairs));

@@ -227,6 +227,24 @@ def test_gemm_tiling_choice_without_a_gpu():
     assert choose(0, 300, 128, 200, policy=4) == TILE128             # 128-wide outputs: only the 128-row kernel exists
 
 
+def test_gemm_default_tiling_follows_rounds_and_row_groups():
+    build = pytest.importorskip("moe_distributed_training_b200.ops.build")
+    try:
+        ext = build.load()
+    except Exception:  # noqa: BLE001
+        pytest.skip("extension not built")
+
+    def pair(mode, M, N, K, G=1, tokens=0, dual=False, acc=False):
+        cap = max(128, (2 * tokens + G * 127) // 128 * 128)
+        return ext.gemm_choose_tiling(mode, M, N, K, 0, G, cap, dual, False, acc, mode != 0, 5, 0, 148) != 0
+    assert pair(0, 9200, 4096, 4096) and pair(0, 1152, 32000, 4096)
+    assert not pair(0, 1152, 4096, 4096)                              # 144 tiles of 128 rows are one round, 80 of 256 two
+    assert not pair(0, 9200, 128, 4096)                               # 128-wide outputs: only the 128-row kernel
+    assert not pair(1, 0, 14336, 4096, G=8, tokens=300, dual=True)    # one block per expert: 256-row tiles half empty
+    assert pair(1, 0, 14336, 4096, G=8, tokens=2000, dual=True) and pair(1, 0, 4096, 14336, G=8, tokens=9200)
+    assert pair(2, 14336, 4096, 0, G=8, tokens=9200, acc=True)
+
+
 def test_profile_trace_flag_writes_a_trace(tmp_path):
     from moe_distributed_training_b200.train.run import run_training
     out = tmp_path / "traces"

@@ -204,6 +204,41 @@ def test_gemm_pair_kernel_matches_single_cta_kernel(ops, policy):
         _close(pair, single, 1e-3, f"pair kernel {name} vs single-CTA kernel")
 
 
+@pytest.mark.parametrize("policy", [0, 2, 5], ids=["tile128", "pair", "default"])
+@pytest.mark.parametrize("M,N,K", [(1, 136, 64), (127, 264, 72), (129, 200, 640), (257, 520, 128), (2305, 328, 192)])
+def test_gemm_epilogue_edges(ops, M, N, K, policy):
+    """Remainders of the 64-column chunks, 32-row quarters and 2048-row panels of the epilogue: plain, accumulating
+    (bf16 and fp32), with a residual, weight gradients, and the SwiGLU form with its gate / up outputs.  fp32 sums of at
+    most 640 products, one bf16 rounding (0.4 %) of each result; 2e-2 as for the other products."""
+    def run():
+        torch.manual_seed(M * 7 + N)
+        x, w, u = _rand(M, K), _rand(N, K, scale=0.05), _rand(N, K, scale=0.05)
+        res, old = _rand(M, N), _rand(M, N)
+        want = x.float() @ w.float().t()
+        _close(ops.mm_nt(x, w), want, name="plain")
+        _close(ops.mm_nt(x, w, residual=res), want + res.float(), name="residual")
+        out = old.clone()
+        ops._gemm(0, x, False, w, False, out, M, N, K, accumulate=True, alpha=0.5)
+        _close(out, old.float() + 0.5 * want, name="accumulate")
+        out = old.float()
+        ops._gemm(0, x, False, w, False, out, M, N, K, accumulate=True)
+        _close(out, old.float() + want, name="accumulate fp32")
+        d = _rand(M, N)
+        dw, old_w = torch.empty(N, K, dtype=torch.bfloat16, device=DEV), _rand(N, K)
+        ops.mm_tn(d, x, out=dw)
+        _close(dw, d.float().t() @ x.float(), name="weight gradient")
+        dw = old_w.clone()
+        ops.mm_tn(d, x, out=dw, accumulate=True)
+        _close(dw, old_w.float() + d.float().t() @ x.float(), name="weight gradient, accumulated")
+        h, g, v = (torch.full((M, N), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(3))
+        ops._gemm(0, x, False, w, False, h, M, N, K, B2=u, C2=g, C3=v)
+        up = x.float() @ u.float().t()
+        _close(g, want, name="gate"); _close(v, up, name="up")
+        _close(h, torch.nn.functional.silu(want) * up, name="swiglu")
+    _under_pair_policy(ops, policy, run)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("policy", [2, 4], ids=["pair", "tall"])
 @pytest.mark.parametrize("T,E,H,F,lora", [(600, 4, 256, 512, True), (1500, 8, 1024, 2048, False), (333, 3, 512, 1024, False)])
 def test_grouped_mlp_pair_kernel_matches_single_cta_kernel(ops, T, E, H, F, lora, policy):
