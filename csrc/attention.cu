@@ -34,14 +34,12 @@ constexpr int TILE_BYTES = AB * HD * 2;   // 32 KB
 constexpr int ATOM_BYTES = AB * 128;      // 16 KB: [128 rows x 64 bf16]
 
 struct AttnParams {
-  CUtensorMap tmQ, tmK, tmV, tmdO;
+  CUtensorMap tmQ, tmK, tmV;
   CUtensorMap tmK64, tmV64;                  // key / value maps with 64-row boxes (pipelined forward)
   const int* cu_seqlens;
   int num_seqs, heads_q, heads_kv;
-  float scale_log2e, scale;
-  bf16* o; float* lse;                       // forward outputs
-  const float* delta; const float* lse_in;   // backward inputs
-  float* dq; float* dk; float* dv;           // backward outputs (fp32, [T, heads_q, 128])
+  float scale_log2e;
+  bf16* o; float* lse;
   int* status;
 };
 
@@ -447,193 +445,414 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
 }
 
 // ------------------------------------------------------------------------------------------- backward
-__global__ void attn_delta_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, float* __restrict__ delta, long long rows) {
-  const int lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);   // (token, head) pair
-  if (row >= rows) return;
-  const uint2 a = reinterpret_cast<const uint2*>(o + row * HD)[lane];
-  const uint2 b = reinterpret_cast<const uint2*>(dout + row * HD)[lane];
-  const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a);
-  const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b);
-  float s = 0.f;
+// Three launches.  `attn_bwd_prepare_kernel` computes, per (128-row block, query head), delta = rowsum(o * do) and the
+// row statistics in log2 units, clears the block's fp32 dQ tile and ranks the blocks by the work they mean as key blocks.
+// `attn_bwd_kernel`: one CTA per (key block, HPC query heads of one kv head), most work first; its loop runs over the
+// query blocks at or below the diagonal of each of its heads.  `attn_bwd_finalize_kernel` converts.
+//
+// The loop keeps everything transposed (keys are the rows, i.e. the TMEM lanes), so that the probabilities never leave
+// TMEM: S^T = K Q^T, P^T = exp2(S^T - lse) is written back over S^T as bf16 and is the A operand of dV += P^T dO.  Only
+// dS^T goes through shared memory, where dK += dS^T Q reads it K-major and dQ = dS K reads the same bytes MN-major.
+// Per 128 x 128 block the five products take 5 x 512 clocks of tensor core and ~350 KB of shared-memory traffic (2800
+// clocks); the exponentials 1024 clocks.  16 warps:
+//   0-3 dQ: TMEM -> fp32 reductions into the block's tile (16-byte pieces of 32 adjacent rows: 512 bytes contiguous)
+//   4-11 softmax: warp -> (32 key rows, 64 of the 128 query columns)      12 TMA      13 MMA issue      14, 15 idle
+//   TMEM columns: [0,128) S^T, then P^T in [0,32) and [64,96);  [128,256) dP^T, then dQ;  [256,384) dV;  [384,512) dK
+// The tensor core works on dK_i, dQ_i while the softmax warps form P_{i+1}, and on dV_i, S_{i+1} while they form dS_i.
+// Measured (4 sequences of 1024-8192, 32 / 8 heads; one block at a time per CTA before): see the launch function.
+constexpr int BWD_THREADS = 512;
+constexpr int BWD_STATS = 2 * AB;                              // lse2 | delta of a block, floats
+constexpr int BWD_SMEM = 7 * TILE_BYTES + 2 * BWD_STATS * 4 + 256 + 768;   // (768: what alignment to 1024 may take)
+static_assert(BWD_SMEM <= 227 * 1024, "attention backward: shared memory of a CTA");
+constexpr int DQ_TILE = AB * HD;                               // fp32 elements, [column / 4][row][4]
+
+struct AttnBwdParams {
+  CUtensorMap tmQ, tmK, tmV, tmdO;
+  const int4* sched;            // by rank: {seq_start, seq_end, block, flat block}; seq_start < 0: none
+  const float* stats;           // [flat block][head][lse2 x 128 | delta x 128]
+  float* dq;                    // [flat block][head] tiles
+  float* dk; float* dv;         // fp32 partial sums [token][head set][128], or NULL: all heads of a kv head in one CTA
+  bf16* dk_out; bf16* dv_out;   // then the results [token][kv head][128]
+  int heads_q, heads_kv, hpc;   // hpc: query heads per CTA
+  float scale_log2e, scale;
+  int* status;
+};
+
+__global__ void __launch_bounds__(256) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
+                                                               const int* __restrict__ cu, int num_seqs, int heads, int4* __restrict__ sched,
+                                                               float* __restrict__ stats, float* __restrict__ dq) {
+  int seq_start, seq_end, blk;
+  const int flat = blockIdx.x, h = blockIdx.y;
+  if (!find_block(cu, num_seqs, flat, seq_start, seq_end, blk)) {
+    if (h == 0 && threadIdx.x == 0) sched[flat] = make_int4(-1, 0, 0, 0);
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (h == 0 && warp == 0) {
+    // rank by the number of query blocks that a key block meets, most first
+    const int n = (seq_end - seq_start + AB - 1) / AB - blk;
+    int rank = 0;
+    for (int s = lane; s < num_seqs; s += 32) {
+      const int nb = (cu[s + 1] - cu[s] + AB - 1) / AB;
+      rank += (nb > n ? nb - n : 0) + (cu[s] < seq_start && nb >= n ? 1 : 0);
+    }
 #pragma unroll
-  for (int i = 0; i < 2; ++i) { float2 x = __bfloat1622float2(pa[i]), y = __bfloat1622float2(pb[i]); s += x.x * y.x + x.y * y.y; }
+    for (int off = 16; off > 0; off >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, off);
+    if (lane == 0) sched[rank] = make_int4(seq_start, seq_end, blk, flat);
+  }
+  const long long tile = (long long)flat * heads + h;
+  // 16 lanes x 16 bytes hold a row, 16 rows per pass; all loads of the block are in flight at once
+  const int sub = lane & 15, r0 = warp * 2 + (lane >> 4);
+  uint4 a[8], b[8];
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) delta[row] = s;
+  for (int k = 0; k < 8; ++k) {
+    const long long row = (long long)(seq_start + blk * AB + k * 16 + r0);
+    const bool valid = row < seq_end;
+    const long long at = ((valid ? row : (long long)seq_start) * heads + h) * HD;
+    a[k] = reinterpret_cast<const uint4*>(o + at)[sub];
+    b[k] = reinterpret_cast<const uint4*>(dout + at)[sub];
+  }
+  float4* z = reinterpret_cast<float4*>(dq + tile * DQ_TILE);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < DQ_TILE / 4; i += 256) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  float* st = stats + tile * BWD_STATS;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int r = k * 16 + r0;
+    const long long row = (long long)(seq_start + blk * AB + r);
+    const bool valid = row < seq_end;
+    const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a[k]);
+    const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b[k]);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 x = __bfloat1622float2(pa[i]), y = __bfloat1622float2(pb[i]); s += x.x * y.x + x.y * y.y; }
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (sub == 0) { st[r] = valid ? lse[row * heads + h] * 1.4426950408889634f : 0.f; st[AB + r] = valid ? s : 0.f; }
+  }
 }
 
-__global__ void __launch_bounds__(128, 1) attn_bwd_kernel(const __grid_constant__ AttnParams p) {
-  int seq_start, seq_end, kb;
-  if (!find_block(p.cu_seqlens, p.num_seqs, blockIdx.x, seq_start, seq_end, kb)) return;
-  const int h = blockIdx.y, kvh = h / (p.heads_q / p.heads_kv);
+__global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
+  const int sets = p.heads_q / p.hpc;                      // head sets; the sets of a block are neighbours in the grid
+  const int4 work = p.sched[blockIdx.x / sets];
+  const int seq_start = work.x, seq_end = work.y, kb = work.z;
+  if (seq_start < 0) return;
+  const int set = blockIdx.x % sets, h0 = set * p.hpc, kvh = h0 / (p.heads_q / p.heads_kv);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem; uint8_t* sV = smem + TILE_BYTES; uint8_t* sQ = smem + 2 * TILE_BYTES;
-  uint8_t* sdO = smem + 3 * TILE_BYTES; uint8_t* sP = smem + 4 * TILE_BYTES; uint8_t* sdS = smem + 5 * TILE_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * TILE_BYTES);
-  uint64_t* barKV = bars; uint64_t* barQ = bars + 1; uint64_t* barS = bars + 2; uint64_t* barD = bars + 3;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+  uint8_t *sK = smem, *sV = smem + TILE_BYTES, *sQ = smem + 2 * TILE_BYTES, *sdO = smem + 4 * TILE_BYTES, *sdS = smem + 6 * TILE_BYTES;
+  float* sStats = reinterpret_cast<float*>(smem + 7 * TILE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * TILE_BYTES + 2 * BWD_STATS * 4);
+  uint64_t *barKV = bars, *barQ = bars + 1, *barQfree = bars + 3, *bardO = bars + 5, *bardOfree = bars + 7, *barS = bars + 9,
+           *barP = bars + 10, *bardP = bars + 11, *bardS = bars + 12, *bardSfree = bars + 13, *bardQ = bars + 14, *bardQfree = bars + 15,
+           *barDone = bars + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (smem + BWD_SMEM - 768 > smem_raw + BWD_SMEM) {       // uniform; never seen: dynamic shared memory starts 1024-aligned
+    if (tid == 0 && p.status != nullptr) atomicCAS(p.status, 0, ST_CAPACITY);
+    return;
+  }
   if (tid == 0) {
-    mbar_init(barKV, 1); mbar_init(barQ, 1); mbar_init(barS, 1); mbar_init(barD, 1);
+    mbar_init(barKV, 1); mbar_init(barS, 1); mbar_init(barP, 8); mbar_init(bardP, 1); mbar_init(bardS, 8); mbar_init(bardSfree, 1);
+    mbar_init(bardQ, 1); mbar_init(bardQfree, 4); mbar_init(barDone, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&barQ[i], 1); mbar_init(&barQfree[i], 1); mbar_init(&bardO[i], 1); mbar_init(&bardOfree[i], 1); }
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 13) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);
   const int k0 = seq_start + kb * AB;
-  const int nq = (seq_end - seq_start + AB - 1) / AB;
-  const int r = tid;
-  const uint32_t id_kk = make_idesc_bf16(128, 128, 0, 0);   // A K-major, B K-major
-  const uint32_t id_mm = make_idesc_bf16(128, 128, 1, 1);   // A MN-major, B MN-major
-  const uint32_t id_km = make_idesc_bf16(128, 128, 0, 1);   // A K-major, B MN-major
-  if (tid == 0) {
-    mbar_expect_tx(barKV, 2 * TILE_BYTES);
-    load_tile(sK, &p.tmK, barKV, kvh * HD, k0);
-    load_tile(sV, &p.tmV, barKV, kvh * HD, k0);
-  }
-  bool ok = true;
-  int it = 0;
-  for (int i = kb; i < nq && ok; ++i, ++it) {
-    const int q0 = seq_start + i * AB;
-    if (tid == 0) {
-      mbar_expect_tx(barQ, 2 * TILE_BYTES);
-      load_tile(sQ, &p.tmQ, barQ, h * HD, q0);
-      load_tile(sdO, &p.tmdO, barQ, h * HD, q0);
-      bool w = (it > 0) || wait_parity(barKV, 0, abort_flag);
-      w = w && wait_parity(barQ, it & 1, abort_flag);
-      if (w) {
-        tc_fence_after();
-        const uint32_t q = smem_u32(sQ), k = smem_u32(sK), d = smem_u32(sdO), v = smem_u32(sV);
+  const int nq = (seq_end - seq_start + AB - 1) / AB - kb;  // query blocks per head
+  const int n_it = nq * p.hpc;
+  auto fail = [&](int code) {
+    *abort_flag = 1;
+    if (p.status != nullptr) atomicCAS(p.status, 0, code);
+  };
+
+  if (warp == 12) {
+    // ---------------------------------------------------------------- loads
+    bool ok = true;
+    if (elect_one()) {
+      mbar_expect_tx(barKV, 2 * TILE_BYTES);
+      load_tile(sK, &p.tmK, barKV, kvh * HD, k0);
+      load_tile(sV, &p.tmV, barKV, kvh * HD, k0);
+    }
+    int head = 0, i = 0;
+    for (int it = 0; it < n_it; ++it) {
+      const int st = it & 1;
+      const uint32_t ph = ((it >> 1) & 1) ^ 1;
+      const int h = h0 + head, q0 = seq_start + (kb + i) * AB;
+      ok = wait_parity_warp(&barQfree[st], ph, abort_flag);
+      if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+      if (elect_one()) {
+        mbar_expect_tx(&barQ[st], TILE_BYTES + BWD_STATS * 4);
+        load_tile(sQ + st * TILE_BYTES, &p.tmQ, &barQ[st], h * HD, q0);
+        bulk_load(sStats + st * BWD_STATS, p.stats + ((long long)(work.w + i) * p.heads_q + h) * BWD_STATS, BWD_STATS * 4, &barQ[st]);
+      }
+      ok = wait_parity_warp(&bardOfree[st], ph, abort_flag);
+      if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+      if (elect_one()) {
+        mbar_expect_tx(&bardO[st], TILE_BYTES);
+        load_tile(sdO + st * TILE_BYTES, &p.tmdO, &bardO[st], h * HD, q0);
+      }
+      if (++i == nq) { i = 0; ++head; }
+    }
+    if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 20000ull) {}
+    }
+  } else if (warp == 13) {
+    // ---------------------------------------------------------------- MMA issue
+    const uint32_t id_kk = make_idesc_bf16(128, 128, 0, 0), id_km = make_idesc_bf16(128, 128, 0, 1), id_mm = make_idesc_bf16(128, 128, 1, 1);
+    const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), adO = smem_u32(sdO), adS = smem_u32(sdS);
+    const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
+    auto issue_s = [&](int it) {      // S^T = K Q^T
+      if (elect_one()) {
+        const uint32_t q = aQ + (it & 1) * TILE_BYTES;
 #pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16(tmem, desc_kmajor(q, s), desc_kmajor(k, s), id_kk, s > 0);          // S = Q K^T
-#pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16(tmem + 128, desc_kmajor(d, s), desc_kmajor(v, s), id_kk, s > 0);    // dP = dO V^T
+        for (int s = 0; s < 8; ++s) umma_bf16(tS, desc_kmajor(aK, s), desc_kmajor(q, s), id_kk, s > 0);
         umma_commit(barS);
-      } else {
-        *abort_flag = 1;
-        if (p.status) atomicCAS(p.status, 0, ST_TIMEOUT_FULL);
       }
-    }
-    __syncwarp();
-    if (!wait_parity(barS, it & 1, abort_flag)) { ok = false; break; }
-    __syncwarp();
-    tc_fence_after();
-    const int qrow = q0 + r;
-    const bool qvalid = qrow < seq_end;
-    const float lse2 = qvalid ? p.lse_in[(long long)qrow * p.heads_q + h] * 1.4426950408889634f : 0.f;
-    const float dl = qvalid ? p.delta[(long long)qrow * p.heads_q + h] : 0.f;
-    const bool diag = (i == kb);
+    };
+    auto issue_dp = [&](int it) {     // dP^T = V dO^T
+      if (elect_one()) {
+        const uint32_t d = adO + (it & 1) * TILE_BYTES;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t rs[32], rp[32];
-      tmem_ld_32x32(t_row + c * 32, rs);
-      tmem_ld_32x32(t_row + 128 + c * 32, rp);
-      tmem_ld_wait();
-#pragma unroll
-      for (int x = 0; x < 32; x += 8) {
-        float pv[8], ds[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const int col = c * 32 + x + t;
-          float pr = fast_exp2(__uint_as_float(rs[x + t]) * p.scale_log2e - lse2);
-          if (!qvalid || (diag && col > r) || (k0 + col >= seq_end)) pr = 0.f;
-          pv[t] = pr;
-          ds[t] = pr * (__uint_as_float(rp[x + t]) - dl) * p.scale;
-        }
-        const uint32_t off = tile_offset(r, c * 32 + x);
-        *reinterpret_cast<uint4*>(sP + off) = make_uint4(pack2(pv[0], pv[1]), pack2(pv[2], pv[3]), pack2(pv[4], pv[5]), pack2(pv[6], pv[7]));
-        *reinterpret_cast<uint4*>(sdS + off) = make_uint4(pack2(ds[0], ds[1]), pack2(ds[2], ds[3]), pack2(ds[4], ds[5]), pack2(ds[6], ds[7]));
+        for (int s = 0; s < 8; ++s) umma_bf16(tdP, desc_kmajor(aV, s), desc_kmajor(d, s), id_kk, s > 0);
+        umma_commit(bardP);
       }
-    }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
+    };
+    bool ok = wait_parity_warp(barKV, 0, abort_flag) && wait_parity_warp(&barQ[0], 0, abort_flag);
+    if (ok) { tc_fence_after(); issue_s(0); ok = wait_parity_warp(&bardO[0], 0, abort_flag); }
+    if (ok) { tc_fence_after(); issue_dp(0); }
+    for (int it = 0; it < n_it && ok; ++it) {
+      const int st = it & 1;
+      ok = wait_parity_warp(barP, it & 1, abort_flag);
+      if (!ok) break;
       tc_fence_after();
-      const uint32_t q = smem_u32(sQ), k = smem_u32(sK), d = smem_u32(sdO), ps = smem_u32(sP), dss = smem_u32(sdS);
-      const uint32_t acc = it > 0;
+      if (elect_one()) {              // dV += P^T dO
+        const uint32_t d = adO + st * TILE_BYTES;
 #pragma unroll
-      for (int s = 0; s < 8; ++s) umma_bf16(tmem + 256, desc_mnmajor(ps, s), desc_mnmajor(d, s), id_mm, acc || s > 0);    // dV += P^T dO
+        for (int s = 0; s < 8; ++s) umma_bf16_ta(tdV, tS + (s >> 2) * 64 + (s & 3) * 8, desc_mnmajor(d, s), id_km, it > 0 || s > 0);
+        umma_commit(&bardOfree[st]);
+      }
+      if (it + 1 < n_it) {            // over P^T: the products execute in the order of issue
+        ok = wait_parity_warp(&barQ[st ^ 1], ((it + 1) >> 1) & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_s(it + 1);
+      }
+      ok = wait_parity_warp(bardS, it & 1, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t q = aQ + st * TILE_BYTES;
 #pragma unroll
-      for (int s = 0; s < 8; ++s) umma_bf16(tmem + 384, desc_mnmajor(dss, s), desc_mnmajor(q, s), id_mm, acc || s > 0);   // dK += dS^T Q
+        for (int s = 0; s < 8; ++s) umma_bf16(tdP, desc_mnmajor(adS, s), desc_mnmajor(aK, s), id_mm, s > 0);              // dQ = dS K, over dP^T
+        umma_commit(bardQ);
 #pragma unroll
-      for (int s = 0; s < 8; ++s) umma_bf16(tmem, desc_kmajor(dss, s), desc_mnmajor(k, s), id_km, s > 0);                 // dQ_i = dS K
-      umma_commit(barD);
+        for (int s = 0; s < 8; ++s) umma_bf16(tdK, desc_kmajor(adS, s), desc_mnmajor(q, s), id_km, it > 0 || s > 0);      // dK += dS^T Q
+        umma_commit(&barQfree[st]);
+        umma_commit(bardSfree);
+      }
+      if (it + 1 < n_it) {
+        ok = wait_parity_warp(&bardO[st ^ 1], ((it + 1) >> 1) & 1, abort_flag) && wait_parity_warp(bardQfree, it & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        issue_dp(it + 1);
+      }
     }
-    __syncwarp();
-    if (!wait_parity(barD, it & 1, abort_flag)) { ok = false; break; }
-    __syncwarp();
-    tc_fence_after();
-    float* dqrow = p.dq + ((long long)qrow * p.heads_q + h) * HD;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t raw[32];
-      tmem_ld_32x32(t_row + c * 32, raw);      // warp-aligned: every lane takes part, valid row or not
-      tmem_ld_wait();
-      if (qvalid) {
+    if (ok) { if (elect_one()) umma_commit(barDone); }
+    else fail(ST_TIMEOUT_FULL);
+  } else if (warp < 4) {
+    // ---------------------------------------------------------------- dQ (lane = query row)
+    const uint32_t t_row = tmem + 128 + ((uint32_t)(warp * 32) << 16);
+    int head = 0, i = 0;
+    for (int it = 0; it < n_it; ++it) {
+      if (!wait_parity_warp(bardQ, it & 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
+      tc_fence_after();
+      float* dst = p.dq + ((long long)(work.w + i) * p.heads_q + h0 + head) * DQ_TILE + (warp * 32 + lane) * 4;
+#pragma unroll 1
+      for (int c = 0; c < HD; c += 64) {
+        uint32_t a[32], b[32];
+        tmem_ld_32x32(t_row + c, a);
+        tmem_ld_32x32(t_row + c + 32, b);
+        tmem_ld_wait();
+        if (c == 64) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bardQfree);
+        }
 #pragma unroll
         for (int x = 0; x < 32; x += 4)
-          red_add_v4_f32(dqrow + c * 32 + x, __uint_as_float(raw[x]), __uint_as_float(raw[x + 1]), __uint_as_float(raw[x + 2]),
-                         __uint_as_float(raw[x + 3]));
+          red_add_v4_f32(dst + ((c + x) >> 2) * (AB * 4), __uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
+#pragma unroll
+        for (int x = 0; x < 32; x += 4)
+          red_add_v4_f32(dst + ((c + 32 + x) >> 2) * (AB * 4), __uint_as_float(b[x]), __uint_as_float(b[x + 1]), __uint_as_float(b[x + 2]), __uint_as_float(b[x + 3]));
       }
-      __syncwarp();
+      if (++i == nq) { i = 0; ++head; }
     }
-    tc_fence_before();
-    __syncthreads();
-  }
-  if (!ok && tid == 0 && p.status) atomicCAS(p.status, 0, ST_TIMEOUT_TMEM_FULL);
-  const int krow = k0 + r;
-  const bool kvalid = krow < seq_end;
-  ok = __all_sync(0xffffffffu, ok);
-  if (ok) {   // warp-uniform: `ok` only changes together with the shared abort flag
-    float* dv = p.dv + ((long long)krow * p.heads_q + h) * HD;
-    float* dk = p.dk + ((long long)krow * p.heads_q + h) * HD;
+  } else if (warp < 12) {
+    // ---------------------------------------------------------------- softmax (lane = key row, 64 query columns)
+    const int half = (warp - 4) >> 2, r = (warp & 3) * 32 + lane;
+    const uint32_t t_row = tmem + half * 64 + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool k_partial = k0 + AB > seq_end, k_valid = k0 + r < seq_end;
+    bool ok = true;
+    int i = 0;
+    for (int it = 0; it < n_it; ++it) {
+      const int st = it & 1;
+      const int q0 = seq_start + (kb + i) * AB;
+      const float* lse2 = sStats + st * BWD_STATS + half * 64;
+      const float* delta = lse2 + AB;
+      // block on the diagonal, last query block or last key block: elements are masked one by one
+      const bool masked = i == 0 || q0 + AB > seq_end || k_partial;
+      auto hidden = [&](int c) {       // query column half * 64 + c
+        const int q = half * 64 + c;
+        return !k_valid || (i == 0 && q < r) || q0 + q >= seq_end;
+      };
+      if (!wait_parity_warp(&barQ[st], (it >> 1) & 1, abort_flag) || !wait_parity_warp(barS, it & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      float pr[64];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      uint32_t a[32], b[32];
-      tmem_ld_32x32(t_row + 256 + c * 32, a);
-      tmem_ld_32x32(t_row + 384 + c * 32, b);
-      tmem_ld_wait();
-      if (kvalid) {
+      for (int c = 0; c < 64; c += 16) {
+        uint32_t s[16];
+        tmem_ld_32x16(t_row + c, s);
+        tmem_ld_wait();
 #pragma unroll
-        for (int x = 0; x < 32; x += 4) {
-          *reinterpret_cast<float4*>(dv + c * 32 + x) = make_float4(__uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
-          *reinterpret_cast<float4*>(dk + c * 32 + x) = make_float4(__uint_as_float(b[x]), __uint_as_float(b[x + 1]), __uint_as_float(b[x + 2]), __uint_as_float(b[x + 3]));
+        for (int x = 0; x < 16; x += 4) {
+          const float4 l = *reinterpret_cast<const float4*>(lse2 + c + x);
+          pr[c + x] = fast_exp2(__uint_as_float(s[x]) * p.scale_log2e - l.x);
+          pr[c + x + 1] = fast_exp2(__uint_as_float(s[x + 1]) * p.scale_log2e - l.y);
+          pr[c + x + 2] = fast_exp2(__uint_as_float(s[x + 2]) * p.scale_log2e - l.z);
+          pr[c + x + 3] = fast_exp2(__uint_as_float(s[x + 3]) * p.scale_log2e - l.w);
+        }
+        if (masked) {
+#pragma unroll
+          for (int x = 0; x < 16; ++x) if (hidden(c + x)) pr[c + x] = 0.f;
         }
       }
+      {
+        uint32_t pk[32];
+#pragma unroll
+        for (int c = 0; c < 32; ++c) pk[c] = pack2(pr[2 * c], pr[2 * c + 1]);
+        tmem_st_32x32(t_row, pk);      // over this warp's own part of S^T
+        tmem_st_wait();
+      }
+      tc_fence_before();
       __syncwarp();
+      if (lane == 0) mbar_arrive(barP);
+      if (!wait_parity_warp(bardP, it & 1, abort_flag)) { ok = false; break; }
+      if (it > 0 && !wait_parity_warp(bardSfree, (it - 1) & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < 64; c += 16) {
+        uint32_t d[16];
+        tmem_ld_32x16(t_row + 128 + c, d);
+        tmem_ld_wait();
+        float ds[16];
+#pragma unroll
+        for (int x = 0; x < 16; x += 4) {
+          const float4 dl = *reinterpret_cast<const float4*>(delta + c + x);
+          ds[x] = pr[c + x] * (__uint_as_float(d[x]) - dl.x) * p.scale;
+          ds[x + 1] = pr[c + x + 1] * (__uint_as_float(d[x + 1]) - dl.y) * p.scale;
+          ds[x + 2] = pr[c + x + 2] * (__uint_as_float(d[x + 2]) - dl.z) * p.scale;
+          ds[x + 3] = pr[c + x + 3] * (__uint_as_float(d[x + 3]) - dl.w) * p.scale;
+        }
+        if (masked) {
+#pragma unroll
+          for (int x = 0; x < 16; ++x) if (hidden(c + x)) ds[x] = 0.f;
+        }
+#pragma unroll
+        for (int x = 0; x < 16; x += 8)
+          *reinterpret_cast<uint4*>(sdS + tile_offset(r, half * 64 + c + x)) =
+              make_uint4(pack2(ds[x], ds[x + 1]), pack2(ds[x + 2], ds[x + 3]), pack2(ds[x + 4], ds[x + 5]), pack2(ds[x + 6], ds[x + 7]));
+      }
+      fence_proxy_async();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bardS);
+      if (++i == nq) i = 0;
+    }
+    ok = ok && wait_parity_warp(barDone, 0, abort_flag);
+    if (!ok) { if (lane == 0) fail(ST_TIMEOUT_TMEM_FULL); }
+    else {
+      // warps 4-7 write dV, warps 8-11 dK
+      tc_fence_after();
+      const uint32_t acc = tmem + 256 + half * 128 + ((uint32_t)((warp & 3) * 32) << 16);
+      const long long krow = k0 + r;
+      float* part = p.dk != nullptr ? (half == 0 ? p.dv : p.dk) + (krow * sets + set) * HD : nullptr;
+      bf16* out = (half == 0 ? p.dv_out : p.dk_out) + (krow * p.heads_kv + kvh) * HD;
+#pragma unroll 1
+      for (int c = 0; c < HD; c += 32) {
+        uint32_t a[32];
+        tmem_ld_32x32(acc + c, a);
+        tmem_ld_wait();
+        if (k_valid) {
+          if (part != nullptr) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 4)
+              *reinterpret_cast<float4*>(part + c + x) = make_float4(__uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
+          } else {
+#pragma unroll
+            for (int x = 0; x < 32; x += 8)
+              *reinterpret_cast<uint4*>(out + c + x) =
+                  make_uint4(pack2(__uint_as_float(a[x]), __uint_as_float(a[x + 1])), pack2(__uint_as_float(a[x + 2]), __uint_as_float(a[x + 3])),
+                             pack2(__uint_as_float(a[x + 4]), __uint_as_float(a[x + 5])), pack2(__uint_as_float(a[x + 6]), __uint_as_float(a[x + 7])));
+          }
+        }
+        __syncwarp();
+      }
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 512); }
+  if (warp == 13) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-// dq bf16 = dq fp32; dk/dv bf16 [T, heads_kv, 128] = sum over the query heads of each group
-__global__ void attn_bwd_finalize_kernel(const float* __restrict__ dq32, const float* __restrict__ dk32, const float* __restrict__ dv32,
-                                         bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv, long long tokens,
-                                         int heads_q, int heads_kv) {
-  const int group = heads_q / heads_kv;
-  const long long nq = tokens * heads_q * HD, nk = tokens * heads_kv * HD;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nq + 2 * nk; i += (long long)gridDim.x * blockDim.x) {
-    if (i < nq) { dq[i] = __float2bfloat16(dq32[i]); continue; }
-    const bool isv = i >= nq + nk;
-    const long long e = i - nq - (isv ? nk : 0);
-    const int d = (int)(e % HD);
-    const long long th = e / HD;
-    const int kvh = (int)(th % heads_kv);
-    const long long t = th / heads_kv;
-    const float* src = (isv ? dv32 : dk32) + ((t * heads_q + (long long)kvh * group) * HD) + d;
-    float s = 0.f;
-    for (int g = 0; g < group; ++g) s += src[(long long)g * HD];
-    (isv ? dv : dk)[e] = __float2bfloat16(s);
+// dQ: tiles [column / 4][row][4] -> bf16 rows, one CTA per (block, head).  dK, dV (`sets` partial sums per kv head, when
+// there are several): the CTAs past the blocks, summed and converted eight columns at a time.
+__global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __restrict__ dq32, const float* __restrict__ dk32, const float* __restrict__ dv32,
+                                                                bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
+                                                                const int* __restrict__ cu, int num_seqs, int blocks, int tokens, int heads_q,
+                                                                int heads_kv, int sets) {
+  if ((int)blockIdx.x < blocks) {
+    int seq_start, seq_end, blk;
+    if (!find_block(cu, num_seqs, blockIdx.x, seq_start, seq_end, blk)) return;
+    const int h = blockIdx.y;
+    const float4* src = reinterpret_cast<const float4*>(dq32 + ((long long)blockIdx.x * heads_q + h) * DQ_TILE);
+    // eight lanes x 4 columns = 64 bytes of a row of dq, four rows per warp and pass; all loads in flight at once
+    const int cg = threadIdx.x & 7, rsub = threadIdx.x >> 3;
+    float4 v[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = __ldcs(src + ((k & 3) * 8 + cg) * AB + (k >> 2) * 32 + rsub);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const long long row = seq_start + blk * AB + (k >> 2) * 32 + rsub;
+      if (row < seq_end)
+        *reinterpret_cast<uint2*>(dq + (row * heads_q + h) * HD + ((k & 3) * 8 + cg) * 4) = make_uint2(pack2(v[k].x, v[k].y), pack2(v[k].z, v[k].w));
+    }
+    return;
+  }
+  const int per = sets / heads_kv;                                       // partial sums per kv head
+  const long long n = (long long)tokens * heads_kv * (HD / 8);           // 8-column vectors of dK (then of dV)
+  const long long stride = (long long)(gridDim.x - blocks) * gridDim.y * 256;
+  for (long long e = (((long long)blockIdx.x - blocks) * gridDim.y + blockIdx.y) * 256 + threadIdx.x; e < 2 * n; e += stride) {
+    const bool isv = e >= n;
+    const long long v = isv ? e - n : e;
+    const int d = (int)(v % (HD / 8)) * 8;
+    const long long th = v / (HD / 8);                                   // token * heads_kv + kv head
+    const float* src = (isv ? dv32 : dk32) + (th * per) * HD + d;
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int g = 0; g < per; ++g) {
+      const float4 a = *reinterpret_cast<const float4*>(src + (long long)g * HD), b = *reinterpret_cast<const float4*>(src + (long long)g * HD + 4);
+      s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w; s[4] += b.x; s[5] += b.y; s[6] += b.z; s[7] += b.w;
+    }
+    *reinterpret_cast<uint4*>((isv ? dv : dk) + th * HD + d) = make_uint4(pack2(s[0], s[1]), pack2(s[2], s[3]), pack2(s[4], s[5]), pack2(s[6], s[7]));
   }
 }
 
@@ -686,13 +905,12 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
   if (!serial) rc |= att_map(&p.tmK64, k, total_tokens, heads_kv, FB) | att_map(&p.tmV64, v, total_tokens, heads_kv, FB);
   if (rc) return rc;
   p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.heads_q = heads_q; p.heads_kv = heads_kv;
-  p.scale = scale; p.scale_log2e = scale * 1.4426950408889634f;
+  p.scale_log2e = scale * 1.4426950408889634f;
   p.o = (bf16*)o; p.lse = lse;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess) return -4;
     if (cudaFuncSetAttribute(attn_fwd_pipelined_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD2_SMEM) != cudaSuccess) return -4;
-    if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess) return -4;
     configured = true;
   }
   dim3 grid((total_tokens + AB - 1) / AB + num_seqs, heads_q);
@@ -703,44 +921,71 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
   return e == cudaSuccess ? 0 : -100 - (int)e;
 }
 
+namespace {
+// How the backward pass is cut: 128-row blocks (upper bound: the sequences are ragged) and query heads per CTA.
+struct BwdPlan { long long blocks; int hpc, sets; long long off_stats, off_dq, off_dk, off_dv, floats; };
+BwdPlan bwd_plan(int num_seqs, int total_tokens, int max_seqlen, int heads_q, int heads_kv) {
+  BwdPlan b;
+  b.blocks = ((long long)total_tokens + AB - 1) / AB + num_seqs;
+  // A CTA that takes all query heads of a kv head adds their dK, dV in TMEM and writes bf16; but its loop is that much
+  // longer.  The longest loop may be half of an SM's share of all iterations (sequences taken as equally long), else
+  // fewer heads per CTA: 613 tokens, 32 / 8 heads run with one head (160 CTAs), four sequences of 1024-8192 with all four.
+  const int group = heads_q / heads_kv;
+  const double seqs = num_seqs > 0 ? num_seqs : 1, n = (double)total_tokens / (AB * seqs);
+  const double share = seqs * n * (n + 1.0) / 2.0 * heads_q / sm_count_of_current_device();
+  const int longest = ((max_seqlen < total_tokens ? max_seqlen : total_tokens) + AB - 1) / AB;
+  b.hpc = group;
+  while (b.hpc > 1 && (double)b.hpc * longest > 0.5 * share) b.hpc = b.hpc % 2 == 0 ? b.hpc / 2 : 1;
+  b.sets = heads_q / b.hpc;
+  b.off_stats = (b.blocks * 4 + 31) / 32 * 32;                                   // after the schedule
+  b.off_dq = b.off_stats + b.blocks * heads_q * BWD_STATS;
+  b.off_dk = b.off_dq + b.blocks * heads_q * DQ_TILE;
+  const long long part = b.hpc == group ? 0 : (long long)total_tokens * b.sets * HD;
+  b.off_dv = b.off_dk + part;
+  b.floats = b.off_dv + part;
+  return b;
+}
+}  // namespace
+
+extern "C" long long mdt_attention_bwd_scratch(int num_seqs, int total_tokens, int max_seqlen, int heads_q, int heads_kv) {
+  return bwd_plan(num_seqs, total_tokens, max_seqlen, heads_q, heads_kv).floats;
+}
+
 extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                                  void* dq, void* dk, void* dv, float* scratch, const int* cu_seqlens, int num_seqs, int total_tokens,
                                  int max_seqlen, int heads_q, int heads_kv, int head_dim, float scale, cudaStream_t s) {
-  // scratch: fp32, (1 + 3*128) * total_tokens * heads_q elements: delta | dq32 | dk32 | dv32
+  // scratch: mdt_attention_bwd_scratch() floats, 128-byte aligned: schedule | row statistics | dq32 | dk32 | dv32
   if (head_dim != HD || heads_q % heads_kv != 0) return -1;
   if (total_tokens == 0) return 0;
+  if (reinterpret_cast<uintptr_t>(scratch) & 127) return -2;
   static thread_local bool bound = false;
   if (!bound) { cudaFree(nullptr); bound = true; }
-  const long long th = (long long)total_tokens * heads_q;
-  float* delta = scratch;
-  float* dq32 = scratch + th;
-  float* dk32 = dq32 + th * HD;
-  float* dv32 = dk32 + th * HD;
-  AttnParams p;
+  const BwdPlan b = bwd_plan(num_seqs, total_tokens, max_seqlen, heads_q, heads_kv);
+  const bool direct = b.off_dk == b.floats;
+  AttnBwdParams p;
   memset(&p, 0, sizeof(p));
   int rc = att_map(&p.tmQ, q, total_tokens, heads_q) | att_map(&p.tmK, k, total_tokens, heads_kv) |
            att_map(&p.tmV, v, total_tokens, heads_kv) | att_map(&p.tmdO, dout, total_tokens, heads_q);
   if (rc) return rc;
-  p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.heads_q = heads_q; p.heads_kv = heads_kv;
+  p.sched = reinterpret_cast<const int4*>(scratch); p.stats = scratch + b.off_stats; p.dq = scratch + b.off_dq;
+  p.dk = direct ? nullptr : scratch + b.off_dk; p.dv = direct ? nullptr : scratch + b.off_dv;
+  p.dk_out = (bf16*)dk; p.dv_out = (bf16*)dv;
+  p.heads_q = heads_q; p.heads_kv = heads_kv; p.hpc = b.hpc;
   p.scale = scale; p.scale_log2e = scale * 1.4426950408889634f;
-  p.delta = delta; p.lse_in = lse; p.dq = dq32; p.dk = dk32; p.dv = dv32;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess) return -4;
-    if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_SMEM) != cudaSuccess) return -4;
+    if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return -4;
     configured = true;
   }
-  cudaMemsetAsync(dq32, 0, sizeof(float) * th * HD, s);
-  attn_delta_kernel<<<(unsigned)((th + 3) / 4), 128, 0, s>>>((const bf16*)o, (const bf16*)dout, delta, th);
+  attn_bwd_prepare_kernel<<<dim3((unsigned)b.blocks, heads_q), 256, 0, s>>>((const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs, heads_q,
+                                                                            reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq);
   ++g_att_launches;
-  dim3 grid((total_tokens + AB - 1) / AB + num_seqs, heads_q);
-  attn_bwd_kernel<<<grid, 128, ATT_SMEM, s>>>(p);
+  attn_bwd_kernel<<<(unsigned)(b.blocks * b.sets), BWD_THREADS, BWD_SMEM, s>>>(p);
   ++g_att_launches;
-  const long long total = th * HD + 2LL * total_tokens * heads_kv * HD;
-  long long blocks = (total + 255) / 256;
-  const long long cap = (long long)sm_count_of_current_device() * 16;
-  if (blocks > cap) blocks = cap;
-  attn_bwd_finalize_kernel<<<(unsigned)blocks, 256, 0, s>>>(dq32, dk32, dv32, (bf16*)dq, (bf16*)dk, (bf16*)dv, total_tokens, heads_q, heads_kv);
+  long long extra = 0;                                       // CTAs (times heads_q) that add up partial dK, dV
+  if (!direct) extra = (2LL * total_tokens * heads_kv * (HD / 8) + 256LL * heads_q - 1) / (256LL * heads_q);
+  attn_bwd_finalize_kernel<<<dim3((unsigned)(b.blocks + extra), heads_q), 256, 0, s>>>(p.dq, p.dk, p.dv, (bf16*)dq, (bf16*)dk, (bf16*)dv, cu_seqlens,
+                                                                                      num_seqs, (int)b.blocks, total_tokens, heads_q, heads_kv, b.sets);
   ++g_att_launches;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - (int)e;

@@ -375,7 +375,8 @@ std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor
   TORCH_CHECK(dout.is_contiguous() && o.is_contiguous());
   const int T = (int)q.size(0), Hq = (int)q.size(1), Hkv = (int)k.size(1), D = (int)q.size(2);
   auto dq = torch::empty_like(q), dk = torch::empty_like(k), dv = torch::empty_like(v);
-  auto scratch = torch::empty({(int64_t)T * Hq * (1 + 3 * D)}, q.options().dtype(at::kFloat));
+  const int nseq = (int)cu_seqlens.numel() - 1;
+  auto scratch = torch::empty({mdt_attention_bwd_scratch(nseq, T, (int)max_seqlen, Hq, Hkv)}, q.options().dtype(at::kFloat));
   check(mdt_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(), dq.data_ptr(),
                           dk.data_ptr(), dv.data_ptr(), scratch.data_ptr<float>(), cu_seqlens.data_ptr<int>(), (int)cu_seqlens.numel() - 1, T,
                           (int)max_seqlen, Hq, Hkv, D, (float)scale, cur_stream()), "attention_bwd");

@@ -473,6 +473,37 @@ def test_attention(ops, lens):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("lens,heads,kv", [([1], 2, 2), ([127, 1, 129], 4, 2), ([255, 257, 128], 6, 2), ([640, 33, 1100, 5], 8, 2),
+                                           ([130] * 40, 4, 4), ([2500, 1300], 32, 8), ([3000], 4, 1)])
+def test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv):
+    """Edges of the 128-row blocks, sequences of one row, more sequences than a warp has lanes, and both ways of adding a
+    kv head's query heads up (in one CTA, over partial sums), against fp64 attention.  bf16 inputs, probabilities and dS
+    rounded to bf16 before the second products: 1e-2 on whole tensors is about three times what is seen."""
+    T, d = sum(lens), 128
+    g = torch.Generator(device=DEV).manual_seed(T + heads)
+    q, k, v, do = (torch.randn(T, h, d, device=DEV, generator=g).to(torch.bfloat16) for h in (heads, kv, kv, heads))
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    from moe_distributed_training_b200.ops.attention_cuda import attention
+    o = attention(q, k, v, cu, max(lens))
+    grads = torch.autograd.grad(o, (q, k, v), do)
+    q2, k2, v2 = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    outs = []
+    for s, n in zip(cu.tolist(), lens):
+        qs, ks, vs = (t[s:s + n].transpose(0, 1) for t in (q2, k2.repeat_interleave(heads // kv, 1), v2.repeat_interleave(heads // kv, 1)))
+        sc = (qs @ ks.transpose(1, 2)) * d ** -0.5
+        sc = sc.masked_fill(torch.ones(n, n, device=DEV, dtype=torch.bool).triu(1), float("-inf"))
+        outs.append((sc.softmax(-1) @ vs).transpose(0, 1))
+    ref = torch.cat(outs)
+    for name, a, b in zip(("o", "dq", "dk", "dv"), (o,) + grads, (ref,) + torch.autograd.grad(ref, (q2, k2, v2), do.double())):
+        if float(b.norm()) == 0.0:            # one key: the softmax is constant
+            assert float(a.float().abs().max()) < 1e-2, name
+        else:
+            assert _rel_err(a, b) < 1e-2, (name, _rel_err(a, b))
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("lora", [False, True])
 def test_fused_attention_block_matches_composed_ops(ops, lora):
     """The single-node attention sub-block against the same layer evaluated op by op."""
