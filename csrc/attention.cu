@@ -225,20 +225,22 @@ __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant_
 // ------------------------------------------------------------------------------------------- forward, pipelined
 // Warp-specialised forward: warps 0-3 do the softmax (one query row per thread), warp 4 loads (TMA) and issues the
 // MMAs.  Keys / values come in blocks of 64 rows; S = Q K^T lives in two 64-column TMEM buffers, so the tensor core
-// computes S of block j+1 while the softmax warps work on block j; O is accumulated in TMEM by the P V products
-// themselves.  The running row maximum used for the exponentials is only raised when the true maximum has grown
+// computes S of block j+1 while the softmax warps work on block j.  The probabilities go back into the first half of
+// their S buffer as bf16 and are the A operand of P V from there: through shared memory they cost 16 KB written and 16
+// read per block, where the products already take 64 KB per 512 clocks of MMA.  O is accumulated in TMEM by the P V
+// products themselves.  The running row maximum used for the exponentials is only raised when the true maximum has grown
 // by more than 2^8 (the sum and O are rescaled then, rarely after the first blocks; the final division by the row
-// sum makes the result independent of the reference point).  96 KB of shared memory and 256 TMEM columns per CTA:
-// two CTAs share an SM, so that one's softmax also overlaps the other's products.
-//   TMEM columns: [0,64) S buffer 0, [64,128) S buffer 1, [128,256) O
-//   barriers: Q, K (one K tile, reloaded as soon as S of the previous block is done), V[2], S[2] (S ready),
-//             Sfree[2] (softmax has read S), P (probabilities stored), O (P V done: O updated, P and V tile free)
+// sum makes the result independent of the reference point); only then does the softmax wait for a P V product.  96 KB of
+// shared memory and 256 TMEM columns per CTA: two CTAs share an SM, so that one's softmax also overlaps the other's
+// products.  The query blocks with the most keys come first in the grid.
+//   TMEM columns: [0,64) S / P buffer 0, [64,128) S / P buffer 1, [128,256) O
+//   barriers: Q, K[2], V[2] (loaded), S[2] (S ready), P[2] (probabilities stored: S read too), O[2] (P V done: O updated,
+//             V tile and P buffer free)
 constexpr int FB = 64;                        // key rows per block
 constexpr int KV_TILE = FB * HD * 2;          // 16 KB: two atoms of [64 rows x 128 B]
 constexpr int KV_ATOM = FB * 128;             // 8 KB
-constexpr int P_TILE = AB * FB * 2;           // 16 KB: one atom of [128 rows x 128 B]
 constexpr int FWD2_THREADS = 160;
-constexpr int FWD2_SMEM = TILE_BYTES + KV_TILE + 2 * KV_TILE + P_TILE + 1024 + 128;
+constexpr int FWD2_SMEM = TILE_BYTES + 4 * KV_TILE + 1024 + 128;
 static_assert(2 * (FWD2_SMEM + 1024) <= 228 * 1024, "two CTAs of the pipelined forward must fit one SM");
 constexpr float RESCALE_THRESHOLD = 8.0f;     // log2 units
 
@@ -249,24 +251,22 @@ __device__ __forceinline__ void load_kv_tile(uint8_t* dst, const CUtensorMap* ma
 
 __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(const __grid_constant__ AttnParams p) {
   int seq_start, seq_end, qb;
-  if (!find_block(p.cu_seqlens, p.num_seqs, blockIdx.x, seq_start, seq_end, qb)) return;
-  const int h = blockIdx.y, kvh = h / (p.heads_q / p.heads_kv);
+  if (!find_block(p.cu_seqlens, p.num_seqs, blockIdx.x / p.heads_q, seq_start, seq_end, qb)) return;
+  qb = (seq_end - seq_start + AB - 1) / AB - 1 - qb;          // last (longest) block of a sequence first
+  const int h = blockIdx.x % p.heads_q, kvh = h / (p.heads_q / p.heads_kv);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sK = smem + TILE_BYTES;
-  uint8_t* sV = sK + KV_TILE;                 // two stages
-  uint8_t* sP = sV + 2 * KV_TILE;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + P_TILE);
-  uint64_t* barQ = bars; uint64_t* barK = bars + 1; uint64_t* barV = bars + 2; uint64_t* barS = bars + 4;
-  uint64_t* barSfree = bars + 6; uint64_t* barP = bars + 8; uint64_t* barO = bars + 9;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  uint8_t* sK = smem + TILE_BYTES;            // two stages
+  uint8_t* sV = sK + 2 * KV_TILE;             // two stages
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * KV_TILE);
+  uint64_t *barQ = bars, *barK = bars + 1, *barV = bars + 3, *barS = bars + 5, *barP = bars + 7, *barO = bars + 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    mbar_init(barQ, 1); mbar_init(barK, 1); mbar_init(&barV[0], 1); mbar_init(&barV[1], 1);
-    mbar_init(&barS[0], 1); mbar_init(&barS[1], 1); mbar_init(&barSfree[0], 4); mbar_init(&barSfree[1], 4);
-    mbar_init(barP, 4); mbar_init(barO, 1);
+    mbar_init(barQ, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&barK[i], 1); mbar_init(&barV[i], 1); mbar_init(&barS[i], 1); mbar_init(&barP[i], 4); mbar_init(&barO[i], 1); }
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -287,131 +287,141 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
   };
 
   if (warp == 4) {
-    if (lane == 0) {
-      // ---------------------------------------------------------------- loads and MMA issue
-      const uint32_t idesc_s = make_idesc_bf16(128, FB, 0, 0);       // Q (K-major) x K^T (K-major)
-      const uint32_t idesc_pv = make_idesc_bf16(128, HD, 0, 1);      // P (K-major) x V (MN-major)
-      const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aP = smem_u32(sP);
+    // ------------------------------------------------------------------ loads and MMA issue
+    const uint32_t idesc_s = make_idesc_bf16(128, FB, 0, 0);       // Q (K-major) x K^T (K-major)
+    const uint32_t idesc_pv = make_idesc_bf16(128, HD, 0, 1);      // P (TMEM) x V (MN-major)
+    const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK), aV = smem_u32(sV);
+    auto load_k = [&](int j) { mbar_expect_tx(&barK[j & 1], KV_TILE); load_kv_tile(sK + (j & 1) * KV_TILE, &p.tmK64, &barK[j & 1], kvh * HD, seq_start + j * FB); };
+    auto load_v = [&](int j) { mbar_expect_tx(&barV[j & 1], KV_TILE); load_kv_tile(sV + (j & 1) * KV_TILE, &p.tmV64, &barV[j & 1], kvh * HD, seq_start + j * FB); };
+    if (elect_one()) {
       mbar_expect_tx(barQ, TILE_BYTES);
       load_tile(sQ, &p.tmQ, barQ, h * HD, q0);
-      mbar_expect_tx(barK, KV_TILE);
-      load_kv_tile(sK, &p.tmK64, barK, kvh * HD, seq_start);
-      mbar_expect_tx(&barV[0], KV_TILE);
-      load_kv_tile(sV, &p.tmV64, &barV[0], kvh * HD, seq_start);
-      bool ok = wait_parity(barQ, 0, abort_flag) && wait_parity(barK, 0, abort_flag);
-      if (!ok) fail(ST_TIMEOUT_FULL);
-      auto issue_s = [&](int j) {     // S_j = Q K_j^T into S buffer j & 1
-        tc_fence_after();
+      load_k(0);
+      load_v(0);
+      if (n_kv > 1) { load_k(1); load_v(1); }
+    }
+    bool ok = wait_parity_warp(barQ, 0, abort_flag) && wait_parity_warp(&barK[0], 0, abort_flag);
+    if (!ok) fail(ST_TIMEOUT_FULL);
+    auto issue_s = [&](int j) {     // S_j = Q K_j^T into buffer j & 1 (P_{j-2} V was issued before: products execute in order)
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t k0 = aK + (j & 1) * KV_TILE;
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          umma_bf16(tmem + (j & 1) * FB, desc_kmajor(aQ, k), make_smem_desc(aK + (k >> 2) * KV_ATOM + (k & 3) * 32, 16, 1024), idesc_s, k > 0);
+          umma_bf16(tmem + (j & 1) * FB, desc_kmajor(aQ, k), make_smem_desc(k0 + (k >> 2) * KV_ATOM + (k & 3) * 32, 16, 1024), idesc_s, k > 0);
         umma_commit(&barS[j & 1]);
-      };
-      if (ok) issue_s(0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        if (j + 1 < n_kv) {
-          // K tile free once S_j is done; S buffer (j+1)&1 free once the softmax of block j-1 has read it
-          ok = wait_parity(&barS[j & 1], (j >> 1) & 1, abort_flag);
-          if (!ok) { fail(ST_TIMEOUT_TMEM_FULL); break; }
-          mbar_expect_tx(barK, KV_TILE);
-          load_kv_tile(sK, &p.tmK64, barK, kvh * HD, seq_start + (j + 1) * FB);
-          ok = wait_parity(barK, (j + 1) & 1, abort_flag);
-          if (ok && j >= 1) ok = wait_parity(&barSfree[(j + 1) & 1], ((j - 1) >> 1) & 1, abort_flag);
-          if (!ok) { fail(ST_TIMEOUT_FULL); break; }
-          issue_s(j + 1);
-        }
-        // P_j stored (which also means P V of block j-1 is complete: the softmax warps waited for it)
-        ok = wait_parity(barP, j & 1, abort_flag);
-        if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
-        if (j + 1 < n_kv) {
-          mbar_expect_tx(&barV[(j + 1) & 1], KV_TILE);
-          load_kv_tile(sV + ((j + 1) & 1) * KV_TILE, &p.tmV64, &barV[(j + 1) & 1], kvh * HD, seq_start + (j + 1) * FB);
-        }
-        ok = wait_parity(&barV[j & 1], (j >> 1) & 1, abort_flag);
+      }
+    };
+    if (ok) issue_s(0);
+    for (int j = 0; j < n_kv && ok; ++j) {
+      if (j + 1 < n_kv) {
+        ok = wait_parity_warp(&barK[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag);
         if (!ok) { fail(ST_TIMEOUT_FULL); break; }
-        tc_fence_after();
-        const uint32_t aV = smem_u32(sV + (j & 1) * KV_TILE);
+        issue_s(j + 1);
+      }
+      if (j + 2 < n_kv) {           // K tile j free: S_j done
+        ok = wait_parity_warp(&barS[j & 1], (j >> 1) & 1, abort_flag);
+        if (!ok) { fail(ST_TIMEOUT_TMEM_FULL); break; }
+        if (elect_one()) load_k(j + 2);
+      }
+      ok = wait_parity_warp(&barP[j & 1], (j >> 1) & 1, abort_flag);
+      if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+      ok = wait_parity_warp(&barV[j & 1], (j >> 1) & 1, abort_flag);
+      if (!ok) { fail(ST_TIMEOUT_FULL); break; }
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t v0 = aV + (j & 1) * KV_TILE;
 #pragma unroll
         for (int k = 0; k < FB / 16; ++k)
-          umma_bf16(tmem + 128, make_smem_desc(aP + k * 32, 16, 1024), make_smem_desc(aV + k * 2048, KV_ATOM, 1024), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
-        umma_commit(barO);
+          umma_bf16_ta(tmem + 128, tmem + (j & 1) * FB + k * 8, make_smem_desc(v0 + k * 2048, KV_ATOM, 1024), idesc_pv, (j > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&barO[j & 1]);
       }
-      if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 20000ull) {}
+      if (j >= 1 && j + 1 < n_kv) { // V tile j-1 free: its product done (this one is under way)
+        ok = wait_parity_warp(&barO[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag);
+        if (!ok) { fail(ST_TIMEOUT_TMEM_FULL); break; }
+        if (elect_one()) load_v(j + 1);
       }
+    }
+    if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 20000ull) {}
     }
   } else {
     // ------------------------------------------------------------------ softmax warps: thread = query row
     const int r = tid;
     const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);
-    float m_ref = -INFINITY, l = 0.f;
+    float m_ref = -INFINITY, l = 0.f;         // reference point (log2 units) and row sum
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
-      if (!wait_parity(&barS[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
-      __syncwarp();
+      if (!wait_parity_warp(&barS[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
+      // the product two blocks back is long done (S_j came after it); waiting for it keeps barO's phases in step
+      if (j >= 2 && !wait_parity_warp(&barO[j & 1], ((j - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t s0[32], s1[32];
       tmem_ld_32x32(t_row + (j & 1) * FB, s0);
       tmem_ld_32x32(t_row + (j & 1) * FB + 32, s1);
       tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&barSfree[j & 1]);
       // causal mask: key column 64j + c is visible to query row 128qb + r iff it is not to the right of it
       const int visible = qb * AB + r - j * FB;         // columns c <= visible are kept
-      float mx = -INFINITY;
+      if (qb * AB - j * FB < FB - 1) {                  // some row of the block sees less than all columns
 #pragma unroll
-      for (int c = 0; c < 32; ++c) {
-        const float a = __uint_as_float(s0[c]) * p.scale_log2e, b = __uint_as_float(s1[c]) * p.scale_log2e;
-        s0[c] = __float_as_uint(c <= visible ? a : -INFINITY);
-        s1[c] = __float_as_uint(c + 32 <= visible ? b : -INFINITY);
-        mx = fmaxf(mx, fmaxf(__uint_as_float(s0[c]), __uint_as_float(s1[c])));
+        for (int c = 0; c < 32; ++c) {
+          if (c > visible) s0[c] = __float_as_uint(-INFINITY);
+          if (c + 32 > visible) s1[c] = __float_as_uint(-INFINITY);
+        }
       }
+      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 32; c += 2) {
+        mx0 = fmaxf(mx0, __uint_as_float(s0[c])); mx1 = fmaxf(mx1, __uint_as_float(s0[c + 1]));
+        mx2 = fmaxf(mx2, __uint_as_float(s1[c])); mx3 = fmaxf(mx3, __uint_as_float(s1[c + 1]));
+      }
+      const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2e;
       // raise the reference point only when the maximum has outgrown it by more than the threshold
-      float alpha = 1.f;
       const bool raise = mx > m_ref + RESCALE_THRESHOLD;    // (also true for the first visible block: m_ref = -inf)
-      if (raise) { alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mx); m_ref = mx; l *= alpha; }
-      if (j > 0) {
-        if (!wait_parity(barO, (j - 1) & 1, abort_flag)) { ok = false; break; }   // O of the blocks so far is complete, P free
-        __syncwarp();
-        if (__any_sync(0xffffffffu, raise)) {
+      if (__any_sync(0xffffffffu, raise)) {
+        float alpha = 1.f;
+        if (raise) { alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2(m_ref - mx); m_ref = mx; l *= alpha; }
+        if (j > 0) {
+          if (!wait_parity_warp(&barO[(j - 1) & 1], ((j - 1) >> 1) & 1, abort_flag)) { ok = false; break; }   // O of the blocks so far is complete
           tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32(t_row + 128 + c * 32, o);
+          for (int c = 0; c < 8; ++c) {
+            uint32_t o[16];
+            tmem_ld_32x16(t_row + 128 + c * 16, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(t_row + 128 + c * 32, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x16(t_row + 128 + c * 16, o);
           }
-          tmem_st_wait();
         }
       }
-      float rs = 0.f;
+      // (a row with nothing visible yet has m_ref = -inf: subtract 0 instead, exp2(-inf) = 0)
+      const float ref = m_ref == -INFINITY ? 0.f : m_ref;
+      float rs0 = 0.f, rs1 = 0.f, rs2 = 0.f, rs3 = 0.f;
+      uint32_t pk[32];
 #pragma unroll
-      for (int c = 0; c < 64; c += 8) {
-        float e[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const float v = __uint_as_float(c < 32 ? s0[c + t] : s1[c - 32 + t]);
-          e[t] = fast_exp2(v - m_ref);      // -inf -> 0; a row with nothing visible yet has m_ref = -inf: (-inf) - (-inf) = nan, guarded below
-          if (m_ref == -INFINITY) e[t] = 0.f;
-          rs += e[t];
-        }
-        *reinterpret_cast<uint4*>(sP + r * 128 + (((c >> 3) ^ (r & 7)) << 4)) =
-            make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]), pack2(e[6], e[7]));
+      for (int c = 0; c < 32; c += 4) {
+        const float a = fast_exp2(fmaf(__uint_as_float(s0[c]), p.scale_log2e, -ref)), b = fast_exp2(fmaf(__uint_as_float(s0[c + 1]), p.scale_log2e, -ref));
+        const float e = fast_exp2(fmaf(__uint_as_float(s0[c + 2]), p.scale_log2e, -ref)), f = fast_exp2(fmaf(__uint_as_float(s0[c + 3]), p.scale_log2e, -ref));
+        rs0 += a; rs1 += b; rs2 += e; rs3 += f;
+        pk[c / 2] = pack2(a, b); pk[c / 2 + 1] = pack2(e, f);
       }
-      l += rs;
-      fence_proxy_async();
+#pragma unroll
+      for (int c = 0; c < 32; c += 4) {
+        const float a = fast_exp2(fmaf(__uint_as_float(s1[c]), p.scale_log2e, -ref)), b = fast_exp2(fmaf(__uint_as_float(s1[c + 1]), p.scale_log2e, -ref));
+        const float e = fast_exp2(fmaf(__uint_as_float(s1[c + 2]), p.scale_log2e, -ref)), f = fast_exp2(fmaf(__uint_as_float(s1[c + 3]), p.scale_log2e, -ref));
+        rs0 += a; rs1 += b; rs2 += e; rs3 += f;
+        pk[16 + c / 2] = pack2(a, b); pk[16 + c / 2 + 1] = pack2(e, f);
+      }
+      tmem_st_32x32(t_row + (j & 1) * FB, pk);
+      tmem_st_wait();
+      l += (rs0 + rs1) + (rs2 + rs3);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(barP);
+      if (lane == 0) mbar_arrive(&barP[j & 1]);
     }
-    if (ok && n_kv > 0 && !wait_parity(barO, (n_kv - 1) & 1, abort_flag)) ok = false;
-    __syncwarp();
-    ok = __all_sync(0xffffffffu, ok);
+    for (int j = n_kv > 1 ? n_kv - 2 : 0; ok && j < n_kv; ++j) ok = wait_parity_warp(&barO[j & 1], (j >> 1) & 1, abort_flag);
     if (!ok && lane == 0) fail(ST_TIMEOUT_TMEM_FULL);
     if (ok) {
       tc_fence_after();
@@ -439,6 +449,7 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
       if (valid) p.lse[(long long)row * p.heads_q + h] = (m_ref + log2f(l)) * 0.6931471805599453f;
     }
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 4) { tc_fence_after(); tmem_dealloc(tmem, 256); }
@@ -915,7 +926,7 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
   }
   dim3 grid((total_tokens + AB - 1) / AB + num_seqs, heads_q);
   if (serial) attn_fwd_kernel<<<grid, 128, ATT_SMEM, s>>>(p);
-  else attn_fwd_pipelined_kernel<<<grid, FWD2_THREADS, FWD2_SMEM, s>>>(p);
+  else attn_fwd_pipelined_kernel<<<grid.x * grid.y, FWD2_THREADS, FWD2_SMEM, s>>>(p);
   ++g_att_launches;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - (int)e;
