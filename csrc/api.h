@@ -40,6 +40,7 @@ typedef struct MdtGemmDesc {
   int c_fp32;          // C is fp32 instead of bf16
   int accumulate;      // C += alpha * (A*B) instead of C = alpha * (A*B)
   float alpha;
+  const float* alpha_dev;   // optional device scalar: alpha is multiplied by it (a factor that only the GPU knows)
   int* status;         // optional device word: set to a non-zero code if a wait inside the kernel gave up
   // mode 1, optional: the A rows are being delivered by peer GPUs.  Before a CTA loads the 128-row tile t of A it
   // waits (bounded) until tile_ready[t] >= tile_expected[t] (counters incremented by the senders with release).
@@ -103,7 +104,8 @@ int mdt_cross_entropy(void* logits, const long long* labels, float* loss_sum, fl
                       long long ld, int ignore_index, float grad_scale, cudaStream_t s);
 typedef struct MdtAdamTensor { void* p; const void* g; void* m; void* v; long long n; int p_fp32, g_fp32, s_fp32; } MdtAdamTensor;
 int mdt_adamw(const MdtAdamTensor* tensors_device, int num_tensors, long long max_n, float lr, float beta1, float beta2,
-              float eps, float weight_decay, float bc1, float bc2, float grad_scale, cudaStream_t s);
+              float eps, float weight_decay, float bc1, float bc2, float grad_scale,
+              const float* grad_scale_dev /* optional device scalar, multiplies grad_scale */, cudaStream_t s);
 int mdt_sumsq(const void* x, long long n, int fp32, float* out_accum, cudaStream_t s);
 // dst_i (fp32) += src_i (bf16 or fp32), i < count <= MDT_MULTI_ADD_MAX, one launch
 #define MDT_MULTI_ADD_MAX 16
@@ -116,9 +118,10 @@ int mdt_axpby(void* y, const void* x, long long n, float a, float b, int y_fp32,
 // stats (optional, fp32 [2 * experts], accumulated into): per-expert slot counts, then per-expert sums of the scores
 int mdt_router_fwd(const void* x, const void* w, void* scores, void* weights, int* idx, int tokens, int hidden,
                    int experts, int top_k, int normalize, float* stats, cudaStream_t s);
-int mdt_router_bwd(const void* x, const void* w, const void* scores, const void* weights, const int* idx,
-                   const void* dweights, const void* dscores, void* dx, float* dw, int tokens, int hidden, int experts,
-                   int top_k, int normalize, int accumulate_dx, cudaStream_t s);
+// dlogits (scratch, tokens * experts floats) and dw (experts * hidden floats, accumulated into): both NULL when no weight
+// gradient is wanted
+int mdt_router_bwd(const void* x, const void* w, const int* idx, const void* dweights, const void* dscores, void* dx, float* dlogits,
+                   float* dw, int tokens, int hidden, int experts, int top_k, int normalize, int accumulate_dx, cudaStream_t s);
 // counting sort of slots by expert id with block-padded groups; all outputs on device
 int mdt_make_plan(const int* expert_ids, int num_slots, int num_experts, int block, int capacity, int* counts,
                   int* padded_offsets, int* dest_row, int* src_slot, int* scratch, cudaStream_t s);

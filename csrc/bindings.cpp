@@ -86,7 +86,7 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
           bool a_mn_l, const OptTensor& B_l, const OptTensor& B2_l, bool b_mn_l, int64_t K_l, const OptTensor& C2,
           const OptTensor& C3, bool accumulate, double alpha, const OptTensor& status, const OptTensor& tile_ready,
           const OptTensor& tile_expected, const OptTensor& row_dest_rank, const OptTensor& row_dest_row, const OptTensor& peer_out,
-          const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt) {
+          const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt, const OptTensor& alpha_dev = std::nullopt) {
   CHECK_BF16(A); CHECK_BF16(B);
   c10::cuda::CUDAGuard guard(A.device());
   MdtGemmDesc d;
@@ -113,6 +113,11 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
   d.c_fp32 = C.scalar_type() == at::kFloat;
   TORCH_CHECK(d.c_fp32 || C.scalar_type() == at::kBFloat16, "C must be bf16 or fp32");
   d.accumulate = accumulate; d.alpha = (float)alpha;
+  if (alpha_dev.has_value()) {
+    TORCH_CHECK(alpha_dev->is_cuda() && alpha_dev->scalar_type() == at::kFloat && alpha_dev->numel() == 1, "alpha_dev must be a CUDA fp32 scalar");
+    TORCH_CHECK(!d.dual, "alpha has no place in the SwiGLU form");
+    d.alpha_dev = alpha_dev->data_ptr<float>();
+  }
   if (residual.has_value()) {
     TORCH_CHECK(residual->scalar_type() == at::kBFloat16 && residual->dim() == 2 && residual->stride(1) == 1 && residual->stride(0) == d.ldc &&
                 residual->size(0) >= M && residual->size(1) == N, "residual must be a bf16 matrix laid out like C");
@@ -145,20 +150,24 @@ std::vector<Tensor> rmsnorm_fwd(const Tensor& x, const Tensor& w, double eps) {
   check(mdt_rmsnorm_fwd(x2.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), (int)x2.size(0), (int)x2.size(1), (float)eps, cur_stream()), "rmsnorm_fwd");
   return {y.view(x.sizes()), rstd};
 }
-// dres (optional): gradient that reaches x over the residual connection, added to dx in the same pass
-std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd, const OptTensor& dres = std::nullopt) {
+// dres (optional): gradient that reaches x over the residual connection, added to dx in the same pass.  need_dw = false
+// (frozen norm): the second result is empty.
+std::vector<Tensor> rmsnorm_bwd(const Tensor& x, const Tensor& w, const Tensor& dy, const Tensor& rstd, const OptTensor& dres = std::nullopt,
+                                bool need_dw = true) {
   c10::cuda::CUDAGuard guard(x.device());
   auto x2 = x.reshape({-1, x.size(-1)}).contiguous();
   auto dy2 = dy.reshape({-1, x.size(-1)}).contiguous();
   auto dx = torch::empty_like(x2);
   const int rows = (int)x2.size(0), cols = (int)x2.size(1);
-  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  const int np = rows < sms ? (rows < 1 ? 1 : rows) : sms;
-  auto dwp = torch::empty({np, cols}, x.options().dtype(at::kFloat));
+  // two CTAs per SM where there are rows for them (each adds a row of partial sums); 4 to 6 rows per CTA hide the start
+  const int cap = 2 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+  const int np = std::max(1, std::min(rows, cap));
+  auto dwp = torch::empty({need_dw ? np : 0, cols}, x.options().dtype(at::kFloat));
   const void* dr = nullptr;
   Tensor drc;
   if (dres.has_value()) { drc = dres->reshape({-1, x.size(-1)}).contiguous(); TORCH_CHECK(drc.scalar_type() == at::kBFloat16); dr = drc.data_ptr(); }
-  check(mdt_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), rstd.data_ptr<float>(), dr, dx.data_ptr(), dwp.data_ptr<float>(), rows, cols, np, cur_stream()), "rmsnorm_bwd");
+  check(mdt_rmsnorm_bwd(x2.data_ptr(), w.data_ptr(), dy2.data_ptr(), rstd.data_ptr<float>(), dr, dx.data_ptr(), need_dw ? dwp.data_ptr<float>() : nullptr,
+                        rows, cols, np, cur_stream()), "rmsnorm_bwd");
   return {dx.view(x.sizes()), dwp};
 }
 // weight gradient of RMSNorm from the per-CTA partial sums of rmsnorm_bwd, in w's dtype
@@ -233,9 +242,11 @@ Tensor cross_entropy(Tensor& logits, const Tensor& labels, int64_t ignore_index,
   return out;
 }
 void adamw(std::vector<Tensor> ps, std::vector<Tensor> gs, std::vector<Tensor> ms, std::vector<Tensor> vs, double lr, double b1,
-           double b2, double eps, double wd, int64_t step, double grad_scale) {
+           double b2, double eps, double wd, int64_t step, double grad_scale, const OptTensor& grad_scale_dev = std::nullopt) {
   if (ps.empty()) return;
   c10::cuda::CUDAGuard guard(ps[0].device());
+  if (grad_scale_dev.has_value())
+    TORCH_CHECK(grad_scale_dev->device() == ps[0].device() && grad_scale_dev->scalar_type() == at::kFloat && grad_scale_dev->numel() == 1, "grad_scale_dev must be an fp32 scalar beside the parameters");
   std::vector<MdtAdamTensor> host(ps.size());
   long long max_n = 0;
   for (size_t i = 0; i < ps.size(); ++i) {
@@ -249,7 +260,7 @@ void adamw(std::vector<Tensor> ps, std::vector<Tensor> gs, std::vector<Tensor> m
   memcpy(staging.data_ptr(), host.data(), bytes);
   auto dev = staging.to(ps[0].device(), /*non_blocking=*/true);
   const float bc1 = 1.0f - (float)std::pow(b1, (double)step), bc2 = 1.0f - (float)std::pow(b2, (double)step);
-  check(mdt_adamw((const MdtAdamTensor*)dev.data_ptr(), (int)host.size(), max_n, (float)lr, (float)b1, (float)b2, (float)eps, (float)wd, bc1, bc2, (float)grad_scale, cur_stream()), "adamw");
+  check(mdt_adamw((const MdtAdamTensor*)dev.data_ptr(), (int)host.size(), max_n, (float)lr, (float)b1, (float)b2, (float)eps, (float)wd, bc1, bc2, (float)grad_scale, (const float*)cptr(grad_scale_dev), cur_stream()), "adamw");
 }
 // dst[i] (fp32, contiguous) += src[i] (bf16 or fp32, same number of elements): the gradient accumulators of one unit
 // in one launch per 16 tensors
@@ -301,19 +312,22 @@ std::vector<Tensor> router_fwd(const Tensor& x, const Tensor& w, int64_t top_k, 
   if (with_stats) return {scores, weights, idx, stats};
   return {scores, weights, idx};
 }
-// dx_accum (optional, bf16 [T, H]): the input gradient is added to it instead of written to a new tensor
+// dx_accum (optional, bf16 [T, H]): the input gradient is added to it instead of written to a new tensor.  need_dw = false
+// (frozen router): the second result is empty.
 std::vector<Tensor> router_bwd(const Tensor& x, const Tensor& w, const Tensor& idx, const Tensor& dweights, const OptTensor& dscores,
-                               bool normalize, const OptTensor& dx_accum = std::nullopt) {
+                               bool normalize, const OptTensor& dx_accum = std::nullopt, bool need_dw = true) {
   c10::cuda::CUDAGuard guard(x.device());
   const int T = (int)x.size(0), H = (int)x.size(1), E = (int)w.size(0), k = (int)idx.size(1);
   if (dx_accum.has_value()) TORCH_CHECK(dx_accum->is_contiguous() && dx_accum->scalar_type() == at::kBFloat16 && dx_accum->numel() == x.numel());
   auto dx = dx_accum.has_value() ? *dx_accum : torch::empty_like(x);
-  auto buf = torch::zeros({(int64_t)E * H + (int64_t)T * E}, x.options().dtype(at::kFloat));
+  auto dw = need_dw ? torch::zeros({E, H}, x.options().dtype(at::kFloat)) : torch::empty({0, H}, x.options().dtype(at::kFloat));
+  auto dlogits = need_dw ? torch::empty({T, E}, dw.options()) : dw;
   auto dwc = dweights.contiguous();
   OptTensor dsc = dscores.has_value() ? OptTensor(dscores->contiguous()) : std::nullopt;
-  check(mdt_router_bwd(x.data_ptr(), w.data_ptr(), nullptr, nullptr, idx.data_ptr<int>(), dwc.data_ptr(), cptr(dsc), dx.data_ptr(),
-                       buf.data_ptr<float>(), T, H, E, k, normalize, dx_accum.has_value() ? 1 : 0, cur_stream()), "router_bwd");
-  return {dx, buf.narrow(0, 0, (int64_t)E * H).view({E, H})};
+  check(mdt_router_bwd(x.data_ptr(), w.data_ptr(), idx.data_ptr<int>(), dwc.data_ptr(), cptr(dsc), dx.data_ptr(),
+                       need_dw ? dlogits.data_ptr<float>() : nullptr, need_dw ? dw.data_ptr<float>() : nullptr, T, H, E, k, normalize,
+                       dx_accum.has_value() ? 1 : 0, cur_stream()), "router_bwd");
+  return {dx, dw};
 }
 // returns counts[E], padded_offsets[E+1], dest_row[n], src_slot[capacity]
 std::vector<Tensor> make_plan(const Tensor& expert_ids, int64_t num_experts, int64_t block, int64_t capacity) {
@@ -522,6 +536,14 @@ bool skinny_ok(const Tensor& x, const Tensor& A, bool a_is_kr) {
          K % 8 == 0 && x.stride(1) == 1 && x.stride(0) % 8 == 0 && A.stride(1) == 1 &&
          (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 && (a_is_kr ? A.size(0) : A.size(1)) == K;
 }
+// Where both can run it, the tensor-core product is faster from about a million elements of x on (16 columns: 8000 x 4096
+// 89-133 us here, 25 there; 576 x 4096 13-17 / 13; 576 x 1024 9 / 13).
+bool skinny_preferred(const Tensor& x, const Tensor& A, bool a_is_kr) {
+  if (!skinny_ok(x, A, a_is_kr)) return false;
+  const int64_t r = a_is_kr ? A.size(1) : A.size(0);
+  const bool product_ok = r % 8 == 0 && A.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(A.data_ptr()) & 15) == 0;
+  return !product_ok || x.size(0) * x.size(1) < (1 << 20);
+}
 Tensor skinny_mm(const Tensor& x, const Tensor& A, bool a_is_kr, double alpha) {
   TORCH_CHECK(skinny_ok(x, A, a_is_kr), "skinny_mm: unsupported operands");
   c10::cuda::CUDAGuard guard(x.device());
@@ -552,7 +574,7 @@ std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTen
   }
   const int64_t r = l.A->size(0);
   Tensor t;
-  if (skinny_ok(x, *l.A, false)) {
+  if (skinny_preferred(x, *l.A, false)) {
     t = skinny_mm(x, *l.A, false, l.s);
   } else {
     t = torch::empty({M, r}, x.options());
@@ -570,7 +592,7 @@ LinGrads lin_bwd(const Tensor& dy, const Tensor& xin, const Lin& l, const OptTen
   OptTensor dt;
   if (l.A.has_value()) {
     const int64_t r = l.A->size(0);
-    if (skinny_ok(dy, *l.B, true)) {
+    if (skinny_preferred(dy, *l.B, true)) {
       dt = skinny_mm(dy, *l.B, true, l.s);                                                                           // s dy B
     } else {
       dt = torch::empty({M, r}, dy.options());
@@ -691,7 +713,7 @@ std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tens
   put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status));
   put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status));
   put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status));
-  auto rb = rmsnorm_bwd(x, params[0], d_xn, rstd, dyc);     // + dy: the residual connection's gradient
+  auto rb = rmsnorm_bwd(x, params[0], d_xn, rstd, dyc, (bool)needs[0]);     // + dy: the residual connection's gradient
   Tensor dx = rb[0];
   if (needs[0]) grads[0] = rmsnorm_dw(rb[1], params[0]);
   std::vector<Tensor> out;
@@ -818,11 +840,12 @@ std::vector<Tensor> moe_block_fwd(const Tensor& x, const Tensor& ln_w, const Ten
   return {out, plan[0], rstd, xn, wts, idx, ys, plan[1], plan[2], plan[3], meta_c, rr, rp, te, xg, *g, *u, h, expert_sorted, offs};
 }
 
-// state = the forward's return list; wg = {dw1, dw2, dw3} accumulation buffers ([El,F,H]) or empty when the experts are frozen.
+// state = the forward's return list; wg = {dw1, dw2, dw3} gradient buffers ([El,F,H]) or empty when the experts are frozen;
+// wg_add[i]: the buffer holds a gradient already and is added to, else it is written.
 // Returns {dx, d_ln, d_Wr}.
 std::vector<Tensor> moe_block_bwd(const Tensor& dy, const std::vector<Tensor>& state, const Tensor& x, const Tensor& ln_w, const Tensor& Wr,
-                                  const Tensor& w1, const Tensor& w2, const Tensor& w3, const std::vector<Tensor>& wg, double wscale,
-                                  int64_t top_k, int64_t E, const std::vector<int64_t>& layout, const std::vector<int64_t>& ep_ints,
+                                  const Tensor& w1, const Tensor& w2, const Tensor& w3, const std::vector<Tensor>& wg,
+                                  const std::vector<bool>& wg_add, double wscale, int64_t top_k, int64_t E, const std::vector<int64_t>& layout, const std::vector<int64_t>& ep_ints,
                                   const std::vector<Tensor>& ep, const Tensor& status_t, bool need_ln, bool need_router) {
   c10::cuda::CUDAGuard guard(dy.device());
   Phase ph("moe.backward");
@@ -854,14 +877,14 @@ std::vector<Tensor> moe_block_bwd(const Tensor& dy, const std::vector<Tensor>& s
   const int64_t R = dyg.size(0);
   Tensor dh = torch::empty({R, F}, x.options());
   ggemm(1, dyg, false, w2, false, dh, R, F, H, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, false, 1.0, status, w0, w1o, NONE, NONE, NONE, NONE);
-  if (!wg.empty()) { Tensor c = wg[1]; ggemm(2, h, true, dyg, true, c, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, true, wscale, status, NONE, NONE, NONE, NONE, NONE, NONE); }
+  if (!wg.empty()) { Tensor c = wg[1]; ggemm(2, h, true, dyg, true, c, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[1], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE); }
   auto gu = swiglu_bwd(g, u, dh, offs);
   Tensor dxg = torch::empty({R, H}, x.options());
   ggemm(1, gu[0], false, w1, true, dxg, R, H, F, El, offs, cap, NONE, gu[1], w3, true, F, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3);
   if (!wg.empty()) {
     Tensor c1 = wg[0], c3 = wg[2];
-    ggemm(2, gu[0], true, xg, true, c1, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, true, wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
-    ggemm(2, gu[1], true, xg, true, c3, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, true, wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
+    ggemm(2, gu[0], true, xg, true, c1, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[0], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
+    ggemm(2, gu[1], true, xg, true, c3, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[2], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
   }
   Tensor back;
   if (!is_ep) {
@@ -871,8 +894,8 @@ std::vector<Tensor> moe_block_bwd(const Tensor& dy, const std::vector<Tensor>& s
     back = ep[5].narrow(0, 0, n_slots);
   }
   Tensor dxn = combine_rows(back, dest_row, NONE, top_k);
-  auto rb = router_bwd(xn, Wr, idx, dwts, NONE, true, dxn);     // adds the router's input gradient to dxn
-  auto nb = rmsnorm_bwd(x, ln_w, dxn, rstd, dyc);               // + dy: the residual connection's gradient
+  auto rb = router_bwd(xn, Wr, idx, dwts, NONE, true, dxn, need_router);     // adds the router's input gradient to dxn
+  auto nb = rmsnorm_bwd(x, ln_w, dxn, rstd, dyc, need_ln);               // + dy: the residual connection's gradient
   Tensor dx = nb[0];
   Tensor none = torch::empty({0}, x.options());
   return {dx, need_ln ? rmsnorm_dw(nb[1], ln_w) : none, need_router ? rb[1].to(Wr.scalar_type()) : none};
@@ -883,9 +906,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("G"), py::arg("offsets"), py::arg("capacity_rows"), py::arg("B2"), py::arg("A_l"), py::arg("a_mn_l"), py::arg("B_l"), py::arg("B2_l"),
         py::arg("b_mn_l"), py::arg("K_l"), py::arg("C2"), py::arg("C3"), py::arg("accumulate"), py::arg("alpha"), py::arg("status"), py::arg("tile_ready"),
         py::arg("tile_expected"), py::arg("row_dest_rank"), py::arg("row_dest_row"), py::arg("peer_out"), py::arg("peer_arrive"),
-        py::arg("residual") = py::none());
+        py::arg("residual") = py::none(), py::arg("alpha_dev") = py::none());
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("x"), py::arg("w"), py::arg("dy"), py::arg("rstd"), py::arg("dres") = py::none());
+  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("x"), py::arg("w"), py::arg("dy"), py::arg("rstd"), py::arg("dres") = py::none(), py::arg("need_dw") = true);
   m.def("rmsnorm_dw", &rmsnorm_dw);
   m.def("rope", &rope);
   m.def("swiglu_fwd", &swiglu_fwd);
@@ -907,14 +930,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("gemm_rows_hint", [](int64_t rows) { mdt_gemm_rows_hint((long long)rows); });
   m.def("gemm_max_pairs", []() { return (int64_t)mdt_gemm_max_pairs(); });
+  m.def("skinny_preferred", &skinny_preferred);
   m.def("skinny_mm", &skinny_mm);
-  m.def("adamw", &adamw);
+  m.def("adamw", &adamw, py::arg("ps"), py::arg("gs"), py::arg("ms"), py::arg("vs"), py::arg("lr"), py::arg("b1"), py::arg("b2"), py::arg("eps"), py::arg("wd"),
+        py::arg("step"), py::arg("grad_scale"), py::arg("grad_scale_dev") = py::none());
   m.def("multi_add", &multi_add);
   m.def("sumsq", &sumsq);
   m.def("axpby", &axpby);
   m.def("router_fwd", &router_fwd, py::arg("x"), py::arg("w"), py::arg("top_k"), py::arg("normalize"), py::arg("with_stats") = false);
   m.def("router_bwd", &router_bwd, py::arg("x"), py::arg("w"), py::arg("idx"), py::arg("dweights"), py::arg("dscores"), py::arg("normalize"),
-        py::arg("dx_accum") = py::none());
+        py::arg("dx_accum") = py::none(), py::arg("need_dw") = true);
   m.def("make_plan", &make_plan);
   m.def("gather_rows", &gather_rows);
   m.def("combine_rows", &combine_rows, py::arg("y"), py::arg("dest_row"), py::arg("weights"), py::arg("top_k"), py::arg("residual") = py::none());

@@ -82,82 +82,147 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
 }
 
 // dx = rstd * (dy*w - x * rstd^2 * mean(dy*w*x)) (+ dres, the gradient that reaches x past the norm through the
-// residual connection);  dw partial sums per CTA (CTA loops over rows)
-__global__ void rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ dy,
-                                   const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
-                                   float* __restrict__ dw_partial, int rows, int cols) {
+// residual connection);  dw partial sums per CTA (CTA loops over rows), unless dw_partial is NULL (frozen norm).
+// Bound by one pass over x, dy, dres and dx.  A thread holds its NV vectors of the row and of the next one in registers,
+// so a row costs one barrier-separated sum and its loads are in flight while the row before it is reduced; several CTAs
+// share an SM.  8000 x 4096 with dres: 165 us with the row read twice by one CTA per SM, without a look ahead.
+template <int NV>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ dy,
+                                                          const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
+                                                          float* __restrict__ dw_partial, int rows, int cols) {
   __shared__ float red[32];
   const int nv = cols / 8;
-  // each thread owns vectors i = threadIdx.x + k*blockDim.x, k < 8 (cols <= 8*8*blockDim.x)
-  float acc[8][8];
+  const uint4* xr = reinterpret_cast<const uint4*>(x);
+  const uint4* dr = reinterpret_cast<const uint4*>(dy);
+  const uint4* rr = reinterpret_cast<const uint4*>(dres);
+  uint4* ox = reinterpret_cast<uint4*>(dx);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  float acc[NV][8];
+  uint4 wv[NV], xn[NV], dn[NV], rn[NV];
+  float rs = 0.f;
+  auto load = [&](int row) {
 #pragma unroll
-  for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < NV; ++k) {
+      const int i = threadIdx.x + k * 256;
+      const bool in = i < nv;
+      const long long at = (long long)row * nv + i;
+      xn[k] = in ? xr[at] : zero; dn[k] = in ? dr[at] : zero; rn[k] = in && rr != nullptr ? rr[at] : zero;
+    }
+    rs = rstd[row];
+  };
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * 256;
+    wv[k] = i < nv ? reinterpret_cast<const uint4*>(w)[i] : zero;
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[k][j] = 0.f;
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  }
+  constexpr bool AHEAD = NV <= 4;      // (more columns: no registers for the next row)
+  if (AHEAD && (int)blockIdx.x < rows) load(blockIdx.x);
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * cols);
-    const uint4* dr = reinterpret_cast<const uint4*>(dy + (long long)row * cols);
-    uint4* ox = reinterpret_cast<uint4*>(dx + (long long)row * cols);
-    const uint4* rr = dres != nullptr ? reinterpret_cast<const uint4*>(dres + (long long)row * cols) : nullptr;
-    const float r = rstd[row];
+    if (!AHEAD) load(row);
+    uint4 xv[NV], dv[NV], rv[NV];
+    const float r = rs;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) { xv[k] = xn[k]; dv[k] = dn[k]; rv[k] = rn[k]; }
+    if (AHEAD && row + (int)gridDim.x < rows) load(row + gridDim.x);
     float dot = 0.f;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      float xf[8], df[8], wf[8]; unpack8(xr[i], xf); unpack8(dr[i], df); unpack8(wr[i], wf);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      float xf[8], df[8], wf[8]; unpack8(xv[k], xf); unpack8(dv[k], df); unpack8(wv[k], wf);
 #pragma unroll
       for (int j = 0; j < 8; ++j) dot += df[j] * wf[j] * xf[j];
     }
     dot = block_sum(dot, red);
     const float c = dot * r * r / cols;
-    int k = 0;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x, ++k) {
-      float xf[8], df[8], wf[8], o[8]; unpack8(xr[i], xf); unpack8(dr[i], df); unpack8(wr[i], wf);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = threadIdx.x + k * 256;
+      float xf[8], df[8], wf[8], rf[8], o[8]; unpack8(xv[k], xf); unpack8(dv[k], df); unpack8(wv[k], wf); unpack8(rv[k], rf);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        o[j] = r * (df[j] * wf[j] - xf[j] * c);
-        if (k < 8) acc[k][j] += df[j] * xf[j] * r;
+        o[j] = r * (df[j] * wf[j] - xf[j] * c) + rf[j];
+        acc[k][j] += df[j] * xf[j] * r;
       }
-      if (rr != nullptr) {
-        float rf[8]; unpack8(rr[i], rf);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += rf[j];
-      }
-      ox[i] = pack8(o);
+      if (i < nv) ox[(long long)row * nv + i] = pack8(o);
     }
   }
-  int k = 0;
-  for (int i = threadIdx.x; i < nv && k < 8; i += blockDim.x, ++k) {
-    float* dst = dw_partial + (long long)blockIdx.x * cols + i * 8;
+  if (dw_partial == nullptr) return;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dst[j] = acc[k][j];
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * 256;
+    if (i < nv) {
+      float4* dst = reinterpret_cast<float4*>(dw_partial + (long long)blockIdx.x * cols + i * 8);
+      dst[0] = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+      dst[1] = make_float4(acc[k][4], acc[k][5], acc[k][6], acc[k][7]);
+    }
   }
 }
 
-// dw[c] = sum over the partial rows (+ cast): finishes the weight gradient of rmsnorm_bwd_kernel in one launch
-__global__ void rmsnorm_dw_finalize_kernel(const float* __restrict__ partial, int n_partial, int cols, bf16* __restrict__ dw_bf16,
-                                           float* __restrict__ dw_f32) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
+// dw[c] = sum over the partial rows (+ cast): finishes the weight gradient of rmsnorm_bwd_kernel in one launch.  The
+// partial rows are spread over the 8 warps of a CTA (32 columns each), eight loads in flight per lane.
+__global__ void __launch_bounds__(256) rmsnorm_dw_finalize_kernel(const float* __restrict__ partial, int n_partial, int cols, bf16* __restrict__ dw_bf16,
+                                                                  float* __restrict__ dw_f32) {
+  __shared__ float part[8][33];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int r = 0; r < n_partial; ++r) s += partial[(long long)r * cols + c];
+  if (c < cols) {
+#pragma unroll 8
+    for (int r = wp; r < n_partial; r += 8) s += partial[(long long)r * cols + c];
+  }
+  part[wp][lane] = s;
+  __syncthreads();
+  if (wp != 0 || c >= cols) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) s += part[k][lane];
   if (dw_bf16 != nullptr) dw_bf16[c] = __float2bfloat16(s);
   if (dw_f32 != nullptr) dw_f32[c] = s;
 }
 
 // ------------------------------------------------------------------------------------ RoPE
 // x: [tokens, heads, d]; pairs (i, i + d/2) rotated by pos * theta^(-2i/d); inverse negates the angle
-__global__ void rope_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const int* __restrict__ pos, int tokens,
-                            int heads, int d, float log2_theta, int inverse) {
+// One CTA per token: its d/2 angles are evaluated once, into shared memory, and used for all heads; a thread then
+// rotates eight pairs with 16-byte accesses (head sizes that are a multiple of 16; else pair by pair).
+// 8000 tokens x 32 heads of 128: 85 us with one sincosf and 2-byte accesses per pair.
+__global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const int* __restrict__ pos, int tokens,
+                                                   int heads, int d, float log2_theta, int inverse, int vec) {
+  extern __shared__ float angles[];            // cos [half] | sin [half]
   const int t = blockIdx.x;
   const int half = d / 2;
   const float p = (float)pos[t];
-  for (int idx = threadIdx.x; idx < heads * half; idx += blockDim.x) {
-    const int h = idx / half, i = idx - h * half;
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
     const float inv_freq = exp2f(-log2_theta * (2.0f * i / d));
     float s, c;
     sincosf(p * inv_freq, &s, &c);
-    if (inverse) s = -s;
-    const long long base = ((long long)t * heads + h) * d;
+    angles[i] = c;
+    angles[half + i] = inverse ? -s : s;
+  }
+  __syncthreads();
+  const long long row = (long long)t * heads * d;
+  if (vec) {
+    const int per = half / 8;
+    for (int idx = threadIdx.x; idx < heads * per; idx += blockDim.x) {
+      const int h = idx / per, i = (idx - h * per) * 8;
+      const long long base = row + (long long)h * d + i;
+      float a[8], b[8], u[8], v[8];
+      unpack8(*reinterpret_cast<const uint4*>(x + base), a);
+      unpack8(*reinterpret_cast<const uint4*>(x + base + half), b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float c = angles[i + j], s = angles[half + i + j];
+        u[j] = a[j] * c - b[j] * s;
+        v[j] = b[j] * c + a[j] * s;
+      }
+      *reinterpret_cast<uint4*>(y + base) = pack8(u);
+      *reinterpret_cast<uint4*>(y + base + half) = pack8(v);
+    }
+    return;
+  }
+  for (int idx = threadIdx.x; idx < heads * half; idx += blockDim.x) {
+    const int h = idx / half, i = idx - h * half;
+    const float s = angles[half + i], c = angles[i];
+    const long long base = row + (long long)h * d;
     const float a = __bfloat162float(x[base + i]), b = __bfloat162float(x[base + i + half]);
     y[base + i] = __float2bfloat16(a * c - b * s);
     y[base + i + half] = __float2bfloat16(b * c + a * s);
@@ -297,8 +362,10 @@ __device__ __forceinline__ bool aligned16(const void* a, const void* b, const vo
 // thread and iteration through 128-bit loads (four loads in flight per thread, 32 warps per SM); everything else,
 // and the tail, element by element.
 __global__ void __launch_bounds__(256, 4) adamw_kernel(const MdtAdamTensor* __restrict__ tensors, float lr, float b1, float b2,
-                                                       float eps, float wd, float ibc1, float ibc2, float gscale) {
+                                                       float eps, float wd, float ibc1, float ibc2, float gscale,
+                                                       const float* __restrict__ gscale_dev) {
   const MdtAdamTensor t = tensors[blockIdx.y];
+  if (gscale_dev != nullptr) gscale *= *gscale_dev;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
   long long done = 0;
@@ -437,20 +504,25 @@ extern "C" int mdt_rmsnorm_fwd(const void* x, const void* w, void* y, float* rst
 extern "C" int mdt_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, const void* dres, void* dx,
                                float* dw_partial, int rows, int cols, int n_partial, cudaStream_t s) {
   if (cols % 8 != 0 || cols > 8 * 8 * 256) return -1;
-  rmsnorm_bwd_kernel<<<n_partial, 256, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd, (const bf16*)dres, (bf16*)dx, dw_partial,
-                                              rows, cols);
+  const int nv = (cols / 8 + 255) / 256;
+#define RMS_BWD(NV) rmsnorm_bwd_kernel<NV><<<n_partial, 256, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd, (const bf16*)dres, (bf16*)dx, dw_partial, rows, cols)
+  if (nv <= 1) RMS_BWD(1); else if (nv <= 2) RMS_BWD(2); else if (nv <= 4) RMS_BWD(4); else RMS_BWD(8);
+#undef RMS_BWD
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_rmsnorm_dw_finalize(const float* dw_partial, int n_partial, int cols, void* dw_bf16, float* dw_f32, cudaStream_t s) {
-  rmsnorm_dw_finalize_kernel<<<(cols + 255) / 256, 256, 0, s>>>(dw_partial, n_partial, cols, (bf16*)dw_bf16, dw_f32);
+  rmsnorm_dw_finalize_kernel<<<(cols + 31) / 32, 256, 0, s>>>(dw_partial, n_partial, cols, (bf16*)dw_bf16, dw_f32);
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_rope(const void* x, void* y, const int* positions, int tokens, int heads, int head_dim, float theta,
                         int inverse, cudaStream_t s) {
   if (tokens == 0) return 0;
-  rope_kernel<<<tokens, 256, 0, s>>>((const bf16*)x, (bf16*)y, positions, tokens, heads, head_dim, log2f(theta), inverse);
+  const int vec = head_dim % 16 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  const int work = vec ? heads * (head_dim / 16) : heads * (head_dim / 2);          // threads that have something to do
+  const int threads = work <= 64 ? 64 : (work <= 128 ? 128 : 256);
+  rope_kernel<<<tokens, threads, (head_dim / 2) * 2 * sizeof(float), s>>>((const bf16*)x, (bf16*)y, positions, tokens, heads, head_dim, log2f(theta), inverse, vec);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -506,10 +578,10 @@ extern "C" int mdt_cross_entropy(void* logits, const long long* labels, float* l
   return 0;
 }
 extern "C" int mdt_adamw(const MdtAdamTensor* tensors_device, int num_tensors, long long max_n, float lr, float beta1, float beta2,
-                         float eps, float weight_decay, float bc1, float bc2, float grad_scale, cudaStream_t s) {
+                         float eps, float weight_decay, float bc1, float bc2, float grad_scale, const float* grad_scale_dev, cudaStream_t s) {
   if (num_tensors == 0) return 0;
   dim3 grid(grid_for((max_n + 7) / 8, 256, -16), num_tensors);
-  adamw_kernel<<<grid, 256, 0, s>>>(tensors_device, lr, beta1, beta2, eps, weight_decay, 1.0f / bc1, 1.0f / bc2, grad_scale);
+  adamw_kernel<<<grid, 256, 0, s>>>(tensors_device, lr, beta1, beta2, eps, weight_decay, 1.0f / bc1, 1.0f / bc2, grad_scale, grad_scale_dev);
   MDT_CHECK_LAUNCH();
   return 0;
 }

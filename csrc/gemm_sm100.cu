@@ -52,6 +52,7 @@ struct GemmParams {
   long long ldc, c_group_stride;
   int c_fp32, accumulate;
   float alpha;
+  const float* alpha_dev;
   int store_gate_up;
   int* status;
   const unsigned* tile_ready; const int* tile_expected;
@@ -353,6 +354,7 @@ __device__ __forceinline__ EpiRow epi_row(const GemmParams& p, int g, int row, b
   }
   return r;
 }
+__device__ __forceinline__ float gemm_alpha(const GemmParams& p) { return p.alpha_dev != nullptr ? p.alpha * *p.alpha_dev : p.alpha; }
 // publish a warp's delivered rows: one count per (row, column tile) and destination
 __device__ __forceinline__ void epi_publish(const GemmParams& p, int dest, int lane) {
   __threadfence_system();
@@ -418,6 +420,7 @@ __device__ __forceinline__ bool epi_tile(const GemmParams& p, uint8_t* stage, ui
   constexpr int CHUNKS = BN / 128;                // 64-column chunks of this warp
   const int col0 = n0 + half * (BN / 2);
   const bool add = fast && (p.accumulate || p.R != nullptr);
+  const float alpha = gemm_alpha(p);
   const unsigned long long src = p.accumulate ? mine : reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(p.R) + r.base);
   uint4 pre[8];                                   // (two chunks' worth of registers would spill, and serialise the loads)
   if (add) epi_fetch(pre, src, row_ok, lane, col0, p.N, p.accumulate ? p.C : p.R);
@@ -437,7 +440,7 @@ __device__ __forceinline__ bool epi_tile(const GemmParams& p, uint8_t* stage, ui
       tmem_ld_32x32(tacc + half * (BN / 2) + ch * 64 + part * 32, acc);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]) * p.alpha;
+      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]) * alpha;
       if (add) {
         epi_stage_row<true>(stage, v, part, lane);
       } else if (fast) {
@@ -673,6 +676,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
         before = __shfl_sync(0xffffffffu, before, 0);
         if (before != (unsigned)w.contributors - 1u) continue;
         __threadfence();
+        const float alpha = gemm_alpha(p);
 #pragma unroll 1
         for (int c = 0; c < BN / 2; c += 8) {
           float o[8];
@@ -681,7 +685,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
             float4* src = ws + (c + i) / 4 * BM;
             const float4 v = __ldcg(src);
             __stcg(src, make_float4(0.f, 0.f, 0.f, 0.f));   // leave the workspace clean
-            o[i] = v.x * p.alpha; o[i + 1] = v.y * p.alpha; o[i + 2] = v.z * p.alpha; o[i + 3] = v.w * p.alpha;
+            o[i] = v.x * alpha; o[i + 1] = v.y * alpha; o[i + 2] = v.z * alpha; o[i + 3] = v.w * alpha;
           }
           const int col = t.n0 + half * (BN / 2) + c;
           if (r.ok && col < p.N) store8(r.C, r.base + col, o, p.c_fp32, p.accumulate, p.R);
@@ -925,6 +929,174 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   tc_fence_before();
   cluster_sync_all();
   if (warp == 1) { tc_fence_after(); tmem_dealloc_pair(tmem_base, TMEM_COLS); }
+}
+
+// ---------------------------------------------------------------------------------------------
+// Products with few output tiles: a cluster of S CTAs shares one 128 x BN tile along the depth.
+//
+// 16 tiles of a 4096-deep projection of one prompt leave 132 SMs idle while each tile's 64 k blocks wait for memory one
+// ring at a time (43 us); the adapters' down projections are one column of tiles, 224 deep for the experts.  Here
+// CTA c of a cluster takes the c-th part of the k blocks; the S partial tiles then go to shared memory (the ring is
+// free by then) and every CTA adds up its share of the tile from all S of them, in the order of the ranks, so that the
+// result does not depend on timing.  BN = 64 serves the adapter ranks (64 columns are one swizzle atom).  Same roles as the 128-row kernel, one tile per cluster, no peers' rows (those products keep the other kernels).
+// ---------------------------------------------------------------------------------------------
+constexpr int MAX_CLUSTER = 8;
+template <int BN> struct SplitShape {
+  static constexpr int STAGE = A_BYTES + BN * BK * 2;
+  static constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 6 : 8);   // 192 KB
+  static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+  static_assert(STAGES * STAGE >= BM * BN * 4, "the ring must hold the fp32 tile");
+  static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
+};
+
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
+  return v;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(const __grid_constant__ GemmParams p) {
+  constexpr int STAGES = SplitShape<BN>::STAGES, STAGE_BYTES = SplitShape<BN>::STAGE;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* done_bar = empty_bar + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank(), S = (int)cluster_nctarank();
+  Tile t;
+  if (!locate_tile<BN, BM>(p, (int)cluster_id_x(), t)) return;      // the same for the whole cluster
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(done_bar, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, BN); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  auto fail = [&](int code) {
+    *abort_flag = 1;
+    if (p.status != nullptr) atomicCAS(p.status, 0, code);
+  };
+  const int total = t.num_kb + (t.num_kb > 0 || p.mode != 2 ? t.num_kb_l : 0);
+  const int kb0 = total * rank / S, kb1 = total * (rank + 1) / S;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (elect_one()) { prefetch_tensormap(&p.tmA); prefetch_tensormap(&p.tmB); }
+    bool ok = true;
+    if (p.mode != 2 && kb1 > kb0 && (p.rdy_b.ready != nullptr || p.rdy_bl.ready != nullptr)) {
+      ok = __all_sync(0xffffffffu, wait_b_tile(p, t.g, t.n0, BN));
+      if (!ok) fail(ST_TIMEOUT_PEER);
+      fence_proxy_async_all();
+    }
+    for (int kb = kb0, it = 0; ok && kb < kb1; ++kb, ++it) {
+      const int s = it % STAGES;
+      ok = wait_parity_warp(&empty_bar[s], ((it / STAGES) & 1) ^ 1, abort_flag);
+      if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+      uint8_t* sA = smem + s * STAGE_BYTES;
+      uint8_t* sB = sA + A_BYTES;
+      const bool lora = kb >= t.num_kb;
+      const int kk = (lora ? kb - t.num_kb : kb) * BK;
+      const CUtensorMap* mA = lora ? &p.tmA_l : &p.tmA;
+      const CUtensorMap* mB = lora ? &p.tmB_l : &p.tmB;
+      const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
+      const int krow = (lora ? 0 : t.krow0) + kk;
+      const int zB = (p.mode == 2) ? 0 : t.g;
+      if (elect_one()) {
+        mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+        if (a_mn == 0) {
+          tma_load_2d(sA, mA, &full_bar[s], kk, t.m0);
+        } else {
+          tma_load_2d(sA, mA, &full_bar[s], t.m0, krow);
+          tma_load_2d(sA + 8192, mA, &full_bar[s], t.m0 + 64, krow);
+        }
+        if (b_mn == 0) {
+          tma_load_3d(sB, mB, &full_bar[s], kk, t.n0, zB);
+        } else {
+#pragma unroll
+          for (int c = 0; c < BN / 64; ++c) tma_load_3d(sB + c * 8192, mB, &full_bar[s], t.n0 + 64 * c, krow, zB);
+        }
+      }
+    }
+    if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {}
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    bool ok = true;
+    for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+      const int s = it % STAGES;
+      ok = wait_parity_warp(&full_bar[s], (it / STAGES) & 1, abort_flag);
+      if (!ok) { fail(ST_TIMEOUT_FULL); break; }
+      tc_fence_after();
+      const bool lora = kb >= t.num_kb;
+      const int a_mn = lora ? p.a_mn_l : p.a_mn, b_mn = lora ? p.b_mn_l : p.b_mn;
+      const uint32_t idesc = make_idesc_bf16(BM, BN, a_mn, b_mn);
+      const uint32_t sA = smem_u32(smem + s * STAGE_BYTES);
+      const uint64_t da = operand_desc(sA, a_mn), db = operand_desc(sA + A_BYTES, b_mn);
+      const uint32_t ka = operand_kstep(a_mn), kbs = operand_kstep(b_mn);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k) umma_bf16(tmem, da + k * ka, db + k * kbs, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+        umma_commit(&empty_bar[s]);
+      }
+    }
+    if (ok && kb1 > kb0 && elect_one()) umma_commit(done_bar);
+  } else {
+    // ------------------------------------------------------------------ partial tile: TMEM -> shared memory [column / 4][row][4]
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    float4* part = reinterpret_cast<float4*>(smem) + q * 32 + lane;
+    if (kb1 > kb0) {
+      const bool ok = wait_parity_warp(done_bar, 0, abort_flag);
+      if (!ok) fail(ST_TIMEOUT_TMEM_FULL);
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = half * (BN / 2); ok && c < (half + 1) * (BN / 2); c += 16) {
+        uint32_t acc[16];
+        tmem_ld_32x16(tmem + c + ((uint32_t)(q * 32) << 16), acc);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i += 4)
+          part[(c + i) / 4 * BM] = make_float4(__uint_as_float(acc[i]), __uint_as_float(acc[i + 1]), __uint_as_float(acc[i + 2]), __uint_as_float(acc[i + 3]));
+      }
+    } else {
+      for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 4) part[c / 4 * BM] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();                                             // all partial tiles are in place
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, BN); }
+  // this CTA's share: units of one row x 8 columns, rows fastest
+  constexpr int UNITS = BM * (BN / 8);
+  const float alpha = gemm_alpha(p);
+  const int row_limit = (p.mode == 1) ? p.offsets[p.G] : p.M;
+  const bool empty = total == 0 && p.accumulate;
+  const uint32_t part0 = smem_u32(smem);
+  for (int u = UNITS * rank / S + (int)threadIdx.x; u < UNITS * (rank + 1) / S && !empty; u += GEMM_THREADS) {
+    const int r = u % BM, g8 = u / BM;
+    const int row = t.m0 + r, col = t.n0 + g8 * 8;
+    if (row >= row_limit || col >= p.N) continue;
+    float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const uint32_t at = part0 + ((2 * g8) * BM + r) * 16;
+    for (int c = 0; c < S; ++c) {
+      const uint32_t a = mapa_shared(at, c);
+      const float4 x = ld_cluster_v4(a), y = ld_cluster_v4(a + BM * 16);
+      o[0] += x.x; o[1] += x.y; o[2] += x.z; o[3] += x.w; o[4] += y.x; o[5] += y.y; o[6] += y.z; o[7] += y.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] *= alpha;
+    store8(p.C, (p.mode == 2 ? (long long)t.g * p.c_group_stride : 0) + (long long)row * p.ldc + col, o, p.c_fp32, p.accumulate, p.R);
+  }
+  cluster_sync_all();                                             // nobody leaves while its partial tile is read
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1181,6 +1353,49 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
   return wide ? 2 : 0;
 }
 
+// Whether a product with few tiles is cut along the depth, and how: cluster size (0 = not) and tile width.  Times in
+// microseconds, measured on B200: 0.48 / 0.28 / 0.22 per k block of a 256 / 128 / 64-wide tile, 5 for the exchange of the
+// partial tiles; against one CTA per tile (0.28 + 1, 128-wide outputs) or the faster of the two 256-wide kernels in one
+// round.  128 CTAs at most: a cluster needs its SMs in one GPC.
+static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int num_sms, int* bn) {
+  if (d->dual || d->tile_ready != nullptr || d->row_dest_rank != nullptr || (d->accumulate && d->R != nullptr)) return 0;
+  const int G = d->G < 1 ? 1 : d->G;
+  *bn = d->N <= 64 ? 64 : (d->N <= 128 ? 128 : 256);
+  double rows = (double)d->M, depth = (double)d->K, n = (double)d->capacity_rows - 127.0 * G;
+  if (n < G) n = G;
+  if (thread_rows_hint > 0 && (double)thread_rows_hint < n) n = (double)thread_rows_hint;
+  double blocks = ceil(rows / BM);
+  if (d->mode == 1) blocks = fmax(n / BM + 0.5 * G, (double)G);
+  if (d->mode == 2 && d->offsets != nullptr) depth = n / G;
+  const double tiles = blocks * ((d->N + *bn - 1) / *bn) * (d->mode == 2 ? G : 1);
+  const double kb = ceil(depth / BK) + ceil((double)d->K_l / BK);
+  const double per = *bn == 256 ? 0.48 : (*bn == 128 ? 0.28 : 0.22);
+  const double whole = d->N <= 128 ? kb * 0.28 + 1.0 : fmin(kb * 0.48 + 1.0, kb * 0.34 + 2.0);
+  for (int S = MAX_CLUSTER; S >= 2; S /= 2)
+    if (tiles * S <= num_sms * 128.0 / 148.0 && kb >= 4.0 * S) return ceil(kb / S) * per + 5.0 < whole ? S : 0;
+  return 0;
+}
+
+template <int BN>
+static cudaError_t launch_cluster(const GemmParams& p, int tiles, int S, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_cluster_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitShape<BN>::SMEM);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(tiles * S)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = SplitShape<BN>::SMEM; cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_cluster_kernel<BN>, p);
+  ++g_launches;
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 }  // namespace mdt
 
 extern "C" long long mdt_gemm_launch_count() { return mdt::g_launches; }
@@ -1217,7 +1432,7 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   p.M = d->M; p.N = d->N; p.K = d->K; p.K_l = d->K_l; p.G = d->G < 1 ? 1 : d->G; p.mode = d->mode;
   p.a_mn = d->a_mn; p.b_mn = d->b_mn; p.a_mn_l = d->a_mn_l; p.b_mn_l = d->b_mn_l; p.dual = d->dual;
   p.offsets = d->offsets; p.C = d->C; p.C2 = d->C2; p.C3 = d->C3; p.ldc = d->ldc; p.c_group_stride = d->c_group_stride;
-  p.c_fp32 = d->c_fp32; p.accumulate = d->accumulate; p.alpha = d->alpha; p.store_gate_up = d->C2 != nullptr;
+  p.c_fp32 = d->c_fp32; p.accumulate = d->accumulate; p.alpha = d->alpha; p.alpha_dev = d->alpha_dev; p.store_gate_up = d->C2 != nullptr;
   p.status = d->status;
   p.tile_ready = d->tile_ready; p.tile_expected = d->tile_expected;
   p.row_dest_rank = d->row_dest_rank; p.row_dest_row = d->row_dest_row; p.peer_out = d->peer_out; p.peer_arrive = d->peer_arrive;
@@ -1234,19 +1449,20 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   if (p.dual && (p.b_mn != 0 || p.c_fp32 || p.accumulate)) return -11;
   const int BN = (p.dual || p.N > 128) ? 256 : 128;
   const int bn_out = p.dual ? BN / 2 : BN;
-  const int tiling = choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms);
-  const bool pair = tiling != 0;
+  int cluster_bn = 0;
+  const int cluster = pair_policy() == MAX_POLICY ? choose_cluster(d, t_rows_hint, g_num_sms, &cluster_bn) : 0;
+  const bool pair = cluster == 0 && choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms) != 0;
   const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
   int rc = 0;
   // A: [a_rows, a_cols] row-major, a_cols contiguous.  K-major: rows = M, cols = K.  MN-major: rows = depth, cols = M.
   rc |= make_map(&p.tmA, d->A, d->a_cols, d->a_rows, 1, d->lda, 0, 64, d->a_mn ? 64 : BM, 2);
   // B: [G, b_rows, b_cols].  K-major: rows = N, cols = K.  MN-major: rows = depth, cols = N.
-  const uint32_t b_box_rows = d->b_mn ? 64 : (half_box ? 128 : bn_out);
+  const uint32_t b_box_rows = d->b_mn ? 64 : (cluster ? cluster_bn : (half_box ? 128 : bn_out));
   rc |= make_map(&p.tmB, d->B, d->b_cols, d->b_rows, p.mode == 2 ? 1 : p.G, d->ldb, d->b_group_stride, 64, b_box_rows, 3);
   if (p.dual) rc |= make_map(&p.tmB2, d->B2, d->b_cols, d->b_rows, p.G, d->ldb, d->b_group_stride, 64, b_box_rows, 3);
   if (p.K_l > 0) {
     rc |= make_map(&p.tmA_l, d->A_l, d->al_cols, d->al_rows, 1, d->lda_l, 0, 64, d->a_mn_l ? 64 : BM, 2);
-    const uint32_t bl_box_rows = d->b_mn_l ? 64 : (half_box ? 128 : bn_out);
+    const uint32_t bl_box_rows = d->b_mn_l ? 64 : (cluster ? cluster_bn : (half_box ? 128 : bn_out));
     rc |= make_map(&p.tmB_l, d->B_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, bl_box_rows, 3);
     if (p.dual) rc |= make_map(&p.tmB2_l, d->B2_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, bl_box_rows, 3);
   }
@@ -1255,6 +1471,12 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   long long rows = (p.mode == 1) ? d->capacity_rows : p.M;
   long long tiles = ((rows + BM - 1) / BM) * ((p.N + bn_out - 1) / bn_out) * (p.mode == 2 ? p.G : 1);
   int grid = (int)(tiles < g_num_sms ? (tiles < 1 ? 1 : tiles) : g_num_sms);
+  if (cluster) {
+    const int nt = (int)(((rows + BM - 1) / BM) * ((p.N + cluster_bn - 1) / cluster_bn) * (p.mode == 2 ? p.G : 1));
+    const cudaError_t e4 = cluster_bn == 256 ? launch_cluster<256>(p, nt, cluster, stream)
+                         : (cluster_bn == 128 ? launch_cluster<128>(p, nt, cluster, stream) : launch_cluster<64>(p, nt, cluster, stream));
+    return e4 == cudaSuccess ? 0 : -100 - (int)e4;
+  }
   if (pair) {
     long long pairs = ((rows + 2 * BM - 1) / (2 * BM) + (p.mode == 1 ? p.G : 0)) * ((p.N + bn_out - 1) / bn_out) * (p.mode == 2 ? p.G : 1);
     const int np = (int)(pairs < 1 ? 1 : (pairs > g_num_sms ? g_num_sms : pairs));

@@ -9,6 +9,7 @@
 
 #include "api.h"
 #include "common/host.h"
+#include "common/ptx.cuh"
 
 namespace mdt {
 
@@ -36,38 +37,53 @@ __device__ __forceinline__ float wsum(float v) {
   return v;
 }
 
-// logits[e] = <x[t,:], w[e,:]> for one token per warp; every lane ends with all E logits.
-// `w` may point to shared memory (see stage_router_weights).  Four 16-byte loads of x are in flight per lane.
-template <int E_T>
-__device__ __forceinline__ void token_logits(const bf16* __restrict__ x, const bf16* w, int hidden, int experts,
-                                             int lane, float (&logit)[E_T]) {
-#pragma unroll
-  for (int e = 0; e < E_T; ++e) logit[e] = 0.f;
-  const uint4* xr = reinterpret_cast<const uint4*>(x);
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
+// logits[u][e] = <x[t0 + u * step,:], w[e,:]> for TOK tokens per warp; every lane ends with all E logits.
+// `w` may point to shared memory (see stage_router_weights): each 16 bytes of it that a lane reads serve TOK tokens, which
+// is what the kernels are bound by.  Four 16-byte loads of x per token are in flight per lane.  Tokens past the end repeat
+// the first one.
+template <int E_T, int TOK>
+__device__ __forceinline__ void token_logits(const bf16* __restrict__ x, int t0, int step, int tokens, const bf16* w, int hidden, int experts,
+                                             int lane, float (&logit)[TOK][E_T]) {
   const int nv = hidden / 8;
+  const uint4* xr[TOK];
+#pragma unroll
+  for (int u = 0; u < TOK; ++u) {
+    const int t = t0 + u * step < tokens ? t0 + u * step : t0;
+    xr[u] = reinterpret_cast<const uint4*>(x + (long long)t * hidden);
+#pragma unroll
+    for (int e = 0; e < E_T; ++e) logit[u][e] = 0.f;
+  }
+  const uint4* wr = reinterpret_cast<const uint4*>(w);
   for (int i0 = lane; i0 < nv; i0 += 128) {
-    uint4 xv[4];
+    uint4 xv[TOK][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) xv[u] = (i0 + 32 * u < nv) ? xr[i0 + 32 * u] : make_uint4(0, 0, 0, 0);
+    for (int u = 0; u < TOK; ++u)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int i = i0 + 32 * u;
+      for (int v = 0; v < 4; ++v) xv[u][v] = (i0 + 32 * v < nv) ? xr[u][i0 + 32 * v] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int i = i0 + 32 * v;
       if (i < nv) {
-        float xf[8]; unpack8r(xv[u], xf);
+        float xf[TOK][8];
+#pragma unroll
+        for (int u = 0; u < TOK; ++u) unpack8r(xv[u][v], xf[u]);
 #pragma unroll
         for (int e = 0; e < E_T; ++e) {
           if (e < experts) {
             float wf[8]; unpack8r(wr[(long long)e * nv + i], wf);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) logit[e] += xf[j] * wf[j];
+            for (int u = 0; u < TOK; ++u)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) logit[u][e] += xf[u][j] * wf[j];
           }
         }
       }
     }
   }
 #pragma unroll
-  for (int e = 0; e < E_T; ++e) logit[e] = wsum(logit[e]);
+  for (int u = 0; u < TOK; ++u)
+#pragma unroll
+    for (int e = 0; e < E_T; ++e) logit[u][e] = wsum(logit[u][e]);
 }
 
 // Copies the router matrix into shared memory once per CTA when the launch provided room for it.
@@ -116,7 +132,7 @@ __device__ __forceinline__ void softmax_topk(const float (&logit)[E_T], int expe
 // (stats[e] += number of (token, choice) slots routed to e) and the per-expert sums of the softmax scores
 // (stats[experts + e] += sum_t scores[t, e]): the f_e and P_e of the load-balancing loss E * sum_e f_e P_e, and the
 // tokens-per-expert counts, produced in the same pass that routes the tokens.
-template <int E_T>
+template <int E_T, int TOK>
 __global__ void router_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ scores,
                                   bf16* __restrict__ weights, int* __restrict__ idx, int tokens, int hidden, int experts,
                                   int top_k, int normalize, int w_staged, float* __restrict__ stats) {
@@ -131,24 +147,31 @@ __global__ void router_fwd_kernel(const bf16* __restrict__ x, const bf16* __rest
   float cnt[E_T], psum[E_T];
 #pragma unroll
   for (int e = 0; e < E_T; ++e) { cnt[e] = 0.f; psum[e] = 0.f; }
-  for (int t = blockIdx.x * warps_per_block + (threadIdx.x >> 5); t < tokens; t += gridDim.x * warps_per_block) {
-    float logit[E_T], prob[E_T], wsel[MAX_K], denom;
-    int sel[MAX_K];
-    token_logits<E_T>(x + (long long)t * hidden, wp, hidden, experts, lane, logit);
-    softmax_topk<E_T>(logit, experts, top_k, normalize, prob, sel, wsel, denom);
-    if (lane == 0) {
+  const int stride = gridDim.x * warps_per_block;
+  for (int t0 = blockIdx.x * warps_per_block + (threadIdx.x >> 5); t0 < tokens; t0 += stride * TOK) {
+    float logits[TOK][E_T];
+    token_logits<E_T, TOK>(x, t0, stride, tokens, wp, hidden, experts, lane, logits);
 #pragma unroll
-      for (int e = 0; e < E_T; ++e) if (e < experts) scores[(long long)t * experts + e] = __float2bfloat16(prob[e]);
-      for (int c = 0; c < top_k; ++c) {
-        weights[(long long)t * top_k + c] = __float2bfloat16(wsel[c] / denom);
-        idx[(long long)t * top_k + c] = sel[c];
-      }
-      if (stats != nullptr) {
+    for (int u = 0; u < TOK; ++u) {
+      const int t = t0 + u * stride;
+      if (t >= tokens) break;
+      float prob[E_T], wsel[MAX_K], denom;
+      int sel[MAX_K];
+      softmax_topk<E_T>(logits[u], experts, top_k, normalize, prob, sel, wsel, denom);
+      if (lane == 0) {
 #pragma unroll
-        for (int e = 0; e < E_T; ++e) {
-          // the rounded score, so that the sum equals what a reader of `scores` would add up
-          if (e < experts) psum[e] += __bfloat162float(__float2bfloat16(prob[e]));
-          for (int c = 0; c < top_k; ++c) cnt[e] += (sel[c] == e) ? 1.f : 0.f;
+        for (int e = 0; e < E_T; ++e) if (e < experts) scores[(long long)t * experts + e] = __float2bfloat16(prob[e]);
+        for (int c = 0; c < top_k; ++c) {
+          weights[(long long)t * top_k + c] = __float2bfloat16(wsel[c] / denom);
+          idx[(long long)t * top_k + c] = sel[c];
+        }
+        if (stats != nullptr) {
+#pragma unroll
+          for (int e = 0; e < E_T; ++e) {
+            // the rounded score, so that the sum equals what a reader of `scores` would add up
+            if (e < experts) psum[e] += __bfloat162float(__float2bfloat16(prob[e]));
+            for (int c = 0; c < top_k; ++c) cnt[e] += (sel[c] == e) ? 1.f : 0.f;
+          }
         }
       }
     }
@@ -164,90 +187,149 @@ __global__ void router_fwd_kernel(const bf16* __restrict__ x, const bf16* __rest
   }
 }
 
-// Backward through normalise, top-k selection and softmax; writes dlogits (fp32 [tokens, experts]) and
-// dx (+)= dlogits * W.  dW is produced by router_dw_kernel from dlogits.
-template <int E_T>
+// Backward through normalise, top-k selection and softmax; writes dlogits (fp32 [tokens, experts], unless NULL) and
+// dx (+)= dlogits * W.  dW is produced from dlogits by router_dw_kernel.
+template <int E_T, int TOK>
 __global__ void router_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const int* __restrict__ idx,
                                   const bf16* __restrict__ dweights, const bf16* __restrict__ dscores, bf16* __restrict__ dx,
                                   float* __restrict__ dlogits, int tokens, int hidden, int experts, int top_k, int normalize,
                                   int accumulate_dx, int w_staged) {
   const int lane = threadIdx.x & 31;
-  const int warps_per_block = blockDim.x >> 5;
+  const int warps_per_block = blockDim.x >> 5, stride = gridDim.x * warps_per_block;
   const bf16* wp = stage_router_weights(w, experts, hidden, w_staged);
-  for (int t = blockIdx.x * warps_per_block + (threadIdx.x >> 5); t < tokens; t += gridDim.x * warps_per_block) {
-    float logit[E_T], prob[E_T], ds[E_T], wsel[MAX_K], denom;
-    int sel[MAX_K];
-    token_logits<E_T>(x + (long long)t * hidden, wp, hidden, experts, lane, logit);
-    softmax_topk<E_T>(logit, experts, top_k, normalize, prob, sel, wsel, denom);
-    // the forward's selection is authoritative (ties): take the saved indices
-    for (int c = 0; c < top_k; ++c) sel[c] = idx[(long long)t * top_k + c];
-    denom = 0.f;
-    for (int c = 0; c < top_k; ++c) {
-      float pv = 0.f;
+  for (int t0 = blockIdx.x * warps_per_block + (threadIdx.x >> 5); t0 < tokens; t0 += stride * TOK) {
+    float dl[TOK][E_T];
+    token_logits<E_T, TOK>(x, t0, stride, tokens, wp, hidden, experts, lane, dl);
 #pragma unroll
-      for (int e = 0; e < E_T; ++e) if (e == sel[c]) pv = prob[e];
-      wsel[c] = pv; denom += pv;
-    }
-    if (!normalize) denom = 1.f;
+    for (int u = 0; u < TOK; ++u) {
+      const int t = t0 + u * stride < tokens ? t0 + u * stride : t0;
+      float prob[E_T], ds[E_T], wsel[MAX_K], denom;
+      int sel[MAX_K];
+      softmax_topk<E_T>(dl[u], experts, top_k, normalize, prob, sel, wsel, denom);
+      // the forward's selection is authoritative (ties): take the saved indices
+      for (int c = 0; c < top_k; ++c) sel[c] = idx[(long long)t * top_k + c];
+      denom = 0.f;
+      for (int c = 0; c < top_k; ++c) {
+        float pv = 0.f;
 #pragma unroll
-    for (int e = 0; e < E_T; ++e) ds[e] = (dscores != nullptr && e < experts) ? __bfloat162float(dscores[(long long)t * experts + e]) : 0.f;
-    float dot = 0.f;
-    if (normalize)
-      for (int c = 0; c < top_k; ++c) dot += __bfloat162float(dweights[(long long)t * top_k + c]) * wsel[c] / denom;
-    for (int c = 0; c < top_k; ++c) {
-      const float g = (__bfloat162float(dweights[(long long)t * top_k + c]) - dot) / denom;
-#pragma unroll
-      for (int e = 0; e < E_T; ++e) if (e == sel[c]) ds[e] += g;
-    }
-    float sdot = 0.f;
-#pragma unroll
-    for (int e = 0; e < E_T; ++e) sdot += prob[e] * ds[e];
-    float dl[E_T];
-#pragma unroll
-    for (int e = 0; e < E_T; ++e) dl[e] = prob[e] * (ds[e] - sdot);
-    if (lane == 0) {
-#pragma unroll
-      for (int e = 0; e < E_T; ++e) if (e < experts) dlogits[(long long)t * experts + e] = dl[e];
-    }
-    uint4* dxr = reinterpret_cast<uint4*>(dx + (long long)t * hidden);
-    for (int i = lane; i < hidden / 8; i += 32) {
-      float acc[8];
-      if (accumulate_dx) unpack8r(dxr[i], acc);
-      else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+        for (int e = 0; e < E_T; ++e) if (e == sel[c]) pv = prob[e];
+        wsel[c] = pv; denom += pv;
       }
+      if (!normalize) denom = 1.f;
 #pragma unroll
-      for (int e = 0; e < E_T; ++e) {
-        if (e < experts) {
-          float wf[8]; unpack8r(reinterpret_cast<const uint4*>(wp + (long long)e * hidden)[i], wf);
+      for (int e = 0; e < E_T; ++e) ds[e] = (dscores != nullptr && e < experts) ? __bfloat162float(dscores[(long long)t * experts + e]) : 0.f;
+      float dot = 0.f;
+      if (normalize)
+        for (int c = 0; c < top_k; ++c) dot += __bfloat162float(dweights[(long long)t * top_k + c]) * wsel[c] / denom;
+      for (int c = 0; c < top_k; ++c) {
+        const float g = (__bfloat162float(dweights[(long long)t * top_k + c]) - dot) / denom;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] += dl[e] * wf[j];
+        for (int e = 0; e < E_T; ++e) if (e == sel[c]) ds[e] += g;
+      }
+      float sdot = 0.f;
+#pragma unroll
+      for (int e = 0; e < E_T; ++e) sdot += prob[e] * ds[e];
+#pragma unroll
+      for (int e = 0; e < E_T; ++e) dl[u][e] = prob[e] * (ds[e] - sdot);
+      if (lane == 0 && dlogits != nullptr && t0 + u * stride < tokens) {
+#pragma unroll
+        for (int e = 0; e < E_T; ++e) if (e < experts) dlogits[(long long)t * experts + e] = dl[u][e];
+      }
+    }
+    const int nv = hidden / 8;
+    for (int i0 = lane; i0 < nv; i0 += 64) {
+      uint4 old[TOK][2];
+#pragma unroll
+      for (int u = 0; u < TOK; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int t = t0 + u * stride, i = i0 + 32 * v;
+          old[u][v] = accumulate_dx && t < tokens && i < nv ? reinterpret_cast<const uint4*>(dx + (long long)t * hidden)[i] : make_uint4(0, 0, 0, 0);
         }
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const int i = i0 + 32 * v;
+        if (i >= nv) break;
+        float acc[TOK][8];
+#pragma unroll
+        for (int u = 0; u < TOK; ++u) unpack8r(old[u][v], acc[u]);
+#pragma unroll
+        for (int e = 0; e < E_T; ++e) {
+          if (e < experts) {
+            float wf[8]; unpack8r(reinterpret_cast<const uint4*>(wp + (long long)e * hidden)[i], wf);
+#pragma unroll
+            for (int u = 0; u < TOK; ++u)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[u][j] += dl[u][e] * wf[j];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < TOK; ++u)
+          if (t0 + u * stride < tokens) reinterpret_cast<uint4*>(dx + (long long)(t0 + u * stride) * hidden)[i] = pack8r(acc[u]);
       }
-      dxr[i] = pack8r(acc);
     }
   }
 }
 
-// dW[e, col] = sum_t dlogits[t, e] * x[t, col]; one thread per column, tokens split over blockIdx.y
-template <int E_T>
-__global__ void router_dw_kernel(const bf16* __restrict__ x, const float* __restrict__ dlogits, float* __restrict__ dw,
-                                 int tokens, int hidden, int experts) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= hidden) return;
-  float acc[E_T];
+// dW[e, col] = sum_t dlogits[t, e] * x[t, col], tokens split over blockIdx.y.  VEC columns per thread, four rows of x in
+// flight; the dlogits of 32 tokens at a time are staged in shared memory.  Bound by one pass over x (8000 x 4096, 8
+// experts: 188 us with one column per thread and one row in flight).  With more than 16 experts VEC is 1 for want of
+// registers.
+constexpr int DW_TOKENS = 32;
+template <int E_T, int VEC>
+__global__ void __launch_bounds__(256) router_dw_kernel(const bf16* __restrict__ x, const float* __restrict__ dlogits, float* __restrict__ dw,
+                                                        int tokens, int hidden, int experts) {
+  __shared__ float s_dl[DW_TOKENS][E_T];
+  const int col = (blockIdx.x * 256 + threadIdx.x) * VEC;
+  float acc[E_T][VEC];
 #pragma unroll
-  for (int e = 0; e < E_T; ++e) acc[e] = 0.f;
-  const int chunk = (tokens + gridDim.y - 1) / gridDim.y;
-  const int t0 = blockIdx.y * chunk, t1 = min(tokens, t0 + chunk);
-  for (int t = t0; t < t1; ++t) {
-    const float xv = __bfloat162float(x[(long long)t * hidden + col]);
+  for (int e = 0; e < E_T; ++e)
 #pragma unroll
-    for (int e = 0; e < E_T; ++e) if (e < experts) acc[e] += dlogits[(long long)t * experts + e] * xv;
+    for (int j = 0; j < VEC; ++j) acc[e][j] = 0.f;
+  for (int t0 = blockIdx.y * DW_TOKENS; t0 < tokens; t0 += gridDim.y * DW_TOKENS) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < DW_TOKENS * E_T; i += 256) {
+      const int t = t0 + i / E_T, e = i % E_T;
+      s_dl[i / E_T][e] = (t < tokens && e < experts) ? dlogits[(long long)t * experts + e] : 0.f;
+    }
+    __syncthreads();
+    if (col >= hidden) continue;
+    const int n = tokens - t0 < DW_TOKENS ? tokens - t0 : DW_TOKENS;
+    for (int k = 0; k < n; k += 4) {
+      float xf[4][8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const long long at = (long long)(t0 + (k + u < n ? k + u : k)) * hidden + col;     // (past the end: weight zero below)
+        if (VEC == 8) {
+          unpack8r(*reinterpret_cast<const uint4*>(x + at), xf[u]);
+        } else {
+          xf[u][0] = __bfloat162float(x[at]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+#pragma unroll
+        for (int e = 0; e < E_T; ++e) {
+          const float d = k + u < n ? s_dl[k + u][e] : 0.f;
+#pragma unroll
+          for (int j = 0; j < VEC; ++j) acc[e][j] += d * xf[u][j];
+        }
+      }
+    }
   }
+  if (col >= hidden) return;
 #pragma unroll
-  for (int e = 0; e < E_T; ++e) if (e < experts) atomicAdd(dw + (long long)e * hidden + col, acc[e]);
+  for (int e = 0; e < E_T; ++e) {
+    if (e < experts) {
+      float* dst = dw + (long long)e * hidden + col;
+      if (VEC == 8) {
+        red_add_v4_f32(dst, acc[e][0], acc[e][1 % VEC], acc[e][2 % VEC], acc[e][3 % VEC]);
+        red_add_v4_f32(dst + 4, acc[e][4 % VEC], acc[e][5 % VEC], acc[e][6 % VEC], acc[e][7 % VEC]);
+      } else {
+        atomicAdd(dst, acc[e][0]);
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------- counting sort
@@ -403,6 +485,9 @@ static int router_grid(int tokens) {
   const int cap = sm_count_of_current_device() * 3;
   return g < 1 ? 1 : (g > cap ? cap : g);
 }
+// Two tokens per warp and pass once every warp of the grid has two (more experts than 8: no registers for it).  8000 x
+// 4096, 8 experts: forward 81 -> 60 us; a micro-batch of 576 tokens would lose (backward 31 -> 42 us).
+static bool router_pairs(int tokens, int grid) { return tokens >= 2 * grid * 4; }
 // The router matrix is staged in shared memory when it fits (E x H bf16 <= 96 KB); opt in above 48 KB once per kernel.
 static int router_smem_ok(const void* kernel, size_t bytes) {
   if (bytes > 96 * 1024) return 0;
@@ -423,39 +508,39 @@ extern "C" int mdt_router_fwd(const void* x, const void* w, void* scores, void* 
   if (tokens == 0) return 0;
   const int grid = router_grid(tokens);
   const size_t wbytes = (size_t)experts * hidden * 2;
-#define RT_FWD(ET)                                                                                                             \
+#define RT_FWD(ET, TOK)                                                                                                        \
   {                                                                                                                            \
-    const int staged = router_smem_ok((const void*)router_fwd_kernel<ET>, wbytes);                                             \
-    router_fwd_kernel<ET><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, \
+    const int staged = router_smem_ok((const void*)router_fwd_kernel<ET, TOK>, wbytes);                                        \
+    router_fwd_kernel<ET, TOK><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, \
                                                                  idx, tokens, hidden, experts, top_k, normalize, staged, stats); \
   }
-  if (experts <= 8) RT_FWD(8) else if (experts <= 16) RT_FWD(16) else RT_FWD(MAX_E)
+  if (experts <= 8 && router_pairs(tokens, grid)) RT_FWD(8, 2) else if (experts <= 8) RT_FWD(8, 1) else if (experts <= 16) RT_FWD(16, 1) else RT_FWD(MAX_E, 1)
 #undef RT_FWD
   MDT_RT_CHECK();
   return 0;
 }
 
-extern "C" int mdt_router_bwd(const void* x, const void* w, const void* scores, const void* weights, const int* idx,
-                              const void* dweights, const void* dscores, void* dx, float* dw, int tokens, int hidden, int experts,
-                              int top_k, int normalize, int accumulate_dx, cudaStream_t s) {
-  // `dw` must hold experts*hidden floats (accumulated into) followed by tokens*experts floats of scratch.
-  if (hidden % 8 != 0 || experts > MAX_E || top_k > MAX_K) return -1;
+extern "C" int mdt_router_bwd(const void* x, const void* w, const int* idx, const void* dweights, const void* dscores, void* dx, float* dlogits,
+                              float* dw, int tokens, int hidden, int experts, int top_k, int normalize, int accumulate_dx, cudaStream_t s) {
+  if (hidden % 8 != 0 || experts > MAX_E || top_k > MAX_K || (dw != nullptr && dlogits == nullptr)) return -1;
   if (tokens == 0) return 0;
-  float* dlogits = dw + (long long)experts * hidden;
   const int grid = router_grid(tokens);
   const size_t wbytes = (size_t)experts * hidden * 2;
-  dim3 g2((hidden + 127) / 128, 16);
-#define RT_BWD(ET)                                                                                                          \
+  // 64 chunks of tokens at most: every chunk adds its sums into all of dW
+  const int chunks = (tokens + DW_TOKENS - 1) / DW_TOKENS < 64 ? (tokens + DW_TOKENS - 1) / DW_TOKENS : 64;
+#define RT_BWD(ET, VEC, TOK)                                                                                                   \
   {                                                                                                                         \
-    const int staged = router_smem_ok((const void*)router_bwd_kernel<ET>, wbytes);                                          \
-    router_bwd_kernel<ET><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, idx, (const bf16*)dweights,  \
+    const int staged = router_smem_ok((const void*)router_bwd_kernel<ET, TOK>, wbytes);                                     \
+    router_bwd_kernel<ET, TOK><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, idx, (const bf16*)dweights,  \
                                                                  (const bf16*)dscores, (bf16*)dx, dlogits, tokens, hidden,  \
                                                                  experts, top_k, normalize, accumulate_dx, staged);         \
-  }                                                                                                                         \
-  MDT_RT_CHECK();                                                                                                           \
-  router_dw_kernel<ET><<<g2, 128, 0, s>>>((const bf16*)x, dlogits, dw, tokens, hidden, experts);                             \
-  MDT_RT_CHECK();
-  if (experts <= 8) { RT_BWD(8) } else if (experts <= 16) { RT_BWD(16) } else { RT_BWD(MAX_E) }
+    MDT_RT_CHECK();                                                                                                         \
+    if (dw != nullptr) {                                                                                                    \
+      router_dw_kernel<ET, VEC><<<dim3((hidden + 256 * VEC - 1) / (256 * VEC), chunks), 256, 0, s>>>((const bf16*)x, dlogits, dw, tokens, hidden, experts); \
+      MDT_RT_CHECK();                                                                                                       \
+    }                                                                                                                       \
+  }
+  if (experts <= 8 && router_pairs(tokens, grid)) RT_BWD(8, 8, 2) else if (experts <= 8) RT_BWD(8, 8, 1) else if (experts <= 16) RT_BWD(16, 8, 1) else RT_BWD(MAX_E, 1, 1)
 #undef RT_BWD
   return 0;
 }

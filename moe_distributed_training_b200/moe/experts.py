@@ -31,6 +31,24 @@ def features_per_rank(args: MoEArguments) -> int:
     return args.ffn_hidden_size // args.tensor_parallel_size
 
 
+class _GradTargets:
+    """Where the weight-gradient kernels put the gradients of w1, w2, w3: straight into `.grad`.
+
+    A buffer is created when the backward pass asks for it, not cleared in the forward pass: the first gradient is then
+    written instead of added to zeros (three passes over all expert weights less per optimizer step).
+    """
+
+    def __init__(self, params, shape):
+        self.params, self.shape = params, shape
+
+    def target(self, i: int):
+        p = self.params[i]
+        fresh = p.grad is None
+        if fresh:
+            p.grad = torch.empty_like(p)
+        return p.grad.view(self.shape), not fresh
+
+
 class SparseMLPv2(nn.Module):
     def __init__(self, args: MoEArguments):
         super().__init__()
@@ -62,7 +80,7 @@ class SparseMLPv2(nn.Module):
         return {name: (A, B, alpha / r) for name, (A, B, r, alpha, _, _) in self._lora_pointers.items()}
 
     def call_args(self, xg: torch.Tensor):
-        """(w1, w2, w3 views, LoRA dict, weight-gradient scale, direct-accumulation buffers) for one call."""
+        """(w1, w2, w3 views, LoRA dict, weight-gradient scale, where their gradients go) for one call."""
         w1, w2, w3 = self.weight_views()
         wgrad_out = None
         # (only for weights this module owns: when the experts are sharded like dense parameters the
@@ -70,10 +88,7 @@ class SparseMLPv2(nn.Module):
         if (xg.is_cuda and ops.get_backend() == "native" and torch.is_grad_enabled() and self.w1.requires_grad
                 and isinstance(self.w1, nn.Parameter)):
             E, Fr, H = self.experts_per_rank, self.features_per_rank, self.args.hidden_size
-            for w in (self.w1, self.w2, self.w3):
-                if w.grad is None:
-                    w.grad = torch.zeros_like(w)
-            wgrad_out = tuple(w.grad.view(E, Fr, H) for w in (self.w1, self.w2, self.w3))
+            wgrad_out = _GradTargets((self.w1, self.w2, self.w3), (E, Fr, H))
         return w1, w2, w3, self.lora_views(), self.gradient_scale or 1.0, wgrad_out
 
     def forward(self, xg: torch.Tensor, plan) -> torch.Tensor:

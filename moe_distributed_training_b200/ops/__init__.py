@@ -81,7 +81,8 @@ def combine_rows(y, plan: RoutingPlan, weights: Optional[torch.Tensor]):
 def grouped_swiglu_mlp(xg, w1, w2, w3, plan: RoutingPlan, lora=None, wgrad_scale: float = 1.0, wgrad_out=None):
     """Expert MLP over block-padded groups; w1, w2, w3 are [E_local, F, H].
 
-    wgrad_out: optional (dw1, dw2, dw3) buffers the CUDA weight-gradient kernels accumulate into
+    wgrad_out: optional object whose target(i) gives the buffer for the gradient of w1, w2 or w3 and whether the CUDA
+    kernels add to it or write it
     directly (no gradient tensor is returned for the weights then)."""
     if _native(xg):
         return _cuda().grouped_swiglu_mlp(xg, w1, w2, w3, plan, lora, wgrad_scale, wgrad_out)

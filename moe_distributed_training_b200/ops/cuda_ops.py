@@ -48,13 +48,13 @@ def launch_count() -> int:
 
 def _gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G=1, offsets=None, capacity=0, B2=None, A_l=None, a_mn_l=False,
           B_l=None, B2_l=None, b_mn_l=False, K_l=0, C2=None, C3=None, accumulate=False, alpha=1.0, wait=None, scatter=None,
-          residual=None):
-    """wait = (tile_ready, tile_expected): A rows arrive from peers, tile by tile.  scatter = (row_rank, row_pos,
+          residual=None, alpha_dev=None):
+    """alpha_dev: optional fp32 scalar on the GPU that multiplies alpha.  wait = (tile_ready, tile_expected): A rows arrive from peers, tile by tile.  scatter = (row_rank, row_pos,
     peer_out table, peer_arrive table): result rows are stored into peers' buffers instead of C."""
     w0, w1 = wait if wait is not None else (None, None)
     s0, s1, s2, s3 = scatter if scatter is not None else (None, None, None, None)
     ext.gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G, offsets, capacity, B2, A_l, a_mn_l, B_l, B2_l, b_mn_l, K_l,
-             C2, C3, accumulate, alpha, status_tensor(A.device), w0, w1, s0, s1, s2, s3, residual)
+             C2, C3, accumulate, alpha, status_tensor(A.device), w0, w1, s0, s1, s2, s3, residual, alpha_dev)
     return C
 
 
@@ -69,31 +69,30 @@ def mm_nt(x, w, out=None, alpha=1.0, lora=None, residual=None):
     return _gemm(0, x, False, w, False, out, M, N, K, A_l=t, B_l=b, b_mn_l=False, K_l=t.shape[1], alpha=alpha, residual=residual)
 
 
-def mm_nn(x, w, out=None, alpha=1.0, accumulate=False, lora=None):
+def mm_nn(x, w, out=None, alpha=1.0, accumulate=False, lora=None, alpha_dev=None):
     """x [M,K] @ w[K,N] (w row-major, N contiguous)."""
     M, K = x.shape
     N = w.shape[1]
     out = out if out is not None else torch.empty(M, N, dtype=x.dtype, device=x.device)
     if lora is None:
-        return _gemm(0, x, False, w, True, out, M, N, K, alpha=alpha, accumulate=accumulate)
+        return _gemm(0, x, False, w, True, out, M, N, K, alpha=alpha, accumulate=accumulate, alpha_dev=alpha_dev)
     t, b = lora  # t [M,r], b [r,N]
     return _gemm(0, x, False, w, True, out, M, N, K, A_l=t, B_l=b, b_mn_l=True, K_l=t.shape[1], alpha=alpha,
-                 accumulate=accumulate)
+                 accumulate=accumulate, alpha_dev=alpha_dev)
 
 
-def mm_tn(a, b, out=None, alpha=1.0, accumulate=False, out_dtype=None):
+def mm_tn(a, b, out=None, alpha=1.0, accumulate=False, out_dtype=None, alpha_dev=None):
     """a[R,M]^T @ b[R,N] -> [M,N] (reduction over rows)."""
     R, M = a.shape
     N = b.shape[1]
     out = out if out is not None else torch.empty(M, N, dtype=out_dtype or a.dtype, device=a.device)
-    return _gemm(2, a, True, b, True, out, M, N, R, alpha=alpha, accumulate=accumulate)
+    return _gemm(2, a, True, b, True, out, M, N, R, alpha=alpha, accumulate=accumulate, alpha_dev=alpha_dev)
 
 
 # ----------------------------------------------------------------------------------------------- dense linear
 def _skinny(x, A, a_is_kr, alpha):
-    """x A^T (A [r, K]) or x A (A [K, r]) for a LoRA rank r: CUDA-core kernel for r <= 32, else the GEMM."""
-    r = A.shape[1] if a_is_kr else A.shape[0]
-    if r <= 32 and x.shape[1] % 8 == 0 and A.is_contiguous() and x.dtype == torch.bfloat16 and A.dtype == torch.bfloat16:
+    """x A^T (A [r, K]) or x A (A [K, r]) for a LoRA rank r: CUDA-core kernel for r <= 32 and few rows, else the GEMM."""
+    if ext.skinny_preferred(x, A, a_is_kr):
         return ext.skinny_mm(x, A, a_is_kr, float(alpha))
     return mm_nn(x, A, alpha=alpha) if a_is_kr else mm_nt(x, A, alpha=alpha)
 
@@ -160,8 +159,9 @@ class _Router(torch.autograd.Function):
         x, w, idx = ctx.saved_tensors
         if dweights is None:
             dweights = torch.zeros(idx.shape, dtype=x.dtype, device=x.device)
-        dx, dw = ext.router_bwd(x.contiguous(), w.contiguous(), idx, dweights.to(x.dtype), dscores, ctx.normalize)
-        return dx, dw.to(w.dtype), None, None, None
+        need_dw = ctx.needs_input_grad[1]
+        dx, dw = ext.router_bwd(x.contiguous(), w.contiguous(), idx, dweights.to(x.dtype), dscores, ctx.normalize, None, need_dw)
+        return dx, dw.to(w.dtype) if need_dw else None, None, None, None
 
 
 def router(x, w_router, top_k, normalize=True, with_stats=False):
@@ -312,7 +312,7 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
         need_w = ctx.needs_input_grad[1] or ctx.needs_input_grad[2] or ctx.needs_input_grad[3]
         if need_w:
             if wg is not None:
-                _g(2, h, True, dy, True, wg[1], H, 0, plan, alpha=ws, accumulate=True)
+                out, add = wg.target(1); _g(2, h, True, dy, True, out, H, 0, plan, alpha=ws, accumulate=add)
             else:
                 dw2 = torch.empty_like(w2)
                 _g(2, h, True, dy, True, dw2, H, 0, plan, alpha=ws)
@@ -328,8 +328,8 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
         _g(1, dg, False, w1, True, dx, H, F, plan, A_l=du, B_l=w3, b_mn_l=True, K_l=F, scatter=scatter)   # dg W1 + du W3
         if need_w:
             if wg is not None:
-                _g(2, dg, True, xg, True, wg[0], H, 0, plan, alpha=ws, accumulate=True)
-                _g(2, du, True, xg, True, wg[2], H, 0, plan, alpha=ws, accumulate=True)
+                out, add = wg.target(0); _g(2, dg, True, xg, True, out, H, 0, plan, alpha=ws, accumulate=add)
+                out, add = wg.target(2); _g(2, du, True, xg, True, out, H, 0, plan, alpha=ws, accumulate=add)
             else:
                 dw1 = torch.empty_like(w1); _g(2, dg, True, xg, True, dw1, H, 0, plan, alpha=ws)
                 dw3 = torch.empty_like(w3); _g(2, du, True, xg, True, dw3, H, 0, plan, alpha=ws)
@@ -428,8 +428,9 @@ class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w, rstd = ctx.saved_tensors
-        dx, dwp = ext.rmsnorm_bwd(x, w, dy.contiguous(), rstd)
-        return dx, ext.rmsnorm_dw(dwp, w), None
+        need_dw = ctx.needs_input_grad[1]
+        dx, dwp = ext.rmsnorm_bwd(x, w, dy.contiguous(), rstd, None, need_dw)
+        return dx, ext.rmsnorm_dw(dwp, w) if need_dw else None, None
 
 
 def rmsnorm(x, weight, eps):
@@ -495,10 +496,11 @@ class _LinearCrossEntropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss_sum, _dn):
         hidden, w_head, dlogits, n = ctx.saved_tensors
-        # the kernel wrote d(mean loss)/dlogits; convert to d(loss_sum) and apply the incoming gradient
-        dlogits.mul_((dloss_sum * n.clamp(min=1.0)).to(dlogits.dtype))
-        dh = mm_nn(dlogits, w_head) if ctx.needs_input_grad[0] else None
-        dw = mm_tn(dlogits, hidden) if ctx.needs_input_grad[1] else None
+        # the kernel wrote d(mean loss)/dlogits; the factor that makes it d(loss_sum) times the incoming gradient goes into
+        # the products' epilogues (a pass over 8192 x 32000 logits for it took 550 us)
+        factor = (dloss_sum * n.clamp(min=1.0)).float()
+        dh = mm_nn(dlogits, w_head, alpha_dev=factor) if ctx.needs_input_grad[0] else None
+        dw = mm_tn(dlogits, hidden, alpha_dev=factor) if ctx.needs_input_grad[1] else None
         return dh, dw, None, None
 
 
@@ -512,4 +514,6 @@ def attention(q, k, v, cu_seqlens, max_seqlen=None):
 
 
 def adamw_multi(ps, gs, ms, vs, lr, b1, b2, eps, wd, step, grad_scale=1.0):
-    ext.adamw(list(ps), list(gs), list(ms), list(vs), lr, b1, b2, eps, wd, int(step), float(grad_scale))
+    """grad_scale: a number, or an fp32 scalar on the GPU (then nothing waits for its value)."""
+    dev = grad_scale if torch.is_tensor(grad_scale) else None
+    ext.adamw(list(ps), list(gs), list(ms), list(vs), lr, b1, b2, eps, wd, int(step), 1.0 if dev is not None else float(grad_scale), dev)

@@ -129,7 +129,7 @@ class _AttentionBlock(torch.autograd.Function):
         d_xn = run(0, dq, xn, tq)
         run(1, dk, xn, tk, dx_out=d_xn, accumulate=True)
         run(2, dv.view(T, Hkv * d), xn, tv, dx_out=d_xn, accumulate=True)
-        dx, dwp = ext.rmsnorm_bwd(x2, ln_w, d_xn, rstd, dy2)   # + dy: the residual connection's gradient
+        dx, dwp = ext.rmsnorm_bwd(x2, ln_w, d_xn, rstd, dy2, need[2])   # + dy: the residual connection's gradient
         if need[2]:
             grads[0] = ext.rmsnorm_dw(dwp, ln_w)
         return (dx, None) + tuple(grads)
@@ -283,8 +283,8 @@ class _MoEBlock(torch.autograd.Function):
             ext.gemm_rows_hint(0)
             dxn = ext.combine_rows(back, plan.dest_row, None, k)
         dxn = dxn.contiguous()
-        _, dWr = ext.router_bwd(xn, Wr.contiguous(), idx, dwts, None, True, dxn)     # adds the router's input gradient to dxn
-        dx, dwp = ext.rmsnorm_bwd(x2, ln_w, dxn, rstd, dy2)                          # + dy: the residual connection's gradient
+        _, dWr = ext.router_bwd(xn, Wr.contiguous(), idx, dwts, None, True, dxn, need[3])     # adds the router's input gradient to dxn
+        dx, dwp = ext.rmsnorm_bwd(x2, ln_w, dxn, rstd, dy2, need[2])                 # + dy: the residual connection's gradient
         grads = [None] * ctx.n_params
         if need[2]:
             grads[0] = ext.rmsnorm_dw(dwp, ln_w)
@@ -361,9 +361,10 @@ class _MoEBlockNative(torch.autograd.Function):
         layout, ints, tens = [], [], []
         if eng is not None:
             layout, ints, tens = _MoEBlockNative._ep_args(eng, eng.next_phase(), x2.shape[1])
-        wg = list(ctx.wgrad_out) if ctx.wgrad_out is not None else []
+        targets = [ctx.wgrad_out.target(i) for i in range(3)] if ctx.wgrad_out is not None else []
         need = ctx.needs_input_grad
-        dx, dln, dWr = ext.moe_block_bwd(dy, state, x2, ln_w, Wr.contiguous(), w1, w2, w3, wg, ctx.ws, a.moe_top_k, a.moe_num_experts,
+        dx, dln, dWr = ext.moe_block_bwd(dy, state, x2, ln_w, Wr.contiguous(), w1, w2, w3, [t for t, _ in targets], [add for _, add in targets],
+                                         ctx.ws, a.moe_top_k, a.moe_num_experts,
                                          layout, ints, tens, C.status_tensor(dy.device), bool(need[2]), bool(need[3]))
         return dx, None, (dln if need[2] else None), (dWr if need[3] else None), None, None, None
 

@@ -42,7 +42,10 @@ def clip_grad_norm_(model, max_norm: float, shard_group=None, ep_group=None, opt
     norm = global_grad_norm(model, shard_group, ep_group)
     coef = (max_norm / (norm + 1e-6)).clamp(max=1.0)
     if optimizer is not None and hasattr(optimizer, "grad_scale"):
-        optimizer.grad_scale = float(coef)  # one host read per optimizer step
+        from .. import ops
+        # On the GPU the factor stays there: reading it back would let the queue run dry once per optimizer step.
+        on_gpu = coef.is_cuda and ops.get_backend() == "native"
+        optimizer.grad_scale = coef if on_gpu else float(coef)
     else:
         for p in model.parameters():
             if p.grad is not None:

@@ -239,6 +239,113 @@ def test_gemm_epilogue_edges(ops, M, N, K, policy):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (77, 1024, 4096), (300, 520, 2056), (129, 64, 8192), (1000, 16, 4096), (33, 128, 1024)])
+def test_gemm_few_tiles_shared_by_a_cluster(ops, M, N, K):
+    """Products with few output tiles under the default policy (the depth is cut over a cluster): K-major and MN-major
+    weights, adapter segment with residual, accumulation, fp32 results, a device scalar as factor, weight gradients; twice,
+    bit for bit the same.  fp32 sums, one bf16 rounding of each result."""
+    torch.manual_seed(K + M)
+    x, w, w2 = _rand(M, K), _rand(N, K, scale=0.05), _rand(K, N, scale=0.05)
+    t, b, res, old = _rand(M, 16), _rand(N, 16, scale=0.1), _rand(M, N), _rand(M, N)
+    want = x.float() @ w.float().t()
+    f = torch.tensor(0.25, device=DEV)
+
+    def run():
+        acc = old.clone()
+        ops._gemm(0, x, False, w, False, acc, M, N, K, accumulate=True, alpha=0.5)
+        acc32 = old.float()
+        ops._gemm(0, x, False, w2, True, acc32, M, N, K, accumulate=True, alpha_dev=f)
+        g = torch.empty(N, K, dtype=torch.bfloat16, device=DEV)
+        ops.mm_tn(res, x, out=g)
+        narrow = torch.empty(K, 16, dtype=torch.bfloat16, device=DEV)       # depth M
+        ops.mm_tn(x, t, out=narrow, alpha_dev=f)
+        return [ops.mm_nt(x, w), ops.mm_nt(x, w, lora=(t, b), residual=res), ops.mm_nn(x, w2), acc, acc32, g, narrow]
+    got, again = run(), run()
+    refs = [want, want + t.float() @ b.float().t() + res.float(), x.float() @ w2.float(), old.float() + 0.5 * want,
+            old.float() + 0.25 * (x.float() @ w2.float()), res.float().t() @ x.float(), 0.25 * (x.float().t() @ t.float())]
+    for i, (a, r, c) in enumerate(zip(got, refs, again)):
+        _close(a, r, name=f"product {i}")
+        assert torch.equal(a, c), f"product {i} differs between two runs"
+    ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("T,E,r,F", [(40, 4, 16, 2048), (700, 8, 32, 4096), (3, 2, 8, 1024)])
+def test_grouped_adapter_products_shared_by_a_cluster(ops, T, E, r, F):
+    """Row-grouped and depth-grouped products with a rank-wide side, some experts without rows, against fp32."""
+    torch.manual_seed(T)
+    top = (torch.arange(T, device=DEV) % max(E - 1, 1)).int()[:, None]
+    plan = ops.make_plan(top, E)
+    offs, R = plan.padded_offsets.tolist(), plan.src_slot.numel()
+    xg = ops.ext.gather_rows(_rand(T, F), plan.src_slot, plan.padded_offsets, E, None, 1)
+    A, B = _rand(E, F, r, scale=0.05), _rand(E, r, F, scale=0.05)
+    t, u = (torch.empty(R, r, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops._g(1, xg, False, A, True, t, r, F, plan, alpha=2.0)
+    ops._g(1, xg, False, B, False, u, r, F, plan)
+    dA, dB = torch.full_like(A, 7.0), torch.full_like(B, 7.0)
+    ops._g(2, xg, True, t, True, dA, r, 0, plan)
+    ops._g(2, t, True, xg, True, dB, F, 0, plan)
+    for e in range(E):
+        a, b = offs[e], offs[e + 1]
+        if b > a:
+            _close(t[a:b], 2.0 * xg[a:b].float() @ A[e].float(), name=f"x A, expert {e}")
+            _close(u[a:b], xg[a:b].float() @ B[e].float().t(), name=f"dy B, expert {e}")
+        _close(dA[e], xg[a:b].float().t() @ t[a:b].float(), name=f"dA {e}")
+        _close(dB[e], t[a:b].float().t() @ xg[a:b].float(), name=f"dB {e}")
+    ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("T,H,E", [(1, 64, 4), (33, 4096, 8), (450, 1032, 8), (97, 256, 16), (70, 512, 40)])
+def test_router_backward_odd_sizes(ops, T, H, E):
+    """Token pairs of a warp, token chunks and column blocks that do not divide, and frozen weights, against fp64."""
+    torch.manual_seed(T + E)
+    x, w = _rand(T, H), _rand(E, H, scale=0.05)
+    k = 2
+    scores, wts, idx = ops.ext.router_fwd(x, w, k, True)
+    x64, w64 = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    p = (x64 @ w64.t()).softmax(-1)
+    sel = p.gather(1, idx.long())
+    gw = sel / sel.sum(1, keepdim=True)
+    _close(wts, gw, 1e-2, name="weights")
+    d = _rand(T, k)
+    rx, rw = torch.autograd.grad(gw, (x64, w64), d.double())
+    dx, dw = ops.ext.router_bwd(x, w, idx, d, None, True)
+    _close(dx, rx, 2e-2, name="dx")
+    assert _rel_err(dw, rw) < 1e-3, _rel_err(dw, rw)
+    base = _rand(T, H)
+    acc = base.clone()
+    _, none = ops.ext.router_bwd(x, w, idx, d, None, True, acc, False)
+    assert none.numel() == 0
+    _close(acc, base.float() + dx.float(), name="dx accumulate")
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 64), (700, 4096), (301, 2056), (40, 8192), (9, 16384)])
+def test_rmsnorm_backward_widths(ops, rows, cols):
+    torch.manual_seed(cols)
+    x, w, dy, dres = _rand(rows, cols), _rand(cols), _rand(rows, cols), _rand(rows, cols)
+    y, rstd = ops.ext.rmsnorm_fwd(x, w, 1e-5)
+    x64, w64 = x.double().requires_grad_(True), w.double().requires_grad_(True)
+    ref = x64 * (x64.square().mean(1, keepdim=True) + 1e-5).rsqrt() * w64
+    rx, rw = torch.autograd.grad(ref, (x64, w64), dy.double())
+    dx, part = ops.ext.rmsnorm_bwd(x, w, dy, rstd, dres)
+    _close(dx, rx + dres.double(), 1e-2, name="dx")
+    _close(ops.ext.rmsnorm_dw(part, w)[None], rw[None], 1e-2, name="dw")
+    dx2, part = ops.ext.rmsnorm_bwd(x, w, dy, rstd, dres, False)
+    assert part.numel() == 0 and torch.equal(dx, dx2)
+
+
+@pytest.mark.parametrize("heads,d", [(1, 16), (3, 24), (5, 64), (32, 128), (8, 256)])
+def test_rope_head_sizes(ops, heads, d):
+    T = 37
+    x = _rand(T, heads, d)
+    pos = torch.randint(0, 9000, (T,), device=DEV, dtype=torch.int32)
+    ang = pos.double()[:, None] * 1e6 ** (-2.0 * torch.arange(d // 2, device=DEV).double() / d)
+    c, s = ang.cos()[:, None], ang.sin()[:, None]
+    a, b = x.double().split(d // 2, -1)
+    # fp32 angles of up to 9000 rad: 9000 * 2^-24 = 5e-4; bf16 results
+    _close(ops.ext.rope(x, pos, 1e6, False).flatten(1), torch.cat([a * c - b * s, b * c + a * s], -1).flatten(1), 1e-2, name="rope")
+    _close(ops.ext.rope(ops.ext.rope(x, pos, 1e6, False), pos, 1e6, True).flatten(1), x.float().flatten(1), 1e-2, name="rope and back")
+
+
 @pytest.mark.parametrize("policy", [2, 4], ids=["pair", "tall"])
 @pytest.mark.parametrize("T,E,H,F,lora", [(600, 4, 256, 512, True), (1500, 8, 1024, 2048, False), (333, 3, 512, 1024, False)])
 def test_grouped_mlp_pair_kernel_matches_single_cta_kernel(ops, T, E, H, F, lora, policy):
