@@ -554,7 +554,30 @@ class ShardedMixtral:
         if g is None:
             return
         scale = 1.0 / (self.ws * self.rep)
-        if self.sync_each_batch or self.ws == 1:
+        if self.ws == 1:
+            # nothing to reduce: straight into the gradient of the flat parameter, written the first time
+            fresh = g.shard.grad is None
+            if fresh:
+                g.shard.grad = torch.empty_like(g.shard.data)
+            flat, dst, src, end = g.shard.grad, [], [], 0
+            for (mod, name, shape, n, o), gr in zip(g.specs, grads):
+                if fresh and end < o:
+                    flat[end:o].zero_()                                      # alignment gaps
+                end = o + n
+                if gr is not None:
+                    dst.append(flat[o:end].view(shape)); src.append(gr if gr.dtype == flat.dtype else gr.to(flat.dtype))
+                elif fresh:
+                    flat[o:end].zero_()
+            if fresh and end < flat.numel():
+                flat[end:].zero_()
+            if dst:
+                if fresh:
+                    torch._foreach_copy_(dst, src)
+                    if scale != 1.0:
+                        flat.mul_(scale)
+                else:
+                    torch._foreach_add_(dst, src, alpha=scale)
+        elif self.sync_each_batch:
             # double-buffered flat gradient: the reduction of one block runs on the side stream while the next block's
             # backward fills the other buffer
             key = (g.padded, g.dtype)
