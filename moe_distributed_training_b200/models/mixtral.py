@@ -159,7 +159,7 @@ def shift_labels(labels: torch.Tensor, cu_seqlens: torch.Tensor, ignore_index: i
     out = torch.full_like(labels, ignore_index)
     out[:-1] = labels[1:]
     ends = (cu_seqlens[1:] - 1).long()
-    out[ends] = ignore_index
+    out.index_fill_(0, ends, ignore_index)       # (assigning a number through an index copies it from the host and waits)
     return out
 
 
