@@ -8,6 +8,8 @@ for it (parallel_linear_lora.py:136-138) — to the base expert weight when it r
 """
 from __future__ import annotations
 
+import dataclasses
+
 import torch
 
 from moe_distributed_training_b200 import ops
@@ -22,8 +24,22 @@ def parallel_linear_lora(inputs, expert_weights, expert_lora_A, expert_lora_B, l
     [T,k] is given (gate-weighted sum over the k choices of a token).
     """
     E = expert_weights.shape[0]
-    plan = ops.make_plan(sorted_expert_idxs.int()[:, None].contiguous(), E)
     idx = sorted_scattered_idxs.long()
+    if (not grouped_in and not grouped_out and inputs.dim() == 2 and idx.numel() == inputs.shape[0] * k
+            and (gates is None or tuple(gates.shape) == (inputs.shape[0], k))):
+        # Rows by slot on both sides: the experts of the slots, in slot order, give a plan whose gather reads the tokens
+        # and whose combine writes the slots (or adds a token's gate-weighted choices up), so that nothing has to be
+        # permuted before or after (3001 tokens, 14336 -> 4096, forward and backward: 1.1 ms of copies less).
+        slot_experts = torch.zeros_like(idx, dtype=torch.int32).index_copy(0, idx, sorted_expert_idxs.reshape(-1).int())
+        plan = ops.make_plan(slot_experts.view(-1, k), E)
+        lora = None
+        if expert_lora_A is not None:
+            lora = (expert_lora_A, expert_lora_B, float(lora_alp) / float(lora_r) if lora_r else float(lora_alp))
+        yg = ops.grouped_linear(ops.gather_rows(inputs, plan), expert_weights, plan, trans_b=False, lora=lora)
+        if gates is not None:
+            return ops.combine_rows(yg, plan, gates.to(yg.dtype))
+        return ops.combine_rows(yg, dataclasses.replace(plan, top_k=1), None)
+    plan = ops.make_plan(sorted_expert_idxs.int()[:, None].contiguous(), E)
     xs = inputs if grouped_in else inputs.index_select(0, torch.div(idx, k, rounding_mode="floor"))
     xg = ops.gather_rows(xs, plan)
     lora = None

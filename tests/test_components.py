@@ -194,6 +194,36 @@ def test_text_dataset_masks_the_prompt_with_a_local_tokenizer(tmp_path):
     assert labels[-3:] == [9, 10, 11] and all(v == -100 for v in labels[:-3])
 
 
+@pytest.mark.parametrize("k,gated,idx_dtype", [(1, False, torch.int64), (2, False, torch.int32), (2, True, torch.int64), (3, True, torch.int32)])
+def test_parallel_linear_lora_slot_order_equals_the_sorted_path(k, gated, idx_dtype):
+    """Slot-ordered calls build their plan from the slots themselves; the sorted path (`grouped_out`) with the permutation
+    and the gates applied outside is the general form.  Experts without rows, ids given as a strided view."""
+    from scattermoe_utils.parallel_linear_lora import parallel_linear_lora
+    torch.manual_seed(5 + k)
+    T, K, N, E, r = 37, 24, 16, 5, 4
+    experts = torch.randint(0, E - 1, (T, k))                      # the last expert gets nothing
+    ids, order = torch.sort(experts.reshape(-1), stable=True)
+    ids = torch.stack([ids, ids], 1).to(idx_dtype)[:, 0]
+    order = order.to(idx_dtype)
+    base = dict(x=torch.randn(T, K), W=torch.randn(E, K, N) * 0.3, A=torch.randn(E, K, r) * 0.3, B=torch.randn(E, r, N) * 0.3,
+                g=torch.rand(T, k) if gated else None)
+
+    def run(sorted_path):
+        v = {n: t.clone().requires_grad_(True) if t is not None else None for n, t in base.items()}
+        if sorted_path:
+            ys = parallel_linear_lora(v["x"], v["W"], v["A"], v["B"], r, 8.0, k, ids, order, grouped_out=True)
+            y = torch.zeros_like(ys).index_copy(0, order.long(), ys)
+            if gated:
+                y = (y.view(T, k, N) * v["g"][..., None]).sum(1)
+        else:
+            y = parallel_linear_lora(v["x"], v["W"], v["A"], v["B"], r, 8.0, k, ids, order, gates=v["g"])
+        (y * torch.linspace(-1, 1, y.numel()).view_as(y)).sum().backward()
+        return [y] + [t.grad for t in v.values() if t is not None]
+    for a, b in zip(run(False), run(True)):
+        assert a.shape == b.shape
+        torch.testing.assert_close(a, b, rtol=2e-5, atol=2e-5)
+
+
 def test_gemm_tiling_choice_without_a_gpu():
     """The host-side rule that picks between the 128-row, CTA-pair and tall GEMM tilings (pure arithmetic)."""
     build = pytest.importorskip("moe_distributed_training_b200.ops.build")
