@@ -36,6 +36,9 @@ typedef struct MdtGemmDesc {
   // output
   void* C; void* C2; void* C3;   // dual mode: C = h, optional C2 = gate, C3 = up (all bf16)
   const void* R;                 // optional (mode 0/1, not dual): bf16 matrix laid out like C, added to the result (residual connection)
+  // optional (mode 1, with g and u bf16 laid out like C): the product is the gradient dh of h = silu(g) * u, and the
+  // epilogue writes dg to C and du to C2 instead of dh
+  const void* swiglu_g; const void* swiglu_u;
   long long ldc, c_group_stride;
   int c_fp32;          // C is fp32 instead of bf16
   int accumulate;      // C += alpha * (A*B) instead of C = alpha * (A*B)
@@ -93,9 +96,6 @@ int mdt_rope(const void* x, void* y, const int* positions, int tokens, int heads
              int inverse, cudaStream_t s);
 // dst[0 : rows_used[0]] = src[0 : rows_used[0]] for row buffers of `cols` bf16 elements sized for a capacity (n elements)
 int mdt_copy_rows_used(const void* src, void* dst, long long n, const int* rows_used, long long cols, cudaStream_t s);
-// rows_used (optional, device): number of leading rows of `cols` elements that hold data; the rest is left untouched
-int mdt_swiglu_bwd(const void* g, const void* u, const void* dh, void* dg, void* du, long long n,
-                   const int* rows_used, long long cols, cudaStream_t s);
 int mdt_swiglu_fwd(const void* g, const void* u, void* h, long long n, cudaStream_t s);
 int mdt_embedding(const void* table, const long long* ids, void* out, int tokens, int cols, cudaStream_t s);
 int mdt_embedding_bwd(const void* dout, const long long* ids, float* dtable, int tokens, int cols, cudaStream_t s);

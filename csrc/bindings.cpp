@@ -86,7 +86,8 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
           bool a_mn_l, const OptTensor& B_l, const OptTensor& B2_l, bool b_mn_l, int64_t K_l, const OptTensor& C2,
           const OptTensor& C3, bool accumulate, double alpha, const OptTensor& status, const OptTensor& tile_ready,
           const OptTensor& tile_expected, const OptTensor& row_dest_rank, const OptTensor& row_dest_row, const OptTensor& peer_out,
-          const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt, const OptTensor& alpha_dev = std::nullopt) {
+          const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt, const OptTensor& alpha_dev = std::nullopt,
+          const OptTensor& swiglu_g = std::nullopt, const OptTensor& swiglu_u = std::nullopt) {
   CHECK_BF16(A); CHECK_BF16(B);
   c10::cuda::CUDAGuard guard(A.device());
   MdtGemmDesc d;
@@ -113,6 +114,12 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
   d.c_fp32 = C.scalar_type() == at::kFloat;
   TORCH_CHECK(d.c_fp32 || C.scalar_type() == at::kBFloat16, "C must be bf16 or fp32");
   d.accumulate = accumulate; d.alpha = (float)alpha;
+  if (swiglu_g.has_value()) {
+    for (const OptTensor* t : {&swiglu_g, &swiglu_u, &C2})
+      TORCH_CHECK(t->has_value() && (*t)->scalar_type() == at::kBFloat16 && (*t)->sizes() == C.sizes() && (*t)->strides() == C.strides(),
+                  "the SwiGLU backward needs g, u and C2 laid out like C");
+    d.swiglu_g = swiglu_g->data_ptr(); d.swiglu_u = swiglu_u->data_ptr();
+  }
   if (alpha_dev.has_value()) {
     TORCH_CHECK(alpha_dev->is_cuda() && alpha_dev->scalar_type() == at::kFloat && alpha_dev->numel() == 1, "alpha_dev must be a CUDA fp32 scalar");
     TORCH_CHECK(!d.dual, "alpha has no place in the SwiGLU form");
@@ -194,19 +201,6 @@ Tensor swiglu_fwd(const Tensor& g, const Tensor& u) {
   auto h = torch::empty_like(g);
   check(mdt_swiglu_fwd(g.data_ptr(), u.data_ptr(), h.data_ptr(), g.numel(), cur_stream()), "swiglu_fwd");
   return h;
-}
-// `offsets` (optional, int32 [G+1]): row-group offsets of block-padded buffers; rows past offsets[G] are not touched
-std::vector<Tensor> swiglu_bwd(const Tensor& g, const Tensor& u, const Tensor& dh, const OptTensor& offsets) {
-  c10::cuda::CUDAGuard guard(g.device());
-  auto dg = torch::empty_like(g), du = torch::empty_like(u);
-  const int* rows_used = nullptr;
-  if (offsets.has_value() && offsets->defined()) {
-    TORCH_CHECK(offsets->scalar_type() == at::kInt && offsets->is_contiguous() && g.dim() == 2);
-    rows_used = offsets->data_ptr<int>() + (offsets->numel() - 1);
-  }
-  check(mdt_swiglu_bwd(g.data_ptr(), u.data_ptr(), dh.data_ptr(), dg.data_ptr(), du.data_ptr(), g.numel(), rows_used,
-                       g.size(-1), cur_stream()), "swiglu_bwd");
-  return {dg, du};
 }
 // Copy of a block-padded row buffer sized for a capacity: only rows below offsets[G] are copied (the rest of the
 // result is uninitialised and, like the source's, never read).
@@ -875,16 +869,16 @@ std::vector<Tensor> moe_block_bwd(const Tensor& dy, const std::vector<Tensor>& s
     w0 = ep[3]; w1o = te; s0 = rr; s1 = rp; s2 = ep[1]; s3 = ep[2];
   }
   const int64_t R = dyg.size(0);
-  Tensor dh = torch::empty({R, F}, x.options());
-  ggemm(1, dyg, false, w2, false, dh, R, F, H, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, false, 1.0, status, w0, w1o, NONE, NONE, NONE, NONE);
+  Tensor dg = torch::empty({R, F}, x.options()), du = torch::empty({R, F}, x.options());
+  gemm(1, dyg, false, w2, false, dg, R, F, H, El, offs, cap, NONE, NONE, false, NONE, NONE, false, 0, du, NONE, false, 1.0, status, w0, w1o, NONE, NONE, NONE,
+       NONE, NONE, NONE, g, u);                                 // dh = dy W2^T, through SwiGLU in the epilogue
   if (!wg.empty()) { Tensor c = wg[1]; ggemm(2, h, true, dyg, true, c, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[1], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE); }
-  auto gu = swiglu_bwd(g, u, dh, offs);
   Tensor dxg = torch::empty({R, H}, x.options());
-  ggemm(1, gu[0], false, w1, true, dxg, R, H, F, El, offs, cap, NONE, gu[1], w3, true, F, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3);
+  ggemm(1, dg, false, w1, true, dxg, R, H, F, El, offs, cap, NONE, du, w3, true, F, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3);
   if (!wg.empty()) {
     Tensor c1 = wg[0], c3 = wg[2];
-    ggemm(2, gu[0], true, xg, true, c1, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[0], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
-    ggemm(2, gu[1], true, xg, true, c3, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[2], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
+    ggemm(2, dg, true, xg, true, c1, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[0], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
+    ggemm(2, du, true, xg, true, c3, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[2], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
   }
   Tensor back;
   if (!is_ep) {
@@ -906,13 +900,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("G"), py::arg("offsets"), py::arg("capacity_rows"), py::arg("B2"), py::arg("A_l"), py::arg("a_mn_l"), py::arg("B_l"), py::arg("B2_l"),
         py::arg("b_mn_l"), py::arg("K_l"), py::arg("C2"), py::arg("C3"), py::arg("accumulate"), py::arg("alpha"), py::arg("status"), py::arg("tile_ready"),
         py::arg("tile_expected"), py::arg("row_dest_rank"), py::arg("row_dest_row"), py::arg("peer_out"), py::arg("peer_arrive"),
-        py::arg("residual") = py::none(), py::arg("alpha_dev") = py::none());
+        py::arg("residual") = py::none(), py::arg("alpha_dev") = py::none(), py::arg("swiglu_g") = py::none(), py::arg("swiglu_u") = py::none());
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("x"), py::arg("w"), py::arg("dy"), py::arg("rstd"), py::arg("dres") = py::none(), py::arg("need_dw") = true);
   m.def("rmsnorm_dw", &rmsnorm_dw);
   m.def("rope", &rope);
   m.def("swiglu_fwd", &swiglu_fwd);
-  m.def("swiglu_bwd", &swiglu_bwd, py::arg("g"), py::arg("u"), py::arg("dh"), py::arg("offsets") = py::none());
   m.def("embedding", &embedding);
   m.def("embedding_bwd", &embedding_bwd);
   m.def("cross_entropy", &cross_entropy);

@@ -49,6 +49,7 @@ struct GemmParams {
   int a_mn, b_mn, a_mn_l, b_mn_l, dual;
   const int* offsets;
   void* C; void* C2; void* C3; const void* R;
+  const void* swiglu_g; const void* swiglu_u;
   long long ldc, c_group_stride;
   int c_fp32, accumulate;
   float alpha;
@@ -375,12 +376,14 @@ __device__ __forceinline__ void epi_zero(const GemmParams& p, const EpiRow& r, b
 
 // One warp's part of a tile: COLS = BN / 2 accumulator columns from TMEM column `taddr` on (dual: COLS / 2 outputs, the
 // up accumulators being 2 * COLS / 2 = BN / 2 columns further).  `wait` is called once, before the first TMEM load.
-template <int BN, class Wait>
+// SWIGLU: the form for p.swiglu_g, in kernels of its own: beside the other forms its registers make them spill (weight
+// gradients of one micro-batch, accumulated, lost 15 %).
+template <int BN, bool SWIGLU, class Wait>
 __device__ __forceinline__ bool epi_tile(const GemmParams& p, uint8_t* stage, uint32_t tacc, int half, int lane, int n0, const EpiRow& r, Wait wait) {
   const bool fast = !p.c_fp32 && !(p.accumulate && p.R != nullptr);
   const unsigned row_ok = __ballot_sync(0xffffffffu, r.ok);
   const unsigned long long mine = reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16*>(r.C) + r.base);
-  if (p.dual) {
+  if (!SWIGLU && p.dual) {
     constexpr int OUT = BN / 4;                   // output columns of this warp
     if (!wait()) return false;
     const int n_mats = p.store_gate_up ? 3 : 1;
@@ -419,47 +422,101 @@ __device__ __forceinline__ bool epi_tile(const GemmParams& p, uint8_t* stage, ui
   }
   constexpr int CHUNKS = BN / 128;                // 64-column chunks of this warp
   const int col0 = n0 + half * (BN / 2);
-  const bool add = fast && (p.accumulate || p.R != nullptr);
   const float alpha = gemm_alpha(p);
-  const unsigned long long src = p.accumulate ? mine : reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(p.R) + r.base);
-  uint4 pre[8];                                   // (two chunks' worth of registers would spill, and serialise the loads)
-  if (add) epi_fetch(pre, src, row_ok, lane, col0, p.N, p.accumulate ? p.C : p.R);
-  if (!wait()) return false;
+  if constexpr (SWIGLU) {
+    // dh in the accumulator -> dg, du.  As a kernel of its own this read dh, g and u and wrote both for 12 000 tokens x
+    // 14336 in 685 us (41 us for 576 tokens), dh rounded to bf16 on the way; here it passes under the next tile's MMAs.
+    if (!wait()) return false;
+    const unsigned long long grow = reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(p.swiglu_g) + r.base);
+    const unsigned long long urow = reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(p.swiglu_u) + r.base);
+    const unsigned long long durow = reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16*>(p.C2) + r.base);
 #pragma unroll 1
-  for (int ch = 0; ch < CHUNKS; ++ch) {
-    const int col = col0 + ch * 64;
-    if (col >= p.N) break;
-    if (add) {
-      epi_stage_in(stage, pre, lane);
-      if (ch + 1 < CHUNKS) epi_fetch(pre, src, row_ok, lane, col + 64, p.N, p.accumulate ? p.C : p.R);
-    }
-#pragma unroll 1
-    for (int part = 0; part < 2; ++part) {
-      uint32_t acc[32];
-      float v[32];
-      tmem_ld_32x32(tacc + half * (BN / 2) + ch * 64 + part * 32, acc);
-      tmem_ld_wait();
+    for (int ch = 0; ch < CHUNKS; ++ch) {
+      const int col = col0 + ch * 64;
+      if (col >= p.N) break;
+      uint4 gk[8], du[8];
+      {
+        uint4 pu[8];
+        epi_fetch(gk, grow, row_ok, lane, col, p.N, p.swiglu_g);
+        epi_fetch(pu, urow, row_ok, lane, col, p.N, p.swiglu_u);
+        epi_stage_in(stage, gk, lane);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]) * alpha;
-      if (add) {
-        epi_stage_row<true>(stage, v, part, lane);
-      } else if (fast) {
-        epi_stage_row<false>(stage, v, part, lane);
-      } else if (r.ok) {
+        for (int j = 0; j < 8; ++j) gk[j] = *epi_slot(stage, lane, j);     // this lane's row of g
+        __syncwarp();
+        epi_stage_in(stage, pu, lane);                                     // u: row by row from the stage
+      }
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const int cc = col + part * 32 + w * 8;
-          if (cc < p.N) {
-            float o[8];
+      for (int part = 0; part < 2; ++part) {
+        uint32_t acc[32];
+        tmem_ld_32x32(tacc + half * (BN / 2) + ch * 64 + part * 32, acc);
+        tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = v[w * 8 + i];
-            store8(r.C, r.base + cc, o, p.c_fp32, p.accumulate, p.R);
+        for (int j = 0; j < 4; ++j) {
+          uint4* slot = epi_slot(stage, lane, part * 4 + j);
+          const uint4 uv = *slot;
+          const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gk[part * 4 + j]);
+          const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&uv);
+          uint4 dgv;
+          __nv_bfloat162* dg2 = reinterpret_cast<__nv_bfloat162*>(&dgv);
+          __nv_bfloat162* du2 = reinterpret_cast<__nv_bfloat162*>(&du[part * 4 + j]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float2 gf = __bfloat1622float2(g2[i]), uf = __bfloat1622float2(u2[i]);
+            const float d0 = __uint_as_float(acc[j * 8 + 2 * i]) * alpha, d1 = __uint_as_float(acc[j * 8 + 2 * i + 1]) * alpha;
+            const float s0 = 1.f / (1.f + __expf(-gf.x)), s1 = 1.f / (1.f + __expf(-gf.y));
+            du2[i] = __floats2bfloat162_rn(d0 * (gf.x * s0), d1 * (gf.y * s1));
+            dg2[i] = __floats2bfloat162_rn(d0 * uf.x * s0 * (1.f + gf.x * (1.f - s0)), d1 * uf.y * s1 * (1.f + gf.y * (1.f - s1)));
           }
+          *slot = dgv;
         }
       }
-      __syncwarp();   // the next TMEM load is warp-aligned
+      epi_flush(stage, mine, row_ok, lane, col, p.N);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) *epi_slot(stage, lane, j) = du[j];
+      epi_flush(stage, durow, row_ok, lane, col, p.N);
     }
-    if (fast) epi_flush(stage, mine, row_ok, lane, col, p.N);
+  } else {
+    const bool add = fast && (p.accumulate || p.R != nullptr);
+    const unsigned long long src = p.accumulate ? mine : reinterpret_cast<unsigned long long>(reinterpret_cast<const __nv_bfloat16*>(p.R) + r.base);
+    uint4 pre[8];                                   // (two chunks' worth of registers would spill, and serialise the loads)
+    if (add) epi_fetch(pre, src, row_ok, lane, col0, p.N, p.accumulate ? p.C : p.R);
+    if (!wait()) return false;
+#pragma unroll 1
+    for (int ch = 0; ch < CHUNKS; ++ch) {
+      const int col = col0 + ch * 64;
+      if (col >= p.N) break;
+      if (add) {
+        epi_stage_in(stage, pre, lane);
+        if (ch + 1 < CHUNKS) epi_fetch(pre, src, row_ok, lane, col + 64, p.N, p.accumulate ? p.C : p.R);
+      }
+#pragma unroll 1
+      for (int part = 0; part < 2; ++part) {
+        uint32_t acc[32];
+        float v[32];
+        tmem_ld_32x32(tacc + half * (BN / 2) + ch * 64 + part * 32, acc);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]) * alpha;
+        if (add) {
+          epi_stage_row<true>(stage, v, part, lane);
+        } else if (fast) {
+          epi_stage_row<false>(stage, v, part, lane);
+        } else if (r.ok) {
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const int cc = col + part * 32 + w * 8;
+            if (cc < p.N) {
+              float o[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] = v[w * 8 + i];
+              store8(r.C, r.base + cc, o, p.c_fp32, p.accumulate, p.R);
+            }
+          }
+        }
+        __syncwarp();   // the next TMEM load is warp-aligned
+      }
+      if (fast) epi_flush(stage, mine, row_ok, lane, col, p.N);
+    }
   }
   return true;
 }
@@ -471,7 +528,7 @@ __device__ __forceinline__ uint64_t operand_desc(uint32_t addr, int mn_major) {
 }
 __device__ __forceinline__ uint32_t operand_kstep(int mn_major) { return mn_major ? 2048 >> 4 : 32 >> 4; }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool SWIGLU>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
   constexpr int B_BYTES = BN * BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -701,7 +758,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
         }
         continue;
       }
-      if (!epi_tile<BN>(p, stage, tacc, half, lane, t.n0, r, wait)) break;
+      if (!epi_tile<BN, SWIGLU>(p, stage, tacc, half, lane, t.n0, r, wait)) break;
       if (publish) {            // by the half that finishes second (before the accumulator is released, see rows_done)
         __threadfence_system();
         __syncwarp();
@@ -745,6 +802,7 @@ constexpr int PAIR_STAGE_BYTES = A_BYTES + PAIR_B_BYTES;
 constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES;
 static_assert(PAIR_SMEM <= 227 * 1024, "pair kernel: stages + barriers + epilogue stages exceed the shared memory of a CTA");
 
+template <bool SWIGLU>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_pair_kernel(const __grid_constant__ GemmParams p) {
   constexpr int STAGES = PAIR_STAGES;
   constexpr int BN = PAIR_BN;
@@ -908,7 +966,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
         tc_fence_after();
         return true;
       };
-      if (!epi_tile<BN>(p, stage, tmem_base + buf * BN + ((uint32_t)(q * 32) << 16), half, lane, t.n0, r, wait)) break;
+      if (!epi_tile<BN, SWIGLU>(p, stage, tmem_base + buf * BN + ((uint32_t)(q * 32) << 16), half, lane, t.n0, r, wait)) break;
       if (p.row_dest_rank != nullptr) {            // by the half that finishes second (see the 128-row kernel)
         __threadfence_system();
         __syncwarp();
@@ -1200,17 +1258,17 @@ static bool split_workspace(cudaStream_t stream, SplitWorkspace* out) {
   return true;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool SWIGLU>
 static cudaError_t launch(const GemmParams& p, int grid, cudaStream_t stream) {
   constexpr int smem = STAGES * (A_BYTES + BN * BK * 2) + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES;
   static_assert(smem <= 227 * 1024, "stages + barriers + epilogue stages exceed the shared memory of a CTA");
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_kernel<BN, STAGES, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  gemm_sm100_kernel<BN, STAGES><<<grid, GEMM_THREADS, smem, stream>>>(p);
+  gemm_sm100_kernel<BN, STAGES, SWIGLU><<<grid, GEMM_THREADS, smem, stream>>>(p);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -1220,11 +1278,12 @@ static cudaError_t launch(const GemmParams& p, int grid, cudaStream_t stream) {
 static int g_max_pairs = 0;
 static int g_pair_cap = 0;   // optional upper bound set through mdt_gemm_set_pair_cap (0 = none)
 
+template <bool SWIGLU>
 static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream_t stream) {
   constexpr int smem = PAIR_SMEM;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_pair_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -1234,13 +1293,13 @@ static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream
     attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
     cfg.attrs = &attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_sm100_pair_kernel, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2; }
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_sm100_pair_kernel<SWIGLU>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2; }
     g_max_pairs = n < g_num_sms / 2 ? n : g_num_sms / 2;
     configured = true;
   }
   const int limit = (g_pair_cap > 0 && g_pair_cap < g_max_pairs) ? g_pair_cap : g_max_pairs;
   const int grid = 2 * (pairs_wanted < limit ? pairs_wanted : limit);
-  gemm_sm100_pair_kernel<<<grid, GEMM_THREADS, smem, stream>>>(p);
+  gemm_sm100_pair_kernel<SWIGLU><<<grid, GEMM_THREADS, smem, stream>>>(p);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -1296,7 +1355,7 @@ static bool pair_is_faster(const MdtGemmDesc* d, long long thread_rows_hint, int
   // rounds: whole ones where the row count is known
   double r1 = d->mode == 1 ? fmax(1.0, e1 + 0.3) : ceil(e1), r2 = d->mode == 1 ? fmax(1.0, e2 + 0.3) : ceil(e2);
   double extra1 = 0.0;
-  if (split_enabled() && d->mode != 2 && !d->dual && e1 > 1.0 && e1 - floor(e1) < 0.875 && kb >= 8.0) {   // shared last round
+  if (split_enabled() && d->mode != 2 && !d->dual && d->swiglu_g == nullptr && e1 > 1.0 && e1 - floor(e1) < 0.875 && kb >= 8.0) {   // shared last round
     r1 = e1 + (d->mode == 1 ? 0.38 : 0.08);
     extra1 = 15.0;
   }
@@ -1358,7 +1417,7 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
 // partial tiles; against one CTA per tile (0.28 + 1, 128-wide outputs) or the faster of the two 256-wide kernels in one
 // round.  128 CTAs at most: a cluster needs its SMs in one GPC.
 static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int num_sms, int* bn) {
-  if (d->dual || d->tile_ready != nullptr || d->row_dest_rank != nullptr || (d->accumulate && d->R != nullptr)) return 0;
+  if (d->dual || d->swiglu_g != nullptr || d->tile_ready != nullptr || d->row_dest_rank != nullptr || (d->accumulate && d->R != nullptr)) return 0;
   const int G = d->G < 1 ? 1 : d->G;
   *bn = d->N <= 64 ? 64 : (d->N <= 128 ? 128 : 256);
   double rows = (double)d->M, depth = (double)d->K, n = (double)d->capacity_rows - 127.0 * G;
@@ -1443,6 +1502,9 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   p.b_rows = d->b_rows; p.ldb = d->ldb; p.b_group_stride = d->b_group_stride;
   p.bl_rows = d->bl_rows; p.ldb_l = d->ldb_l; p.bl_group_stride = d->bl_group_stride;
   p.R = d->R;
+  p.swiglu_g = d->swiglu_g; p.swiglu_u = d->swiglu_u;
+  if (p.swiglu_g != nullptr && (p.dual || p.mode == 2 || p.c_fp32 || p.accumulate || p.R != nullptr || p.row_dest_rank != nullptr || p.swiglu_u == nullptr || p.C2 == nullptr))
+    return -14;
   if (p.R != nullptr && (p.dual || p.mode == 2 || p.row_dest_rank != nullptr || (reinterpret_cast<uintptr_t>(p.R) & 15))) return -13;
   if (p.row_dest_rank != nullptr && (p.dual || p.c_fp32 || p.accumulate || p.mode == 2)) return -12;
   if (p.N % 8 != 0 || p.ldc % 8 != 0) return -10;
@@ -1480,10 +1542,10 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   if (pair) {
     long long pairs = ((rows + 2 * BM - 1) / (2 * BM) + (p.mode == 1 ? p.G : 0)) * ((p.N + bn_out - 1) / bn_out) * (p.mode == 2 ? p.G : 1);
     const int np = (int)(pairs < 1 ? 1 : (pairs > g_num_sms ? g_num_sms : pairs));
-    cudaError_t e2 = launch_pair(p, np, stream);
+    cudaError_t e2 = p.swiglu_g != nullptr ? launch_pair<true>(p, np, stream) : launch_pair<false>(p, np, stream);
     return e2 == cudaSuccess ? 0 : -100 - (int)e2;
   }
-  if (split_enabled() && p.mode != 2 && !p.dual) {
+  if (split_enabled() && p.mode != 2 && !p.dual && p.swiglu_g == nullptr) {
     // the last, partly filled round of tiles may be cut along the depth and shared by all SMs (get_work)
     const long long kbt = (p.K + BK - 1) / BK + (p.K_l + BK - 1) / BK;
     SplitWorkspace w;
@@ -1492,6 +1554,8 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
       grid = g_num_sms;
     }
   }
-  cudaError_t e = (BN == 256) ? launch<256, 4>(p, grid, stream) : launch<128, 6>(p, grid, stream);
+  cudaError_t e;
+  if (p.swiglu_g != nullptr) e = (BN == 256) ? launch<256, 4, true>(p, grid, stream) : launch<128, 6, true>(p, grid, stream);
+  else e = (BN == 256) ? launch<256, 4, false>(p, grid, stream) : launch<128, 6, false>(p, grid, stream);
   return e == cudaSuccess ? 0 : -100 - (int)e;
 }

@@ -271,6 +271,173 @@ __global__ void router_bwd_kernel(const bf16* __restrict__ x, const bf16* __rest
   }
 }
 
+// Up to 8 experts and 4096 columns (the usual router): four tokens per CTA and pass instead of one or two per warp.  The
+// 8 warps share the columns, so a token's logits take two vectors per thread rather than a walk over the row with the
+// whole router matrix staged first, which is what few tokens waited for (576 tokens: forward 17 us, backward 31 us); the
+// 32 sums of a pass are reduced by one transposing butterfly (31 shuffles), and a quarter-warp per token does softmax,
+// selection and their backward.  The router matrix stays in L1.  With launch overhead, 4096 columns, 8 experts: 77 tokens
+// forward 21 -> 15 us, backward 34 -> 19; 576: 24 -> 15, 34 -> 22; 8000: 63 -> 44, 120 -> 85.
+constexpr int RR_TOK = 4, RR_E = 8, RR_VEC = 2, RR_THREADS = 256;
+__device__ __forceinline__ float rr_sum8(float v) {
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ uint4 rr_vec(const bf16* row, int i, int nv) {
+  return i < nv ? reinterpret_cast<const uint4*>(row)[i] : make_uint4(0, 0, 0, 0);
+}
+template <bool BWD>
+__global__ void __launch_bounds__(RR_THREADS, 2) router_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ scores,
+                                                                    bf16* __restrict__ weights, int* __restrict__ idx_out, const int* __restrict__ idx,
+                                                                    const bf16* __restrict__ dweights, const bf16* __restrict__ dscores,
+                                                                    bf16* __restrict__ dx, float* __restrict__ dlogits, int tokens, int hidden,
+                                                                    int experts, int top_k, int normalize, int accumulate_dx,
+                                                                    float* __restrict__ stats) {
+  __shared__ float red[2][RR_THREADS / 32][32];
+  __shared__ float s_dl[RR_TOK][RR_E];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = hidden / 8;
+  int buf = 0;
+  float cnt = 0.f, psum = 0.f;                     // of this lane's expert (warp 0), see router_fwd_kernel
+  for (int t0 = blockIdx.x * RR_TOK; t0 < tokens; t0 += gridDim.x * RR_TOK, buf ^= 1) {
+    uint4 xv[RR_VEC][RR_TOK];
+#pragma unroll
+    for (int v = 0; v < RR_VEC; ++v)
+#pragma unroll
+      for (int u = 0; u < RR_TOK; ++u)
+        xv[v][u] = rr_vec(x + (long long)(t0 + u < tokens ? t0 + u : t0) * hidden, threadIdx.x + v * RR_THREADS, nv);
+    float a[32];                                   // [token][expert]
+#pragma unroll
+    for (int i = 0; i < 32; ++i) a[i] = 0.f;
+#pragma unroll
+    for (int v = 0; v < RR_VEC; ++v) {
+      float xf[RR_TOK][8];
+#pragma unroll
+      for (int u = 0; u < RR_TOK; ++u) unpack8r(xv[v][u], xf[u]);
+#pragma unroll
+      for (int e = 0; e < RR_E; ++e) {
+        if (e < experts) {
+          float wf[8]; unpack8r(rr_vec(w + (long long)e * hidden, threadIdx.x + v * RR_THREADS, nv), wf);
+#pragma unroll
+          for (int u = 0; u < RR_TOK; ++u)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[u * RR_E + e] += xf[u][j] * wf[j];
+        }
+      }
+    }
+    // lane l ends with the warp's sum of a[l]
+#pragma unroll
+    for (int n = 16; n > 0; n >>= 1) {
+      const bool up = (lane & n) != 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i < n) {
+          const float keep = up ? a[i + n] : a[i], send = up ? a[i] : a[i + n];
+          a[i] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+        }
+      }
+    }
+    red[buf][warp][lane] = a[0];
+    __syncthreads();
+    if (warp == 0) {
+      const int u = lane / RR_E, e = lane % RR_E, t = t0 + u, base = lane - e;
+      const bool live = e < experts, valid = t < tokens;
+      float logit = 0.f;
+#pragma unroll
+      for (int k = 0; k < RR_THREADS / 32; ++k) logit += red[buf][k][lane];
+      float mx = live ? logit : -INFINITY;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      float prob = live ? __expf(logit - mx) : 0.f;
+      prob *= 1.f / rr_sum8(prob);
+      if (!BWD) {
+        float left = live ? prob : -2.f, mine = 0.f, denom = 0.f;
+        int my_sel = 0;
+        for (int c = 0; c < top_k; ++c) {
+          float bv = left;
+          int best = e;
+#pragma unroll
+          for (int o = 4; o > 0; o >>= 1) {        // the largest, of equal ones the first
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const int oe = __shfl_xor_sync(0xffffffffu, best, o);
+            if (ov > bv || (ov == bv && oe < best)) { bv = ov; best = oe; }
+          }
+          bv = __shfl_sync(0xffffffffu, bv, base);
+          best = __shfl_sync(0xffffffffu, best, base);
+          if (e == best) { left = -1.f; cnt += valid ? 1.f : 0.f; }
+          if (e == c) { mine = bv; my_sel = best; }        // (top_k <= experts <= 8)
+          denom += bv;
+        }
+        if (!normalize) denom = 1.f;
+        if (valid) {
+          if (live) scores[(long long)t * experts + e] = __float2bfloat16(prob);
+          psum += __bfloat162float(__float2bfloat16(prob));
+          if (e < top_k) {
+            weights[(long long)t * top_k + e] = __float2bfloat16(mine / denom);
+            idx_out[(long long)t * top_k + e] = my_sel < experts ? my_sel : 0;
+          }
+        }
+      } else {
+        // the forward's selection is authoritative (ties): take the saved indices
+        const long long at = (long long)(valid ? t : t0) * top_k;
+        float denom = 0.f, dot = 0.f;
+        for (int c = 0; c < top_k; ++c) {
+          const int sel = idx[at + c];
+          const float pv = __shfl_sync(0xffffffffu, prob, base + (sel & (RR_E - 1)));
+          const float pc = sel >= 0 && sel < experts ? pv : 0.f;
+          denom += pc;
+          dot += __bfloat162float(dweights[at + c]) * pc;
+        }
+        if (!normalize) denom = 1.f;
+        dot = normalize ? dot / denom : 0.f;
+        float ds = (dscores != nullptr && live) ? __bfloat162float(dscores[(long long)(valid ? t : t0) * experts + e]) : 0.f;
+        for (int c = 0; c < top_k; ++c)
+          if (idx[at + c] == e) ds += (__bfloat162float(dweights[at + c]) - dot) / denom;
+        const float dl = prob * (ds - rr_sum8(prob * ds));
+        s_dl[u][e] = live ? dl : 0.f;
+        if (valid && live && dlogits != nullptr) dlogits[(long long)t * experts + e] = dl;
+      }
+    }
+    if (BWD) {
+      __syncthreads();
+#pragma unroll
+      for (int v = 0; v < RR_VEC; ++v) {
+        const int i = threadIdx.x + v * RR_THREADS;
+        if (i >= nv) break;
+        float acc[RR_TOK][8];
+#pragma unroll
+        for (int u = 0; u < RR_TOK; ++u)
+          unpack8r(accumulate_dx && t0 + u < tokens ? reinterpret_cast<const uint4*>(dx + (long long)(t0 + u) * hidden)[i] : make_uint4(0, 0, 0, 0), acc[u]);
+#pragma unroll
+        for (int e = 0; e < RR_E; ++e) {
+          if (e < experts) {
+            float wf[8]; unpack8r(reinterpret_cast<const uint4*>(w + (long long)e * hidden)[i], wf);
+#pragma unroll
+            for (int u = 0; u < RR_TOK; ++u) {
+              const float d = s_dl[u][e];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[u][j] += d * wf[j];
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < RR_TOK; ++u)
+          if (t0 + u < tokens) reinterpret_cast<uint4*>(dx + (long long)(t0 + u) * hidden)[i] = pack8r(acc[u]);
+      }
+      __syncthreads();                             // s_dl is rewritten by the next pass
+    }
+  }
+  if (!BWD && stats != nullptr && warp == 0) {
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) { cnt += __shfl_xor_sync(0xffffffffu, cnt, o); psum += __shfl_xor_sync(0xffffffffu, psum, o); }
+    if (lane < experts) { atomicAdd(stats + lane, cnt); atomicAdd(stats + experts + lane, psum); }
+  }
+}
+static bool router_rows_ok(int hidden, int experts) { return experts <= RR_E && hidden <= 8 * RR_VEC * RR_THREADS; }
+static int router_rows_grid(int tokens) {
+  const int g = (tokens + RR_TOK - 1) / RR_TOK, cap = sm_count_of_current_device() * 2;
+  return g < cap ? g : cap;
+}
+
 // dW[e, col] = sum_t dlogits[t, e] * x[t, col], tokens split over blockIdx.y.  VEC columns per thread, four rows of x in
 // flight; the dlogits of 32 tokens at a time are staged in shared memory.  Bound by one pass over x (8000 x 4096, 8
 // experts: 188 us with one column per thread and one row in flight).  With more than 16 experts VEC is 1 for want of
@@ -485,8 +652,8 @@ static int router_grid(int tokens) {
   const int cap = sm_count_of_current_device() * 3;
   return g < 1 ? 1 : (g > cap ? cap : g);
 }
-// Two tokens per warp and pass once every warp of the grid has two (more experts than 8: no registers for it).  8000 x
-// 4096, 8 experts: forward 81 -> 60 us; a micro-batch of 576 tokens would lose (backward 31 -> 42 us).
+// (Rows too wide for router_rows_kernel.)  Two tokens per warp and pass once every warp of the grid has two (more experts
+// than 8: no registers for it).  8000 x 4096, 8 experts: forward 81 -> 60 us; 576 tokens would lose (backward 31 -> 42 us).
 static bool router_pairs(int tokens, int grid) { return tokens >= 2 * grid * 4; }
 // The router matrix is staged in shared memory when it fits (E x H bf16 <= 96 KB); opt in above 48 KB once per kernel.
 static int router_smem_ok(const void* kernel, size_t bytes) {
@@ -506,6 +673,12 @@ extern "C" int mdt_router_fwd(const void* x, const void* w, void* scores, void* 
                               int experts, int top_k, int normalize, float* stats, cudaStream_t s) {
   if (hidden % 8 != 0 || experts > MAX_E || top_k > MAX_K || top_k > experts) return -1;
   if (tokens == 0) return 0;
+  if (router_rows_ok(hidden, experts)) {
+    router_rows_kernel<false><<<router_rows_grid(tokens), RR_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, idx, nullptr, nullptr,
+                                                                            nullptr, nullptr, nullptr, tokens, hidden, experts, top_k, normalize, 0, stats);
+    MDT_RT_CHECK();
+    return 0;
+  }
   const int grid = router_grid(tokens);
   const size_t wbytes = (size_t)experts * hidden * 2;
 #define RT_FWD(ET, TOK)                                                                                                        \
@@ -531,7 +704,10 @@ extern "C" int mdt_router_bwd(const void* x, const void* w, const int* idx, cons
 #define RT_BWD(ET, VEC, TOK)                                                                                                   \
   {                                                                                                                         \
     const int staged = router_smem_ok((const void*)router_bwd_kernel<ET, TOK>, wbytes);                                     \
-    router_bwd_kernel<ET, TOK><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, idx, (const bf16*)dweights,  \
+    if (router_rows_ok(hidden, experts))                                                                                    \
+      router_rows_kernel<true><<<router_rows_grid(tokens), RR_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, nullptr, nullptr, nullptr, idx, (const bf16*)dweights, \
+                                                                             (const bf16*)dscores, (bf16*)dx, dlogits, tokens, hidden, experts, top_k, normalize, accumulate_dx, nullptr); \
+    else router_bwd_kernel<ET, TOK><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, idx, (const bf16*)dweights,  \
                                                                  (const bf16*)dscores, (bf16*)dx, dlogits, tokens, hidden,  \
                                                                  experts, top_k, normalize, accumulate_dx, staged);         \
     MDT_RT_CHECK();                                                                                                         \

@@ -48,13 +48,14 @@ def launch_count() -> int:
 
 def _gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G=1, offsets=None, capacity=0, B2=None, A_l=None, a_mn_l=False,
           B_l=None, B2_l=None, b_mn_l=False, K_l=0, C2=None, C3=None, accumulate=False, alpha=1.0, wait=None, scatter=None,
-          residual=None, alpha_dev=None):
+          residual=None, alpha_dev=None, swiglu=None):
     """alpha_dev: optional fp32 scalar on the GPU that multiplies alpha.  wait = (tile_ready, tile_expected): A rows arrive from peers, tile by tile.  scatter = (row_rank, row_pos,
-    peer_out table, peer_arrive table): result rows are stored into peers' buffers instead of C."""
+    peer_out table, peer_arrive table): result rows are stored into peers' buffers instead of C.  swiglu = (g, u): the product
+    is the gradient of silu(g) * u; the gradients of g and u go to C and C2."""
     w0, w1 = wait if wait is not None else (None, None)
     s0, s1, s2, s3 = scatter if scatter is not None else (None, None, None, None)
     ext.gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G, offsets, capacity, B2, A_l, a_mn_l, B_l, B2_l, b_mn_l, K_l,
-             C2, C3, accumulate, alpha, status_tensor(A.device), w0, w1, s0, s1, s2, s3, residual, alpha_dev)
+             C2, C3, accumulate, alpha, status_tensor(A.device), w0, w1, s0, s1, s2, s3, residual, alpha_dev, *(swiglu if swiglu is not None else (None, None)))
     return C
 
 
@@ -305,8 +306,9 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
             _g(1, dy, False, B2, False, dt2, r, H, plan, alpha=s2, wait=wait)  # s * dy B2^T
             wait = None
             kw = dict(A_l=dt2, B_l=A2, b_mn_l=False, K_l=r)
-        dh = torch.empty(R, F, dtype=dt, device=dev)
-        _g(1, dy, False, w2, False, dh, F, H, plan, wait=wait, **kw)            # dy W2^T (W2 stored [F,H])
+        dg, du = torch.empty(R, F, dtype=dt, device=dev), torch.empty(R, F, dtype=dt, device=dev)
+        # dh = dy W2^T (W2 stored [F,H]), through SwiGLU in the epilogue
+        _g(1, dy, False, w2, False, dg, F, H, plan, C2=du, swiglu=(g, u), wait=wait, **kw)
         wg = ctx.wgrad_out
         dw1 = dw2 = dw3 = None
         need_w = ctx.needs_input_grad[1] or ctx.needs_input_grad[2] or ctx.needs_input_grad[3]
@@ -321,8 +323,6 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
             dA2 = torch.empty_like(A2); _g(2, h, True, dt2, True, dA2, A2.shape[2], 0, plan, alpha=ws)
             dB2 = torch.empty_like(B2); _g(2, t2, True, dy, True, dB2, H, 0, plan, alpha=ws)
             grads[id(A2)], grads[id(B2)] = dA2, dB2
-        # ---- SwiGLU
-        dg, du = ext.swiglu_bwd(g, u, dh, plan.padded_offsets)
         # ---- up projections
         dx = torch.empty(R, H, dtype=dt, device=dev)
         _g(1, dg, False, w1, True, dx, H, F, plan, A_l=du, B_l=w3, b_mn_l=True, K_l=F, scatter=scatter)   # dg W1 + du W3

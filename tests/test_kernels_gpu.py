@@ -239,6 +239,33 @@ def test_gemm_epilogue_edges(ops, M, N, K, policy):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("policy", [0, 2, 5], ids=["tile128", "pair", "default"])
+@pytest.mark.parametrize("T,E,H,F", [(5, 2, 64, 72), (300, 3, 192, 520), (1500, 4, 512, 1024)])
+def test_swiglu_backward_in_the_product(ops, T, E, H, F, policy):
+    """dg and du of silu(g) * u from the down projection's input gradient, remainders of the 64-column chunks and empty
+    experts included, against fp64 on the same bf16 g, u, dy, w2: one bf16 rounding of each result; rows past the groups
+    stay untouched."""
+    torch.manual_seed(T)
+    top = (torch.arange(T, device=DEV) % max(E - 1, 1)).int()[:, None]
+    plan = ops.make_plan(top, E)
+    R, used, offs = plan.src_slot.numel(), int(plan.padded_offsets[-1]), plan.padded_offsets.tolist()
+    dy = ops.ext.gather_rows(_rand(T, H), plan.src_slot, plan.padded_offsets, E, None, 1)
+    g, u, w2 = _rand(R, F, scale=2.0), _rand(R, F), _rand(E, F, H, scale=0.1)
+    dg, du = (torch.full((R, F), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    _under_pair_policy(ops, policy, lambda: ops._g(1, dy, False, w2, False, dg, F, H, plan, C2=du, swiglu=(g, u)))
+    for e in range(E):
+        a, b = offs[e], offs[e + 1]
+        if a == b:
+            continue
+        g64, u64 = g[a:b].double().requires_grad_(True), u[a:b].double().requires_grad_(True)
+        dh = dy[a:b].double() @ w2[e].double().t()
+        rg, ru = torch.autograd.grad(torch.nn.functional.silu(g64) * u64, (g64, u64), dh)
+        _close(dg[a:b], rg, 1e-2, name=f"dg {e}")
+        _close(du[a:b], ru, 1e-2, name=f"du {e}")
+    assert bool((dg[used:] == 7.0).all()) and bool((du[used:] == 7.0).all())
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (77, 1024, 4096), (300, 520, 2056), (129, 64, 8192), (1000, 16, 4096), (33, 128, 1024)])
 def test_gemm_few_tiles_shared_by_a_cluster(ops, M, N, K):
     """Products with few output tiles under the default policy (the depth is cut over a cluster): K-major and MN-major
