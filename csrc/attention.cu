@@ -912,8 +912,9 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
   memset(&p, 0, sizeof(p));
   // MDT_ATTN_FWD=serial selects the one-block-at-a-time kernel (for comparisons); default: the pipelined kernel
   static const bool serial = []() { const char* e = getenv("MDT_ATTN_FWD"); return e != nullptr && e[0] == 's'; }();
-  int rc = att_map(&p.tmQ, q, total_tokens, heads_q) | att_map(&p.tmK, k, total_tokens, heads_kv) | att_map(&p.tmV, v, total_tokens, heads_kv);
-  if (!serial) rc |= att_map(&p.tmK64, k, total_tokens, heads_kv, FB) | att_map(&p.tmV64, v, total_tokens, heads_kv, FB);
+  int rc = att_map(&p.tmQ, q, total_tokens, heads_q);
+  if (serial) rc |= att_map(&p.tmK, k, total_tokens, heads_kv) | att_map(&p.tmV, v, total_tokens, heads_kv);
+  else rc |= att_map(&p.tmK64, k, total_tokens, heads_kv, FB) | att_map(&p.tmV64, v, total_tokens, heads_kv, FB);
   if (rc) return rc;
   p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.heads_q = heads_q; p.heads_kv = heads_kv;
   p.scale_log2e = scale * 1.4426950408889634f;

@@ -631,7 +631,8 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
   Tensor q, k, v, qr, kr;
   OptTensor tq, tk, tv;
   static const bool side_streams = []() { const char* e = getenv("MDT_QKV_STREAMS"); return !(e != nullptr && e[0] == '0'); }();
-  if (side_streams) {
+  // (products of a few microseconds are not worth the ~25 us that the host spends on streams and events)
+  if (side_streams && T * xn.size(1) * Hkv * d >= (int64_t)1 << 27) {
     auto main_stream = at::cuda::getCurrentCUDAStream();
     auto s1 = at::cuda::getStreamFromPool(false, x.device().index()), s2 = at::cuda::getStreamFromPool(false, x.device().index());
     at::cuda::CUDAEvent ready, done1, done2;

@@ -1412,11 +1412,33 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
   return wide ? 2 : 0;
 }
 
+// Clusters of S CTAs of the cluster kernel that are resident at once (all its widths take the SM's shared memory).
+static int max_clusters(int S) {
+  static int cached[MAX_CLUSTER + 1];
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  if (cached[S] == 0) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(g_num_sms / S * S)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = SplitShape<256>::SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(gemm_sm100_cluster_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitShape<256>::SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_sm100_cluster_kernel<256>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2 / S; }
+    cached[S] = n;
+  }
+  return cached[S];
+}
+
 // Whether a product with few tiles is cut along the depth, and how: cluster size (0 = not) and tile width.  Times in
 // microseconds, measured on B200: 0.48 / 0.28 / 0.22 per k block of a 256 / 128 / 64-wide tile, 5 for the exchange of the
 // partial tiles; against one CTA per tile (0.28 + 1, 128-wide outputs) or the faster of the two 256-wide kernels in one
-// round.  128 CTAs at most: a cluster needs its SMs in one GPC.
-static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int num_sms, int* bn) {
+// round.  All clusters have to be resident at once (max_clusters: a cluster needs its SMs in one GPC, so 16 clusters of 8
+// are more than a B200 holds: 16 tiles 64 deep took 25 us that way, in two rounds, 4 tiles 13).
+static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int* bn) {
   if (d->dual || d->swiglu_g != nullptr || d->tile_ready != nullptr || d->row_dest_rank != nullptr || (d->accumulate && d->R != nullptr)) return 0;
   const int G = d->G < 1 ? 1 : d->G;
   *bn = d->N <= 64 ? 64 : (d->N <= 128 ? 128 : 256);
@@ -1431,7 +1453,7 @@ static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int 
   const double per = *bn == 256 ? 0.48 : (*bn == 128 ? 0.28 : 0.22);
   const double whole = d->N <= 128 ? kb * 0.28 + 1.0 : fmin(kb * 0.48 + 1.0, kb * 0.34 + 2.0);
   for (int S = MAX_CLUSTER; S >= 2; S /= 2)
-    if (tiles * S <= num_sms * 128.0 / 148.0 && kb >= 4.0 * S) return ceil(kb / S) * per + 5.0 < whole ? S : 0;
+    if (kb >= 4.0 * S && tiles <= max_clusters(S)) return ceil(kb / S) * per + 5.0 < whole ? S : 0;
   return 0;
 }
 
@@ -1512,7 +1534,7 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   const int BN = (p.dual || p.N > 128) ? 256 : 128;
   const int bn_out = p.dual ? BN / 2 : BN;
   int cluster_bn = 0;
-  const int cluster = pair_policy() == MAX_POLICY ? choose_cluster(d, t_rows_hint, g_num_sms, &cluster_bn) : 0;
+  const int cluster = pair_policy() == MAX_POLICY ? choose_cluster(d, t_rows_hint, &cluster_bn) : 0;
   const bool pair = cluster == 0 && choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms) != 0;
   const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
   int rc = 0;
