@@ -895,6 +895,35 @@ def test_gemm_last_round_shared_along_the_depth(ops):
     ops.check_status(DEV)
 
 
+def test_shared_last_round_first_used_on_a_stream_beside_a_busy_default_stream(ops):
+    """The fp32 workspace of the shared last round is made on a stream's first such product.  It has to be clean for that
+    product and for the next ones although the default stream, against which pool streams are not ordered, is busy."""
+    ext = ops.ext
+    torch.manual_seed(62)
+    M, N, K = 1280, 4096, 2048                          # 160 tiles of 128 rows: 12 of them shared on 148 SMs
+    x, w = _rand(M, K), _rand(N, K, scale=0.05)
+    prev_policy, prev_split = ext.gemm_set_pair_policy(0), ext.gemm_set_split(0)
+    try:
+        unsplit = ops.mm_nt(x, w).float()
+        ext.gemm_set_split(1)
+        for priority in (0, -1, 0, -1):
+            side = torch.cuda.Stream(priority=priority)
+            side.wait_stream(torch.cuda.current_stream())
+            torch.cuda._sleep(20_000_000)               # about 10 ms of the default stream
+            with torch.cuda.stream(side):
+                got = [ops.mm_nt(x, w) for _ in range(6)]
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                got.append(ops.mm_nt(x, w))
+            torch.cuda.synchronize()
+            for i, y in enumerate(got):                 # the same products, their fp32 sums in another order: one bf16 rounding apart
+                _close(y, unsplit, 1e-2, name=f"shared last round on a fresh stream, product {i}")
+    finally:
+        ext.gemm_set_split(prev_split)
+        ext.gemm_set_pair_policy(prev_policy)
+    ops.check_status(DEV)
+
+
 def test_multi_tensor_gradient_accumulate(ops):
     """fp32 accumulators += bf16 / fp32 gradients of many tensors in one launch per 16."""
     torch.manual_seed(71)
