@@ -263,7 +263,10 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_smem_addr, uint32
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta_rank));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {   // every thread of every CTA of the cluster
+// Every thread of every CTA of the cluster.  The .aligned forms want whole warps, so the warp is brought together first:
+// loops that lanes leave at different iterations may stand before a call.
+__device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

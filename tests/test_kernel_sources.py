@@ -1,0 +1,21 @@
+"""Rules of the kernel sources whose violation shows only as a rare hang, checked on the text (no GPU)."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc")
+
+
+def _read(*parts):
+    with open(os.path.join(CSRC, *parts)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_cluster_barriers_bring_the_warp_together_first():
+    """`barrier.cluster.*.aligned` is undefined for a diverged warp; callers reach it after loops with per-lane exits."""
+    bodies = [b for b in re.findall(r"__device__ __forceinline__ [^{;]*\{(.*?)\n\}", _read("common", "ptx.cuh"), re.S) if "barrier.cluster" in b]
+    assert bodies
+    for body in bodies:
+        assert body.index("__syncwarp()") < body.index("barrier.cluster"), body
+    for name in os.listdir(CSRC):
+        if name.endswith(".cu"):
+            assert "barrier.cluster" not in _read(name), name + ": use the wrapper"
