@@ -139,8 +139,7 @@ __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant_
       }
     }
     __syncwarp();
-    if (!wait_parity(barS, j & 1, abort_flag)) { ok = false; break; }
-    __syncwarp();
+    if (!wait_parity_warp(barS, j & 1, abort_flag)) { ok = false; break; }
     tc_fence_after();
     // ---- online softmax on this thread's row (two passes over TMEM: row maximum, then exponentials)
     float mx = m;
@@ -190,8 +189,7 @@ __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant_
 #pragma unroll
     for (int i = 0; i < HD; ++i) o[i] *= alpha;
     __syncwarp();
-    if (!wait_parity(barO, j & 1, abort_flag)) { ok = false; break; }
-    __syncwarp();
+    if (!wait_parity_warp(barO, j & 1, abort_flag)) { ok = false; break; }
     tc_fence_after();
 #pragma unroll
     for (int c = 0; c < 4; ++c) {

@@ -696,8 +696,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
       auto wait = [&]() {
-        if (!wait_parity(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
-        __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
+        // (one answer for the warp: the TMEM loads and shuffles that follow are warp-wide)
+        if (!wait_parity_warp(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
         tc_fence_after();
         return true;
       };
@@ -774,6 +774,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
     }
   }
 
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, TMEM_COLS); }
@@ -961,8 +962,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
       auto wait = [&]() {
-        if (!wait_parity(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
-        __syncwarp();   // lanes may leave the wait loop at different times; the TMEM loads below are warp-aligned
+        // (one answer for the warp: the TMEM loads and shuffles that follow are warp-wide)
+        if (!wait_parity_warp(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
         tc_fence_after();
         return true;
       };

@@ -19,3 +19,11 @@ def test_cluster_barriers_bring_the_warp_together_first():
     for name in os.listdir(CSRC):
         if name.endswith(".cu"):
             assert "barrier.cluster" not in _read(name), name + ": use the wrapper"
+
+
+def test_waits_before_warp_wide_instructions_give_the_warp_one_answer():
+    """TMEM loads, shuffles and __syncwarp follow the waits of whole warps: lanes that give up (time limit, abort flag) must
+    do so together.  The per-lane wait is left to branches of a single thread."""
+    for name in ("gemm_sm100.cu", "attention.cu"):
+        lone = [line.strip() for line in _read(name).splitlines() if re.search(r"\bwait_parity\(", line)]
+        assert all(re.match(r"(bool )?w = ", line) for line in lone), (name, lone)      # issuing thread of the serial attention forward
