@@ -37,7 +37,7 @@ struct AttnParams {
   CUtensorMap tmQ, tmK, tmV;
   CUtensorMap tmK64, tmV64;                  // key / value maps with 64-row boxes (pipelined forward)
   const int* cu_seqlens;
-  int num_seqs, heads_q, heads_kv;
+  int num_seqs, heads_q, heads_kv, tokens;
   float scale_log2e;
   bf16* o; float* lse;
   int* status;
@@ -62,21 +62,30 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// locate the block handled by this CTA: blockIdx.x enumerates 128-row blocks over all sequences
-__device__ __forceinline__ bool find_block(const int* cu, int num_seqs, int flat, int& seq_start, int& seq_end, int& blk) {
+// 128-row blocks of a sequence; none if it is empty or reaches outside the tensors' rows
+__device__ __forceinline__ int blocks_of(int seq_start, int seq_end, int tokens) {
+  return seq_start >= 0 && seq_end > seq_start && seq_end <= tokens ? (seq_end - seq_start + AB - 1) / AB : 0;
+}
+// Locate block `flat` of the 128-row blocks over all sequences: its sequence (-1: there is no such block) and its place there.
+// Grids have at least one block more than the sequences do; the CTA that comes past the last one reports (`status`, optional)
+// sequences that were left out because they reach outside the tensors.
+__device__ __forceinline__ int find_block(const int* cu, int num_seqs, int tokens, int flat, int& seq_start, int& seq_end, int& blk, int* status) {
+  bool outside = false;
   for (int s = 0; s < num_seqs; ++s) {
     const int a = cu[s], b = cu[s + 1];
-    const int nb = (b - a + AB - 1) / AB;
-    if (flat < nb) { seq_start = a; seq_end = b; blk = flat; return true; }
+    const int nb = blocks_of(a, b, tokens);
+    if (flat < nb) { seq_start = a; seq_end = b; blk = flat; return s; }
+    outside = outside || (nb == 0 && b > a);
     flat -= nb;
   }
-  return false;
+  if (outside && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, ST_CAPACITY);
+  return -1;
 }
 
 // ------------------------------------------------------------------------------------------- forward
 __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
   int seq_start, seq_end, qb;
-  if (!find_block(p.cu_seqlens, p.num_seqs, blockIdx.x, seq_start, seq_end, qb)) return;
+  if (find_block(p.cu_seqlens, p.num_seqs, p.tokens, blockIdx.x, seq_start, seq_end, qb, p.status) < 0) return;
   const int h = blockIdx.y, kvh = h / (p.heads_q / p.heads_kv);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -249,7 +258,7 @@ __device__ __forceinline__ void load_kv_tile(uint8_t* dst, const CUtensorMap* ma
 
 __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(const __grid_constant__ AttnParams p) {
   int seq_start, seq_end, qb;
-  if (!find_block(p.cu_seqlens, p.num_seqs, blockIdx.x / p.heads_q, seq_start, seq_end, qb)) return;
+  if (find_block(p.cu_seqlens, p.num_seqs, p.tokens, blockIdx.x / p.heads_q, seq_start, seq_end, qb, p.status) < 0) return;
   qb = (seq_end - seq_start + AB - 1) / AB - 1 - qb;          // last (longest) block of a sequence first
   const int h = blockIdx.x % p.heads_q, kvh = h / (p.heads_q / p.heads_kv);
   extern __shared__ uint8_t smem_raw[];
@@ -485,31 +494,34 @@ struct AttnBwdParams {
   float* dk; float* dv;         // fp32 partial sums [token][head set][128], or NULL: all heads of a kv head in one CTA
   bf16* dk_out; bf16* dv_out;   // then the results [token][kv head][128]
   int heads_q, heads_kv, hpc;   // hpc: query heads per CTA
+  int tokens, blocks;           // rows of the tensors; entries of the schedule
   float scale_log2e, scale;
   int* status;
 };
 
 __global__ void __launch_bounds__(256) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
-                                                               const int* __restrict__ cu, int num_seqs, int heads, int4* __restrict__ sched,
-                                                               float* __restrict__ stats, float* __restrict__ dq) {
+                                                               const int* __restrict__ cu, int num_seqs, int tokens, int heads, int4* __restrict__ sched,
+                                                               float* __restrict__ stats, float* __restrict__ dq, int* status) {
   int seq_start, seq_end, blk;
   const int flat = blockIdx.x, h = blockIdx.y;
-  if (!find_block(cu, num_seqs, flat, seq_start, seq_end, blk)) {
+  const int seq = find_block(cu, num_seqs, tokens, flat, seq_start, seq_end, blk, status);
+  if (seq < 0) {
     if (h == 0 && threadIdx.x == 0) sched[flat] = make_int4(-1, 0, 0, 0);
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (h == 0 && warp == 0) {
     // rank by the number of query blocks that a key block meets, most first
-    const int n = (seq_end - seq_start + AB - 1) / AB - blk;
+    const int n = blocks_of(seq_start, seq_end, tokens) - blk;
     int rank = 0;
     for (int s = lane; s < num_seqs; s += 32) {
-      const int nb = (cu[s + 1] - cu[s] + AB - 1) / AB;
-      rank += (nb > n ? nb - n : 0) + (cu[s] < seq_start && nb >= n ? 1 : 0);
+      const int nb = blocks_of(cu[s], cu[s + 1], tokens);
+      rank += (nb > n ? nb - n : 0) + (s < seq && nb >= n ? 1 : 0);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, off);
-    if (lane == 0) sched[rank] = make_int4(seq_start, seq_end, blk, flat);
+    // (sequences that overlap may have more blocks than the schedule has entries)
+    if (lane == 0 && rank < (int)gridDim.x) sched[rank] = make_int4(seq_start, seq_end, blk, flat);
   }
   const long long tile = (long long)flat * heads + h;
   // 16 lanes x 16 bytes hold a row, 16 rows per pass; all loads of the block are in flight at once
@@ -548,6 +560,12 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   const int4 work = p.sched[blockIdx.x / sets];
   const int seq_start = work.x, seq_end = work.y, kb = work.z;
   if (seq_start < 0) return;
+  const int nb = blocks_of(seq_start, seq_end, p.tokens);
+  // an entry of sequences that overlap, or one that nobody wrote for them: what it leads to has to exist
+  if (kb < 0 || kb >= nb || work.w < 0 || work.w + nb - kb > p.blocks) {
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, ST_CAPACITY);
+    return;
+  }
   const int set = blockIdx.x % sets, h0 = set * p.hpc, kvh = h0 / (p.heads_q / p.heads_kv);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -577,7 +595,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const int k0 = seq_start + kb * AB;
-  const int nq = (seq_end - seq_start + AB - 1) / AB - kb;  // query blocks per head
+  const int nq = nb - kb;                                   // query blocks per head
   const int n_it = nq * p.hpc;
   auto fail = [&](int code) {
     *abort_flag = 1;
@@ -833,7 +851,7 @@ __global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __r
                                                                 int heads_kv, int sets) {
   if ((int)blockIdx.x < blocks) {
     int seq_start, seq_end, blk;
-    if (!find_block(cu, num_seqs, blockIdx.x, seq_start, seq_end, blk)) return;
+    if (find_block(cu, num_seqs, tokens, blockIdx.x, seq_start, seq_end, blk, nullptr) < 0) return;
     const int h = blockIdx.y;
     const float4* src = reinterpret_cast<const float4*>(dq32 + ((long long)blockIdx.x * heads_q + h) * DQ_TILE);
     // eight lanes x 4 columns = 64 bytes of a row of dq, four rows per warp and pass; all loads in flight at once
@@ -903,7 +921,7 @@ extern "C" long long mdt_attention_launch_count() { return g_att_launches; }
 
 extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu_seqlens,
                                  int num_seqs, int total_tokens, int max_seqlen, int heads_q, int heads_kv, int head_dim,
-                                 float scale, cudaStream_t s) {
+                                 float scale, int* status, cudaStream_t s) {
   if (head_dim != HD || heads_q % heads_kv != 0) return -1;
   if (total_tokens == 0) return 0;
   static thread_local bool bound = false;
@@ -916,7 +934,8 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
   if (serial) rc |= att_map(&p.tmK, k, total_tokens, heads_kv) | att_map(&p.tmV, v, total_tokens, heads_kv);
   else rc |= att_map(&p.tmK64, k, total_tokens, heads_kv, FB) | att_map(&p.tmV64, v, total_tokens, heads_kv, FB);
   if (rc) return rc;
-  p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.heads_q = heads_q; p.heads_kv = heads_kv;
+  p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.heads_q = heads_q; p.heads_kv = heads_kv; p.tokens = total_tokens;
+  p.status = status;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.o = (bf16*)o; p.lse = lse;
   static bool configured = false;
@@ -965,7 +984,7 @@ extern "C" long long mdt_attention_bwd_scratch(int num_seqs, int total_tokens, i
 
 extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                                  void* dq, void* dk, void* dv, float* scratch, const int* cu_seqlens, int num_seqs, int total_tokens,
-                                 int max_seqlen, int heads_q, int heads_kv, int head_dim, float scale, cudaStream_t s) {
+                                 int max_seqlen, int heads_q, int heads_kv, int head_dim, float scale, int* status, cudaStream_t s) {
   // scratch: mdt_attention_bwd_scratch() floats, 128-byte aligned: schedule | row statistics | dq32 | dk32 | dv32
   if (head_dim != HD || heads_q % heads_kv != 0) return -1;
   if (total_tokens == 0) return 0;
@@ -982,15 +1001,16 @@ extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, co
   p.sched = reinterpret_cast<const int4*>(scratch); p.stats = scratch + b.off_stats; p.dq = scratch + b.off_dq;
   p.dk = direct ? nullptr : scratch + b.off_dk; p.dv = direct ? nullptr : scratch + b.off_dv;
   p.dk_out = (bf16*)dk; p.dv_out = (bf16*)dv;
-  p.heads_q = heads_q; p.heads_kv = heads_kv; p.hpc = b.hpc;
+  p.heads_q = heads_q; p.heads_kv = heads_kv; p.hpc = b.hpc; p.tokens = total_tokens; p.blocks = (int)b.blocks;
+  p.status = status;
   p.scale = scale; p.scale_log2e = scale * 1.4426950408889634f;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return -4;
     configured = true;
   }
-  attn_bwd_prepare_kernel<<<dim3((unsigned)b.blocks, heads_q), 256, 0, s>>>((const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs, heads_q,
-                                                                            reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq);
+  attn_bwd_prepare_kernel<<<dim3((unsigned)b.blocks, heads_q), 256, 0, s>>>((const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs,
+                                                                            total_tokens, heads_q, reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq, status);
   ++g_att_launches;
   attn_bwd_kernel<<<(unsigned)(b.blocks * b.sets), BWD_THREADS, BWD_SMEM, s>>>(p);
   ++g_att_launches;

@@ -365,8 +365,11 @@ Tensor combine_wgrad(const Tensor& y, const Tensor& dest_row, const Tensor& dout
   return dw;
 }
 
+static int* status_ptr(const OptTensor& status) { return status.has_value() ? status->data_ptr<int>() : nullptr; }
+
 // q [T, Hq, 128], k/v [T, Hkv, 128] -> (o [T, Hq, 128], lse [T, Hq])
-std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_seqlens, int64_t max_seqlen, double scale) {
+std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_seqlens, int64_t max_seqlen, double scale,
+                                  const OptTensor& status = std::nullopt) {
   CHECK_BF16(q); CHECK_BF16(k); CHECK_BF16(v);
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(q.is_contiguous() && k.is_contiguous() && v.is_contiguous() && cu_seqlens.scalar_type() == at::kInt);
@@ -374,11 +377,11 @@ std::vector<Tensor> attention_fwd(const Tensor& q, const Tensor& k, const Tensor
   auto o = torch::empty_like(q);
   auto lse = torch::empty({T, Hq}, q.options().dtype(at::kFloat));
   check(mdt_attention_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), cu_seqlens.data_ptr<int>(),
-                          (int)cu_seqlens.numel() - 1, T, (int)max_seqlen, Hq, Hkv, D, (float)scale, cur_stream()), "attention_fwd");
+                          (int)cu_seqlens.numel() - 1, T, (int)max_seqlen, Hq, Hkv, D, (float)scale, status_ptr(status), cur_stream()), "attention_fwd");
   return {o, lse};
 }
 std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& dout, const Tensor& lse,
-                                  const Tensor& cu_seqlens, int64_t max_seqlen, double scale) {
+                                  const Tensor& cu_seqlens, int64_t max_seqlen, double scale, const OptTensor& status = std::nullopt) {
   c10::cuda::CUDAGuard guard(q.device());
   TORCH_CHECK(dout.is_contiguous() && o.is_contiguous());
   const int T = (int)q.size(0), Hq = (int)q.size(1), Hkv = (int)k.size(1), D = (int)q.size(2);
@@ -387,7 +390,7 @@ std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor
   auto scratch = torch::empty({mdt_attention_bwd_scratch(nseq, T, (int)max_seqlen, Hq, Hkv)}, q.options().dtype(at::kFloat));
   check(mdt_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), dout.data_ptr(), lse.data_ptr<float>(), dq.data_ptr(),
                           dk.data_ptr(), dv.data_ptr(), scratch.data_ptr<float>(), cu_seqlens.data_ptr<int>(), (int)cu_seqlens.numel() - 1, T,
-                          (int)max_seqlen, Hq, Hkv, D, (float)scale, cur_stream()), "attention_bwd");
+                          (int)max_seqlen, Hq, Hkv, D, (float)scale, status_ptr(status), cur_stream()), "attention_bwd");
   return {dq, dk, dv};
 }
 
@@ -665,7 +668,7 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
     kr = rope(k.view({T, Hkv, d}), positions, theta, false);
   }
   Tensor v3 = v.view({T, Hkv, d});
-  auto at = attention_fwd(qr, kr, v3, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d));
+  auto at = attention_fwd(qr, kr, v3, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d), status);
   Tensor o = at[0], lse = at[1];
   auto [out, to] = lin_fwd(o.view({T, Hq * d}), lo, status, x.is_contiguous() ? OptTensor(x) : OptTensor(x.contiguous()));   // + x in the epilogue
   Tensor none = torch::empty({0}, x.options());
@@ -700,7 +703,7 @@ std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tens
   Tensor o2 = o.view({T, Hq * d});
   Tensor d_o = torch::empty({T, Hq * d}, x.options());
   put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status));
-  auto g3 = attention_bwd(qr, kr, v3, o, d_o.view({T, Hq, d}), lse, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d));
+  auto g3 = attention_bwd(qr, kr, v3, o, d_o.view({T, Hq, d}), lse, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d), status);
   Tensor dq = rope(g3[0], positions, theta, true).view({T, Hq * d});
   Tensor dk = rope(g3[1], positions, theta, true).view({T, Hkv * d});
   Tensor dv = g3[2].view({T, Hkv * d});
@@ -938,8 +941,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gather_rows", &gather_rows);
   m.def("combine_rows", &combine_rows, py::arg("y"), py::arg("dest_row"), py::arg("weights"), py::arg("top_k"), py::arg("residual") = py::none());
   m.def("combine_wgrad", &combine_wgrad);
-  m.def("attention_fwd", &attention_fwd);
-  m.def("attention_bwd", &attention_bwd);
+  m.def("attention_fwd", &attention_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("cu_seqlens"), py::arg("max_seqlen"), py::arg("scale"),
+        py::arg("status") = py::none());
+  m.def("attention_bwd", &attention_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("dout"), py::arg("lse"), py::arg("cu_seqlens"),
+        py::arg("max_seqlen"), py::arg("scale"), py::arg("status") = py::none());
   m.def("ep_counts_send", &ep_counts_send);
   m.def("ep_counts_wait_meta", &ep_counts_wait_meta);
   m.def("ep_dispatch", &ep_dispatch, py::arg("x"), py::arg("src_slot"), py::arg("expert_of_slot"), py::arg("slot_scale"), py::arg("meta"),

@@ -46,18 +46,18 @@ def _sdpa_attention(q, k, v, cu_seqlens, max_seqlen=None):
 class _Attention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cu_seqlens, max_seqlen, scale):
-        from .cuda_ops import ext
+        from .cuda_ops import ext, status_tensor
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o, lse = ext.attention_fwd(q, k, v, cu_seqlens, max_seqlen, scale)
+        o, lse = ext.attention_fwd(q, k, v, cu_seqlens, max_seqlen, scale, status_tensor(q.device))
         ctx.save_for_backward(q, k, v, o, lse, cu_seqlens)
         ctx.max_seqlen, ctx.scale = max_seqlen, scale
         return o
 
     @staticmethod
     def backward(ctx, dout):
-        from .cuda_ops import ext
+        from .cuda_ops import ext, status_tensor
         q, k, v, o, lse, cu = ctx.saved_tensors
-        dq, dk, dv = ext.attention_bwd(q, k, v, o, dout.contiguous(), lse, cu, ctx.max_seqlen, ctx.scale)
+        dq, dk, dv = ext.attention_bwd(q, k, v, o, dout.contiguous(), lse, cu, ctx.max_seqlen, ctx.scale, status_tensor(q.device))
         return dq, dk, dv, None, None, None
 
 

@@ -28,7 +28,8 @@ _status = {}
 
 
 def status_tensor(device) -> torch.Tensor:
-    """Per-device int32 word that kernels set when one of their bounded waits gives up."""
+    """Per-device int32 word that kernels set when one of their bounded waits gives up, or when sizes on the device do not
+    fit the buffers."""
     key = torch.device(device).index or 0
     if key not in _status:
         _status[key] = torch.zeros(1, dtype=torch.int32, device=device)
@@ -39,7 +40,7 @@ def check_status(device) -> None:
     code = int(status_tensor(device).item())
     if code != 0:
         status_tensor(device).zero_()
-        raise RuntimeError(f"a kernel reported a wait that ran out of time (status code {code})")
+        raise RuntimeError(f"a kernel reported a wait that ran out of time, or sizes that do not fit (status code {code})")
 
 
 def launch_count() -> int:

@@ -85,7 +85,7 @@ class _AttentionBlock(torch.autograd.Function):
         kr = ext.rope(k.view(T, Hkv, d), positions, theta, False)
         v3 = v.view(T, Hkv, d)
         scale = float(d) ** -0.5
-        o, lse = ext.attention_fwd(qr, kr, v3, cu, max_seqlen, scale)
+        o, lse = ext.attention_fwd(qr, kr, v3, cu, max_seqlen, scale, C.status_tensor(x2.device))
         o2 = o.view(T, Hq * d)
         out, to = _lin_fwd(o2, *lins[3][:4], residual=x2)      # + x in the GEMM's epilogue
         if any(ctx.needs_input_grad):
@@ -123,7 +123,7 @@ class _AttentionBlock(torch.autograd.Function):
         o2 = o.view(T, Hq * d)
         d_o = run(3, dy2, o2, to)
         scale = float(d) ** -0.5
-        dq, dk, dv = ext.attention_bwd(qr, kr, v3, o, d_o.view(T, Hq, d), lse, cu, max_seqlen, scale)
+        dq, dk, dv = ext.attention_bwd(qr, kr, v3, o, d_o.view(T, Hq, d), lse, cu, max_seqlen, scale, C.status_tensor(x2.device))
         dq = ext.rope(dq, positions, theta, True).view(T, Hq * d)
         dk = ext.rope(dk, positions, theta, True).view(T, Hkv * d)
         d_xn = run(0, dq, xn, tq)

@@ -638,6 +638,36 @@ def test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("bounds", [[0, 150, 300], [0, 150, 40000], [0, 150, 200, 90, 260]])
+def test_attention_reports_sequences_outside_its_rows(ops, bounds):
+    """cu_seqlens that go past the tensors (by a little, by far, or on a detour): what lies outside is left out and the status
+    word says so, in the forward and in the backward pass; the sequence inside is as without the others."""
+    from moe_distributed_training_b200.ops.attention_cuda import attention
+    torch.manual_seed(83)
+    T, n = 200, 150
+    q, k, v, do = (_rand(T, h, 128) for h in (4, 2, 2, 4))
+    for t in (q, k, v):
+        t.requires_grad_(True)
+
+    def cu(values):
+        return torch.tensor(values, dtype=torch.int32, device=DEV)
+    want = attention(q, k, v, cu([0, n, T]), T)
+    want_grads = torch.autograd.grad(want, (q, k, v), do)
+    ops.check_status(DEV)
+    with torch.no_grad():
+        got = attention(q, k, v, cu(bounds), T)
+        with pytest.raises(RuntimeError, match="status code 7"):
+            ops.check_status(DEV)
+        lse = ops.ext.attention_fwd(q, k, v, cu([0, n, T]), T, 128 ** -0.5)[1]
+        grads = ops.ext.attention_bwd(q, k, v, want, do, lse, cu(bounds), T, 128 ** -0.5, ops.status_tensor(DEV))
+    with pytest.raises(RuntimeError, match="status code 7"):
+        ops.check_status(DEV)
+    if max(bounds) > 260:
+        assert torch.equal(got[:n], want[:n])
+        for a, b in zip(grads, want_grads):
+            _close(a[:n].flatten(1), b[:n].flatten(1), 1e-3)
+
+
 @pytest.mark.parametrize("lora", [False, True])
 def test_fused_attention_block_matches_composed_ops(ops, lora):
     """The single-node attention sub-block against the same layer evaluated op by op."""
