@@ -66,7 +66,8 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 __device__ __forceinline__ int blocks_of(int seq_start, int seq_end, int tokens) {
   return seq_start >= 0 && seq_end > seq_start && seq_end <= tokens ? (seq_end - seq_start + AB - 1) / AB : 0;
 }
-// Locate block `flat` of the 128-row blocks over all sequences: its sequence (-1: there is no such block) and its place there.
+// Locate block `flat` of the 128-row blocks over all sequences: its sequence (-1: there is no such block, and blk is its number
+// past the last one) and its place there.
 // Grids have at least one block more than the sequences do; the CTA that comes past the last one reports (`status`, optional)
 // sequences that were left out because they reach outside the tensors.
 __device__ __forceinline__ int find_block(const int* cu, int num_seqs, int tokens, int flat, int& seq_start, int& seq_end, int& blk, int* status) {
@@ -79,6 +80,7 @@ __device__ __forceinline__ int find_block(const int* cu, int num_seqs, int token
     flat -= nb;
   }
   if (outside && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, ST_CAPACITY);
+  blk = flat;
   return -1;
 }
 
@@ -844,15 +846,29 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
 }
 
 // dQ: tiles [column / 4][row][4] -> bf16 rows, one CTA per (block, head).  dK, dV (`sets` partial sums per kv head, when
-// there are several): the CTAs past the blocks, summed and converted eight columns at a time.
+// there are several): the CTAs past the blocks, summed and converted eight columns at a time.  Rows before the first and
+// after the last sequence get zeros, from the CTAs that have no block.
 __global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __restrict__ dq32, const float* __restrict__ dk32, const float* __restrict__ dv32,
                                                                 bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
                                                                 const int* __restrict__ cu, int num_seqs, int blocks, int tokens, int heads_q,
                                                                 int heads_kv, int sets) {
+  const int first = num_seqs > 0 ? min(max(cu[0], 0), tokens) : 0, end = num_seqs > 0 ? min(max(cu[num_seqs], first), tokens) : 0;
   if ((int)blockIdx.x < blocks) {
     int seq_start, seq_end, blk;
-    if (find_block(cu, num_seqs, tokens, blockIdx.x, seq_start, seq_end, blk, nullptr) < 0) return;
     const int h = blockIdx.y;
+    if (find_block(cu, num_seqs, tokens, blockIdx.x, seq_start, seq_end, blk, nullptr) < 0) {
+      const int idle = blocks - ((int)blockIdx.x - blk), sub = threadIdx.x & 15;         // CTAs like this one, per head
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      for (int u = blk * 16 + (threadIdx.x >> 4); u < first + tokens - end; u += idle * 16) {
+        const long long row = u < first ? u : end + (u - first);
+        reinterpret_cast<uint4*>(dq + (row * heads_q + h) * HD)[sub] = zero;
+        if (dk32 == nullptr && h < heads_kv) {
+          reinterpret_cast<uint4*>(dk + (row * heads_kv + h) * HD)[sub] = zero;
+          reinterpret_cast<uint4*>(dv + (row * heads_kv + h) * HD)[sub] = zero;
+        }
+      }
+      return;
+    }
     const float4* src = reinterpret_cast<const float4*>(dq32 + ((long long)blockIdx.x * heads_q + h) * DQ_TILE);
     // eight lanes x 4 columns = 64 bytes of a row of dq, four rows per warp and pass; all loads in flight at once
     const int cg = threadIdx.x & 7, rsub = threadIdx.x >> 3;
@@ -877,7 +893,8 @@ __global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __r
     const long long th = v / (HD / 8);                                   // token * heads_kv + kv head
     const float* src = (isv ? dv32 : dk32) + (th * per) * HD + d;
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int g = 0; g < per; ++g) {
+    const long long row = th / heads_kv;
+    for (int g = 0; g < per && row >= first && row < end; ++g) {
       const float4 a = *reinterpret_cast<const float4*>(src + (long long)g * HD), b = *reinterpret_cast<const float4*>(src + (long long)g * HD + 4);
       s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w; s[4] += b.x; s[5] += b.y; s[6] += b.z; s[7] += b.w;
     }

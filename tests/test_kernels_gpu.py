@@ -638,6 +638,28 @@ def test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("T,first,end,heads,kv", [(512, 5, 300, 4, 4), (512, 5, 300, 32, 8), (700, 0, 1, 8, 2), (300, 290, 300, 4, 2), (4000, 1000, 1600, 4, 1)])
+def test_attention_gradients_of_rows_outside_the_sequences_are_zero(ops, T, first, end, heads, kv):
+    """Rows before the first and after the last sequence (a padded stream) get zero gradients, whatever the memory held, with
+    dK / dV added up in one CTA and over partial sums; the rows inside are those of the call without the padding."""
+    torch.manual_seed(T + first)
+    q, k, v, do = (_rand(T, h, 128) for h in (heads, kv, kv, heads))
+
+    def cu(*values):
+        return torch.tensor(values, dtype=torch.int32, device=DEV)
+    o, lse = ops.ext.attention_fwd(q, k, v, cu(first, end), T, 128 ** -0.5)
+    poison = [torch.full((T * h * 128 * mult,), float("nan"), dtype=dt, device=DEV)
+              for h in (heads, kv, kv) for mult, dt in ((1, torch.bfloat16), (1, torch.float32), (3, torch.float32))]
+    del poison                                   # what the next allocations find
+    grads = ops.ext.attention_bwd(q, k, v, o, do, lse, cu(first, end), T, 128 ** -0.5, ops.status_tensor(DEV))
+    inside = [t[first:end].contiguous() for t in (q, k, v, o, do, lse)]
+    ref = ops.ext.attention_bwd(*inside, cu(0, end - first), end - first, 128 ** -0.5, ops.status_tensor(DEV))
+    for name, a, b in zip(("dq", "dk", "dv"), grads, ref):
+        assert bool((a[:first] == 0).all()) and bool((a[end:] == 0).all()), name
+        assert float((a[first:end].float() - b.float()).norm()) <= 1e-2 * float(b.float().norm()) + 1e-3, name
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("bounds", [[0, 150, 300], [0, 150, 40000], [0, 150, 200, 90, 260]])
 def test_attention_reports_sequences_outside_its_rows(ops, bounds):
     """cu_seqlens that go past the tensors (by a little, by far, or on a detour): what lies outside is left out and the status
