@@ -14,6 +14,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include <stdlib.h>
@@ -486,13 +487,17 @@ constexpr int BWD_THREADS = 512;
 constexpr int BWD_STATS = 2 * AB;                              // lse2 | delta of a block, floats
 constexpr int BWD_SMEM = 7 * TILE_BYTES + 2 * BWD_STATS * 4 + 256 + 768;   // (768: what alignment to 1024 may take)
 static_assert(BWD_SMEM <= 227 * 1024, "attention backward: shared memory of a CTA");
-constexpr int DQ_TILE = AB * HD;                               // fp32 elements, [column / 4][row][4]
+// The fp32 dQ of a (block, query head) is a tile [column / 4][row][4] of the rows that the block has: a sequence's last block
+// takes no more room, clearing or reading back than its rows, which is what many short sequences consist of (1024 sequences
+// of 8 tokens, 32 heads, in whole tiles of 128 rows: 2.3 GB).
+__device__ __forceinline__ int rows_of_block(int row0, int seq_end) { return min(AB, seq_end - row0); }
+__device__ __forceinline__ long long dq_tile(int row0, int rows, int heads, int h) { return ((long long)row0 * heads + (long long)h * rows) * HD; }
 
 struct AttnBwdParams {
   CUtensorMap tmQ, tmK, tmV, tmdO;
   const int4* sched;            // by rank: {seq_start, seq_end, block, flat block}; seq_start < 0: none
   const float* stats;           // [flat block][head][lse2 x 128 | delta x 128]
-  float* dq;                    // [flat block][head] tiles
+  float* dq;                    // tiles, see dq_tile
   float* dk; float* dv;         // fp32 partial sums [token][head set][128], or NULL: all heads of a kv head in one CTA
   bf16* dk_out; bf16* dv_out;   // then the results [token][kv head][128]
   int heads_q, heads_kv, hpc;   // hpc: query heads per CTA
@@ -501,7 +506,7 @@ struct AttnBwdParams {
   int* status;
 };
 
-__global__ void __launch_bounds__(256) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
+__global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
                                                                const int* __restrict__ cu, int num_seqs, int tokens, int heads, int4* __restrict__ sched,
                                                                float* __restrict__ stats, float* __restrict__ dq, int* status) {
   int seq_start, seq_end, blk;
@@ -528,24 +533,24 @@ __global__ void __launch_bounds__(256) attn_bwd_prepare_kernel(const bf16* __res
   const long long tile = (long long)flat * heads + h;
   // 16 lanes x 16 bytes hold a row, 16 rows per pass; all loads of the block are in flight at once
   const int sub = lane & 15, r0 = warp * 2 + (lane >> 4);
+  const int row0 = seq_start + blk * AB, rows = rows_of_block(row0, seq_end);
   uint4 a[8], b[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    const long long row = (long long)(seq_start + blk * AB + k * 16 + r0);
-    const bool valid = row < seq_end;
-    const long long at = ((valid ? row : (long long)seq_start) * heads + h) * HD;
+    const int r = k * 16 + r0;
+    const long long at = ((long long)(row0 + (r < rows ? r : 0)) * heads + h) * HD;     // (past the end: one row again and again)
     a[k] = reinterpret_cast<const uint4*>(o + at)[sub];
     b[k] = reinterpret_cast<const uint4*>(dout + at)[sub];
   }
-  float4* z = reinterpret_cast<float4*>(dq + tile * DQ_TILE);
-#pragma unroll 8
-  for (int i = threadIdx.x; i < DQ_TILE / 4; i += 256) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4* z = reinterpret_cast<float4*>(dq + dq_tile(row0, rows, heads, h));
+#pragma unroll 4
+  for (int i = threadIdx.x; i < rows * (HD / 4); i += 256) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   float* st = stats + tile * BWD_STATS;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int r = k * 16 + r0;
-    const long long row = (long long)(seq_start + blk * AB + r);
-    const bool valid = row < seq_end;
+    const long long row = row0 + r;
+    const bool valid = r < rows;
     const __nv_bfloat162* pa = reinterpret_cast<const __nv_bfloat162*>(&a[k]);
     const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&b[k]);
     float s = 0.f;
@@ -706,7 +711,9 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
     for (int it = 0; it < n_it; ++it) {
       if (!wait_parity_warp(bardQ, it & 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
       tc_fence_after();
-      float* dst = p.dq + ((long long)(work.w + i) * p.heads_q + h0 + head) * DQ_TILE + (warp * 32 + lane) * 4;
+      const int q0 = seq_start + (kb + i) * AB, rows = rows_of_block(q0, seq_end);
+      const bool valid = warp * 32 + lane < rows;
+      float* dst = p.dq + dq_tile(q0, rows, p.heads_q, h0 + head) + (warp * 32 + lane) * 4;
 #pragma unroll 1
       for (int c = 0; c < HD; c += 64) {
         uint32_t a[32], b[32];
@@ -718,12 +725,17 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
           __syncwarp();
           if (lane == 0) mbar_arrive(bardQfree);
         }
+        auto add = [&](int step) {       // floats from one group of four columns to the next
 #pragma unroll
-        for (int x = 0; x < 32; x += 4)
-          red_add_v4_f32(dst + ((c + x) >> 2) * (AB * 4), __uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
+          for (int x = 0; x < 32; x += 4)
+            red_add_v4_f32(dst + ((c + x) >> 2) * step, __uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
 #pragma unroll
-        for (int x = 0; x < 32; x += 4)
-          red_add_v4_f32(dst + ((c + 32 + x) >> 2) * (AB * 4), __uint_as_float(b[x]), __uint_as_float(b[x + 1]), __uint_as_float(b[x + 2]), __uint_as_float(b[x + 3]));
+          for (int x = 0; x < 32; x += 4)
+            red_add_v4_f32(dst + ((c + 32 + x) >> 2) * step, __uint_as_float(b[x]), __uint_as_float(b[x + 1]), __uint_as_float(b[x + 2]), __uint_as_float(b[x + 3]));
+        };
+        if (rows == AB) add(AB * 4);     // (offsets in the instructions: 2 % of the loop at 16384 tokens)
+        else if (valid) add(rows * 4);
+        __syncwarp();
       }
       if (++i == nq) { i = 0; ++head; }
     }
@@ -869,17 +881,21 @@ __global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __r
       }
       return;
     }
-    const float4* src = reinterpret_cast<const float4*>(dq32 + ((long long)blockIdx.x * heads_q + h) * DQ_TILE);
+    const int row0 = seq_start + blk * AB, rows = rows_of_block(row0, seq_end);
+    const float4* src = reinterpret_cast<const float4*>(dq32 + dq_tile(row0, rows, heads_q, h));
     // eight lanes x 4 columns = 64 bytes of a row of dq, four rows per warp and pass; all loads in flight at once
     const int cg = threadIdx.x & 7, rsub = threadIdx.x >> 3;
     float4 v[16];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = __ldcs(src + ((k & 3) * 8 + cg) * AB + (k >> 2) * 32 + rsub);
+    for (int k = 0; k < 16; ++k) {
+      const int r = (k >> 2) * 32 + rsub;
+      if (r < rows) v[k] = __ldcs(src + ((k & 3) * 8 + cg) * rows + r);
+    }
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
-      const long long row = seq_start + blk * AB + (k >> 2) * 32 + rsub;
-      if (row < seq_end)
-        *reinterpret_cast<uint2*>(dq + (row * heads_q + h) * HD + ((k & 3) * 8 + cg) * 4) = make_uint2(pack2(v[k].x, v[k].y), pack2(v[k].z, v[k].w));
+      const int r = (k >> 2) * 32 + rsub;
+      if (r < rows)
+        *reinterpret_cast<uint2*>(dq + ((long long)(row0 + r) * heads_q + h) * HD + ((k & 3) * 8 + cg) * 4) = make_uint2(pack2(v[k].x, v[k].y), pack2(v[k].z, v[k].w));
     }
     return;
   }
@@ -976,10 +992,11 @@ BwdPlan bwd_plan(int num_seqs, int total_tokens, int max_seqlen, int heads_q, in
   BwdPlan b;
   b.blocks = ((long long)total_tokens + AB - 1) / AB + num_seqs;
   // A CTA that takes all query heads of a kv head adds their dK, dV in TMEM and writes bf16; but its loop is that much
-  // longer.  The longest loop may be half of an SM's share of all iterations (sequences taken as equally long), else
+  // longer.  The longest loop may be half of an SM's share of all iterations (sequences taken as equally long, one block at
+  // least), else
   // fewer heads per CTA: 613 tokens, 32 / 8 heads run with one head (160 CTAs), four sequences of 1024-8192 with all four.
   const int group = heads_q / heads_kv;
-  const double seqs = num_seqs > 0 ? num_seqs : 1, n = (double)total_tokens / (AB * seqs);
+  const double seqs = num_seqs > 0 ? num_seqs : 1, n = fmax((double)total_tokens / (AB * seqs), 1.0);
   const double share = seqs * n * (n + 1.0) / 2.0 * heads_q / sm_count_of_current_device();
   const int longest = ((max_seqlen < total_tokens ? max_seqlen : total_tokens) + AB - 1) / AB;
   b.hpc = group;
@@ -987,7 +1004,7 @@ BwdPlan bwd_plan(int num_seqs, int total_tokens, int max_seqlen, int heads_q, in
   b.sets = heads_q / b.hpc;
   b.off_stats = (b.blocks * 4 + 31) / 32 * 32;                                   // after the schedule
   b.off_dq = b.off_stats + b.blocks * heads_q * BWD_STATS;
-  b.off_dk = b.off_dq + b.blocks * heads_q * DQ_TILE;
+  b.off_dk = b.off_dq + (long long)total_tokens * heads_q * HD;
   const long long part = b.hpc == group ? 0 : (long long)total_tokens * b.sets * HD;
   b.off_dv = b.off_dk + part;
   b.floats = b.off_dv + part;

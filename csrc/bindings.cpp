@@ -943,6 +943,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("combine_wgrad", &combine_wgrad);
   m.def("attention_fwd", &attention_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("cu_seqlens"), py::arg("max_seqlen"), py::arg("scale"),
         py::arg("status") = py::none());
+  m.def("attention_bwd_scratch", [](int64_t num_seqs, int64_t tokens, int64_t max_seqlen, int64_t heads_q, int64_t heads_kv) {   // floats
+    return (int64_t)mdt_attention_bwd_scratch((int)num_seqs, (int)tokens, (int)max_seqlen, (int)heads_q, (int)heads_kv);
+  });
   m.def("attention_bwd", &attention_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("o"), py::arg("dout"), py::arg("lse"), py::arg("cu_seqlens"),
         py::arg("max_seqlen"), py::arg("scale"), py::arg("status") = py::none());
   m.def("ep_counts_send", &ep_counts_send);

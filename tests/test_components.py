@@ -275,6 +275,23 @@ def test_gemm_default_tiling_follows_rounds_and_row_groups():
     assert pair(2, 14336, 4096, 0, G=8, tokens=9200, acc=True)
 
 
+@pytest.mark.parametrize("seqs,length", [(1, 1), (1, 613), (4, 4375), (40, 130), (1024, 8), (4096, 1), (300, 129)])
+@pytest.mark.parametrize("heads,kv", [(32, 8), (8, 8), (4, 1)])
+def test_attention_backward_scratch_grows_with_tokens_not_with_sequences(seqs, length, heads, kv):
+    """At most fp32 dQ, dK and dV of every (token, query head) plus the row statistics (256 floats per block and head) and
+    the schedule, however short the sequences are."""
+    build = pytest.importorskip("moe_distributed_training_b200.ops.build")
+    try:
+        ext = build.load()
+    except Exception:  # noqa: BLE001
+        pytest.skip("extension not built")
+    T = seqs * length
+    blocks = (T + 127) // 128 + seqs
+    floats = ext.attention_bwd_scratch(seqs, T, length, heads, kv)
+    assert floats <= 3 * 128 * T * heads + 256 * blocks * heads + 4 * blocks + 32
+    assert floats <= 1.01 * (1 + 3 * 128) * T * heads + 256 * 2 * heads + 64
+
+
 def test_profile_trace_flag_writes_a_trace(tmp_path):
     from moe_distributed_training_b200.train.run import run_training
     out = tmp_path / "traces"

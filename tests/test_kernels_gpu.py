@@ -638,6 +638,12 @@ def test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("lens,heads,kv", [([8] * 200, 8, 2), ([1, 3, 0, 127, 2] * 30, 4, 2), ([64, 200] * 10, 4, 4)])
+def test_attention_many_short_sequences(ops, lens, heads, kv):
+    """Blocks with few rows: their dQ tiles take just those rows, and neighbours must not touch."""
+    test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv)
+
+
 @pytest.mark.parametrize("T,first,end,heads,kv", [(512, 5, 300, 4, 4), (512, 5, 300, 32, 8), (700, 0, 1, 8, 2), (300, 290, 300, 4, 2), (4000, 1000, 1600, 4, 1)])
 def test_attention_gradients_of_rows_outside_the_sequences_are_zero(ops, T, first, end, heads, kv):
     """Rows before the first and after the last sequence (a padded stream) get zero gradients, whatever the memory held, with
