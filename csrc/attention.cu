@@ -68,19 +68,35 @@ __device__ __forceinline__ int blocks_of(int seq_start, int seq_end, int tokens)
   return seq_start >= 0 && seq_end > seq_start && seq_end <= tokens ? (seq_end - seq_start + AB - 1) / AB : 0;
 }
 // Locate block `flat` of the 128-row blocks over all sequences: its sequence (-1: there is no such block, and blk is its number
-// past the last one) and its place there.
+// past the last one) and its place there.  Called by whole warps: 32 sequences at a time, a scan over their block counts
+// (one sequence after the other, each step waiting for its bounds, a CTA of 1024 sequences took 70 us to find its block).
 // Grids have at least one block more than the sequences do; the CTA that comes past the last one reports (`status`, optional)
 // sequences that were left out because they reach outside the tensors.
 __device__ __forceinline__ int find_block(const int* cu, int num_seqs, int tokens, int flat, int& seq_start, int& seq_end, int& blk, int* status) {
+  const int lane = threadIdx.x & 31;
   bool outside = false;
-  for (int s = 0; s < num_seqs; ++s) {
-    const int a = cu[s], b = cu[s + 1];
+  for (int s0 = 0; s0 < num_seqs; s0 += 32) {
+    const bool live = s0 + lane < num_seqs;
+    const int a = live ? cu[s0 + lane] : 0, b = live ? cu[s0 + lane + 1] : 0;
     const int nb = blocks_of(a, b, tokens);
-    if (flat < nb) { seq_start = a; seq_end = b; blk = flat; return s; }
     outside = outside || (nb == 0 && b > a);
-    flat -= nb;
+    int upto = nb;                               // blocks of the window's sequences up to this lane's
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, off);
+      if (lane >= off) upto += v;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, flat < upto);
+    if (past != 0) {
+      const int l = __ffs(past) - 1;
+      seq_start = __shfl_sync(0xffffffffu, a, l);
+      seq_end = __shfl_sync(0xffffffffu, b, l);
+      blk = flat - __shfl_sync(0xffffffffu, upto - nb, l);
+      return s0 + l;
+    }
+    flat -= __shfl_sync(0xffffffffu, upto, 31);
   }
-  if (outside && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, ST_CAPACITY);
+  if (__any_sync(0xffffffffu, outside) && threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, ST_CAPACITY);
   blk = flat;
   return -1;
 }

@@ -638,9 +638,11 @@ def test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv):
     ops.check_status(DEV)
 
 
-@pytest.mark.parametrize("lens,heads,kv", [([8] * 200, 8, 2), ([1, 3, 0, 127, 2] * 30, 4, 2), ([64, 200] * 10, 4, 4)])
+@pytest.mark.parametrize("lens,heads,kv", [([8] * 200, 8, 2), ([1, 3, 0, 127, 2] * 30, 4, 2), ([64, 200] * 10, 4, 4),
+                                           ([5] * 31, 4, 2), ([150] * 32, 4, 2), ([9] * 33, 2, 1), ([0] * 40 + [300, 0, 20], 4, 2), ([130, 0] * 33, 2, 2)])
 def test_attention_many_short_sequences(ops, lens, heads, kv):
-    """Blocks with few rows: their dQ tiles take just those rows, and neighbours must not touch."""
+    """Blocks with few rows: their dQ tiles take just those rows, and neighbours must not touch.  Blocks are looked up 32
+    sequences at a time: one window less one, one, one more, and windows of empty sequences."""
     test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv)
 
 
