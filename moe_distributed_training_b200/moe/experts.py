@@ -35,18 +35,27 @@ class _GradTargets:
     """Where the weight-gradient kernels put the gradients of w1, w2, w3: straight into `.grad`.
 
     A buffer is created when the backward pass asks for it, not cleared in the forward pass: the first gradient is then
-    written instead of added to zeros (three passes over all expert weights less per optimizer step).
+    written instead of added to zeros (three passes over all expert weights less per optimizer step).  It becomes `.grad`
+    with `publish`, once the products that write it have been launched: a backward pass that fails before that (out of
+    memory, a refused launch) leaves no `.grad` of uninitialised memory behind.
     """
 
     def __init__(self, params, shape):
         self.params, self.shape = params, shape
+        self._fresh = {}
 
     def target(self, i: int):
-        p = self.params[i]
-        fresh = p.grad is None
-        if fresh:
-            p.grad = torch.empty_like(p)
-        return p.grad.view(self.shape), not fresh
+        """The buffer for parameter i's gradient and whether it holds one already (the product is then added to it)."""
+        grad = self.params[i].grad
+        if grad is not None:
+            return grad.view(self.shape), True
+        self._fresh[i] = torch.empty_like(self.params[i])
+        return self._fresh[i].view(self.shape), False
+
+    def publish(self):
+        fresh, self._fresh = self._fresh, {}
+        for i, grad in fresh.items():
+            self.params[i].grad = grad
 
 
 class SparseMLPv2(nn.Module):

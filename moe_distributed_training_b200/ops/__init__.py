@@ -82,8 +82,8 @@ def grouped_swiglu_mlp(xg, w1, w2, w3, plan: RoutingPlan, lora=None, wgrad_scale
     """Expert MLP over block-padded groups; w1, w2, w3 are [E_local, F, H].
 
     wgrad_out: optional object whose target(i) gives the buffer for the gradient of w1, w2 or w3 and whether the CUDA
-    kernels add to it or write it
-    directly (no gradient tensor is returned for the weights then)."""
+    kernels add to it or write it, and whose publish() is called once all of them are launched (no gradient tensor is
+    returned for the weights then)."""
     if _native(xg):
         return _cuda().grouped_swiglu_mlp(xg, w1, w2, w3, plan, lora, wgrad_scale, wgrad_out)
     return reference.grouped_swiglu_mlp(xg, w1, w2, w3, plan.padded_offsets, plan.tokens_per_expert, lora, wgrad_scale)

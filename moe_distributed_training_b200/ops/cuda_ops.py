@@ -331,6 +331,7 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
             if wg is not None:
                 out, add = wg.target(0); _g(2, dg, True, xg, True, out, H, 0, plan, alpha=ws, accumulate=add)
                 out, add = wg.target(2); _g(2, du, True, xg, True, out, H, 0, plan, alpha=ws, accumulate=add)
+                wg.publish()
             else:
                 dw1 = torch.empty_like(w1); _g(2, dg, True, xg, True, dw1, H, 0, plan, alpha=ws)
                 dw3 = torch.empty_like(w3); _g(2, du, True, xg, True, dw3, H, 0, plan, alpha=ws)

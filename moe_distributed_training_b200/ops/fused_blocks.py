@@ -366,6 +366,8 @@ class _MoEBlockNative(torch.autograd.Function):
         dx, dln, dWr = ext.moe_block_bwd(dy, state, x2, ln_w, Wr.contiguous(), w1, w2, w3, [t for t, _ in targets], [add for _, add in targets],
                                          ctx.ws, a.moe_top_k, a.moe_num_experts,
                                          layout, ints, tens, C.status_tensor(dy.device), bool(need[2]), bool(need[3]))
+        if ctx.wgrad_out is not None:
+            ctx.wgrad_out.publish()
         return dx, None, (dln if need[2] else None), (dWr if need[3] else None), None, None, None
 
 

@@ -292,6 +292,52 @@ def test_attention_backward_scratch_grows_with_tokens_not_with_sequences(seqs, l
     assert floats <= 1.01 * (1 + 3 * 128) * T * heads + 256 * 2 * heads + 64
 
 
+def test_expert_gradient_buffers_become_grad_only_once_they_are_written(monkeypatch):
+    """A backward pass that fails before its weight-gradient products are launched leaves `.grad` as it was; one that
+    succeeds hands over exactly the buffers that it wrote, and the next one adds to them."""
+    from types import SimpleNamespace
+    from moe_distributed_training_b200.moe.experts import _GradTargets
+    pytest.importorskip("moe_distributed_training_b200.ops.build")
+    try:
+        from moe_distributed_training_b200.ops import fused_blocks
+    except RuntimeError:
+        pytest.skip("extension not built")
+    params = [torch.nn.Parameter(torch.randn(6, 4)) for _ in range(3)]
+    params[1].grad = torch.ones(6, 4)
+    seen = []
+
+    class Ext:
+        fail = True
+
+        def moe_block_bwd(self, dy, state, x, ln, wr, w1, w2, w3, wg, add, *rest):
+            assert [p.grad is None for p in params] == ([True, False, True] if not seen else [False] * 3)
+            assert add == ([False, True, False] if not seen else [True] * 3)
+            if self.fail:
+                raise RuntimeError("out of memory")
+            for i, (buf, more) in enumerate(zip(wg, add)):
+                assert buf.shape == (2, 3, 4)
+                buf.add_(i + 2.0) if more else buf.fill_(i + 2.0)
+            seen.append(wg)
+            return dy, None, None
+    monkeypatch.setattr(fused_blocks, "ext", Ext())
+    monkeypatch.setattr(fused_blocks.C, "status_tensor", lambda device: None)
+    args = SimpleNamespace(moe_top_k=1, moe_num_experts=2)
+    ctx = SimpleNamespace(layer=SimpleNamespace(block_sparse_moe=SimpleNamespace(args=args)), eng=None, ws=1.0, views=(None,) * 3,
+                          wgrad_out=_GradTargets(params, (2, 3, 4)), saved_tensors=[torch.zeros(5, 4)] * 3,
+                          needs_input_grad=[True, False, False, False])
+
+    def backward():
+        fused_blocks._MoEBlockNative.backward(ctx, torch.zeros(5, 4))
+    with pytest.raises(RuntimeError, match="out of memory"):
+        backward()
+    assert params[0].grad is None and params[2].grad is None and bool((params[1].grad == 1).all())
+    Ext.fail = False
+    backward()
+    assert [float(p.grad.mean()) for p in params] == [2.0, 1.0 + 3.0, 4.0]
+    backward()
+    assert [float(p.grad.mean()) for p in params] == [4.0, 1.0 + 6.0, 8.0]
+
+
 def test_profile_trace_flag_writes_a_trace(tmp_path):
     from moe_distributed_training_b200.train.run import run_training
     out = tmp_path / "traces"
