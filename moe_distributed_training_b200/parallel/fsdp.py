@@ -555,11 +555,11 @@ class ShardedMixtral:
             return
         scale = 1.0 / (self.ws * self.rep)
         if self.ws == 1:
-            # nothing to reduce: straight into the gradient of the flat parameter, written the first time
+            # nothing to reduce: straight into the gradient of the flat parameter, written the first time (and published
+            # when it is complete: a failure on the way leaves no uninitialised memory behind)
             fresh = g.shard.grad is None
-            if fresh:
-                g.shard.grad = torch.empty_like(g.shard.data)
-            flat, dst, src, end = g.shard.grad, [], [], 0
+            flat = torch.empty_like(g.shard.data) if fresh else g.shard.grad
+            dst, src, end = [], [], 0
             for (mod, name, shape, n, o), gr in zip(g.specs, grads):
                 if fresh and end < o:
                     flat[end:o].zero_()                                      # alignment gaps
@@ -577,6 +577,8 @@ class ShardedMixtral:
                         flat.mul_(scale)
                 else:
                     torch._foreach_add_(dst, src, alpha=scale)
+            if fresh:
+                g.shard.grad = flat
         elif self.sync_each_batch:
             # double-buffered flat gradient: the reduction of one block runs on the side stream while the next block's
             # backward fills the other buffer

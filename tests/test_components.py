@@ -338,6 +338,47 @@ def test_expert_gradient_buffers_become_grad_only_once_they_are_written(monkeypa
     assert [float(p.grad.mean()) for p in params] == [4.0, 1.0 + 6.0, 8.0]
 
 
+def test_one_rank_flat_gradient_equals_the_accumulated_one(monkeypatch):
+    """Parameters whose sizes leave alignment gaps, one that gets no gradient in the first micro-batch and one in none, over
+    three micro-batches: the flat gradient is the sum that clearing and adding gives, gaps and tail are zero, and a failure
+    while it is first filled leaves it unset."""
+    from types import SimpleNamespace
+    from moe_distributed_training_b200.parallel import fsdp
+    torch.manual_seed(3)
+    mod = torch.nn.Module()
+    shapes = [(3, 5), (7,), (16, 8), (1,), (11, 3)]
+    for i, s in enumerate(shapes):
+        mod.register_parameter(f"p{i}", torch.nn.Parameter(torch.randn(s)))
+    group = fsdp.FlatParamGroup([(mod, f"p{i}", mod._parameters[f"p{i}"], f"layer.p{i}") for i in range(len(shapes))], None, True)
+    runner = SimpleNamespace(ws=1, rep=2, sync_each_batch=True)
+    unit = SimpleNamespace(trainable_group=group)
+
+    def grads(used):
+        return [torch.randn(s, dtype=torch.float64 if i == 4 else torch.float32) if i in used else None for i, s in enumerate(shapes)]
+    batches = [grads({0, 1, 4}), grads({0, 1, 2, 4}), grads({1, 2})]
+
+    def failing(dst, src):
+        raise RuntimeError("out of memory")
+    with monkeypatch.context() as m:
+        m.setattr(torch, "_foreach_copy_", failing)
+        with pytest.raises(RuntimeError, match="out of memory"):
+            fsdp.ShardedMixtral._reduce_unit_grads(runner, unit, batches[0])
+    assert group.shard.grad is None
+    want = torch.zeros_like(group.shard.data)
+    for batch in batches:
+        fsdp.ShardedMixtral._reduce_unit_grads(runner, unit, batch)
+        for (_, _, shape, n, o), gr in zip(group.specs, batch):
+            if gr is not None:
+                want[o:o + n] += 0.5 * gr.reshape(-1).float()
+        torch.testing.assert_close(group.shard.grad, want, rtol=1e-6, atol=1e-6)
+    covered = torch.zeros_like(want, dtype=torch.bool)
+    for _, _, _, n, o in group.specs:
+        covered[o:o + n] = True
+    assert int((~covered).sum()) > 0 and bool((group.shard.grad[~covered] == 0).all())
+    (_, _, _, n, o) = next(sp for sp in group.specs if sp[1] == "p3")
+    assert bool((group.shard.grad[o:o + n] == 0).all())
+
+
 def test_profile_trace_flag_writes_a_trace(tmp_path):
     from moe_distributed_training_b200.train.run import run_training
     out = tmp_path / "traces"
