@@ -516,6 +516,6 @@ def attention(q, k, v, cu_seqlens, max_seqlen=None):
 
 
 def adamw_multi(ps, gs, ms, vs, lr, b1, b2, eps, wd, step, grad_scale=1.0):
-    """grad_scale: a number, or an fp32 scalar on the GPU (then nothing waits for its value)."""
-    dev = grad_scale if torch.is_tensor(grad_scale) else None
+    """grad_scale: a number, or an fp32 scalar on the parameters' GPU (then nothing waits for its value)."""
+    dev = grad_scale if torch.is_tensor(grad_scale) and grad_scale.dtype == torch.float32 and grad_scale.device == ps[0].device else None
     ext.adamw(list(ps), list(gs), list(ms), list(vs), lr, b1, b2, eps, wd, int(step), 1.0 if dev is not None else float(grad_scale), dev)

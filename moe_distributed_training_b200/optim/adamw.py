@@ -21,7 +21,21 @@ class FusedAdamW(torch.optim.Optimizer):
         defaults = dict(lr=lr, betas=betas, eps=eps, weight_decay=weight_decay)
         super().__init__(params, defaults)
         self.state_dtype = state_dtype
-        self.grad_scale = 1.0  # folded into the update (used by gradient clipping)
+        self._grad_scale = 1.0
+
+    @property
+    def grad_scale(self) -> float:
+        """Factor on all gradients, folded into the next update (gradient clipping sets it).  Reading it back waits for the
+        GPU if it is known only there."""
+        return float(self._grad_scale)
+
+    @grad_scale.setter
+    def grad_scale(self, value):
+        self._grad_scale = value
+
+    def set_device_grad_scale(self, value: torch.Tensor) -> None:
+        """The same from an fp32 scalar on the GPU, which the update kernel reads there."""
+        self._grad_scale = value
 
     @torch.no_grad()
     def step(self, closure=None):
@@ -48,7 +62,7 @@ class FusedAdamW(torch.optim.Optimizer):
             if ps[0].is_cuda and _ops.get_backend() == "native":
                 from ..ops import cuda_ops
                 cuda_ops.adamw_multi(ps, gs, ms, vs, group["lr"], b1, b2, group["eps"],
-                                     group["weight_decay"], step, self.grad_scale)
+                                     group["weight_decay"], step, self._grad_scale)
             else:
                 for p, g, m, v in zip(ps, gs, ms, vs):
                     reference.adamw_step(p, g, m, v, group["lr"], b1, b2, group["eps"],

@@ -44,8 +44,10 @@ def clip_grad_norm_(model, max_norm: float, shard_group=None, ep_group=None, opt
     if optimizer is not None and hasattr(optimizer, "grad_scale"):
         from .. import ops
         # On the GPU the factor stays there: reading it back would let the queue run dry once per optimizer step.
-        on_gpu = coef.is_cuda and ops.get_backend() == "native"
-        optimizer.grad_scale = coef if on_gpu else float(coef)
+        if coef.is_cuda and ops.get_backend() == "native" and hasattr(optimizer, "set_device_grad_scale"):
+            optimizer.set_device_grad_scale(coef)
+        else:
+            optimizer.grad_scale = float(coef)
     else:
         for p in model.parameters():
             if p.grad is not None:

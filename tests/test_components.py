@@ -379,6 +379,30 @@ def test_one_rank_flat_gradient_equals_the_accumulated_one(monkeypatch):
     assert bool((group.shard.grad[o:o + n] == 0).all())
 
 
+def test_clipping_factor_reads_as_a_number():
+    """`optimizer.grad_scale` is a float to whoever reads it, also when the factor was handed over as a tensor; an optimizer
+    that only has the attribute is given a float."""
+    from moe_distributed_training_b200.optim.adamw import FusedAdamW
+    from moe_distributed_training_b200.optim.clip import clip_grad_norm_
+    lin = torch.nn.Linear(4, 3)
+    opt = FusedAdamW(lin.parameters(), lr=0.1)
+    assert type(opt.grad_scale) is float and opt.grad_scale == 1.0
+    opt.set_device_grad_scale(torch.tensor(0.25))
+    assert type(opt.grad_scale) is float and opt.grad_scale == 0.25
+    for p in lin.parameters():
+        p.grad = torch.ones_like(p)
+    clip_grad_norm_(lin, 0.5, optimizer=opt)
+    assert type(opt.grad_scale) is float and abs(opt.grad_scale - 0.5 / 15 ** 0.5) < 1e-5
+    opt.step()
+    assert opt.grad_scale == 1.0
+
+    class Plain:
+        grad_scale = 1.0
+    other = Plain()
+    clip_grad_norm_(lin, 0.5, optimizer=other)
+    assert type(other.grad_scale) is float
+
+
 def test_profile_trace_flag_writes_a_trace(tmp_path):
     from moe_distributed_training_b200.train.run import run_training
     out = tmp_path / "traces"

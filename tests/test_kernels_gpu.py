@@ -984,6 +984,34 @@ def test_shared_last_round_first_used_on_a_stream_beside_a_busy_default_stream(o
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("where", ["number", "gpu", "cpu tensor", "fp64 gpu"])
+def test_clipping_factor_in_the_update(ops, where):
+    """AdamW with the factor as a number and as a scalar on the GPU: the same update, against the fp32 statement; a scalar that
+    the kernel cannot read there is read by the host.  bf16 results: one rounding (0.4 %)."""
+    from moe_distributed_training_b200.ops import reference
+    torch.manual_seed(5)
+    for n in (1, 7, 4096, 33333):
+        p, g = _rand(n), _rand(n)
+        m, v = torch.zeros_like(p), torch.zeros_like(p)
+        want = [t.float().clone() for t in (p, m, v)]
+        reference.adamw_step(want[0], g.float(), want[1], want[2], 1e-2, 0.9, 0.999, 1e-8, 0.01, 1, 0.125)
+        scale = {"number": 0.125, "gpu": torch.tensor(0.125, device=DEV), "cpu tensor": torch.tensor(0.125),
+                 "fp64 gpu": torch.tensor(0.125, device=DEV, dtype=torch.float64)}[where]
+        ops.adamw_multi([p], [g], [m], [v], 1e-2, 0.9, 0.999, 1e-8, 0.01, 1, scale)
+        for name, a, b in zip(("p", "m", "v"), (p, m, v), want):
+            torch.testing.assert_close(a.float(), b, rtol=8e-3, atol=1e-6, msg=lambda t: f"{name} of {n}, {where}: {t}")
+
+
+def test_clipping_factor_set_on_the_gpu_reads_as_a_number(ops):
+    from moe_distributed_training_b200.optim.adamw import FusedAdamW
+    from moe_distributed_training_b200.optim.clip import clip_grad_norm_
+    lin = torch.nn.Linear(64, 8, bias=False, device=DEV, dtype=torch.bfloat16)
+    opt = FusedAdamW(lin.parameters(), lr=0.1)
+    lin.weight.grad = torch.ones_like(lin.weight)
+    clip_grad_norm_(lin, 1.0, optimizer=opt)
+    assert type(opt.grad_scale) is float and abs(opt.grad_scale - 1.0 / 512 ** 0.5) < 1e-5
+
+
 def test_multi_tensor_gradient_accumulate(ops):
     """fp32 accumulators += bf16 / fp32 gradients of many tensors in one launch per 16."""
     torch.manual_seed(71)
