@@ -159,7 +159,10 @@ def shift_labels(labels: torch.Tensor, cu_seqlens: torch.Tensor, ignore_index: i
     out = torch.full_like(labels, ignore_index)
     out[:-1] = labels[1:]
     ends = (cu_seqlens[1:] - 1).long()
-    out.index_fill_(0, ends, ignore_index)       # (assigning a number through an index copies it from the host and waits)
+    if ends.device == out.device:
+        out.index_fill_(0, ends, ignore_index)   # (assigning a number through an index copies it from the host and waits)
+    else:
+        out[ends] = ignore_index                 # bounds on the host
     return out
 
 

@@ -1012,6 +1012,16 @@ def test_clipping_factor_set_on_the_gpu_reads_as_a_number(ops):
     assert type(opt.grad_scale) is float and abs(opt.grad_scale - 1.0 / 512 ** 0.5) < 1e-5
 
 
+@pytest.mark.parametrize("bounds_on", ["cuda", "cpu"])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_shifted_labels_with_bounds_on_either_device(bounds_on, dtype):
+    from moe_distributed_training_b200.models.mixtral import shift_labels
+    labels = torch.arange(10, 21, device=DEV)
+    cu = torch.tensor([0, 0, 4, 5, 11], dtype=dtype, device=bounds_on)        # an empty first sequence, and one of a single token
+    want = [11, 12, 13, -100, -100, 16, 17, 18, 19, 20, -100]
+    assert shift_labels(labels, cu).tolist() == want
+
+
 def test_multi_tensor_gradient_accumulate(ops):
     """fp32 accumulators += bf16 / fp32 gradients of many tensors in one launch per 16."""
     torch.manual_seed(71)
