@@ -336,10 +336,12 @@ std::vector<Tensor> make_plan(const Tensor& expert_ids, int64_t num_experts, int
                       dest.data_ptr<int>(), src.data_ptr<int>(), scratch.data_ptr<int>(), cur_stream()), "make_plan");
   return {counts, offs, dest, src};
 }
+// the row kernels move 16 bytes at a time
+static bool rows_aligned(const Tensor& t) { return t.is_contiguous() && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 Tensor gather_rows(const Tensor& x, const Tensor& src_slot, const OptTensor& padded_offsets, int64_t num_experts, const OptTensor& slot_scale, int64_t top_k) {
   CHECK_BF16(x);
   c10::cuda::CUDAGuard guard(x.device());
-  TORCH_CHECK(x.is_contiguous());
+  TORCH_CHECK(rows_aligned(x), "gather_rows: rows must be contiguous and 16-byte aligned");
   auto out = torch::empty({src_slot.numel(), x.size(1)}, x.options());
   check(mdt_gather_rows(x.data_ptr(), src_slot.data_ptr<int>(), padded_offsets.has_value() ? padded_offsets->data_ptr<int>() : nullptr, (int)num_experts,
                         cptr(slot_scale), out.data_ptr(), (int)src_slot.numel(), (int)x.size(1), (int)top_k, cur_stream()), "gather_rows");
@@ -348,17 +350,17 @@ Tensor gather_rows(const Tensor& x, const Tensor& src_slot, const OptTensor& pad
 Tensor combine_rows(const Tensor& y, const Tensor& dest_row, const OptTensor& weights, int64_t top_k, const OptTensor& residual = std::nullopt) {
   CHECK_BF16(y);
   c10::cuda::CUDAGuard guard(y.device());
-  TORCH_CHECK(y.is_contiguous());
+  TORCH_CHECK(rows_aligned(y), "combine_rows: rows must be contiguous and 16-byte aligned");
   const int T = (int)(dest_row.numel() / top_k);
   auto out = torch::empty({T, y.size(1)}, y.options());
   if (residual.has_value())
-    TORCH_CHECK(residual->is_contiguous() && residual->scalar_type() == at::kBFloat16 && residual->numel() == out.numel(), "residual must match the output");
+    TORCH_CHECK(rows_aligned(*residual) && residual->scalar_type() == at::kBFloat16 && residual->numel() == out.numel(), "residual must match the output");
   check(mdt_combine_rows(y.data_ptr(), dest_row.data_ptr<int>(), cptr(weights), cptr(residual), out.data_ptr(), T, (int)y.size(1), (int)top_k, cur_stream()), "combine_rows");
   return out;
 }
 Tensor combine_wgrad(const Tensor& y, const Tensor& dest_row, const Tensor& dout, int64_t top_k) {
   c10::cuda::CUDAGuard guard(y.device());
-  TORCH_CHECK(y.is_contiguous() && dout.is_contiguous());
+  TORCH_CHECK(rows_aligned(y) && rows_aligned(dout), "combine_wgrad: rows must be contiguous and 16-byte aligned");
   const int T = (int)(dest_row.numel() / top_k);
   auto dw = torch::empty({T, top_k}, y.options());
   check(mdt_combine_wgrad(y.data_ptr(), dest_row.data_ptr<int>(), dout.data_ptr(), dw.data_ptr(), T, (int)y.size(1), (int)top_k, cur_stream()), "combine_wgrad");

@@ -185,23 +185,30 @@ def make_plan(top_experts, num_experts, block=BLOCK_ROWS, capacity=None) -> Rout
     return RoutingPlan(counts, offs, dest, src, k, num_experts)
 
 
+def _rows(x):
+    """x as the row kernels read it, in 16-byte pieces: contiguous, and copied if it starts between two of them (a view into a
+    larger buffer, the callers' own tensors come here without another copy)."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 class _Gather(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, plan: RoutingPlan):
         ctx.plan = plan
-        return ext.gather_rows(x.contiguous(), plan.src_slot, plan.padded_offsets, plan.num_experts, None, plan.top_k)
+        return ext.gather_rows(_rows(x), plan.src_slot, plan.padded_offsets, plan.num_experts, None, plan.top_k)
 
     @staticmethod
     def backward(ctx, dxg):
         plan = ctx.plan
-        return ext.combine_rows(dxg.contiguous(), plan.dest_row, None, plan.top_k), None
+        return ext.combine_rows(_rows(dxg), plan.dest_row, None, plan.top_k), None
 
 
 class _Combine(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, weights, plan: RoutingPlan):
         ctx.plan = plan
-        y = y.contiguous()
+        y = _rows(y)
         w = weights.contiguous() if weights is not None else None
         ctx.save_for_backward(y, w)
         return ext.combine_rows(y, plan.dest_row, w, plan.top_k)
@@ -210,7 +217,7 @@ class _Combine(torch.autograd.Function):
     def backward(ctx, dout):
         plan = ctx.plan
         y, w = ctx.saved_tensors
-        dout = dout.contiguous()
+        dout = _rows(dout)
         dy = ext.gather_rows(dout, plan.src_slot, plan.padded_offsets, plan.num_experts,
                              w.reshape(-1) if w is not None else None, plan.top_k)
         dw = ext.combine_wgrad(y, plan.dest_row, dout, plan.top_k) if (w is not None and ctx.needs_input_grad[1]) else None

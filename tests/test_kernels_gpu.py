@@ -1022,6 +1022,61 @@ def test_shifted_labels_with_bounds_on_either_device(bounds_on, dtype):
     assert shift_labels(labels, cu).tolist() == want
 
 
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("layout", ["plain", "strided", "odd start"])
+def test_parallel_linear_lora_slot_order_on_the_gpu(ops, gated, layout):
+    """Slot-ordered calls (plan from the slots, no permutation) against fp64 of the definition: experts without rows, tokens and
+    output gradients that are strided or that start between two 16-byte pieces (a view into a larger buffer).  bf16 inputs,
+    intermediates (hidden rank products, gate weights) and results: 2e-2 as for the other products, gradients of gates and
+    factors included."""
+    from scattermoe_utils.parallel_linear_lora import parallel_linear_lora
+    torch.manual_seed(17)
+    T, K, N, E, r, k = 203, 264, 136, 5, 16, 2
+
+    def place(t):
+        if layout == "plain":
+            return t
+        if layout == "strided":
+            return torch.stack([t, t], -1)[..., 0]
+        buf = torch.empty(t.numel() + 3, dtype=t.dtype, device=DEV)[3:]
+        return buf.copy_(t.reshape(-1)).view(t.shape)
+    experts = torch.randint(0, E - 1, (T, k), device=DEV)                   # the last expert gets nothing
+    ids, order = torch.sort(experts.reshape(-1), stable=True)
+    x = place(_rand(T, K)).requires_grad_(True)
+    W = _rand(E, K, N, scale=0.05)
+    A, B = _rand(E, K, r, scale=0.05).requires_grad_(True), _rand(E, r, N, scale=0.05).requires_grad_(True)
+    g = torch.rand(T, k, device=DEV).to(torch.bfloat16).requires_grad_(True) if gated else None
+    dy = place(_rand(T if gated else T * k, N))
+    if layout == "odd start":
+        assert x.is_contiguous() and x.data_ptr() % 16 != 0 and dy.data_ptr() % 16 != 0
+    y = parallel_linear_lora(x, W, A, B, r, 32.0, k, ids, order, gates=g)
+    wrt = [x, A, B] + ([g] if gated else [])
+    grads = torch.autograd.grad(y, wrt, dy)
+    x64, A64, B64 = (t.detach().double().requires_grad_(True) for t in (x, A, B))
+    g64 = g.detach().double().requires_grad_(True) if gated else None
+    eff = W.double() + 2.0 * A64 @ B64                                      # lora_alpha / r = 2
+    slots = torch.einsum("tk,tckn->tcn", x64, eff[experts])
+    ref = (slots * g64[..., None]).sum(1) if gated else slots.reshape(T * k, N)
+    ref_grads = torch.autograd.grad(ref, [x64, A64, B64] + ([g64] if gated else []), dy.double())
+    _close(y, ref, name="y")
+    for name, a, b in zip(("x", "A", "B", "gates"), grads, ref_grads):
+        assert a.shape == b.shape and _rel_err(a, b) < 2e-2, (name, _rel_err(a, b))
+    ops.check_status(DEV)
+
+
+def test_row_kernels_refuse_rows_that_start_between_two_pieces(ops):
+    """The kernels move 16 bytes at a time: the bindings answer with an error instead of a misaligned access."""
+    top = torch.zeros(8, 1, dtype=torch.int32, device=DEV)
+    plan = ops.make_plan(top, 1)
+    odd = torch.zeros(8 * 64 + 1, dtype=torch.bfloat16, device=DEV)[1:].view(8, 64)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        ops.ext.gather_rows(odd, plan.src_slot, plan.padded_offsets, 1, None, 1)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        ops.ext.combine_rows(odd, plan.dest_row, None, 1)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        ops.ext.combine_wgrad(torch.zeros(8, 64, dtype=torch.bfloat16, device=DEV), plan.dest_row, odd, 1)
+
+
 def test_multi_tensor_gradient_accumulate(ops):
     """fp32 accumulators += bf16 / fp32 gradients of many tensors in one launch per 16."""
     torch.manual_seed(71)
