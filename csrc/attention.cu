@@ -978,7 +978,10 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
   AttnParams p;
   memset(&p, 0, sizeof(p));
   // MDT_ATTN_FWD=serial selects the one-block-at-a-time kernel (for comparisons); default: the pipelined kernel
-  static const bool serial = []() { const char* e = getenv("MDT_ATTN_FWD"); return e != nullptr && e[0] == 's'; }();
+  static const bool forced = []() { const char* e = getenv("MDT_ATTN_FWD"); return e != nullptr && e[0] == 's'; }();
+  // The pipelined kernel masks and compares scores before they are scaled, which takes a positive scale; any other one goes
+  // through the serial kernel, which scales first.
+  const bool serial = forced || !(scale > 0.f);
   int rc = att_map(&p.tmQ, q, total_tokens, heads_q);
   if (serial) rc |= att_map(&p.tmK, k, total_tokens, heads_kv) | att_map(&p.tmV, v, total_tokens, heads_kv);
   else rc |= att_map(&p.tmK64, k, total_tokens, heads_kv, FB) | att_map(&p.tmV64, v, total_tokens, heads_kv, FB);

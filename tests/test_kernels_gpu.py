@@ -646,6 +646,32 @@ def test_attention_many_short_sequences(ops, lens, heads, kv):
     test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv)
 
 
+@pytest.mark.parametrize("scale", [0.3, 0.0, -0.08])
+def test_attention_scale_of_any_sign(ops, scale):
+    """Forward and backward against fp64, 1e-2 as for the other attention tests."""
+    lens, heads, kv, d = [200, 77, 1, 130], 4, 2, 128
+    T = sum(lens)
+    torch.manual_seed(9)
+    q, k, v, do = (_rand(T, h, d) for h in (heads, kv, kv, heads))
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    o, lse = ops.ext.attention_fwd(q, k, v, cu, max(lens), scale, ops.status_tensor(DEV))
+    grads = ops.ext.attention_bwd(q, k, v, o, do, lse, cu, max(lens), scale, ops.status_tensor(DEV))
+    q2, k2, v2 = (t.double().requires_grad_(True) for t in (q, k, v))
+    outs = []
+    for s, n in zip(cu.tolist(), lens):
+        qs, ks, vs = (t[s:s + n].transpose(0, 1) for t in (q2, k2.repeat_interleave(heads // kv, 1), v2.repeat_interleave(heads // kv, 1)))
+        sc = (qs @ ks.transpose(1, 2)) * scale
+        sc = sc.masked_fill(torch.ones(n, n, device=DEV, dtype=torch.bool).triu(1), float("-inf"))
+        outs.append((sc.softmax(-1) @ vs).transpose(0, 1))
+    ref = torch.cat(outs)
+    for name, a, b in zip(("o", "dq", "dk", "dv"), [o] + list(grads), (ref,) + torch.autograd.grad(ref, (q2, k2, v2), do.double())):
+        if float(b.norm()) == 0.0:            # scale 0: the scores do not depend on q and k
+            assert float(a.float().abs().max()) == 0.0, name
+        else:
+            assert _rel_err(a, b) < 1e-2, (name, _rel_err(a, b))
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("T,first,end,heads,kv", [(512, 5, 300, 4, 4), (512, 5, 300, 32, 8), (700, 0, 1, 8, 2), (300, 290, 300, 4, 2), (4000, 1000, 1600, 4, 1)])
 def test_attention_gradients_of_rows_outside_the_sequences_are_zero(ops, T, first, end, heads, kv):
     """Rows before the first and after the last sequence (a padded stream) get zero gradients, whatever the memory held, with
