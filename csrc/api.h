@@ -78,6 +78,9 @@ void mdt_gemm_rows_hint(long long rows);
 // `num_sms` SMs: 0 = 128-row tiles, otherwise CTA-pair tiles (2 under policies 3 to 5).  Reads only M, N, K, K_l, G, mode, dual, c_fp32, accumulate,
 // capacity_rows and whether offsets is set; needs no GPU.
 int mdt_gemm_choose_tiling(const MdtGemmDesc* d, int policy, long long rows_hint, int num_sms);
+// Under the default policy the cluster kernel is asked first: the number of CTAs that share one tile's depth (0: it does not
+// take the product) and the tile's width, on a GPU that holds num_sms / S clusters of S.  Needs no GPU.
+int mdt_gemm_choose_cluster(const MdtGemmDesc* d, long long rows_hint, int num_sms, int* width);
 // Sharing of the last, partly filled round of 128-row tiles by all SMs along the depth (partial sums through an fp32
 // workspace, finished by the last contributor): 1 on (default; MDT_GEMM_SPLIT=0 turns it off), 0 off; returns the
 // previous setting (other values only read it).  Results of shared tiles depend on the order of fp32 additions.

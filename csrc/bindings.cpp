@@ -927,6 +927,17 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     d.dual = dual; d.c_fp32 = c_fp32; d.accumulate = accumulate; d.offsets = has_offsets ? &dummy_offsets : nullptr;
     return (int64_t)mdt_gemm_choose_tiling(&d, (int)policy, rows_hint, (int)num_sms);
   });
+  m.def("gemm_choose_cluster", [](int64_t mode, int64_t M, int64_t N, int64_t K, int64_t K_l, int64_t G, int64_t capacity_rows, bool dual, bool accumulate,
+                                  bool has_residual, bool has_offsets, int64_t rows_hint, int64_t num_sms) {        // (CTAs per tile or 0, tile width)
+    MdtGemmDesc d;
+    memset(&d, 0, sizeof(d));
+    static const int dummy_offsets = 0;
+    d.mode = (int)mode; d.M = (int)M; d.N = (int)N; d.K = (int)K; d.K_l = (int)K_l; d.G = (int)G; d.capacity_rows = capacity_rows;
+    d.dual = dual; d.accumulate = accumulate; d.R = has_residual ? &dummy_offsets : nullptr; d.offsets = has_offsets ? &dummy_offsets : nullptr;
+    int width = 0;
+    const int ctas = mdt_gemm_choose_cluster(&d, rows_hint, (int)num_sms, &width);
+    return std::make_pair((int64_t)ctas, (int64_t)width);
+  });
   m.def("gemm_rows_hint", [](int64_t rows) { mdt_gemm_rows_hint((long long)rows); });
   m.def("gemm_max_pairs", []() { return (int64_t)mdt_gemm_max_pairs(); });
   m.def("skinny_preferred", &skinny_preferred);

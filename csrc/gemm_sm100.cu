@@ -1448,7 +1448,9 @@ static int max_clusters(int S) {
 // partial tiles; against one CTA per tile (0.28 + 1, 128-wide outputs) or the faster of the two 256-wide kernels in one
 // round.  All clusters have to be resident at once (max_clusters: a cluster needs its SMs in one GPC, so 16 clusters of 8
 // are more than a B200 holds: 16 tiles 64 deep took 25 us that way, in two rounds, 4 tiles 13).
-static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int* bn) {
+// `resident`: clusters of S CTAs that the GPU holds at once.
+template <class Resident>
+static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, Resident resident, int* bn) {
   if (d->dual || d->swiglu_g != nullptr || d->tile_ready != nullptr || d->row_dest_rank != nullptr || (d->accumulate && d->R != nullptr)) return 0;
   const int G = d->G < 1 ? 1 : d->G;
   *bn = d->N <= 64 ? 64 : (d->N <= 128 ? 128 : 256);
@@ -1463,7 +1465,7 @@ static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, int*
   const double per = *bn == 256 ? 0.48 : (*bn == 128 ? 0.28 : 0.22);
   const double whole = d->N <= 128 ? kb * 0.28 + 1.0 : fmin(kb * 0.48 + 1.0, kb * 0.34 + 2.0);
   for (int S = MAX_CLUSTER; S >= 2; S /= 2)
-    if (kb >= 4.0 * S && tiles <= max_clusters(S)) return ceil(kb / S) * per + 5.0 < whole ? S : 0;
+    if (kb >= 4.0 * S && tiles <= resident(S)) return ceil(kb / S) * per + 5.0 < whole ? S : 0;
   return 0;
 }
 
@@ -1494,6 +1496,10 @@ extern "C" void mdt_gemm_rows_hint(long long rows) { mdt::t_rows_hint = rows; }
 extern "C" int mdt_gemm_max_pairs() { return mdt::g_max_pairs; }
 extern "C" int mdt_gemm_choose_tiling(const MdtGemmDesc* d, int policy, long long rows_hint, int num_sms) {
   return mdt::choose_tiling(d, policy, rows_hint, num_sms);
+}
+extern "C" int mdt_gemm_choose_cluster(const MdtGemmDesc* d, long long rows_hint, int num_sms, int* width) {
+  *width = 0;
+  return mdt::choose_cluster(d, rows_hint, [num_sms](int S) { return num_sms / S; }, width);
 }
 extern "C" void mdt_gemm_set_pair_cap(int pairs) { mdt::g_pair_cap = pairs; }
 extern "C" int mdt_gemm_set_split(int on) {
@@ -1544,7 +1550,7 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   const int BN = (p.dual || p.N > 128) ? 256 : 128;
   const int bn_out = p.dual ? BN / 2 : BN;
   int cluster_bn = 0;
-  const int cluster = pair_policy() == MAX_POLICY ? choose_cluster(d, t_rows_hint, &cluster_bn) : 0;
+  const int cluster = pair_policy() == MAX_POLICY ? choose_cluster(d, t_rows_hint, max_clusters, &cluster_bn) : 0;
   const bool pair = cluster == 0 && choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms) != 0;
   const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
   int rc = 0;

@@ -403,6 +403,38 @@ def test_clipping_factor_reads_as_a_number():
     assert type(other.grad_scale) is float
 
 
+def test_gemm_cluster_choice_without_a_gpu():
+    """Which products share their few tiles' depth over a cluster, with how many CTAs and at which tile width."""
+    build = pytest.importorskip("moe_distributed_training_b200.ops.build")
+    try:
+        ext = build.load()
+    except Exception:  # noqa: BLE001
+        pytest.skip("extension not built")
+
+    def choose(mode, M, N, K, K_l=0, G=1, cap=0, dual=False, acc=False, res=False, hint=0, sms=148):
+        return ext.gemm_choose_cluster(mode, M, N, K, K_l, G, cap, dual, acc, res, mode != 0, hint, sms)
+    # tile widths follow the output columns
+    assert choose(0, 100, 16, 4096) == (8, 64) and choose(0, 100, 64, 4096) == (8, 64)
+    assert choose(0, 100, 72, 4096) == (8, 128) and choose(0, 100, 128, 4096) == (8, 128)
+    assert choose(0, 100, 136, 4096) == (8, 256)
+    # the largest cluster of which all tiles are resident at once: 16 tiles, 20 tiles, 80 tiles
+    assert choose(0, 77, 4096, 4096) == (8, 256) and choose(0, 576, 1024, 4096) == (4, 256)
+    assert choose(0, 576, 4096, 4096)[0] == 0
+    assert choose(0, 77, 4096, 4096, sms=64) == (4, 256) and choose(0, 77, 4096, 4096, sms=16)[0] == 0
+    # four k blocks per CTA at least, and only where the exchange of the partial tiles is earned back
+    assert choose(0, 100, 128, 64 * 7)[0] == 0 and choose(0, 100, 128, 1024)[0] == 0
+    assert choose(0, 100, 128, 64 * 31)[0] == 4 and choose(0, 100, 128, 64 * 32)[0] == 8
+    assert choose(0, 100, 256, 0)[0] == 0
+    # excluded forms
+    assert choose(0, 77, 4096, 4096, dual=True)[0] == 0 and choose(0, 77, 4096, 4096, acc=True, res=True)[0] == 0
+    assert choose(0, 77, 4096, 4096, acc=True)[0] == 8 and choose(0, 77, 4096, 4096, res=True)[0] == 8
+    # row groups: the capacity minus the padding, or what the caller expects
+    assert choose(1, 0, 16, 14336, G=8, cap=1024 + 8 * 127)[0] == 8
+    assert choose(1, 0, 16, 14336, G=8, cap=16384 + 8 * 127)[0] == 0 and choose(1, 0, 16, 14336, G=8, cap=16384 + 8 * 127, hint=1000)[0] == 8
+    # depth groups: the average group's rows are the depth
+    assert choose(2, 512, 16, 0, G=1, cap=4096 + 127)[0] == 8 and choose(2, 14336, 16, 0, G=8, cap=4096 + 8 * 127)[0] == 0
+
+
 def test_profile_trace_flag_writes_a_trace(tmp_path):
     from moe_distributed_training_b200.train.run import run_training
     out = tmp_path / "traces"
