@@ -345,6 +345,37 @@ def test_router_backward_odd_sizes(ops, T, H, E):
     _close(acc, base.float() + dx.float(), name="dx accumulate")
 
 
+@pytest.mark.parametrize("T,H,E", [(50, 4104, 8), (3700, 4104, 8), (4001, 6144, 3), (300, 8192, 8)])
+def test_router_rows_wider_than_4096_columns(ops, T, H, E):
+    """The general kernels, one token per warp and (from 3552 tokens on 148 SMs) two, with the statistics, against fp64."""
+    test_router_backward_odd_sizes(ops, T, H, E)
+    x, w = _rand(T, H), _rand(E, H, scale=0.05)
+    scores, wts, idx, stats = ops.ext.router_fwd(x, w, 2, True, True)
+    p = (x.double() @ w.double().t()).softmax(-1)
+    _close(scores, p, 1e-2, name="scores")
+    assert torch.equal(stats[:E], torch.bincount(idx.reshape(-1).long(), minlength=E).float())
+    assert torch.allclose(stats[E:], scores.float().sum(0), rtol=1e-4, atol=1e-3)
+
+
+@pytest.mark.parametrize("T,H,E", [(40, 512, 8), (37, 4104, 8), (29, 256, 20)])
+def test_router_with_nan_and_infinite_tokens(ops, T, H, E):
+    """A token with a NaN or an infinity gets NaN scores, indices that are experts, and a NaN gradient; the others' scores,
+    choices and gradients are what they are without it."""
+    torch.manual_seed(H)
+    x, w, d = _rand(T, H), _rand(E, H, scale=0.05), _rand(T, 2)
+    clean = ops.ext.router_fwd(x, w, 2, True)
+    clean_dx = ops.ext.router_bwd(x, w, clean[2], d, None, True, None, False)[0]
+    bad = x.clone()
+    bad[3, 5], bad[T - 1, H - 1] = float("nan"), float("inf")
+    rest = [t for t in range(T) if t not in (3, T - 1)]
+    scores, wts, idx = ops.ext.router_fwd(bad, w, 2, True)
+    assert bool(scores[[3, T - 1]].isnan().all()) and bool(((idx >= 0) & (idx < E)).all())
+    for a, b in zip((scores, wts, idx), clean):
+        assert torch.equal(a[rest], b[rest])
+    dx = ops.ext.router_bwd(bad, w, idx, d, None, True, None, False)[0]
+    assert torch.equal(dx[rest], clean_dx[rest]) and bool(dx[[3, T - 1]].isnan().all())
+
+
 @pytest.mark.parametrize("rows,cols", [(1, 64), (700, 4096), (301, 2056), (40, 8192), (9, 16384)])
 def test_rmsnorm_backward_widths(ops, rows, cols):
     torch.manual_seed(cols)
@@ -669,6 +700,47 @@ def test_attention_scale_of_any_sign(ops, scale):
             assert float(a.float().abs().max()) == 0.0, name
         else:
             assert _rel_err(a, b) < 1e-2, (name, _rel_err(a, b))
+    ops.check_status(DEV)
+
+
+@pytest.mark.parametrize("T", [100, 700])
+def test_attention_with_nan_and_infinite_rows(ops, T):
+    """NaN in a query row and infinities in a key row reach what they reach in fp64 attention, and nothing else: the other rows
+    and heads are bit for bit those of the clean call.  In the backward pass, a NaN in a row of dO makes that row of dQ NaN and
+    leaves the other rows and the other heads' gradients as they were (dQ: fp32 sums in another order)."""
+    torch.manual_seed(T)
+    heads, kv, d, bad, hot = 4, 2, 128, 70, 33
+    q, k, v, do = (_rand(T, h, d) for h in (heads, kv, kv, heads))
+    cu = torch.tensor([0, T], dtype=torch.int32, device=DEV)
+
+    def fwd(q, k):
+        return ops.ext.attention_fwd(q, k, v, cu, T, d ** -0.5, ops.status_tensor(DEV))
+    o, lse = fwd(q, k)
+    q2 = q.clone()
+    q2[bad, 1] = float("nan")
+    o2, _ = fwd(q2, k)
+    assert bool(o2[bad, 1].isnan().all())
+    keep = torch.ones(T, heads, dtype=torch.bool, device=DEV)
+    keep[bad, 1] = False
+    assert torch.equal(o2[keep], o[keep])
+    k2 = k.clone()
+    k2[hot, 0, 7] = float("inf")
+    o3, _ = fwd(q, k2)
+    qs, ks, vs = (t.double().transpose(0, 1) for t in (q, k2.repeat_interleave(2, 1), v.repeat_interleave(2, 1)))
+    sc = (qs @ ks.transpose(1, 2)) * d ** -0.5
+    ref = (sc.masked_fill(torch.ones(T, T, device=DEV, dtype=torch.bool).triu(1), float("-inf")).softmax(-1) @ vs).transpose(0, 1)
+    nan = ref.isnan()
+    assert bool(nan.any()) and torch.equal(o3.isnan(), nan)
+    assert float((o3.double() - ref)[~nan].norm()) < 1e-2 * float(ref[~nan].norm())
+    assert torch.equal(o3[:hot], o[:hot]) and torch.equal(o3[:, 2:], o[:, 2:])
+    grads = ops.ext.attention_bwd(q, k, v, o, do, lse, cu, T, d ** -0.5, ops.status_tensor(DEV))
+    do2 = do.clone()
+    do2[bad, 1] = float("nan")
+    grads2 = ops.ext.attention_bwd(q, k, v, o, do2, lse, cu, T, d ** -0.5, ops.status_tensor(DEV))
+    assert bool(grads2[0][bad, 1].isnan().all())
+    _close(grads2[0][keep], grads[0][keep], 1e-3, name="dq")
+    for i in (1, 2):
+        assert torch.equal(grads2[i][:, 1], grads[i][:, 1])          # the other kv head
     ops.check_status(DEV)
 
 
@@ -1101,6 +1173,50 @@ def test_row_kernels_refuse_rows_that_start_between_two_pieces(ops):
         ops.ext.combine_rows(odd, plan.dest_row, None, 1)
     with pytest.raises(RuntimeError, match="16-byte"):
         ops.ext.combine_wgrad(torch.zeros(8, 64, dtype=torch.bfloat16, device=DEV), plan.dest_row, odd, 1)
+
+
+@pytest.mark.parametrize("block", [False, True])
+def test_expert_gradients_written_then_added(ops, block):
+    """Two micro-batches into fresh `.grad`s (the first product writes, the second adds), for the experts on their own and for
+    the decoder layers' MoE sub-block, against the same module on torch's operators.  bf16 gradients, rounded after each
+    micro-batch on both sides: 2e-2 as for the other products."""
+    from moe_distributed_training_b200 import MixtralConfig, ops as front
+    from moe_distributed_training_b200.config import MoEArguments
+    from moe_distributed_training_b200.models.mixtral import MixtralForCausalLM
+    from moe_distributed_training_b200.moe.layer import dMoE
+    torch.manual_seed(23)
+    if block:
+        cfg = MixtralConfig(vocab_size=256, hidden_size=256, intermediate_size=384, num_hidden_layers=1, num_attention_heads=2,
+                            num_key_value_heads=1, head_dim=128, num_local_experts=4, num_experts_per_tok=2)
+        module = MixtralForCausalLM(cfg, dtype=torch.bfloat16, device=DEV)
+        batches = [torch.randint(0, 256, (1, n), device=DEV) for n in (150, 211)]
+    else:
+        module = dMoE(MoEArguments(hidden_size=256, ffn_hidden_size=384, moe_num_experts=4, moe_top_k=2, bf16=True, device=DEV))
+        batches = [_rand(1, n, 256) for n in (150, 211)]
+    with torch.no_grad():
+        for name, p in module.named_parameters():
+            if "norm" not in name:
+                p.normal_(0.0, 0.2 if "router" in name else 0.05)
+
+    def run():
+        module.zero_grad(set_to_none=True)
+        for b in batches:
+            if block:
+                module(b, labels=b).loss.backward()
+            else:
+                y, _ = module(b)
+                (y.float() * torch.linspace(-1, 1, y.numel(), device=DEV).view_as(y)).sum().backward()
+        return {n: p.grad.clone() for n, p in module.named_parameters() if n.endswith((".w1", ".w2", ".w3"))}
+    got = run()
+    front.set_backend("library")
+    try:
+        want = run()
+    finally:
+        front.set_backend("native")
+    assert len(got) == 3 and got.keys() == want.keys()
+    for n in got:
+        assert _rel_err(got[n], want[n]) < 2e-2, (n, _rel_err(got[n], want[n]))
+    ops.check_status(DEV)
 
 
 def test_multi_tensor_gradient_accumulate(ops):
