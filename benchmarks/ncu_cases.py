@@ -1,6 +1,6 @@
 """Small single-GPU cases for profiler captures: one kernel family per case, a handful of launches.
 
-    python benchmarks/ncu_cases.py gemm|gemm_pair|gemm_split|gather_gemm|rs_block|expert_mlp|attention|dispatch|gemm_exchange
+    python benchmarks/ncu_cases.py gemm|gemm_pair|gemm_cluster|gemm_split|gather_gemm|rs_block|expert_mlp|attention|attention_long|dispatch|gemm_exchange
 
 Sizes keep the working set above the 126 MB L2 where DRAM figures matter, but far below a GB of launches.
 """
@@ -24,6 +24,12 @@ def main():
         C.ext.gemm_set_pair_policy(2 if case == "gemm_pair" else 0)   # CTA-pair kernel or single-CTA kernel
         for _ in range(4):
             C.mm_nt(x, w, out=out)
+    elif case == "gemm_cluster":
+        # one projection of a short prompt: 16 tiles, the depth of each shared by a cluster
+        x = torch.randn(77, 4096, device=dev, dtype=bf)
+        w = torch.randn(4096, 4096, device=dev, dtype=bf) * 0.02
+        for _ in range(4):
+            C.mm_nt(x, w)
     elif case == "gemm_split":
         # down-projection shape of one micro-batch: 10 x 16 = 160 tiles on 148 SMs, the last round shared along the depth
         x = torch.randn(1280, 14336, device=dev, dtype=bf)
@@ -63,8 +69,8 @@ def main():
         with torch.no_grad():
             for _ in range(3):
                 C.grouped_swiglu_mlp(xg, w1, w2, w3, plan)
-    elif case == "attention":
-        T, Hq, Hkv, d = 1024, 32, 8, 128
+    elif case in ("attention", "attention_long"):
+        T, Hq, Hkv, d = (1024 if case == "attention" else 8192), 32, 8, 128
         q = torch.randn(T, Hq, d, device=dev, dtype=bf, requires_grad=True)
         k = torch.randn(T, Hkv, d, device=dev, dtype=bf, requires_grad=True)
         v = torch.randn(T, Hkv, d, device=dev, dtype=bf, requires_grad=True)

@@ -182,9 +182,10 @@ struct Work {
 // Tiles are dealt to the CTAs round robin; when the last round would leave most SMs idle (fewer than 7/8 of them
 // get a tile), the tiles of that round are not handed out whole: their k blocks, taken together, are cut into one
 // contiguous piece per CTA (a piece spans at most two tiles).  Every CTA adds its piece's partial sums into an fp32
-// workspace tile and counts itself in (per 32-row quarter of the tile, i.e. per epilogue warp); the warp that arrives
-// last at a quarter reads the sums back and runs the normal epilogue for it.  Nobody waits for anybody.  With 160 tiles of depth 224 on 148 SMs that is 1 round + 18 k blocks per CTA instead of
-// 2 rounds (measured 0.136 instead of 0.192 ms).  Products of less than one round are left alone.
+// workspace tile and counts itself in, per 32-row quarter and column half of the tile, i.e. per epilogue warp; the warp that
+// arrives last at such a part reads the sums back and runs the normal epilogue for it.  Nobody waits for anybody.  With 160
+// tiles of depth 224 on 148 SMs that is 1 round + 18 k blocks per CTA instead of 2 rounds (0.136 instead of 0.192 ms).
+// Products of less than one round are left alone.
 // it = 0, 1, ... enumerates the CTA's work in order; returns false when there is no more.
 template <int BN_OUT>
 __host__ __device__ __forceinline__ bool get_work(const GemmParams& p, int cta, int num_ctas, int it, Work& w) {
@@ -200,9 +201,8 @@ __host__ __device__ __forceinline__ bool get_work(const GemmParams& p, int cta, 
   int whole = total_tiles;
   if (p.sk_ws != nullptr && p.mode != 2 && !p.dual && kbt >= 8) {
     const int rem = total_tiles % num_ctas;
-    // (pieces shorter than 8 k blocks are not worth their partial-sum traffic)
-    // and a product of less than one full round stays as it is: measured, 80 tiles of depth 64 cut into 148 pieces lose
-    // more to the partial sums than they gain)
+    // (pieces shorter than 8 k blocks are not worth their partial-sum traffic, and a product of less than one full round
+    // stays as it is: 80 tiles of depth 64 cut into 148 pieces lose more to the partial sums than they gain)
     if (rem != 0 && total_tiles > num_ctas && rem * 8 < num_ctas * 7 && (long long)rem * kbt >= 8ll * num_ctas) whole = total_tiles - rem;
   }
   const int n_whole = whole > cta ? (whole - cta + num_ctas - 1) / num_ctas : 0;
@@ -1318,8 +1318,8 @@ static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream
 static thread_local long long t_rows_hint = 0;
 
 // Which kernel takes the 256-wide tiles: 0 = the 128-row kernel always, 1 = the CTA-pair kernel where the shape
-// fills 256-row tiles, 2 and 4 = the CTA-pair kernel always, 3 = the CTA-pair kernel where 256-row tiles win by a margin
-// even with an exposed epilogue, 5 = whichever is faster by the measured model (default).  Initial value from
+// fills 256-row tiles, 2 and 4 = the CTA-pair kernel always (4: an older name of it), 3 = the CTA-pair kernel only where
+// 256-row tiles would win by a wide margin, 5 = whichever is faster by the measured model (default).  Initial value from
 // MDT_GEMM_PAIR; mdt_gemm_set_pair_policy() changes it.
 constexpr int MAX_POLICY = 5;
 static int g_pair_policy = -1;
@@ -1335,7 +1335,8 @@ static int pair_policy() {
 //   128-row kernel: 0.48 per 64-deep k block and CTA (bound by the 48 KB it brings in) + 1 per tile
 //   pair kernel:    0.34 per k block and pair (32 KB per CTA; near the tensor core's 0.27) + 2 per tile
 //   a tile takes at least its epilogue: 3.4 / 3.1, and 2.3 more where C is read as well
-//   weights arrive at no more than 5.6 TB/s, so below that the two are the same and the smaller tiles stay
+//   weights arrive at no more than 5.6 TB/s, so below that the two are taken for the same and the smaller tiles stay (not
+//   always right: dy W2^T of 576 tokens, 8 experts, 226 us against the pair's 208, with the SwiGLU epilogue 254 / 241)
 // E.g. gate/up of 8 experts, 4096 -> 14336: 400 tokens 342 against 387, 800 tokens 467 / 439, 2000 tokens 929 / 846, 9200
 // tokens 3058 / 2853; dense 9200 x 4096 x 4096 249 / 183; dense 1152 x 4096 x 4096 (144 or 80 tiles) 40 / 52.
 static bool pair_is_faster(const MdtGemmDesc* d, long long thread_rows_hint, int num_sms, int bn_out) {
@@ -1390,9 +1391,9 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
   if (policy == 4) return 2;
   if (policy == 5) return pair_is_faster(d, thread_rows_hint, num_sms, bn_out) ? 2 : 0;
   if (policy != 3) return 0;
-  // Policy 3 weighs 256-row tiles as if they had no second accumulator (0.70 us per k block of a tile whose epilogue, ~5 us
-  // or ~14 with SwiGLU, is not hidden) and wants 10 % in return; without a row count it takes them for products of
-  // >= 2048 rows and >= 3 waves of 128-row tiles only.
+  // Policy 3, for comparisons: a cautious rule that charges 256-row tiles more than the pair kernel takes (0.70 us per k
+  // block and an epilogue of 5 us, 14 with SwiGLU, that nothing hides: the costs of a single CTA with 256 rows) and wants
+  // 10 % in return; without a row count it takes them for products of >= 2048 rows and >= 3 waves of 128-row tiles only.
   long long r = rows_hint;
   const bool hinted = d->mode == 1 && thread_rows_hint > 0;
   if (hinted && thread_rows_hint < r) r = thread_rows_hint;
@@ -1405,7 +1406,7 @@ static int choose_tiling(const MdtGemmDesc* d, int policy, long long thread_rows
   bool wide;
   if (d->mode != 1 || hinted) {
     const double sms = num_sms;
-    const double slow_epilogue = (!d->c_fp32 && !d->accumulate) ? 0.0 : 6.0;   // the uncoalesced epilogue costs more
+    const double slow_epilogue = (!d->c_fp32 && !d->accumulate) ? 0.0 : 6.0;
     // rounds of 128-row tiles: whole rounds, except that a last round that fills less than 7/8 of the SMs is shared
     // by all of them along the depth (get_work), which costs about its share plus the partial-sum traffic
     double rounds = ceil(ceil(blocks) * nb / sms);
@@ -1447,7 +1448,8 @@ static int max_clusters(int S) {
 // microseconds, measured on B200: 0.48 / 0.28 / 0.22 per k block of a 256 / 128 / 64-wide tile, 5 for the exchange of the
 // partial tiles; against one CTA per tile (0.28 + 1, 128-wide outputs) or the faster of the two 256-wide kernels in one
 // round.  All clusters have to be resident at once (max_clusters: a cluster needs its SMs in one GPC, so 16 clusters of 8
-// are more than a B200 holds: 16 tiles 64 deep took 25 us that way, in two rounds, 4 tiles 13).
+// are more than a B200 holds: 16 tiles 64 deep took 25 us that way, in two rounds, 4 tiles 13).  That counts each product as
+// alone on the GPU; the q, k and v projections of a block run at the same time (bindings.cpp) and share it.
 // `resident`: clusters of S CTAs that the GPU holds at once.
 template <class Resident>
 static int choose_cluster(const MdtGemmDesc* d, long long thread_rows_hint, Resident resident, int* bn) {

@@ -652,8 +652,9 @@ static int router_grid(int tokens) {
   const int cap = sm_count_of_current_device() * 3;
   return g < 1 ? 1 : (g > cap ? cap : g);
 }
-// (Rows too wide for router_rows_kernel.)  Two tokens per warp and pass once every warp of the grid has two (more experts
-// than 8: no registers for it).  8000 x 4096, 8 experts: forward 81 -> 60 us; 576 tokens would lose (backward 31 -> 42 us).
+// (More than 4096 columns, which router_rows_kernel does not hold.)  Two tokens per warp and pass once every warp of the grid
+// has two (more experts than 8: no registers for it).  Measured at 4096 columns and 8 experts, before router_rows_kernel took
+// that width: 8000 tokens forward 81 -> 60 us; 576 would lose (backward 31 -> 42 us).
 static bool router_pairs(int tokens, int grid) { return tokens >= 2 * grid * 4; }
 // The router matrix is staged in shared memory when it fits (E x H bf16 <= 96 KB); opt in above 48 KB once per kernel.
 static int router_smem_ok(const void* kernel, size_t bytes) {

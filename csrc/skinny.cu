@@ -1,8 +1,9 @@
 // Products with a very narrow output, y[M, r] = alpha * x[M, K] * A^T with r <= 32 (LoRA down-projections:
 // x A^T in the forward pass, dy B in the backward pass).
 //
-// A 128-row tensor-core tile would be 7/8 empty here and only M/128 CTAs would each walk the whole depth, so
-// these run on the CUDA cores instead.  A CTA of 8 warps owns 4 rows of x; the warps split the depth in
+// A 128-row tensor-core tile would be 7/8 empty here and only M/128 CTAs would each walk the whole depth, so small
+// x (below a million elements) and operands that TMA cannot address run on the CUDA cores; larger ones are faster as
+// products whose depth a cluster shares (see skinny_preferred in bindings.cpp).  A CTA of 8 warps owns 4 rows of x; the warps split the depth in
 // interleaved 256-element slabs, every lane holding 8 consecutive depth positions of the 4 rows and of all r
 // rows of A in registers (no staging, every load independent), then the partial sums are reduced over lanes
 // and warps.  M/4 CTAs are in flight and the op is bound by one pass over x and an L2-resident A.

@@ -106,9 +106,9 @@ def test_peer_wait_gives_up_with_a_status_code(cops):
     assert int(status.item()) == 0
 
 
-@pytest.fixture(params=[0, 4], ids=["tile128", "tall"])
+@pytest.fixture(params=[0, 2], ids=["tile128", "pair"])
 def gemm_tile_policy(request, cops):
-    """Runs a test with the 128-row GEMM kernel and with the tall 256 x 256 kernel forced."""
+    """Runs a test with the 128-row GEMM kernel and with the CTA-pair kernel forced."""
     prev = cops.ext.gemm_set_pair_policy(request.param)
     yield request.param
     cops.ext.gemm_set_pair_policy(prev)

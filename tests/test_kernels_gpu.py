@@ -176,9 +176,9 @@ def _under_pair_policy(ops, policy, fn):
         ops.ext.gemm_set_pair_policy(prev)
 
 
-@pytest.mark.parametrize("policy", [2, 4], ids=["pair", "tall"])
+@pytest.mark.parametrize("policy", [2, 5], ids=["pair", "default"])
 def test_gemm_pair_kernel_matches_single_cta_kernel(ops, policy):
-    """The CTA-pair (cta_group::2) kernel and the tall 256 x 256 kernel, forced for every 256-wide tile, against
+    """The CTA-pair (cta_group::2) kernel, forced for every 256-wide tile, and the default choice of kernel against
     the 128-row kernel."""
     torch.manual_seed(21)
     cases = []
@@ -404,7 +404,7 @@ def test_rope_head_sizes(ops, heads, d):
     _close(ops.ext.rope(ops.ext.rope(x, pos, 1e6, False), pos, 1e6, True).flatten(1), x.float().flatten(1), 1e-2, name="rope and back")
 
 
-@pytest.mark.parametrize("policy", [2, 4], ids=["pair", "tall"])
+@pytest.mark.parametrize("policy", [2, 5], ids=["pair", "default"])
 @pytest.mark.parametrize("T,E,H,F,lora", [(600, 4, 256, 512, True), (1500, 8, 1024, 2048, False), (333, 3, 512, 1024, False)])
 def test_grouped_mlp_pair_kernel_matches_single_cta_kernel(ops, T, E, H, F, lora, policy):
     """Row groups with odd and even numbers of 128-row blocks (idle second halves), forward and backward."""
@@ -919,7 +919,7 @@ def test_residual_connections_fused_into_their_producers(ops):
     ext = ops.ext
     M, K, N = 333, 512, 768
     x, w, res = _rand(M, K), _rand(N, K, scale=0.05), _rand(M, N)
-    for policy in (0, 4):                                   # 128-row tiles and the tall kernel (coalescing epilogue off)
+    for policy in (0, 2, 5):                                # 128-row tiles, the CTA pair, the default choice
         prev = ext.gemm_set_pair_policy(policy)
         try:
             got = ops.mm_nt(x, w, residual=res)
