@@ -1219,6 +1219,32 @@ def test_expert_gradients_written_then_added(ops, block):
     ops.check_status(DEV)
 
 
+def test_shared_last_round_on_a_stream_first_used_under_capture(ops):
+    """A capture can neither allocate the workspace nor clear it: the product runs unsplit, in the capture and in every replay."""
+    ext = ops.ext
+    torch.manual_seed(63)
+    x, w = _rand(1280, 2048), _rand(4096, 2048, scale=0.05)
+    prev_policy, prev_split = ext.gemm_set_pair_policy(0), ext.gemm_set_split(0)
+    try:
+        unsplit = ops.mm_nt(x, w)
+        ext.gemm_set_split(1)
+        out = torch.empty_like(unsplit)
+        side = [torch.cuda.Stream(priority=-1) for _ in range(7)][-1]        # further on in the pool than the other tests
+        graph = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            ops.mm_nt(x, w, out=out)
+        for _ in range(2):
+            out.fill_(float("nan"))
+            graph.replay()
+            torch.cuda.synchronize()
+            _close(out, unsplit.float(), 1e-2, name="captured product")
+    finally:
+        ext.gemm_set_split(prev_split)
+        ext.gemm_set_pair_policy(prev_policy)
+    ops.check_status(DEV)
+
+
 def test_multi_tensor_gradient_accumulate(ops):
     """fp32 accumulators += bf16 / fp32 gradients of many tensors in one launch per 16."""
     torch.manual_seed(71)
