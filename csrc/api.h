@@ -24,6 +24,7 @@ typedef struct MdtGemmDesc {
   int G;               // number of groups (1 for dense)
   const int* offsets;  // [G+1] device: first row of every group (multiples of 128); mode 0: NULL
   long long capacity_rows;  // mode 1: host-known upper bound of offsets[G]
+  const int* group_rows;    // optional (modes 1, 2): [G] device, rows of each group that hold something; the rest up to the next group are zero
   // A operand: bf16 [a_rows, a_cols], row stride lda.  a_mn = 0: rows are M, cols are depth.  a_mn = 1: rows are depth, cols are M.
   const void* A; long long a_rows, a_cols, lda; int a_mn;
   // B operand: bf16 [G, b_rows, b_cols].  b_mn = 0: rows are N, cols are depth.  b_mn = 1: rows are depth, cols are N.
@@ -67,7 +68,8 @@ int mdt_skinny_mm(const void* x, const void* A, void* y, int M, int K, int r, lo
                   int a_is_kr, float alpha, cudaStream_t s);
 // Kernel for 256-wide tiles: 0 the 128-row kernel, 1 / 2 the CTA-pair (cta_group::2) kernel where the shape fills
 // 256-row tiles / always, 3 / 4 the same where 256-row tiles win by a margin / always, 5 (default) the one that the
-// measured model finds faster; returns the previous policy (policy < 0 only reads it).
+// measured model finds faster, the cluster and the transposed kernel among them, 6 the transposed kernel wherever it can run
+// (modes 0 and 1, bf16 results that nothing is added to, no peers, at most 64 groups); returns the previous policy (policy < 0 only reads it).
 int mdt_gemm_set_pair_policy(int policy);
 // CTA pairs resident at once on this device (0 until the pair kernel has been launched)
 int mdt_gemm_max_pairs(void);

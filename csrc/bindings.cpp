@@ -87,7 +87,7 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
           const OptTensor& C3, bool accumulate, double alpha, const OptTensor& status, const OptTensor& tile_ready,
           const OptTensor& tile_expected, const OptTensor& row_dest_rank, const OptTensor& row_dest_row, const OptTensor& peer_out,
           const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt, const OptTensor& alpha_dev = std::nullopt,
-          const OptTensor& swiglu_g = std::nullopt, const OptTensor& swiglu_u = std::nullopt) {
+          const OptTensor& swiglu_g = std::nullopt, const OptTensor& swiglu_u = std::nullopt, const OptTensor& group_rows = std::nullopt) {
   CHECK_BF16(A); CHECK_BF16(B);
   c10::cuda::CUDAGuard guard(A.device());
   MdtGemmDesc d;
@@ -95,6 +95,10 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
   d.mode = (int)mode; d.M = (int)M; d.N = (int)N; d.K = (int)K; d.G = (int)G;
   d.offsets = offsets.has_value() ? offsets->data_ptr<int>() : nullptr;
   d.capacity_rows = capacity_rows;
+  if (group_rows.has_value()) {
+    TORCH_CHECK(group_rows->is_cuda() && group_rows->scalar_type() == at::kInt && group_rows->is_contiguous() && group_rows->numel() == G, "group_rows must be int32 [G]");
+    d.group_rows = group_rows->data_ptr<int>();
+  }
   d.A = A.data_ptr(); fill_operand(A, d.a_rows, d.a_cols, d.lda); d.a_mn = a_mn;
   d.B = B.data_ptr(); fill_operand3(B, d.b_rows, d.b_cols, d.ldb, d.b_group_stride); d.b_mn = b_mn;
   d.dual = B2.has_value();
@@ -734,8 +738,9 @@ namespace {
 void ggemm(int mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, int64_t M, int64_t N, int64_t K, int64_t G,
            const Tensor& offs, int64_t cap, const OptTensor& B2, const OptTensor& A_l, const OptTensor& B_l, bool b_mn_l, int64_t K_l,
            const OptTensor& C2, const OptTensor& C3, bool acc, double alpha, const OptTensor& status, const OptTensor& w0, const OptTensor& w1,
-           const OptTensor& s0, const OptTensor& s1, const OptTensor& s2, const OptTensor& s3) {
-  gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G, offs, cap, B2, A_l, false, B_l, std::nullopt, b_mn_l, K_l, C2, C3, acc, alpha, status, w0, w1, s0, s1, s2, s3);
+           const OptTensor& s0, const OptTensor& s1, const OptTensor& s2, const OptTensor& s3, const OptTensor& group_rows) {
+  gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G, offs, cap, B2, A_l, false, B_l, std::nullopt, b_mn_l, K_l, C2, C3, acc, alpha, status, w0, w1, s0, s1, s2, s3,
+       std::nullopt, std::nullopt, std::nullopt, std::nullopt, group_rows);
 }
 const OptTensor NONE = std::nullopt;
 }  // namespace
@@ -766,10 +771,11 @@ std::vector<Tensor> moe_block_fwd(const Tensor& x, const Tensor& ln_w, const Ten
                  &meta_c = stash[7], &rr = stash[8], &rp = stash[9], &te = stash[10], &xg = stash[11], &expert_sorted = stash[12],
                  &offs = stash[13];
     RowsHint rows_hint(meta_c.numel() > 0 ? T * top_k : 0);
+    const OptTensor rows_of = meta_c.numel() > 0 ? NONE : OptTensor(tpe);     // (rows that peers deliver are not counted here)
     auto nr = rmsnorm_fwd(x, ln_w, eps);
     const int64_t R = xg.size(0);
     Tensor h = torch::empty({R, F}, x.options()), g = torch::empty({R, F}, x.options()), u = torch::empty({R, F}, x.options());
-    ggemm(1, xg, false, w1, false, h, R, F, H, El, offs, R, w3, NONE, NONE, false, 0, g, u, false, 1.0, status, NONE, NONE, NONE, NONE, NONE, NONE);
+    ggemm(1, xg, false, w1, false, h, R, F, H, El, offs, R, w3, NONE, NONE, false, 0, g, u, false, 1.0, status, NONE, NONE, NONE, NONE, NONE, NONE, rows_of);
     Tensor out = torch::empty({T, H}, x.options());
     return {out, tpe, nr[1], nr[0], wts, idx, ys, p1, p2, p3, meta_c, rr, rp, te, xg, g, u, h, expert_sorted, offs};
   }
@@ -817,14 +823,15 @@ std::vector<Tensor> moe_block_fwd(const Tensor& x, const Tensor& ln_w, const Ten
     w0 = ep[3]; w1o = te; s0 = rr; s1 = rp; s2 = ep[1]; s3 = ep[2];
   }
   Phase::next("moe.experts");
+  const OptTensor rows_of = is_ep ? NONE : OptTensor(plan[0]);
   const int64_t R = xg.size(0);
   Tensor h = torch::empty({R, F}, x.options());
   OptTensor g, u;
   if (grad_mode) { g = torch::empty({R, F}, x.options()); u = torch::empty({R, F}, x.options()); }
-  ggemm(1, xg, false, w1, false, h, R, F, H, El, offs, cap, w3, NONE, NONE, false, 0, g, u, false, 1.0, status, w0, w1o, NONE, NONE, NONE, NONE);
+  ggemm(1, xg, false, w1, false, h, R, F, H, El, offs, cap, w3, NONE, NONE, false, 0, g, u, false, 1.0, status, w0, w1o, NONE, NONE, NONE, NONE, rows_of);
   if (is_ep && keep) xg = clone_used_rows(xg, offs);   // the receive buffer is reused by the next exchange
   Tensor y = torch::empty({R, H}, x.options());
-  ggemm(1, h, false, w2, true, y, R, H, F, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3);
+  ggemm(1, h, false, w2, true, y, R, H, F, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3, rows_of);
   Phase::next("moe.combine");
   if (!is_ep) {
     ys = y;
@@ -875,17 +882,18 @@ std::vector<Tensor> moe_block_bwd(const Tensor& dy, const std::vector<Tensor>& s
     dyg = ep[4]; cap = L.capacity_rows;
     w0 = ep[3]; w1o = te; s0 = rr; s1 = rp; s2 = ep[1]; s3 = ep[2];
   }
+  const OptTensor rows_of = is_ep ? NONE : OptTensor(state[1]);
   const int64_t R = dyg.size(0);
   Tensor dg = torch::empty({R, F}, x.options()), du = torch::empty({R, F}, x.options());
   gemm(1, dyg, false, w2, false, dg, R, F, H, El, offs, cap, NONE, NONE, false, NONE, NONE, false, 0, du, NONE, false, 1.0, status, w0, w1o, NONE, NONE, NONE,
-       NONE, NONE, NONE, g, u);                                 // dh = dy W2^T, through SwiGLU in the epilogue
-  if (!wg.empty()) { Tensor c = wg[1]; ggemm(2, h, true, dyg, true, c, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[1], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE); }
+       NONE, NONE, NONE, g, u, rows_of);                        // dh = dy W2^T, through SwiGLU in the epilogue
+  if (!wg.empty()) { Tensor c = wg[1]; ggemm(2, h, true, dyg, true, c, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[1], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE, rows_of); }
   Tensor dxg = torch::empty({R, H}, x.options());
-  ggemm(1, dg, false, w1, true, dxg, R, H, F, El, offs, cap, NONE, du, w3, true, F, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3);
+  ggemm(1, dg, false, w1, true, dxg, R, H, F, El, offs, cap, NONE, du, w3, true, F, NONE, NONE, false, 1.0, status, NONE, NONE, s0, s1, s2, s3, rows_of);
   if (!wg.empty()) {
     Tensor c1 = wg[0], c3 = wg[2];
-    ggemm(2, dg, true, xg, true, c1, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[0], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
-    ggemm(2, du, true, xg, true, c3, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[2], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE);
+    ggemm(2, dg, true, xg, true, c1, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[0], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE, rows_of);
+    ggemm(2, du, true, xg, true, c3, F, H, 0, El, offs, cap, NONE, NONE, NONE, false, 0, NONE, NONE, wg_add[2], wscale, status, NONE, NONE, NONE, NONE, NONE, NONE, rows_of);
   }
   Tensor back;
   if (!is_ep) {
@@ -907,7 +915,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("G"), py::arg("offsets"), py::arg("capacity_rows"), py::arg("B2"), py::arg("A_l"), py::arg("a_mn_l"), py::arg("B_l"), py::arg("B2_l"),
         py::arg("b_mn_l"), py::arg("K_l"), py::arg("C2"), py::arg("C3"), py::arg("accumulate"), py::arg("alpha"), py::arg("status"), py::arg("tile_ready"),
         py::arg("tile_expected"), py::arg("row_dest_rank"), py::arg("row_dest_row"), py::arg("peer_out"), py::arg("peer_arrive"),
-        py::arg("residual") = py::none(), py::arg("alpha_dev") = py::none(), py::arg("swiglu_g") = py::none(), py::arg("swiglu_u") = py::none());
+        py::arg("residual") = py::none(), py::arg("alpha_dev") = py::none(), py::arg("swiglu_g") = py::none(), py::arg("swiglu_u") = py::none(), py::arg("group_rows") = py::none());
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("x"), py::arg("w"), py::arg("dy"), py::arg("rstd"), py::arg("dres") = py::none(), py::arg("need_dw") = true);
   m.def("rmsnorm_dw", &rmsnorm_dw);

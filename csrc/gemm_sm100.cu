@@ -1158,6 +1158,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(con
   cluster_sync_all();                                             // nobody leaves while its partial tile is read
 }
 
+#include "gemm_transposed.cuh"
+
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
@@ -1314,19 +1316,72 @@ static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream
   return cudaGetLastError();
 }
 
+// The transposed pair kernel: what it can run at all.
+static bool transposed_ok(const MdtGemmDesc* d) {
+  const int G = d->G < 1 ? 1 : d->G;
+  return (d->mode == 0 || d->mode == 1) && G <= TP_GROUPS && d->a_mn == 0 && (d->K_l == 0 || d->a_mn_l == 0) && !d->c_fp32 && !d->accumulate &&
+         d->R == nullptr && d->tile_ready == nullptr && d->row_dest_rank == nullptr && d->b_ready.ready == nullptr && d->b2_ready.ready == nullptr &&
+         d->bl_ready.ready == nullptr && d->N > 128 && (!d->dual || (d->b_mn == 0 && (d->K_l == 0 || d->b_mn_l == 0)));
+}
+
+// Which row-grouped products it takes under the default policy (those that the cluster kernel would take stay there).
+// Measured in turn, microseconds, 128-row or pair kernel / transposed, 8 experts of 4096 x 14336:
+//   tokens                     77           576          1000         2000         9200
+//   gate and up (K-major)      333 / 301    395 / 342    540 / 466    800 / 735    3130 / 3110
+//   dy W2^T, SwiGLU (K-major)  208 / 175    253 / 218    330 / 300    530 / 490    1900 / 1860
+//   down (MN-major)            146 / 150    176 / 165    275 / 255    430 / 360    1940 / 1900
+//   dx, two matrices (MN)      275 / 289    360 / 322    545 / 505    920 / 785    3800 / 3950
+// MN-major weights of up to about 96 rows a group stay: 128 x 256 tiles ask for 512 adjacent bytes at a time, one CTA per tile,
+// and at one row block a group nothing is gained by exact rows.
+static bool transposed_preferred(const MdtGemmDesc* d, long long thread_rows_hint) {
+  if (d->mode != 1) return false;
+  const int G = d->G < 1 ? 1 : d->G;
+  long long rows = d->capacity_rows - 127ll * G;
+  if (thread_rows_hint > 0 && thread_rows_hint < rows) rows = thread_rows_hint;
+  return d->b_mn == 0 || rows > 96ll * G;
+}
+
+template <int KIND>
+static cudaError_t launch_transposed(const TPParams& p, long long tiles, cudaStream_t stream) {
+  static bool configured = false;
+  static int max_pairs = 0;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_tpair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(g_num_sms & ~1)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = TP_SMEM;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_sm100_tpair_kernel<KIND>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2; }
+    max_pairs = n < g_num_sms / 2 ? n : g_num_sms / 2;
+    configured = true;
+  }
+  const int limit = (g_pair_cap > 0 && g_pair_cap < max_pairs) ? g_pair_cap : max_pairs;
+  const int grid = 2 * (int)(tiles < limit ? tiles : limit);
+  gemm_sm100_tpair_kernel<KIND><<<grid, GEMM_THREADS, TP_SMEM, stream>>>(p);
+  ++g_launches;
+  return cudaGetLastError();
+}
+
 // Expected number of rows of the row-grouped products issued by this thread (0 = unknown); see mdt_gemm_rows_hint.
 static thread_local long long t_rows_hint = 0;
 
 // Which kernel takes the 256-wide tiles: 0 = the 128-row kernel always, 1 = the CTA-pair kernel where the shape
 // fills 256-row tiles, 2 and 4 = the CTA-pair kernel always (4: an older name of it), 3 = the CTA-pair kernel only where
-// 256-row tiles would win by a wide margin, 5 = whichever is faster by the measured model (default).  Initial value from
+// 256-row tiles would win by a wide margin, 5 = whichever is faster by the measured models (default; the cluster and the
+// transposed pair kernel only here), 6 = the transposed pair kernel wherever it can run.  Initial value from
 // MDT_GEMM_PAIR; mdt_gemm_set_pair_policy() changes it.
-constexpr int MAX_POLICY = 5;
+constexpr int MAX_POLICY = 6;
+constexpr int DEFAULT_POLICY = 5;
 static int g_pair_policy = -1;
 static int pair_policy() {
   if (g_pair_policy < 0) {
     const char* e = getenv("MDT_GEMM_PAIR");
-    g_pair_policy = (e != nullptr && e[0] >= '0' && e[0] <= '0' + MAX_POLICY) ? e[0] - '0' : MAX_POLICY;
+    g_pair_policy = (e != nullptr && e[0] >= '0' && e[0] <= '0' + MAX_POLICY) ? e[0] - '0' : DEFAULT_POLICY;
   }
   return g_pair_policy;
 }
@@ -1515,6 +1570,37 @@ extern "C" int mdt_gemm_set_pair_policy(int policy) {
   return old;
 }
 
+namespace mdt {
+// The descriptor for the transposed pair kernel (transposed_ok has answered for it).
+static int gemm_transposed(const MdtGemmDesc* d, cudaStream_t stream) {
+  TPParams p;
+  memset(&p, 0, sizeof(p));
+  p.M = d->M; p.N = d->N; p.K = d->K; p.K_l = d->K_l; p.G = d->G < 1 ? 1 : d->G; p.mode = d->mode;
+  p.w_mn = d->b_mn; p.w_mn_l = d->b_mn_l;
+  p.offsets = d->offsets; p.group_rows = d->group_rows;
+  p.C = d->C; p.C2 = d->C2; p.C3 = d->C3; p.swiglu_g = d->swiglu_g; p.swiglu_u = d->swiglu_u;
+  p.ldc = d->ldc; p.alpha = d->alpha; p.alpha_dev = d->alpha_dev; p.status = d->status;
+  const uint32_t w_rows = d->dual ? 16 : (d->b_mn ? 64 : BM), wl_rows = d->dual ? 16 : (d->b_mn_l ? 64 : BM);
+  int rc = make_map(&p.tmW, d->B, d->b_cols, d->b_rows, p.G, d->ldb, d->b_group_stride, 64, w_rows, 3);
+  if (d->dual) rc |= make_map(&p.tmW2, d->B2, d->b_cols, d->b_rows, p.G, d->ldb, d->b_group_stride, 64, w_rows, 3);
+  for (int i = 0; i < 4; ++i) rc |= make_map(&p.tmX[i], d->A, d->a_cols, d->a_rows, 1, d->lda, 0, 64, 16u << i, 2);
+  if (d->K_l > 0) {
+    rc |= make_map(&p.tmW_l, d->B_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, wl_rows, 3);
+    if (d->dual) rc |= make_map(&p.tmW2_l, d->B2_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, wl_rows, 3);
+    for (int i = 0; i < 4; ++i) rc |= make_map(&p.tmX_l[i], d->A_l, d->al_cols, d->al_rows, 1, d->lda_l, 0, 64, 16u << i, 2);
+  }
+  if (rc != 0) return rc;
+  const int width = d->dual ? 128 : 256;
+  const long long rows = d->mode == 1 ? d->capacity_rows : d->M;
+  const long long tiles = ((rows + 255) / 256 + (d->mode == 1 ? p.G : 0)) * ((p.N + width - 1) / width);       // an upper bound
+  SplitWorkspace w;
+  if (split_enabled() && tiles > g_num_sms / 2 && split_workspace(stream, &w)) { p.sk_ws = w.ws; p.sk_ctr = w.ctr; }
+  const cudaError_t e = d->dual ? launch_transposed<TP_DUAL>(p, tiles, stream)
+                      : (d->swiglu_g != nullptr ? launch_transposed<TP_SWIGLU_BWD>(p, tiles, stream) : launch_transposed<TP_PLAIN>(p, tiles, stream));
+  return e == cudaSuccess ? 0 : -100 - (int)e;
+}
+}  // namespace mdt
+
 extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   using namespace mdt;
   // Tensor-map encoding is a driver call: make sure this host thread has the device's primary context
@@ -1552,7 +1638,9 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   const int BN = (p.dual || p.N > 128) ? 256 : 128;
   const int bn_out = p.dual ? BN / 2 : BN;
   int cluster_bn = 0;
-  const int cluster = pair_policy() == MAX_POLICY ? choose_cluster(d, t_rows_hint, max_clusters, &cluster_bn) : 0;
+  const int cluster = pair_policy() == DEFAULT_POLICY ? choose_cluster(d, t_rows_hint, max_clusters, &cluster_bn) : 0;
+  if (cluster == 0 && pair_policy() >= DEFAULT_POLICY && transposed_ok(d) && (pair_policy() == MAX_POLICY || transposed_preferred(d, t_rows_hint)))
+    return gemm_transposed(d, stream);
   const bool pair = cluster == 0 && choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms) != 0;
   const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
   int rc = 0;

@@ -1,0 +1,478 @@
+// Transposed CTA-pair kernel of the GEMM family: the weight matrix is the 256-row operand of the MMA, the token rows are its N.
+// Included by gemm_sm100.cu, whose helpers it uses.
+//
+//   D[features, rows] = W[features, k] * X[rows, k]^T,   C[row, feature] = D^T through SwiGLU, its backward, or nothing
+//
+// Why: the token rows of an expert come in any number (a micro-batch leaves 30 to 300 for each of 8), the weights always in
+// thousands.  With tokens as M a group of 144 rows is two 128-row tiles, one of them holding 16 rows, and the weights pass
+// through the SMs once for each; as N it is one 160-wide tile.  A pair takes 256 + n clocks per k block of n rows (shared
+// memory: 2 x (32 KB of weights + n x 128 bytes) through 2 SMs' 128 bytes per clock), against 700 that the weights' 32 KB take
+// from HBM, so that up to about 400 rows a group the products run at the rate of the weights.
+//
+// Rows of a group are cut into tiles of equal numbers of 32-row units, at most 8 (256 rows).  Only rows that exist are
+// multiplied where the caller passes their number (group_rows); the padding up to the next 128-row boundary, zero by contract,
+// gives zeros, which are written without being computed.  The tiles of the last, partly filled round are cut along the depth
+// over all pairs as in the 128-row kernel (get_work): 128 tiles of a down projection are 1.73 rounds of 74 pairs.
+//
+// Epilogue: TMEM is read in 16 x 256-bit pieces, whose register layout is the one that stmatrix transposes, so that rows of C
+// leave through a 4 KB stage per warp in 16-byte pieces without shuffles.  In the gate / up form the 128 rows of a CTA's
+// operand alternate between 16 gate and 16 up features: both values of one output then land in the same thread.
+
+constexpr int TP_GROUPS = 64;      // row groups that fit the table in shared memory
+constexpr int TP_UNIT = 32;        // rows: N of a pair's MMA is a multiple of 32
+constexpr int TP_A_BYTES = BM * BK * 2;
+// The ring: stages of 16 KB of weights and as many rows as the widest tile has.  Six of 256 rows, ten of 32: what bounds the
+// products of few rows is the bytes of weights in flight.
+constexpr int TP_RING_BYTES = 6 * (TP_A_BYTES + 128 * BK * 2);
+constexpr int TP_MAX_STAGES = 10;
+struct TPTable { int start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, units, groups, row_tiles; };
+constexpr int TP_SMEM = TP_RING_BYTES + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES + (int)sizeof(TPTable);
+static_assert(TP_SMEM <= 227 * 1024, "transposed pair kernel: shared memory of a CTA");
+
+enum : int { TP_PLAIN = 0, TP_DUAL = 1, TP_SWIGLU_BWD = 2 };
+
+struct TPParams {
+  CUtensorMap tmW, tmW2, tmW_l, tmW2_l;   // weights (tmW2: the up matrix of the gate / up form), main and short depth segment
+  CUtensorMap tmX[4], tmX_l[4];           // token rows in boxes of 16, 32, 64 and 128 rows
+  int M, N, K, K_l, G, mode, w_mn, w_mn_l;
+  const int* offsets; const int* group_rows;
+  void* C; void* C2; void* C3;
+  const void* swiglu_g; const void* swiglu_u;
+  long long ldc;
+  float alpha; const float* alpha_dev;
+  int* status;
+  float* sk_ws; unsigned* sk_ctr;
+};
+// rows [row0, row0 + n) x features [f0, f0 + 256 or 128), rows below `end` are stored; zero0: first row to be cleared (= end: none)
+struct TPTile { int g, f0, row0, n, end, zero0; };
+struct TPWork { TPTile t; int kb0, kb1, split, contributors; };
+
+__host__ __device__ __forceinline__ int tp_tiles_of_rows(int rows) { return ((rows + TP_UNIT - 1) / TP_UNIT + 7) / 8; }
+
+// One thread per group fills the table; a warp scan gives the first tile of each group.
+__device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, int f_tiles, int lane) {
+  int carry = 0, widest = 0, units_all = 0, groups = 0;
+  for (int g0 = 0; g0 < p.G; g0 += 32) {
+    const int g = g0 + lane;
+    int tiles = 0;
+    if (g < p.G) {
+      const int start = p.mode == 1 ? p.offsets[g] : 0, end = p.mode == 1 ? p.offsets[g + 1] : p.M;
+      int rows = end - start;
+      if (p.group_rows != nullptr && p.group_rows[g] < rows) rows = p.group_rows[g];
+      tb->start[g] = start; tb->rows[g] = rows; tb->end[g] = end;
+      tiles = tp_tiles_of_rows(rows) * f_tiles;
+      const int units = (rows + TP_UNIT - 1) / TP_UNIT, nt = (units + 7) / 8;
+      if (nt > 0) { widest = max(widest, (units + nt - 1) / nt * TP_UNIT); ++groups; }
+      units_all += units;
+    }
+    int incl = tiles;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+    if (g < p.G) tb->tile0[g] = carry + incl - tiles;
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  widest = __reduce_max_sync(0xffffffffu, widest);
+  units_all = __reduce_add_sync(0xffffffffu, units_all);
+  groups = __reduce_add_sync(0xffffffffu, groups);
+  if (lane == 0) { tb->tile0[p.G] = carry; tb->widest = widest; tb->units = units_all; tb->groups = groups; tb->row_tiles = carry / f_tiles; }
+}
+
+__host__ __device__ __forceinline__ void tp_tile(const TPTable* tb, int G, int f_tiles, int f_width, int t, TPTile& o) {
+  int g = 0;
+  while (g + 1 < G && t >= tb->tile0[g + 1]) ++g;
+  const int units = (tb->rows[g] + TP_UNIT - 1) / TP_UNIT, nt = (units + 7) / 8;
+  int n, f;
+  panel_order(t - tb->tile0[g], nt, f_tiles, 8, n, f);      // rows fastest: the tiles that share weights run together
+  const int base = units / nt, extra = units % nt;
+  o.g = g;
+  o.f0 = f * f_width;
+  o.row0 = tb->start[g] + (n * base + (n < extra ? n : extra)) * TP_UNIT;
+  o.n = (base + (n < extra ? 1 : 0)) * TP_UNIT;
+  o.end = tb->end[g];
+  o.zero0 = n == nt - 1 && o.row0 + o.n < o.end ? o.row0 + o.n : o.end;
+}
+
+// Whether the last round of `rem` tiles is shared along the depth by all pairs.  In clocks: a k block of n rows takes a pair
+// 1.25 * (256 + n), or 704 where its weights come from memory and all pairs ask for some (a tile's share of that is smaller
+// where several tiles read the same weights); sharing costs 8 000 and 90 for each row of the tiles.  Measured, microseconds with
+// / without sharing: down projection, 8 experts, 16 tokens 159 / 152, 1000 tokens 261 / 253, 2000 tokens 357 / 395; gate and up of 16
+// tokens 303 / 313; dense 9200 x 4096 x 4096 197 / 184, 1152 x 4096 x 4096 49 / 53.
+__host__ __device__ __forceinline__ bool tp_split_pays(const TPTable* tb, int f_tiles, int kbt, int rem, int pairs) {
+  const int row_tiles = tb->row_tiles;
+  const float rows = 32.f * (float)tb->units / (float)row_tiles, shared = (float)row_tiles / (float)tb->groups;
+  const float step = 1.25f * (256.f + rows), memory = 704.f / shared, part = (float)rem / (float)pairs;
+  return (float)kbt * fmaxf(step, memory * part) > (float)kbt * fmaxf(step, memory) * part + 8000.f + 90.f * rows;
+}
+
+// it = 0, 1, ...: the work of pair `pair` of `pairs`.  The tiles of a last round that leaves more than an eighth of the pairs
+// idle are cut into one contiguous piece of k blocks per pair (see get_work), no piece shorter than 4 blocks.
+__host__ __device__ __forceinline__ bool tp_work(const TPTable* tb, int G, int f_tiles, int f_width, int kbt, bool may_split, int pair, int pairs, int it, TPWork& w) {
+  const int total = tb->tile0[G];
+  int whole = total;
+  const int rem = total % pairs;
+  if (may_split && total > pairs && rem != 0 && kbt >= 8 && tp_split_pays(tb, f_tiles, kbt, rem, pairs)) whole = total - rem;
+  const int n_whole = whole > pair ? (whole - pair + pairs - 1) / pairs : 0;
+  w.split = -1; w.contributors = 1;
+  if (it < n_whole) {
+    tp_tile(tb, G, f_tiles, f_width, pair + it * pairs, w.t);
+    w.kb0 = 0; w.kb1 = kbt;
+    return true;
+  }
+  if (whole == total) return false;
+  const int units = rem * kbt;
+  int per = (units + pairs - 1) / pairs;
+  if (per < 4) per = 4;
+  const int u0 = pair * per, u1 = u0 + per < units ? u0 + per : units;
+  if (u0 >= u1) return false;
+  const int tt = u0 / kbt + (it - n_whole);
+  if (tt > (u1 - 1) / kbt) return false;
+  tp_tile(tb, G, f_tiles, f_width, whole + tt, w.t);
+  const int lo = tt * kbt, hi = lo + kbt;
+  w.kb0 = (u0 > lo ? u0 : lo) - lo;
+  w.kb1 = (u1 < hi ? u1 : hi) - lo;
+  w.contributors = (hi - 1) / per - lo / per + 1;
+  w.split = w.contributors > 1 ? tt : -1;
+  return true;
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// A warp's stage: rows of 64 bytes (32 features) or, in the gate / up form, of 32 bytes (16 features); the 16-byte pieces are
+// swizzled by the row so that eight consecutive rows' pieces fall into different banks.
+__device__ __forceinline__ uint32_t tp_slot64(int row, int piece) { return row * 64 + ((piece ^ ((row >> 1) & 3)) << 4); }
+__device__ __forceinline__ uint32_t tp_slot32(int row, int piece) { return row * 32 + ((piece ^ ((row >> 2) & 1)) << 4); }
+
+// Rows [first, end) of a warp's features are cleared.
+template <int KIND>
+__device__ __forceinline__ void tp_clear(const TPParams& p, int first, int end, int col, int half, int lane) {
+  constexpr int PIECES = KIND == TP_DUAL ? 2 : 4, STEP = 32 / PIECES;
+  const int c = col + (lane % PIECES) * 8;
+  if (c >= p.N) return;
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  for (int row = first + half * STEP + lane / PIECES; row < end; row += 2 * STEP) {
+    const long long at = (long long)row * p.ldc + c;
+    *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C) + at) = z;
+    if (KIND != TP_PLAIN && p.C2 != nullptr) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C2) + at) = z;
+    if (KIND == TP_DUAL && p.C3 != nullptr) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.C3) + at) = z;
+  }
+}
+// The stage's 32 rows to the rows of `out` from `row0` on.
+template <int KIND>
+__device__ __forceinline__ void tp_store(const TPParams& p, void* out, const uint8_t* stage, int row0, int end, int col, int lane) {
+  constexpr int PIECES = KIND == TP_DUAL ? 2 : 4, STEP = 32 / PIECES;
+  const int piece = lane % PIECES, c = col + piece * 8;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int r = i * STEP + lane / PIECES;
+    const uint4 v = *reinterpret_cast<const uint4*>(stage + (KIND == TP_DUAL ? tp_slot32(r, piece) : tp_slot64(r, piece)));
+    if (row0 + r < end && c < p.N) *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + (long long)(row0 + r) * p.ldc + c) = v;
+  }
+}
+// 32 rows of `src` into registers, as tp_store lays them out
+__device__ __forceinline__ void tp_fetch(uint4 (&v)[4], const TPParams& p, const void* src, int row0, int end, int col, int lane) {
+  const int c = col + (lane & 3) * 8;
+  const uint4* at[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + i * 8 + (lane >> 2);
+    at[i] = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(src) + (row < end && c < p.N ? (long long)row * p.ldc + c : 0));
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __ldcg(at[i]);
+}
+
+// One warp's part of a tile: its 32 TMEM lanes, every second chunk of 32 rows from `half` on.  `load(c, lo, hi)` brings the
+// accumulators of chunk c: lo of the lanes 0-15, hi of 16-31 of the warp's quarter.  `ready` is called before the first one.
+template <int KIND, class Ready, class Load>
+__device__ __forceinline__ bool tp_epilogue(const TPParams& p, uint8_t* stage, const TPTile& t, int col, int half, int lane, float alpha, Ready ready, Load load) {
+  const int chunks = t.n / TP_UNIT;
+  const uint32_t st = smem_u32(stage);
+  uint4 pg[4], pu[4];
+  if constexpr (KIND == TP_SWIGLU_BWD) {
+    if (half < chunks) { tp_fetch(pg, p, p.swiglu_g, t.row0 + half * 32, t.end, col, lane); tp_fetch(pu, p, p.swiglu_u, t.row0 + half * 32, t.end, col, lane); }
+  }
+  if (!ready()) return false;
+#pragma unroll 1
+  for (int c = half; c < chunks; c += 2) {
+    const int row0 = t.row0 + c * 32;
+    uint32_t lo[16], hi[16];
+    load(c, lo, hi);
+    if constexpr (KIND == TP_PLAIN) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        auto v = [&](const uint32_t (&a)[16], int i) { return __uint_as_float(a[4 * j + i]) * alpha; };
+        stmatrix_x4_trans(st + tp_slot64(8 * j + (lane & 7), lane >> 3), pack_bf16(v(lo, 0), v(lo, 1)), pack_bf16(v(lo, 2), v(lo, 3)),
+                          pack_bf16(v(hi, 0), v(hi, 1)), pack_bf16(v(hi, 2), v(hi, 3)));
+      }
+      __syncwarp();
+      tp_store<KIND>(p, p.C, stage, row0, t.end, col, lane);
+    } else if constexpr (KIND == TP_DUAL) {
+      auto put = [&](int mat, auto value) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int r = 16 * j + (lane >> 4) * 8 + (lane & 7);
+          stmatrix_x4_trans(st + mat * 1024 + tp_slot32(r, (lane >> 3) & 1), pack_bf16(value(8 * j), value(8 * j + 1)), pack_bf16(value(8 * j + 2), value(8 * j + 3)),
+                            pack_bf16(value(8 * j + 4), value(8 * j + 5)), pack_bf16(value(8 * j + 6), value(8 * j + 7)));
+        }
+      };
+      const bool keep = p.C2 != nullptr;
+      if (keep) {
+        put(1, [&](int i) { return __uint_as_float(lo[i]); });
+        put(2, [&](int i) { return __uint_as_float(hi[i]); });
+      }
+      put(0, [&](int i) { const float g = __uint_as_float(lo[i]); return g / (1.0f + __expf(-g)) * __uint_as_float(hi[i]); });
+      __syncwarp();
+      tp_store<KIND>(p, p.C, stage, row0, t.end, col, lane);
+      if (keep) {
+        tp_store<KIND>(p, p.C2, stage + 1024, row0, t.end, col, lane);
+        tp_store<KIND>(p, p.C3, stage + 2048, row0, t.end, col, lane);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = i * 8 + (lane >> 2);
+        *reinterpret_cast<uint4*>(stage + tp_slot64(r, lane & 3)) = pg[i];
+        *reinterpret_cast<uint4*>(stage + 2048 + tp_slot64(r, lane & 3)) = pu[i];
+      }
+      __syncwarp();
+      if (c + 2 < chunks) { tp_fetch(pg, p, p.swiglu_g, row0 + 64, t.end, col, lane); tp_fetch(pu, p, p.swiglu_u, row0 + 64, t.end, col, lane); }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // (each piece of the stage is read here by the lanes of one instruction before the same instruction group writes it)
+        const uint32_t at = st + tp_slot64(8 * j + (lane & 7), lane >> 3);
+        uint32_t g[4], u[4];
+        ldmatrix_x4_trans(at, g[0], g[1], g[2], g[3]);
+        ldmatrix_x4_trans(at + 2048, u[0], u[1], u[2], u[3]);
+        uint32_t dg[4], du[4];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+          const float2 gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g[m])), uf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[m]));
+          const float d0 = __uint_as_float(m < 2 ? lo[4 * j + 2 * m] : hi[4 * j + 2 * (m - 2)]) * alpha;
+          const float d1 = __uint_as_float(m < 2 ? lo[4 * j + 2 * m + 1] : hi[4 * j + 2 * (m - 2) + 1]) * alpha;
+          const float s0 = 1.f / (1.f + __expf(-gf.x)), s1 = 1.f / (1.f + __expf(-gf.y));
+          du[m] = pack_bf16(d0 * (gf.x * s0), d1 * (gf.y * s1));
+          dg[m] = pack_bf16(d0 * uf.x * s0 * (1.f + gf.x * (1.f - s0)), d1 * uf.y * s1 * (1.f + gf.y * (1.f - s1)));
+        }
+        __syncwarp();
+        stmatrix_x4_trans(at, dg[0], dg[1], dg[2], dg[3]);
+        stmatrix_x4_trans(at + 2048, du[0], du[1], du[2], du[3]);
+      }
+      __syncwarp();
+      tp_store<KIND>(p, p.C, stage, row0, t.end, col, lane);
+      tp_store<KIND>(p, p.C2, stage + 2048, row0, t.end, col, lane);
+    }
+    __syncwarp();       // the stage is free again
+  }
+  return true;
+}
+
+template <int KIND>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_tpair_kernel(const __grid_constant__ TPParams p) {
+  constexpr int F_WIDTH = KIND == TP_DUAL ? 128 : 256;      // output features of a tile
+  constexpr uint32_t TMEM_COLS = 512;
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + TP_RING_BYTES);
+  uint64_t* empty_bar = full_bar + TP_MAX_STAGES;
+  uint64_t* tfull_bar = empty_bar + TP_MAX_STAGES;
+  uint64_t* tempty_bar = tfull_bar + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint8_t* epi_stage = smem + TP_RING_BYTES + 256;
+  TPTable* tb = reinterpret_cast<TPTable*>(epi_stage + EPI_WARPS * EPI_STAGE_BYTES);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_ctarank();          // 0 = leader
+  const int pair_id = (int)cluster_id_x(), num_pairs = (int)num_clusters_x();
+  const int f_tiles = (p.N + F_WIDTH - 1) / F_WIDTH;
+  const int num_kb = (p.K + BK - 1) / BK, kbt = num_kb + (p.K_l + BK - 1) / BK;
+  const bool may_split = p.sk_ws != nullptr;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < TP_MAX_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * EPI_WARPS); }
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
+  if (warp == 2) tp_fill_table(p, tb, f_tiles, lane);
+  tc_fence_before();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int stage_bytes = TP_A_BYTES + tb->widest * (BK * 2 / 2);
+  const int stages = min(TP_RING_BYTES / stage_bytes, TP_MAX_STAGES);
+
+  auto fail = [&](int code) {
+    *abort_flag = 1;
+    if (p.status != nullptr) atomicCAS(p.status, 0, code);
+  };
+  TPWork w;
+  auto next = [&](int it) { return tp_work(tb, p.G, f_tiles, F_WIDTH, kbt, may_split, pair_id, num_pairs, it, w); };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer (one per CTA)
+    if (elect_one()) { prefetch_tensormap(&p.tmW); prefetch_tensormap(&p.tmX[3]); }
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int wi = 0; ok && next(wi); ++wi) {
+      const TPTile& t = w.t;
+      const int rows = t.n / 2, row0 = t.row0 + rank * rows;       // this CTA's rows of the N operand
+      const int f0 = t.f0 + rank * (F_WIDTH / 2);
+      const uint32_t bytes = 2 * (TP_A_BYTES + rows * (BK * 2));
+      for (int kb = w.kb0; kb < w.kb1; ++kb) {
+        if (!wait_parity_warp(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
+        uint8_t* sW = smem + s * stage_bytes;
+        uint8_t* sX = sW + TP_A_BYTES;
+        // (only the leader arrives, see the pair kernel)
+        const uint32_t bar = mapa_shared(smem_u32(&full_bar[s]), 0);
+        const bool second = kb >= num_kb;
+        const int kk = (second ? kb - num_kb : kb) * BK;
+        const CUtensorMap* mW = second ? &p.tmW_l : &p.tmW;
+        const CUtensorMap* mW2 = second ? &p.tmW2_l : &p.tmW2;
+        const int w_mn = second ? p.w_mn_l : p.w_mn;
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(&full_bar[s], bytes);
+          if (KIND == TP_DUAL) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              tma_load_3d_pair(sW + j * 4096, mW, bar, kk, f0 + 16 * j, t.g);
+              tma_load_3d_pair(sW + j * 4096 + 2048, mW2, bar, kk, f0 + 16 * j, t.g);
+            }
+          } else if (w_mn == 0) {
+            tma_load_3d_pair(sW, mW, bar, kk, f0, t.g);
+          } else {
+            tma_load_3d_pair(sW, mW, bar, f0, kk, t.g);
+            tma_load_3d_pair(sW + 8192, mW, bar, f0 + 64, kk, t.g);
+          }
+          const CUtensorMap* mX = second ? p.tmX_l : p.tmX;
+          int done = 0;
+#pragma unroll
+          for (int b = 3; b >= 0; --b)
+            if (rows & (16 << b)) { tma_load_2d_pair(sX + done * (BK * 2), mX + b, bar, kk, row0 + done); done += 16 << b; }
+        }
+        if (++s == stages) { s = 0; ph ^= 1; }
+      }
+    }
+    if (!ok) {  // give this CTA's copies already in flight a bounded time to land before it leaves
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {}
+    }
+  } else if (warp == 1 && rank == 0) {
+    // ------------------------------------------------------------------ MMA issuer (leader only)
+    int s = 0;
+    uint32_t ph = 0, acc_it = 0;
+    bool ok = true;
+    for (int wi = 0; ok && next(wi); ++wi) {
+      const int buf = acc_it & 1;
+      const uint32_t aph = (acc_it >> 1) & 1;
+      if (!wait_parity_warp(&tempty_bar[buf], aph ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * 256;
+      for (int kb = w.kb0; kb < w.kb1; ++kb) {
+        if (!wait_parity_warp(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
+        tc_fence_after();
+        const int w_mn = kb >= num_kb ? p.w_mn_l : p.w_mn;
+        const uint32_t idesc = make_idesc_bf16(2 * BM, w.t.n, w_mn, 0);
+        const uint32_t sW = smem_u32(smem + s * stage_bytes);
+        const uint64_t dw = operand_desc(sW, w_mn), dx = operand_desc(sW + TP_A_BYTES, 0);
+        const uint32_t kw = operand_kstep(w_mn), kx = operand_kstep(0);
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16_pair(d_tmem, dw + k * kw, dx + k * kx, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+          umma_commit_pair(&empty_bar[s], 3);   // frees the stage in both CTAs
+        }
+        if (++s == stages) { s = 0; ph ^= 1; }
+      }
+      if (!ok) break;
+      if (elect_one()) umma_commit_pair(&tfull_bar[buf], 3);   // accumulators complete, in both CTAs
+      ++acc_it;
+    }
+  } else if (warp >= 2) {
+    // ------------------------------------------------------------------ epilogue (both CTAs, own 128 operand rows)
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint8_t* stage = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
+    const float alpha = p.alpha_dev != nullptr ? p.alpha * *p.alpha_dev : p.alpha;
+    uint32_t acc_it = 0;
+    for (int wi = 0; next(wi); ++wi) {
+      const TPTile& t = w.t;
+      const int col = t.f0 + rank * (F_WIDTH / 2) + q * (F_WIDTH / 8);        // this warp's first output feature
+      const int buf = acc_it & 1;
+      const uint32_t aph = (acc_it >> 1) & 1;
+      const uint32_t tacc = tmem_base + buf * 256 + ((uint32_t)(q * 32) << 16);
+      if (w.kb0 == 0) tp_clear<KIND>(p, t.zero0, t.end, col, half, lane);     // under the wait for the accumulator
+      auto ready = [&]() {
+        if (!wait_parity_warp(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
+        tc_fence_after();
+        return true;
+      };
+      auto from_tmem = [&](int c, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
+        tmem_ld_16x256b_x4(tacc + c * 32, lo);
+        tmem_ld_16x256b_x4(tacc + c * 32 + (16u << 16), hi);
+        tmem_ld_wait();
+      };
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
+        ++acc_it;
+      };
+      if (w.split < 0) {
+        if (!tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, ready, from_tmem)) break;
+        release();
+        continue;
+      }
+      // A piece of a shared tile: partial sums into the fp32 workspace, whole 512-byte lines per reduction; the warp that
+      // comes last at its part of the tile reads them back, clears them and finishes the part.
+      const int part = (w.split * 2 + rank) * EPI_WARPS + half * 4 + q;
+      float4* ws = reinterpret_cast<float4*>(p.sk_ws) + (long long)part * (4 * 8 * 32) + lane;
+      if (!ready()) break;
+#pragma unroll 1
+      for (int c = half; c < t.n / TP_UNIT; c += 2) {
+        uint32_t lo[16], hi[16];
+        from_tmem(c, lo, hi);
+        float4* at = ws + (c >> 1) * 256;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          red_add_v4_f32(reinterpret_cast<float*>(at + i * 32), __uint_as_float(lo[4 * i]), __uint_as_float(lo[4 * i + 1]), __uint_as_float(lo[4 * i + 2]), __uint_as_float(lo[4 * i + 3]));
+          red_add_v4_f32(reinterpret_cast<float*>(at + (4 + i) * 32), __uint_as_float(hi[4 * i]), __uint_as_float(hi[4 * i + 1]), __uint_as_float(hi[4 * i + 2]), __uint_as_float(hi[4 * i + 3]));
+        }
+      }
+      release();
+      if (half >= t.n / TP_UNIT) continue;
+      __threadfence();
+      __syncwarp();
+      unsigned before = 0;
+      if (lane == 0) before = atomicAdd(p.sk_ctr + part, 1u);
+      before = __shfl_sync(0xffffffffu, before, 0);
+      if (before != (unsigned)w.contributors - 1u) continue;
+      __threadfence();
+      auto from_ws = [&](int c, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
+        float4* at = ws + (c >> 1) * 256;
+        float4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __ldcg(at + i * 32);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) __stcg(at + i * 32, make_float4(0.f, 0.f, 0.f, 0.f));     // leave the workspace clean
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          lo[4 * i] = __float_as_uint(v[i].x); lo[4 * i + 1] = __float_as_uint(v[i].y); lo[4 * i + 2] = __float_as_uint(v[i].z); lo[4 * i + 3] = __float_as_uint(v[i].w);
+          hi[4 * i] = __float_as_uint(v[4 + i].x); hi[4 * i + 1] = __float_as_uint(v[4 + i].y); hi[4 * i + 2] = __float_as_uint(v[4 + i].z); hi[4 * i + 3] = __float_as_uint(v[4 + i].w);
+        }
+      };
+      tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, []() { return true; }, from_ws);
+      if (lane == 0) p.sk_ctr[part] = 0;
+    }
+  }
+
+  // Neither CTA may leave while its partner can still read its shared memory or arrive on its barriers.
+  __syncwarp();
+  tc_fence_before();
+  cluster_sync_all();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc_pair(tmem_base, TMEM_COLS); }
+}

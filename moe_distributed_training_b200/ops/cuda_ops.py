@@ -49,14 +49,14 @@ def launch_count() -> int:
 
 def _gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G=1, offsets=None, capacity=0, B2=None, A_l=None, a_mn_l=False,
           B_l=None, B2_l=None, b_mn_l=False, K_l=0, C2=None, C3=None, accumulate=False, alpha=1.0, wait=None, scatter=None,
-          residual=None, alpha_dev=None, swiglu=None):
+          residual=None, alpha_dev=None, swiglu=None, group_rows=None):
     """alpha_dev: optional fp32 scalar on the GPU that multiplies alpha.  wait = (tile_ready, tile_expected): A rows arrive from peers, tile by tile.  scatter = (row_rank, row_pos,
     peer_out table, peer_arrive table): result rows are stored into peers' buffers instead of C.  swiglu = (g, u): the product
     is the gradient of silu(g) * u; the gradients of g and u go to C and C2."""
     w0, w1 = wait if wait is not None else (None, None)
     s0, s1, s2, s3 = scatter if scatter is not None else (None, None, None, None)
     ext.gemm(mode, A, a_mn, B, b_mn, C, M, N, K, G, offsets, capacity, B2, A_l, a_mn_l, B_l, B2_l, b_mn_l, K_l,
-             C2, C3, accumulate, alpha, status_tensor(A.device), w0, w1, s0, s1, s2, s3, residual, alpha_dev, *(swiglu if swiglu is not None else (None, None)))
+             C2, C3, accumulate, alpha, status_tensor(A.device), w0, w1, s0, s1, s2, s3, residual, alpha_dev, *(swiglu if swiglu is not None else (None, None)), group_rows)
     return C
 
 
@@ -235,8 +235,10 @@ def combine_rows(y, plan, weights):
 # ----------------------------------------------------------------------------------------------- expert MLP
 def _g(mode, A, a_mn, B, b_mn, C, N, K, plan, **kw):
     G = C.shape[0] if mode == 2 else (B.shape[0] if B.dim() == 3 else 1)
+    # (a plan without a slot map describes a receive buffer, which peers fill while the product runs)
+    rows = plan.tokens_per_expert if plan.src_slot is not None else None
     return _gemm(mode, A, a_mn, B, b_mn, C, C.shape[-2] if mode == 2 else A.shape[0], N, K, G=G,
-                 offsets=plan.padded_offsets, capacity=plan.capacity, **kw)
+                 offsets=plan.padded_offsets, capacity=plan.capacity, group_rows=rows, **kw)
 
 
 class _GroupedSwiGLUMLP(torch.autograd.Function):
@@ -263,9 +265,10 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
             t13 = torch.empty(R, 2 * r, dtype=dt, device=dev)
             _g(1, xg, False, A13, True, t13, 2 * r, H, plan, wait=wait)
             wait = None
-            z = torch.zeros_like(B1)
-            B1p, B3p = torch.cat([B1, z], dim=1).contiguous(), torch.cat([z, B3], dim=1).contiguous()  # [E,2r,F]
-            kw = dict(A_l=t13, B_l=B1p, B2_l=B3p, b_mn_l=True, K_l=2 * r)
+            # [E, F, 2r]: the gate / up product wants adapters laid out like w1 and w3
+            z = B1.new_zeros(E, F, r)
+            B1p, B3p = torch.cat([B1.transpose(1, 2), z], dim=2), torch.cat([z, B3.transpose(1, 2)], dim=2)
+            kw = dict(A_l=t13, B_l=B1p, B2_l=B3p, b_mn_l=False, K_l=2 * r)
         h = torch.empty(R, F, dtype=dt, device=dev)
         g = u = None
         if need_grad:

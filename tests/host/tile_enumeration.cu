@@ -94,8 +94,83 @@ static int check_work(const GemmParams& p, int num_ctas, const std::vector<int>&
   return bad;
 }
 
+// The transposed pair kernel (tp_work): every (32-row unit, feature tile, k block) of the rows that exist exactly once; tiles inside
+// their group; the padding of a group cleared by exactly one whole column of tiles; shared tiles as above, one per pair at most.
+static int check_transposed(const std::vector<int>& start, const std::vector<int>& rows, const std::vector<int>& end, int N, int f_width, int kbt, int pairs, bool split) {
+  TPTable tb;
+  const int G = (int)rows.size(), f_tiles = (N + f_width - 1) / f_width;
+  int tiles = 0;
+  tb.widest = tb.units = tb.groups = 0;
+  for (int g = 0; g < G; ++g) {
+    const int units = (rows[g] + TP_UNIT - 1) / TP_UNIT, nt = (units + 7) / 8;
+    tb.start[g] = start[g]; tb.rows[g] = rows[g]; tb.end[g] = end[g]; tb.tile0[g] = tiles;
+    if (nt != tp_tiles_of_rows(rows[g])) return 1;
+    tiles += nt * f_tiles;
+    tb.units += units;
+    if (nt > 0) { ++tb.groups; const int w = (units + nt - 1) / nt * TP_UNIT; if (w > tb.widest) tb.widest = w; }
+  }
+  tb.tile0[G] = tiles;
+  tb.row_tiles = tiles / f_tiles;
+  const int top = G ? end[G - 1] : 0, units = (top + TP_UNIT - 1) / TP_UNIT + 1;
+  std::vector<int> seen((size_t)units * f_tiles * kbt, 0), cleared((size_t)(top + 1) * f_tiles, 0), pieces(pairs + 1, 0), claimed(pairs + 1, 0);
+  int bad = 0;
+  for (int p = 0; p < pairs; ++p) {
+    int shared = 0;
+    for (int it = 0;; ++it) {
+      TPWork w;
+      if (!tp_work(&tb, G, f_tiles, f_width, kbt, split, p, pairs, it, w)) break;
+      if (it > tiles + 4) { printf("work list does not end\n"); return 1; }
+      const TPTile& t = w.t;
+      if (t.n < TP_UNIT || t.n > 256 || t.n % TP_UNIT || t.n > tb.widest || t.f0 % f_width || t.f0 >= N || t.g >= G || t.row0 < start[t.g] ||
+          (t.row0 - start[t.g]) % TP_UNIT || t.row0 - start[t.g] >= rows[t.g] || t.end != end[t.g] || w.kb0 < 0 || w.kb1 > kbt || w.kb0 >= w.kb1) { ++bad; continue; }
+      for (int u = 0; u < t.n / TP_UNIT; ++u)
+        for (int kb = w.kb0; kb < w.kb1; ++kb) seen[((size_t)(t.row0 / TP_UNIT + u) * f_tiles + t.f0 / f_width) * kbt + kb] += 1;
+      if (w.kb0 == 0) for (int r = t.zero0; r < t.end; ++r) cleared[(size_t)r * f_tiles + t.f0 / f_width] += 1;
+      if (w.split >= 0) {
+        ++shared;
+        if (w.split >= pairs) { ++bad; continue; }
+        pieces[w.split] += 1;
+        if (claimed[w.split] != 0 && claimed[w.split] != w.contributors) ++bad;
+        claimed[w.split] = w.contributors;
+      } else if (w.kb0 != 0 || w.kb1 != kbt) {
+        ++bad;
+      }
+    }
+    if (shared > 2) ++bad;
+  }
+  for (int i = 0; i <= pairs; ++i) if (pieces[i] != claimed[i]) ++bad;
+  for (int g = 0; g < G; ++g) {
+    const int covered = (rows[g] + TP_UNIT - 1) / TP_UNIT;
+    for (int u = 0; u < (end[g] - start[g] + TP_UNIT - 1) / TP_UNIT; ++u)
+      for (int f = 0; f < f_tiles; ++f)
+        for (int kb = 0; kb < kbt; ++kb)
+          if (seen[((size_t)(start[g] / TP_UNIT + u) * f_tiles + f) * kbt + kb] != (u < covered ? 1 : 0)) ++bad;
+    for (int r = start[g]; r < end[g]; ++r)
+      for (int f = 0; f < f_tiles; ++f)
+        if (rows[g] > 0 && cleared[(size_t)r * f_tiles + f] != (r >= start[g] + covered * TP_UNIT ? 1 : 0)) ++bad;
+  }
+  return bad;
+}
+
 int main() {
   int failures = 0, cases = 0;
+  for (int it = 0; it < 400; ++it) {
+    std::vector<int> start, rows, end;
+    const int G = it % 5 == 0 ? 1 : 1 + rnd(12);
+    int at = 0;
+    for (int g = 0; g < G; ++g) {
+      const int n = rnd(4) == 0 ? 0 : 1 + rnd(rnd(3) == 0 ? 2500 : 300);
+      start.push_back(at); rows.push_back(n);
+      at += it % 5 == 0 ? n : (n + BM - 1) / BM * BM;                // (dense: no padding)
+      end.push_back(at);
+    }
+    const int N = 8 * (17 + rnd(500)), kbt = 1 + rnd(40), ps[3] = {74, 66, 5};
+    for (int c = 0; c < 3; ++c) {
+      const int b1 = check_transposed(start, rows, end, N, 256, kbt, ps[c], it % 3 != 0), b2 = check_transposed(start, rows, end, N, 128, kbt, ps[c], it % 3 != 0);
+      ++cases;
+      if (b1 || b2) { ++failures; printf("transposed: G %d N %d kbt %d pairs %d: %d / %d errors\n", G, N, kbt, ps[c], b1, b2); }
+    }
+  }
   for (int it = 0; it < 300; ++it) {
     GemmParams p;
     memset(&p, 0, sizeof(p));

@@ -266,6 +266,69 @@ def test_swiglu_backward_in_the_product(ops, T, E, H, F, policy):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("counts", [[1], [0, 31, 32, 33], [255, 0, 256, 257], [513, 64, 95], [2100, 1, 300]])
+@pytest.mark.parametrize("H,F", [(72, 136), (264, 1032), (1024, 768)])
+def test_transposed_pair_kernel(ops, counts, H, F):
+    """Weights as the 256-row operand, rows of every group counted exactly: remainders of the 32-row units, of 256-row tiles
+    and 8-tile panels, of feature tiles and of the depth; gate / up with and without its outputs and with adapters, SwiGLU
+    backward, K-major and MN-major weights, two depth segments; shared last rounds (2100 rows).  fp32 reference, one bf16
+    rounding of each result (2e-2 as for the other products); padding becomes zeros, rows past the groups stay untouched."""
+    torch.manual_seed(sum(counts) + F)
+    E, r = len(counts), 16
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(sum(counts))].to(DEV).int()
+    plan = ops.make_plan(ids[:, None], E)
+    R, used, offs = plan.src_slot.numel(), int(plan.padded_offsets[-1]), plan.padded_offsets.tolist()
+    real = plan.src_slot[:used] >= 0
+    rows = lambda n, scale=1.0: torch.where((plan.src_slot >= 0)[:, None], _rand(R, n, scale=scale), 0.0).to(torch.bfloat16)
+    x, dy, t = rows(H), rows(H), rows(2 * r)
+    w1, w3, w2 = (_rand(E, F, H, scale=0.1) for _ in range(3))
+    b1, b3 = _rand(E, F, 2 * r, scale=0.1), _rand(E, F, 2 * r, scale=0.1)
+    a2 = _rand(E, 2 * r, H, scale=0.1)
+
+    def ref(fn):
+        out = []
+        for e in range(E):
+            out.append(fn(slice(offs[e], offs[e + 1]), e))
+        return torch.cat(out)
+    new = lambda n: torch.full((R, n), 7.0, dtype=torch.bfloat16, device=DEV)
+    check = lambda got, want, name: (_close(got[:used][real], want[real], name=name), _zero_pads(got, name))
+
+    def _zero_pads(got, name):
+        assert bool((got[:used][~real] == 0).all()) and bool((got[used:] == 7.0).all()), name
+    f = lambda v: v.float()
+    gate = ref(lambda s, e: f(x[s]) @ f(w1[e]).t())
+    up = ref(lambda s, e: f(x[s]) @ f(w3[e]).t())
+    prev = ops.ext.gemm_set_pair_policy(6)
+    try:
+        h, g, u = new(F), new(F), new(F)
+        ops._g(1, x, False, w1, False, h, F, H, plan, B2=w3)
+        check(h, torch.nn.functional.silu(gate) * up, "gate and up")
+        ops._g(1, x, False, w1, False, h, F, H, plan, B2=w3, C2=g, C3=u, A_l=t, B_l=b1, B2_l=b3, b_mn_l=False, K_l=2 * r)
+        gl, ul = gate + ref(lambda s, e: f(t[s]) @ f(b1[e]).t()), up + ref(lambda s, e: f(t[s]) @ f(b3[e]).t())
+        check(g, gl, "gate"); check(u, ul, "up"); check(h, torch.nn.functional.silu(gl) * ul, "gate and up with adapters")
+        y = new(H)
+        ops._g(1, h, False, w2, True, y, H, F, plan, A_l=t, B_l=a2, b_mn_l=True, K_l=2 * r, alpha=0.5)
+        hf = f(h)
+        check(y, 0.5 * ref(lambda s, e: hf[s] @ f(w2[e]) + f(t[s]) @ f(a2[e])), "down")
+        dg, du = new(F), new(F)
+        ops._g(1, dy, False, w2, False, dg, F, H, plan, C2=du, swiglu=(g, u))
+        gf, uf = f(g[:used]).requires_grad_(True), f(u[:used]).requires_grad_(True)
+        want = torch.autograd.grad(torch.nn.functional.silu(gf) * uf, (gf, uf), ref(lambda s, e: f(dy[s]) @ f(w2[e]).t()))
+        check(dg, want[0], "dg"); check(du, want[1], "du")
+        dx = new(H)
+        ops._g(1, dg, False, w1, True, dx, H, F, plan, A_l=du, B_l=w3, b_mn_l=True, K_l=F)
+        dgf, duf = f(dg), f(du)
+        check(dx, ref(lambda s, e: dgf[s] @ f(w1[e]) + duf[s] @ f(w3[e])), "dx")
+        m = sum(counts)                                   # dense, no padding: rows of any number
+        x2, out, factor = _rand(m, H), torch.full((m + 1, F), 7.0, dtype=torch.bfloat16, device=DEV), torch.tensor(0.25, device=DEV)
+        ops._gemm(0, x2, False, w1[0], False, out, m, F, H, alpha_dev=factor)
+        _close(out[:m], 0.25 * (f(x2) @ f(w1[0]).t()), name="dense")
+        assert bool((out[m:] == 7.0).all())
+    finally:
+        ops.ext.gemm_set_pair_policy(prev)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (77, 1024, 4096), (300, 520, 2056), (129, 64, 8192), (1000, 16, 4096), (33, 128, 1024)])
 def test_gemm_few_tiles_shared_by_a_cluster(ops, M, N, K):
     """Products with few output tiles under the default policy (the depth is cut over a cluster): K-major and MN-major

@@ -1,5 +1,5 @@
 """Index arithmetic of the GEMM kernels, checked on the host: the persistent kernels' tile enumeration
-(`get_tile`, `get_pair_tile` in csrc/gemm_sm100.cu) is compiled for the CPU and run over random dense, row-grouped
+(`get_tile`, `get_pair_tile` in csrc/gemm_sm100.cu, `tp_work` in csrc/gemm_transposed.cuh) is compiled for the CPU and run over random dense, row-grouped
 and depth-grouped problems (tests/host/tile_enumeration.cu)."""
 import os
 import shutil
