@@ -1159,6 +1159,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(con
 }
 
 #include "gemm_transposed.cuh"
+#include "gemm_wgrad.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // host side
@@ -1290,6 +1291,20 @@ static cudaError_t launch(const GemmParams& p, int grid, cudaStream_t stream) {
 static int g_max_pairs = 0;
 static int g_pair_cap = 0;   // optional upper bound set through mdt_gemm_set_pair_cap (0 = none)
 
+template <class Kernel>
+static int resident_pairs(Kernel kernel, int smem) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(g_num_sms & ~1)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2; }
+  return n < g_num_sms / 2 ? n : g_num_sms / 2;
+}
+
 template <bool SWIGLU>
 static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream_t stream) {
   constexpr int smem = PAIR_SMEM;
@@ -1297,16 +1312,7 @@ static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_sm100_pair_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(g_num_sms & ~1)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_sm100_pair_kernel<SWIGLU>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2; }
-    g_max_pairs = n < g_num_sms / 2 ? n : g_num_sms / 2;
+    g_max_pairs = resident_pairs(gemm_sm100_pair_kernel<SWIGLU>, smem);
     configured = true;
   }
   const int limit = (g_pair_cap > 0 && g_pair_cap < g_max_pairs) ? g_pair_cap : g_max_pairs;
@@ -1322,6 +1328,44 @@ static bool transposed_ok(const MdtGemmDesc* d) {
   return (d->mode == 0 || d->mode == 1) && G <= TP_GROUPS && d->a_mn == 0 && (d->K_l == 0 || d->a_mn_l == 0) && !d->c_fp32 && !d->accumulate &&
          d->R == nullptr && d->tile_ready == nullptr && d->row_dest_rank == nullptr && d->b_ready.ready == nullptr && d->b2_ready.ready == nullptr &&
          d->bl_ready.ready == nullptr && d->N > 128 && (!d->dual || (d->b_mn == 0 && (d->K_l == 0 || d->b_mn_l == 0)));
+}
+
+// The weight gradient kernel: what it can run at all.
+static bool wgrad_ok(const MdtGemmDesc* d) {
+  const int G = d->G < 1 ? 1 : d->G;
+  return d->mode == 2 && G <= WG_GROUPS && d->a_mn == 1 && d->b_mn == 1 && !d->c_fp32 && d->K_l == 0 && !d->dual && (reinterpret_cast<uintptr_t>(d->C) & 15) == 0 &&
+         d->N > 128 && d->M > 128 && (G == 1 || (d->c_group_stride % 8 == 0 && d->c_group_stride >= 0));
+}
+
+// Which weight gradients it takes under the default policy: those of up to 12 k blocks, where the result bounds them, and deeper ones
+// that are written and that the cluster kernel leaves alone (adding to C costs the ring stages that a deep product needs).
+// Microseconds, pair / this kernel, 8 x 14336 x 4096: 576 tokens (3 k blocks) written 353 / 182, added to 533 / 355; 2000 tokens (8)
+// 414 / 348, 636 / 490; 4000 tokens (16) 687 / 627, 810 / 835; 12000 tokens 1787 / 1742, 2233 / 2688.  Dense 32000 x 4096 of 576 rows
+// 165 / 147, 235 / 183, of 1000 rows 182 / 168, 195 / 214.
+static bool wgrad_preferred(const MdtGemmDesc* d, long long thread_rows_hint, int cluster) {
+  const int G = d->G < 1 ? 1 : d->G;
+  double depth = (double)d->K;
+  if (d->offsets != nullptr) {
+    double n = (double)d->capacity_rows - 127.0 * G;
+    if (thread_rows_hint > 0 && (double)thread_rows_hint < n) n = (double)thread_rows_hint;
+    depth = n / G;
+  }
+  return depth <= 12.0 * BK || (!d->accumulate && cluster == 0);
+}
+
+template <bool ACC>
+static cudaError_t launch_wgrad(const WgParams& p, cudaStream_t stream) {
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_sm100_wgrad_kernel<ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM);
+    if (e != cudaSuccess) return e;
+    max_pairs = resident_pairs(gemm_sm100_wgrad_kernel<ACC>, WG_SMEM);
+  }
+  const long long tiles = (long long)p.G * ((p.M + 255) / 256) * ((p.N + 255) / 256);
+  const int limit = (g_pair_cap > 0 && g_pair_cap < max_pairs) ? g_pair_cap : max_pairs;
+  gemm_sm100_wgrad_kernel<ACC><<<2 * (int)(tiles < limit ? tiles : limit), GEMM_THREADS, WG_SMEM, stream>>>(p);
+  ++g_launches;
+  return cudaGetLastError();
 }
 
 // Which row-grouped products it takes under the default policy (those that the cluster kernel would take stay there).
@@ -1348,16 +1392,7 @@ static cudaError_t launch_transposed(const TPParams& p, long long tiles, cudaStr
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_sm100_tpair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(g_num_sms & ~1)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = TP_SMEM;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_sm100_tpair_kernel<KIND>, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = g_num_sms / 2; }
-    max_pairs = n < g_num_sms / 2 ? n : g_num_sms / 2;
+    max_pairs = resident_pairs(gemm_sm100_tpair_kernel<KIND>, TP_SMEM);
     configured = true;
   }
   const int limit = (g_pair_cap > 0 && g_pair_cap < max_pairs) ? g_pair_cap : max_pairs;
@@ -1601,6 +1636,23 @@ static int gemm_transposed(const MdtGemmDesc* d, cudaStream_t stream) {
 }
 }  // namespace mdt
 
+namespace mdt {
+static int gemm_wgrad(const MdtGemmDesc* d, cudaStream_t stream) {
+  WgParams p;
+  memset(&p, 0, sizeof(p));
+  p.M = d->M; p.N = d->N; p.K = d->K; p.G = d->G < 1 ? 1 : d->G;
+  p.offsets = d->offsets; p.group_rows = d->group_rows;
+  p.alpha = d->alpha; p.alpha_dev = d->alpha_dev; p.status = d->status;
+  int rc = make_map(&p.tmA, d->A, d->a_cols, d->a_rows, 1, d->lda, 0, 64, 64, 2);
+  rc |= make_map(&p.tmB, d->B, d->b_cols, d->b_rows, 1, d->ldb, 0, 64, 64, 2);
+  // (a stride that one matrix does not use still has to be a valid one)
+  rc |= make_map(&p.tmC, d->C, d->N, d->M, p.G, d->ldc, p.G > 1 ? d->c_group_stride : d->ldc * (long long)d->M, 64, 32, 3);
+  if (rc != 0) return rc;
+  const cudaError_t e = d->accumulate ? launch_wgrad<true>(p, stream) : launch_wgrad<false>(p, stream);
+  return e == cudaSuccess ? 0 : -100 - (int)e;
+}
+}  // namespace mdt
+
 extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   using namespace mdt;
   // Tensor-map encoding is a driver call: make sure this host thread has the device's primary context
@@ -1641,6 +1693,7 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   const int cluster = pair_policy() == DEFAULT_POLICY ? choose_cluster(d, t_rows_hint, max_clusters, &cluster_bn) : 0;
   if (cluster == 0 && pair_policy() >= DEFAULT_POLICY && transposed_ok(d) && (pair_policy() == MAX_POLICY || transposed_preferred(d, t_rows_hint)))
     return gemm_transposed(d, stream);
+  if (pair_policy() >= DEFAULT_POLICY && wgrad_ok(d) && (pair_policy() == MAX_POLICY || wgrad_preferred(d, t_rows_hint, cluster))) return gemm_wgrad(d, stream);
   const bool pair = cluster == 0 && choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms) != 0;
   const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
   int rc = 0;

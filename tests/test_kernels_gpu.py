@@ -329,6 +329,40 @@ def test_transposed_pair_kernel(ops, counts, H, F):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("counts", [[1, 0, 5], [64, 65, 127, 128], [300, 0, 1], [700], [1600, 900]])
+@pytest.mark.parametrize("M,N", [(136, 136), (264, 1032), (1024, 520), (2312, 264)])
+def test_weight_gradient_kernel(ops, counts, M, N):
+    """Weight gradients whose result moves through shared memory by TMA: written and added to, edges of the 32 x 64 pieces, of
+    256-wide tiles and of the panels, groups without rows (zeros, or untouched when adding), depths of 0 to 25 k blocks, the
+    gradients as a slice of a larger buffer.  fp32 sums, one bf16 rounding of each result."""
+    torch.manual_seed(sum(counts) + M)
+    E = len(counts)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(sum(counts))].to(DEV).int()
+    plan = ops.make_plan(ids[:, None], E)
+    R, offs = plan.src_slot.numel(), plan.padded_offsets.tolist()
+    rows = lambda n: torch.where((plan.src_slot >= 0)[:, None], _rand(R, n), 0.0).to(torch.bfloat16)
+    a, b = rows(M), rows(N)
+    want = torch.stack([a[offs[e]:offs[e + 1]].float().t() @ b[offs[e]:offs[e + 1]].float() for e in range(E)])
+    old = _rand(E, M, N, scale=4.0)
+    prev = ops.ext.gemm_set_pair_policy(6)
+    try:
+        for add in (False, True):
+            room = torch.full((E, M + 8, N + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+            out = room[:, :M, :N]
+            out.copy_(old if add else torch.full_like(old, float("nan")))
+            ops._g(2, a, True, b, True, out, N, 0, plan, alpha=0.5, accumulate=add)
+            _close(out, 0.5 * want + (old.float() if add else 0.0), 1e-2, name=f"add {add}")
+            for e in range(E):
+                if counts[e] == 0:
+                    assert torch.equal(out[e], old[e] if add else torch.zeros_like(old[e]))
+            assert bool((room[:, M:] == 7.0).all()) and bool((room[:, :, N:] == 7.0).all())
+        x, y, f = _rand(sum(counts), M), _rand(sum(counts), N), torch.tensor(0.25, device=DEV)      # dense, any number of rows
+        _close(ops.mm_tn(x, y, alpha_dev=f), 0.25 * (x.float().t() @ y.float()), 1e-2, name="dense")
+    finally:
+        ops.ext.gemm_set_pair_policy(prev)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (77, 1024, 4096), (300, 520, 2056), (129, 64, 8192), (1000, 16, 4096), (33, 128, 1024)])
 def test_gemm_few_tiles_shared_by_a_cluster(ops, M, N, K):
     """Products with few output tiles under the default policy (the depth is cut over a cluster): K-major and MN-major
