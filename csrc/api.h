@@ -103,7 +103,10 @@ int mdt_rope(const void* x, void* y, const int* positions, int tokens, int heads
 int mdt_copy_rows_used(const void* src, void* dst, long long n, const int* rows_used, long long cols, cudaStream_t s);
 int mdt_swiglu_fwd(const void* g, const void* u, void* h, long long n, cudaStream_t s);
 int mdt_embedding(const void* table, const long long* ids, void* out, int tokens, int cols, cudaStream_t s);
-int mdt_embedding_bwd(const void* dout, const long long* ids, float* dtable, int tokens, int cols, cudaStream_t s);
+// rows of dtable (bf16 or fp32, [rows, cols]) that ids names: written with, or (add) increased by, the sum of their tokens' rows of
+// dout; other rows are left alone.  scratch: tokens + rows ints
+int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int table_fp32, int add, int* scratch, int tokens, int rows, int cols,
+                      cudaStream_t s);
 // in place: logits (bf16, [rows, vocab]) become d(loss_sum)/dlogits * grad_scale; loss_sum/count accumulate
 int mdt_cross_entropy(void* logits, const long long* labels, float* loss_sum, float* count, int rows, int vocab,
                       long long ld, int ignore_index, float grad_scale, cudaStream_t s);

@@ -224,10 +224,17 @@ Tensor embedding(const Tensor& table, const Tensor& ids) {
   check(mdt_embedding(table.data_ptr(), ids.data_ptr<int64_t>() ? (const long long*)ids.data_ptr<int64_t>() : nullptr, out.data_ptr(), (int)ids.numel(), (int)table.size(1), cur_stream()), "embedding");
   return out;
 }
-void embedding_bwd(const Tensor& dout, const Tensor& ids, Tensor& dtable) {
+// add: to what the table's gradient holds; otherwise rows that no token names are cleared
+void embedding_bwd(const Tensor& dout, const Tensor& ids, Tensor& dtable, bool add) {
+  CHECK_BF16(dout);
   c10::cuda::CUDAGuard guard(dout.device());
-  TORCH_CHECK(dtable.scalar_type() == at::kFloat && dout.is_contiguous());
-  check(mdt_embedding_bwd(dout.data_ptr(), (const long long*)ids.data_ptr<int64_t>(), dtable.data_ptr<float>(), (int)ids.numel(), (int)dout.size(1), cur_stream()), "embedding_bwd");
+  TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && dout.is_contiguous() && dtable.is_contiguous() && dtable.dim() == 2 &&
+              (dtable.scalar_type() == at::kFloat || dtable.scalar_type() == at::kBFloat16) && dout.size(-1) == dtable.size(1));
+  for (const Tensor* t : {&dout, (const Tensor*)&dtable}) TORCH_CHECK((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "embedding_bwd: rows must be 16-byte aligned");
+  if (!add) dtable.zero_();
+  auto scratch = torch::empty({ids.numel() + dtable.size(0)}, ids.options().dtype(at::kInt));
+  check(mdt_embedding_bwd(dout.data_ptr(), (const long long*)ids.data_ptr<int64_t>(), dtable.data_ptr(), dtable.scalar_type() == at::kFloat, add ? 1 : 0,
+                          scratch.data_ptr<int>(), (int)ids.numel(), (int)dtable.size(0), (int)dtable.size(1), cur_stream()), "embedding_bwd");
 }
 // logits are overwritten with d(mean loss)/dlogits * grad_scale; returns [loss_sum, count]
 Tensor cross_entropy(Tensor& logits, const Tensor& labels, int64_t ignore_index, double grad_scale) {
@@ -588,8 +595,9 @@ std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTen
 }
 // dx (+)= dy W (+ LoRA), and the requested parameter gradients
 struct LinGrads { OptTensor dW, dA, dB; };
+// w_out: where the weight gradient goes (and whether it is added to what is there) instead of a new tensor
 LinGrads lin_bwd(const Tensor& dy, const Tensor& xin, const Lin& l, const OptTensor& t, bool need_w, bool need_a, bool need_b,
-                 Tensor& dx, bool accumulate, const OptTensor& status) {
+                 Tensor& dx, bool accumulate, const OptTensor& status, const OptTensor& w_out = std::nullopt, bool w_add = false) {
   const int64_t M = dy.size(0), N = dy.size(1), K = l.W.size(1);
   LinGrads g;
   OptTensor dt;
@@ -607,7 +615,11 @@ LinGrads lin_bwd(const Tensor& dy, const Tensor& xin, const Lin& l, const OptTen
   } else {
     gemm_raw(0, dy, false, l.W, true, dx, M, K, N, std::nullopt, std::nullopt, false, 0, accumulate, 1.0, status);
   }
-  if (need_w) { g.dW = torch::empty_like(l.W); gemm_raw(2, dy, true, xin, true, *g.dW, N, K, M, std::nullopt, std::nullopt, false, 0, false, 1.0, status); }
+  if (need_w) {
+    Tensor w = w_out.has_value() ? *w_out : torch::empty_like(l.W);
+    gemm_raw(2, dy, true, xin, true, w, N, K, M, std::nullopt, std::nullopt, false, 0, w_out.has_value() && w_add, 1.0, status);
+    if (!w_out.has_value()) g.dW = w;
+  }
   return g;
 }
 Lin make_lin(const std::vector<Tensor>& p, size_t& i, double s) {
@@ -682,13 +694,17 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
   return {out, rstd, xn, qr, kr, v3, o, lse, tq.value_or(none), tk.value_or(none), tv.value_or(none), to.value_or(none)};
 }
 
-// needs[j] for params[j]; returns {dx, grads of params in order (empty tensor where not needed)}
+// needs[j] for params[j]; w_out / w_add: for q, k, v, o where the weight's gradient goes and whether it is added there (an empty
+// tensor: a new one).  Returns {dx, grads of params in order (empty tensor where not needed or given a place)}
 std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tensor>& saved, const std::vector<Tensor>& params,
                                         const std::vector<double>& scalings, const std::vector<bool>& needs, const Tensor& positions,
                                         const Tensor& cu_seqlens, int64_t max_seqlen, double theta, int64_t Hq, int64_t Hkv, int64_t d,
-                                        const Tensor& status_t) {
+                                        const Tensor& status_t, const std::vector<Tensor>& w_out, const std::vector<bool>& w_add) {
   c10::cuda::CUDAGuard guard(dy.device());
   Phase ph("attention.backward");
+  TORCH_CHECK(w_out.size() == w_add.size() && (w_out.empty() || w_out.size() == 4), "attention_block_bwd: four places or none");
+  auto place = [&](int j) -> OptTensor { return w_out.empty() || !w_out[j].numel() ? std::nullopt : OptTensor(w_out[j]); };
+  auto adds = [&](int j) { return !w_add.empty() && (bool)w_add[j]; };
   OptTensor status = status_t;
   const Tensor &x = saved[0], &rstd = saved[1], &xn = saved[2], &qr = saved[3], &kr = saved[4], &v3 = saved[5], &o = saved[6], &lse = saved[7];
   auto opt = [](const Tensor& t) -> OptTensor { return t.numel() ? OptTensor(t) : std::nullopt; };
@@ -709,15 +725,15 @@ std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tens
   Tensor dyc = dy.contiguous();
   Tensor o2 = o.view({T, Hq * d});
   Tensor d_o = torch::empty({T, Hq * d}, x.options());
-  put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status));
+  put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status, place(3), adds(3)));
   auto g3 = attention_bwd(qr, kr, v3, o, d_o.view({T, Hq, d}), lse, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d), status);
   Tensor dq = rope(g3[0], positions, theta, true).view({T, Hq * d});
   Tensor dk = rope(g3[1], positions, theta, true).view({T, Hkv * d});
   Tensor dv = g3[2].view({T, Hkv * d});
   Tensor d_xn = torch::empty({T, H}, x.options());
-  put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status));
-  put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status));
-  put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status));
+  put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status, place(0), adds(0)));
+  put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status, place(1), adds(1)));
+  put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status, place(2), adds(2)));
   auto rb = rmsnorm_bwd(x, params[0], d_xn, rstd, dyc, (bool)needs[0]);     // + dy: the residual connection's gradient
   Tensor dx = rb[0];
   if (needs[0]) grads[0] = rmsnorm_dw(rb[1], params[0]);

@@ -253,11 +253,42 @@ __global__ void embedding_kernel(const bf16* __restrict__ table, const long long
   uint4* dst = reinterpret_cast<uint4*>(out + (long long)blockIdx.x * cols);
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) dst[i] = src[i];
 }
-__global__ void embedding_bwd_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, float* __restrict__ dtable, int cols) {
+// Gradient of the table, added to (or written over) the rows of `dtable` that the tokens name.  The tokens of one id form a list
+// (head[id], then next[token]); the CTA of the token at the head adds their rows up in fp32 and rounds once.  A table of
+// 32000 x 4096 in fp32, cleared, added to with atomics and converted, took 198 us however few the tokens; this 9 for 576 of them.
+__global__ void embedding_list_kernel(const long long* __restrict__ ids, int* __restrict__ head, int* __restrict__ next, int tokens) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < tokens) next[t] = atomicExch(head + ids[t], t);
+}
+template <bool F32>
+__global__ void embedding_bwd_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, const int* __restrict__ head, const int* __restrict__ next,
+                                     void* __restrict__ dtable, int cols, int add) {
   const long long id = ids[blockIdx.x];
-  const bf16* src = dout + (long long)blockIdx.x * cols;
-  float* dst = dtable + id * cols;
-  for (int i = threadIdx.x; i < cols; i += blockDim.x) atomicAdd(dst + i, __bfloat162float(src[i]));
+  if (head[id] != (int)blockIdx.x) return;
+  for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
+    float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (add) {
+      if (F32) {
+        const float4* o = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(dtable) + id * cols + i * 8);
+        const float4 x = o[0], y = o[1];
+        f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
+      } else {
+        unpack8(reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(dtable) + id * cols)[i], f);
+      }
+    }
+    for (int t = blockIdx.x; t >= 0; t = next[t]) {
+      float g[8];
+      unpack8(reinterpret_cast<const uint4*>(dout + (long long)t * cols)[i], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] += g[j];
+    }
+    if (F32) {
+      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(dtable) + id * cols + i * 8);
+      o[0] = make_float4(f[0], f[1], f[2], f[3]); o[1] = make_float4(f[4], f[5], f[6], f[7]);
+    } else {
+      reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(dtable) + id * cols)[i] = pack8(f);
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------ cross entropy
@@ -529,9 +560,15 @@ extern "C" int mdt_embedding(const void* table, const long long* ids, void* out,
   MDT_CHECK_LAUNCH();
   return 0;
 }
-extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, float* dtable, int tokens, int cols, cudaStream_t s) {
+extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int table_fp32, int add, int* scratch, int tokens, int rows, int cols, cudaStream_t s) {
+  if (cols % 8 != 0) return -1;
   if (tokens == 0) return 0;
-  embedding_bwd_kernel<<<tokens, 256, 0, s>>>((const bf16*)dout, ids, dtable, cols);
+  int* head = scratch + tokens;
+  if (cudaMemsetAsync(head, 0xff, (size_t)rows * sizeof(int), s) != cudaSuccess) return -2;
+  embedding_list_kernel<<<(tokens + 255) / 256, 256, 0, s>>>(ids, head, scratch, tokens);
+  MDT_CHECK_LAUNCH();
+  if (table_fp32) embedding_bwd_kernel<true><<<tokens, 256, 0, s>>>((const bf16*)dout, ids, head, scratch, dtable, cols, add);
+  else embedding_bwd_kernel<false><<<tokens, 256, 0, s>>>((const bf16*)dout, ids, head, scratch, dtable, cols, add);
   MDT_CHECK_LAUNCH();
   return 0;
 }

@@ -466,20 +466,31 @@ def rope(x, positions, theta):
     return _Rope.apply(x, positions.int(), float(theta))
 
 
+def grad_place(w):
+    """Where the gradient of `w` is collected (an object whose target() gives the tensor and whether to add to it), or None: an
+    ordinary gradient tensor.  Set on the weight views of a flat parameter that only one rank holds."""
+    return getattr(w, "_grad_place", None)
+
+
 class _Embedding(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ids, weight):
         ids = ids.long().contiguous()
         ctx.save_for_backward(ids)
-        ctx.shape = weight.shape
+        ctx.shape, ctx.place = weight.shape, grad_place(weight)
         return ext.embedding(weight, ids)
 
     @staticmethod
     def backward(ctx, dout):
         (ids,) = ctx.saved_tensors
-        dtable = torch.zeros(ctx.shape, dtype=torch.float32, device=dout.device)
-        ext.embedding_bwd(dout.contiguous(), ids, dtable)
-        return None, dtable.to(dout.dtype)
+        dout = _rows(dout)
+        if ctx.place is not None:
+            dtable, add = ctx.place.target()
+            ext.embedding_bwd(dout, ids, dtable, add)
+            return None, None
+        dtable = torch.empty(ctx.shape, dtype=dout.dtype, device=dout.device)
+        ext.embedding_bwd(dout, ids, dtable, False)
+        return None, dtable
 
 
 def embedding(ids, weight):
@@ -499,6 +510,7 @@ class _LinearCrossEntropy(torch.autograd.Function):
         logits = mm_nt(hidden, w_head)
         out = ext.cross_entropy(logits, labels.long().contiguous(), ignore_index, 1.0)
         n = out[1]
+        ctx.place = grad_place(w_head)
         ctx.save_for_backward(hidden, w_head, logits, out[1].clone())
         loss_sum = out[0].clone()
         n = n.clone()
@@ -512,7 +524,12 @@ class _LinearCrossEntropy(torch.autograd.Function):
         # the products' epilogues (a pass over 8192 x 32000 logits for it took 550 us)
         factor = (dloss_sum * n.clamp(min=1.0)).float()
         dh = mm_nn(dlogits, w_head, alpha_dev=factor) if ctx.needs_input_grad[0] else None
-        dw = mm_tn(dlogits, hidden, alpha_dev=factor) if ctx.needs_input_grad[1] else None
+        dw = None
+        if ctx.needs_input_grad[1] and ctx.place is not None:
+            out, add = ctx.place.target()
+            mm_tn(dlogits, hidden, out=out, accumulate=add, alpha_dev=factor)
+        elif ctx.needs_input_grad[1]:
+            dw = mm_tn(dlogits, hidden, alpha_dev=factor)
         return dh, dw, None, None
 
 

@@ -39,13 +39,13 @@ class _AttentionBlockNative(torch.autograd.Function):
     """Same sub-block with the kernel sequence issued from C++ (one binding call per direction)."""
 
     @staticmethod
-    def forward(ctx, x, meta, *params):
+    def forward(ctx, x, meta, places, *params):
         eps, theta, Hq, Hkv, d, positions, cu, max_seqlen, scalings = meta
         sc = [-1.0 if s is None else float(s) for s in scalings]
         res = ext.attention_block_fwd(x.contiguous(), list(params), sc, positions, cu, max_seqlen, eps, theta, Hq, Hkv, d,
                                       C.status_tensor(x.device))
         if any(ctx.needs_input_grad):
-            ctx.meta, ctx.sc, ctx.n_params = meta, sc, len(params)
+            ctx.meta, ctx.sc, ctx.places = meta, sc, places
             ctx.save_for_backward(x, *res[1:], *params)
         return res[0]
 
@@ -54,11 +54,18 @@ class _AttentionBlockNative(torch.autograd.Function):
         eps, theta, Hq, Hkv, d, positions, cu, max_seqlen, scalings = ctx.meta
         saved = ctx.saved_tensors
         state, params = list(saved[:12]), list(saved[12:])
-        needs = [bool(n) for n in ctx.needs_input_grad[2:]]
+        needs = [bool(n) for n in ctx.needs_input_grad[3:]]
+        out, add = [], []
+        if ctx.places is not None:            # frozen weights have no place either
+            at, targets = 1, []
+            for p, s in zip(ctx.places, scalings):
+                targets.append(p.target() if p is not None and needs[at] else (dy.new_empty(0), False))
+                at += 1 if s is None else 3
+            out, add = [t for t, _ in targets], [a for _, a in targets]
         res = ext.attention_block_bwd(dy, state, params, ctx.sc, needs, positions, cu, max_seqlen, theta, Hq, Hkv, d,
-                                      C.status_tensor(dy.device))
+                                      C.status_tensor(dy.device), out, add)
         grads = tuple(g if (g.numel() and need) else None for g, need in zip(res[1:], needs))
-        return (res[0], None) + grads
+        return (res[0], None, None) + grads
 
 
 NATIVE_ISSUE = os.environ.get("MDT_NATIVE_BLOCKS", "1") != "0"
@@ -139,9 +146,10 @@ def attention_block(layer, x, batch):
     """x + self_attn(input_layernorm(x)) for a `MixtralDecoderLayer` on CUDA (head_dim 128)."""
     attn = layer.self_attn
     params = [layer.input_layernorm.weight]
-    scalings = []
+    scalings, places = [], []
     for lin in (attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj):
         params.append(lin.weight)
+        places.append(C.grad_place(lin.weight))
         if lin.lora_A is not None:
             params += [lin.lora_A["default"].weight, lin.lora_B["default"].weight]
             scalings.append(float(lin.scaling))
@@ -149,7 +157,9 @@ def attention_block(layer, x, batch):
             scalings.append(None)
     meta = (layer.input_layernorm.eps, float(attn.cfg.rope_theta), attn.num_heads, attn.num_kv_heads, attn.head_dim,
             batch.positions, batch.cu_seqlens, int(batch.max_seqlen), tuple(scalings))
-    return (_AttentionBlockNative if NATIVE_ISSUE else _AttentionBlock).apply(x, meta, *params)
+    if NATIVE_ISSUE:
+        return _AttentionBlockNative.apply(x, meta, places if any(p is not None for p in places) else None, *params)
+    return _AttentionBlock.apply(x, meta, *params)
 
 
 # ---------------------------------------------------------------------------------------------------------

@@ -52,6 +52,19 @@ def _gemm_only_weight(qualname: str, p) -> bool:
     return qualname.endswith("_proj.weight") or (len(leaf) >= 2 and leaf[-1] in ("w1", "w2", "w3") and ".experts." in qualname)
 
 
+class _GradPlace:
+    """Where the gradient of one weight of a flat parameter is collected; the products that compute it write or add there."""
+
+    __slots__ = ("group", "index")
+
+    def __init__(self, group, index):
+        self.group, self.index = group, index
+
+    def target(self):
+        """The weight's part of the flat gradient, and whether it holds a gradient already."""
+        return self.group.grad_target(self.index)
+
+
 class FlatParamGroup:
     """Parameters of one unit flattened into a single buffer sharded over `group`."""
 
@@ -93,6 +106,10 @@ class FlatParamGroup:
         self.shard = nn.Parameter(shard, requires_grad=trainable)
         self.full: Optional[torch.Tensor] = None
         self.acc: Optional[torch.Tensor] = None  # fp32 full-size local accumulation (sync_each_batch=False)
+        # Set where nothing has to be reduced (one rank): products put weight gradients straight into the flat gradient.  Until
+        # that is complete it is kept here with the indices of the weights written so far.
+        self.collect_in_place = False
+        self._collecting: Optional[tuple] = None
 
     def install(self, full: torch.Tensor, as_leaves: bool) -> List[torch.Tensor]:
         """Point the modules' weights at views of `full`.
@@ -107,10 +124,12 @@ class FlatParamGroup:
         entry = cache.get(key)
         if entry is None:
             views, leaves = [], []
-            for mod, name, shape, n, o in self.specs:
+            for i, (mod, name, shape, n, o) in enumerate(self.specs):
                 v = full[o:o + n].view(shape)
                 if self.trainable:
                     v = v.detach().requires_grad_(True)
+                    if self.collect_in_place:
+                        v._grad_place = _GradPlace(self, i)
                     leaves.append(v)
                 views.append(v)
             entry = cache[key] = (views, leaves)
@@ -119,6 +138,17 @@ class FlatParamGroup:
                 setattr(mod, name, v)
             self._installed_key = key
         return entry[1]
+
+    def grad_target(self, index: int):
+        mod, name, shape, n, o = self.specs[index]
+        if self.shard.grad is not None:
+            return self.shard.grad[o:o + n].view(shape), True
+        if self._collecting is None:
+            self._collecting = (torch.empty_like(self.shard.data), set())
+        flat, written = self._collecting
+        add = index in written
+        written.add(index)
+        return flat[o:o + n].view(shape), add
 
     def installed_leaves(self) -> List[torch.Tensor]:
         """Autograd-leaf views of the buffer that is currently installed (empty for frozen groups)."""
@@ -232,6 +262,7 @@ class _LayerFn(torch.autograd.Function):
         leaves = []
         for g, buf in zip(unit.groups, unit.buffers):
             leaves += g.install(buf, as_leaves=True)
+            g._collecting = None        # (left behind by a backward pass that failed in this block)
         local = [p for p in unit.local_params if p.requires_grad]
         xin = x.detach().requires_grad_(True)
         layer = runner.model.model.layers[idx]
@@ -281,6 +312,9 @@ class ShardedMixtral:
             self.units.append(FsdpUnit(f"layers.{i}", [(f"model.layers.{i}", layer)], shard_group, exclude))
         self.root = FsdpUnit("root", [("model.embed_tokens", model.model.embed_tokens),
                                       ("model.norm", model.model.norm), ("lm_head", model.lm_head)], shard_group)
+        for u in self.units + [self.root]:
+            for g in u.groups:
+                g.collect_in_place = g.trainable and self.ws == 1 and self.rep == 1
         # register the flat shards so that model.parameters() / the optimizer see them
         shards = nn.ParameterList()
         for u in self.units + [self.root]:
@@ -558,15 +592,21 @@ class ShardedMixtral:
             # nothing to reduce: straight into the gradient of the flat parameter, written the first time (and published
             # when it is complete: a failure on the way leaves no uninitialised memory behind)
             fresh = g.shard.grad is None
-            flat = torch.empty_like(g.shard.data) if fresh else g.shard.grad
+            flat, written = g.shard.grad, ()
+            if fresh:
+                # (what the products have written already: only where scale is 1, see collect_in_place)
+                flat, written = g._collecting if g._collecting is not None else (torch.empty_like(g.shard.data), ())
+                g._collecting = None
             dst, src, end = [], [], 0
-            for (mod, name, shape, n, o), gr in zip(g.specs, grads):
+            for i, ((mod, name, shape, n, o), gr) in enumerate(zip(g.specs, grads)):
                 if fresh and end < o:
                     flat[end:o].zero_()                                      # alignment gaps
                 end = o + n
-                if gr is not None:
+                if gr is not None and i in written:
+                    flat[o:end].view(shape).add_(gr)
+                elif gr is not None:
                     dst.append(flat[o:end].view(shape)); src.append(gr if gr.dtype == flat.dtype else gr.to(flat.dtype))
-                elif fresh:
+                elif fresh and i not in written:
                     flat[o:end].zero_()
             if fresh and end < flat.numel():
                 flat[end:].zero_()
@@ -762,7 +802,7 @@ class ShardedMixtral:
             if tg is not None:
                 leaves = tg.installed_leaves()
                 grads = [leaf.grad for leaf in leaves]
-                if any(gr is not None for gr in grads):
+                if any(gr is not None for gr in grads) or tg._collecting is not None:
                     self._reduce_unit_grads(unit, grads)
                 for leaf in leaves:
                     leaf.grad = None
