@@ -107,6 +107,9 @@ int mdt_embedding(const void* table, const long long* ids, void* out, int tokens
 // dout; other rows are left alone.  scratch: tokens + rows ints
 int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int table_fp32, int add, int* scratch, int tokens, int rows, int cols,
                       cudaStream_t s);
+// A13 [E, H, 2r] = [s1 A1 | s3 A3], B1p = [B1^T | 0] and B3p = [0 | B3^T], both [E, F, 2r], from A [E, H, r], B [E, r, F]; r a multiple of 4
+int mdt_adapter_pack(const void* A1, const void* A3, float s1, float s3, const void* B1, const void* B3, void* A13, void* B1p, void* B3p, int E, int H,
+                     int F, int r, cudaStream_t s);
 // in place: logits (bf16, [rows, vocab]) become d(loss_sum)/dlogits * grad_scale; loss_sum/count accumulate
 int mdt_cross_entropy(void* logits, const long long* labels, float* loss_sum, float* count, int rows, int vocab,
                       long long ld, int ignore_index, float grad_scale, cudaStream_t s);

@@ -9,6 +9,7 @@
 
 #include <mutex>
 #include <optional>
+#include <string>
 #include <vector>
 
 #include "api.h"
@@ -36,7 +37,9 @@ struct Phase {
 };
 
 static cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
-static void check(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed with code ", rc); }
+// (the number goes in as text: this library carries its own copy of the C++ stream classes, whose number formatting looks for locale
+// facets that the process initialised in another copy, and crashed)
+static void check(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed with code ", std::to_string(rc)); }
 static const void* cptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 static void* mptr(const OptTensor& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 #define CHECK_BF16(t) TORCH_CHECK((t).scalar_type() == at::kBFloat16 && (t).is_cuda(), #t " must be a CUDA bf16 tensor")
@@ -235,6 +238,19 @@ void embedding_bwd(const Tensor& dout, const Tensor& ids, Tensor& dtable, bool a
   auto scratch = torch::empty({ids.numel() + dtable.size(0)}, ids.options().dtype(at::kInt));
   check(mdt_embedding_bwd(dout.data_ptr(), (const long long*)ids.data_ptr<int64_t>(), dtable.data_ptr(), dtable.scalar_type() == at::kFloat, add ? 1 : 0,
                           scratch.data_ptr<int>(), (int)ids.numel(), (int)dtable.size(0), (int)dtable.size(1), cur_stream()), "embedding_bwd");
+}
+// gate and up adapters as the expert products want them: {A13, B1p, B3p} (see api.h)
+std::vector<Tensor> adapter_pack(const Tensor& A1, const Tensor& A3, double s1, double s3, const Tensor& B1, const Tensor& B3) {
+  for (const Tensor* t : {&A1, &A3, &B1, &B3}) { CHECK_BF16(*t); TORCH_CHECK(t->dim() == 3, "adapter_pack: [E, rows, columns] factors"); }
+  c10::cuda::CUDAGuard guard(A1.device());
+  const int64_t E = A1.size(0), H = A1.size(1), r = A1.size(2), F = B1.size(2);
+  TORCH_CHECK(A3.sizes() == A1.sizes() && B3.sizes() == B1.sizes() && B1.size(0) == E && B1.size(1) == r, "adapter_pack: factors that do not belong together");
+  auto aligned = [](const Tensor& t) { Tensor c = t.contiguous(); return (reinterpret_cast<uintptr_t>(c.data_ptr()) & 7) == 0 ? c : c.clone(); };   // 8-byte loads
+  Tensor a1 = aligned(A1), a3 = aligned(A3), b1 = B1.contiguous(), b3 = B3.contiguous();
+  Tensor A13 = torch::empty({E, H, 2 * r}, A1.options()), B1p = torch::empty({E, F, 2 * r}, A1.options()), B3p = torch::empty({E, F, 2 * r}, A1.options());
+  check(mdt_adapter_pack(a1.data_ptr(), a3.data_ptr(), (float)s1, (float)s3, b1.data_ptr(), b3.data_ptr(), A13.data_ptr(), B1p.data_ptr(), B3p.data_ptr(), (int)E,
+                         (int)H, (int)F, (int)r, cur_stream()), "adapter_pack");
+  return {A13, B1p, B3p};
 }
 // logits are overwritten with d(mean loss)/dlogits * grad_scale; returns [loss_sum, count]
 Tensor cross_entropy(Tensor& logits, const Tensor& labels, int64_t ignore_index, double grad_scale) {
@@ -939,6 +955,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("embedding", &embedding);
   m.def("embedding_bwd", &embedding_bwd);
+  m.def("adapter_pack", &adapter_pack);
   m.def("cross_entropy", &cross_entropy);
   m.def("gemm_set_pair_policy", [](int64_t policy) { return (int64_t)mdt_gemm_set_pair_policy((int)policy); });
   m.def("gemm_set_pair_cap", [](int64_t n) { mdt_gemm_set_pair_cap((int)n); });

@@ -246,6 +246,12 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, xg, w1, w2, w3, plan, lora, wgrad_scale, wgrad_out, lora_ids, *lora_tensors):
+        return _GroupedSwiGLUMLP.run(ctx, xg, w1, w2, w3, plan, lora, wgrad_scale, wgrad_out, lora_ids, lora_tensors)[0]
+
+    @staticmethod
+    def run(ctx, xg, w1, w2, w3, plan, lora, wgrad_scale, wgrad_out, lora_ids, lora_tensors, kept=None):
+        """(y, (t13, t2)), the latter the adapters' intermediate products.  `kept`: those of an earlier pass over the same rows; then
+        only what the backward pass needs besides them is computed, and y is None."""
         E, F, H = w1.shape
         R = xg.shape[0]
         dev, dt = xg.device, xg.dtype
@@ -261,13 +267,13 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
             assert l1 is not None and l3 is not None, "expert LoRA must cover w1 and w3 together"
             (A1, B1, s1), (A3, B3, s3) = l1, l3
             r = A1.shape[2]
-            A13 = torch.cat([A1 * s1 if s1 != 1.0 else A1, A3 * s3 if s3 != 1.0 else A3], dim=2).contiguous()  # [E,H,2r], scale folded
-            t13 = torch.empty(R, 2 * r, dtype=dt, device=dev)
-            _g(1, xg, False, A13, True, t13, 2 * r, H, plan, wait=wait)
+            A13, B1p, B3p = ext.adapter_pack(A1, A3, s1, s3, B1, B3)          # scales folded into A13
+            if kept is None:
+                t13 = torch.empty(R, 2 * r, dtype=dt, device=dev)
+                _g(1, xg, False, A13, True, t13, 2 * r, H, plan, wait=wait)
+            else:
+                t13 = kept[0]
             wait = None
-            # [E, F, 2r]: the gate / up product wants adapters laid out like w1 and w3
-            z = B1.new_zeros(E, F, r)
-            B1p, B3p = torch.cat([B1.transpose(1, 2), z], dim=2), torch.cat([z, B3.transpose(1, 2)], dim=2)
             kw = dict(A_l=t13, B_l=B1p, B2_l=B3p, b_mn_l=False, K_l=2 * r)
         h = torch.empty(R, F, dtype=dt, device=dev)
         g = u = None
@@ -278,19 +284,23 @@ class _GroupedSwiGLUMLP(torch.autograd.Function):
             xg = xg.clone()          # all rows have arrived now; the receive buffer is re-used by later exchanges
         t2 = None
         kw2 = {}
-        if l2 is not None:
+        if l2 is not None and kept is None:
             A2, B2, s2 = l2
             t2 = torch.empty(R, A2.shape[2], dtype=dt, device=dev)
             _g(1, h, False, A2, True, t2, A2.shape[2], F, plan, alpha=s2)
             kw2 = dict(A_l=t2, B_l=B2, b_mn_l=True, K_l=A2.shape[2])
-        y = torch.empty(R, H, dtype=dt, device=dev)
-        # with ep_scatter the result rows go straight into the source ranks' buffers (y itself stays unwritten)
-        _g(1, h, False, w2, True, y, H, F, plan, scatter=getattr(plan, "ep_scatter", None), **kw2)
+        elif l2 is not None:
+            t2 = kept[1]
+        y = None
+        if kept is None:
+            y = torch.empty(R, H, dtype=dt, device=dev)
+            # with ep_scatter the result rows go straight into the source ranks' buffers (y itself stays unwritten)
+            _g(1, h, False, w2, True, y, H, F, plan, scatter=getattr(plan, "ep_scatter", None), **kw2)
         if need_grad:
             ctx.plan, ctx.lora, ctx.wgrad_scale, ctx.wgrad_out = plan, lora, wgrad_scale, wgrad_out
             ctx.n_lora, ctx.lora_ids = len(lora_tensors), lora_ids
             ctx.save_for_backward(xg, w1, w2, w3, g, u, h, t13, t2)
-        return y
+        return y, (t13, t2)
 
     @staticmethod
     def backward(ctx, dy):

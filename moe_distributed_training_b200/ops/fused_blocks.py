@@ -194,7 +194,8 @@ def moe_block_supported(layer, x) -> bool:
 
 class _MoEBlock(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, layer, *params):
+    def forward(ctx, x, call, *params):
+        layer, graph = call
         moe = layer.block_sparse_moe
         ex, mlp, a = moe.experts, moe.experts.mlp, moe.args
         E, k = a.moe_num_experts, a.moe_top_k
@@ -202,9 +203,8 @@ class _MoEBlock(torch.autograd.Function):
         lora_tensors = params[5:]
         x2 = x.contiguous()
         need = ctx.needs_input_grad
-        grad_mode = any(need)
+        grad_mode = graph and any(need)
         xn, rstd = ext.rmsnorm_fwd(x2, ln_w, layer.post_attention_layernorm.eps)
-        scores, wts, idx = ext.router_fwd(xn, Wr.contiguous(), k, True)
         with torch.set_grad_enabled(grad_mode):
             w1, w2, w3, lora, ws, wgrad_out = mlp.call_args(xn)
         # experts' own autograd body, run directly
@@ -212,12 +212,27 @@ class _MoEBlock(torch.autograd.Function):
         mctx = _Ctx(mneeds)
         ids = tuple(id(t) for t in lora_tensors)
         ep = ex.ep_group is not None and ex.ep_size > 1
+        # A block that is recomputed in the backward pass (layer._ckpt_mode, see _MoEBlockNative) keeps routing, grouped rows, expert
+        # outputs and the adapters' intermediate products of its first pass: the recomputation is RMSNorm and the gate / up product.
+        # (Local experts: an exchange would have to be kept as well.)
+        ckpt_mode = getattr(layer, "_ckpt_mode", 0) if not ep else 0
+        stash = getattr(layer, "_moe_stash", None)
+        if ckpt_mode == 2 and grad_mode and stash is not None:
+            layer._moe_stash = None
+            plan, wts, idx, xg, ys, kept = stash
+            C._GroupedSwiGLUMLP.run(mctx, xg, w1, w2, w3, plan, lora, float(ws), wgrad_out, ids, lora_tensors, kept)
+            ctx.layer, ctx.plan, ctx.mctx, ctx.eng, ctx.meta_c, ctx.n_params = layer, plan, mctx, None, None, len(params)
+            ctx.save_for_backward(x2, rstd, xn, wts, idx, ys, None, ln_w, Wr)
+            return torch.empty_like(x2)        # (the backward pass does not read the block's output)
+        scores, wts, idx = ext.router_fwd(xn, Wr.contiguous(), k, True)
         if not ep:
             plan = C.make_plan(idx, E)
             ex.last_tokens_per_expert = plan.tokens_per_expert
             xg = ext.gather_rows(xn, plan.src_slot, plan.padded_offsets, E, None, k)
-            yg = C._GroupedSwiGLUMLP.forward(mctx, xg, w1, w2, w3, plan, lora, float(ws), wgrad_out, ids, *lora_tensors)
+            yg, kept = C._GroupedSwiGLUMLP.run(mctx, xg, w1, w2, w3, plan, lora, float(ws), wgrad_out, ids, lora_tensors)
             ys = yg
+            if ckpt_mode == 1 and not grad_mode:
+                layer._moe_stash = (plan, wts, idx, xg, ys, kept)
             comb = ext.combine_rows(yg, plan.dest_row, wts, k, x2)      # + x
             eng = meta_c = expert_sorted = None
         else:
@@ -320,12 +335,13 @@ class _MoEBlockNative(torch.autograd.Function):
         return w.layout, ints, tens
 
     @staticmethod
-    def forward(ctx, x, layer, *params):
+    def forward(ctx, x, call, *params):
+        layer, graph = call
         moe = layer.block_sparse_moe
         ex, mlp, a = moe.experts, moe.experts.mlp, moe.args
         ln_w, Wr = params[0], params[1]
         x2 = x.contiguous()
-        grad_mode = any(ctx.needs_input_grad)
+        grad_mode = graph and any(ctx.needs_input_grad)
         with torch.set_grad_enabled(grad_mode):
             w1, w2, w3, _, ws, wgrad_out = mlp.call_args(x2)
         eng, layout, ints, tens = None, [], [], []
@@ -400,6 +416,9 @@ def moe_block(layer, x):
         for name in ("w1", "w2", "w3"):
             if name in lora.lora_A:
                 params += [lora.lora_A[name], lora.lora_B[name]]
+    # (inside a Function's forward pass gradients are off, and trainable weights count as needing one even where the caller has
+    # switched them off: whether a graph is built is known only here.  Without one the gate / up product stores h alone.)
+    call = (layer, torch.is_grad_enabled())
     if NATIVE_ISSUE and GEMM_FUSION and _native_moe_ok(layer):
-        return _MoEBlockNative.apply(x, layer, *params[:5])
-    return _MoEBlock.apply(x, layer, *params)
+        return _MoEBlockNative.apply(x, call, *params[:5])
+    return _MoEBlock.apply(x, call, *params)

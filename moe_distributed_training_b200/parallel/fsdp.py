@@ -245,10 +245,13 @@ class _LayerFn(torch.autograd.Function):
         ctx.save_for_backward(x)
         layer = runner.model.model.layers[idx]
         layer._ckpt_mode = 1 if runner.stash_exchange else 0     # the MoE sub-block may keep its exchange results
+        layer._moe_stash = None
         try:
             with torch.no_grad():
                 return layer(x, batch)
         finally:
+            # (kept with this pass: the layer may run on other batches before this one's backward pass)
+            ctx.moe_stash, layer._moe_stash = layer._moe_stash, None
             layer._ckpt_mode = 0
 
     @staticmethod
@@ -267,6 +270,7 @@ class _LayerFn(torch.autograd.Function):
         xin = x.detach().requires_grad_(True)
         layer = runner.model.model.layers[idx]
         layer._ckpt_mode = 2 if runner.stash_exchange else 0
+        layer._moe_stash, ctx.moe_stash = ctx.moe_stash, None
         try:
             with torch.enable_grad():
                 y = layer(xin, batch)

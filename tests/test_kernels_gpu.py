@@ -696,6 +696,54 @@ def test_weight_gradients_collected_in_place(recompute):
             _close(a, b, 1e-3, "gradient after a failure")
 
 
+@pytest.mark.parametrize("lora", ["none", "attn-only", "all"])
+@pytest.mark.parametrize("keep", [True, False])
+def test_two_micro_batches_before_their_backward_pass(lora, keep):
+    """Recomputed blocks keep routing and expert results of their own first pass, also where another batch has gone through the
+    layer since: the gradient of a sum of two losses is the sum of the two gradients (bf16 gradients, rounded twice)."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
+    from moe_distributed_training_b200.train.engine import build_engine
+    cfg = MixtralConfig(vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=2, num_key_value_heads=1,
+                        head_dim=128, num_local_experts=4, num_experts_per_tok=2)
+    mbs = list(batches(SyntheticInstructionDataset(cfg.vocab_size, 2, 60, 150), 1))
+
+    def grads(together):
+        eng = build_engine(cfg, dtype=torch.bfloat16, device_type="cuda", learning_rate=1e-3, seed=0, use_lora=lora)
+        torch.manual_seed(5)
+        for n, p in eng.model.named_parameters():
+            if "lora_B" in n:
+                p.data.normal_(0.0, 0.05)
+        eng.runner.stash_exchange = keep
+        losses = []
+        for mb in mbs:
+            mb = {k: (v.to(DEV) if torch.is_tensor(v) else v) for k, v in mb.items()}
+            loss = eng.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb["cu_seqlens"], max_seqlen=mb["max_seqlen"]).loss
+            if not together:
+                loss.backward()
+                eng.runner.finish_microbatch()
+            losses.append(loss)
+        if together:
+            sum(losses).backward()
+            eng.runner.finish_microbatch()
+        return [p.grad for p in eng.model.parameters() if p.grad is not None]
+    apart, together = grads(False), grads(True)
+    assert len(apart) == len(together) > 0
+    for a, b in zip(apart, together):
+        _close(a.reshape(-1), b.reshape(-1), 1.5e-2, "gradient")
+
+
+@pytest.mark.parametrize("E,H,F,r", [(1, 8, 8, 4), (3, 72, 200, 12), (8, 256, 1032, 16), (2, 64, 136, 100)])
+def test_adapter_pack(ops, E, H, F, r):
+    A1, A3, B1, B3 = _rand(E, H, r), _rand(E, H, r), _rand(E, r, F), _rand(E, r, F)
+    a13, b1, b3 = ops.ext.adapter_pack(A1, A3, 1.5, 2.0, B1, B3)
+    z = torch.zeros_like(B1.transpose(1, 2))
+    assert torch.equal(a13, torch.cat([A1 * 1.5, A3 * 2.0], dim=2))
+    assert torch.equal(b1, torch.cat([B1.transpose(1, 2), z], dim=2)) and torch.equal(b3, torch.cat([z, B3.transpose(1, 2)], dim=2))
+    with pytest.raises(RuntimeError):
+        ops.ext.adapter_pack(A1[:, :, :3], A3[:, :, :3], 1.0, 1.0, B1[:, :3], B3[:, :3])
+
+
 def test_embedding_and_cross_entropy(ops):
     from moe_distributed_training_b200.ops import reference
     torch.manual_seed(10)
