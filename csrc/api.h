@@ -61,6 +61,8 @@ typedef struct MdtGemmDesc {
 } MdtGemmDesc;
 
 int mdt_gemm(const MdtGemmDesc* desc, cudaStream_t stream);
+// n independent products; those with one narrow side (adapters of rank <= 64 and their gradients) run as one launch of up to 8
+int mdt_gemm_list(const MdtGemmDesc* descs, int n, cudaStream_t stream);
 long long mdt_gemm_launch_count(void);
 long long mdt_skinny_launch_count(void);
 // y[M, r] = alpha * x[M, K] * op(A), r <= 32: a_is_kr = 0 -> A is [r, K] (row stride lda), 1 -> A is [K, r]

@@ -84,7 +84,7 @@ void gather_registry_clear() {
 }
 
 // C = alpha * op(A) op(B) (+ LoRA segment) with the options of MdtGemmDesc; see csrc/api.h
-void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, int64_t M, int64_t N, int64_t K,
+MdtGemmDesc describe(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, int64_t M, int64_t N, int64_t K,
           int64_t G, const OptTensor& offsets, int64_t capacity_rows, const OptTensor& B2, const OptTensor& A_l,
           bool a_mn_l, const OptTensor& B_l, const OptTensor& B2_l, bool b_mn_l, int64_t K_l, const OptTensor& C2,
           const OptTensor& C3, bool accumulate, double alpha, const OptTensor& status, const OptTensor& tile_ready,
@@ -92,7 +92,6 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
           const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt, const OptTensor& alpha_dev = std::nullopt,
           const OptTensor& swiglu_g = std::nullopt, const OptTensor& swiglu_u = std::nullopt, const OptTensor& group_rows = std::nullopt) {
   CHECK_BF16(A); CHECK_BF16(B);
-  c10::cuda::CUDAGuard guard(A.device());
   MdtGemmDesc d;
   memset(&d, 0, sizeof(d));
   d.mode = (int)mode; d.M = (int)M; d.N = (int)N; d.K = (int)K; d.G = (int)G;
@@ -152,6 +151,18 @@ void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, 
     if (d.dual) lookup_ready(d.B2, &d.b2_ready);
     if (d.K_l > 0) lookup_ready(d.B_l, &d.bl_ready);
   }
+  return d;
+}
+
+void gemm(int64_t mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, int64_t M, int64_t N, int64_t K,
+          int64_t G, const OptTensor& offsets, int64_t capacity_rows, const OptTensor& B2, const OptTensor& A_l,
+          bool a_mn_l, const OptTensor& B_l, const OptTensor& B2_l, bool b_mn_l, int64_t K_l, const OptTensor& C2,
+          const OptTensor& C3, bool accumulate, double alpha, const OptTensor& status, const OptTensor& tile_ready,
+          const OptTensor& tile_expected, const OptTensor& row_dest_rank, const OptTensor& row_dest_row, const OptTensor& peer_out,
+          const OptTensor& peer_arrive, const OptTensor& residual = std::nullopt, const OptTensor& alpha_dev = std::nullopt,
+          const OptTensor& swiglu_g = std::nullopt, const OptTensor& swiglu_u = std::nullopt, const OptTensor& group_rows = std::nullopt) {
+  c10::cuda::CUDAGuard guard(A.device());
+  const MdtGemmDesc d = describe(mode, A, a_mn, B, b_mn, C, M, N, K, G, offsets, capacity_rows, B2, A_l, a_mn_l, B_l, B2_l, b_mn_l, K_l, C2, C3, accumulate, alpha, status, tile_ready, tile_expected, row_dest_rank, row_dest_row, peer_out, peer_arrive, residual, alpha_dev, swiglu_g, swiglu_u, group_rows);
   check(mdt_gemm(&d, cur_stream()), "mdt_gemm");
 }
 
@@ -584,14 +595,37 @@ namespace {
 
 struct Lin { Tensor W; OptTensor A, B; double s; };   // y = x W^T + s (x A^T) B^T
 
+// Small products that do not depend on one another, issued together (mdt_gemm_list).  It keeps its operands alive until then.
+struct ProductsTogether {
+  std::vector<MdtGemmDesc> list;
+  std::vector<Tensor> keep;
+  void add(int mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, int64_t M, int64_t N, int64_t K, double alpha, const OptTensor& status) {
+    list.push_back(describe(mode, A, a_mn, B, b_mn, C, M, N, K, 1, std::nullopt, 0, std::nullopt, std::nullopt, false, std::nullopt, std::nullopt, false, 0, std::nullopt,
+                            std::nullopt, false, alpha, status, std::nullopt, std::nullopt, std::nullopt, std::nullopt, std::nullopt, std::nullopt));
+    keep.insert(keep.end(), {A, B, C});
+  }
+  void launch() {
+    if (list.empty()) return;
+    check(mdt_gemm_list(list.data(), (int)list.size(), cur_stream()), "mdt_gemm_list");
+    list.clear();
+    keep.clear();
+  }
+};
+// Whether the products can take an adapter factor of rank r (the CUDA-core kernel takes any rank)
+bool product_rank(const Tensor& A, bool a_is_kr) {
+  const int64_t r = a_is_kr ? A.size(1) : A.size(0);
+  return r % 8 == 0 && r <= 64 && A.dim() == 2 && A.stride(1) == 1 && A.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(A.data_ptr()) & 15) == 0;
+}
+
 void gemm_raw(int mode, const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, int64_t M, int64_t N, int64_t K,
               const OptTensor& A_l, const OptTensor& B_l, bool b_mn_l, int64_t K_l, bool accumulate, double alpha, const OptTensor& status,
               const OptTensor& residual = std::nullopt) {
   gemm(mode, A, a_mn, B, b_mn, C, M, N, K, 1, std::nullopt, 0, std::nullopt, A_l, false, B_l, std::nullopt, b_mn_l, K_l, std::nullopt,
        std::nullopt, accumulate, alpha, status, std::nullopt, std::nullopt, std::nullopt, std::nullopt, std::nullopt, std::nullopt, residual);
 }
-// y = x W^T (+ LoRA) (+ residual, added in the GEMM's epilogue); returns (y, t) with t = s x A^T
-std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTensor& status, const OptTensor& residual = std::nullopt) {
+// y = x W^T (+ LoRA) (+ residual, added in the GEMM's epilogue); returns (y, t) with t = s x A^T (`given`: t where it is there already)
+std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTensor& status, const OptTensor& residual = std::nullopt,
+                                     const OptTensor& given = std::nullopt) {
   const int64_t M = x.size(0), K = x.size(1), N = l.W.size(0);
   auto y = torch::empty({M, N}, x.options());
   if (!l.A.has_value()) {
@@ -600,7 +634,9 @@ std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTen
   }
   const int64_t r = l.A->size(0);
   Tensor t;
-  if (skinny_preferred(x, *l.A, false)) {
+  if (given.has_value()) {
+    t = *given;
+  } else if (skinny_preferred(x, *l.A, false)) {
     t = skinny_mm(x, *l.A, false, l.s);
   } else {
     t = torch::empty({M, r}, x.options());
@@ -611,21 +647,30 @@ std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTen
 }
 // dx (+)= dy W (+ LoRA), and the requested parameter gradients
 struct LinGrads { OptTensor dW, dA, dB; };
-// w_out: where the weight gradient goes (and whether it is added to what is there) instead of a new tensor
+// w_out: where the weight gradient goes (and whether it is added to what is there) instead of a new tensor.  given: s dy B where it is
+// there already.  later: adapter gradients join these products instead of being launched here.
 LinGrads lin_bwd(const Tensor& dy, const Tensor& xin, const Lin& l, const OptTensor& t, bool need_w, bool need_a, bool need_b,
-                 Tensor& dx, bool accumulate, const OptTensor& status, const OptTensor& w_out = std::nullopt, bool w_add = false) {
+                 Tensor& dx, bool accumulate, const OptTensor& status, const OptTensor& w_out = std::nullopt, bool w_add = false,
+                 const OptTensor& given = std::nullopt, ProductsTogether* later = nullptr) {
   const int64_t M = dy.size(0), N = dy.size(1), K = l.W.size(1);
   LinGrads g;
   OptTensor dt;
   if (l.A.has_value()) {
     const int64_t r = l.A->size(0);
-    if (skinny_preferred(dy, *l.B, true)) {
+    if (given.has_value()) {
+      dt = given;
+    } else if (skinny_preferred(dy, *l.B, true)) {
       dt = skinny_mm(dy, *l.B, true, l.s);                                                                           // s dy B
     } else {
       dt = torch::empty({M, r}, dy.options());
       gemm_raw(0, dy, false, *l.B, true, *dt, M, r, N, std::nullopt, std::nullopt, false, 0, false, l.s, status);
     }
     gemm_raw(0, dy, false, l.W, true, dx, M, K, N, dt, l.A, true, r, accumulate, 1.0, status);                       // dy W + dt A
+    if (later != nullptr && product_rank(*dt, true) && product_rank(*t, true)) {
+      if (need_a) { g.dA = torch::empty_like(*l.A); later->add(2, *dt, true, xin, true, *g.dA, r, K, M, 1.0, status); }
+      if (need_b) { g.dB = torch::empty_like(*l.B); later->add(2, dy, true, *t, true, *g.dB, N, r, M, 1.0, status); }
+      need_a = need_b = false;
+    }
     if (need_a) { g.dA = torch::empty_like(*l.A); gemm_raw(2, *dt, true, xin, true, *g.dA, r, K, M, std::nullopt, std::nullopt, false, 0, false, 1.0, status); }
     if (need_b) { g.dB = torch::empty_like(*l.B); gemm_raw(2, dy, true, *t, true, *g.dB, N, r, M, std::nullopt, std::nullopt, false, 0, false, 1.0, status); }
   } else {
@@ -668,6 +713,17 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
   // 77 tokens 67 / 93 us, 576 110 / 134, 1152 149 / 179, 4096 423 / 446, 9200 the same; with rank-16 adapters 576 145 / 185.
   Tensor q, k, v, qr, kr;
   OptTensor tq, tk, tv;
+  // the adapters' x A^T of all three in one launch (rank 16, 576 tokens: 9 us against three of 8 to 14)
+  if (lq.A.has_value() && lk.A.has_value() && lv.A.has_value() && product_rank(*lq.A, false) && product_rank(*lk.A, false) && product_rank(*lv.A, false)) {
+    ProductsTogether ts;
+    auto t_of = [&](const Lin& l) {
+      Tensor t = torch::empty({T, l.A->size(0)}, x.options());
+      ts.add(0, xn, false, *l.A, false, t, T, l.A->size(0), xn.size(1), l.s, status);
+      return t;
+    };
+    tq = t_of(lq); tk = t_of(lk); tv = t_of(lv);
+    ts.launch();
+  }
   static const bool side_streams = []() { const char* e = getenv("MDT_QKV_STREAMS"); return !(e != nullptr && e[0] == '0'); }();
   // (products of a few microseconds are not worth the ~25 us that the host spends on streams and events)
   if (side_streams && T * xn.size(1) * Hkv * d >= (int64_t)1 << 27) {
@@ -679,7 +735,7 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
     {
       c10::cuda::CUDAStreamGuard g1(s1);
       ready.block(s1);
-      std::tie(k, tk) = lin_fwd(xn, lk, status);
+      std::tie(k, tk) = lin_fwd(xn, lk, status, std::nullopt, tk);
       kr = rope(k.view({T, Hkv, d}), positions, theta, false);
       keep(k); keep(kr); if (tk.has_value()) keep(*tk);
       done1.record(s1);
@@ -687,18 +743,18 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
     {
       c10::cuda::CUDAStreamGuard g2(s2);
       ready.block(s2);
-      std::tie(v, tv) = lin_fwd(xn, lv, status);
+      std::tie(v, tv) = lin_fwd(xn, lv, status, std::nullopt, tv);
       keep(v); if (tv.has_value()) keep(*tv);
       done2.record(s2);
     }
-    std::tie(q, tq) = lin_fwd(xn, lq, status);
+    std::tie(q, tq) = lin_fwd(xn, lq, status, std::nullopt, tq);
     qr = rope(q.view({T, Hq, d}), positions, theta, false);
     done1.block(main_stream);
     done2.block(main_stream);
   } else {
-    std::tie(q, tq) = lin_fwd(xn, lq, status);
-    std::tie(k, tk) = lin_fwd(xn, lk, status);
-    std::tie(v, tv) = lin_fwd(xn, lv, status);
+    std::tie(q, tq) = lin_fwd(xn, lq, status, std::nullopt, tq);
+    std::tie(k, tk) = lin_fwd(xn, lk, status, std::nullopt, tk);
+    std::tie(v, tv) = lin_fwd(xn, lv, status, std::nullopt, tv);
     qr = rope(q.view({T, Hq, d}), positions, theta, false);
     kr = rope(k.view({T, Hkv, d}), positions, theta, false);
   }
@@ -740,16 +796,29 @@ std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tens
   auto nd = [&](size_t at, int k2) { return at + k2 < needs.size() ? (bool)needs[at + k2] : false; };
   Tensor dyc = dy.contiguous();
   Tensor o2 = o.view({T, Hq * d});
+  ProductsTogether grads_together;           // the adapters' gradients, all in one launch at the end
   Tensor d_o = torch::empty({T, Hq * d}, x.options());
-  put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status, place(3), adds(3)));
+  put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status, place(3), adds(3), std::nullopt, &grads_together));
   auto g3 = attention_bwd(qr, kr, v3, o, d_o.view({T, Hq, d}), lse, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d), status);
   Tensor dq = rope(g3[0], positions, theta, true).view({T, Hq * d});
   Tensor dk = rope(g3[1], positions, theta, true).view({T, Hkv * d});
   Tensor dv = g3[2].view({T, Hkv * d});
   Tensor d_xn = torch::empty({T, H}, x.options());
-  put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status, place(0), adds(0)));
-  put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status, place(1), adds(1)));
-  put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status, place(2), adds(2)));
+  OptTensor dtq, dtk, dtv;                   // s dy B of the three, one launch
+  if (lq.B.has_value() && lk.B.has_value() && lv.B.has_value() && product_rank(*lq.B, true) && product_rank(*lk.B, true) && product_rank(*lv.B, true)) {
+    ProductsTogether ts;
+    auto dt_of = [&](const Lin& l, const Tensor& g) {
+      Tensor t = torch::empty({T, l.B->size(1)}, x.options());
+      ts.add(0, g, false, *l.B, true, t, T, l.B->size(1), g.size(1), l.s, status);
+      return t;
+    };
+    dtq = dt_of(lq, dq); dtk = dt_of(lk, dk); dtv = dt_of(lv, dv);
+    ts.launch();
+  }
+  put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status, place(0), adds(0), dtq, &grads_together));
+  put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status, place(1), adds(1), dtk, &grads_together));
+  put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status, place(2), adds(2), dtv, &grads_together));
+  grads_together.launch();
   auto rb = rmsnorm_bwd(x, params[0], d_xn, rstd, dyc, (bool)needs[0]);     // + dy: the residual connection's gradient
   Tensor dx = rb[0];
   if (needs[0]) grads[0] = rmsnorm_dw(rb[1], params[0]);

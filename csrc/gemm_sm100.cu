@@ -1015,7 +1015,7 @@ __device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
 }
 
 template <int BN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(const __grid_constant__ GemmParams p) {
+__device__ __forceinline__ void cluster_product(const GemmParams& p, int index) {
   constexpr int STAGES = SplitShape<BN>::STAGES, STAGE_BYTES = SplitShape<BN>::STAGE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank(), S = (int)cluster_nctarank();
   Tile t;
-  if (!locate_tile<BN, BM>(p, (int)cluster_id_x(), t)) return;      // the same for the whole cluster
+  if (!locate_tile<BN, BM>(p, index, t)) return;                    // the same for the whole cluster
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(done_bar, 1);
@@ -1156,6 +1156,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(con
     store8(p.C, (p.mode == 2 ? (long long)t.g * p.c_group_stride : 0) + (long long)row * p.ldc + col, o, p.c_fp32, p.accumulate, p.R);
   }
   cluster_sync_all();                                             // nobody leaves while its partial tile is read
+}
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_cluster_kernel(const __grid_constant__ GemmParams p) {
+  cluster_product<BN>(p, (int)cluster_id_x());
+}
+// Several small products in one launch: the adapter products of a block, each a few tiles of some microseconds, of which the
+// launch, the set-up of the CTAs and the exchange are most.
+constexpr int MAX_PRODUCTS = 8;
+struct ProductList { int count, tile0[MAX_PRODUCTS + 1]; GemmParams p[MAX_PRODUCTS]; };
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_list_kernel(const __grid_constant__ ProductList list) {
+  const int c = (int)cluster_id_x();
+  int i = 0;
+  while (i + 1 < list.count && c >= list.tile0[i + 1]) ++i;
+  cluster_product<BN>(list.p[i], c - list.tile0[i]);
 }
 
 #include "gemm_transposed.cuh"
@@ -1653,18 +1668,9 @@ static int gemm_wgrad(const MdtGemmDesc* d, cudaStream_t stream) {
 }
 }  // namespace mdt
 
-extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
-  using namespace mdt;
-  // Tensor-map encoding is a driver call: make sure this host thread has the device's primary context
-  // bound (a thread that has issued no runtime work yet, e.g. a fresh autograd worker, has none).
-  static thread_local bool context_bound = false;
-  if (!context_bound) { cudaFree(nullptr); context_bound = true; }
-  if (g_num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
-  GemmParams p;
+namespace mdt {
+// The parameter block without its tensor maps; negative: a combination that no kernel takes.
+static int fill_params(const MdtGemmDesc* d, GemmParams& p) {
   memset(&p, 0, sizeof(p));
   p.M = d->M; p.N = d->N; p.K = d->K; p.K_l = d->K_l; p.G = d->G < 1 ? 1 : d->G; p.mode = d->mode;
   p.a_mn = d->a_mn; p.b_mn = d->b_mn; p.a_mn_l = d->a_mn_l; p.b_mn_l = d->b_mn_l; p.dual = d->dual;
@@ -1687,6 +1693,114 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
   if (p.row_dest_rank != nullptr && (p.dual || p.c_fp32 || p.accumulate || p.mode == 2)) return -12;
   if (p.N % 8 != 0 || p.ldc % 8 != 0) return -10;
   if (p.dual && (p.b_mn != 0 || p.c_fp32 || p.accumulate)) return -11;
+  return 0;
+}
+// Tensor maps; b_rows: rows of a box of a K-major B.
+static int fill_maps(const MdtGemmDesc* d, GemmParams& p, int b_rows) {
+  int rc = 0;
+  // A: [a_rows, a_cols] row-major, a_cols contiguous.  K-major: rows = M, cols = K.  MN-major: rows = depth, cols = M.
+  rc |= make_map(&p.tmA, d->A, d->a_cols, d->a_rows, 1, d->lda, 0, 64, d->a_mn ? 64 : BM, 2);
+  // B: [G, b_rows, b_cols].  K-major: rows = N, cols = K.  MN-major: rows = depth, cols = N.
+  const uint32_t box = d->b_mn ? 64 : b_rows;
+  rc |= make_map(&p.tmB, d->B, d->b_cols, d->b_rows, p.mode == 2 ? 1 : p.G, d->ldb, d->b_group_stride, 64, box, 3);
+  if (p.dual) rc |= make_map(&p.tmB2, d->B2, d->b_cols, d->b_rows, p.G, d->ldb, d->b_group_stride, 64, box, 3);
+  if (p.K_l > 0) {
+    rc |= make_map(&p.tmA_l, d->A_l, d->al_cols, d->al_rows, 1, d->lda_l, 0, 64, d->a_mn_l ? 64 : BM, 2);
+    const uint32_t box_l = d->b_mn_l ? 64 : b_rows;
+    rc |= make_map(&p.tmB_l, d->B_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, box_l, 3);
+    if (p.dual) rc |= make_map(&p.tmB2_l, d->B2_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, box_l, 3);
+  }
+  return rc;
+}
+static void prepare_host() {
+  // Tensor-map encoding is a driver call: make sure this host thread has the device's primary context
+  // bound (a thread that has issued no runtime work yet, e.g. a fresh autograd worker, has none).
+  static thread_local bool context_bound = false;
+  if (!context_bound) { cudaFree(nullptr); context_bound = true; }
+  if (g_num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+}
+
+// Whether a product may be one of a list: what the cluster kernel computes, with one 64-wide column of tiles in one of its directions.
+static bool listable(const MdtGemmDesc* d) {
+  return !d->dual && d->swiglu_g == nullptr && d->tile_ready == nullptr && d->row_dest_rank == nullptr && !(d->accumulate && d->R != nullptr) &&
+         d->mode != 1 && d->G <= 1 && d->offsets == nullptr && d->N % 8 == 0 && (d->mode == 2 ? (d->M <= BM || d->N <= 64) : d->N <= 64);
+}
+static int list_tiles(const MdtGemmDesc* d, int n, int bn) {
+  int tiles = 0;
+  for (int i = 0; i < n; ++i) tiles += ((d[i].M + BM - 1) / BM) * ((d[i].N + bn - 1) / bn);
+  return tiles;
+}
+template <int BN>
+static int launch_list(const MdtGemmDesc* d, int n, cudaStream_t stream) {
+  ProductList list;
+  memset(&list, 0, sizeof(list));
+  list.count = n;
+  int kb = 0;
+  for (int i = 0; i < n; ++i) {
+    const int refused = fill_params(d + i, list.p[i]);
+    if (refused != 0) return refused;
+    const int rc = fill_maps(d + i, list.p[i], BN);
+    if (rc != 0) return rc;
+    list.tile0[i + 1] = list.tile0[i] + list_tiles(d + i, 1, BN);
+    const int k = (d[i].K + BK - 1) / BK + (d[i].K_l + BK - 1) / BK;
+    if (k > kb) kb = k;
+  }
+  const int tiles = list.tile0[n];
+  if (tiles == 0) return 0;
+  // the depth over as many CTAs as are there at once, four k blocks for each of the deepest product
+  int S = MAX_CLUSTER;
+  while (S > 1 && (kb < 4 * S || tiles > max_clusters(S))) S /= 2;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_sm100_list_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitShape<BN>::SMEM);
+    if (e != cudaSuccess) return -100 - (int)e;
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(tiles * S)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = SplitShape<BN>::SMEM; cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_list_kernel<BN>, list);
+  ++g_launches;
+  if (e == cudaSuccess) e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -100 - (int)e;
+}
+// Tiles as narrow as leaves one round of them: a k block costs 0.22 us of a 64-wide tile and 0.48 of a 256-wide one, a round 5 besides.
+// The eight adapter gradients of an attention block (rank 16, 4096 columns, 576 rows) are 352 tiles of 64 columns or 144 of 256:
+// 30 and 15 us, one by one 8 of 11 to 15 and the gaps between them.
+static int launch_products(const MdtGemmDesc* d, int n, cudaStream_t stream) {
+  if (list_tiles(d, n, 64) <= g_num_sms) return launch_list<64>(d, n, stream);
+  return list_tiles(d, n, 128) <= g_num_sms ? launch_list<128>(d, n, stream) : launch_list<256>(d, n, stream);
+}
+}  // namespace mdt
+
+extern "C" int mdt_gemm_list(const MdtGemmDesc* d, int n, cudaStream_t stream) {
+  using namespace mdt;
+  prepare_host();
+  bool together = pair_policy() >= DEFAULT_POLICY && n > 1;
+  for (int i = 0; i < n; ++i) together = together && listable(d + i);
+  for (int i = 0; i < n; ) {
+    const int m = together ? (n - i < MAX_PRODUCTS ? n - i : MAX_PRODUCTS) : 1;
+    const int rc = m > 1 ? launch_products(d + i, m, stream) : mdt_gemm(d + i, stream);
+    if (rc != 0) return rc;
+    i += m;
+  }
+  return 0;
+}
+
+extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
+  using namespace mdt;
+  prepare_host();
+  GemmParams p;
+  const int refused = fill_params(d, p);
+  if (refused != 0) return refused;
   const int BN = (p.dual || p.N > 128) ? 256 : 128;
   const int bn_out = p.dual ? BN / 2 : BN;
   int cluster_bn = 0;
@@ -1695,20 +1809,8 @@ extern "C" int mdt_gemm(const MdtGemmDesc* d, cudaStream_t stream) {
     return gemm_transposed(d, stream);
   if (pair_policy() >= DEFAULT_POLICY && wgrad_ok(d) && (pair_policy() == MAX_POLICY || wgrad_preferred(d, t_rows_hint, cluster))) return gemm_wgrad(d, stream);
   const bool pair = cluster == 0 && choose_tiling(d, pair_policy(), t_rows_hint, g_num_sms) != 0;
-  const bool half_box = pair;           // each CTA of a pair loads its half of B in boxes of 128 rows
-  int rc = 0;
-  // A: [a_rows, a_cols] row-major, a_cols contiguous.  K-major: rows = M, cols = K.  MN-major: rows = depth, cols = M.
-  rc |= make_map(&p.tmA, d->A, d->a_cols, d->a_rows, 1, d->lda, 0, 64, d->a_mn ? 64 : BM, 2);
-  // B: [G, b_rows, b_cols].  K-major: rows = N, cols = K.  MN-major: rows = depth, cols = N.
-  const uint32_t b_box_rows = d->b_mn ? 64 : (cluster ? cluster_bn : (half_box ? 128 : bn_out));
-  rc |= make_map(&p.tmB, d->B, d->b_cols, d->b_rows, p.mode == 2 ? 1 : p.G, d->ldb, d->b_group_stride, 64, b_box_rows, 3);
-  if (p.dual) rc |= make_map(&p.tmB2, d->B2, d->b_cols, d->b_rows, p.G, d->ldb, d->b_group_stride, 64, b_box_rows, 3);
-  if (p.K_l > 0) {
-    rc |= make_map(&p.tmA_l, d->A_l, d->al_cols, d->al_rows, 1, d->lda_l, 0, 64, d->a_mn_l ? 64 : BM, 2);
-    const uint32_t bl_box_rows = d->b_mn_l ? 64 : (cluster ? cluster_bn : (half_box ? 128 : bn_out));
-    rc |= make_map(&p.tmB_l, d->B_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, bl_box_rows, 3);
-    if (p.dual) rc |= make_map(&p.tmB2_l, d->B2_l, d->bl_cols, d->bl_rows, p.G, d->ldb_l, d->bl_group_stride, 64, bl_box_rows, 3);
-  }
+  // (each CTA of a pair loads its half of B in boxes of 128 rows)
+  const int rc = fill_maps(d, p, cluster ? cluster_bn : (pair ? 128 : bn_out));
   if (rc != 0) return rc;
   // upper bound on the number of tiles (the exact count may depend on device-side offsets)
   long long rows = (p.mode == 1) ? d->capacity_rows : p.M;

@@ -1059,6 +1059,45 @@ def test_fused_attention_block_matches_composed_ops(ops, lora):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("T,r", [(1, 16), (130, 8), (257, 64), (700, 72), (1100, 32)])
+@pytest.mark.parametrize("which", ["all", "q and v", "frozen o"])
+def test_adapter_products_of_a_block_together(ops, T, r, which):
+    """The adapters' x A^T, dy B and gradients as one launch for several projections, against the block issued product by product:
+    the same fp32 sums in another order and one bf16 rounding each (5e-3).  Rank 72 and partial adapters keep single launches."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.models.mixtral import MixtralDecoderLayer, PackedBatch, moe_args_from_config
+    from moe_distributed_training_b200.ops import fused_blocks
+    torch.manual_seed(T + r)
+    cfg = MixtralConfig(vocab_size=64, hidden_size=384, intermediate_size=128, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=1,
+                        head_dim=128, num_local_experts=2, num_experts_per_tok=1)
+    layer = MixtralDecoderLayer(cfg, moe_args_from_config(cfg, torch.bfloat16, DEV), torch.bfloat16, DEV)
+    attn = layer.self_attn
+    lins = [attn.q_proj, attn.v_proj] if which == "q and v" else [attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj]
+    for lin in lins:
+        lin.add_lora(r, 2 * r)
+    with torch.no_grad():
+        for n, p in layer.named_parameters():
+            p.copy_(1 + 0.1 * torch.randn_like(p)) if "layernorm" in n else p.normal_(0, 0.05)
+            p.requires_grad_("lora" in n)
+    if which == "frozen o":
+        attn.o_proj.lora_A["default"].weight.requires_grad_(False)
+    batch = PackedBatch(torch.tensor([0, T], dtype=torch.int32, device=DEV), torch.arange(T, device=DEV).int(), T)
+    x, go = _rand(T, 384), _rand(T, 384)
+    params = [p for p in attn.parameters() if p.requires_grad]
+    res = []
+    for native in (True, False):
+        xi = x.clone().requires_grad_(True)
+        fused_blocks.NATIVE_ISSUE = native
+        try:
+            y = fused_blocks.attention_block(layer, xi, batch)
+        finally:
+            fused_blocks.NATIVE_ISSUE = True
+        res.append([y] + list(torch.autograd.grad(y, [xi] + params, go)))
+    for i, (a, b) in enumerate(zip(*res)):
+        _close(a, b, 5e-3, f"output or gradient {i}")
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("lora", [False, True])
 def test_fused_moe_block_matches_composed_ops(ops, lora):
     """The single-node MoE sub-block (local experts) against the same layer evaluated op by op."""
