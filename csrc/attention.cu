@@ -105,6 +105,7 @@ __device__ __forceinline__ int find_block(const int* cu, int num_seqs, int token
 
 // ------------------------------------------------------------------------------------------- forward
 __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
+  after_predecessor();
   int seq_start, seq_end, qb;
   if (find_block(p.cu_seqlens, p.num_seqs, p.tokens, blockIdx.x, seq_start, seq_end, qb, p.status) < 0) return;
   const int h = blockIdx.y, kvh = h / (p.heads_q / p.heads_kv);
@@ -278,6 +279,7 @@ __device__ __forceinline__ void load_kv_tile(uint8_t* dst, const CUtensorMap* ma
 }
 
 __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(const __grid_constant__ AttnParams p) {
+  after_predecessor();
   int seq_start, seq_end, qb;
   if (find_block(p.cu_seqlens, p.num_seqs, p.tokens, blockIdx.x / p.heads_q, seq_start, seq_end, qb, p.status) < 0) return;
   qb = (seq_end - seq_start + AB - 1) / AB - 1 - qb;          // last (longest) block of a sequence first
@@ -528,6 +530,7 @@ struct AttnBwdParams {
 __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
                                                                const int* __restrict__ cu, int num_seqs, int tokens, int heads, int4* __restrict__ sched,
                                                                float* __restrict__ stats, float* __restrict__ dq, int* status) {
+  after_predecessor();
   int seq_start, seq_end, blk;
   const int flat = blockIdx.x, h = blockIdx.y;
   const int seq = find_block(cu, num_seqs, tokens, flat, seq_start, seq_end, blk, status);
@@ -582,6 +585,7 @@ __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __
 }
 
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
+  after_predecessor();
   const int sets = p.heads_q / p.hpc;                      // head sets; the sets of a block are neighbours in the grid
   const int4 work = p.sched[blockIdx.x / sets];
   const int seq_start = work.x, seq_end = work.y, kb = work.z;
@@ -883,6 +887,7 @@ __global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __r
                                                                 bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
                                                                 const int* __restrict__ cu, int num_seqs, int blocks, int tokens, int heads_q,
                                                                 int heads_kv, int sets) {
+  after_predecessor();
   const int first = num_seqs > 0 ? min(max(cu[0], 0), tokens) : 0, end = num_seqs > 0 ? min(max(cu[num_seqs], first), tokens) : 0;
   if ((int)blockIdx.x < blocks) {
     int seq_start, seq_end, blk;
@@ -1000,8 +1005,8 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
     configured = true;
   }
   dim3 grid((total_tokens + AB - 1) / AB + num_seqs, heads_q);
-  if (serial) attn_fwd_kernel<<<grid, 128, ATT_SMEM, s>>>(p);
-  else attn_fwd_pipelined_kernel<<<grid.x * grid.y, FWD2_THREADS, FWD2_SMEM, s>>>(p);
+  if (serial) launch_after(attn_fwd_kernel, grid, 128, ATT_SMEM, s, p);
+  else launch_after(attn_fwd_pipelined_kernel, grid.x * grid.y, FWD2_THREADS, FWD2_SMEM, s, p);
   ++g_att_launches;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - (int)e;
@@ -1065,14 +1070,14 @@ extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, co
     if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM) != cudaSuccess) return -4;
     configured = true;
   }
-  attn_bwd_prepare_kernel<<<dim3((unsigned)b.blocks, heads_q), 256, 0, s>>>((const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs,
+  launch_after(attn_bwd_prepare_kernel, dim3((unsigned)b.blocks, heads_q), 256, 0, s, (const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs,
                                                                             total_tokens, heads_q, reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq, status);
   ++g_att_launches;
-  attn_bwd_kernel<<<(unsigned)(b.blocks * b.sets), BWD_THREADS, BWD_SMEM, s>>>(p);
+  launch_after(attn_bwd_kernel, (unsigned)(b.blocks * b.sets), BWD_THREADS, BWD_SMEM, s, p);
   ++g_att_launches;
   long long extra = 0;                                       // CTAs (times heads_q) that add up partial dK, dV
   if (!direct) extra = (2LL * total_tokens * heads_kv * (HD / 8) + 256LL * heads_q - 1) / (256LL * heads_q);
-  attn_bwd_finalize_kernel<<<dim3((unsigned)(b.blocks + extra), heads_q), 256, 0, s>>>(p.dq, p.dk, p.dv, (bf16*)dq, (bf16*)dk, (bf16*)dv, cu_seqlens,
+  launch_after(attn_bwd_finalize_kernel, dim3((unsigned)(b.blocks + extra), heads_q), 256, 0, s, p.dq, p.dk, p.dv, (bf16*)dq, (bf16*)dk, (bf16*)dv, cu_seqlens,
                                                                                       num_seqs, (int)b.blocks, total_tokens, heads_q, heads_kv, b.sets);
   ++g_att_launches;
   cudaError_t e = cudaGetLastError();

@@ -58,6 +58,7 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 // ------------------------------------------------------------------------------------ RMSNorm
 __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y,
                                    float* __restrict__ rstd, int rows, int cols, float eps) {
+  after_predecessor();
   __shared__ float red[32];
   const int row = blockIdx.x;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (long long)row * cols);
@@ -90,6 +91,7 @@ template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ dy,
                                                           const float* __restrict__ rstd, const bf16* __restrict__ dres, bf16* __restrict__ dx,
                                                           float* __restrict__ dw_partial, int rows, int cols) {
+  after_predecessor();
   __shared__ float red[32];
   const int nv = cols / 8;
   const uint4* xr = reinterpret_cast<const uint4*>(x);
@@ -163,6 +165,7 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_kernel(const bf16* __restrict
 // partial rows are spread over the 8 warps of a CTA (32 columns each), eight loads in flight per lane.
 __global__ void __launch_bounds__(256) rmsnorm_dw_finalize_kernel(const float* __restrict__ partial, int n_partial, int cols, bf16* __restrict__ dw_bf16,
                                                                   float* __restrict__ dw_f32) {
+  after_predecessor();
   __shared__ float part[8][33];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(256) rmsnorm_dw_finalize_kernel(const float* _
 // 8000 tokens x 32 heads of 128: 85 us with one sincosf and 2-byte accesses per pair.
 __global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, const int* __restrict__ pos, int tokens,
                                                    int heads, int d, float log2_theta, int inverse, int vec) {
+  after_predecessor();
   extern __shared__ float angles[];            // cos [half] | sin [half]
   const int t = blockIdx.x;
   const int half = d / 2;
@@ -231,6 +235,7 @@ __global__ void __launch_bounds__(256) rope_kernel(const bf16* __restrict__ x, b
 
 // ------------------------------------------------------------------------------------ SwiGLU
 __global__ void swiglu_fwd_kernel(const uint4* __restrict__ g, const uint4* __restrict__ u, uint4* __restrict__ h, long long nv) {
+  after_predecessor();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
     float a[8], b[8]; unpack8(g[i], a); unpack8(u[i], b);
 #pragma unroll
@@ -241,6 +246,7 @@ __global__ void swiglu_fwd_kernel(const uint4* __restrict__ g, const uint4* __re
 // Copy of a capacity-sized row buffer that touches only the rows in use (count read from device memory).
 __global__ void copy_rows_used_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, long long nv,
                                       const int* __restrict__ rows_used, long long vecs_per_row) {
+  after_predecessor();
   const long long lim = (long long)rows_used[0] * vecs_per_row;
   nv = lim < nv ? lim : nv;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) dst[i] = src[i];
@@ -248,6 +254,7 @@ __global__ void copy_rows_used_kernel(const uint4* __restrict__ src, uint4* __re
 
 // ------------------------------------------------------------------------------------ embedding
 __global__ void embedding_kernel(const bf16* __restrict__ table, const long long* __restrict__ ids, bf16* __restrict__ out, int cols) {
+  after_predecessor();
   const long long id = ids[blockIdx.x];
   const uint4* src = reinterpret_cast<const uint4*>(table + id * cols);
   uint4* dst = reinterpret_cast<uint4*>(out + (long long)blockIdx.x * cols);
@@ -257,12 +264,14 @@ __global__ void embedding_kernel(const bf16* __restrict__ table, const long long
 // (head[id], then next[token]); the CTA of the token at the head adds their rows up in fp32 and rounds once.  A table of
 // 32000 x 4096 in fp32, cleared, added to with atomics and converted, took 198 us however few the tokens; this 9 for 576 of them.
 __global__ void embedding_list_kernel(const long long* __restrict__ ids, int* __restrict__ head, int* __restrict__ next, int tokens) {
+  after_predecessor();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < tokens) next[t] = atomicExch(head + ids[t], t);
 }
 template <bool F32>
 __global__ void embedding_bwd_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, const int* __restrict__ head, const int* __restrict__ next,
                                      void* __restrict__ dtable, int cols, int add) {
+  after_predecessor();
   const long long id = ids[blockIdx.x];
   if (head[id] != (int)blockIdx.x) return;
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
@@ -301,6 +310,7 @@ constexpr int ADAPTER_COLS = 64, ADAPTER_RANKS = 64;
 __global__ void __launch_bounds__(256) adapter_pack_kernel(const bf16* __restrict__ A1, const bf16* __restrict__ A3, float s1, float s3, const bf16* __restrict__ B1,
                                                            const bf16* __restrict__ B3, bf16* __restrict__ A13, bf16* __restrict__ B1p, bf16* __restrict__ B3p,
                                                            int E, int H, int F, int r) {
+  after_predecessor();
   __shared__ bf16 tile[2][ADAPTER_RANKS][ADAPTER_COLS + 2];
   const int strips = (F + ADAPTER_COLS - 1) / ADAPTER_COLS;
   if ((int)blockIdx.x < E * strips) {
@@ -359,6 +369,7 @@ __global__ void __launch_bounds__(256) adapter_pack_kernel(const bf16* __restric
 // ignored rows; loss_sum += lse - logit[label].  `count` must already hold the number of counted rows.
 __global__ void cross_entropy_kernel(bf16* __restrict__ logits, const long long* __restrict__ labels, float* __restrict__ loss_sum,
                                      const float* __restrict__ count, int vocab, long long ld, int ignore_index, float grad_scale) {
+  after_predecessor();
   extern __shared__ uint4 row_smem[];
   __shared__ float red[32];
   const int row = blockIdx.x;
@@ -402,6 +413,7 @@ __global__ void cross_entropy_kernel(bf16* __restrict__ logits, const long long*
   }
 }
 __global__ void count_labels_kernel(const long long* __restrict__ labels, int rows, int ignore_index, float* __restrict__ count) {
+  after_predecessor();
   __shared__ float red[32];
   float c = 0.f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) c += labels[i] != ignore_index ? 1.f : 0.f;
@@ -439,6 +451,7 @@ __device__ __forceinline__ bool aligned16(const void* a, const void* b, const vo
 __global__ void __launch_bounds__(256, 4) adamw_kernel(const MdtAdamTensor* __restrict__ tensors, float lr, float b1, float b2,
                                                        float eps, float wd, float ibc1, float ibc2, float gscale,
                                                        const float* __restrict__ gscale_dev) {
+  after_predecessor();
   const MdtAdamTensor t = tensors[blockIdx.y];
   if (gscale_dev != nullptr) gscale *= *gscale_dev;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -478,6 +491,7 @@ __global__ void __launch_bounds__(256, 4) adamw_kernel(const MdtAdamTensor* __re
 }
 
 __global__ void __launch_bounds__(256) sumsq_kernel(const void* __restrict__ x, long long n, int fp32, float* __restrict__ out) {
+  after_predecessor();
   __shared__ float red[32];
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
@@ -511,6 +525,7 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const void* __restrict__ x, 
 // y = a*y + b*x
 __global__ void __launch_bounds__(256) axpby_kernel(void* __restrict__ y, const void* __restrict__ x, long long n, float a, float b,
                                                     int y_fp32, int x_fp32) {
+  after_predecessor();
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
   long long done = 0;
@@ -542,6 +557,7 @@ __global__ void __launch_bounds__(256) axpby_kernel(void* __restrict__ y, const 
 // cap: upper bound on the grid in CTAs; <= 0 means -cap CTAs per SM of the current device (default 16 per SM)
 // dst_i (fp32) += src_i (bf16 or fp32) for up to MDT_MULTI_ADD_MAX tensors in one launch (pointers passed by value)
 __global__ void multi_add_kernel(const MdtMultiAdd a) {
+  after_predecessor();
   const int t = blockIdx.y;
   if (t >= a.count) return;
   float* __restrict__ dst = a.dst[t];
@@ -572,7 +588,7 @@ extern "C" long long mdt_elementwise_launch_count() { return g_ew_launches; }
 extern "C" int mdt_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int rows, int cols, float eps, cudaStream_t s) {
   if (cols % 8 != 0) return -1;
   if (rows == 0) return 0;
-  rmsnorm_fwd_kernel<<<rows, 256, 0, s>>>((const bf16*)x, (const bf16*)w, (bf16*)y, rstd, rows, cols, eps);
+  launch_after(rmsnorm_fwd_kernel, rows, 256, 0, s, (const bf16*)x, (const bf16*)w, (bf16*)y, rstd, rows, cols, eps);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -580,14 +596,14 @@ extern "C" int mdt_rmsnorm_bwd(const void* x, const void* w, const void* dy, con
                                float* dw_partial, int rows, int cols, int n_partial, cudaStream_t s) {
   if (cols % 8 != 0 || cols > 8 * 8 * 256) return -1;
   const int nv = (cols / 8 + 255) / 256;
-#define RMS_BWD(NV) rmsnorm_bwd_kernel<NV><<<n_partial, 256, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd, (const bf16*)dres, (bf16*)dx, dw_partial, rows, cols)
+#define RMS_BWD(NV) launch_after(rmsnorm_bwd_kernel<NV>, n_partial, 256, 0, s, (const bf16*)x, (const bf16*)w, (const bf16*)dy, rstd, (const bf16*)dres, (bf16*)dx, dw_partial, rows, cols)
   if (nv <= 1) RMS_BWD(1); else if (nv <= 2) RMS_BWD(2); else if (nv <= 4) RMS_BWD(4); else RMS_BWD(8);
 #undef RMS_BWD
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_rmsnorm_dw_finalize(const float* dw_partial, int n_partial, int cols, void* dw_bf16, float* dw_f32, cudaStream_t s) {
-  rmsnorm_dw_finalize_kernel<<<(cols + 31) / 32, 256, 0, s>>>(dw_partial, n_partial, cols, (bf16*)dw_bf16, dw_f32);
+  launch_after(rmsnorm_dw_finalize_kernel, (cols + 31) / 32, 256, 0, s, dw_partial, n_partial, cols, (bf16*)dw_bf16, dw_f32);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -597,28 +613,28 @@ extern "C" int mdt_rope(const void* x, void* y, const int* positions, int tokens
   const int vec = head_dim % 16 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
   const int work = vec ? heads * (head_dim / 16) : heads * (head_dim / 2);          // threads that have something to do
   const int threads = work <= 64 ? 64 : (work <= 128 ? 128 : 256);
-  rope_kernel<<<tokens, threads, (head_dim / 2) * 2 * sizeof(float), s>>>((const bf16*)x, (bf16*)y, positions, tokens, heads, head_dim, log2f(theta), inverse, vec);
+  launch_after(rope_kernel, tokens, threads, (head_dim / 2) * 2 * sizeof(float), s, (const bf16*)x, (bf16*)y, positions, tokens, heads, head_dim, log2f(theta), inverse, vec);
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_swiglu_fwd(const void* g, const void* u, void* h, long long n, cudaStream_t s) {
   if (n % 8 != 0) return -1;
   if (n == 0) return 0;
-  swiglu_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, s>>>((const uint4*)g, (const uint4*)u, (uint4*)h, n / 8);
+  launch_after(swiglu_fwd_kernel, grid_for(n / 8, 256), 256, 0, s, (const uint4*)g, (const uint4*)u, (uint4*)h, n / 8);
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_copy_rows_used(const void* src, void* dst, long long n, const int* rows_used, long long cols, cudaStream_t s) {
   if (n % 8 != 0 || cols % 8 != 0 || rows_used == nullptr) return -1;
   if (n == 0) return 0;
-  copy_rows_used_kernel<<<grid_for(n / 8, 256), 256, 0, s>>>((const uint4*)src, (uint4*)dst, n / 8, rows_used, cols / 8);
+  launch_after(copy_rows_used_kernel, grid_for(n / 8, 256), 256, 0, s, (const uint4*)src, (uint4*)dst, n / 8, rows_used, cols / 8);
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_embedding(const void* table, const long long* ids, void* out, int tokens, int cols, cudaStream_t s) {
   if (cols % 8 != 0) return -1;
   if (tokens == 0) return 0;
-  embedding_kernel<<<tokens, 128, 0, s>>>((const bf16*)table, ids, (bf16*)out, cols);
+  launch_after(embedding_kernel, tokens, 128, 0, s, (const bf16*)table, ids, (bf16*)out, cols);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -627,10 +643,10 @@ extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* d
   if (tokens == 0) return 0;
   int* head = scratch + tokens;
   if (cudaMemsetAsync(head, 0xff, (size_t)rows * sizeof(int), s) != cudaSuccess) return -2;
-  embedding_list_kernel<<<(tokens + 255) / 256, 256, 0, s>>>(ids, head, scratch, tokens);
+  launch_after(embedding_list_kernel, (tokens + 255) / 256, 256, 0, s, ids, head, scratch, tokens);
   MDT_CHECK_LAUNCH();
-  if (table_fp32) embedding_bwd_kernel<true><<<tokens, 256, 0, s>>>((const bf16*)dout, ids, head, scratch, dtable, cols, add);
-  else embedding_bwd_kernel<false><<<tokens, 256, 0, s>>>((const bf16*)dout, ids, head, scratch, dtable, cols, add);
+  if (table_fp32) launch_after(embedding_bwd_kernel<true>, tokens, 256, 0, s, (const bf16*)dout, ids, head, scratch, dtable, cols, add);
+  else launch_after(embedding_bwd_kernel<false>, tokens, 256, 0, s, (const bf16*)dout, ids, head, scratch, dtable, cols, add);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -639,7 +655,7 @@ extern "C" int mdt_adapter_pack(const void* A1, const void* A3, float s1, float 
   if (r < 4 || r % 4 != 0) return -1;
   const int strips = (F + ADAPTER_COLS - 1) / ADAPTER_COLS;
   const long long stretch = ((long long)E * H * r / 4 + 255) / 256;
-  adapter_pack_kernel<<<E * strips + (int)(stretch < 1024 ? stretch : 1024), 256, 0, s>>>((const bf16*)A1, (const bf16*)A3, s1, s3, (const bf16*)B1, (const bf16*)B3, (bf16*)A13,
+  launch_after(adapter_pack_kernel, E * strips + (int)(stretch < 1024 ? stretch : 1024), 256, 0, s, (const bf16*)A1, (const bf16*)A3, s1, s3, (const bf16*)B1, (const bf16*)B3, (bf16*)A13,
                                                                                         (bf16*)B1p, (bf16*)B3p, E, H, F, r);
   MDT_CHECK_LAUNCH();
   return 0;
@@ -654,9 +670,9 @@ extern "C" int mdt_cross_entropy(void* logits, const long long* labels, float* l
     if (cudaFuncSetAttribute(cross_entropy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
     configured = smem;
   }
-  count_labels_kernel<<<grid_for(rows, 256, 64), 256, 0, s>>>(labels, rows, ignore_index, count);
+  launch_after(count_labels_kernel, grid_for(rows, 256, 64), 256, 0, s, labels, rows, ignore_index, count);
   MDT_CHECK_LAUNCH();
-  cross_entropy_kernel<<<rows, 512, smem, s>>>((bf16*)logits, labels, loss_sum, count, vocab, ld, ignore_index, grad_scale);
+  launch_after(cross_entropy_kernel, rows, 512, smem, s, (bf16*)logits, labels, loss_sum, count, vocab, ld, ignore_index, grad_scale);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -664,7 +680,7 @@ extern "C" int mdt_adamw(const MdtAdamTensor* tensors_device, int num_tensors, l
                          float eps, float weight_decay, float bc1, float bc2, float grad_scale, const float* grad_scale_dev, cudaStream_t s) {
   if (num_tensors == 0) return 0;
   dim3 grid(grid_for((max_n + 7) / 8, 256, -16), num_tensors);
-  adamw_kernel<<<grid, 256, 0, s>>>(tensors_device, lr, beta1, beta2, eps, weight_decay, 1.0f / bc1, 1.0f / bc2, grad_scale, grad_scale_dev);
+  launch_after(adamw_kernel, grid, 256, 0, s, tensors_device, lr, beta1, beta2, eps, weight_decay, 1.0f / bc1, 1.0f / bc2, grad_scale, grad_scale_dev);
   MDT_CHECK_LAUNCH();
   return 0;
 }
@@ -675,19 +691,19 @@ extern "C" int mdt_multi_add(const MdtMultiAdd* a, cudaStream_t s) {
   for (int i = 0; i < a->count; ++i) max_n = a->n[i] > max_n ? a->n[i] : max_n;
   if (max_n == 0) return 0;
   dim3 grid(grid_for(max_n, 256, -4), a->count);
-  multi_add_kernel<<<grid, 256, 0, s>>>(*a);
+  launch_after(multi_add_kernel, grid, 256, 0, s, *a);
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_sumsq(const void* x, long long n, int fp32, float* out_accum, cudaStream_t s) {
   if (n == 0) return 0;
-  sumsq_kernel<<<grid_for(n, 256 * 8, -4), 256, 0, s>>>(x, n, fp32, out_accum);
+  launch_after(sumsq_kernel, grid_for(n, 256 * 8, -4), 256, 0, s, x, n, fp32, out_accum);
   MDT_CHECK_LAUNCH();
   return 0;
 }
 extern "C" int mdt_axpby(void* y, const void* x, long long n, float a, float b, int y_fp32, int x_fp32, cudaStream_t s) {
   if (n == 0) return 0;
-  axpby_kernel<<<grid_for(n, 256 * 4), 256, 0, s>>>(y, x, n, a, b, y_fp32, x_fp32);
+  launch_after(axpby_kernel, grid_for(n, 256 * 4), 256, 0, s, y, x, n, a, b, y_fp32, x_fp32);
   MDT_CHECK_LAUNCH();
   return 0;
 }

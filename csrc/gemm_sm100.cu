@@ -32,6 +32,7 @@
 
 #include "api.h"
 #include "comm.h"
+#include "common/host.h"
 #include "common/ptx.cuh"
 
 namespace mdt {
@@ -97,6 +98,13 @@ __device__ __forceinline__ bool wait_b_tile(const GemmParams& p, int g, int n0, 
 // exchange ran out: its metadata describe no rows and nothing may be stored into a peer on the strength of them).
 __device__ __forceinline__ bool gemm_dead(const GemmParams& p) {
   return p.status != nullptr && (p.tile_ready != nullptr || p.row_dest_rank != nullptr) && *reinterpret_cast<const volatile int*>(p.status) != 0;
+}
+
+// Set-up is done: from here on the kernel touches what others touch.  One that waits for peers or for a gather on another stream
+// keeps its successors out until it ends, so that their CTAs never take the place of those it waits for.
+__device__ __forceinline__ void gemm_begin(const GemmParams& p) {
+  wait_for_predecessor();
+  if (p.tile_ready == nullptr && p.row_dest_rank == nullptr && p.rdy_b.ready == nullptr && p.rdy_b2.ready == nullptr && p.rdy_bl.ready == nullptr) admit_successor();
 }
 
 // Order of the output tiles.  A persistent grid works on a window of consecutive tiles at a time; what that window
@@ -562,6 +570,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_kernel(const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  gemm_begin(p);
 
   auto fail = [&](int code) {
     *abort_flag = 1;
@@ -838,6 +847,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  gemm_begin(p);
 
   auto fail = [&](int code) {
     *abort_flag = 1;
@@ -1027,6 +1037,7 @@ __device__ __forceinline__ void cluster_product(const GemmParams& p, int index) 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)cluster_ctarank(), S = (int)cluster_nctarank();
   Tile t;
+  if (p.offsets != nullptr) wait_for_predecessor();
   if (!locate_tile<BN, BM>(p, index, t)) return;                    // the same for the whole cluster
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -1039,6 +1050,7 @@ __device__ __forceinline__ void cluster_product(const GemmParams& p, int index) 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  gemm_begin(p);
   auto fail = [&](int code) {
     *abort_flag = 1;
     if (p.status != nullptr) atomicCAS(p.status, 0, code);
@@ -1296,7 +1308,7 @@ static cudaError_t launch(const GemmParams& p, int grid, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  gemm_sm100_kernel<BN, STAGES, SWIGLU><<<grid, GEMM_THREADS, smem, stream>>>(p);
+  launch_after(gemm_sm100_kernel<BN, STAGES, SWIGLU>, grid, GEMM_THREADS, smem, stream, p);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -1332,7 +1344,7 @@ static cudaError_t launch_pair(const GemmParams& p, int pairs_wanted, cudaStream
   }
   const int limit = (g_pair_cap > 0 && g_pair_cap < g_max_pairs) ? g_pair_cap : g_max_pairs;
   const int grid = 2 * (pairs_wanted < limit ? pairs_wanted : limit);
-  gemm_sm100_pair_kernel<SWIGLU><<<grid, GEMM_THREADS, smem, stream>>>(p);
+  launch_after(gemm_sm100_pair_kernel<SWIGLU>, grid, GEMM_THREADS, smem, stream, p);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -1378,7 +1390,7 @@ static cudaError_t launch_wgrad(const WgParams& p, cudaStream_t stream) {
   }
   const long long tiles = (long long)p.G * ((p.M + 255) / 256) * ((p.N + 255) / 256);
   const int limit = (g_pair_cap > 0 && g_pair_cap < max_pairs) ? g_pair_cap : max_pairs;
-  gemm_sm100_wgrad_kernel<ACC><<<2 * (int)(tiles < limit ? tiles : limit), GEMM_THREADS, WG_SMEM, stream>>>(p);
+  launch_after(gemm_sm100_wgrad_kernel<ACC>, 2 * (int)(tiles < limit ? tiles : limit), GEMM_THREADS, WG_SMEM, stream, p);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -1412,7 +1424,7 @@ static cudaError_t launch_transposed(const TPParams& p, long long tiles, cudaStr
   }
   const int limit = (g_pair_cap > 0 && g_pair_cap < max_pairs) ? g_pair_cap : max_pairs;
   const int grid = 2 * (int)(tiles < limit ? tiles : limit);
-  gemm_sm100_tpair_kernel<KIND><<<grid, GEMM_THREADS, TP_SMEM, stream>>>(p);
+  launch_after(gemm_sm100_tpair_kernel<KIND>, grid, GEMM_THREADS, TP_SMEM, stream, p);
   ++g_launches;
   return cudaGetLastError();
 }
@@ -1587,10 +1599,12 @@ static cudaError_t launch_cluster(const GemmParams& p, int tiles, int S, cudaStr
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(tiles * S)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = SplitShape<BN>::SMEM; cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;         // (see launch_after)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_cluster_kernel<BN>, p);
   ++g_launches;
   return e != cudaSuccess ? e : cudaGetLastError();
@@ -1763,10 +1777,12 @@ static int launch_list(const MdtGemmDesc* d, int n, cudaStream_t stream) {
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3((unsigned)(tiles * S)); cfg.blockDim = dim3(GEMM_THREADS); cfg.dynamicSmemBytes = SplitShape<BN>::SMEM; cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = S; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr; cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;         // (see launch_after)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_list_kernel<BN>, list);
   ++g_launches;
   if (e == cudaSuccess) e = cudaGetLastError();

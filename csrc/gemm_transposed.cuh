@@ -298,11 +298,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
-  if (warp == 2) tp_fill_table(p, tb, f_tiles, lane);
+  if (warp == 2) { wait_for_predecessor(); tp_fill_table(p, tb, f_tiles, lane); }
   tc_fence_before();
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  after_predecessor();
   const int stage_bytes = TP_A_BYTES + tb->widest * (BK * 2 / 2);
   const int stages = min(TP_RING_BYTES / stage_bytes, TP_MAX_STAGES);
 

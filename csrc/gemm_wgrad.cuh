@@ -85,6 +85,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   }
   if (warp == 1) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
   if (warp == 2) {
+    wait_for_predecessor();
     for (int g = lane; g < p.G; g += 32) {
       const int begin = p.offsets != nullptr ? p.offsets[g] : 0;
       int rows = p.offsets != nullptr ? p.offsets[g + 1] - begin : p.K;
@@ -97,6 +98,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  after_predecessor();
   auto fail = [&](int code) {
     *abort_flag = 1;
     if (p.status != nullptr) atomicCAS(p.status, 0, code);

@@ -136,6 +136,7 @@ template <int E_T, int TOK>
 __global__ void router_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ scores,
                                   bf16* __restrict__ weights, int* __restrict__ idx, int tokens, int hidden, int experts,
                                   int top_k, int normalize, int w_staged, float* __restrict__ stats) {
+  after_predecessor();
   const int lane = threadIdx.x & 31;
   const int warps_per_block = blockDim.x >> 5;
   __shared__ float s_stats[2 * MAX_E];
@@ -194,6 +195,7 @@ __global__ void router_bwd_kernel(const bf16* __restrict__ x, const bf16* __rest
                                   const bf16* __restrict__ dweights, const bf16* __restrict__ dscores, bf16* __restrict__ dx,
                                   float* __restrict__ dlogits, int tokens, int hidden, int experts, int top_k, int normalize,
                                   int accumulate_dx, int w_staged) {
+  after_predecessor();
   const int lane = threadIdx.x & 31;
   const int warps_per_block = blockDim.x >> 5, stride = gridDim.x * warps_per_block;
   const bf16* wp = stage_router_weights(w, experts, hidden, w_staged);
@@ -293,6 +295,7 @@ __global__ void __launch_bounds__(RR_THREADS, 2) router_rows_kernel(const bf16* 
                                                                     bf16* __restrict__ dx, float* __restrict__ dlogits, int tokens, int hidden,
                                                                     int experts, int top_k, int normalize, int accumulate_dx,
                                                                     float* __restrict__ stats) {
+  after_predecessor();
   __shared__ float red[2][RR_THREADS / 32][32];
   __shared__ float s_dl[RR_TOK][RR_E];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = hidden / 8;
@@ -446,6 +449,7 @@ constexpr int DW_TOKENS = 32;
 template <int E_T, int VEC>
 __global__ void __launch_bounds__(256) router_dw_kernel(const bf16* __restrict__ x, const float* __restrict__ dlogits, float* __restrict__ dw,
                                                         int tokens, int hidden, int experts) {
+  after_predecessor();
   __shared__ float s_dl[DW_TOKENS][E_T];
   const int col = (blockIdx.x * 256 + threadIdx.x) * VEC;
   float acc[E_T][VEC];
@@ -503,6 +507,7 @@ __global__ void __launch_bounds__(256) router_dw_kernel(const bf16* __restrict__
 constexpr int PLAN_CHUNK = 256;
 
 __global__ void plan_hist_kernel(const int* __restrict__ ids, int n, int experts, int* __restrict__ block_counts) {
+  after_predecessor();
   __shared__ int hist[MAX_E];
   for (int e = threadIdx.x; e < experts; e += blockDim.x) hist[e] = 0;
   __syncthreads();
@@ -518,6 +523,7 @@ __global__ void plan_hist_kernel(const int* __restrict__ ids, int n, int experts
 // single CTA: totals, padded group offsets, and per-(block, expert) first rows (in place in block_counts)
 __global__ void plan_scan_kernel(int* __restrict__ block_counts, int num_blocks, int experts, int block,
                                  int* __restrict__ counts, int* __restrict__ padded_offsets) {
+  after_predecessor();
   __shared__ int total[MAX_E];
   __shared__ int start[MAX_E + 1];
   for (int e = threadIdx.x; e < experts; e += blockDim.x) {
@@ -547,6 +553,7 @@ __global__ void plan_scan_kernel(int* __restrict__ block_counts, int num_blocks,
 
 __global__ void plan_scatter_kernel(const int* __restrict__ ids, int n, int experts, const int* __restrict__ block_base,
                                     int capacity, int* __restrict__ dest_row, int* __restrict__ src_slot) {
+  after_predecessor();
   __shared__ int warp_cnt[PLAN_CHUNK / 32][MAX_E];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = blockIdx.x * PLAN_CHUNK + threadIdx.x;
@@ -575,6 +582,7 @@ __global__ void plan_scatter_kernel(const int* __restrict__ ids, int n, int expe
 // rows at or beyond padded_offsets[E] are not touched.
 __global__ void gather_rows_kernel(const bf16* __restrict__ x, const int* __restrict__ src_slot, const int* __restrict__ padded_offsets,
                                    int experts, const bf16* __restrict__ slot_scale, bf16* __restrict__ out, int cols, int top_k) {
+  after_predecessor();
   const int r = blockIdx.x;
   if (padded_offsets != nullptr && r >= padded_offsets[experts]) return;
   const int slot = src_slot[r];
@@ -601,6 +609,7 @@ __global__ void gather_rows_kernel(const bf16* __restrict__ x, const int* __rest
 // (+ residual[t, :] when given)
 __global__ void combine_rows_kernel(const bf16* __restrict__ y, const int* __restrict__ dest_row, const bf16* __restrict__ weights,
                                     const bf16* __restrict__ residual, bf16* __restrict__ out, int cols, int top_k) {
+  after_predecessor();
   const int t = blockIdx.x;
   uint4* dst = reinterpret_cast<uint4*>(out + (long long)t * cols);
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
@@ -622,6 +631,7 @@ __global__ void combine_rows_kernel(const bf16* __restrict__ y, const int* __res
 // dweights[t, c] = <y[dest_row[t*k + c], :], dout[t, :]>; one warp per (t, c)
 __global__ void combine_wgrad_kernel(const bf16* __restrict__ y, const int* __restrict__ dest_row, const bf16* __restrict__ dout,
                                      bf16* __restrict__ dweights, int slots, int cols, int top_k) {
+  after_predecessor();
   const int lane = threadIdx.x & 31;
   const int s = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (s >= slots) return;
@@ -675,7 +685,7 @@ extern "C" int mdt_router_fwd(const void* x, const void* w, void* scores, void* 
   if (hidden % 8 != 0 || experts > MAX_E || top_k > MAX_K || top_k > experts) return -1;
   if (tokens == 0) return 0;
   if (router_rows_ok(hidden, experts)) {
-    router_rows_kernel<false><<<router_rows_grid(tokens), RR_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, idx, nullptr, nullptr,
+    launch_after(router_rows_kernel<false>, router_rows_grid(tokens), RR_THREADS, 0, s, (const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, idx, nullptr, nullptr,
                                                                             nullptr, nullptr, nullptr, tokens, hidden, experts, top_k, normalize, 0, stats);
     MDT_RT_CHECK();
     return 0;
@@ -685,7 +695,7 @@ extern "C" int mdt_router_fwd(const void* x, const void* w, void* scores, void* 
 #define RT_FWD(ET, TOK)                                                                                                        \
   {                                                                                                                            \
     const int staged = router_smem_ok((const void*)router_fwd_kernel<ET, TOK>, wbytes);                                        \
-    router_fwd_kernel<ET, TOK><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, \
+    launch_after(router_fwd_kernel<ET, TOK>, grid, 128, staged ? wbytes : 0, s, (const bf16*)x, (const bf16*)w, (bf16*)scores, (bf16*)weights, \
                                                                  idx, tokens, hidden, experts, top_k, normalize, staged, stats); \
   }
   if (experts <= 8 && router_pairs(tokens, grid)) RT_FWD(8, 2) else if (experts <= 8) RT_FWD(8, 1) else if (experts <= 16) RT_FWD(16, 1) else RT_FWD(MAX_E, 1)
@@ -706,14 +716,14 @@ extern "C" int mdt_router_bwd(const void* x, const void* w, const int* idx, cons
   {                                                                                                                         \
     const int staged = router_smem_ok((const void*)router_bwd_kernel<ET, TOK>, wbytes);                                     \
     if (router_rows_ok(hidden, experts))                                                                                    \
-      router_rows_kernel<true><<<router_rows_grid(tokens), RR_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, nullptr, nullptr, nullptr, idx, (const bf16*)dweights, \
+      launch_after(router_rows_kernel<true>, router_rows_grid(tokens), RR_THREADS, 0, s, (const bf16*)x, (const bf16*)w, nullptr, nullptr, nullptr, idx, (const bf16*)dweights, \
                                                                              (const bf16*)dscores, (bf16*)dx, dlogits, tokens, hidden, experts, top_k, normalize, accumulate_dx, nullptr); \
-    else router_bwd_kernel<ET, TOK><<<grid, 128, staged ? wbytes : 0, s>>>((const bf16*)x, (const bf16*)w, idx, (const bf16*)dweights,  \
+    else launch_after(router_bwd_kernel<ET, TOK>, grid, 128, staged ? wbytes : 0, s, (const bf16*)x, (const bf16*)w, idx, (const bf16*)dweights,  \
                                                                  (const bf16*)dscores, (bf16*)dx, dlogits, tokens, hidden,  \
                                                                  experts, top_k, normalize, accumulate_dx, staged);         \
     MDT_RT_CHECK();                                                                                                         \
     if (dw != nullptr) {                                                                                                    \
-      router_dw_kernel<ET, VEC><<<dim3((hidden + 256 * VEC - 1) / (256 * VEC), chunks), 256, 0, s>>>((const bf16*)x, dlogits, dw, tokens, hidden, experts); \
+      launch_after(router_dw_kernel<ET, VEC>, dim3((hidden + 256 * VEC - 1) / (256 * VEC), chunks), 256, 0, s, (const bf16*)x, dlogits, dw, tokens, hidden, experts); \
       MDT_RT_CHECK();                                                                                                       \
     }                                                                                                                       \
   }
@@ -728,13 +738,13 @@ extern "C" int mdt_make_plan(const int* expert_ids, int num_slots, int num_exper
   const int nb = (num_slots + PLAN_CHUNK - 1) / PLAN_CHUNK;
   cudaMemsetAsync(src_slot, 0xFF, (size_t)capacity * sizeof(int), s);
   if (nb > 0) {
-    plan_hist_kernel<<<nb, PLAN_CHUNK, 0, s>>>(expert_ids, num_slots, num_experts, scratch);
+    launch_after(plan_hist_kernel, nb, PLAN_CHUNK, 0, s, expert_ids, num_slots, num_experts, scratch);
     MDT_RT_CHECK();
   }
-  plan_scan_kernel<<<1, 256, 0, s>>>(scratch, nb, num_experts, block, counts, padded_offsets);
+  launch_after(plan_scan_kernel, 1, 256, 0, s, scratch, nb, num_experts, block, counts, padded_offsets);
   MDT_RT_CHECK();
   if (nb > 0) {
-    plan_scatter_kernel<<<nb, PLAN_CHUNK, 0, s>>>(expert_ids, num_slots, num_experts, scratch, capacity, dest_row, src_slot);
+    launch_after(plan_scatter_kernel, nb, PLAN_CHUNK, 0, s, expert_ids, num_slots, num_experts, scratch, capacity, dest_row, src_slot);
     MDT_RT_CHECK();
   }
   return 0;
@@ -744,7 +754,7 @@ extern "C" int mdt_gather_rows(const void* x, const int* src_slot, const int* pa
                                void* out, int capacity, int cols, int top_k, cudaStream_t s) {
   if (cols % 8 != 0) return -1;
   if (capacity == 0) return 0;
-  gather_rows_kernel<<<capacity, 128, 0, s>>>((const bf16*)x, src_slot, padded_offsets, num_experts, (const bf16*)slot_scale, (bf16*)out, cols, top_k);
+  launch_after(gather_rows_kernel, capacity, 128, 0, s, (const bf16*)x, src_slot, padded_offsets, num_experts, (const bf16*)slot_scale, (bf16*)out, cols, top_k);
   MDT_RT_CHECK();
   return 0;
 }
@@ -752,7 +762,7 @@ extern "C" int mdt_combine_rows(const void* y, const int* dest_row, const void* 
                                 int top_k, cudaStream_t s) {
   if (cols % 8 != 0) return -1;
   if (tokens == 0) return 0;
-  combine_rows_kernel<<<tokens, 128, 0, s>>>((const bf16*)y, dest_row, (const bf16*)weights, (const bf16*)residual, (bf16*)out, cols, top_k);
+  launch_after(combine_rows_kernel, tokens, 128, 0, s, (const bf16*)y, dest_row, (const bf16*)weights, (const bf16*)residual, (bf16*)out, cols, top_k);
   MDT_RT_CHECK();
   return 0;
 }
@@ -761,7 +771,7 @@ extern "C" int mdt_combine_wgrad(const void* y, const int* dest_row, const void*
   if (cols % 8 != 0) return -1;
   const int slots = tokens * top_k;
   if (slots == 0) return 0;
-  combine_wgrad_kernel<<<(slots + 3) / 4, 128, 0, s>>>((const bf16*)y, dest_row, (const bf16*)dout, (bf16*)dweights, slots, cols, top_k);
+  launch_after(combine_wgrad_kernel, (slots + 3) / 4, 128, 0, s, (const bf16*)y, dest_row, (const bf16*)dout, (bf16*)dweights, slots, cols, top_k);
   MDT_RT_CHECK();
   return 0;
 }
@@ -815,13 +825,13 @@ extern "C" int mdt_make_plan_noalloc(const int* expert_ids, int num_slots, int n
     if (me != cudaSuccess) { cudaGetLastError(); return -100 - (int)me; }
   }
   if (nb > 0) {
-    plan_hist_kernel<<<nb, PLAN_CHUNK, 0, s>>>(expert_ids, num_slots, num_experts, scratch);
+    launch_after(plan_hist_kernel, nb, PLAN_CHUNK, 0, s, expert_ids, num_slots, num_experts, scratch);
     MDT_RT_CHECK();
   }
-  plan_scan_kernel<<<1, 256, 0, s>>>(scratch, nb, num_experts, block, counts, padded_offsets);
+  launch_after(plan_scan_kernel, 1, 256, 0, s, scratch, nb, num_experts, block, counts, padded_offsets);
   MDT_RT_CHECK();
   if (nb > 0) {
-    plan_scatter_kernel<<<nb, PLAN_CHUNK, 0, s>>>(expert_ids, num_slots, num_experts, scratch, capacity, dest_row, src_slot);
+    launch_after(plan_scatter_kernel, nb, PLAN_CHUNK, 0, s, expert_ids, num_slots, num_experts, scratch, capacity, dest_row, src_slot);
     MDT_RT_CHECK();
   }
   return 0;

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "api.h"
+#include "common/host.h"
 
 namespace mdt {
 
@@ -35,6 +36,7 @@ template <int R, bool TRANS>
 __global__ void __launch_bounds__(SK_WARPS * 32) skinny_kernel(const bf16* __restrict__ x, const bf16* __restrict__ A,
                                                                bf16* __restrict__ y, int M, int K, int r, long long ldx,
                                                                long long lda, float alpha, int a_vec) {
+  after_predecessor();
   __shared__ float red[SK_WARPS][SK_ROWS][R];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * SK_ROWS;
@@ -158,11 +160,11 @@ extern "C" int mdt_skinny_mm(const void* x, const void* A, void* y, int M, int K
   const bf16 *xp = (const bf16*)x, *ap = (const bf16*)A;
   bf16* yp = (bf16*)y;
   if (r <= 16) {
-    if (a_is_kr) skinny_kernel<16, true><<<grid, SK_WARPS * 32, 0, s>>>(xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
-    else skinny_kernel<16, false><<<grid, SK_WARPS * 32, 0, s>>>(xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
+    if (a_is_kr) launch_after(skinny_kernel<16, true>, grid, SK_WARPS * 32, 0, s, xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
+    else launch_after(skinny_kernel<16, false>, grid, SK_WARPS * 32, 0, s, xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
   } else {
-    if (a_is_kr) skinny_kernel<32, true><<<grid, SK_WARPS * 32, 0, s>>>(xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
-    else skinny_kernel<32, false><<<grid, SK_WARPS * 32, 0, s>>>(xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
+    if (a_is_kr) launch_after(skinny_kernel<32, true>, grid, SK_WARPS * 32, 0, s, xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
+    else launch_after(skinny_kernel<32, false>, grid, SK_WARPS * 32, 0, s, xp, ap, yp, M, K, r, ldx, lda, alpha, a_vec);
   }
   ++g_skinny_launches;
   cudaError_t e = cudaGetLastError();
