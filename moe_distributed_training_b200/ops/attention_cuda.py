@@ -43,25 +43,8 @@ def _sdpa_attention(q, k, v, cu_seqlens, max_seqlen=None):
     return outs[0].contiguous() if len(outs) == 1 else torch.cat(outs, 0)
 
 
-class _Attention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, cu_seqlens, max_seqlen, scale):
-        from .cuda_ops import ext, status_tensor
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        o, lse = ext.attention_fwd(q, k, v, cu_seqlens, max_seqlen, scale, status_tensor(q.device))
-        ctx.save_for_backward(q, k, v, o, lse, cu_seqlens)
-        ctx.max_seqlen, ctx.scale = max_seqlen, scale
-        return o
-
-    @staticmethod
-    def backward(ctx, dout):
-        from .cuda_ops import ext, status_tensor
-        q, k, v, o, lse, cu = ctx.saved_tensors
-        dq, dk, dv = ext.attention_bwd(q, k, v, o, dout.contiguous(), lse, cu, ctx.max_seqlen, ctx.scale, status_tensor(q.device))
-        return dq, dk, dv, None, None, None
-
-
 def attention(q, k, v, cu_seqlens, max_seqlen=None):
     if q.shape[-1] != 128 or os.environ.get("MDT_ATTENTION_IMPL") == "sdpa":  # env switch: A/B timing against the library
         return sdpa_attention(q, k, v, cu_seqlens, max_seqlen)
-    return _Attention.apply(q, k, v, cu_seqlens.int(), int(max_seqlen or q.shape[0]), float(q.shape[-1]) ** -0.5)
+    from .cuda_ops import ext, status_tensor
+    return ext.attention(q, k, v, cu_seqlens.int(), int(max_seqlen or q.shape[0]), float(q.shape[-1]) ** -0.5, status_tensor(q.device))

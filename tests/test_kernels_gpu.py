@@ -861,6 +861,37 @@ def test_attention(ops, lens):
     ops.check_status(DEV)
 
 
+def test_attention_node_in_the_graph(ops):
+    """The node is part of autograd as any other: hooks on what it saves, inputs of other layouts, a frozen input, no graph without
+    gradients; transforms that it has no rule for refuse it."""
+    from moe_distributed_training_b200 import ops as front
+    torch.manual_seed(3)
+    q, k, v, do = (_rand(96, h, 128) for h in (4, 2, 2, 4))
+    cu = torch.tensor([0, 40, 96], device=DEV)                    # (any integer type)
+    want = None
+    for layout in ("plain", "strided", "hooks"):
+        leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        ins = [t.transpose(0, 1).contiguous().transpose(0, 1) if layout == "strided" else t for t in leaves]
+        packed = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(1), t.cpu())[1], lambda t: t.to(DEV)) if layout == "hooks" else torch.enable_grad():
+            o = front.attention(*ins, cu, 56)
+        assert o.requires_grad and (layout != "hooks" or len(packed) >= 5)
+        got = [o.detach()] + list(torch.autograd.grad(o, leaves, do))
+        want = want or got
+        for a, b in zip(got, want):
+            _close(a, b, 2e-3, layout)                            # (dQ sums in any order)
+    kf = k.clone().requires_grad_(True)
+    (front.attention(q, kf, v, cu, 56) * do).sum().backward()
+    _close(kf.grad, want[2], 2e-3, "only k")
+    with torch.no_grad():
+        assert not front.attention(q, kf, v, cu, 56).requires_grad
+    with pytest.raises(Exception):
+        torch.func.vmap(lambda a: front.attention(a, k, v, cu, 56))(torch.stack([q, q]))
+    with pytest.raises(Exception):
+        torch.func.jvp(lambda a: front.attention(a, k, v, cu, 56), (q,), (q,))
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("lens,heads,kv", [([1], 2, 2), ([127, 1, 129], 4, 2), ([255, 257, 128], 6, 2), ([640, 33, 1100, 5], 8, 2),
                                            ([130] * 40, 4, 4), ([2500, 1300], 32, 8), ([3000], 4, 1)])
 def test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv):
