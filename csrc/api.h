@@ -150,8 +150,7 @@ int mdt_combine_wgrad(const void* y, const int* dest_row, const void* dout, void
 int mdt_attention_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu_seqlens,
                       int num_seqs, int total_tokens, int max_seqlen, int heads_q, int heads_kv, int head_dim,
                       float scale, int* status /* optional device word, as in MdtGemmDesc; also set for sequences outside the rows */, cudaStream_t s);
-// scratch: mdt_attention_bwd_scratch() floats, 128-byte aligned (row statistics, fp32 dQ, and partial dK / dV where the
-// query heads of a kv head are spread over several CTAs)
+// scratch: mdt_attention_bwd_scratch() floats, 128-byte aligned (schedule and row statistics)
 long long mdt_attention_bwd_scratch(int num_seqs, int total_tokens, int max_seqlen, int heads_q, int heads_kv);
 int mdt_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                       void* dq, void* dk, void* dv, float* scratch, const int* cu_seqlens, int num_seqs, int total_tokens,

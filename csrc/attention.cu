@@ -5,10 +5,8 @@
 // stay in TMEM, where they are the A operand of P V.  attn_fwd_kernel is the serial form, one 128-row block at a time with P
 // through shared memory, for comparisons and for scales that are not positive.
 //
-// Backward: attn_bwd_prepare_kernel (row statistics, cleared dQ, schedule), attn_bwd_kernel (one CTA per 128-row key block
-// and set of query heads of one kv head, looping over the query blocks at or below the diagonal; keys are the rows, so that
-// P^T never leaves TMEM and only dS^T goes through shared memory; dV, dK in TMEM, dQ by fp32 reductions) and
-// attn_bwd_finalize_kernel (conversion to bf16, zeros for rows outside the sequences).
+// Backward: attn_bwd_prepare_kernel (row statistics, schedule, zeros for rows outside the sequences) and attn_bwd_kernel, whose
+// CTAs are of two kinds: dK, dV of a key block and a set of query heads, and dQ of a query block and head.
 //
 // A [128 x 128] bf16 tile in shared memory is always held as two [128 rows x 128 bytes] swizzled atoms; the same bytes serve
 // as a K-major or an MN-major operand, only the descriptor changes, so the transposed products need no data movement.
@@ -19,6 +17,7 @@
 #include <stdint.h>
 
 #include <stdlib.h>
+#include <string.h>
 
 #include <mutex>
 
@@ -486,56 +485,67 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
 }
 
 // ------------------------------------------------------------------------------------------- backward
-// Three launches.  `attn_bwd_prepare_kernel` computes, per (128-row block, query head), delta = rowsum(o * do) and the
-// row statistics in log2 units, clears the block's fp32 dQ tile and ranks the blocks by the work they mean as key blocks.
-// `attn_bwd_kernel`: one CTA per (key block, HPC query heads of one kv head), most work first; its loop runs over the
-// query blocks at or below the diagonal of each of its heads.  `attn_bwd_finalize_kernel` converts.
+// Two launches.  `attn_bwd_prepare_kernel` computes, per (128-row block, query head), delta = rowsum(o * do) and the row statistics in
+// log2 units, ranks the blocks by the work they mean as key blocks, and clears the gradients of rows outside the sequences.
+// `attn_bwd_kernel` holds two kinds of CTAs, most work first within each kind:
+//   dK, dV: one per (key block, HPC query heads of one kv head); its loop runs over the query blocks at or below the diagonal
+//   dQ:     one per (query block, head); its loop runs over the key blocks up to the diagonal
+// Each forms S and dP for itself, 7 products a 128 x 128 block instead of the 5 of a kernel that also adds dQ up from its key
+// blocks.  Those additions were what bounded it: 64 KB of fp32 reductions into L2 a block (25 % of its loop), dQ's place in TMEM that held
+// up the next block's dP, and a buffer of 128 floats a token and head to be cleared and converted.  Without them nothing leaves TMEM
+// but the results: P^T and dS^T (dK, dV) and dS (dQ) are operands of their products from there.
+// All launches, 32 / 8 heads, us, with dQ by reductions -> so: 613 tokens 53 -> 41, 2048 196 -> 177, 8192 1693 -> 1543, 16384 6851 -> 6697
+// (8192 alone: dK, dV of all blocks about 870, dQ 680: 216 and 226 a product).  What bounds it is the chain of a CTA, scores ->
+// exponentials -> product, with one CTA an SM (its operands fill shared memory and its accumulators TMEM) and half a block to overlap with.
+// Slower at 8192: 16 softmax warps (2379, they spill), two blocks in flight through halves of TMEM (1581), one wait for scores and
+// statistics together (1912), a share of the exponentials on the fp32 units (1604 with a quarter, 1688 with half).
 //
-// The loop keeps everything transposed (keys are the rows, i.e. the TMEM lanes), so that the probabilities never leave
-// TMEM: S^T = K Q^T, P^T = exp2(S^T - lse) is written back over S^T as bf16 and is the A operand of dV += P^T dO.  Only
-// dS^T goes through shared memory, where dK += dS^T Q reads it K-major and dQ = dS K reads the same bytes MN-major.
-// Per 128 x 128 block the five products take 5 x 512 clocks of tensor core and ~350 KB of shared-memory traffic (2800
-// clocks); the exponentials 1024 clocks.  16 warps:
-//   0-3 dQ: TMEM -> fp32 reductions into the block's tile (16-byte pieces of 32 adjacent rows: 512 bytes contiguous)
-//   4-11 softmax: warp -> (32 key rows, 64 of the 128 query columns)      12 TMA      13 MMA issue      14, 15 idle
-//   TMEM columns: [0,128) S^T, then P^T in [0,32) and [64,96);  [128,256) dP^T, then dQ;  [256,384) dV;  [384,512) dK
-// The tensor core works on dK_i, dQ_i while the softmax warps form P_{i+1}, and on dV_i, S_{i+1} while they form dS_i.
-// All three launches, 32 / 8 heads, against one block at a time per CTA of 128 threads: four sequences of 2124-7966 (23 372
-// tokens) 8.4 -> 4.4 ms, one of 16 384 13.0 -> 6.6 ms (830 TFLOP/s), 613 tokens 83 -> 63-71 us.  The reductions of dQ are what
-// bounds it: 16 384 tokens 6.4 ms, 4.8 ms without them (bulk reductions from shared memory took as long); without masks or
-// exponentials nothing changes.
-constexpr int BWD_THREADS = 512;
+// dK, dV keep keys as rows (TMEM lanes): S^T = K Q^T, P^T = exp2(S^T - lse) over S^T, dV += P^T dO, dS^T over dP^T = V dO^T, dK += dS^T Q.
+// 4 products of 512 clocks a block, 1024 clocks of exponentials; while the softmax warps form dS_i the tensor core works on dV_i and
+// S_{i+1}, while they form P_{i+1} on dK_i and dP_{i+1}.   TMEM columns: [0,128) S^T / P^T, [128,256) dP^T / dS^T, dV, dK
+// dQ keeps queries as rows: S = Q K^T in two buffers, dP = dO V^T, dS over dP, dQ += dS K; 3 products.   TMEM: S, S, dP / dS, dQ
+// (P^T and dS^T are stored by two warps for half of the columns each: the first 32 columns of each half's 64.)
+// Warps 0-7 softmax (warp -> 32 rows, 64 columns), 8 TMA, 9 MMA issue.
+// Where the query heads of a kv head are spread over several CTAs these form a cluster, which adds their dK, dV in the order of the
+// ranks through distributed shared memory; all results are the same in every run.
+constexpr int BWD_THREADS = 320;
 constexpr int BWD_STATS = 2 * AB;                              // lse2 | delta of a block, floats
 constexpr int BWD_SMEM = 7 * TILE_BYTES + 2 * BWD_STATS * 4 + 256 + 768;   // (768: what alignment to 1024 may take)
+constexpr int MAX_SETS = 8;                                    // CTAs that share a kv head's query heads: a cluster
 static_assert(BWD_SMEM <= 227 * 1024, "attention backward: shared memory of a CTA");
-// The fp32 dQ of a (block, query head) is a tile [column / 4][row][4] of the rows that the block has: a sequence's last block
-// takes no more room, clearing or reading back than its rows, which is what many short sequences consist of (1024 sequences
-// of 8 tokens, 32 heads, in whole tiles of 128 rows: 2.3 GB).
-__device__ __forceinline__ int rows_of_block(int row0, int seq_end) { return min(AB, seq_end - row0); }
-__device__ __forceinline__ long long dq_tile(int row0, int rows, int heads, int h) { return ((long long)row0 * heads + (long long)h * rows) * HD; }
 
 struct AttnBwdParams {
   CUtensorMap tmQ, tmK, tmV, tmdO;
   const int4* sched;            // by rank: {seq_start, seq_end, block, flat block}; seq_start < 0: none
   const float* stats;           // [flat block][head][lse2 x 128 | delta x 128]
-  float* dq;                    // tiles, see dq_tile
-  float* dk; float* dv;         // fp32 partial sums [token][head set][128], or NULL: all heads of a kv head in one CTA
-  bf16* dk_out; bf16* dv_out;   // then the results [token][kv head][128]
-  int heads_q, heads_kv, hpc;   // hpc: query heads per CTA
+  bf16* dq; bf16* dk; bf16* dv;
+  int heads_q, heads_kv, hpc;   // hpc: query heads per dK, dV CTA
   int tokens, blocks;           // rows of the tensors; entries of the schedule
   float scale_log2e, scale;
   int* status;
 };
 
 __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
-                                                               const int* __restrict__ cu, int num_seqs, int tokens, int heads, int4* __restrict__ sched,
-                                                               float* __restrict__ stats, float* __restrict__ dq, int* status) {
+                                                               const int* __restrict__ cu, int num_seqs, int tokens, int heads, int heads_kv, int4* __restrict__ sched,
+                                                               float* __restrict__ stats, bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv, int* status) {
   after_predecessor();
   int seq_start, seq_end, blk;
   const int flat = blockIdx.x, h = blockIdx.y;
   const int seq = find_block(cu, num_seqs, tokens, flat, seq_start, seq_end, blk, status);
   if (seq < 0) {
     if (h == 0 && threadIdx.x == 0) sched[flat] = make_int4(-1, 0, 0, 0);
+    // rows before the first and after the last sequence: zeros, from the CTAs that have no block
+    const int first = num_seqs > 0 ? min(max(cu[0], 0), tokens) : 0, end = num_seqs > 0 ? min(max(cu[num_seqs], first), tokens) : 0;
+    const int idle = (int)gridDim.x - (flat - blk), sub = threadIdx.x & 15;            // CTAs like this one, per head
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int u = blk * 16 + (threadIdx.x >> 4); u < first + tokens - end; u += idle * 16) {
+      const long long row = u < first ? u : end + (u - first);
+      reinterpret_cast<uint4*>(dq + (row * heads + h) * HD)[sub] = zero;
+      if (h < heads_kv) {
+        reinterpret_cast<uint4*>(dk + (row * heads_kv + h) * HD)[sub] = zero;
+        reinterpret_cast<uint4*>(dv + (row * heads_kv + h) * HD)[sub] = zero;
+      }
+    }
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -555,7 +565,7 @@ __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __
   const long long tile = (long long)flat * heads + h;
   // 16 lanes x 16 bytes hold a row, 16 rows per pass; all loads of the block are in flight at once
   const int sub = lane & 15, r0 = warp * 2 + (lane >> 4);
-  const int row0 = seq_start + blk * AB, rows = rows_of_block(row0, seq_end);
+  const int row0 = seq_start + blk * AB, rows = min(AB, seq_end - row0);
   uint4 a[8], b[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -564,9 +574,6 @@ __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __
     a[k] = reinterpret_cast<const uint4*>(o + at)[sub];
     b[k] = reinterpret_cast<const uint4*>(dout + at)[sub];
   }
-  float4* z = reinterpret_cast<float4*>(dq + dq_tile(row0, rows, heads, h));
-#pragma unroll 4
-  for (int i = threadIdx.x; i < rows * (HD / 4); i += 256) z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   float* st = stats + tile * BWD_STATS;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -584,362 +591,444 @@ __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __
   }
 }
 
+__device__ __forceinline__ uint4 pack8(const uint32_t* a) {
+  return make_uint4(pack2(__uint_as_float(a[0]), __uint_as_float(a[1])), pack2(__uint_as_float(a[2]), __uint_as_float(a[3])),
+                    pack2(__uint_as_float(a[4]), __uint_as_float(a[5])), pack2(__uint_as_float(a[6]), __uint_as_float(a[7])));
+}
+
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   after_predecessor();
-  const int sets = p.heads_q / p.hpc;                      // head sets; the sets of a block are neighbours in the grid
-  const int4 work = p.sched[blockIdx.x / sets];
+  const int sets = p.heads_q / p.hpc, per = sets / p.heads_kv;     // head sets; of one kv head: a cluster of the dK, dV CTAs
+  const int kv_ctas = p.blocks * sets;
+  const bool is_dq = (int)blockIdx.x >= kv_ctas;
+  const int unit = is_dq ? (int)blockIdx.x - kv_ctas : (int)blockIdx.x, width = is_dq ? p.heads_q : sets;   // the sets / heads of a block are neighbours
+  const int4 work = p.sched[unit / width];
   const int seq_start = work.x, seq_end = work.y, kb = work.z;
   if (seq_start < 0) return;
   const int nb = blocks_of(seq_start, seq_end, p.tokens);
   // an entry of sequences that overlap, or one that nobody wrote for them: what it leads to has to exist
-  if (kb < 0 || kb >= nb || work.w < 0 || work.w + nb - kb > p.blocks) {
+  if (kb < 0 || kb >= nb || work.w - kb < 0 || work.w + nb - kb > p.blocks) {
     if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, ST_CAPACITY);
     return;
   }
-  const int set = blockIdx.x % sets, h0 = set * p.hpc, kvh = h0 / (p.heads_q / p.heads_kv);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t *sK = smem, *sV = smem + TILE_BYTES, *sQ = smem + 2 * TILE_BYTES, *sdO = smem + 4 * TILE_BYTES, *sdS = smem + 6 * TILE_BYTES;
-  float* sStats = reinterpret_cast<float*>(smem + 7 * TILE_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * TILE_BYTES + 2 * BWD_STATS * 4);
-  uint64_t *barKV = bars, *barQ = bars + 1, *barQfree = bars + 3, *bardO = bars + 5, *bardOfree = bars + 7, *barS = bars + 9,
-           *barP = bars + 10, *bardP = bars + 11, *bardS = bars + 12, *bardSfree = bars + 13, *bardQ = bars + 14, *bardQfree = bars + 15,
-           *barDone = bars + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (smem + BWD_SMEM - 768 > smem_raw + BWD_SMEM) {       // uniform; never seen: dynamic shared memory starts 1024-aligned
-    if (tid == 0 && p.status != nullptr) atomicCAS(p.status, 0, ST_CAPACITY);
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, ST_CAPACITY);
     return;
   }
+  float* sStats = reinterpret_cast<float*>(smem + 7 * TILE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 7 * TILE_BYTES + 2 * BWD_STATS * 4);
+  // fixed operands | streamed ones, three stages of X and two of Y: loaded, free | row statistics loaded | S, P (by columns), dP, dS | all products done
+  uint64_t *barFix = bars, *barX = bars + 1, *barXfree = bars + 4, *barY = bars + 7, *barYfree = bars + 9, *barT = bars + 11, *barS = bars + 13, *barP = bars + 15,
+           *bardP = bars + 17, *bardS = bars + 18, *barDone = bars + 19;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    mbar_init(barKV, 1); mbar_init(barS, 1); mbar_init(barP, 8); mbar_init(bardP, 1); mbar_init(bardS, 8); mbar_init(bardSfree, 1);
-    mbar_init(bardQ, 1); mbar_init(bardQfree, 4); mbar_init(barDone, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&barQ[i], 1); mbar_init(&barQfree[i], 1); mbar_init(&bardO[i], 1); mbar_init(&bardOfree[i], 1); }
+    mbar_init(barFix, 1); mbar_init(bardP, 1); mbar_init(bardS, 8); mbar_init(barDone, 1);
+    for (int i = 0; i < 3; ++i) { mbar_init(&barX[i], 1); mbar_init(&barXfree[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&barY[i], 1); mbar_init(&barYfree[i], 1); mbar_init(&barT[i], 1); mbar_init(&barS[i], 1); mbar_init(&barP[i], 8); }
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 13) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int k0 = seq_start + kb * AB;
-  const int nq = nb - kb;                                   // query blocks per head
-  const int n_it = nq * p.hpc;
   auto fail = [&](int code) {
     *abort_flag = 1;
     if (p.status != nullptr) atomicCAS(p.status, 0, code);
   };
+  const int half = warp >> 2, r = (warp & 3) * 32 + lane;         // softmax warps: 64 columns, row
+  const uint32_t t_lane = (uint32_t)((warp & 3) * 32) << 16;
+  const uint32_t id_kk = make_idesc_bf16(128, 128, 0, 0), id_km = make_idesc_bf16(128, 128, 0, 1);
+  // fixed: K, V or Q, dO; streamed: X = Q or K, Y = dO or V
+  uint8_t *sF0 = smem, *sF1 = smem + TILE_BYTES, *sX = smem + 2 * TILE_BYTES, *sY = smem + 5 * TILE_BYTES;
+  const uint32_t aF0 = smem_u32(sF0), aF1 = smem_u32(sF1), aX = smem_u32(sX), aY = smem_u32(sY);
 
-  if (warp == 12) {
-    // ---------------------------------------------------------------- loads
-    bool ok = true;
-    if (elect_one()) {
-      mbar_expect_tx(barKV, 2 * TILE_BYTES);
-      load_tile(sK, &p.tmK, barKV, kvh * HD, k0);
-      load_tile(sV, &p.tmV, barKV, kvh * HD, k0);
-    }
-    int head = 0, i = 0;
-    for (int it = 0; it < n_it; ++it) {
-      const int st = it & 1;
-      const uint32_t ph = ((it >> 1) & 1) ^ 1;
-      const int h = h0 + head, q0 = seq_start + (kb + i) * AB;
-      ok = wait_parity_warp(&barQfree[st], ph, abort_flag);
-      if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
-      if (elect_one()) {
-        mbar_expect_tx(&barQ[st], TILE_BYTES + BWD_STATS * 4);
-        load_tile(sQ + st * TILE_BYTES, &p.tmQ, &barQ[st], h * HD, q0);
-        bulk_load(sStats + st * BWD_STATS, p.stats + ((long long)(work.w + i) * p.heads_q + h) * BWD_STATS, BWD_STATS * 4, &barQ[st]);
-      }
-      ok = wait_parity_warp(&bardOfree[st], ph, abort_flag);
-      if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
-      if (elect_one()) {
-        mbar_expect_tx(&bardO[st], TILE_BYTES);
-        load_tile(sdO + st * TILE_BYTES, &p.tmdO, &bardO[st], h * HD, q0);
-      }
-      if (++i == nq) { i = 0; ++head; }
-    }
-    if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
-      const uint64_t t0 = global_timer_ns();
-      while (global_timer_ns() - t0 < 20000ull) {}
-    }
-  } else if (warp == 13) {
-    // ---------------------------------------------------------------- MMA issue
-    const uint32_t id_kk = make_idesc_bf16(128, 128, 0, 0), id_km = make_idesc_bf16(128, 128, 0, 1), id_mm = make_idesc_bf16(128, 128, 1, 1);
-    const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aQ = smem_u32(sQ), adO = smem_u32(sdO), adS = smem_u32(sdS);
+  if (!is_dq) {
+    // ================================================================== dK, dV of a key block
+    const int set = unit % width, h0 = set * p.hpc, kvh = h0 / (p.heads_q / p.heads_kv);
+    const int k0 = seq_start + kb * AB, nq = nb - kb, n_it = nq * p.hpc;
     const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
-    auto issue_s = [&](int it) {      // S^T = K Q^T
+    if (warp == 8) {
+      // ---------------------------------------------------------------- loads
+      bool ok = true;
       if (elect_one()) {
-        const uint32_t q = aQ + (it & 1) * TILE_BYTES;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16(tS, desc_kmajor(aK, s), desc_kmajor(q, s), id_kk, s > 0);
-        umma_commit(barS);
+        mbar_expect_tx(barFix, 2 * TILE_BYTES);
+        load_tile(sF0, &p.tmK, barFix, kvh * HD, k0);
+        load_tile(sF1, &p.tmV, barFix, kvh * HD, k0);
       }
-    };
-    auto issue_dp = [&](int it) {     // dP^T = V dO^T
-      if (elect_one()) {
-        const uint32_t d = adO + (it & 1) * TILE_BYTES;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16(tdP, desc_kmajor(aV, s), desc_kmajor(d, s), id_kk, s > 0);
-        umma_commit(bardP);
-      }
-    };
-    bool ok = wait_parity_warp(barKV, 0, abort_flag) && wait_parity_warp(&barQ[0], 0, abort_flag);
-    if (ok) { tc_fence_after(); issue_s(0); ok = wait_parity_warp(&bardO[0], 0, abort_flag); }
-    if (ok) { tc_fence_after(); issue_dp(0); }
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int st = it & 1;
-      ok = wait_parity_warp(barP, it & 1, abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      if (elect_one()) {              // dV += P^T dO
-        const uint32_t d = adO + st * TILE_BYTES;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16_ta(tdV, tS + (s >> 2) * 64 + (s & 3) * 8, desc_mnmajor(d, s), id_km, it > 0 || s > 0);
-        umma_commit(&bardOfree[st]);
-      }
-      if (it + 1 < n_it) {            // over P^T: the products execute in the order of issue
-        ok = wait_parity_warp(&barQ[st ^ 1], ((it + 1) >> 1) & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        issue_s(it + 1);
-      }
-      ok = wait_parity_warp(bardS, it & 1, abort_flag);
-      if (!ok) break;
-      tc_fence_after();
-      if (elect_one()) {
-        const uint32_t q = aQ + st * TILE_BYTES;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16(tdP, desc_mnmajor(adS, s), desc_mnmajor(aK, s), id_mm, s > 0);              // dQ = dS K, over dP^T
-        umma_commit(bardQ);
-#pragma unroll
-        for (int s = 0; s < 8; ++s) umma_bf16(tdK, desc_kmajor(adS, s), desc_mnmajor(q, s), id_km, it > 0 || s > 0);      // dK += dS^T Q
-        umma_commit(&barQfree[st]);
-        umma_commit(bardSfree);
-      }
-      if (it + 1 < n_it) {
-        ok = wait_parity_warp(&bardO[st ^ 1], ((it + 1) >> 1) & 1, abort_flag) && wait_parity_warp(bardQfree, it & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        issue_dp(it + 1);
-      }
-    }
-    if (ok) { if (elect_one()) umma_commit(barDone); }
-    else fail(ST_TIMEOUT_FULL);
-  } else if (warp < 4) {
-    // ---------------------------------------------------------------- dQ (lane = query row)
-    const uint32_t t_row = tmem + 128 + ((uint32_t)(warp * 32) << 16);
-    int head = 0, i = 0;
-    for (int it = 0; it < n_it; ++it) {
-      if (!wait_parity_warp(bardQ, it & 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); break; }
-      tc_fence_after();
-      const int q0 = seq_start + (kb + i) * AB, rows = rows_of_block(q0, seq_end);
-      const bool valid = warp * 32 + lane < rows;
-      float* dst = p.dq + dq_tile(q0, rows, p.heads_q, h0 + head) + (warp * 32 + lane) * 4;
-#pragma unroll 1
-      for (int c = 0; c < HD; c += 64) {
-        uint32_t a[32], b[32];
-        tmem_ld_32x32(t_row + c, a);
-        tmem_ld_32x32(t_row + c + 32, b);
-        tmem_ld_wait();
-        if (c == 64) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bardQfree);
-        }
-        auto add = [&](int step) {       // floats from one group of four columns to the next
-#pragma unroll
-          for (int x = 0; x < 32; x += 4)
-            red_add_v4_f32(dst + ((c + x) >> 2) * step, __uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
-#pragma unroll
-          for (int x = 0; x < 32; x += 4)
-            red_add_v4_f32(dst + ((c + 32 + x) >> 2) * step, __uint_as_float(b[x]), __uint_as_float(b[x + 1]), __uint_as_float(b[x + 2]), __uint_as_float(b[x + 3]));
-        };
-        if (rows == AB) add(AB * 4);     // (offsets in the instructions: 2 % of the loop at 16384 tokens)
-        else if (valid) add(rows * 4);
-        __syncwarp();
-      }
-      if (++i == nq) { i = 0; ++head; }
-    }
-  } else if (warp < 12) {
-    // ---------------------------------------------------------------- softmax (lane = key row, 64 query columns)
-    const int half = (warp - 4) >> 2, r = (warp & 3) * 32 + lane;
-    const uint32_t t_row = tmem + half * 64 + ((uint32_t)((warp & 3) * 32) << 16);
-    const bool k_partial = k0 + AB > seq_end, k_valid = k0 + r < seq_end;
-    bool ok = true;
-    int i = 0;
-    for (int it = 0; it < n_it; ++it) {
-      const int st = it & 1;
-      const int q0 = seq_start + (kb + i) * AB;
-      const float* lse2 = sStats + st * BWD_STATS + half * 64;
-      const float* delta = lse2 + AB;
-      // block on the diagonal, last query block or last key block: elements are masked one by one
-      const bool masked = i == 0 || q0 + AB > seq_end || k_partial;
-      auto hidden = [&](int c) {       // query column half * 64 + c
-        const int q = half * 64 + c;
-        return !k_valid || (i == 0 && q < r) || q0 + q >= seq_end;
+      // (the statistics of a block go into one of two places, free once dK of two blocks ago is done: they come one block behind X)
+      auto load_stats = [&](int it, int h, int i) {
+        mbar_expect_tx(&barT[it & 1], BWD_STATS * 4);
+        bulk_load(sStats + (it & 1) * BWD_STATS, p.stats + ((long long)(work.w + i) * p.heads_q + h) * BWD_STATS, BWD_STATS * 4, &barT[it & 1]);
       };
-      if (!wait_parity_warp(&barQ[st], (it >> 1) & 1, abort_flag) || !wait_parity_warp(barS, it & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      float pr[64];
-#pragma unroll
-      for (int c = 0; c < 64; c += 16) {
-        uint32_t s[16];
-        tmem_ld_32x16(t_row + c, s);
-        tmem_ld_wait();
-#pragma unroll
-        for (int x = 0; x < 16; x += 4) {
-          const float4 l = *reinterpret_cast<const float4*>(lse2 + c + x);
-          pr[c + x] = fast_exp2(__uint_as_float(s[x]) * p.scale_log2e - l.x);
-          pr[c + x + 1] = fast_exp2(__uint_as_float(s[x + 1]) * p.scale_log2e - l.y);
-          pr[c + x + 2] = fast_exp2(__uint_as_float(s[x + 2]) * p.scale_log2e - l.z);
-          pr[c + x + 3] = fast_exp2(__uint_as_float(s[x + 3]) * p.scale_log2e - l.w);
+      int head = 0, i = 0, h_last = h0, i_last = 0;
+      for (int it = 0; it < n_it; ++it) {
+        const int h = h0 + head, q0 = seq_start + (kb + i) * AB;
+        ok = wait_parity_warp(&barXfree[it % 3], (it / 3 & 1) ^ 1, abort_flag);
+        if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+        if (elect_one()) {
+          mbar_expect_tx(&barX[it % 3], TILE_BYTES);
+          load_tile(sX + it % 3 * TILE_BYTES, &p.tmQ, &barX[it % 3], h * HD, q0);
+          if (it > 0) load_stats(it - 1, h_last, i_last);
+          if (it == n_it - 1 && it < 2) load_stats(it, h, i);
         }
-        if (masked) {
-#pragma unroll
-          for (int x = 0; x < 16; ++x) if (hidden(c + x)) pr[c + x] = 0.f;
+        h_last = h; i_last = i;
+        ok = wait_parity_warp(&barYfree[it & 1], ((it >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+        if (elect_one()) {
+          mbar_expect_tx(&barY[it & 1], TILE_BYTES);
+          load_tile(sY + (it & 1) * TILE_BYTES, &p.tmdO, &barY[it & 1], h * HD, q0);
         }
+        if (++i == nq) { i = 0; ++head; }
       }
-      {
-        uint32_t pk[32];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) pk[c] = pack2(pr[2 * c], pr[2 * c + 1]);
-        tmem_st_32x32(t_row, pk);      // over this warp's own part of S^T
-        tmem_st_wait();
+      if (ok && n_it > 2) {
+        ok = wait_parity_warp(&barXfree[n_it % 3], (n_it / 3 & 1) ^ 1, abort_flag);
+        if (!ok) fail(ST_TIMEOUT_EMPTY);
+        else if (elect_one()) load_stats(n_it - 1, h_last, i_last);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(barP);
-      if (!wait_parity_warp(bardP, it & 1, abort_flag)) { ok = false; break; }
-      if (it > 0 && !wait_parity_warp(bardSfree, (it - 1) & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < 64; c += 16) {
-        uint32_t d[16];
-        tmem_ld_32x16(t_row + 128 + c, d);
-        tmem_ld_wait();
-        float ds[16];
-#pragma unroll
-        for (int x = 0; x < 16; x += 4) {
-          const float4 dl = *reinterpret_cast<const float4*>(delta + c + x);
-          ds[x] = pr[c + x] * (__uint_as_float(d[x]) - dl.x) * p.scale;
-          ds[x + 1] = pr[c + x + 1] * (__uint_as_float(d[x + 1]) - dl.y) * p.scale;
-          ds[x + 2] = pr[c + x + 2] * (__uint_as_float(d[x + 2]) - dl.z) * p.scale;
-          ds[x + 3] = pr[c + x + 3] * (__uint_as_float(d[x + 3]) - dl.w) * p.scale;
-        }
-        if (masked) {
-#pragma unroll
-          for (int x = 0; x < 16; ++x) if (hidden(c + x)) ds[x] = 0.f;
-        }
-#pragma unroll
-        for (int x = 0; x < 16; x += 8)
-          *reinterpret_cast<uint4*>(sdS + tile_offset(r, half * 64 + c + x)) =
-              make_uint4(pack2(ds[x], ds[x + 1]), pack2(ds[x + 2], ds[x + 3]), pack2(ds[x + 4], ds[x + 5]), pack2(ds[x + 6], ds[x + 7]));
+      if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 20000ull) {}
       }
-      fence_proxy_async();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bardS);
-      if (++i == nq) i = 0;
-    }
-    ok = ok && wait_parity_warp(barDone, 0, abort_flag);
-    if (!ok) { if (lane == 0) fail(ST_TIMEOUT_TMEM_FULL); }
-    else {
-      // warps 4-7 write dV, warps 8-11 dK
-      tc_fence_after();
-      const uint32_t acc = tmem + 256 + half * 128 + ((uint32_t)((warp & 3) * 32) << 16);
-      const long long krow = k0 + r;
-      float* part = p.dk != nullptr ? (half == 0 ? p.dv : p.dk) + (krow * sets + set) * HD : nullptr;
-      bf16* out = (half == 0 ? p.dv_out : p.dk_out) + (krow * p.heads_kv + kvh) * HD;
-#pragma unroll 1
-      for (int c = 0; c < HD; c += 32) {
-        uint32_t a[32];
-        tmem_ld_32x32(acc + c, a);
-        tmem_ld_wait();
-        if (k_valid) {
-          if (part != nullptr) {
+    } else if (warp == 9) {
+      // ---------------------------------------------------------------- MMA issue (products execute in the order of issue)
+      auto issue_s = [&](int it) {      // S^T = K Q^T
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-            for (int x = 0; x < 32; x += 4)
-              *reinterpret_cast<float4*>(part + c + x) = make_float4(__uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
-          } else {
+          for (int s = 0; s < 8; ++s) umma_bf16(tS, desc_kmajor(aF0, s), desc_kmajor(aX + it % 3 * TILE_BYTES, s), id_kk, s > 0);
+          umma_commit(barS);
+        }
+      };
+      auto issue_dp = [&](int it) {     // dP^T = V dO^T
+        tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-            for (int x = 0; x < 32; x += 8)
-              *reinterpret_cast<uint4*>(out + c + x) =
-                  make_uint4(pack2(__uint_as_float(a[x]), __uint_as_float(a[x + 1])), pack2(__uint_as_float(a[x + 2]), __uint_as_float(a[x + 3])),
-                             pack2(__uint_as_float(a[x + 4]), __uint_as_float(a[x + 5])), pack2(__uint_as_float(a[x + 6]), __uint_as_float(a[x + 7])));
+          for (int s = 0; s < 8; ++s) umma_bf16(tdP, desc_kmajor(aF1, s), desc_kmajor(aY + (it & 1) * TILE_BYTES, s), id_kk, s > 0);
+          umma_commit(bardP);
+        }
+      };
+      bool ok = wait_parity_warp(barFix, 0, abort_flag) && wait_parity_warp(&barX[0], 0, abort_flag);
+      if (ok) { issue_s(0); ok = wait_parity_warp(&barY[0], 0, abort_flag); }
+      if (ok) issue_dp(0);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int st = it & 1;
+        for (int c = 0; c < 2 && ok; ++c) {     // dV += P^T dO: the first 32 columns of both halves while the others are formed
+          ok = wait_parity_warp(&barP[c], it & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              const int s = (x >> 1) * 4 + c * 2 + (x & 1);
+              umma_bf16_ta(tdV, tS + (s >> 2) * 64 + (s & 3) * 8, desc_mnmajor(aY + st * TILE_BYTES, s), id_km, it > 0 || c > 0 || x > 0);
+            }
+            if (c == 1) umma_commit(&barYfree[st]);
           }
         }
+        if (!ok) break;
+        if (it + 1 < n_it) {            // over P^T
+          ok = wait_parity_warp(&barX[(it + 1) % 3], (it + 1) / 3 & 1, abort_flag);
+          if (!ok) break;
+          issue_s(it + 1);
+        }
+        ok = wait_parity_warp(bardS, it & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {              // dK += dS^T Q
+#pragma unroll
+          for (int s = 0; s < 8; ++s) umma_bf16_ta(tdK, tdP + (s >> 2) * 64 + (s & 3) * 8, desc_mnmajor(aX + it % 3 * TILE_BYTES, s), id_km, it > 0 || s > 0);
+          umma_commit(&barXfree[it % 3]);
+        }
+        if (it + 1 < n_it) {            // over dS^T
+          ok = wait_parity_warp(&barY[st ^ 1], ((it + 1) >> 1) & 1, abort_flag);
+          if (!ok) break;
+          issue_dp(it + 1);
+        }
+      }
+      if (ok) { if (elect_one()) umma_commit(barDone); }
+      else fail(ST_TIMEOUT_FULL);
+    } else {
+      // ---------------------------------------------------------------- softmax (lane = key row, 64 query columns)
+      const uint32_t t_row = tmem + half * 64 + t_lane;
+      const bool k_valid = k0 + r < seq_end;
+      bool ok = true;
+      int i = 0;
+      for (int it = 0; it < n_it; ++it) {
+        const int st = it & 1;
+        const int q0 = seq_start + (kb + i) * AB;
+        const float* lse2 = sStats + st * BWD_STATS + half * 64;
+        const float* delta = lse2 + AB;
+        // block on the diagonal or last query block: elements are masked one by one (rows past the sequence are not stored)
+        const bool masked = i == 0 || q0 + AB > seq_end;
+        auto hidden = [&](int c) {       // query column half * 64 + c
+          const int q = half * 64 + c;
+          return (i == 0 && q < r) || q0 + q >= seq_end;
+        };
+        // (statistics come into registers before the waits: between the tensor core's reads of its operands a load from shared
+        // memory takes long, and 64 of them one by one made the loop a third longer)
+        if (!wait_parity_warp(&barT[st], (it >> 1) & 1, abort_flag)) { ok = false; break; }
+        float pr[64];
+#pragma unroll
+        for (int x = 0; x < 64; x += 4) {
+          const float4 l = *reinterpret_cast<const float4*>(lse2 + x);
+          pr[x] = l.x; pr[x + 1] = l.y; pr[x + 2] = l.z; pr[x + 3] = l.w;
+        }
+        if (!wait_parity_warp(barS, it & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        {
+          uint32_t s[2][32];
+          tmem_ld_32x32(t_row, s[0]);
+          tmem_ld_32x32(t_row + 32, s[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+              float& v = pr[c * 32 + x];
+              v = fast_exp2(fmaf(__uint_as_float(s[c][x]), p.scale_log2e, -v));
+            }
+            if (masked) {
+#pragma unroll
+              for (int x = 0; x < 32; ++x) if (hidden(c * 32 + x)) pr[c * 32 + x] = 0.f;
+            }
+#pragma unroll
+            for (int x = 0; x < 16; ++x) pk[x] = pack2(pr[c * 32 + 2 * x], pr[c * 32 + 2 * x + 1]);
+            tmem_st_32x16(t_row + c * 16, pk);      // over this warp's own part of S^T
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&barP[c]);
+          }
+        }
+        float dl[32];
+#pragma unroll
+        for (int x = 0; x < 32; x += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(delta + x);
+          dl[x] = v.x; dl[x + 1] = v.y; dl[x + 2] = v.z; dl[x + 3] = v.w;
+        }
+        if (!wait_parity_warp(bardP, it & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t pk[32];                 // dS^T without the factor `scale`, which dK gets at the end
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t d[32];
+          tmem_ld_32x32(t_row + 128 + c, d);
+          tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - dl[x]));
+          if (masked) {                  // (a branch of its own: tests between the products cost 900 clocks a block)
+#pragma unroll
+            for (int x = 0; x < 32; ++x) if (hidden(c + x)) d[x] = 0u;
+          }
+#pragma unroll
+          for (int x = 0; x < 16; ++x) pk[c / 2 + x] = pack2(__uint_as_float(d[2 * x]), __uint_as_float(d[2 * x + 1]));
+          if (c == 0) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 4) {
+              const float4 v = *reinterpret_cast<const float4*>(delta + 32 + x);
+              dl[x] = v.x; dl[x + 1] = v.y; dl[x + 2] = v.z; dl[x + 3] = v.w;
+            }
+          }
+        }
+        tmem_st_32x32(t_row + 128, pk);  // over this warp's own part of dP^T
+        tmem_st_wait();
+        tc_fence_before();
         __syncwarp();
+        if (lane == 0) mbar_arrive(bardS);
+        if (++i == nq) i = 0;
+      }
+      ok = ok && wait_parity_warp(barDone, 0, abort_flag);
+      if (!ok) { if (lane == 0) fail(ST_TIMEOUT_TMEM_FULL); }
+      else {
+        // warps 0-3 write dV, warps 4-7 dK
+        tc_fence_after();
+        const uint32_t acc = tmem + 256 + half * 128 + t_lane;
+        bf16* out = (half == 0 ? p.dv : p.dk) + ((long long)(k0 + r) * p.heads_kv + kvh) * HD;
+        float4* part = reinterpret_cast<float4*>(smem + half * 2 * TILE_BYTES) + r;      // [column / 4][row], over the operands
+#pragma unroll 1
+        for (int c = 0; c < HD; c += 32) {
+          uint32_t a[32];
+          tmem_ld_32x32(acc + c, a);
+          tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 32; ++x) a[x] = __float_as_uint(__uint_as_float(a[x]) * (half == 0 ? 1.f : p.scale));
+          if (per > 1) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 4)
+              part[(c + x) / 4 * AB] = make_float4(__uint_as_float(a[x]), __uint_as_float(a[x + 1]), __uint_as_float(a[x + 2]), __uint_as_float(a[x + 3]));
+          } else if (k_valid) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 8) *reinterpret_cast<uint4*>(out + c + x) = pack8(a + x);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (per > 1) {
+      // add up the cluster's partial tiles, an equal share of dV | dK by each CTA
+      cluster_sync_all();
+      const int rank = (int)cluster_ctarank();
+      constexpr int UNITS = 2 * AB * (HD / 8);                    // eight columns of a row; rows fastest
+      const uint32_t base = smem_u32(smem);
+      for (int u = UNITS * rank / per + tid; u < UNITS * (rank + 1) / per; u += BWD_THREADS) {
+        const int row = u % AB, g8 = u / AB % (HD / 8), mat = u / (AB * (HD / 8));
+        if (k0 + row >= seq_end) continue;
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        const uint32_t at = base + mat * 2 * TILE_BYTES + (2 * g8 * AB + row) * 16;
+        for (int c = 0; c < per; ++c) {
+          const uint32_t a = mapa_shared(at, c);
+          const float4 x = ld_cluster_v4(a), y = ld_cluster_v4(a + AB * 16);
+          s[0] += x.x; s[1] += x.y; s[2] += x.z; s[3] += x.w; s[4] += y.x; s[5] += y.y; s[6] += y.z; s[7] += y.w;
+        }
+        *reinterpret_cast<uint4*>((mat == 0 ? p.dv : p.dk) + ((long long)(k0 + row) * p.heads_kv + kvh) * HD + g8 * 8) =
+            make_uint4(pack2(s[0], s[1]), pack2(s[2], s[3]), pack2(s[4], s[5]), pack2(s[6], s[7]));
+      }
+      cluster_sync_all();                                         // nobody leaves while its tiles are read
+    }
+  } else {
+    // ================================================================== dQ of a query block: as many key blocks as its mirror image has query blocks
+    const int h = unit % width, kvh = h / (p.heads_q / p.heads_kv);
+    const int qb = nb - 1 - kb, q0 = seq_start + qb * AB, n = qb + 1;
+    const uint32_t tdP = tmem + 256, tdQ = tmem + 384;
+    if (warp == 8) {
+      // ---------------------------------------------------------------- loads
+      bool ok = true;
+      if (elect_one()) {
+        mbar_expect_tx(barFix, 2 * TILE_BYTES);
+        load_tile(sF0, &p.tmQ, barFix, h * HD, q0);
+        load_tile(sF1, &p.tmdO, barFix, h * HD, q0);
+      }
+      for (int j = 0; j < n; ++j) {
+        const int st = j & 1, sx = j % 3;
+        ok = wait_parity_warp(&barXfree[sx], (j / 3 & 1) ^ 1, abort_flag);
+        if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+        if (elect_one()) { mbar_expect_tx(&barX[sx], TILE_BYTES); load_tile(sX + sx * TILE_BYTES, &p.tmK, &barX[sx], kvh * HD, seq_start + j * AB); }
+        ok = wait_parity_warp(&barYfree[st], ((j >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) { fail(ST_TIMEOUT_EMPTY); break; }
+        if (elect_one()) { mbar_expect_tx(&barY[st], TILE_BYTES); load_tile(sY + st * TILE_BYTES, &p.tmV, &barY[st], kvh * HD, seq_start + j * AB); }
+      }
+      if (!ok) {   // give copies in flight a bounded time to land before the CTA leaves
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 20000ull) {}
+      }
+    } else if (warp == 9) {
+      // ---------------------------------------------------------------- MMA issue
+      auto issue_s = [&](int j) {       // S = Q K^T (the buffer's scores of two blocks ago were read before dS of that block came)
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int s = 0; s < 8; ++s) umma_bf16(tmem + (j & 1) * 128, desc_kmajor(aF0, s), desc_kmajor(aX + j % 3 * TILE_BYTES, s), id_kk, s > 0);
+          umma_commit(&barS[j & 1]);
+        }
+      };
+      auto issue_dp = [&](int j) {      // dP = dO V^T
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int s = 0; s < 8; ++s) umma_bf16(tdP, desc_kmajor(aF1, s), desc_kmajor(aY + (j & 1) * TILE_BYTES, s), id_kk, s > 0);
+          umma_commit(bardP);
+          umma_commit(&barYfree[j & 1]);
+        }
+      };
+      bool ok = wait_parity_warp(barFix, 0, abort_flag) && wait_parity_warp(&barX[0], 0, abort_flag);
+      if (ok) { issue_s(0); ok = wait_parity_warp(&barY[0], 0, abort_flag); }
+      if (ok) issue_dp(0);
+      for (int j = 0; j < n && ok; ++j) {
+        if (j + 1 < n) {
+          ok = wait_parity_warp(&barX[(j + 1) % 3], (j + 1) / 3 & 1, abort_flag);
+          if (!ok) break;
+          issue_s(j + 1);
+        }
+        ok = wait_parity_warp(bardS, j & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {              // dQ += dS K
+#pragma unroll
+          for (int s = 0; s < 8; ++s) umma_bf16_ta(tdQ, tdP + (s >> 2) * 64 + (s & 3) * 8, desc_mnmajor(aX + j % 3 * TILE_BYTES, s), id_km, j > 0 || s > 0);
+          umma_commit(&barXfree[j % 3]);
+        }
+        if (j + 1 < n) {                // over dS
+          ok = wait_parity_warp(&barY[(j + 1) & 1], ((j + 1) >> 1) & 1, abort_flag);
+          if (!ok) break;
+          issue_dp(j + 1);
+        }
+      }
+      if (ok) { if (elect_one()) umma_commit(barDone); }
+      else fail(ST_TIMEOUT_FULL);
+    } else {
+      // ---------------------------------------------------------------- softmax (lane = query row, 64 key columns)
+      const float* st = p.stats + ((long long)(work.w - kb + qb) * p.heads_q + h) * BWD_STATS;
+      const float lse2 = st[r], delta = st[AB + r];
+      bool ok = true;
+      for (int j = 0; j < n; ++j) {
+        const uint32_t t_s = tmem + (j & 1) * 128 + half * 64 + t_lane, t_dp = tdP + half * 64 + t_lane;
+        if (!wait_parity_warp(&barS[j & 1], (j >> 1) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        float pr[64];
+        {
+          uint32_t s[2][32];
+          tmem_ld_32x32(t_s, s[0]);
+          tmem_ld_32x32(t_s + 32, s[1]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 64; ++x) pr[x] = fast_exp2(fmaf(__uint_as_float(s[x >> 5][x & 31]), p.scale_log2e, -lse2));
+        }
+        if (!wait_parity_warp(bardP, j & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t pk[32];
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t d[32];
+          tmem_ld_32x32(t_dp + c, d);
+          tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - delta));
+          if (j == qb) {                 // diagonal: keys to the right of the query
+#pragma unroll
+            for (int x = 0; x < 32; ++x) if (half * 64 + c + x > r) d[x] = 0u;
+          }
+#pragma unroll
+          for (int x = 0; x < 16; ++x) pk[c / 2 + x] = pack2(__uint_as_float(d[2 * x]), __uint_as_float(d[2 * x + 1]));
+        }
+        tmem_st_32x32(t_dp, pk);         // over this warp's own part of dP
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bardS);
+      }
+      ok = ok && wait_parity_warp(barDone, 0, abort_flag);
+      if (!ok) { if (lane == 0) fail(ST_TIMEOUT_TMEM_FULL); }
+      else {
+        tc_fence_after();
+        const bool valid = q0 + r < seq_end;
+        bf16* out = p.dq + ((long long)(q0 + r) * p.heads_q + h) * HD + half * 64;
+#pragma unroll 1
+        for (int c = 0; c < 64; c += 32) {
+          uint32_t a[32];
+          tmem_ld_32x32(tdQ + half * 64 + t_lane + c, a);
+          tmem_ld_wait();
+#pragma unroll
+          for (int x = 0; x < 32; ++x) a[x] = __float_as_uint(__uint_as_float(a[x]) * p.scale);
+          if (valid) {
+#pragma unroll
+            for (int x = 0; x < 32; x += 8) *reinterpret_cast<uint4*>(out + c + x) = pack8(a + x);
+          }
+          __syncwarp();
+        }
       }
     }
   }
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 13) { tc_fence_after(); tmem_dealloc(tmem, 512); }
-}
-
-// dQ: tiles [column / 4][row][4] -> bf16 rows, one CTA per (block, head).  dK, dV (`sets` partial sums per kv head, when
-// there are several): the CTAs past the blocks, summed and converted eight columns at a time.  Rows before the first and
-// after the last sequence get zeros, from the CTAs that have no block.
-__global__ void __launch_bounds__(256) attn_bwd_finalize_kernel(const float* __restrict__ dq32, const float* __restrict__ dk32, const float* __restrict__ dv32,
-                                                                bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv,
-                                                                const int* __restrict__ cu, int num_seqs, int blocks, int tokens, int heads_q,
-                                                                int heads_kv, int sets) {
-  after_predecessor();
-  const int first = num_seqs > 0 ? min(max(cu[0], 0), tokens) : 0, end = num_seqs > 0 ? min(max(cu[num_seqs], first), tokens) : 0;
-  if ((int)blockIdx.x < blocks) {
-    int seq_start, seq_end, blk;
-    const int h = blockIdx.y;
-    if (find_block(cu, num_seqs, tokens, blockIdx.x, seq_start, seq_end, blk, nullptr) < 0) {
-      const int idle = blocks - ((int)blockIdx.x - blk), sub = threadIdx.x & 15;         // CTAs like this one, per head
-      const uint4 zero = make_uint4(0, 0, 0, 0);
-      for (int u = blk * 16 + (threadIdx.x >> 4); u < first + tokens - end; u += idle * 16) {
-        const long long row = u < first ? u : end + (u - first);
-        reinterpret_cast<uint4*>(dq + (row * heads_q + h) * HD)[sub] = zero;
-        if (dk32 == nullptr && h < heads_kv) {
-          reinterpret_cast<uint4*>(dk + (row * heads_kv + h) * HD)[sub] = zero;
-          reinterpret_cast<uint4*>(dv + (row * heads_kv + h) * HD)[sub] = zero;
-        }
-      }
-      return;
-    }
-    const int row0 = seq_start + blk * AB, rows = rows_of_block(row0, seq_end);
-    const float4* src = reinterpret_cast<const float4*>(dq32 + dq_tile(row0, rows, heads_q, h));
-    // eight lanes x 4 columns = 64 bytes of a row of dq, four rows per warp and pass; all loads in flight at once
-    const int cg = threadIdx.x & 7, rsub = threadIdx.x >> 3;
-    float4 v[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int r = (k >> 2) * 32 + rsub;
-      if (r < rows) v[k] = __ldcs(src + ((k & 3) * 8 + cg) * rows + r);
-    }
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int r = (k >> 2) * 32 + rsub;
-      if (r < rows)
-        *reinterpret_cast<uint2*>(dq + ((long long)(row0 + r) * heads_q + h) * HD + ((k & 3) * 8 + cg) * 4) = make_uint2(pack2(v[k].x, v[k].y), pack2(v[k].z, v[k].w));
-    }
-    return;
-  }
-  const int per = sets / heads_kv;                                       // partial sums per kv head
-  const long long n = (long long)tokens * heads_kv * (HD / 8);           // 8-column vectors of dK (then of dV)
-  const long long stride = (long long)(gridDim.x - blocks) * gridDim.y * 256;
-  for (long long e = (((long long)blockIdx.x - blocks) * gridDim.y + blockIdx.y) * 256 + threadIdx.x; e < 2 * n; e += stride) {
-    const bool isv = e >= n;
-    const long long v = isv ? e - n : e;
-    const int d = (int)(v % (HD / 8)) * 8;
-    const long long th = v / (HD / 8);                                   // token * heads_kv + kv head
-    const float* src = (isv ? dv32 : dk32) + (th * per) * HD + d;
-    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const long long row = th / heads_kv;
-    for (int g = 0; g < per && row >= first && row < end; ++g) {
-      const float4 a = *reinterpret_cast<const float4*>(src + (long long)g * HD), b = *reinterpret_cast<const float4*>(src + (long long)g * HD + 4);
-      s[0] += a.x; s[1] += a.y; s[2] += a.z; s[3] += a.w; s[4] += b.x; s[5] += b.y; s[6] += b.z; s[7] += b.w;
-    }
-    *reinterpret_cast<uint4*>((isv ? dv : dk) + th * HD + d) = make_uint4(pack2(s[0], s[1]), pack2(s[2], s[3]), pack2(s[4], s[5]), pack2(s[6], s[7]));
-  }
+  if (warp == 9) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
 typedef CUresult (*EncodeTiledFnA)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -1013,28 +1102,25 @@ extern "C" int mdt_attention_fwd(const void* q, const void* k, const void* v, vo
 }
 
 namespace {
-// How the backward pass is cut: 128-row blocks (upper bound: the sequences are ragged) and query heads per CTA.
-struct BwdPlan { long long blocks; int hpc, sets; long long off_stats, off_dq, off_dk, off_dv, floats; };
+// How the backward pass is cut: 128-row blocks (upper bound: the sequences are ragged) and query heads per dK, dV CTA.
+struct BwdPlan { long long blocks; int hpc, sets; long long off_stats, floats; };
 BwdPlan bwd_plan(int num_seqs, int total_tokens, int max_seqlen, int heads_q, int heads_kv) {
   BwdPlan b;
   b.blocks = ((long long)total_tokens + AB - 1) / AB + num_seqs;
-  // A CTA that takes all query heads of a kv head adds their dK, dV in TMEM and writes bf16; but its loop is that much
-  // longer.  The longest loop may be half of an SM's share of all iterations (sequences taken as equally long, one block at
-  // least), else
-  // fewer heads per CTA: 613 tokens, 32 / 8 heads run with one head (160 CTAs), four sequences of 1024-8192 with all four.
+  // A CTA that takes all query heads of a kv head adds their dK, dV in TMEM; but its loop is that much longer.  The longest loop may be
+  // a third of an SM's share of all work (sequences taken as equally long, one block at least; a round of dK, dV is 1.3 of dQ's),
+  // else fewer heads per CTA, in clusters of at most 8 CTAs: 613 tokens, 32 / 8 heads run with one head, four sequences of 1024-8192
+  // with all four.
   const int group = heads_q / heads_kv;
   const double seqs = num_seqs > 0 ? num_seqs : 1, n = fmax((double)total_tokens / (AB * seqs), 1.0);
-  const double share = seqs * n * (n + 1.0) / 2.0 * heads_q / sm_count_of_current_device();
+  const double share = 2.3 * seqs * n * (n + 1.0) / 2.0 * heads_q / sm_count_of_current_device();
   const int longest = ((max_seqlen < total_tokens ? max_seqlen : total_tokens) + AB - 1) / AB;
   b.hpc = group;
-  while (b.hpc > 1 && (double)b.hpc * longest > 0.5 * share) b.hpc = b.hpc % 2 == 0 ? b.hpc / 2 : 1;
+  for (int h = group - 1; h >= 1 && 1.3 * b.hpc * longest > 0.33 * share; --h)
+    if (group % h == 0 && group / h <= MAX_SETS) b.hpc = h;
   b.sets = heads_q / b.hpc;
   b.off_stats = (b.blocks * 4 + 31) / 32 * 32;                                   // after the schedule
-  b.off_dq = b.off_stats + b.blocks * heads_q * BWD_STATS;
-  b.off_dk = b.off_dq + (long long)total_tokens * heads_q * HD;
-  const long long part = b.hpc == group ? 0 : (long long)total_tokens * b.sets * HD;
-  b.off_dv = b.off_dk + part;
-  b.floats = b.off_dv + part;
+  b.floats = b.off_stats + b.blocks * heads_q * BWD_STATS;
   return b;
 }
 }  // namespace
@@ -1046,22 +1132,20 @@ extern "C" long long mdt_attention_bwd_scratch(int num_seqs, int total_tokens, i
 extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout, const float* lse,
                                  void* dq, void* dk, void* dv, float* scratch, const int* cu_seqlens, int num_seqs, int total_tokens,
                                  int max_seqlen, int heads_q, int heads_kv, int head_dim, float scale, int* status, cudaStream_t s) {
-  // scratch: mdt_attention_bwd_scratch() floats, 128-byte aligned: schedule | row statistics | dq32 | dk32 | dv32
+  // scratch: mdt_attention_bwd_scratch() floats, 128-byte aligned: schedule | row statistics
   if (head_dim != HD || heads_q % heads_kv != 0) return -1;
   if (total_tokens == 0) return 0;
   if (reinterpret_cast<uintptr_t>(scratch) & 127) return -2;
   static thread_local bool bound = false;
   if (!bound) { cudaFree(nullptr); bound = true; }
   const BwdPlan b = bwd_plan(num_seqs, total_tokens, max_seqlen, heads_q, heads_kv);
-  const bool direct = b.off_dk == b.floats;
   AttnBwdParams p;
   memset(&p, 0, sizeof(p));
   int rc = att_map(&p.tmQ, q, total_tokens, heads_q) | att_map(&p.tmK, k, total_tokens, heads_kv) |
            att_map(&p.tmV, v, total_tokens, heads_kv) | att_map(&p.tmdO, dout, total_tokens, heads_q);
   if (rc) return rc;
-  p.sched = reinterpret_cast<const int4*>(scratch); p.stats = scratch + b.off_stats; p.dq = scratch + b.off_dq;
-  p.dk = direct ? nullptr : scratch + b.off_dk; p.dv = direct ? nullptr : scratch + b.off_dv;
-  p.dk_out = (bf16*)dk; p.dv_out = (bf16*)dv;
+  p.sched = reinterpret_cast<const int4*>(scratch); p.stats = scratch + b.off_stats;
+  p.dq = (bf16*)dq; p.dk = (bf16*)dk; p.dv = (bf16*)dv;
   p.heads_q = heads_q; p.heads_kv = heads_kv; p.hpc = b.hpc; p.tokens = total_tokens; p.blocks = (int)b.blocks;
   p.status = status;
   p.scale = scale; p.scale_log2e = scale * 1.4426950408889634f;
@@ -1071,14 +1155,18 @@ extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, co
     configured = true;
   }
   launch_after(attn_bwd_prepare_kernel, dim3((unsigned)b.blocks, heads_q), 256, 0, s, (const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs,
-                                                                            total_tokens, heads_q, reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq, status);
+               total_tokens, heads_q, heads_kv, reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq, p.dk, p.dv, status);
   ++g_att_launches;
-  launch_after(attn_bwd_kernel, (unsigned)(b.blocks * b.sets), BWD_THREADS, BWD_SMEM, s, p);
-  ++g_att_launches;
-  long long extra = 0;                                       // CTAs (times heads_q) that add up partial dK, dV
-  if (!direct) extra = (2LL * total_tokens * heads_kv * (HD / 8) + 256LL * heads_q - 1) / (256LL * heads_q);
-  launch_after(attn_bwd_finalize_kernel, dim3((unsigned)(b.blocks + extra), heads_q), 256, 0, s, p.dq, p.dk, p.dv, (bf16*)dq, (bf16*)dk, (bf16*)dv, cu_seqlens,
-                                                                                      num_seqs, (int)b.blocks, total_tokens, heads_q, heads_kv, b.sets);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(b.blocks * (b.sets + heads_q))); cfg.blockDim = dim3(BWD_THREADS); cfg.dynamicSmemBytes = BWD_SMEM; cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;                                // the sets of a kv head add up their dK, dV
+  attr[1].val.clusterDim.x = b.sets / heads_kv; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = b.sets > heads_kv ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, attn_bwd_kernel, p);
   ++g_att_launches;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -100 - (int)e;

@@ -290,6 +290,12 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t local_smem_addr, uint32
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(cta_rank));
   return r;
 }
+// 16 bytes from the shared memory of a CTA of this cluster
+__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
+  return v;
+}
 // Every thread of every CTA of the cluster.  The .aligned forms want whole warps, so the warp is brought together first:
 // loops that lanes leave at different iterations may stand before a call.
 __device__ __forceinline__ void cluster_sync_all() {

@@ -1018,12 +1018,6 @@ template <int BN> struct SplitShape {
   static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
 };
 
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t cluster_addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr));
-  return v;
-}
-
 template <int BN>
 __device__ __forceinline__ void cluster_product(const GemmParams& p, int index) {
   constexpr int STAGES = SplitShape<BN>::STAGES, STAGE_BYTES = SplitShape<BN>::STAGE;

@@ -879,7 +879,7 @@ def test_attention_node_in_the_graph(ops):
         got = [o.detach()] + list(torch.autograd.grad(o, leaves, do))
         want = want or got
         for a, b in zip(got, want):
-            _close(a, b, 2e-3, layout)                            # (dQ sums in any order)
+            _close(a, b, 2e-3, layout)                            # (the same kernels; one bf16 rounding)
     kf = k.clone().requires_grad_(True)
     (front.attention(q, kf, v, cu, 56) * do).sum().backward()
     _close(kf.grad, want[2], 2e-3, "only k")
@@ -929,6 +929,22 @@ def test_attention_many_short_sequences(ops, lens, heads, kv):
     """Blocks with few rows: their dQ tiles take just those rows, and neighbours must not touch.  Blocks are looked up 32
     sequences at a time: one window less one, one, one more, and windows of empty sequences."""
     test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv)
+
+
+@pytest.mark.parametrize("lens,heads,kv", [([128], 12, 2), ([257], 16, 1), ([129, 2, 640], 16, 1), ([384, 1], 8, 1), ([300], 6, 2),
+                                           ([1], 24, 3), ([513], 22, 2), ([2, 900], 24, 1)])
+def test_attention_backward_clusters_of_head_sets(ops, lens, heads, kv):
+    """The query heads of a kv head over clusters of 2 to 8 CTAs and, where the group has no divisor that leaves at most 8, over one,
+    at whole blocks, one row more and one block; the loops' first turns (one to three blocks), whose operands' places are not yet in
+    rotation.  Bounds as in the test above; every sum has one order, so two runs are the same bit for bit."""
+    test_attention_ragged_blocks_and_head_sets(ops, lens, heads, kv)
+    T = sum(lens)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    q, k, v, do = (torch.randn(T, h, 128, device=DEV, generator=g).to(torch.bfloat16) for h in (heads, kv, kv, heads))
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+    o, lse = ops.ext.attention_fwd(q, k, v, cu, max(lens), 128 ** -0.5)
+    runs = [ops.ext.attention_bwd(q, k, v, o, do, lse, cu, max(lens), 128 ** -0.5, ops.status_tensor(DEV)) for _ in range(2)]
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
 
 
 @pytest.mark.parametrize("scale", [0.3, 0.0, -0.08])
