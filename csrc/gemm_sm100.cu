@@ -28,6 +28,7 @@
 #include <unordered_map>
 #include <string.h>
 #include <mutex>
+#include <type_traits>
 #include <tuple>
 
 #include "api.h"
@@ -1249,11 +1250,12 @@ static int make_map_uncached(CUtensorMap* m, const void* ptr, uint64_t d0, uint6
 static int g_num_sms = 0;
 static long long g_launches = 0;
 
-// Workspace of the split last wave: one fp32 tile per SM plus SPLIT_COUNTERS counters per tile, zero between launches (the
-// warp that finishes a shared tile clears what it read).  One workspace per stream, since launches on different streams may
-// overlap on the GPU; created on the stream's first product that can use it and cleared by that stream itself: a clear on
-// the default stream is not ordered against a non-blocking stream, and one that comes late takes back partial sums and
-// counts, so that a part never sees its last contributor and stays unwritten.  MDT_GEMM_SPLIT=0 switches the split off.
+// Workspace of the split last wave: two fp32 tiles per SM (a tile of the transposed pair kernel has up to 512 x 256 values) plus
+// SPLIT_COUNTERS counters per tile, zero between launches (the warp that finishes a shared tile clears what it read).  One
+// workspace per stream, since launches on different streams may overlap on the GPU; created on the stream's first product that
+// can use it and cleared by that stream itself: a clear on the default stream is not ordered against a non-blocking stream, and
+// one that comes late takes back partial sums and counts, so that a part never sees its last contributor and stays unwritten.
+// MDT_GEMM_SPLIT=0 switches the split off.
 struct SplitWorkspace { float* ws; unsigned* ctr; };
 static std::mutex g_split_mutex;
 static std::map<std::pair<int, cudaStream_t>, SplitWorkspace> g_split_ws;
@@ -1277,7 +1279,7 @@ static bool split_workspace(cudaStream_t stream, SplitWorkspace* out) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
     SplitWorkspace w{nullptr, nullptr};
-    const size_t ws_bytes = (size_t)g_num_sms * BM * 256 * sizeof(float), ctr_bytes = (size_t)g_num_sms * SPLIT_COUNTERS * sizeof(unsigned);
+    const size_t ws_bytes = (size_t)g_num_sms * 2 * BM * 256 * sizeof(float), ctr_bytes = (size_t)g_num_sms * 2 * SPLIT_COUNTERS * sizeof(unsigned);
     if (cudaMalloc(&w.ws, ws_bytes) != cudaSuccess) { cudaGetLastError(); return false; }
     if (cudaMalloc(&w.ctr, ctr_bytes) != cudaSuccess) { cudaGetLastError(); cudaFree(w.ws); return false; }
     if (cudaMemsetAsync(w.ws, 0, ws_bytes, stream) != cudaSuccess || cudaMemsetAsync(w.ctr, 0, ctr_bytes, stream) != cudaSuccess) {

@@ -9,7 +9,8 @@
 // memory: 2 x (32 KB of weights + n x 128 bytes) through 2 SMs' 128 bytes per clock), against 700 that the weights' 32 KB take
 // from HBM, so that up to about 400 rows a group the products run at the rate of the weights.
 //
-// Rows of a group are cut into tiles of equal numbers of 32-row units, at most 8 (256 rows).  Only rows that exist are
+// Rows of a group are cut into tiles of equal numbers of 32-row units, at most 8 (256 rows), or 16 where tp_joint_pays says so: such a
+// tile is two products with one copy of the weights in shared memory, in both accumulators.  Only rows that exist are
 // multiplied where the caller passes their number (group_rows); the padding up to the next 128-row boundary, zero by contract,
 // gives zeros, which are written without being computed.  The tiles of the last, partly filled round are cut along the depth
 // over all pairs as in the 128-row kernel (get_work): 128 tiles of a down projection are 1.73 rounds of 74 pairs.
@@ -25,7 +26,8 @@ constexpr int TP_A_BYTES = BM * BK * 2;
 // products of few rows is the bytes of weights in flight.
 constexpr int TP_RING_BYTES = 6 * (TP_A_BYTES + 128 * BK * 2);
 constexpr int TP_MAX_STAGES = 10;
-struct TPTable { int start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, units, groups, row_tiles; };
+// (groups in the order of the rows of their tiles, most first: see tp_work)
+struct TPTable { int group[TP_GROUPS], start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, units, groups, row_tiles, cap; };
 constexpr int TP_SMEM = TP_RING_BYTES + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES + (int)sizeof(TPTable);
 static_assert(TP_SMEM <= 227 * 1024, "transposed pair kernel: shared memory of a CTA");
 
@@ -47,23 +49,99 @@ struct TPParams {
 struct TPTile { int g, f0, row0, n, end, zero0; };
 struct TPWork { TPTile t; int kb0, kb1, split, contributors; };
 
-__host__ __device__ __forceinline__ int tp_tiles_of_rows(int rows) { return ((rows + TP_UNIT - 1) / TP_UNIT + 7) / 8; }
+__host__ __device__ __forceinline__ int tp_tiles_of_rows(int rows, int cap) { return ((rows + TP_UNIT - 1) / TP_UNIT + cap - 1) / cap; }
+// rows of its widest tile
+__host__ __device__ __forceinline__ int tp_tile_rows(int rows, int cap) {
+  const int units = (rows + TP_UNIT - 1) / TP_UNIT, nt = tp_tiles_of_rows(rows, cap);
+  return nt > 0 ? (units + nt - 1) / nt * TP_UNIT : 0;
+}
+// rows of the first accumulator of a tile of n rows
+__host__ __device__ __forceinline__ int tp_first(int n) { return n > 256 ? (n / TP_UNIT + 1) / 2 * TP_UNIT : n; }
 
-// One thread per group fills the table; a warp scan gives the first tile of each group.
-__device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, int f_tiles, int lane) {
+// Clocks of a k block for a tile of n rows with little else on the chip (measured: n = 128 430, 160 525, 192 556, 256 640), and for one
+// with two accumulators, which copies the weights to shared memory once: what the measurements below ask for.
+__host__ __device__ __forceinline__ float tp_clocks(int n) { return n <= 256 ? 220.f + 1.64f * (float)n : 150.f + 2.1f * (float)n; }
+// Clocks of a pair for all tiles: `row_tiles` of them for each of f_tiles, `step` a k block of one (`longest`: of the longest),
+// `rows` rows each; what the last round takes if it is shared is that of tp_split_pays.
+__host__ __device__ __forceinline__ float tp_clocks_of_all(int row_tiles, int f_tiles, int pairs, int kbt, float step, float longest, float rows, float epilogue, bool may_split) {
+  const int total = row_tiles * f_tiles, rounds = total / pairs, rem = total % pairs;
+  const float tile = (float)kbt * step + epilogue * rows;
+  if (total <= pairs) return (float)kbt * longest + epilogue * rows;
+  if (rem == 0) return (float)rounds * tile;
+  const float shared = (float)kbt * step * (float)rem / (float)pairs + 8000.f + 90.f * rows;
+  return (float)rounds * tile + (may_split && shared < tile ? shared : tile);
+}
+// Whether tiles of up to 512 rows are taken (sums over the groups: tiles, k block clocks; longest, of both forms).  Such a tile reads
+// its weights once for twice the rows, but takes both accumulators, so that nothing hides its epilogue (8 clocks a row), and there are
+// fewer of them to go round.  us in turn, up to 256 / up to 512 rows, 8 experts of 4096 x 14336: down 1000 tokens 261 / 245, 2000 423 /
+// 417, 4000 757 / 728, 9200 1803 / 1795; dx (two matrices) 513 / 456, 802 / 822, 1478 / 1394, 3780 / 3691; 1500 tokens, which the model
+// misses, 347 / 355 and 611 / 624; 9200 x 4096 of depth 1024 146 / 153, 4096 433 / 419; 2 experts of 500 tokens, half of whose tiles are
+// too few, 97 / 165.  Not for more than one result a product: gate and up of 2000 tokens 892 / 937, with their inputs kept of 9200
+// 3320 / 3856, SwiGLU backward 1896 / 2704.
+struct TPForm { int row_tiles; float step, longest; };
+__host__ __device__ __forceinline__ bool tp_joint_pays(const TPForm& one, const TPForm& two, int units, int f_tiles, int pairs, int kbt, bool may_split) {
+  if (two.row_tiles == one.row_tiles || two.row_tiles == 0) return false;
+  const float rows = 32.f * (float)units;
+  const float a = tp_clocks_of_all(one.row_tiles, f_tiles, pairs, kbt, one.step / (float)one.row_tiles, one.longest, rows / (float)one.row_tiles, 0.f, may_split);
+  const float b = tp_clocks_of_all(two.row_tiles, f_tiles, pairs, kbt, two.step / (float)two.row_tiles, two.longest, rows / (float)two.row_tiles, 8.f, may_split);
+  return b < 0.98f * a;
+}
+__host__ __device__ __forceinline__ void tp_add_group(TPForm& f, int rows, int cap) {
+  const int nt = tp_tiles_of_rows(rows, cap);
+  if (nt == 0) return;
+  const float most = tp_clocks(tp_tile_rows(rows, cap));
+  f.row_tiles += nt;
+  f.step += (float)nt * most;
+  f.longest = fmaxf(f.longest, most);
+}
+
+__device__ __forceinline__ int tp_rows_of(const TPParams& p, int g, int& start, int& end) {
+  start = p.mode == 1 ? p.offsets[g] : 0;
+  end = p.mode == 1 ? p.offsets[g + 1] : p.M;
+  const int rows = end - start;
+  return p.group_rows != nullptr && p.group_rows[g] < rows ? p.group_rows[g] : rows;
+}
+// One thread per group fills the table, after the groups' places in it are counted; a warp scan gives the first tile of each.
+template <bool JOINT>
+__device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, int f_tiles, int kbt, int pairs, int lane) {
+  int cap = 8, start, end;
+  if (JOINT) {
+    TPForm one{0, 0.f, 0.f}, two{0, 0.f, 0.f};
+    int units = 0;
+    for (int g = lane; g < p.G; g += 32) {
+      const int rows = tp_rows_of(p, g, start, end);
+      units += (rows + TP_UNIT - 1) / TP_UNIT;
+      tp_add_group(one, rows, 8);
+      tp_add_group(two, rows, 16);
+    }
+    auto over_lanes = [&](TPForm& f) {
+      f.row_tiles = __reduce_add_sync(0xffffffffu, f.row_tiles);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) { f.step += __shfl_xor_sync(0xffffffffu, f.step, o); f.longest = fmaxf(f.longest, __shfl_xor_sync(0xffffffffu, f.longest, o)); }
+    };
+    over_lanes(one); over_lanes(two);
+    units = __reduce_add_sync(0xffffffffu, units);
+    if (tp_joint_pays(one, two, units, f_tiles, pairs, kbt, p.sk_ws != nullptr)) cap = 16;
+  }
+  for (int g = lane; g < p.G; g += 32) tb->tile0[g] = tp_tile_rows(tp_rows_of(p, g, start, end), cap);
+  __syncwarp();
+  for (int g = lane; g < p.G; g += 32) {
+    const int rows = tp_rows_of(p, g, start, end), mine = tb->tile0[g];
+    int place = 0;
+    for (int o = 0; o < p.G; ++o) place += tb->tile0[o] > mine || (tb->tile0[o] == mine && o < g) ? 1 : 0;
+    tb->group[place] = g; tb->start[place] = start; tb->rows[place] = rows; tb->end[place] = end;
+  }
+  __syncwarp();
   int carry = 0, widest = 0, units_all = 0, groups = 0;
   for (int g0 = 0; g0 < p.G; g0 += 32) {
     const int g = g0 + lane;
     int tiles = 0;
     if (g < p.G) {
-      const int start = p.mode == 1 ? p.offsets[g] : 0, end = p.mode == 1 ? p.offsets[g + 1] : p.M;
-      int rows = end - start;
-      if (p.group_rows != nullptr && p.group_rows[g] < rows) rows = p.group_rows[g];
-      tb->start[g] = start; tb->rows[g] = rows; tb->end[g] = end;
-      tiles = tp_tiles_of_rows(rows) * f_tiles;
-      const int units = (rows + TP_UNIT - 1) / TP_UNIT, nt = (units + 7) / 8;
-      if (nt > 0) { widest = max(widest, (units + nt - 1) / nt * TP_UNIT); ++groups; }
-      units_all += units;
+      const int rows = tb->rows[g];
+      tiles = tp_tiles_of_rows(rows, cap) * f_tiles;
+      widest = max(widest, tp_tile_rows(rows, cap));
+      groups += tiles > 0 ? 1 : 0;
+      units_all += (rows + TP_UNIT - 1) / TP_UNIT;
     }
     int incl = tiles;
 #pragma unroll
@@ -74,17 +152,17 @@ __device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, in
   widest = __reduce_max_sync(0xffffffffu, widest);
   units_all = __reduce_add_sync(0xffffffffu, units_all);
   groups = __reduce_add_sync(0xffffffffu, groups);
-  if (lane == 0) { tb->tile0[p.G] = carry; tb->widest = widest; tb->units = units_all; tb->groups = groups; tb->row_tiles = carry / f_tiles; }
+  if (lane == 0) { tb->tile0[p.G] = carry; tb->widest = widest; tb->units = units_all; tb->groups = groups; tb->row_tiles = carry / f_tiles; tb->cap = cap; }
 }
 
 __host__ __device__ __forceinline__ void tp_tile(const TPTable* tb, int G, int f_tiles, int f_width, int t, TPTile& o) {
   int g = 0;
   while (g + 1 < G && t >= tb->tile0[g + 1]) ++g;
-  const int units = (tb->rows[g] + TP_UNIT - 1) / TP_UNIT, nt = (units + 7) / 8;
+  const int units = (tb->rows[g] + TP_UNIT - 1) / TP_UNIT, nt = tp_tiles_of_rows(tb->rows[g], tb->cap);
   int n, f;
   panel_order(t - tb->tile0[g], nt, f_tiles, 8, n, f);      // rows fastest: the tiles that share weights run together
   const int base = units / nt, extra = units % nt;
-  o.g = g;
+  o.g = tb->group[g];
   o.f0 = f * f_width;
   o.row0 = tb->start[g] + (n * base + (n < extra ? n : extra)) * TP_UNIT;
   o.n = (base + (n < extra ? 1 : 0)) * TP_UNIT;
@@ -100,21 +178,24 @@ __host__ __device__ __forceinline__ void tp_tile(const TPTable* tb, int G, int f
 __host__ __device__ __forceinline__ bool tp_split_pays(const TPTable* tb, int f_tiles, int kbt, int rem, int pairs) {
   const int row_tiles = tb->row_tiles;
   const float rows = 32.f * (float)tb->units / (float)row_tiles, shared = (float)row_tiles / (float)tb->groups;
-  const float step = 1.25f * (256.f + rows), memory = 704.f / shared, part = (float)rem / (float)pairs;
+  const float step = rows > 256.f ? tp_clocks((int)rows) : 1.25f * (256.f + rows), memory = 704.f / shared, part = (float)rem / (float)pairs;
   return (float)kbt * fmaxf(step, memory * part) > (float)kbt * fmaxf(step, memory) * part + 8000.f + 90.f * rows;
 }
 
-// it = 0, 1, ...: the work of pair `pair` of `pairs`.  The tiles of a last round that leaves more than an eighth of the pairs
+// it = 0, 1, ...: the work of pair `pair` of `pairs`.  The tiles come by their rows, most first, and every second round goes through
+// the pairs backwards, so that all have about the same to do (us, groups in their own order, each round forwards /
+// so: SwiGLU backward of 600 tokens 226 / 214, down 1000 tokens 271 / 261, dx 527 / 513).  The tiles of a last round that leaves more than an eighth of the pairs
 // idle are cut into one contiguous piece of k blocks per pair (see get_work), no piece shorter than 4 blocks.
 __host__ __device__ __forceinline__ bool tp_work(const TPTable* tb, int G, int f_tiles, int f_width, int kbt, bool may_split, int pair, int pairs, int it, TPWork& w) {
   const int total = tb->tile0[G];
   int whole = total;
   const int rem = total % pairs;
   if (may_split && total > pairs && rem != 0 && kbt >= 8 && tp_split_pays(tb, f_tiles, kbt, rem, pairs)) whole = total - rem;
-  const int n_whole = whole > pair ? (whole - pair + pairs - 1) / pairs : 0;
+  const int n_whole = whole / pairs;                     // (of the pieces of a shared round: what comes before)
   w.split = -1; w.contributors = 1;
-  if (it < n_whole) {
-    tp_tile(tb, G, f_tiles, f_width, pair + it * pairs, w.t);
+  const int t = it * pairs + (it & 1 ? pairs - 1 - pair : pair);
+  if (t < whole) {
+    tp_tile(tb, G, f_tiles, f_width, t, w.t);
     w.kb0 = 0; w.kb1 = kbt;
     return true;
   }
@@ -271,6 +352,7 @@ __device__ __forceinline__ bool tp_epilogue(const TPParams& p, uint8_t* stage, c
 template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gemm_sm100_tpair_kernel(const __grid_constant__ TPParams p) {
   constexpr int F_WIDTH = KIND == TP_DUAL ? 128 : 256;      // output features of a tile
+  constexpr bool JOINT = KIND == TP_PLAIN;                  // tiles of two accumulators at all (tp_joint_pays)
   constexpr uint32_t TMEM_COLS = 512;
 
   extern __shared__ uint8_t smem_raw[];
@@ -298,7 +380,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     fence_barrier_init();
   }
   if (warp == 1) { tmem_alloc_pair(tmem_slot, TMEM_COLS); tmem_relinquish_pair(); }
-  if (warp == 2) { wait_for_predecessor(); tp_fill_table(p, tb, f_tiles, lane); }
+  if (warp == 2) { wait_for_predecessor(); tp_fill_table<JOINT>(p, tb, f_tiles, kbt, num_pairs, lane); }
   tc_fence_before();
   cluster_sync_all();
   tc_fence_after();
@@ -322,42 +404,51 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     bool ok = true;
     for (int wi = 0; ok && next(wi); ++wi) {
       const TPTile& t = w.t;
-      const int rows = t.n / 2, row0 = t.row0 + rank * rows;       // this CTA's rows of the N operand
       const int f0 = t.f0 + rank * (F_WIDTH / 2);
-      const uint32_t bytes = 2 * (TP_A_BYTES + rows * (BK * 2));
-      for (int kb = w.kb0; kb < w.kb1; ++kb) {
-        if (!wait_parity_warp(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
-        uint8_t* sW = smem + s * stage_bytes;
-        uint8_t* sX = sW + TP_A_BYTES;
-        // (only the leader arrives, see the pair kernel)
-        const uint32_t bar = mapa_shared(smem_u32(&full_bar[s]), 0);
-        const bool second = kb >= num_kb;
-        const int kk = (second ? kb - num_kb : kb) * BK;
-        const CUtensorMap* mW = second ? &p.tmW_l : &p.tmW;
-        const CUtensorMap* mW2 = second ? &p.tmW2_l : &p.tmW2;
-        const int w_mn = second ? p.w_mn_l : p.w_mn;
-        if (elect_one()) {
-          if (rank == 0) mbar_expect_tx(&full_bar[s], bytes);
-          if (KIND == TP_DUAL) {
+      const uint32_t bytes = 2 * (TP_A_BYTES + t.n / 2 * (BK * 2));
+      // (a loop for each of one and two accumulators, here and in the issuer: with the choice inside, tiles of 256 rows took 25 % longer)
+      auto load = [&](auto two) {
+        const int n0 = decltype(two)::value ? tp_first(t.n) : t.n;
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+          if (!wait_parity_warp(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
+          uint8_t* sW = smem + s * stage_bytes;
+          uint8_t* sX = sW + TP_A_BYTES;
+          // (only the leader arrives, see the pair kernel)
+          const uint32_t bar = mapa_shared(smem_u32(&full_bar[s]), 0);
+          const bool second = kb >= num_kb;
+          const int kk = (second ? kb - num_kb : kb) * BK;
+          const CUtensorMap* mW = second ? &p.tmW_l : &p.tmW;
+          const CUtensorMap* mW2 = second ? &p.tmW2_l : &p.tmW2;
+          const int w_mn = second ? p.w_mn_l : p.w_mn;
+          if (elect_one()) {
+            if (rank == 0) mbar_expect_tx(&full_bar[s], bytes);
+            if (KIND == TP_DUAL) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              tma_load_3d_pair(sW + j * 4096, mW, bar, kk, f0 + 16 * j, t.g);
-              tma_load_3d_pair(sW + j * 4096 + 2048, mW2, bar, kk, f0 + 16 * j, t.g);
+              for (int j = 0; j < 4; ++j) {
+                tma_load_3d_pair(sW + j * 4096, mW, bar, kk, f0 + 16 * j, t.g);
+                tma_load_3d_pair(sW + j * 4096 + 2048, mW2, bar, kk, f0 + 16 * j, t.g);
+              }
+            } else if (w_mn == 0) {
+              tma_load_3d_pair(sW, mW, bar, kk, f0, t.g);
+            } else {
+              tma_load_3d_pair(sW, mW, bar, f0, kk, t.g);
+              tma_load_3d_pair(sW + 8192, mW, bar, f0 + 64, kk, t.g);
             }
-          } else if (w_mn == 0) {
-            tma_load_3d_pair(sW, mW, bar, kk, f0, t.g);
-          } else {
-            tma_load_3d_pair(sW, mW, bar, f0, kk, t.g);
-            tma_load_3d_pair(sW + 8192, mW, bar, f0 + 64, kk, t.g);
-          }
-          const CUtensorMap* mX = second ? p.tmX_l : p.tmX;
-          int done = 0;
+            const CUtensorMap* mX = second ? p.tmX_l : p.tmX;
+            auto rows = [&](uint8_t* to, int n, int first) {      // this CTA's half of n rows
+              int done = 0;
 #pragma unroll
-          for (int b = 3; b >= 0; --b)
-            if (rows & (16 << b)) { tma_load_2d_pair(sX + done * (BK * 2), mX + b, bar, kk, row0 + done); done += 16 << b; }
+              for (int b = 3; b >= 0; --b)
+                if ((n / 2) & (16 << b)) { tma_load_2d_pair(to + done * (BK * 2), mX + b, bar, kk, first + rank * (n / 2) + done); done += 16 << b; }
+            };
+            rows(sX, n0, t.row0);
+            if (decltype(two)::value) rows(sX + n0 / 2 * (BK * 2), t.n - n0, t.row0 + n0);
+          }
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
-        if (++s == stages) { s = 0; ph ^= 1; }
-      }
+      };
+      if (!JOINT || t.n <= 256) load(std::false_type());
+      else load(std::integral_constant<bool, JOINT>());
     }
     if (!ok) {  // give this CTA's copies already in flight a bounded time to land before it leaves
       const uint64_t t0 = global_timer_ns();
@@ -369,30 +460,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     uint32_t ph = 0, acc_it = 0;
     bool ok = true;
     for (int wi = 0; ok && next(wi); ++wi) {
-      const int buf = acc_it & 1;
-      const uint32_t aph = (acc_it >> 1) & 1;
-      if (!wait_parity_warp(&tempty_bar[buf], aph ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); break; }
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + buf * 256;
-      for (int kb = w.kb0; kb < w.kb1; ++kb) {
-        if (!wait_parity_warp(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; break; }
+      auto multiply = [&](auto two) {
+        const int n0 = decltype(two)::value ? tp_first(w.t.n) : w.t.n, n1 = w.t.n - n0, buf = acc_it & 1;
+        if (!wait_parity_warp(&tempty_bar[buf], ((acc_it >> 1) & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); ok = false; return; }
+        if (decltype(two)::value && !wait_parity_warp(&tempty_bar[buf ^ 1], (((acc_it + 1) >> 1) & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); ok = false; return; }
         tc_fence_after();
-        const int w_mn = kb >= num_kb ? p.w_mn_l : p.w_mn;
-        const uint32_t idesc = make_idesc_bf16(2 * BM, w.t.n, w_mn, 0);
-        const uint32_t sW = smem_u32(smem + s * stage_bytes);
-        const uint64_t dw = operand_desc(sW, w_mn), dx = operand_desc(sW + TP_A_BYTES, 0);
-        const uint32_t kw = operand_kstep(w_mn), kx = operand_kstep(0);
-        if (elect_one()) {
+        const uint32_t d_tmem = tmem_base + buf * 256, d_tmem1 = tmem_base + (buf ^ 1) * 256;
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+          if (!wait_parity_warp(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; return; }
+          tc_fence_after();
+          const int w_mn = kb >= num_kb ? p.w_mn_l : p.w_mn;
+          const uint32_t idesc = make_idesc_bf16(2 * BM, n0, w_mn, 0);
+          const uint32_t sW = smem_u32(smem + s * stage_bytes);
+          const uint64_t dw = operand_desc(sW, w_mn), dx = operand_desc(sW + TP_A_BYTES, 0);
+          const uint32_t kw = operand_kstep(w_mn), kx = operand_kstep(0);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_bf16_pair(d_tmem, dw + k * kw, dx + k * kx, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
-          umma_commit_pair(&empty_bar[s], 3);   // frees the stage in both CTAs
+            for (int k = 0; k < BK / 16; ++k)
+              umma_bf16_pair(d_tmem, dw + k * kw, dx + k * kx, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+            if (decltype(two)::value) {
+              const uint32_t idesc1 = make_idesc_bf16(2 * BM, n1, w_mn, 0);
+              const uint64_t dx1 = operand_desc(sW + TP_A_BYTES + n0 / 2 * (BK * 2), 0);
+#pragma unroll
+              for (int k = 0; k < BK / 16; ++k)
+                umma_bf16_pair(d_tmem1, dw + k * kw, dx1 + k * kx, idesc1, (kb > w.kb0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit_pair(&empty_bar[s], 3);   // frees the stage in both CTAs
+          }
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
-        if (++s == stages) { s = 0; ph ^= 1; }
-      }
-      if (!ok) break;
-      if (elect_one()) umma_commit_pair(&tfull_bar[buf], 3);   // accumulators complete, in both CTAs
-      ++acc_it;
+        if (elect_one()) {                          // accumulators complete, in both CTAs
+          umma_commit_pair(&tfull_bar[buf], 3);
+          if (decltype(two)::value) umma_commit_pair(&tfull_bar[buf ^ 1], 3);
+        }
+        acc_it += decltype(two)::value ? 2 : 1;
+      };
+      if (!JOINT || w.t.n <= 256) multiply(std::false_type());
+      else multiply(std::integral_constant<bool, JOINT>());
     }
   } else if (warp >= 2) {
     // ------------------------------------------------------------------ epilogue (both CTAs, own 128 operand rows)
@@ -400,13 +504,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     uint8_t* stage = epi_stage + (warp - 2) * EPI_STAGE_BYTES;
     const float alpha = p.alpha_dev != nullptr ? p.alpha * *p.alpha_dev : p.alpha;
     uint32_t acc_it = 0;
-    for (int wi = 0; next(wi); ++wi) {
-      const TPTile& t = w.t;
+    bool ok = true;
+    for (int wi = 0, sub = 0; ok && (sub > 0 || next(wi)); sub > 0 ? 0 : ++wi) {
+      // (a tile of more than 256 rows: its two accumulators one after the other)
+      TPTile t = w.t;
+      const int mine = sub;
+      if (JOINT) {
+        const int n0 = tp_first(t.n);
+        sub = mine == 0 && t.n > n0 ? 1 : 0;
+        t.row0 += mine * n0;
+        t.n = mine == 0 ? n0 : t.n - n0;
+      }
       const int col = t.f0 + rank * (F_WIDTH / 2) + q * (F_WIDTH / 8);        // this warp's first output feature
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
       const uint32_t tacc = tmem_base + buf * 256 + ((uint32_t)(q * 32) << 16);
-      if (w.kb0 == 0) tp_clear<KIND>(p, t.zero0, t.end, col, half, lane);     // under the wait for the accumulator
+      if (w.kb0 == 0 && mine == 0) tp_clear<KIND>(p, t.zero0, t.end, col, half, lane);     // under the wait for the accumulator
       auto ready = [&]() {
         if (!wait_parity_warp(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
         tc_fence_after();
@@ -424,15 +537,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
         ++acc_it;
       };
       if (w.split < 0) {
-        if (!tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, ready, from_tmem)) break;
-        release();
+        ok = tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, ready, from_tmem);
+        if (ok) release();
         continue;
       }
       // A piece of a shared tile: partial sums into the fp32 workspace, whole 512-byte lines per reduction; the warp that
       // comes last at its part of the tile reads them back, clears them and finishes the part.
-      const int part = (w.split * 2 + rank) * EPI_WARPS + half * 4 + q;
+      const int part = ((JOINT ? w.split * (tb->cap / 8) + mine : w.split) * 2 + rank) * EPI_WARPS + half * 4 + q;
       float4* ws = reinterpret_cast<float4*>(p.sk_ws) + (long long)part * (4 * 8 * 32) + lane;
-      if (!ready()) break;
+      ok = ready();
+      if (!ok) break;
 #pragma unroll 1
       for (int c = half; c < t.n / TP_UNIT; c += 2) {
         uint32_t lo[16], hi[16];

@@ -3,6 +3,7 @@
 // inside one row group, and report the right group.  Built and run by tests/test_tile_enumeration.py.
 #include <stdio.h>
 #include <stdlib.h>
+#include <algorithm>
 #include <vector>
 
 #include "../../csrc/gemm_sm100.cu"
@@ -96,18 +97,22 @@ static int check_work(const GemmParams& p, int num_ctas, const std::vector<int>&
 
 // The transposed pair kernel (tp_work): every (32-row unit, feature tile, k block) of the rows that exist exactly once; tiles inside
 // their group; the padding of a group cleared by exactly one whole column of tiles; shared tiles as above, one per pair at most.
-static int check_transposed(const std::vector<int>& start, const std::vector<int>& rows, const std::vector<int>& end, int N, int f_width, int kbt, int pairs, bool split) {
+static int check_transposed(const std::vector<int>& start, const std::vector<int>& rows, const std::vector<int>& end, int N, int f_width, int kbt, int pairs, bool split, int cap) {
   TPTable tb;
+  tb.cap = cap;
   const int G = (int)rows.size(), f_tiles = (N + f_width - 1) / f_width;
   int tiles = 0;
   tb.widest = tb.units = tb.groups = 0;
-  for (int g = 0; g < G; ++g) {
-    const int units = (rows[g] + TP_UNIT - 1) / TP_UNIT, nt = (units + 7) / 8;
-    tb.start[g] = start[g]; tb.rows[g] = rows[g]; tb.end[g] = end[g]; tb.tile0[g] = tiles;
-    if (nt != tp_tiles_of_rows(rows[g])) return 1;
+  std::vector<int> order(G);
+  for (int g = 0; g < G; ++g) order[g] = g;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return tp_tile_rows(rows[a], cap) > tp_tile_rows(rows[b], cap); });
+  for (int i = 0; i < G; ++i) {
+    const int g = order[i], units = (rows[g] + TP_UNIT - 1) / TP_UNIT, nt = (units + cap - 1) / cap;
+    tb.group[i] = g; tb.start[i] = start[g]; tb.rows[i] = rows[g]; tb.end[i] = end[g]; tb.tile0[i] = tiles;
+    if (nt != tp_tiles_of_rows(rows[g], cap)) return 1;
     tiles += nt * f_tiles;
     tb.units += units;
-    if (nt > 0) { ++tb.groups; const int w = (units + nt - 1) / nt * TP_UNIT; if (w > tb.widest) tb.widest = w; }
+    if (nt > 0) { ++tb.groups; const int w = (units + nt - 1) / nt * TP_UNIT; if (w > tb.widest) tb.widest = w; if (w != tp_tile_rows(rows[g], cap)) return 1; }
   }
   tb.tile0[G] = tiles;
   tb.row_tiles = tiles / f_tiles;
@@ -121,7 +126,8 @@ static int check_transposed(const std::vector<int>& start, const std::vector<int
       if (!tp_work(&tb, G, f_tiles, f_width, kbt, split, p, pairs, it, w)) break;
       if (it > tiles + 4) { printf("work list does not end\n"); return 1; }
       const TPTile& t = w.t;
-      if (t.n < TP_UNIT || t.n > 256 || t.n % TP_UNIT || t.n > tb.widest || t.f0 % f_width || t.f0 >= N || t.g >= G || t.row0 < start[t.g] ||
+      const int n0 = tp_first(t.n);        // first accumulator; the rest is the second
+      if (t.n < TP_UNIT || t.n > 32 * cap || t.n % TP_UNIT || n0 > 256 || n0 % TP_UNIT || t.n - n0 > 256 || (t.n > 256) != (t.n > n0) || t.n > tb.widest || t.f0 % f_width || t.f0 >= N || t.g >= G || t.row0 < start[t.g] ||
           (t.row0 - start[t.g]) % TP_UNIT || t.row0 - start[t.g] >= rows[t.g] || t.end != end[t.g] || w.kb0 < 0 || w.kb1 > kbt || w.kb0 >= w.kb1) { ++bad; continue; }
       for (int u = 0; u < t.n / TP_UNIT; ++u)
         for (int kb = w.kb0; kb < w.kb1; ++kb) seen[((size_t)(t.row0 / TP_UNIT + u) * f_tiles + t.f0 / f_width) * kbt + kb] += 1;
@@ -152,8 +158,27 @@ static int check_transposed(const std::vector<int>& start, const std::vector<int
   return bad;
 }
 
+// The choice of tiles of up to 512 rows: for deep products that keep every pair busy; not where their number is too small.
+static int check_joint() {
+  auto pays = [](std::vector<int> rows, int f_tiles, int kbt) {
+    TPForm one{0, 0.f, 0.f}, two{0, 0.f, 0.f};
+    int units = 0;
+    for (int r : rows) { units += (r + TP_UNIT - 1) / TP_UNIT; tp_add_group(one, r, 8); tp_add_group(two, r, 16); }
+    return tp_joint_pays(one, two, units, f_tiles, 74, kbt, true);
+  };
+  int bad = 0;
+  bad += !pays({211, 281, 92, 321, 302, 269, 245, 279}, 16, 224);
+  bad += !pays({1901, 2461, 870, 3124, 2866, 2298, 2253, 2627}, 16, 448);
+  bad += !pays({300, 300, 300, 300, 300, 300, 300, 300, 300}, 16, 64);
+  bad += pays({500, 500}, 16, 224);
+  bad += pays({256, 200, 31, 0}, 16, 224);
+  bad += pays({0, 0}, 16, 224);
+  bad += pays({1901, 2461, 870, 3124, 2866, 2298, 2253, 2627}, 16, 16);
+  return bad;
+}
+
 int main() {
-  int failures = 0, cases = 0;
+  int failures = check_joint(), cases = 7;
   for (int it = 0; it < 400; ++it) {
     std::vector<int> start, rows, end;
     const int G = it % 5 == 0 ? 1 : 1 + rnd(12);
@@ -166,7 +191,7 @@ int main() {
     }
     const int N = 8 * (17 + rnd(500)), kbt = 1 + rnd(40), ps[3] = {74, 66, 5};
     for (int c = 0; c < 3; ++c) {
-      const int b1 = check_transposed(start, rows, end, N, 256, kbt, ps[c], it % 3 != 0), b2 = check_transposed(start, rows, end, N, 128, kbt, ps[c], it % 3 != 0);
+      const int b1 = check_transposed(start, rows, end, N, 256, kbt, ps[c], it % 3 != 0, it % 2 ? 8 : 16), b2 = check_transposed(start, rows, end, N, 128, kbt, ps[c], it % 3 != 0, it % 2 ? 8 : 16);
       ++cases;
       if (b1 || b2) { ++failures; printf("transposed: G %d N %d kbt %d pairs %d: %d / %d errors\n", G, N, kbt, ps[c], b1, b2); }
     }

@@ -329,6 +329,35 @@ def test_transposed_pair_kernel(ops, counts, H, F):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("counts,depth", [([300] * 9, 4096), ([257, 290, 64, 512, 301, 480, 33, 320, 350], 4100),
+                                          ([211, 281, 92, 321, 302, 269, 245, 279], 14336)])
+def test_transposed_pair_kernel_with_two_accumulators(ops, counts, depth):
+    """Depths and numbers of tiles at which tiles of more than 256 rows are taken (tests/host/tile_enumeration.cu has the choice):
+    both accumulators equal and not, beside tiles of one, with and without a last round that is shared, K-major and MN-major weights
+    and two depth segments.  fp32 reference, 2e-2 as above; padding becomes zeros."""
+    torch.manual_seed(depth)
+    E, N, r = len(counts), 4096, 16
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(sum(counts))].to(DEV).int()
+    plan = ops.make_plan(ids[:, None], E)
+    R, used, offs = plan.src_slot.numel(), int(plan.padded_offsets[-1]), plan.padded_offsets.tolist()
+    real = plan.src_slot[:used] >= 0
+    rows = lambda n: torch.where((plan.src_slot >= 0)[:, None], _rand(R, n), 0.0).to(torch.bfloat16)
+    depth = depth // 8 * 8
+    x, t, a = rows(depth), rows(2 * r), _rand(E, 2 * r, N, scale=0.1)
+    prev = ops.ext.gemm_set_pair_policy(6)
+    try:
+        for mn in (True, False):
+            w = _rand(E, depth, N, scale=0.1) if mn else _rand(E, N, depth, scale=0.1)
+            y = torch.full((R, N), 7.0, dtype=torch.bfloat16, device=DEV)
+            ops._g(1, x, False, w, mn, y, N, depth, plan, A_l=t, B_l=a, b_mn_l=True, K_l=2 * r)
+            want = torch.cat([x[s:e].float() @ (w[g] if mn else w[g].t()).float() + t[s:e].float() @ a[g].float() for g, (s, e) in enumerate(zip(offs[:-1], offs[1:]))])
+            _close(y[:used][real], want[real], name=f"mn {mn}")
+            assert bool((y[:used][~real] == 0).all()) and bool((y[used:] == 7.0).all())
+    finally:
+        ops.ext.gemm_set_pair_policy(prev)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("counts", [[1, 0, 5], [64, 65, 127, 128], [300, 0, 1], [700], [1600, 900]])
 @pytest.mark.parametrize("M,N", [(136, 136), (264, 1032), (1024, 520), (2312, 264)])
 def test_weight_gradient_kernel(ops, counts, M, N):
