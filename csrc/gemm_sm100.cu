@@ -1400,8 +1400,19 @@ static cudaError_t launch_wgrad(const WgParams& p, cudaStream_t stream) {
 //   dx, two matrices (MN)      275 / 289    360 / 322    545 / 505    920 / 785    3800 / 3950
 // MN-major weights of up to about 96 rows a group stay: 128 x 256 tiles ask for 512 adjacent bytes at a time, one CTA per tile,
 // and at one row block a group nothing is gained by exact rows.
+// Dense products of more than 128 rows (those that the cluster kernel leaves): where 256-row tiles of tokens would hold an eighth more
+// rows than there are in 32-row units, if the tiles give five pairs of eight something to do and, past two rounds, the last round
+// wastes no more than a fifth.  us, pair or 128-row kernel / transposed, rows x features x depth: 200 x 32000 x 4096 60 / 60, 300 123 / 71,
+// 576 141 / 130, 800 168 / 161, 1300 259 / 249; 576 x 4096 x 4096 34 / 32, x 32000 170 / 155, 1300 284 / 249; 1300 x 4096 x 4096 53 / 50.
+// Left: 512 x 4096 x 4096 28 / 34 and 1024 35 / 36 (whole tiles), 300 27 / 30 (32 tiles), 640 x 14336 x 4096 70 / 73 (2.3 rounds).
+static bool transposed_preferred_dense(const MdtGemmDesc* d) {
+  if (d->dual || d->swiglu_g != nullptr || d->M <= BM) return false;
+  const long long pairs = g_num_sms / 2, exact = (d->M + 31) / 32 * 32ll, whole = (d->M + 255) / 256 * 256ll;
+  const long long tiles = (whole / 256) * ((d->N + 255) / 256), rounds = (tiles + pairs - 1) / pairs;
+  return 8 * whole >= 9 * exact && 8 * tiles >= 5 * pairs && (tiles <= 2 * pairs || 4 * rounds * pairs <= 5 * tiles);
+}
 static bool transposed_preferred(const MdtGemmDesc* d, long long thread_rows_hint) {
-  if (d->mode != 1) return false;
+  if (d->mode != 1) return d->mode == 0 && transposed_preferred_dense(d);
   const int G = d->G < 1 ? 1 : d->G;
   long long rows = d->capacity_rows - 127ll * G;
   if (thread_rows_hint > 0 && thread_rows_hint < rows) rows = thread_rows_hint;

@@ -329,6 +329,21 @@ def test_transposed_pair_kernel(ops, counts, H, F):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("M,N", [(129, 12000), (144, 32008), (300, 32000), (576, 4096), (577, 4100), (1300, 4096)])
+@pytest.mark.parametrize("K", [264, 4096])
+def test_dense_products_of_odd_row_counts(ops, M, N, K):
+    """Row counts at which dense products leave 256-row tiles of tokens: both layouts of the weights, with and without an adapter
+    segment, against fp32 (one bf16 rounding: 2e-2 as for the other products)."""
+    torch.manual_seed(M)
+    N = N // 8 * 8
+    x, t = _rand(M, K), _rand(M, 16)
+    w, wt, b = _rand(N, K, scale=0.1), _rand(K, N, scale=0.1), _rand(N, 16, scale=0.1)
+    _close(ops.mm_nt(x, w), x.float() @ w.float().t(), name="nt")
+    _close(ops.mm_nn(x, wt), x.float() @ wt.float(), name="nn")
+    _close(ops.mm_nt(x, w, lora=(t, b)), x.float() @ w.float().t() + t.float() @ b.float().t(), name="nt, adapter")
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("counts,depth", [([300] * 9, 4096), ([257, 290, 64, 512, 301, 480, 33, 320, 350], 4100),
                                           ([211, 281, 92, 321, 302, 269, 245, 279], 14336)])
 def test_transposed_pair_kernel_with_two_accumulators(ops, counts, depth):
