@@ -1392,7 +1392,8 @@ static cudaError_t launch_wgrad(const WgParams& p, cudaStream_t stream) {
 }
 
 // Which row-grouped products it takes under the default policy (those that the cluster kernel would take stay there).
-// Measured in turn, microseconds, 128-row or pair kernel / transposed, 8 experts of 4096 x 14336:
+// Measured in turn, microseconds, 128-row or pair kernel / transposed with tiles of up to 256 rows (tp_joint_pays has the larger ones),
+// 8 experts of 4096 x 14336:
 //   tokens                     77           576          1000         2000         9200
 //   gate and up (K-major)      333 / 301    395 / 342    540 / 466    800 / 735    3130 / 3110
 //   dy W2^T, SwiGLU (K-major)  208 / 175    253 / 218    330 / 300    530 / 490    1900 / 1860
