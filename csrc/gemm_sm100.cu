@@ -1250,12 +1250,11 @@ static int make_map_uncached(CUtensorMap* m, const void* ptr, uint64_t d0, uint6
 static int g_num_sms = 0;
 static long long g_launches = 0;
 
-// Workspace of the split last wave: two fp32 tiles per SM (a tile of the transposed pair kernel has up to 512 x 256 values) plus
-// SPLIT_COUNTERS counters per tile, zero between launches (the warp that finishes a shared tile clears what it read).  One
-// workspace per stream, since launches on different streams may overlap on the GPU; created on the stream's first product that
-// can use it and cleared by that stream itself: a clear on the default stream is not ordered against a non-blocking stream, and
-// one that comes late takes back partial sums and counts, so that a part never sees its last contributor and stays unwritten.
-// MDT_GEMM_SPLIT=0 switches the split off.
+// Workspace of the split last wave: one fp32 tile per SM plus SPLIT_COUNTERS counters per tile, zero between launches (the
+// warp that finishes a shared tile clears what it read).  One workspace per stream, since launches on different streams may
+// overlap on the GPU; created on the stream's first product that can use it and cleared by that stream itself: a clear on
+// the default stream is not ordered against a non-blocking stream, and one that comes late takes back partial sums and
+// counts, so that a part never sees its last contributor and stays unwritten.  MDT_GEMM_SPLIT=0 switches the split off.
 struct SplitWorkspace { float* ws; unsigned* ctr; };
 static std::mutex g_split_mutex;
 static std::map<std::pair<int, cudaStream_t>, SplitWorkspace> g_split_ws;
@@ -1279,7 +1278,7 @@ static bool split_workspace(cudaStream_t stream, SplitWorkspace* out) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
     SplitWorkspace w{nullptr, nullptr};
-    const size_t ws_bytes = (size_t)g_num_sms * 2 * BM * 256 * sizeof(float), ctr_bytes = (size_t)g_num_sms * 2 * SPLIT_COUNTERS * sizeof(unsigned);
+    const size_t ws_bytes = (size_t)g_num_sms * BM * 256 * sizeof(float), ctr_bytes = (size_t)g_num_sms * SPLIT_COUNTERS * sizeof(unsigned);
     if (cudaMalloc(&w.ws, ws_bytes) != cudaSuccess) { cudaGetLastError(); return false; }
     if (cudaMalloc(&w.ctr, ctr_bytes) != cudaSuccess) { cudaGetLastError(); cudaFree(w.ws); return false; }
     if (cudaMemsetAsync(w.ws, 0, ws_bytes, stream) != cudaSuccess || cudaMemsetAsync(w.ctr, 0, ctr_bytes, stream) != cudaSuccess) {
@@ -1665,8 +1664,6 @@ static int gemm_transposed(const MdtGemmDesc* d, cudaStream_t stream) {
   const int width = d->dual ? 128 : 256;
   const long long rows = d->mode == 1 ? d->capacity_rows : d->M;
   const long long tiles = ((rows + 255) / 256 + (d->mode == 1 ? p.G : 0)) * ((p.N + width - 1) / width);       // an upper bound
-  SplitWorkspace w;
-  if (split_enabled() && tiles > g_num_sms / 2 && split_workspace(stream, &w)) { p.sk_ws = w.ws; p.sk_ctr = w.ctr; }
   const cudaError_t e = d->dual ? launch_transposed<TP_DUAL>(p, tiles, stream)
                       : (d->swiglu_g != nullptr ? launch_transposed<TP_SWIGLU_BWD>(p, tiles, stream) : launch_transposed<TP_PLAIN>(p, tiles, stream));
   return e == cudaSuccess ? 0 : -100 - (int)e;

@@ -12,8 +12,8 @@
 // Rows of a group are cut into tiles of equal numbers of 32-row units, at most 8 (256 rows), or 16 where tp_joint_pays says so: such a
 // tile is two products with one copy of the weights in shared memory, in both accumulators.  Only rows that exist are
 // multiplied where the caller passes their number (group_rows); the padding up to the next 128-row boundary, zero by contract,
-// gives zeros, which are written without being computed.  The tiles of the last, partly filled round are cut along the depth
-// over all pairs as in the 128-row kernel (get_work): 128 tiles of a down projection are 1.73 rounds of 74 pairs.
+// gives zeros, which are written without being computed.  Every tile is multiplied by one pair, its depth in ascending order as in the
+// pair kernel: results are the same bits in every run, and those of that kernel.
 //
 // Epilogue: TMEM is read in 16 x 256-bit pieces, whose register layout is the one that stmatrix transposes, so that rows of C
 // leave through a 4 KB stage per warp in 16-byte pieces without shuffles.  In the gate / up form the 128 rows of a CTA's
@@ -27,7 +27,7 @@ constexpr int TP_A_BYTES = BM * BK * 2;
 constexpr int TP_RING_BYTES = 6 * (TP_A_BYTES + 128 * BK * 2);
 constexpr int TP_MAX_STAGES = 10;
 // (groups in the order of the rows of their tiles, most first: see tp_work)
-struct TPTable { int group[TP_GROUPS], start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, units, groups, row_tiles, cap; };
+struct TPTable { int group[TP_GROUPS], start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, cap; };
 constexpr int TP_SMEM = TP_RING_BYTES + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES + (int)sizeof(TPTable);
 static_assert(TP_SMEM <= 227 * 1024, "transposed pair kernel: shared memory of a CTA");
 
@@ -43,11 +43,9 @@ struct TPParams {
   long long ldc;
   float alpha; const float* alpha_dev;
   int* status;
-  float* sk_ws; unsigned* sk_ctr;
 };
 // rows [row0, row0 + n) x features [f0, f0 + 256 or 128), rows below `end` are stored; zero0: first row to be cleared (= end: none)
 struct TPTile { int g, f0, row0, n, end, zero0; };
-struct TPWork { TPTile t; int kb0, kb1, split, contributors; };
 
 __host__ __device__ __forceinline__ int tp_tiles_of_rows(int rows, int cap) { return ((rows + TP_UNIT - 1) / TP_UNIT + cap - 1) / cap; }
 // rows of its widest tile
@@ -62,28 +60,25 @@ __host__ __device__ __forceinline__ int tp_first(int n) { return n > 256 ? (n / 
 // with two accumulators, which copies the weights to shared memory once: what the measurements below ask for.
 __host__ __device__ __forceinline__ float tp_clocks(int n) { return n <= 256 ? 220.f + 1.64f * (float)n : 150.f + 2.1f * (float)n; }
 // Clocks of a pair for all tiles: `row_tiles` of them for each of f_tiles, `step` a k block of one (`longest`: of the longest),
-// `rows` rows each; what the last round takes if it is shared is that of tp_split_pays.
-__host__ __device__ __forceinline__ float tp_clocks_of_all(int row_tiles, int f_tiles, int pairs, int kbt, float step, float longest, float rows, float epilogue, bool may_split) {
-  const int total = row_tiles * f_tiles, rounds = total / pairs, rem = total % pairs;
-  const float tile = (float)kbt * step + epilogue * rows;
-  if (total <= pairs) return (float)kbt * longest + epilogue * rows;
-  if (rem == 0) return (float)rounds * tile;
-  const float shared = (float)kbt * step * (float)rem / (float)pairs + 8000.f + 90.f * rows;
-  return (float)rounds * tile + (may_split && shared < tile ? shared : tile);
+// `rows` rows each.
+__host__ __device__ __forceinline__ float tp_clocks_of_all(int row_tiles, int f_tiles, int pairs, int kbt, float step, float longest, float rows, float epilogue) {
+  const int total = row_tiles * f_tiles, rounds = (total + pairs - 1) / pairs;
+  return (float)rounds * ((float)kbt * (total <= pairs ? longest : step) + epilogue * rows);
 }
 // Whether tiles of up to 512 rows are taken (sums over the groups: tiles, k block clocks; longest, of both forms).  Such a tile reads
 // its weights once for twice the rows, but takes both accumulators, so that nothing hides its epilogue (8 clocks a row), and there are
-// fewer of them to go round.  us in turn, up to 256 / up to 512 rows, 8 experts of 4096 x 14336: down 1000 tokens 261 / 245, 2000 423 /
-// 417, 4000 757 / 728, 9200 1803 / 1795; dx (two matrices) 513 / 456, 802 / 822, 1478 / 1394, 3780 / 3691; 1500 tokens, which the model
-// misses, 347 / 355 and 611 / 624; 9200 x 4096 of depth 1024 146 / 153, 4096 433 / 419; 2 experts of 500 tokens, half of whose tiles are
-// too few, 97 / 165.  Not for more than one result a product: gate and up of 2000 tokens 892 / 937, with their inputs kept of 9200
-// 3320 / 3856, SwiGLU backward 1896 / 2704.
+// fewer of them to go round.  us in turn, up to 256 / up to 512 rows, 8 experts of 4096 x 14336: down 800 tokens 247 / 194, 1250 345 / 271,
+// 1750 425 / 462, 2000 386 / 427, 4000 794 / 736, 9200 1494 / 1457; dx (two matrices) 474 / 366, 658 / 511, 763 / 821, 816 / 902,
+// 1568 / 1449, 3652 / 3557; 2 experts of 1000 tokens, half of whose tiles are too few, 175 / 261; dense of depth 14336 2300 x 4096
+// 208 / 349.  Where the two are close the model may miss: 4 experts of 3001 tokens, 14336 x 4096, 552 / 572 and dense 576 x 32000 of
+// depth 4096 151 / 140 run with the slower.  Not for more than one result a product: gate and up of 2000 tokens 892 / 937, with
+// their inputs kept of 9200 3320 / 3856, SwiGLU backward 1896 / 2704.
 struct TPForm { int row_tiles; float step, longest; };
-__host__ __device__ __forceinline__ bool tp_joint_pays(const TPForm& one, const TPForm& two, int units, int f_tiles, int pairs, int kbt, bool may_split) {
+__host__ __device__ __forceinline__ bool tp_joint_pays(const TPForm& one, const TPForm& two, int units, int f_tiles, int pairs, int kbt) {
   if (two.row_tiles == one.row_tiles || two.row_tiles == 0) return false;
   const float rows = 32.f * (float)units;
-  const float a = tp_clocks_of_all(one.row_tiles, f_tiles, pairs, kbt, one.step / (float)one.row_tiles, one.longest, rows / (float)one.row_tiles, 0.f, may_split);
-  const float b = tp_clocks_of_all(two.row_tiles, f_tiles, pairs, kbt, two.step / (float)two.row_tiles, two.longest, rows / (float)two.row_tiles, 8.f, may_split);
+  const float a = tp_clocks_of_all(one.row_tiles, f_tiles, pairs, kbt, one.step / (float)one.row_tiles, one.longest, rows / (float)one.row_tiles, 0.f);
+  const float b = tp_clocks_of_all(two.row_tiles, f_tiles, pairs, kbt, two.step / (float)two.row_tiles, two.longest, rows / (float)two.row_tiles, 8.f);
   return b < 0.98f * a;
 }
 __host__ __device__ __forceinline__ void tp_add_group(TPForm& f, int rows, int cap) {
@@ -121,7 +116,7 @@ __device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, in
     };
     over_lanes(one); over_lanes(two);
     units = __reduce_add_sync(0xffffffffu, units);
-    if (tp_joint_pays(one, two, units, f_tiles, pairs, kbt, p.sk_ws != nullptr)) cap = 16;
+    if (tp_joint_pays(one, two, units, f_tiles, pairs, kbt)) cap = 16;
   }
   for (int g = lane; g < p.G; g += 32) tb->tile0[g] = tp_tile_rows(tp_rows_of(p, g, start, end), cap);
   __syncwarp();
@@ -132,7 +127,7 @@ __device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, in
     tb->group[place] = g; tb->start[place] = start; tb->rows[place] = rows; tb->end[place] = end;
   }
   __syncwarp();
-  int carry = 0, widest = 0, units_all = 0, groups = 0;
+  int carry = 0, widest = 0;
   for (int g0 = 0; g0 < p.G; g0 += 32) {
     const int g = g0 + lane;
     int tiles = 0;
@@ -140,8 +135,6 @@ __device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, in
       const int rows = tb->rows[g];
       tiles = tp_tiles_of_rows(rows, cap) * f_tiles;
       widest = max(widest, tp_tile_rows(rows, cap));
-      groups += tiles > 0 ? 1 : 0;
-      units_all += (rows + TP_UNIT - 1) / TP_UNIT;
     }
     int incl = tiles;
 #pragma unroll
@@ -150,9 +143,7 @@ __device__ __forceinline__ void tp_fill_table(const TPParams& p, TPTable* tb, in
     carry += __shfl_sync(0xffffffffu, incl, 31);
   }
   widest = __reduce_max_sync(0xffffffffu, widest);
-  units_all = __reduce_add_sync(0xffffffffu, units_all);
-  groups = __reduce_add_sync(0xffffffffu, groups);
-  if (lane == 0) { tb->tile0[p.G] = carry; tb->widest = widest; tb->units = units_all; tb->groups = groups; tb->row_tiles = carry / f_tiles; tb->cap = cap; }
+  if (lane == 0) { tb->tile0[p.G] = carry; tb->widest = widest; tb->cap = cap; }
 }
 
 __host__ __device__ __forceinline__ void tp_tile(const TPTable* tb, int G, int f_tiles, int f_width, int t, TPTile& o) {
@@ -170,49 +161,13 @@ __host__ __device__ __forceinline__ void tp_tile(const TPTable* tb, int G, int f
   o.zero0 = n == nt - 1 && o.row0 + o.n < o.end ? o.row0 + o.n : o.end;
 }
 
-// Whether the last round of `rem` tiles is shared along the depth by all pairs.  In clocks: a k block of n rows takes a pair
-// 1.25 * (256 + n), or 704 where its weights come from memory and all pairs ask for some (a tile's share of that is smaller
-// where several tiles read the same weights); sharing costs 8 000 and 90 for each row of the tiles.  Measured, microseconds with
-// / without sharing: down projection, 8 experts, 16 tokens 159 / 152, 1000 tokens 261 / 253, 2000 tokens 357 / 395; gate and up of 16
-// tokens 303 / 313; dense 9200 x 4096 x 4096 197 / 184, 1152 x 4096 x 4096 49 / 53.
-__host__ __device__ __forceinline__ bool tp_split_pays(const TPTable* tb, int f_tiles, int kbt, int rem, int pairs) {
-  const int row_tiles = tb->row_tiles;
-  const float rows = 32.f * (float)tb->units / (float)row_tiles, shared = (float)row_tiles / (float)tb->groups;
-  const float step = rows > 256.f ? tp_clocks((int)rows) : 1.25f * (256.f + rows), memory = 704.f / shared, part = (float)rem / (float)pairs;
-  return (float)kbt * fmaxf(step, memory * part) > (float)kbt * fmaxf(step, memory) * part + 8000.f + 90.f * rows;
-}
-
-// it = 0, 1, ...: the work of pair `pair` of `pairs`.  The tiles come by their rows, most first, and every second round goes through
+// it = 0, 1, ...: the tile of pair `pair` of `pairs`.  The tiles come by their rows, most first, and every second round goes through
 // the pairs backwards, so that all have about the same to do (us, groups in their own order, each round forwards /
-// so: SwiGLU backward of 600 tokens 226 / 214, down 1000 tokens 271 / 261, dx 527 / 513).  The tiles of a last round that leaves more than an eighth of the pairs
-// idle are cut into one contiguous piece of k blocks per pair (see get_work), no piece shorter than 4 blocks.
-__host__ __device__ __forceinline__ bool tp_work(const TPTable* tb, int G, int f_tiles, int f_width, int kbt, bool may_split, int pair, int pairs, int it, TPWork& w) {
-  const int total = tb->tile0[G];
-  int whole = total;
-  const int rem = total % pairs;
-  if (may_split && total > pairs && rem != 0 && kbt >= 8 && tp_split_pays(tb, f_tiles, kbt, rem, pairs)) whole = total - rem;
-  const int n_whole = whole / pairs;                     // (of the pieces of a shared round: what comes before)
-  w.split = -1; w.contributors = 1;
-  const int t = it * pairs + (it & 1 ? pairs - 1 - pair : pair);
-  if (t < whole) {
-    tp_tile(tb, G, f_tiles, f_width, t, w.t);
-    w.kb0 = 0; w.kb1 = kbt;
-    return true;
-  }
-  if (whole == total) return false;
-  const int units = rem * kbt;
-  int per = (units + pairs - 1) / pairs;
-  if (per < 4) per = 4;
-  const int u0 = pair * per, u1 = u0 + per < units ? u0 + per : units;
-  if (u0 >= u1) return false;
-  const int tt = u0 / kbt + (it - n_whole);
-  if (tt > (u1 - 1) / kbt) return false;
-  tp_tile(tb, G, f_tiles, f_width, whole + tt, w.t);
-  const int lo = tt * kbt, hi = lo + kbt;
-  w.kb0 = (u0 > lo ? u0 : lo) - lo;
-  w.kb1 = (u1 < hi ? u1 : hi) - lo;
-  w.contributors = (hi - 1) / per - lo / per + 1;
-  w.split = w.contributors > 1 ? tt : -1;
+// so: SwiGLU backward of 600 tokens 226 / 214, down 1000 tokens 271 / 261, dx 527 / 513).
+__host__ __device__ __forceinline__ bool tp_work(const TPTable* tb, int G, int f_tiles, int f_width, int pair, int pairs, int it, TPTile& t) {
+  const int i = it * pairs + (it & 1 ? pairs - 1 - pair : pair);
+  if (i >= tb->tile0[G]) return false;
+  tp_tile(tb, G, f_tiles, f_width, i, t);
   return true;
 }
 
@@ -264,10 +219,10 @@ __device__ __forceinline__ void tp_fetch(uint4 (&v)[4], const TPParams& p, const
   for (int i = 0; i < 4; ++i) v[i] = __ldcg(at[i]);
 }
 
-// One warp's part of a tile: its 32 TMEM lanes, every second chunk of 32 rows from `half` on.  `load(c, lo, hi)` brings the
-// accumulators of chunk c: lo of the lanes 0-15, hi of 16-31 of the warp's quarter.  `ready` is called before the first one.
-template <int KIND, class Ready, class Load>
-__device__ __forceinline__ bool tp_epilogue(const TPParams& p, uint8_t* stage, const TPTile& t, int col, int half, int lane, float alpha, Ready ready, Load load) {
+// One warp's part of a tile: its 32 TMEM lanes (from `acc`), every second chunk of 32 rows from `half` on.  `ready` is called before the
+// first read of the accumulator.
+template <int KIND, class Ready>
+__device__ __forceinline__ bool tp_epilogue(const TPParams& p, uint8_t* stage, const TPTile& t, int col, int half, int lane, float alpha, uint32_t acc, Ready ready) {
   const int chunks = t.n / TP_UNIT;
   const uint32_t st = smem_u32(stage);
   uint4 pg[4], pu[4];
@@ -278,8 +233,10 @@ __device__ __forceinline__ bool tp_epilogue(const TPParams& p, uint8_t* stage, c
 #pragma unroll 1
   for (int c = half; c < chunks; c += 2) {
     const int row0 = t.row0 + c * 32;
-    uint32_t lo[16], hi[16];
-    load(c, lo, hi);
+    uint32_t lo[16], hi[16];                      // lanes 0-15 and 16-31 of the warp's quarter
+    tmem_ld_16x256b_x4(acc + c * 32, lo);
+    tmem_ld_16x256b_x4(acc + c * 32 + (16u << 16), hi);
+    tmem_ld_wait();
     if constexpr (KIND == TP_PLAIN) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -371,7 +328,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
   const int pair_id = (int)cluster_id_x(), num_pairs = (int)num_clusters_x();
   const int f_tiles = (p.N + F_WIDTH - 1) / F_WIDTH;
   const int num_kb = (p.K + BK - 1) / BK, kbt = num_kb + (p.K_l + BK - 1) / BK;
-  const bool may_split = p.sk_ws != nullptr;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TP_MAX_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -393,8 +349,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     *abort_flag = 1;
     if (p.status != nullptr) atomicCAS(p.status, 0, code);
   };
-  TPWork w;
-  auto next = [&](int it) { return tp_work(tb, p.G, f_tiles, F_WIDTH, kbt, may_split, pair_id, num_pairs, it, w); };
+  TPTile w;
+  auto next = [&](int it) { return tp_work(tb, p.G, f_tiles, F_WIDTH, pair_id, num_pairs, it, w); };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (one per CTA)
@@ -403,13 +359,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     uint32_t ph = 0;
     bool ok = true;
     for (int wi = 0; ok && next(wi); ++wi) {
-      const TPTile& t = w.t;
+      const TPTile& t = w;
       const int f0 = t.f0 + rank * (F_WIDTH / 2);
       const uint32_t bytes = 2 * (TP_A_BYTES + t.n / 2 * (BK * 2));
       // (a loop for each of one and two accumulators, here and in the issuer: with the choice inside, tiles of 256 rows took 25 % longer)
       auto load = [&](auto two) {
         const int n0 = decltype(two)::value ? tp_first(t.n) : t.n;
-        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+        for (int kb = 0; kb < kbt; ++kb) {
           if (!wait_parity_warp(&empty_bar[s], ph ^ 1, abort_flag)) { fail(ST_TIMEOUT_EMPTY); ok = false; break; }
           uint8_t* sW = smem + s * stage_bytes;
           uint8_t* sX = sW + TP_A_BYTES;
@@ -461,12 +417,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     bool ok = true;
     for (int wi = 0; ok && next(wi); ++wi) {
       auto multiply = [&](auto two) {
-        const int n0 = decltype(two)::value ? tp_first(w.t.n) : w.t.n, n1 = w.t.n - n0, buf = acc_it & 1;
+        const int n0 = decltype(two)::value ? tp_first(w.n) : w.n, n1 = w.n - n0, buf = acc_it & 1;
         if (!wait_parity_warp(&tempty_bar[buf], ((acc_it >> 1) & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); ok = false; return; }
         if (decltype(two)::value && !wait_parity_warp(&tempty_bar[buf ^ 1], (((acc_it + 1) >> 1) & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); ok = false; return; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256, d_tmem1 = tmem_base + (buf ^ 1) * 256;
-        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+        for (int kb = 0; kb < kbt; ++kb) {
           if (!wait_parity_warp(&full_bar[s], ph, abort_flag)) { fail(ST_TIMEOUT_FULL); ok = false; return; }
           tc_fence_after();
           const int w_mn = kb >= num_kb ? p.w_mn_l : p.w_mn;
@@ -477,13 +433,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k)
-              umma_bf16_pair(d_tmem, dw + k * kw, dx + k * kx, idesc, (kb > w.kb0 || k > 0) ? 1u : 0u);
+              umma_bf16_pair(d_tmem, dw + k * kw, dx + k * kx, idesc, (kb > 0 || k > 0) ? 1u : 0u);
             if (decltype(two)::value) {
               const uint32_t idesc1 = make_idesc_bf16(2 * BM, n1, w_mn, 0);
               const uint64_t dx1 = operand_desc(sW + TP_A_BYTES + n0 / 2 * (BK * 2), 0);
 #pragma unroll
               for (int k = 0; k < BK / 16; ++k)
-                umma_bf16_pair(d_tmem1, dw + k * kw, dx1 + k * kx, idesc1, (kb > w.kb0 || k > 0) ? 1u : 0u);
+                umma_bf16_pair(d_tmem1, dw + k * kw, dx1 + k * kx, idesc1, (kb > 0 || k > 0) ? 1u : 0u);
             }
             umma_commit_pair(&empty_bar[s], 3);   // frees the stage in both CTAs
           }
@@ -495,7 +451,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
         }
         acc_it += decltype(two)::value ? 2 : 1;
       };
-      if (!JOINT || w.t.n <= 256) multiply(std::false_type());
+      if (!JOINT || w.n <= 256) multiply(std::false_type());
       else multiply(std::integral_constant<bool, JOINT>());
     }
   } else if (warp >= 2) {
@@ -507,7 +463,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     bool ok = true;
     for (int wi = 0, sub = 0; ok && (sub > 0 || next(wi)); sub > 0 ? 0 : ++wi) {
       // (a tile of more than 256 rows: its two accumulators one after the other)
-      TPTile t = w.t;
+      TPTile t = w;
       const int mine = sub;
       if (JOINT) {
         const int n0 = tp_first(t.n);
@@ -519,69 +475,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
       const int buf = acc_it & 1;
       const uint32_t aph = (acc_it >> 1) & 1;
       const uint32_t tacc = tmem_base + buf * 256 + ((uint32_t)(q * 32) << 16);
-      if (w.kb0 == 0 && mine == 0) tp_clear<KIND>(p, t.zero0, t.end, col, half, lane);     // under the wait for the accumulator
+      if (mine == 0) tp_clear<KIND>(p, t.zero0, t.end, col, half, lane);     // under the wait for the accumulator
       auto ready = [&]() {
         if (!wait_parity_warp(&tfull_bar[buf], aph, abort_flag)) { fail(ST_TIMEOUT_TMEM_FULL); return false; }
         tc_fence_after();
         return true;
       };
-      auto from_tmem = [&](int c, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
-        tmem_ld_16x256b_x4(tacc + c * 32, lo);
-        tmem_ld_16x256b_x4(tacc + c * 32 + (16u << 16), hi);
-        tmem_ld_wait();
-      };
-      auto release = [&]() {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
-        ++acc_it;
-      };
-      if (w.split < 0) {
-        ok = tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, ready, from_tmem);
-        if (ok) release();
-        continue;
-      }
-      // A piece of a shared tile: partial sums into the fp32 workspace, whole 512-byte lines per reduction; the warp that
-      // comes last at its part of the tile reads them back, clears them and finishes the part.
-      const int part = ((JOINT ? w.split * (tb->cap / 8) + mine : w.split) * 2 + rank) * EPI_WARPS + half * 4 + q;
-      float4* ws = reinterpret_cast<float4*>(p.sk_ws) + (long long)part * (4 * 8 * 32) + lane;
-      ok = ready();
+      ok = tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, tacc, ready);
       if (!ok) break;
-#pragma unroll 1
-      for (int c = half; c < t.n / TP_UNIT; c += 2) {
-        uint32_t lo[16], hi[16];
-        from_tmem(c, lo, hi);
-        float4* at = ws + (c >> 1) * 256;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          red_add_v4_f32(reinterpret_cast<float*>(at + i * 32), __uint_as_float(lo[4 * i]), __uint_as_float(lo[4 * i + 1]), __uint_as_float(lo[4 * i + 2]), __uint_as_float(lo[4 * i + 3]));
-          red_add_v4_f32(reinterpret_cast<float*>(at + (4 + i) * 32), __uint_as_float(hi[4 * i]), __uint_as_float(hi[4 * i + 1]), __uint_as_float(hi[4 * i + 2]), __uint_as_float(hi[4 * i + 3]));
-        }
-      }
-      release();
-      if (half >= t.n / TP_UNIT) continue;
-      __threadfence();
+      tc_fence_before();
       __syncwarp();
-      unsigned before = 0;
-      if (lane == 0) before = atomicAdd(p.sk_ctr + part, 1u);
-      before = __shfl_sync(0xffffffffu, before, 0);
-      if (before != (unsigned)w.contributors - 1u) continue;
-      __threadfence();
-      auto from_ws = [&](int c, uint32_t (&lo)[16], uint32_t (&hi)[16]) {
-        float4* at = ws + (c >> 1) * 256;
-        float4 v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = __ldcg(at + i * 32);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) __stcg(at + i * 32, make_float4(0.f, 0.f, 0.f, 0.f));     // leave the workspace clean
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          lo[4 * i] = __float_as_uint(v[i].x); lo[4 * i + 1] = __float_as_uint(v[i].y); lo[4 * i + 2] = __float_as_uint(v[i].z); lo[4 * i + 3] = __float_as_uint(v[i].w);
-          hi[4 * i] = __float_as_uint(v[4 + i].x); hi[4 * i + 1] = __float_as_uint(v[4 + i].y); hi[4 * i + 2] = __float_as_uint(v[4 + i].z); hi[4 * i + 3] = __float_as_uint(v[4 + i].w);
-        }
-      };
-      tp_epilogue<KIND>(p, stage, t, col, half, lane, alpha, []() { return true; }, from_ws);
-      if (lane == 0) p.sk_ctr[part] = 0;
+      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty_bar[buf]), 0));
+      ++acc_it;
     }
   }
 

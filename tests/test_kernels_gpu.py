@@ -271,8 +271,8 @@ def test_swiglu_backward_in_the_product(ops, T, E, H, F, policy):
 def test_transposed_pair_kernel(ops, counts, H, F):
     """Weights as the 256-row operand, rows of every group counted exactly: remainders of the 32-row units, of 256-row tiles
     and 8-tile panels, of feature tiles and of the depth; gate / up with and without its outputs and with adapters, SwiGLU
-    backward, K-major and MN-major weights, two depth segments; shared last rounds (2100 rows).  fp32 reference, one bf16
-    rounding of each result (2e-2 as for the other products); padding becomes zeros, rows past the groups stay untouched."""
+    backward, K-major and MN-major weights, two depth segments.  fp32 reference, one bf16 rounding of each result (2e-2 as
+    for the other products); padding becomes zeros, rows past the groups stay untouched."""
     torch.manual_seed(sum(counts) + F)
     E, r = len(counts), 16
     ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(sum(counts))].to(DEV).int()
@@ -329,6 +329,40 @@ def test_transposed_pair_kernel(ops, counts, H, F):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("counts", [[211, 281, 92, 321, 302, 269, 245, 279], [19, 0, 23, 31, 7, 40, 18, 16], [1024, 700, 513, 65]])
+def test_transposed_products_have_one_order_of_sums(ops, counts):
+    """Several rounds of tiles, the last one partly filled: results are the same bits in every run, and those of the CTA-pair kernel, which
+    adds the depth up in the same order."""
+    torch.manual_seed(sum(counts))
+    E, H, F, r = len(counts), 1024, 4096, 16
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(sum(counts))].to(DEV).int()
+    plan = ops.make_plan(ids[:, None], E)
+    R = plan.src_slot.numel()
+    rows = lambda n: torch.where((plan.src_slot >= 0)[:, None], _rand(R, n), 0.0).to(torch.bfloat16)
+    x, a, t = rows(H), rows(F), rows(2 * r)
+    w1, w3, w2, v = _rand(E, F, H, scale=0.1), _rand(E, F, H, scale=0.1), _rand(E, F, H, scale=0.1), _rand(E, 4 * H, F, scale=0.1)
+    b1, b3 = _rand(E, F, 2 * r, scale=0.1), _rand(E, F, 2 * r, scale=0.1)
+
+    def products():
+        h, g, u, y, z, dg, du, dx = (torch.zeros(R, n, dtype=torch.bfloat16, device=DEV) for n in (F, F, F, H, 4 * H, F, F, H))
+        ops._g(1, x, False, w1, False, h, F, H, plan, B2=w3, C2=g, C3=u, A_l=t, B_l=b1, B2_l=b3, b_mn_l=False, K_l=2 * r)
+        ops._g(1, a, False, w2, True, y, H, F, plan)
+        ops._g(1, a, False, v, False, z, 4 * H, F, plan)
+        ops._g(1, x, False, w2, False, dg, F, H, plan, C2=du, swiglu=(g, u))
+        ops._g(1, dg, False, w1, True, dx, H, F, plan, A_l=du, B_l=w3, b_mn_l=True, K_l=F)
+        return h, g, u, y, z, dg, du, dx
+    prev = ops.ext.gemm_set_pair_policy(6)
+    try:
+        runs = [products() for _ in range(3)]
+        ops.ext.gemm_set_pair_policy(2)
+        runs.append(products())
+    finally:
+        ops.ext.gemm_set_pair_policy(prev)
+    for name, first, *others in zip(("h", "g", "u", "y", "z", "dg", "du", "dx"), *runs):
+        assert all(torch.equal(first, o) for o in others), name
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("M,N", [(129, 12000), (144, 32008), (300, 32000), (576, 4096), (577, 4100), (1300, 4096)])
 @pytest.mark.parametrize("K", [264, 4096])
 def test_dense_products_of_odd_row_counts(ops, M, N, K):
@@ -348,7 +382,7 @@ def test_dense_products_of_odd_row_counts(ops, M, N, K):
                                           ([211, 281, 92, 321, 302, 269, 245, 279], 14336)])
 def test_transposed_pair_kernel_with_two_accumulators(ops, counts, depth):
     """Depths and numbers of tiles at which tiles of more than 256 rows are taken (tests/host/tile_enumeration.cu has the choice):
-    both accumulators equal and not, beside tiles of one, with and without a last round that is shared, K-major and MN-major weights
+    both accumulators equal and not, beside tiles of one, K-major and MN-major weights
     and two depth segments.  fp32 reference, 2e-2 as above; padding becomes zeros."""
     torch.manual_seed(depth)
     E, N, r = len(counts), 4096, 16
