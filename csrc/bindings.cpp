@@ -671,10 +671,10 @@ std::pair<Tensor, OptTensor> lin_fwd(const Tensor& x, const Lin& l, const OptTen
 }
 // dx (+)= dy W (+ LoRA), and the requested parameter gradients
 struct LinGrads { OptTensor dW, dA, dB; };
-// w_out: where the weight gradient goes (and whether it is added to what is there) instead of a new tensor.  given: s dy B where it is
-// there already.  later: adapter gradients join these products instead of being launched here.
+// w_out: where the weight gradient is written instead of a new tensor.  given: s dy B where it is there already.  later: adapter
+// gradients join these products instead of being launched here.
 LinGrads lin_bwd(const Tensor& dy, const Tensor& xin, const Lin& l, const OptTensor& t, bool need_w, bool need_a, bool need_b,
-                 Tensor& dx, bool accumulate, const OptTensor& status, const OptTensor& w_out = std::nullopt, bool w_add = false,
+                 Tensor& dx, bool accumulate, const OptTensor& status, const OptTensor& w_out = std::nullopt,
                  const OptTensor& given = std::nullopt, ProductsTogether* later = nullptr) {
   const int64_t M = dy.size(0), N = dy.size(1), K = l.W.size(1);
   LinGrads g;
@@ -701,9 +701,8 @@ LinGrads lin_bwd(const Tensor& dy, const Tensor& xin, const Lin& l, const OptTen
     gemm_raw(0, dy, false, l.W, true, dx, M, K, N, std::nullopt, std::nullopt, false, 0, accumulate, 1.0, status);
   }
   if (need_w) {
-    Tensor w = w_out.has_value() ? *w_out : torch::empty_like(l.W);
-    gemm_raw(2, dy, true, xin, true, w, N, K, M, std::nullopt, std::nullopt, false, 0, w_out.has_value() && w_add, 1.0, status);
-    if (!w_out.has_value()) g.dW = w;
+    g.dW = w_out.has_value() ? *w_out : torch::empty_like(l.W);
+    gemm_raw(2, dy, true, xin, true, *g.dW, N, K, M, std::nullopt, std::nullopt, false, 0, false, 1.0, status);
   }
   return g;
 }
@@ -790,17 +789,16 @@ std::vector<Tensor> attention_block_fwd(const Tensor& x, const std::vector<Tenso
   return {out, rstd, xn, qr, kr, v3, o, lse, tq.value_or(none), tk.value_or(none), tv.value_or(none), to.value_or(none)};
 }
 
-// needs[j] for params[j]; w_out / w_add: for q, k, v, o where the weight's gradient goes and whether it is added there (an empty
-// tensor: a new one).  Returns {dx, grads of params in order (empty tensor where not needed or given a place)}
+// needs[j] for params[j]; w_out: for q, k, v, o the tensor that the weight's gradient is written to (an empty one: a new tensor).
+// Returns {dx, grads of params in order (empty tensor where not needed)}
 std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tensor>& saved, const std::vector<Tensor>& params,
                                         const std::vector<double>& scalings, const std::vector<bool>& needs, const Tensor& positions,
                                         const Tensor& cu_seqlens, int64_t max_seqlen, double theta, int64_t Hq, int64_t Hkv, int64_t d,
-                                        const Tensor& status_t, const std::vector<Tensor>& w_out, const std::vector<bool>& w_add) {
+                                        const Tensor& status_t, const std::vector<Tensor>& w_out) {
   c10::cuda::CUDAGuard guard(dy.device());
   Phase ph("attention.backward");
-  TORCH_CHECK(w_out.size() == w_add.size() && (w_out.empty() || w_out.size() == 4), "attention_block_bwd: four places or none");
+  TORCH_CHECK(w_out.empty() || w_out.size() == 4, "attention_block_bwd: four places or none");
   auto place = [&](int j) -> OptTensor { return w_out.empty() || !w_out[j].numel() ? std::nullopt : OptTensor(w_out[j]); };
-  auto adds = [&](int j) { return !w_add.empty() && (bool)w_add[j]; };
   OptTensor status = status_t;
   const Tensor &x = saved[0], &rstd = saved[1], &xn = saved[2], &qr = saved[3], &kr = saved[4], &v3 = saved[5], &o = saved[6], &lse = saved[7];
   auto opt = [](const Tensor& t) -> OptTensor { return t.numel() ? OptTensor(t) : std::nullopt; };
@@ -822,7 +820,7 @@ std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tens
   Tensor o2 = o.view({T, Hq * d});
   ProductsTogether grads_together;           // the adapters' gradients, all in one launch at the end
   Tensor d_o = torch::empty({T, Hq * d}, x.options());
-  put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status, place(3), adds(3), std::nullopt, &grads_together));
+  put(io, lo, lin_bwd(dyc, o2, lo, to, nd(io, 0), lo.A.has_value() && nd(io, 1), lo.A.has_value() && nd(io, 2), d_o, false, status, place(3), std::nullopt, &grads_together));
   auto g3 = attention_bwd(qr, kr, v3, o, d_o.view({T, Hq, d}), lse, cu_seqlens, max_seqlen, 1.0 / std::sqrt((double)d), status);
   Tensor dq = rope(g3[0], positions, theta, true).view({T, Hq * d});
   Tensor dk = rope(g3[1], positions, theta, true).view({T, Hkv * d});
@@ -839,9 +837,9 @@ std::vector<Tensor> attention_block_bwd(const Tensor& dy, const std::vector<Tens
     dtq = dt_of(lq, dq); dtk = dt_of(lk, dk); dtv = dt_of(lv, dv);
     ts.launch();
   }
-  put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status, place(0), adds(0), dtq, &grads_together));
-  put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status, place(1), adds(1), dtk, &grads_together));
-  put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status, place(2), adds(2), dtv, &grads_together));
+  put(iq, lq, lin_bwd(dq, xn, lq, tq, nd(iq, 0), lq.A.has_value() && nd(iq, 1), lq.A.has_value() && nd(iq, 2), d_xn, false, status, place(0), dtq, &grads_together));
+  put(ik, lk, lin_bwd(dk, xn, lk, tk, nd(ik, 0), lk.A.has_value() && nd(ik, 1), lk.A.has_value() && nd(ik, 2), d_xn, true, status, place(1), dtk, &grads_together));
+  put(iv, lv, lin_bwd(dv, xn, lv, tv, nd(iv, 0), lv.A.has_value() && nd(iv, 1), lv.A.has_value() && nd(iv, 2), d_xn, true, status, place(2), dtv, &grads_together));
   grads_together.launch();
   auto rb = rmsnorm_bwd(x, params[0], d_xn, rstd, dyc, (bool)needs[0]);     // + dy: the residual connection's gradient
   Tensor dx = rb[0];

@@ -477,8 +477,8 @@ def rope(x, positions, theta):
 
 
 def grad_place(w):
-    """Where the gradient of `w` is collected (an object whose target() gives the tensor and whether to add to it), or None: an
-    ordinary gradient tensor.  Set on the weight views of a flat parameter that only one rank holds."""
+    """Where the gradient of `w` may be written (an object whose tensor() gives the tensor, or None), or None: an ordinary gradient
+    tensor.  Set on the weight views of a flat parameter that only one rank holds.  The tensor is returned as the gradient."""
     return getattr(w, "_grad_place", None)
 
 
@@ -494,11 +494,9 @@ class _Embedding(torch.autograd.Function):
     def backward(ctx, dout):
         (ids,) = ctx.saved_tensors
         dout = _rows(dout)
-        if ctx.place is not None:
-            dtable, add = ctx.place.target()
-            ext.embedding_bwd(dout, ids, dtable, add)
-            return None, None
-        dtable = torch.empty(ctx.shape, dtype=dout.dtype, device=dout.device)
+        dtable = ctx.place.tensor() if ctx.place is not None else None
+        if dtable is None:
+            dtable = torch.empty(ctx.shape, dtype=dout.dtype, device=dout.device)
         ext.embedding_bwd(dout, ids, dtable, False)
         return None, dtable
 
@@ -535,11 +533,8 @@ class _LinearCrossEntropy(torch.autograd.Function):
         factor = (dloss_sum * n.clamp(min=1.0)).float()
         dh = mm_nn(dlogits, w_head, alpha_dev=factor) if ctx.needs_input_grad[0] else None
         dw = None
-        if ctx.needs_input_grad[1] and ctx.place is not None:
-            out, add = ctx.place.target()
-            mm_tn(dlogits, hidden, out=out, accumulate=add, alpha_dev=factor)
-        elif ctx.needs_input_grad[1]:
-            dw = mm_tn(dlogits, hidden, alpha_dev=factor)
+        if ctx.needs_input_grad[1]:
+            dw = mm_tn(dlogits, hidden, out=ctx.place.tensor() if ctx.place is not None else None, alpha_dev=factor)
         return dh, dw, None, None
 
 

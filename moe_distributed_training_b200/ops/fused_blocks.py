@@ -55,15 +55,15 @@ class _AttentionBlockNative(torch.autograd.Function):
         saved = ctx.saved_tensors
         state, params = list(saved[:12]), list(saved[12:])
         needs = [bool(n) for n in ctx.needs_input_grad[3:]]
-        out, add = [], []
+        out = []
         if ctx.places is not None:            # frozen weights have no place either
-            at, targets = 1, []
+            at = 1
             for p, s in zip(ctx.places, scalings):
-                targets.append(p.target() if p is not None and needs[at] else (dy.new_empty(0), False))
+                t = p.tensor() if p is not None and needs[at] else None
+                out.append(dy.new_empty(0) if t is None else t)
                 at += 1 if s is None else 3
-            out, add = [t for t, _ in targets], [a for _, a in targets]
         res = ext.attention_block_bwd(dy, state, params, ctx.sc, needs, positions, cu, max_seqlen, theta, Hq, Hkv, d,
-                                      C.status_tensor(dy.device), out, add)
+                                      C.status_tensor(dy.device), out)
         grads = tuple(g if (g.numel() and need) else None for g, need in zip(res[1:], needs))
         return (res[0], None, None) + grads
 

@@ -53,16 +53,16 @@ def _gemm_only_weight(qualname: str, p) -> bool:
 
 
 class _GradPlace:
-    """Where the gradient of one weight of a flat parameter is collected; the products that compute it write or add there."""
+    """Where a product may write the gradient of one weight of a flat parameter."""
 
     __slots__ = ("group", "index")
 
     def __init__(self, group, index):
         self.group, self.index = group, index
 
-    def target(self):
-        """The weight's part of the flat gradient, and whether it holds a gradient already."""
-        return self.group.grad_target(self.index)
+    def tensor(self):
+        """The weight's part of the flat gradient in the making, or None: the gradient needs a tensor of its own."""
+        return self.group.grad_tensor(self.index)
 
 
 class FlatParamGroup:
@@ -106,10 +106,11 @@ class FlatParamGroup:
         self.shard = nn.Parameter(shard, requires_grad=trainable)
         self.full: Optional[torch.Tensor] = None
         self.acc: Optional[torch.Tensor] = None  # fp32 full-size local accumulation (sync_each_batch=False)
-        # Set where nothing has to be reduced (one rank): products put weight gradients straight into the flat gradient.  Until
-        # that is complete it is kept here with the indices of the weights written so far.
+        # Set where nothing has to be reduced (one rank): products write a step's first weight gradients into the buffer that becomes
+        # the flat gradient and return those parts of it as gradients, so that only autograd decides what they count for (a
+        # pass that was not asked for them, hooks, sums of several uses).  Here: that buffer and the weights whose part was given out.
         self.collect_in_place = False
-        self._collecting: Optional[tuple] = None
+        self._places: Optional[tuple] = None
 
     def install(self, full: torch.Tensor, as_leaves: bool) -> List[torch.Tensor]:
         """Point the modules' weights at views of `full`.
@@ -139,16 +140,33 @@ class FlatParamGroup:
             self._installed_key = key
         return entry[1]
 
-    def grad_target(self, index: int):
-        mod, name, shape, n, o = self.specs[index]
+    def grad_tensor(self, index: int) -> Optional[torch.Tensor]:
+        """The part of weight `index` in the flat gradient that is in the making; None once there is a flat gradient (the new one is
+        added to it) or where the part has been given out (whoever has it may still need it)."""
         if self.shard.grad is not None:
-            return self.shard.grad[o:o + n].view(shape), True
-        if self._collecting is None:
-            self._collecting = (torch.empty_like(self.shard.data), set())
-        flat, written = self._collecting
-        add = index in written
-        written.add(index)
-        return flat[o:o + n].view(shape), add
+            return None
+        if self._places is None:
+            self._places = (torch.empty_like(self.shard.data), set())
+        flat, given = self._places
+        if index in given:
+            return None
+        given.add(index)
+        mod, name, shape, n, o = self.specs[index]
+        return flat[o:o + n].view(shape)
+
+    def take_places(self, grads: List[Optional[torch.Tensor]]):
+        """(buffer for the flat gradient, indices of the weights whose gradient in `grads` is its part already).  A part that was given
+        out and did not come back may be in somebody's hands (a gradient that was asked for by itself, one that a hook
+        kept): then the buffer is left to them and another one taken."""
+        places, self._places = self._places, None
+        if places is not None:
+            flat, given = places
+            base, size = flat.data_ptr(), flat.element_size()
+            there = {i for i in given if grads[i] is not None and grads[i].data_ptr() == base + self.specs[i][4] * size
+                     and grads[i].shape == self.specs[i][2] and grads[i].dtype == flat.dtype and grads[i].is_contiguous()}
+            if len(there) == len(given):
+                return flat, there
+        return torch.empty_like(self.shard.data), set()
 
     def installed_leaves(self) -> List[torch.Tensor]:
         """Autograd-leaf views of the buffer that is currently installed (empty for frozen groups)."""
@@ -265,7 +283,7 @@ class _LayerFn(torch.autograd.Function):
         leaves = []
         for g, buf in zip(unit.groups, unit.buffers):
             leaves += g.install(buf, as_leaves=True)
-            g._collecting = None        # (left behind by a backward pass that failed in this block)
+            g._places = None            # (left behind by a backward pass that failed in this block)
         local = [p for p in unit.local_params if p.requires_grad]
         xin = x.detach().requires_grad_(True)
         layer = runner.model.model.layers[idx]
@@ -599,18 +617,18 @@ class ShardedMixtral:
             flat, written = g.shard.grad, ()
             if fresh:
                 # (what the products have written already: only where scale is 1, see collect_in_place)
-                flat, written = g._collecting if g._collecting is not None else (torch.empty_like(g.shard.data), ())
-                g._collecting = None
+                flat, written = g.take_places(grads)
+            g._places = None
             dst, src, end = [], [], 0
             for i, ((mod, name, shape, n, o), gr) in enumerate(zip(g.specs, grads)):
                 if fresh and end < o:
                     flat[end:o].zero_()                                      # alignment gaps
                 end = o + n
-                if gr is not None and i in written:
-                    flat[o:end].view(shape).add_(gr)
-                elif gr is not None:
+                if i in written:
+                    continue
+                if gr is not None:
                     dst.append(flat[o:end].view(shape)); src.append(gr if gr.dtype == flat.dtype else gr.to(flat.dtype))
-                elif fresh and i not in written:
+                elif fresh:
                     flat[o:end].zero_()
             if fresh and end < flat.numel():
                 flat[end:].zero_()
@@ -806,7 +824,7 @@ class ShardedMixtral:
             if tg is not None:
                 leaves = tg.installed_leaves()
                 grads = [leaf.grad for leaf in leaves]
-                if any(gr is not None for gr in grads) or tg._collecting is not None:
+                if any(gr is not None for gr in grads):
                     self._reduce_unit_grads(unit, grads)
                 for leaf in leaves:
                     leaf.grad = None

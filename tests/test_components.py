@@ -293,6 +293,53 @@ def test_attention_backward_scratch_grows_with_tokens_not_with_sequences(seqs, l
     assert floats <= 1.01 * (1 + 3 * 128) * T * heads + 256 * 2 * heads + 64
 
 
+def test_parts_of_the_flat_gradient_are_given_out_once():
+    """The buffer becomes the flat gradient where every part that was given out comes back as its weight's gradient; otherwise whoever
+    has a part keeps it, and the flat gradient is another buffer.  Parts are never read before they came back."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.train.engine import build_engine
+    cfg = MixtralConfig(vocab_size=64, hidden_size=32, intermediate_size=32, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1,
+                        num_local_experts=2, num_experts_per_tok=1)
+    eng = build_engine(cfg, dtype=torch.float32, device_type="cpu", learning_rate=1e-3, seed=0)
+    unit = eng.runner.root
+    g = unit.trainable_group
+    n = len(g.specs)
+    assert g.collect_in_place and n == 3
+    one = lambda i: torch.full(g.specs[i][2], float(i + 1))
+    want = torch.zeros_like(g.shard.data)
+    for i, (mod, name, shape, size, o) in enumerate(g.specs):
+        want[o:o + size] = i + 1.0
+
+    def parts(*which):
+        out = [g.grad_tensor(i) for i in which]
+        for i, t in zip(which, out):
+            t.copy_(one(i))
+        return out
+    # all parts come back: no copy
+    a, b = parts(0, 2)
+    buffer = g._places[0]
+    eng.runner._reduce_unit_grads(unit, [a, one(1), b])
+    assert g.shard.grad is buffer and torch.equal(g.shard.grad, want)
+    # there is a flat gradient: no parts, the next gradients are added
+    assert g.grad_tensor(0) is None
+    eng.runner._reduce_unit_grads(unit, [one(0), one(1), one(2)])
+    assert torch.equal(g.shard.grad, 2 * want)
+    # a part that somebody else has
+    for grads in ([None, one(1), None], [one(0), one(1), one(2)]):
+        eng.optimizer.zero_grad(set_to_none=True)
+        (held,) = parts(0)
+        assert g.grad_tensor(0) is None and g.grad_tensor(1) is not None
+        g._places[0][g.specs[1][4]:] = float("nan")
+        eng.runner._reduce_unit_grads(unit, grads)
+        expected = want.clone()
+        for i, (mod, name, shape, size, o) in enumerate(g.specs):
+            if grads[i] is None:
+                expected[o:o + size] = 0.0
+        assert torch.equal(g.shard.grad, expected) and torch.equal(held, one(0))
+        g.shard.grad.fill_(7.0)
+        assert torch.equal(held, one(0))
+
+
 def test_expert_gradient_buffers_become_grad_only_once_they_are_written(monkeypatch):
     """A backward pass that fails before its weight-gradient products are launched leaves `.grad` as it was; one that
     succeeds hands over exactly the buffers that it wrote, and the next one adds to them."""

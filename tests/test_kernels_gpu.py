@@ -717,61 +717,106 @@ def test_embedding_gradient_written_and_added(ops, T, V, H, repeat, dtype):
     assert torch.equal(out[untouched], old[untouched])
 
 
-@pytest.mark.parametrize("recompute", [True, False])
-def test_weight_gradients_collected_in_place(recompute):
-    """One rank: products write or add the dense weights' gradients in the flat gradient; the same step through ordinary gradient
-    tensors, two micro-batches (each of the latter's gradients is rounded once more, 0.4 % each), and again after a backward pass that
-    failed in a block."""
+def _small_engine(recompute):
     from moe_distributed_training_b200 import MixtralConfig
     from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
-    from moe_distributed_training_b200.ops import fused_blocks
     from moe_distributed_training_b200.train.engine import build_engine
     cfg = MixtralConfig(vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=2, num_key_value_heads=1,
                         head_dim=128, num_local_experts=4, num_experts_per_tok=2)
-    mbs = list(batches(SyntheticInstructionDataset(cfg.vocab_size, 2, 60, 150), 1))
+    mbs = [{k: (v.to(DEV) if torch.is_tensor(v) else v) for k, v in mb.items()} for mb in batches(SyntheticInstructionDataset(cfg.vocab_size, 2, 60, 150), 1)]
+    eng = build_engine(cfg, dtype=torch.bfloat16, device_type="cuda", learning_rate=1e-3, seed=0, activation_checkpointing=recompute)
+    assert eng.runner.recompute == recompute
+    return eng, mbs, [u.trainable_group for u in eng.runner.all_units()]
 
-    def step(place, fail=False):
-        eng = build_engine(cfg, dtype=torch.bfloat16, device_type="cuda", learning_rate=1e-3, seed=0, activation_checkpointing=recompute)
-        assert eng.runner.recompute == recompute
-        groups = [u.trainable_group for u in eng.runner.all_units()]
+
+def _forward(eng, mb):
+    return eng.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb["cu_seqlens"], max_seqlen=mb["max_seqlen"])
+
+
+def _all_grads(eng, groups):
+    return [g.shard.grad.clone() for g in groups] + [p.grad.clone() for p in eng.model.parameters() if p.grad is not None]
+
+
+@pytest.mark.parametrize("recompute", [True, False])
+def test_weight_gradients_collected_in_place(recompute):
+    """One rank: products write the dense weights' first gradients in the flat gradient; the same step through ordinary gradient
+    tensors, two micro-batches (sums in another order, one bf16 rounding: 0.4 %)."""
+    def step(place):
+        eng, mbs, groups = _small_engine(recompute)
         for g in groups:
             assert g.collect_in_place
             g.collect_in_place = place
-        def run():
-            for mb in mbs:
-                mb = {k: (v.to(DEV) if torch.is_tensor(v) else v) for k, v in mb.items()}
-                out = eng.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb["cu_seqlens"], max_seqlen=mb["max_seqlen"])
-                out.loss.backward()
-                eng.runner.finish_microbatch()
-        if fail:
-            class Failing:
-                def __getattr__(self, name):
-                    return getattr(fused_blocks_ext, name)
 
-                def attention_block_bwd(self, *a):
-                    raise RuntimeError("refused")
-            fused_blocks_ext, fused_blocks.ext = fused_blocks.ext, Failing()
-            try:
-                with pytest.raises(RuntimeError, match="refused"):
-                    run()
-            finally:
-                fused_blocks.ext = fused_blocks_ext
-            for leaf in eng.runner._root_leaves:
-                leaf.grad = None
-            groups[-1]._collecting = None
-            for p in eng.model.parameters():
-                p.grad = None
-        run()
-        return [g.shard.grad.clone() for g in groups], [p.grad.clone() for p in eng.model.parameters() if p.grad is not None]
-    flat, every = step(True)
-    want, want_every = step(False)
-    assert len(every) == len(want_every)
-    for a, b in zip(flat + every, want + want_every):
-        _close(a, b, 1.5e-2, "gradient")
-    if recompute:
-        again, _ = step(True, fail=True)
-        for a, b in zip(again, flat):
-            _close(a, b, 1e-3, "gradient after a failure")
+        for mb in mbs:
+            _forward(eng, mb).loss.backward()
+            eng.runner.finish_microbatch()
+        return _all_grads(eng, groups)
+    flat, want = step(True), step(False)
+    assert len(flat) == len(want)
+    for a, b in zip(flat, want):
+        _close(a, b, 4e-3, "gradient")
+
+
+@pytest.mark.parametrize("recompute", [True, False])
+@pytest.mark.parametrize("second", [False, True])
+def test_partial_backward_passes_leave_weight_gradients_alone(recompute, second):
+    """A backward pass that is asked for something else, before the one for the weights, does not count towards them, whether there is
+    a flat gradient already or not; and a weight's gradient that is asked for by itself stays what it was."""
+    grads = []
+    for partial in (False, True):
+        eng, mbs, groups = _small_engine(recompute)
+        if second:
+            _forward(eng, mbs[1]).loss.backward()
+            eng.runner.finish_microbatch()
+        out = _forward(eng, mbs[0])
+        if partial:
+            (dh,) = torch.autograd.grad(out.loss, out.hidden_states, retain_graph=True)
+            assert bool(dh.any())
+            head = eng.model.lm_head.weight
+            (dw,) = torch.autograd.grad(out.loss, head, retain_graph=True)
+            kept = dw.clone()
+        out.loss.backward()
+        eng.runner.finish_microbatch()
+        if partial:
+            assert head.grad is None and torch.equal(dw, kept)
+            if not second:
+                place = groups[-1].specs[[m is eng.model.lm_head for m, *_ in groups[-1].specs].index(True)]
+                _close(groups[-1].shard.grad[place[4]:place[4] + place[3]].view(place[2]), kept, 4e-3, "lm_head")
+        grads.append(_all_grads(eng, groups))
+    assert len(grads[0]) == len(grads[1])
+    for a, b in zip(*grads):
+        _close(a, b, 4e-3, "gradient")
+
+
+@pytest.mark.parametrize("recompute", [True, False])
+def test_gradients_of_dense_weights_pass_through_autograd(recompute):
+    """On one rank too: hooks on a weight see its gradient and may change it, and .grad holds the micro-batch's gradient until the
+    micro-batch is finished; the flat gradient is the buffer that the products wrote to where nobody else has a part of it."""
+    eng, mbs, groups = _small_engine(recompute)
+    _forward(eng, mbs[0]).loss.backward()
+    root = [eng.model.lm_head.weight, eng.model.model.embed_tokens.weight]
+    kept = [] if recompute else [getattr(layer.self_attn, n).weight for layer in eng.model.model.layers for n in ("q_proj", "k_proj", "v_proj", "o_proj")]
+    assert all(w.grad is not None and bool(w.grad.any()) for w in root + kept)
+    pointer = root[0].grad.data_ptr()
+    eng.runner.finish_microbatch()
+    flat = groups[-1].shard.grad
+    assert flat.data_ptr() <= pointer < flat.data_ptr() + flat.numel() * flat.element_size()          # (no copy)
+    want = _all_grads(eng, groups)
+    eng, mbs, groups = _small_engine(recompute)
+    with torch.no_grad():
+        _forward(eng, mbs[0])                        # (the weights' views exist from here on)
+    seen = []
+    hooked = [eng.model.lm_head.weight, eng.model.model.embed_tokens.weight, eng.model.model.layers[0].self_attn.q_proj.weight]
+    for w in hooked:
+        w.register_hook(lambda g: (seen.append(g), 2 * g)[1])
+    _forward(eng, mbs[0]).loss.backward()
+    eng.runner.finish_microbatch()
+    assert len(seen) == 3
+    got = _all_grads(eng, groups)
+    for unit, g in enumerate(groups):
+        for i, (mod, name, shape, n, o) in enumerate(g.specs):
+            factor = 2.0 if any(getattr(mod, name) is w for w in hooked) else 1.0
+            _close(got[unit][o:o + n], factor * want[unit][o:o + n].float(), 4e-3, g.qualnames[i])
 
 
 @pytest.mark.parametrize("lora", ["none", "attn-only", "all"])
