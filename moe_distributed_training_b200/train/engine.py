@@ -92,9 +92,13 @@ class Engine:
 
     def forward_backward(self, mb: dict, scale: float):
         mb = self.to_device(mb)
-        out = self.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb.get("cu_seqlens"),
-                         max_seqlen=mb.get("max_seqlen"))
-        (out.loss * scale).backward()
+        try:
+            out = self.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb.get("cu_seqlens"),
+                             max_seqlen=mb.get("max_seqlen"))
+            (out.loss * scale).backward()
+        except BaseException:
+            self.runner.discard_microbatch()     # (a caller that goes on must not find half of its gradients)
+            raise
         self.runner.finish_microbatch()
         return out.loss.detach()
 

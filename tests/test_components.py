@@ -338,6 +338,13 @@ def test_parts_of_the_flat_gradient_are_given_out_once():
         assert torch.equal(g.shard.grad, expected) and torch.equal(held, one(0))
         g.shard.grad.fill_(7.0)
         assert torch.equal(held, one(0))
+    # a micro-batch that failed
+    for drop in (eng.runner.discard_microbatch, eng.runner.zero_grad):
+        eng.optimizer.zero_grad(set_to_none=True)
+        parts(0, 1)
+        drop()
+        assert g._places is None and g.grad_tensor(0) is not None
+        g._places = None
 
 
 def test_expert_gradient_buffers_become_grad_only_once_they_are_written(monkeypatch):

@@ -740,21 +740,49 @@ def _all_grads(eng, groups):
 @pytest.mark.parametrize("recompute", [True, False])
 def test_weight_gradients_collected_in_place(recompute):
     """One rank: products write the dense weights' first gradients in the flat gradient; the same step through ordinary gradient
-    tensors, two micro-batches (sums in another order, one bf16 rounding: 0.4 %)."""
-    def step(place):
+    tensors, two micro-batches (sums in another order, one bf16 rounding: 0.4 %), and again after a backward pass that failed in a
+    block, with the head's gradient written already: nothing of the failed one is left."""
+    from moe_distributed_training_b200.ops import fused_blocks
+
+    def step(place, fail=None):
         eng, mbs, groups = _small_engine(recompute)
         for g in groups:
             assert g.collect_in_place
             g.collect_in_place = place
 
-        for mb in mbs:
-            _forward(eng, mb).loss.backward()
-            eng.runner.finish_microbatch()
+        def run(engine_call):
+            for mb in mbs:
+                if engine_call:
+                    eng.forward_backward(mb, 1.0)
+                else:
+                    _forward(eng, mb).loss.backward()
+                    eng.runner.finish_microbatch()
+        if fail is not None:
+            class Failing:
+                def __getattr__(self, name):
+                    return getattr(fused_blocks_ext, name)
+
+                def attention_block_bwd(self, *a):
+                    raise RuntimeError("refused")
+            fused_blocks_ext, fused_blocks.ext = fused_blocks.ext, Failing()
+            try:
+                with pytest.raises(RuntimeError, match="refused"):
+                    run(fail == "engine")
+            finally:
+                fused_blocks.ext = fused_blocks_ext
+            if fail == "loop":
+                eng.runner.zero_grad()
+            else:
+                eng.optimizer.zero_grad(set_to_none=True)
+        run(False)
         return _all_grads(eng, groups)
     flat, want = step(True), step(False)
     assert len(flat) == len(want)
     for a, b in zip(flat, want):
         _close(a, b, 4e-3, "gradient")
+    for fail in ("engine", "loop"):
+        for a, b in zip(step(True, fail), flat):
+            _close(a, b, 1e-3, f"gradient after a failure ({fail})")
 
 
 @pytest.mark.parametrize("recompute", [True, False])
