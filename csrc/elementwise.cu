@@ -6,6 +6,7 @@
 
 #include "api.h"
 #include "common/host.h"
+#include "common/ptx.cuh"
 
 namespace mdt {
 
@@ -260,43 +261,97 @@ __global__ void embedding_kernel(const bf16* __restrict__ table, const long long
   uint4* dst = reinterpret_cast<uint4*>(out + (long long)blockIdx.x * cols);
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) dst[i] = src[i];
 }
-// Gradient of the table, added to (or written over) the rows of `dtable` that the tokens name.  The tokens of one id form a list
-// (head[id], then next[token]); the CTA of the token at the head adds their rows up in fp32 and rounds once.  A table of
-// 32000 x 4096 in fp32, cleared, added to with atomics and converted, took 198 us however few the tokens; this 9 for 576 of them.
-__global__ void embedding_list_kernel(const long long* __restrict__ ids, int* __restrict__ head, int* __restrict__ next, int tokens) {
+// Gradient of the table: rows that tokens name are written with the sum of their tokens' rows of dout, in fp32 and rounded once (the
+// others are cleared before).  Text is not uniform: most ids have one or two tokens, a filler token may have nearly all.  The
+// first EMB_LIST tokens of an id form a list (head[id], then next[token]) that the CTA of the token at its head adds up.  Later ones are
+// added to a row of fp32 sums that the id gets then, 16 tokens by a CTA, equal ids among them first; the CTA at the head adds that.
+// 32000 x 4096, us, of which clearing the table takes about 75: 576 tokens uniform 87, 90 % of one id 110; 8192 tokens 116 and 136.  Lists
+// of all tokens took 83, 617, 108 and 7630 (one CTA walks them), a table in fp32, added to with atomics and converted, 204 to 286.
+constexpr int EMB_LIST = 32, EMB_LATE = 16, EMB_LATE_MARK = -2;
+__global__ void __launch_bounds__(256) embedding_list_kernel(const long long* __restrict__ ids, int* __restrict__ next, int* __restrict__ head, int* __restrict__ count,
+                                                             int* __restrict__ sum_row, int* __restrict__ sum_rows, float4* __restrict__ sums, long long nv, int tokens) {
   after_predecessor();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < tokens) next[t] = atomicExch(head + ids[t], t);
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) sums[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const long long id = t < tokens ? ids[t] : -1;
+  // (one addition for all lanes of an id; head, count, sum_row and sum_rows start at -1)
+  const unsigned same = __match_any_sync(0xffffffffu, id);
+  const int first = __ffs(same) - 1;
+  int rank = 0;
+  if (id >= 0 && lane == first) rank = atomicAdd(count + id, __popc(same)) + 1;
+  rank = __shfl_sync(0xffffffffu, rank, first) + __popc(same & ((1u << lane) - 1));
+  if (id < 0) return;
+  next[t] = rank < EMB_LIST ? atomicExch(head + id, t) : EMB_LATE_MARK;
+  if (rank == EMB_LIST) sum_row[id] = atomicAdd(sum_rows, 1) + 1;
 }
-template <bool F32>
-__global__ void embedding_bwd_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, const int* __restrict__ head, const int* __restrict__ next,
-                                     void* __restrict__ dtable, int cols, int add) {
+__global__ void __launch_bounds__(256) embedding_late_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, const int* __restrict__ next,
+                                                             const int* __restrict__ sum_row, float* __restrict__ sums, int tokens, int cols) {
+  after_predecessor();
+  __shared__ int rows[EMB_LATE];
+  const int t0 = blockIdx.x * EMB_LATE;
+  int row = -1;
+  if (threadIdx.x < EMB_LATE) {
+    const int t = t0 + threadIdx.x;
+    if (t < tokens && next[t] == EMB_LATE_MARK) row = sum_row[ids[t]];
+    rows[threadIdx.x] = row;
+  }
+  if (!__syncthreads_or(row >= 0)) return;
+  const int col = (blockIdx.y * 256 + threadIdx.x) * 8;
+  if (col >= cols) return;
+  uint4 v[EMB_LATE];
+#pragma unroll
+  for (int i = 0; i < EMB_LATE; ++i)
+    if (rows[i] >= 0) v[i] = *reinterpret_cast<const uint4*>(dout + (long long)(t0 + i) * cols + col);
+#pragma unroll
+  for (int i = 0; i < EMB_LATE; ++i) {
+    const int r = rows[i];
+    bool done = r < 0;
+#pragma unroll
+    for (int j = 0; j < i; ++j) done = done || rows[j] == r;
+    if (done) continue;
+    float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int j = i; j < EMB_LATE; ++j)
+      if (rows[j] == r) {
+        float g[8];
+        unpack8(v[j], g);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] += g[k];
+      }
+    float* to = sums + (long long)r * cols + col;
+    red_add_v4_f32(to, f[0], f[1], f[2], f[3]);
+    red_add_v4_f32(to + 4, f[4], f[5], f[6], f[7]);
+  }
+}
+__global__ void __launch_bounds__(256) embedding_bwd_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, const int* __restrict__ next,
+                                                            const int* __restrict__ head, const int* __restrict__ sum_row, const float* __restrict__ sums,
+                                                            bf16* __restrict__ dtable, int cols) {
   after_predecessor();
   const long long id = ids[blockIdx.x];
   if (head[id] != (int)blockIdx.x) return;
+  __shared__ int list[EMB_LIST], length;
+  if (threadIdx.x == 0) {
+    int n = 0;
+    for (int t = blockIdx.x; t >= 0 && n < EMB_LIST; t = next[t]) list[n++] = t;
+    length = n;
+  }
+  __syncthreads();
+  const int n = length, row = sum_row[id];
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
     float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (add) {
-      if (F32) {
-        const float4* o = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(dtable) + id * cols + i * 8);
-        const float4 x = o[0], y = o[1];
-        f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
-      } else {
-        unpack8(reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(dtable) + id * cols)[i], f);
-      }
+    if (row >= 0) {
+      const float4* o = reinterpret_cast<const float4*>(sums + (long long)row * cols + i * 8);
+      const float4 x = o[0], y = o[1];
+      f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
     }
-    for (int t = blockIdx.x; t >= 0; t = next[t]) {
+#pragma unroll 4
+    for (int k = 0; k < n; ++k) {
       float g[8];
-      unpack8(reinterpret_cast<const uint4*>(dout + (long long)t * cols)[i], g);
+      unpack8(reinterpret_cast<const uint4*>(dout + (long long)list[k] * cols)[i], g);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += g[j];
     }
-    if (F32) {
-      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(dtable) + id * cols + i * 8);
-      o[0] = make_float4(f[0], f[1], f[2], f[3]); o[1] = make_float4(f[4], f[5], f[6], f[7]);
-    } else {
-      reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(dtable) + id * cols)[i] = pack8(f);
-    }
+    reinterpret_cast<uint4*>(dtable + id * cols)[i] = pack8(f);
   }
 }
 
@@ -638,15 +693,23 @@ extern "C" int mdt_embedding(const void* table, const long long* ids, void* out,
   MDT_CHECK_LAUNCH();
   return 0;
 }
-extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int table_fp32, int add, int* scratch, int tokens, int rows, int cols, cudaStream_t s) {
+extern "C" void mdt_embedding_bwd_scratch(int tokens, int rows, int cols, long long* ints, long long* floats) {
+  *ints = (long long)tokens + 3ll * rows + 1;
+  *floats = (long long)(tokens / (EMB_LIST + 1)) * cols;       // ids with more tokens than a list takes
+}
+extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int* scratch, float* sums, int tokens, int rows, int cols, cudaStream_t s) {
   if (cols % 8 != 0) return -1;
   if (tokens == 0) return 0;
-  int* head = scratch + tokens;
-  if (cudaMemsetAsync(head, 0xff, (size_t)rows * sizeof(int), s) != cudaSuccess) return -2;
-  launch_after(embedding_list_kernel, (tokens + 255) / 256, 256, 0, s, ids, head, scratch, tokens);
+  int *next = scratch, *head = next + tokens, *count = head + rows, *sum_row = count + rows, *sum_rows = sum_row + rows;
+  if (cudaMemsetAsync(head, 0xff, (3 * (size_t)rows + 1) * sizeof(int), s) != cudaSuccess) return -2;
+  const int late = tokens / (EMB_LIST + 1);
+  launch_after(embedding_list_kernel, (tokens + 255) / 256, 256, 0, s, ids, next, head, count, sum_row, sum_rows, (float4*)sums, (long long)late * cols / 4, tokens);
   MDT_CHECK_LAUNCH();
-  if (table_fp32) launch_after(embedding_bwd_kernel<true>, tokens, 256, 0, s, (const bf16*)dout, ids, head, scratch, dtable, cols, add);
-  else launch_after(embedding_bwd_kernel<false>, tokens, 256, 0, s, (const bf16*)dout, ids, head, scratch, dtable, cols, add);
+  if (late > 0) {
+    launch_after(embedding_late_kernel, dim3((tokens + EMB_LATE - 1) / EMB_LATE, (cols + 2047) / 2048), 256, 0, s, (const bf16*)dout, ids, next, sum_row, sums, tokens, cols);
+    MDT_CHECK_LAUNCH();
+  }
+  launch_after(embedding_bwd_kernel, tokens, 256, 0, s, (const bf16*)dout, ids, next, head, sum_row, sums, (bf16*)dtable, cols);
   MDT_CHECK_LAUNCH();
   return 0;
 }

@@ -497,7 +497,7 @@ class _Embedding(torch.autograd.Function):
         dtable = ctx.place.tensor() if ctx.place is not None else None
         if dtable is None:
             dtable = torch.empty(ctx.shape, dtype=dout.dtype, device=dout.device)
-        ext.embedding_bwd(dout, ids, dtable, False)
+        ext.embedding_bwd(dout, ids, dtable)
         return None, dtable
 
 
