@@ -104,7 +104,7 @@ __device__ __forceinline__ int find_block(const int* cu, int num_seqs, int token
 
 // ------------------------------------------------------------------------------------------- forward
 __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
-  after_predecessor();
+  wait_for_predecessor();
   int seq_start, seq_end, qb;
   if (find_block(p.cu_seqlens, p.num_seqs, p.tokens, blockIdx.x, seq_start, seq_end, qb, p.status) < 0) return;
   const int h = blockIdx.y, kvh = h / (p.heads_q / p.heads_kv);
@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(128, 1) attn_fwd_kernel(const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  admit_successor();              // (not before TMEM is allocated: a product's CTA could take the columns and wait for this kernel)
   const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);   // this warp's lane quarter
   const int q0 = seq_start + qb * AB;
   const int n_kv = qb + 1;
@@ -278,7 +279,7 @@ __device__ __forceinline__ void load_kv_tile(uint8_t* dst, const CUtensorMap* ma
 }
 
 __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(const __grid_constant__ AttnParams p) {
-  after_predecessor();
+  wait_for_predecessor();
   int seq_start, seq_end, qb;
   if (find_block(p.cu_seqlens, p.num_seqs, p.tokens, blockIdx.x / p.heads_q, seq_start, seq_end, qb, p.status) < 0) return;
   qb = (seq_end - seq_start + AB - 1) / AB - 1 - qb;          // last (longest) block of a sequence first
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  admit_successor();              // (not before TMEM is allocated: a product's CTA could take the columns and wait for this kernel)
   const int q0 = seq_start + qb * AB;
   // key blocks up to the diagonal, and not past the end of the sequence
   const int len = seq_end - seq_start;
@@ -597,7 +599,7 @@ __device__ __forceinline__ uint4 pack8(const uint32_t* a) {
 }
 
 __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
-  after_predecessor();
+  wait_for_predecessor();
   const int sets = p.heads_q / p.hpc, per = sets / p.heads_kv;     // head sets; of one kv head: a cluster of the dK, dV CTAs
   const int kv_ctas = p.blocks * sets;
   const bool is_dq = (int)blockIdx.x >= kv_ctas;
@@ -637,6 +639,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  admit_successor();              // (not before TMEM is allocated: a product's CTA could take the columns and wait for this kernel)
   auto fail = [&](int code) {
     *abort_flag = 1;
     if (p.status != nullptr) atomicCAS(p.status, 0, code);

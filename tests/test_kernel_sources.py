@@ -27,3 +27,21 @@ def test_waits_before_warp_wide_instructions_give_the_warp_one_answer():
     for name in ("gemm_sm100.cu", "attention.cu"):
         lone = [line.strip() for line in _read(name).splitlines() if re.search(r"\bwait_parity\(", line)]
         assert all(re.match(r"(bool )?w = ", line) for line in lone), (name, lone)      # issuing thread of the serial attention forward
+
+
+def test_tensor_memory_is_allocated_before_a_successor_is_admitted():
+    """A kernel that is set up while its predecessor runs allocates TMEM before it waits for it.  If the predecessor still had to allocate
+    on the same SM, each could hold what the other waits for, without a time limit."""
+    admits = r"\b(after_predecessor|admit_successor|gemm_begin)\("
+    seen = 0
+    for name in ("gemm_sm100.cu", "gemm_transposed.cuh", "gemm_wgrad.cuh", "attention.cu"):
+        text = _read(name)
+        # bodies of kernels and of what they share: from a template or __global__ / __device__ line to the brace in the first column
+        for body in re.findall(r"^__(?:global|device)__[^;{]*\{\n(.*?)^\}", text, re.S | re.M):
+            alloc = re.search(r"\btmem_alloc(_pair)?\(", body)
+            if alloc is None:
+                continue
+            seen += 1
+            first = re.search(admits, body)
+            assert first is not None and first.start() > alloc.start(), (name, body[:120])
+    assert seen == sum(len(re.findall(r"\btmem_alloc(?:_pair)?\(", _read(n))) for n in ("gemm_sm100.cu", "gemm_transposed.cuh", "gemm_wgrad.cuh", "attention.cu")) == 8
