@@ -1165,7 +1165,7 @@ extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, co
   cfg.gridDim = dim3((unsigned)(b.blocks * (b.sets + heads_q))); cfg.blockDim = dim3(BWD_THREADS); cfg.dynamicSmemBytes = BWD_SMEM; cfg.stream = s;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].val.programmaticStreamSerializationAllowed = early_setup_pays(cfg.gridDim.x);
   attr[1].id = cudaLaunchAttributeClusterDimension;                                // the sets of a kv head add up their dK, dV
   attr[1].val.clusterDim.x = b.sets / heads_kv; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = b.sets > heads_kv ? 2 : 1;

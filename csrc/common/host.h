@@ -12,17 +12,18 @@ namespace mdt {
 // TMEM is allocated before a successor is admitted: that one allocates too before it waits, and an allocation waits without limit.
 // A two-layer training step is 600 to 900 launches of 2 to 400 microseconds with about 2 us between any two: 19.2 -> 18.7 ms with
 // adapters on attention, 23.0 -> 21.9 with adapters everywhere; logits of a 77-token prompt (42 launches) 1.21 -> 1.14 ms.
-// Grids of many rounds of small CTAs keep plain launches: every CTA would pay for the wait (attention backward of 19 120 tokens, 4 800 and
-// 9 600 CTAs before and after the main kernel: 126 and 95 us plain, 141 and 130).
+// Grids of many rounds of CTAs keep plain launches: every CTA would pay for the wait, which small ones feel (attention backward of
+// 19 120 tokens: the 4 900 CTAs before the main kernel 126 us plain, 141 so; the main kernel's 6 160 CTAs 3.0 to 3.2 ms either way).
 // Kernels that wait for other GPUs or streams keep plain launches (csrc/comm.cu), or do not admit successors early: a successor's CTAs
 // could take the place of those that are waited for.
+inline int early_setup_pays(long long ctas) { return ctas <= 2048 ? 1 : 0; }
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = (unsigned long long)grid.x * grid.y * grid.z <= 2048 ? 1 : 0;
+  attr.val.programmaticStreamSerializationAllowed = early_setup_pays((long long)grid.x * grid.y * grid.z);
   cfg.attrs = &attr; cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }

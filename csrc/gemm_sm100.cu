@@ -1610,7 +1610,7 @@ static cudaError_t launch_cluster(const GemmParams& p, int tiles, int S, cudaStr
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;         // (see launch_after)
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].val.programmaticStreamSerializationAllowed = early_setup_pays(cfg.gridDim.x);
   cfg.attrs = attr; cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_cluster_kernel<BN>, p);
   ++g_launches;
@@ -1786,7 +1786,7 @@ static int launch_list(const MdtGemmDesc* d, int n, cudaStream_t stream) {
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = S; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;         // (see launch_after)
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].val.programmaticStreamSerializationAllowed = early_setup_pays(cfg.gridDim.x);
   cfg.attrs = attr; cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_sm100_list_kernel<BN>, list);
   ++g_launches;

@@ -45,3 +45,11 @@ def test_tensor_memory_is_allocated_before_a_successor_is_admitted():
             first = re.search(admits, body)
             assert first is not None and first.start() > alloc.start(), (name, body[:120])
     assert seen == sum(len(re.findall(r"\btmem_alloc(?:_pair)?\(", _read(n))) for n in ("gemm_sm100.cu", "gemm_transposed.cuh", "gemm_wgrad.cuh", "attention.cu")) == 8
+
+
+def test_every_launch_follows_one_rule_for_early_set_up():
+    """Programmatic launch pays for grids of up to a number of CTAs: no launcher sets it by itself."""
+    for name in sorted(os.listdir(CSRC)) + [os.path.join("common", "host.h")]:
+        if name.endswith((".cu", ".cuh", ".h", ".cpp")):
+            for value in re.findall(r"programmaticStreamSerializationAllowed = ([^;]*);", _read(name)):
+                assert value.startswith("early_setup_pays("), (name, value)
