@@ -208,8 +208,8 @@ class _MoEBlock(torch.autograd.Function):
         with torch.set_grad_enabled(grad_mode):
             w1, w2, w3, lora, ws, wgrad_out = mlp.call_args(xn)
         # experts' own autograd body, run directly
-        mneeds = [grad_mode, need[4], need[5], need[6], False, False, False, False, False] + [need[7 + i] for i in range(len(lora_tensors))]
-        mctx = _Ctx(mneeds)
+        mneeds = [True, need[4], need[5], need[6], False, False, False, False, False] + [need[7 + i] for i in range(len(lora_tensors))]
+        mctx = _Ctx(grad_mode and n for n in mneeds)
         ids = tuple(id(t) for t in lora_tensors)
         ep = ex.ep_group is not None and ex.ep_size > 1
         # A block that is recomputed in the backward pass (layer._ckpt_mode, see _MoEBlockNative) keeps routing, grouped rows, expert

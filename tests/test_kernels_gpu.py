@@ -849,6 +849,32 @@ def test_gradients_of_dense_weights_pass_through_autograd(recompute):
             _close(got[unit][o:o + n], factor * want[unit][o:o + n].float(), 4e-3, g.qualnames[i])
 
 
+def test_adapter_blocks_store_gate_and_up_only_for_a_graph(ops, monkeypatch):
+    """Passes without a graph (evaluation, the first pass of recomputed blocks) leave the inputs of SwiGLU unwritten, trainable adapters or not."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
+    from moe_distributed_training_b200.train.engine import build_engine
+    cfg = MixtralConfig(vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=2, num_key_value_heads=1,
+                        head_dim=128, num_local_experts=4, num_experts_per_tok=2)
+    eng = build_engine(cfg, dtype=torch.bfloat16, device_type="cuda", learning_rate=1e-3, seed=0, use_lora="all")
+    (mb,) = list(batches(SyntheticInstructionDataset(cfg.vocab_size, 1, 60, 150), 1))
+    stored, real = [], ops._gemm
+
+    def spy(*a, **kw):
+        if kw.get("B2") is not None:
+            stored.append(kw.get("C2") is not None)
+        return real(*a, **kw)
+    monkeypatch.setattr(ops, "_gemm", spy)
+    before = eng.eval_loss(mb)
+    assert stored == [False, False]
+    stored.clear()
+    loss = eng.forward_backward(mb, 1.0)
+    assert stored == [False, False, True, True]
+    _close(before, loss, 1e-5, "loss")
+    assert all(bool(p.grad.any()) for n, p in eng.model.named_parameters() if "lora_B" in n and p.grad is not None)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("lora", ["none", "attn-only", "all"])
 @pytest.mark.parametrize("keep", [True, False])
 def test_two_micro_batches_before_their_backward_pass(lora, keep):
