@@ -105,10 +105,11 @@ int mdt_rope(const void* x, void* y, const int* positions, int tokens, int heads
 int mdt_copy_rows_used(const void* src, void* dst, long long n, const int* rows_used, long long cols, cudaStream_t s);
 int mdt_swiglu_fwd(const void* g, const void* u, void* h, long long n, cudaStream_t s);
 int mdt_embedding(const void* table, const long long* ids, void* out, int tokens, int cols, cudaStream_t s);
-// rows of dtable (bf16, [rows, cols]) that ids names are written with the sum of their tokens' rows of dout; other rows are left alone.
-// scratch, sums: as many ints and floats (16-byte aligned) as mdt_embedding_bwd_scratch says
+// rows of dtable (bf16 or fp32, [rows, cols]) that ids names: written with, or (add) increased by, the sum of their tokens' rows of
+// dout; other rows are left alone.  scratch, sums: as many ints and floats (16-byte aligned) as mdt_embedding_bwd_scratch says
 void mdt_embedding_bwd_scratch(int tokens, int rows, int cols, long long* ints, long long* floats);
-int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int* scratch, float* sums, int tokens, int rows, int cols, cudaStream_t s);
+int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int table_fp32, int add, int* scratch, float* sums, int tokens, int rows, int cols,
+                      cudaStream_t s);
 // A13 [E, H, 2r] = [s1 A1 | s3 A3], B1p = [B1^T | 0] and B3p = [0 | B3^T], both [E, F, 2r], from A [E, H, r], B [E, r, F]; r a multiple of 4
 int mdt_adapter_pack(const void* A1, const void* A3, float s1, float s3, const void* B1, const void* B3, void* A13, void* B1p, void* B3p, int E, int H,
                      int F, int r, cudaStream_t s);

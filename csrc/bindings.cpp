@@ -238,20 +238,21 @@ Tensor embedding(const Tensor& table, const Tensor& ids) {
   check(mdt_embedding(table.data_ptr(), ids.data_ptr<int64_t>() ? (const long long*)ids.data_ptr<int64_t>() : nullptr, out.data_ptr(), (int)ids.numel(), (int)table.size(1), cur_stream()), "embedding");
   return out;
 }
-// gradient of the embedding table (rows that no token names are cleared)
-void embedding_bwd(const Tensor& dout, const Tensor& ids, Tensor& dtable) {
-  CHECK_BF16(dout); CHECK_BF16(dtable);
+// add: to what the table's gradient holds; otherwise rows that no token names are cleared
+void embedding_bwd(const Tensor& dout, const Tensor& ids, Tensor& dtable, bool add) {
+  CHECK_BF16(dout);
   c10::cuda::CUDAGuard guard(dout.device());
   TORCH_CHECK(ids.scalar_type() == at::kLong && ids.is_contiguous() && dout.is_contiguous() && dtable.is_contiguous() && dtable.dim() == 2 &&
+              dtable.is_cuda() && (dtable.scalar_type() == at::kFloat || dtable.scalar_type() == at::kBFloat16) &&
               dout.numel() == ids.numel() * dtable.size(1), "embedding_bwd: a row of dout for every id, as wide as the table's");
   for (const Tensor* t : {&dout, (const Tensor*)&dtable}) TORCH_CHECK((reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0, "embedding_bwd: rows must be 16-byte aligned");
-  dtable.zero_();
+  if (!add) dtable.zero_();
   long long ints = 0, floats = 0;
   mdt_embedding_bwd_scratch((int)ids.numel(), (int)dtable.size(0), (int)dtable.size(1), &ints, &floats);
   auto scratch = torch::empty({ints}, ids.options().dtype(at::kInt));
   auto sums = torch::empty({floats}, ids.options().dtype(at::kFloat));
-  check(mdt_embedding_bwd(dout.data_ptr(), (const long long*)ids.data_ptr<int64_t>(), dtable.data_ptr(), scratch.data_ptr<int>(), sums.data_ptr<float>(),
-                          (int)ids.numel(), (int)dtable.size(0), (int)dtable.size(1), cur_stream()), "embedding_bwd");
+  check(mdt_embedding_bwd(dout.data_ptr(), (const long long*)ids.data_ptr<int64_t>(), dtable.data_ptr(), dtable.scalar_type() == at::kFloat, add ? 1 : 0,
+                          scratch.data_ptr<int>(), sums.data_ptr<float>(), (int)ids.numel(), (int)dtable.size(0), (int)dtable.size(1), cur_stream()), "embedding_bwd");
 }
 // gate and up adapters as the expert products want them: {A13, B1p, B3p} (see api.h)
 std::vector<Tensor> adapter_pack(const Tensor& A1, const Tensor& A3, double s1, double s3, const Tensor& B1, const Tensor& B3) {
@@ -1048,7 +1049,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rope", &rope);
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("embedding", &embedding);
-  m.def("embedding_bwd", &embedding_bwd);
+  m.def("embedding_bwd", &embedding_bwd, py::arg("dout"), py::arg("ids"), py::arg("dtable"), py::arg("add") = false);
   m.def("adapter_pack", &adapter_pack);
   m.def("cross_entropy", &cross_entropy);
   m.def("gemm_set_pair_policy", [](int64_t policy) { return (int64_t)mdt_gemm_set_pair_policy((int)policy); });

@@ -261,8 +261,8 @@ __global__ void embedding_kernel(const bf16* __restrict__ table, const long long
   uint4* dst = reinterpret_cast<uint4*>(out + (long long)blockIdx.x * cols);
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) dst[i] = src[i];
 }
-// Gradient of the table: rows that tokens name are written with the sum of their tokens' rows of dout, in fp32 and rounded once (the
-// others are cleared before).  Text is not uniform: most ids have one or two tokens, a filler token may have nearly all.  The
+// Gradient of the table: rows that tokens name are written with, or (add) increased by, the sum of their tokens' rows of dout, in fp32
+// and rounded once (the others are left alone).  Text is not uniform: most ids have one or two tokens, a filler token may have nearly all.  The
 // first EMB_LIST tokens of an id form a list (head[id], then next[token]) that the CTA of the token at its head adds up.  Later ones are
 // added to a row of fp32 sums that the id gets then, 16 tokens by a CTA, equal ids among them first; the CTA at the head adds that.
 // 32000 x 4096, us, of which clearing the table takes about 75: 576 tokens uniform 87, 90 % of one id 110; 8192 tokens 116 and 136.  Lists
@@ -323,9 +323,10 @@ __global__ void __launch_bounds__(256) embedding_late_kernel(const bf16* __restr
     red_add_v4_f32(to + 4, f[4], f[5], f[6], f[7]);
   }
 }
+template <bool F32>
 __global__ void __launch_bounds__(256) embedding_bwd_kernel(const bf16* __restrict__ dout, const long long* __restrict__ ids, const int* __restrict__ next,
                                                             const int* __restrict__ head, const int* __restrict__ sum_row, const float* __restrict__ sums,
-                                                            bf16* __restrict__ dtable, int cols) {
+                                                            void* __restrict__ dtable, int cols, int add) {
   after_predecessor();
   const long long id = ids[blockIdx.x];
   if (head[id] != (int)blockIdx.x) return;
@@ -339,11 +340,16 @@ __global__ void __launch_bounds__(256) embedding_bwd_kernel(const bf16* __restri
   const int n = length, row = sum_row[id];
   for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
     float f[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (row >= 0) {
-      const float4* o = reinterpret_cast<const float4*>(sums + (long long)row * cols + i * 8);
-      const float4 x = o[0], y = o[1];
-      f[0] = x.x; f[1] = x.y; f[2] = x.z; f[3] = x.w; f[4] = y.x; f[5] = y.y; f[6] = y.z; f[7] = y.w;
+    auto plus = [&](const float* src) {
+      const float4 x = reinterpret_cast<const float4*>(src)[0], y = reinterpret_cast<const float4*>(src)[1];
+      f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w; f[4] += y.x; f[5] += y.y; f[6] += y.z; f[7] += y.w;
+    };
+    const long long at = id * cols + i * 8;
+    if (add) {
+      if (F32) plus(reinterpret_cast<const float*>(dtable) + at);
+      else unpack8(*reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(dtable) + at), f);
     }
+    if (row >= 0) plus(sums + (long long)row * cols + i * 8);
 #pragma unroll 4
     for (int k = 0; k < n; ++k) {
       float g[8];
@@ -351,7 +357,12 @@ __global__ void __launch_bounds__(256) embedding_bwd_kernel(const bf16* __restri
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += g[j];
     }
-    reinterpret_cast<uint4*>(dtable + id * cols)[i] = pack8(f);
+    if (F32) {
+      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(dtable) + at);
+      o[0] = make_float4(f[0], f[1], f[2], f[3]); o[1] = make_float4(f[4], f[5], f[6], f[7]);
+    } else {
+      *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(dtable) + at) = pack8(f);
+    }
   }
 }
 
@@ -697,7 +708,8 @@ extern "C" void mdt_embedding_bwd_scratch(int tokens, int rows, int cols, long l
   *ints = (long long)tokens + 3ll * rows + 1;
   *floats = (long long)(tokens / (EMB_LIST + 1)) * cols;       // ids with more tokens than a list takes
 }
-extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int* scratch, float* sums, int tokens, int rows, int cols, cudaStream_t s) {
+extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* dtable, int table_fp32, int add, int* scratch, float* sums, int tokens, int rows, int cols,
+                                 cudaStream_t s) {
   if (cols % 8 != 0) return -1;
   if (tokens == 0) return 0;
   int *next = scratch, *head = next + tokens, *count = head + rows, *sum_row = count + rows, *sum_rows = sum_row + rows;
@@ -709,7 +721,8 @@ extern "C" int mdt_embedding_bwd(const void* dout, const long long* ids, void* d
     launch_after(embedding_late_kernel, dim3((tokens + EMB_LATE - 1) / EMB_LATE, (cols + 2047) / 2048), 256, 0, s, (const bf16*)dout, ids, next, sum_row, sums, tokens, cols);
     MDT_CHECK_LAUNCH();
   }
-  launch_after(embedding_bwd_kernel, tokens, 256, 0, s, (const bf16*)dout, ids, next, head, sum_row, sums, (bf16*)dtable, cols);
+  if (table_fp32) launch_after(embedding_bwd_kernel<true>, tokens, 256, 0, s, (const bf16*)dout, ids, next, head, sum_row, sums, dtable, cols, add);
+  else launch_after(embedding_bwd_kernel<false>, tokens, 256, 0, s, (const bf16*)dout, ids, next, head, sum_row, sums, dtable, cols, add);
   MDT_CHECK_LAUNCH();
   return 0;
 }

@@ -279,7 +279,8 @@ def test_gemm_default_tiling_follows_rounds_and_row_groups():
 @pytest.mark.parametrize("seqs,length", [(1, 1), (1, 613), (4, 4375), (40, 130), (1024, 8), (4096, 1), (300, 129)])
 @pytest.mark.parametrize("heads,kv", [(32, 8), (8, 8), (4, 1)])
 def test_attention_backward_scratch_grows_with_tokens_not_with_sequences(seqs, length, heads, kv):
-    """The row statistics (256 floats per block and query head) and the schedule, no more, however short the sequences are."""
+    """At most fp32 dQ, dK and dV of every (token, query head) plus the row statistics (256 floats per block and head) and
+    the schedule, however short the sequences are."""
     build = pytest.importorskip("moe_distributed_training_b200.ops.build")
     try:
         ext = build.load()
@@ -288,7 +289,22 @@ def test_attention_backward_scratch_grows_with_tokens_not_with_sequences(seqs, l
     T = seqs * length
     blocks = (T + 127) // 128 + seqs
     floats = ext.attention_bwd_scratch(seqs, T, length, heads, kv)
-    assert floats <= 256 * blocks * heads + 4 * blocks + 32
+    assert floats <= 3 * 128 * T * heads + 256 * blocks * heads + 4 * blocks + 32
+    assert floats <= 1.01 * (1 + 3 * 128) * T * heads + 256 * 2 * heads + 64
+
+
+@pytest.mark.parametrize("seqs,length", [(1, 1), (1, 613), (4, 4375), (40, 130), (1024, 8), (4096, 1), (300, 129)])
+@pytest.mark.parametrize("heads,kv", [(32, 8), (8, 8), (4, 1)])
+def test_attention_backward_scratch_holds_statistics_and_schedule_only(seqs, length, heads, kv):
+    """The row statistics (256 floats per block and query head) and the schedule, no more, however short the sequences are."""
+    build = pytest.importorskip("moe_distributed_training_b200.ops.build")
+    try:
+        ext = build.load()
+    except Exception as e:
+        pytest.skip(f"extension not built: {e}")
+    T = seqs * length
+    blocks = (T + 127) // 128 + seqs
+    assert ext.attention_bwd_scratch(seqs, T, length, heads, kv) <= 256 * blocks * heads + 4 * blocks + 32
 
 
 def test_parts_of_the_flat_gradient_are_given_out_once():

@@ -271,8 +271,8 @@ def test_swiglu_backward_in_the_product(ops, T, E, H, F, policy):
 def test_transposed_pair_kernel(ops, counts, H, F):
     """Weights as the 256-row operand, rows of every group counted exactly: remainders of the 32-row units, of 256-row tiles
     and 8-tile panels, of feature tiles and of the depth; gate / up with and without its outputs and with adapters, SwiGLU
-    backward, K-major and MN-major weights, two depth segments.  fp32 reference, one bf16 rounding of each result (2e-2 as
-    for the other products); padding becomes zeros, rows past the groups stay untouched."""
+    backward, K-major and MN-major weights, two depth segments; shared last rounds (2100 rows).  fp32 reference, one bf16
+    rounding of each result (2e-2 as for the other products); padding becomes zeros, rows past the groups stay untouched."""
     torch.manual_seed(sum(counts) + F)
     E, r = len(counts), 16
     ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(sum(counts))].to(DEV).int()
@@ -382,7 +382,7 @@ def test_dense_products_of_odd_row_counts(ops, M, N, K):
                                           ([211, 281, 92, 321, 302, 269, 245, 279], 14336)])
 def test_transposed_pair_kernel_with_two_accumulators(ops, counts, depth):
     """Depths and numbers of tiles at which tiles of more than 256 rows are taken (tests/host/tile_enumeration.cu has the choice):
-    both accumulators equal and not, beside tiles of one, K-major and MN-major weights
+    both accumulators equal and not, beside tiles of one, with and without a last round that is shared, K-major and MN-major weights
     and two depth segments.  fp32 reference, 2e-2 as above; padding becomes zeros."""
     torch.manual_seed(depth)
     E, N, r = len(counts), 4096, 16
@@ -696,6 +696,27 @@ def test_router(ops):
     _close(w.grad, wr.grad, 3e-2, "router dw")
 
 
+@pytest.mark.parametrize("T,V,H,repeat", [(1, 8, 8, 1), (300, 40, 264, 1), (700, 2048, 4096, 1), (64, 4, 1032, 16)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_embedding_gradient_written_and_added(ops, T, V, H, repeat, dtype):
+    """Table gradients by lists of equal ids: fp32 sums, one rounding (bf16: 0.4 %; fp32: the order of up to T additions)."""
+    torch.manual_seed(T + V)
+    ids = torch.randint(0, max(V // repeat, 1), (T,), device=DEV)
+    d = _rand(T, H)
+    old = _rand(V, H).to(dtype)
+    want = torch.zeros(V, H, device=DEV, dtype=torch.float64).index_add_(0, ids, d.double())
+    out = torch.full((V, H), float("nan"), device=DEV, dtype=dtype)
+    tol = 1e-2 if dtype == torch.bfloat16 else 1e-5
+    ops.ext.embedding_bwd(d, ids, out, False)
+    _close(out, want, tol, "written")
+    out = old.clone()
+    ops.ext.embedding_bwd(d, ids, out, True)
+    _close(out, old.double() + want, tol, "added")
+    untouched = torch.ones(V, dtype=torch.bool, device=DEV)
+    untouched[ids] = False
+    assert torch.equal(out[untouched], old[untouched])
+
+
 @pytest.mark.parametrize("T,V,H,hot", [(1, 8, 8, 0.0), (300, 40, 264, 0.0), (700, 2048, 4096, 0.0), (64, 4, 1032, 0.0), (32, 3, 16, 1.0), (33, 3, 2048, 1.0),
                                        (34, 3, 2056, 1.0), (257, 5, 520, 0.3), (2000, 7, 264, 0.0), (8192, 1000, 4096, 0.9)])
 def test_embedding_gradient(ops, T, V, H, hot):
@@ -719,6 +740,63 @@ def test_embedding_gradient(ops, T, V, H, hot):
         ops.ext.embedding_bwd(_rand(T + 1, H), ids, out)
 
 
+@pytest.mark.parametrize("recompute", [True, False])
+def test_weight_gradients_collected_in_place(recompute):
+    """One rank: products write or add the dense weights' gradients in the flat gradient; the same step through ordinary gradient
+    tensors, two micro-batches (each of the latter's gradients is rounded once more, 0.4 % each), and again after a backward pass that
+    failed in a block."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
+    from moe_distributed_training_b200.ops import fused_blocks
+    from moe_distributed_training_b200.train.engine import build_engine
+    cfg = MixtralConfig(vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=2, num_key_value_heads=1,
+                        head_dim=128, num_local_experts=4, num_experts_per_tok=2)
+    mbs = list(batches(SyntheticInstructionDataset(cfg.vocab_size, 2, 60, 150), 1))
+
+    def step(place, fail=False):
+        eng = build_engine(cfg, dtype=torch.bfloat16, device_type="cuda", learning_rate=1e-3, seed=0, activation_checkpointing=recompute)
+        assert eng.runner.recompute == recompute
+        groups = [u.trainable_group for u in eng.runner.all_units()]
+        for g in groups:
+            assert g.collect_in_place
+            g.collect_in_place = place
+        def run():
+            for mb in mbs:
+                mb = {k: (v.to(DEV) if torch.is_tensor(v) else v) for k, v in mb.items()}
+                out = eng.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb["cu_seqlens"], max_seqlen=mb["max_seqlen"])
+                out.loss.backward()
+                eng.runner.finish_microbatch()
+        if fail:
+            class Failing:
+                def __getattr__(self, name):
+                    return getattr(fused_blocks_ext, name)
+
+                def attention_block_bwd(self, *a):
+                    raise RuntimeError("refused")
+            fused_blocks_ext, fused_blocks.ext = fused_blocks.ext, Failing()
+            try:
+                with pytest.raises(RuntimeError, match="refused"):
+                    run()
+            finally:
+                fused_blocks.ext = fused_blocks_ext
+            for leaf in eng.runner._root_leaves:
+                leaf.grad = None
+            groups[-1]._collecting = None
+            for p in eng.model.parameters():
+                p.grad = None
+        run()
+        return [g.shard.grad.clone() for g in groups], [p.grad.clone() for p in eng.model.parameters() if p.grad is not None]
+    flat, every = step(True)
+    want, want_every = step(False)
+    assert len(every) == len(want_every)
+    for a, b in zip(flat + every, want + want_every):
+        _close(a, b, 1.5e-2, "gradient")
+    if recompute:
+        again, _ = step(True, fail=True)
+        for a, b in zip(again, flat):
+            _close(a, b, 1e-3, "gradient after a failure")
+
+
 def _small_engine(recompute):
     from moe_distributed_training_b200 import MixtralConfig
     from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
@@ -740,7 +818,7 @@ def _all_grads(eng, groups):
 
 
 @pytest.mark.parametrize("recompute", [True, False])
-def test_weight_gradients_collected_in_place(recompute):
+def test_first_weight_gradients_are_written_in_place(recompute):
     """One rank: products write the dense weights' first gradients in the flat gradient; the same step through ordinary gradient
     tensors, two micro-batches (sums in another order, one bf16 rounding: 0.4 %), and again after a backward pass that failed in a
     block, with the head's gradient written already: nothing of the failed one is left."""
