@@ -26,8 +26,9 @@ constexpr int TP_A_BYTES = BM * BK * 2;
 // products of few rows is the bytes of weights in flight.
 constexpr int TP_RING_BYTES = 6 * (TP_A_BYTES + 128 * BK * 2);
 constexpr int TP_MAX_STAGES = 10;
-// (groups in the order of the rows of their tiles, most first: see tp_work)
-struct TPTable { int group[TP_GROUPS], start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, cap; };
+// (groups in the order of the rows of their tiles, most first: see tp_work; units, groups, row_tiles: totals that the host check of the
+// enumeration keeps)
+struct TPTable { int group[TP_GROUPS], start[TP_GROUPS], rows[TP_GROUPS], end[TP_GROUPS], tile0[TP_GROUPS + 1], widest, units, groups, row_tiles, cap; };
 constexpr int TP_SMEM = TP_RING_BYTES + 1024 + 256 + EPI_WARPS * EPI_STAGE_BYTES + (int)sizeof(TPTable);
 static_assert(TP_SMEM <= 227 * 1024, "transposed pair kernel: shared memory of a CTA");
 
@@ -46,6 +47,8 @@ struct TPParams {
 };
 // rows [row0, row0 + n) x features [f0, f0 + 256 or 128), rows below `end` are stored; zero0: first row to be cleared (= end: none)
 struct TPTile { int g, f0, row0, n, end, zero0; };
+// A pair's work: a tile and its k blocks.  No tile is shared along the depth, so these are all of them: split < 0, one contributor.
+struct TPWork { TPTile t; int kb0, kb1, split, contributors; };
 
 __host__ __device__ __forceinline__ int tp_tiles_of_rows(int rows, int cap) { return ((rows + TP_UNIT - 1) / TP_UNIT + cap - 1) / cap; }
 // rows of its widest tile
@@ -74,7 +77,7 @@ __host__ __device__ __forceinline__ float tp_clocks_of_all(int row_tiles, int f_
 // depth 4096 151 / 140 run with the slower.  Not for more than one result a product: gate and up of 2000 tokens 892 / 937, with
 // their inputs kept of 9200 3320 / 3856, SwiGLU backward 1896 / 2704.
 struct TPForm { int row_tiles; float step, longest; };
-__host__ __device__ __forceinline__ bool tp_joint_pays(const TPForm& one, const TPForm& two, int units, int f_tiles, int pairs, int kbt) {
+__host__ __device__ __forceinline__ bool tp_joint_pays(const TPForm& one, const TPForm& two, int units, int f_tiles, int pairs, int kbt, bool = false) {
   if (two.row_tiles == one.row_tiles || two.row_tiles == 0) return false;
   const float rows = 32.f * (float)units;
   const float a = tp_clocks_of_all(one.row_tiles, f_tiles, pairs, kbt, one.step / (float)one.row_tiles, one.longest, rows / (float)one.row_tiles, 0.f);
@@ -164,10 +167,12 @@ __host__ __device__ __forceinline__ void tp_tile(const TPTable* tb, int G, int f
 // it = 0, 1, ...: the tile of pair `pair` of `pairs`.  The tiles come by their rows, most first, and every second round goes through
 // the pairs backwards, so that all have about the same to do (us, groups in their own order, each round forwards /
 // so: SwiGLU backward of 600 tokens 226 / 214, down 1000 tokens 271 / 261, dx 527 / 513).
-__host__ __device__ __forceinline__ bool tp_work(const TPTable* tb, int G, int f_tiles, int f_width, int pair, int pairs, int it, TPTile& t) {
+// (The unnamed flags here and in tp_joint_pays asked for a last round shared along the depth; its sums came in any order.)
+__host__ __device__ __forceinline__ bool tp_work(const TPTable* tb, int G, int f_tiles, int f_width, int kbt, bool, int pair, int pairs, int it, TPWork& w) {
   const int i = it * pairs + (it & 1 ? pairs - 1 - pair : pair);
   if (i >= tb->tile0[G]) return false;
-  tp_tile(tb, G, f_tiles, f_width, i, t);
+  tp_tile(tb, G, f_tiles, f_width, i, w.t);
+  w.kb0 = 0; w.kb1 = kbt; w.split = -1; w.contributors = 1;
   return true;
 }
 
@@ -349,8 +354,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     *abort_flag = 1;
     if (p.status != nullptr) atomicCAS(p.status, 0, code);
   };
-  TPTile w;
-  auto next = [&](int it) { return tp_work(tb, p.G, f_tiles, F_WIDTH, pair_id, num_pairs, it, w); };
+  TPWork w;
+  auto next = [&](int it) { return tp_work(tb, p.G, f_tiles, F_WIDTH, kbt, false, pair_id, num_pairs, it, w); };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (one per CTA)
@@ -359,7 +364,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     uint32_t ph = 0;
     bool ok = true;
     for (int wi = 0; ok && next(wi); ++wi) {
-      const TPTile& t = w;
+      const TPTile& t = w.t;
       const int f0 = t.f0 + rank * (F_WIDTH / 2);
       const uint32_t bytes = 2 * (TP_A_BYTES + t.n / 2 * (BK * 2));
       // (a loop for each of one and two accumulators, here and in the issuer: with the choice inside, tiles of 256 rows took 25 % longer)
@@ -417,7 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     bool ok = true;
     for (int wi = 0; ok && next(wi); ++wi) {
       auto multiply = [&](auto two) {
-        const int n0 = decltype(two)::value ? tp_first(w.n) : w.n, n1 = w.n - n0, buf = acc_it & 1;
+        const int n0 = decltype(two)::value ? tp_first(w.t.n) : w.t.n, n1 = w.t.n - n0, buf = acc_it & 1;
         if (!wait_parity_warp(&tempty_bar[buf], ((acc_it >> 1) & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); ok = false; return; }
         if (decltype(two)::value && !wait_parity_warp(&tempty_bar[buf ^ 1], (((acc_it + 1) >> 1) & 1) ^ 1, abort_flag)) { fail(ST_TIMEOUT_TMEM_EMPTY); ok = false; return; }
         tc_fence_after();
@@ -451,7 +456,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
         }
         acc_it += decltype(two)::value ? 2 : 1;
       };
-      if (!JOINT || w.n <= 256) multiply(std::false_type());
+      if (!JOINT || w.t.n <= 256) multiply(std::false_type());
       else multiply(std::integral_constant<bool, JOINT>());
     }
   } else if (warp >= 2) {
@@ -463,7 +468,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1) gem
     bool ok = true;
     for (int wi = 0, sub = 0; ok && (sub > 0 || next(wi)); sub > 0 ? 0 : ++wi) {
       // (a tile of more than 256 rows: its two accumulators one after the other)
-      TPTile t = w;
+      TPTile t = w.t;
       const int mine = sub;
       if (JOINT) {
         const int n0 = tp_first(t.n);

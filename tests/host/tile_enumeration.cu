@@ -95,14 +95,14 @@ static int check_work(const GemmParams& p, int num_ctas, const std::vector<int>&
   return bad;
 }
 
-// The transposed pair kernel (tp_work): every (32-row unit, feature tile) of the rows that exist exactly once, in a tile of one pair;
-// tiles inside their group; the padding of a group cleared by exactly one whole column of tiles.
-static int check_transposed(const std::vector<int>& start, const std::vector<int>& rows, const std::vector<int>& end, int N, int f_width, int pairs, int cap) {
+// The transposed pair kernel (tp_work): every (32-row unit, feature tile, k block) of the rows that exist exactly once; tiles inside
+// their group; the padding of a group cleared by exactly one whole column of tiles; shared tiles as above, one per pair at most.
+static int check_transposed(const std::vector<int>& start, const std::vector<int>& rows, const std::vector<int>& end, int N, int f_width, int kbt, int pairs, bool split, int cap) {
   TPTable tb;
   tb.cap = cap;
   const int G = (int)rows.size(), f_tiles = (N + f_width - 1) / f_width;
   int tiles = 0;
-  tb.widest = 0;
+  tb.widest = tb.units = tb.groups = 0;
   std::vector<int> order(G);
   for (int g = 0; g < G; ++g) order[g] = g;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return tp_tile_rows(rows[a], cap) > tp_tile_rows(rows[b], cap); });
@@ -111,28 +111,46 @@ static int check_transposed(const std::vector<int>& start, const std::vector<int
     tb.group[i] = g; tb.start[i] = start[g]; tb.rows[i] = rows[g]; tb.end[i] = end[g]; tb.tile0[i] = tiles;
     if (nt != tp_tiles_of_rows(rows[g], cap)) return 1;
     tiles += nt * f_tiles;
-    if (nt > 0) { const int w = (units + nt - 1) / nt * TP_UNIT; if (w > tb.widest) tb.widest = w; if (w != tp_tile_rows(rows[g], cap)) return 1; }
+    tb.units += units;
+    if (nt > 0) { ++tb.groups; const int w = (units + nt - 1) / nt * TP_UNIT; if (w > tb.widest) tb.widest = w; if (w != tp_tile_rows(rows[g], cap)) return 1; }
   }
   tb.tile0[G] = tiles;
+  tb.row_tiles = tiles / f_tiles;
   const int top = G ? end[G - 1] : 0, units = (top + TP_UNIT - 1) / TP_UNIT + 1;
-  std::vector<int> seen((size_t)units * f_tiles, 0), cleared((size_t)(top + 1) * f_tiles, 0);
+  std::vector<int> seen((size_t)units * f_tiles * kbt, 0), cleared((size_t)(top + 1) * f_tiles, 0), pieces(pairs + 1, 0), claimed(pairs + 1, 0);
   int bad = 0;
   for (int p = 0; p < pairs; ++p) {
-    TPTile t;
-    for (int it = 0; tp_work(&tb, G, f_tiles, f_width, p, pairs, it, t); ++it) {
+    int shared = 0;
+    for (int it = 0;; ++it) {
+      TPWork w;
+      if (!tp_work(&tb, G, f_tiles, f_width, kbt, split, p, pairs, it, w)) break;
       if (it > tiles + 4) { printf("work list does not end\n"); return 1; }
+      const TPTile& t = w.t;
       const int n0 = tp_first(t.n);        // first accumulator; the rest is the second
       if (t.n < TP_UNIT || t.n > 32 * cap || t.n % TP_UNIT || n0 > 256 || n0 % TP_UNIT || t.n - n0 > 256 || (t.n > 256) != (t.n > n0) || t.n > tb.widest || t.f0 % f_width || t.f0 >= N || t.g >= G || t.row0 < start[t.g] ||
-          (t.row0 - start[t.g]) % TP_UNIT || t.row0 - start[t.g] >= rows[t.g] || t.end != end[t.g]) { ++bad; continue; }
-      for (int u = 0; u < t.n / TP_UNIT; ++u) seen[(size_t)(t.row0 / TP_UNIT + u) * f_tiles + t.f0 / f_width] += 1;
-      for (int r = t.zero0; r < t.end; ++r) cleared[(size_t)r * f_tiles + t.f0 / f_width] += 1;
+          (t.row0 - start[t.g]) % TP_UNIT || t.row0 - start[t.g] >= rows[t.g] || t.end != end[t.g] || w.kb0 < 0 || w.kb1 > kbt || w.kb0 >= w.kb1) { ++bad; continue; }
+      for (int u = 0; u < t.n / TP_UNIT; ++u)
+        for (int kb = w.kb0; kb < w.kb1; ++kb) seen[((size_t)(t.row0 / TP_UNIT + u) * f_tiles + t.f0 / f_width) * kbt + kb] += 1;
+      if (w.kb0 == 0) for (int r = t.zero0; r < t.end; ++r) cleared[(size_t)r * f_tiles + t.f0 / f_width] += 1;
+      if (w.split >= 0) {
+        ++shared;
+        if (w.split >= pairs) { ++bad; continue; }
+        pieces[w.split] += 1;
+        if (claimed[w.split] != 0 && claimed[w.split] != w.contributors) ++bad;
+        claimed[w.split] = w.contributors;
+      } else if (w.kb0 != 0 || w.kb1 != kbt) {
+        ++bad;
+      }
     }
+    if (shared > 2) ++bad;
   }
+  for (int i = 0; i <= pairs; ++i) if (pieces[i] != claimed[i]) ++bad;
   for (int g = 0; g < G; ++g) {
     const int covered = (rows[g] + TP_UNIT - 1) / TP_UNIT;
     for (int u = 0; u < (end[g] - start[g] + TP_UNIT - 1) / TP_UNIT; ++u)
       for (int f = 0; f < f_tiles; ++f)
-        if (seen[(size_t)(start[g] / TP_UNIT + u) * f_tiles + f] != (u < covered ? 1 : 0)) ++bad;
+        for (int kb = 0; kb < kbt; ++kb)
+          if (seen[((size_t)(start[g] / TP_UNIT + u) * f_tiles + f) * kbt + kb] != (u < covered ? 1 : 0)) ++bad;
     for (int r = start[g]; r < end[g]; ++r)
       for (int f = 0; f < f_tiles; ++f)
         if (rows[g] > 0 && cleared[(size_t)r * f_tiles + f] != (r >= start[g] + covered * TP_UNIT ? 1 : 0)) ++bad;
@@ -146,7 +164,7 @@ static int check_joint() {
     TPForm one{0, 0.f, 0.f}, two{0, 0.f, 0.f};
     int units = 0;
     for (int r : rows) { units += (r + TP_UNIT - 1) / TP_UNIT; tp_add_group(one, r, 8); tp_add_group(two, r, 16); }
-    return tp_joint_pays(one, two, units, f_tiles, 74, kbt);
+    return tp_joint_pays(one, two, units, f_tiles, 74, kbt, true);
   };
   int bad = 0;
   bad += !pays({211, 281, 92, 321, 302, 269, 245, 279}, 16, 224);
@@ -171,11 +189,11 @@ int main() {
       at += it % 5 == 0 ? n : (n + BM - 1) / BM * BM;                // (dense: no padding)
       end.push_back(at);
     }
-    const int N = 8 * (17 + rnd(500)), ps[3] = {74, 66, 5};
+    const int N = 8 * (17 + rnd(500)), kbt = 1 + rnd(40), ps[3] = {74, 66, 5};
     for (int c = 0; c < 3; ++c) {
-      const int b1 = check_transposed(start, rows, end, N, 256, ps[c], it % 2 ? 8 : 16), b2 = check_transposed(start, rows, end, N, 128, ps[c], it % 2 ? 8 : 16);
+      const int b1 = check_transposed(start, rows, end, N, 256, kbt, ps[c], it % 3 != 0, it % 2 ? 8 : 16), b2 = check_transposed(start, rows, end, N, 128, kbt, ps[c], it % 3 != 0, it % 2 ? 8 : 16);
       ++cases;
-      if (b1 || b2) { ++failures; printf("transposed: G %d N %d pairs %d: %d / %d errors\n", G, N, ps[c], b1, b2); }
+      if (b1 || b2) { ++failures; printf("transposed: G %d N %d kbt %d pairs %d: %d / %d errors\n", G, N, kbt, ps[c], b1, b2); }
     }
   }
   for (int it = 0; it < 300; ++it) {
