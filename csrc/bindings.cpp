@@ -462,6 +462,13 @@ Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor
   return AttentionNode::apply(q, k, v, cu_seqlens, max_seqlen, scale, status);
 }
 
+// {bytes of the GPU's memory that no tensor takes, all of them}, without a call to the driver
+std::vector<int64_t> memory_room(int64_t device) {
+  const auto stats = c10::cuda::CUDACachingAllocator::getDeviceStats((c10::DeviceIndex)device);
+  const int64_t total = (int64_t)at::cuda::getDeviceProperties((c10::DeviceIndex)device)->totalGlobalMem;
+  return {total - stats.allocated_bytes[0].current, total};
+}
+
 // ---- peer-memory communication (comm.cu).  `layout` = [ws, E, capacity_rows, capacity_slots, off_counts,
 // off_count_flags, off_arrive_x, off_arrive_y, off_recv_x, off_recv_y]; peer_base = int64 device tensor of
 // the peers' workspace base addresses.
@@ -1051,6 +1058,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding", &embedding);
   m.def("embedding_bwd", &embedding_bwd, py::arg("dout"), py::arg("ids"), py::arg("dtable"), py::arg("add") = false);
   m.def("adapter_pack", &adapter_pack);
+  m.def("memory_room", &memory_room);
   m.def("cross_entropy", &cross_entropy);
   m.def("gemm_set_pair_policy", [](int64_t policy) { return (int64_t)mdt_gemm_set_pair_policy((int)policy); });
   m.def("gemm_set_pair_cap", [](int64_t n) { mdt_gemm_set_pair_cap((int)n); });

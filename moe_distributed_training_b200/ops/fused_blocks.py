@@ -192,6 +192,16 @@ def moe_block_supported(layer, x) -> bool:
     return True
 
 
+def _room_to_keep(tensors) -> bool:
+    """Whether a recomputed block may keep `tensors` (allocated already) until its backward pass.  A step that fits without them has to
+    fit with them, so only where what is still to come fits beside them: an eighth of the GPU for what does not grow with the batch, 24
+    times what one block keeps for what does.  (A block keeps two rows of `hidden` for every token and choice.  Its own
+    backward pass takes 11 times that with ffn = 3.5 hidden, logits up to 4 times, the inputs of 32 more blocks 8 times.)"""
+    first = next(t for t in tensors if t is not None)
+    free, total = ext.memory_room(first.get_device())
+    return free >= max(total // 8, 24 * sum(t.numel() * t.element_size() for t in tensors if t is not None))
+
+
 class _MoEBlock(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, call, *params):
@@ -213,8 +223,8 @@ class _MoEBlock(torch.autograd.Function):
         ids = tuple(id(t) for t in lora_tensors)
         ep = ex.ep_group is not None and ex.ep_size > 1
         # A block that is recomputed in the backward pass (layer._ckpt_mode, see _MoEBlockNative) keeps routing, grouped rows, expert
-        # outputs and the adapters' intermediate products of its first pass: the recomputation is RMSNorm and the gate / up product.
-        # (Local experts: an exchange would have to be kept as well.)
+        # outputs and the adapters' intermediate products of its first pass where there is room for them: the recomputation is RMSNorm
+        # and the gate / up product.  (Local experts: an exchange would have to be kept as well.)
         ckpt_mode = getattr(layer, "_ckpt_mode", 0) if not ep else 0
         stash = getattr(layer, "_moe_stash", None)
         if ckpt_mode == 2 and grad_mode and stash is not None:
@@ -231,7 +241,7 @@ class _MoEBlock(torch.autograd.Function):
             xg = ext.gather_rows(xn, plan.src_slot, plan.padded_offsets, E, None, k)
             yg, kept = C._GroupedSwiGLUMLP.run(mctx, xg, w1, w2, w3, plan, lora, float(ws), wgrad_out, ids, lora_tensors)
             ys = yg
-            if ckpt_mode == 1 and not grad_mode:
+            if ckpt_mode == 1 and not grad_mode and _room_to_keep((xg, ys, *kept)):
                 layer._moe_stash = (plan, wts, idx, xg, ys, kept)
             comb = ext.combine_rows(yg, plan.dest_row, wts, k, x2)      # + x
             eng = meta_c = expert_sorted = None

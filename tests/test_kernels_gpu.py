@@ -990,6 +990,53 @@ def test_two_micro_batches_before_their_backward_pass(lora, keep):
         _close(a.reshape(-1), b.reshape(-1), 1.5e-2, "gradient")
 
 
+def test_recomputed_adapter_blocks_keep_results_only_where_there_is_room(ops, monkeypatch):
+    """A step that fits in memory without what blocks with expert adapters keep for their recomputation fits with it: nothing is kept
+    where an eighth of the GPU, or 24 times what a block keeps, is not free beside it.  Gradients are the same either way."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
+    from moe_distributed_training_b200.ops import fused_blocks
+    from moe_distributed_training_b200.train.engine import build_engine
+    real = fused_blocks.ext
+    free, total = real.memory_room(0)
+    big = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+    after, same = real.memory_room(0)
+    assert free - after >= big.numel() and total == same == torch.cuda.get_device_properties(0).total_memory
+    room = [0, 0]
+
+    class Ext:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def memory_room(self, device):
+            return room
+    monkeypatch.setattr(fused_blocks, "ext", Ext())
+    small = torch.empty(1000, dtype=torch.bfloat16, device=DEV)
+    for room[:], fits in (((48000, 80000), True), ((47999, 80000), False), ((48000, 384000), True), ((48000, 384008), False), ((10**11, 18 * 10**10), True)):
+        assert fused_blocks._room_to_keep((small, None)) == fits, room
+    room[:] = (120, 800)
+    assert not fused_blocks._room_to_keep((None, small))
+    cfg = MixtralConfig(vocab_size=512, hidden_size=256, intermediate_size=512, num_hidden_layers=2, num_attention_heads=2, num_key_value_heads=1,
+                        head_dim=128, num_local_experts=4, num_experts_per_tok=2)
+    (mb,) = list(batches(SyntheticInstructionDataset(cfg.vocab_size, 1, 60, 150), 1))
+    grads, plans = [], []
+    make_plan = ops.make_plan
+    monkeypatch.setattr(ops, "make_plan", lambda *a, **kw: (plans.append(1), make_plan(*a, **kw))[1])
+    for room[:], times in (((10**11, 18 * 10**10), 1), ((10**9, 18 * 10**10), 2)):
+        eng = build_engine(cfg, dtype=torch.bfloat16, device_type="cuda", learning_rate=1e-3, seed=0, use_lora="all")
+        for n, p in eng.model.named_parameters():
+            if "lora_B" in n:
+                p.data.fill_(0.01)
+        plans.clear()
+        eng.forward_backward(mb, 1.0)
+        assert len(plans) == times * cfg.num_hidden_layers          # (routed again where nothing was kept)
+        grads.append([p.grad for p in eng.model.parameters() if p.grad is not None])
+    assert len(grads[0]) == len(grads[1]) > 0
+    for a, b in zip(*grads):
+        _close(a, b, 4e-3, "gradient")
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("E,H,F,r", [(1, 8, 8, 4), (3, 72, 200, 12), (8, 256, 1032, 16), (2, 64, 136, 100)])
 def test_adapter_pack(ops, E, H, F, r):
     A1, A3, B1, B3 = _rand(E, H, r), _rand(E, H, r), _rand(E, r, F), _rand(E, r, F)
