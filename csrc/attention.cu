@@ -818,14 +818,14 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
         }
         if (!wait_parity_warp(bardP, it & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        uint32_t pk[32];                 // dS^T without the factor `scale`, which dK gets at the end
+        uint32_t pk[32];                 // dS^T with the factor `scale`, then rounded once
 #pragma unroll
         for (int c = 0; c < 64; c += 32) {
           uint32_t d[32];
           tmem_ld_32x32(t_row + 128 + c, d);
           tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - dl[x]));
+          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - dl[x]) * p.scale);
           if (masked) {                  // (a branch of its own: tests between the products cost 900 clocks a block)
 #pragma unroll
             for (int x = 0; x < 32; ++x) if (hidden(c + x)) d[x] = 0u;
@@ -860,8 +860,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
           uint32_t a[32];
           tmem_ld_32x32(acc + c, a);
           tmem_ld_wait();
-#pragma unroll
-          for (int x = 0; x < 32; ++x) a[x] = __float_as_uint(__uint_as_float(a[x]) * (half == 0 ? 1.f : p.scale));
           if (per > 1) {
 #pragma unroll
             for (int x = 0; x < 32; x += 4)
@@ -992,7 +990,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
           tmem_ld_32x32(t_dp + c, d);
           tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - delta));
+          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - delta) * p.scale);
           if (j == qb) {                 // diagonal: keys to the right of the query
 #pragma unroll
             for (int x = 0; x < 32; ++x) if (half * 64 + c + x > r) d[x] = 0u;
@@ -1017,8 +1015,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
           uint32_t a[32];
           tmem_ld_32x32(tdQ + half * 64 + t_lane + c, a);
           tmem_ld_wait();
-#pragma unroll
-          for (int x = 0; x < 32; ++x) a[x] = __float_as_uint(__uint_as_float(a[x]) * p.scale);
           if (valid) {
 #pragma unroll
             for (int x = 0; x < 32; x += 8) *reinterpret_cast<uint4*>(out + c + x) = pack8(a + x);

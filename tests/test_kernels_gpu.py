@@ -1146,6 +1146,31 @@ def test_end_to_end_matches_reference_path(ops):
     assert l_gpu[-1] < l_gpu[0]
 
 
+@pytest.mark.parametrize("T,Hq,Hkv", [(2, 1, 1), (77, 2, 2), (128, 4, 1), (300, 4, 2), (613, 8, 2)])
+def test_attention_backward_rounds_ds_with_its_scale(ops, T, Hq, Hkv):
+    """dQ and dK against the same sums in fp64 with dS = P (dP - delta) scale rounded to bf16 once, as the operand of their products.  The
+    kernel's own errors (fp32 sums, 1e-6) move 1 in 2000 of these roundings and as many of the result's, 1e-4 of the 2-norm together; dS rounded
+    without the factor, which is no power of two, is 2.4e-3 away: 1e-3 lies between."""
+    torch.manual_seed(T)
+    q, k, v, do = (_rand(T, h, 128) for h in (Hq, Hkv, Hkv, Hq))
+    leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    o = ops.attention(*leaves, torch.tensor([0, T], dtype=torch.int32, device=DEV), T)
+    dq, dk, dv = torch.autograd.grad(o, leaves, do)
+    scale = 128 ** -0.5
+    groups = Hq // Hkv
+    Q, K, V, dO, O = (t.detach().double().transpose(0, 1) for t in (q, k.repeat_interleave(groups, 1), v.repeat_interleave(groups, 1), do, o))
+    S = Q @ K.transpose(1, 2) * scale
+    P = torch.softmax(S.masked_fill(torch.ones(T, T, dtype=torch.bool, device=DEV).triu(1), float("-inf")), -1)
+    dS = (P * (dO @ V.transpose(1, 2) - (dO * O).sum(-1, keepdim=True)) * scale).bfloat16().double()
+    per_kv = lambda t: t.view(Hkv, groups, T, 128).sum(1).transpose(0, 1)
+    for name, got, want in (("dq", dq, (dS @ K).transpose(0, 1)), ("dk", dk, per_kv(dS.transpose(1, 2) @ Q)),
+                            ("dv", dv, per_kv(P.bfloat16().double().transpose(1, 2) @ dO))):
+        want = want.bfloat16().double()
+        off, norm = float((got.double() - want).norm()), float(want.norm())
+        assert off <= 1e-3 * norm + 1e-6, (name, off, norm)
+    ops.check_status(DEV)
+
+
 @pytest.mark.parametrize("lens", [[128], [200], [577], [1024], [100, 300, 77], [256, 256]])
 def test_attention(ops, lens):
     from moe_distributed_training_b200.ops import reference
