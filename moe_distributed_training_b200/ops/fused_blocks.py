@@ -198,7 +198,10 @@ def _room_to_keep(tensors) -> bool:
     times what one block keeps for what does.  (A block keeps two rows of `hidden` for every token and choice.  Its own
     backward pass takes 11 times that with ffn = 3.5 hidden, logits up to 4 times, the inputs of 32 more blocks 8 times.)"""
     first = next(t for t in tensors if t is not None)
-    free, total = ext.memory_room(first.get_device())
+    try:
+        free, total = ext.memory_room(first.get_device())
+    except RuntimeError:          # (an allocator of the user's own that keeps no statistics)
+        return False
     return free >= max(total // 8, 24 * sum(t.numel() * t.element_size() for t in tensors if t is not None))
 
 

@@ -1037,6 +1037,16 @@ def test_recomputed_adapter_blocks_keep_results_only_where_there_is_room(ops, mo
     ops.check_status(DEV)
 
 
+def test_blocks_keep_nothing_under_an_allocator_without_statistics(ops, monkeypatch):
+    from moe_distributed_training_b200.ops import fused_blocks
+
+    class Ext:
+        def memory_room(self, device):
+            raise RuntimeError("the allocator does not support getDeviceStats")
+    monkeypatch.setattr(fused_blocks, "ext", Ext())
+    assert not fused_blocks._room_to_keep((torch.empty(8, device=DEV),))
+
+
 @pytest.mark.parametrize("E,H,F,r", [(1, 8, 8, 4), (3, 72, 200, 12), (8, 256, 1032, 16), (2, 64, 136, 100)])
 def test_adapter_pack(ops, E, H, F, r):
     A1, A3, B1, B3 = _rand(E, H, r), _rand(E, H, r), _rand(E, r, F), _rand(E, r, F)
