@@ -496,10 +496,12 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
 // blocks.  Those additions were what bounded it: 64 KB of fp32 reductions into L2 a block (25 % of its loop), dQ's place in TMEM that held
 // up the next block's dP, and a buffer of 128 floats a token and head to be cleared and converted.  Without them nothing leaves TMEM
 // but the results: P^T and dS^T (dK, dV) and dS (dQ) are operands of their products from there.
-// All launches, 32 / 8 heads, us, with dQ by reductions -> so: 613 tokens 53 -> 41, 2048 196 -> 177, 8192 1693 -> 1543, 16384 6851 -> 6697
-// (8192 alone: dK, dV of all blocks about 870, dQ 680: 216 and 226 a product).  What bounds it is the chain of a CTA, scores ->
+// Whole calls, 32 / 8 heads, us, with dQ by reductions -> so: 77 tokens 33.8 -> 21.5, 613 62.5 -> 48.1, 2048 207.9 -> 187.4, 8192
+// 1716 -> 1578, 16384 6741 -> 6720 (8192: dK, dV of all blocks about 0.56 of it, dQ 0.44).  What bounds it is the chain of a CTA, scores ->
 // exponentials -> product, with one CTA an SM (its operands fill shared memory and its accumulators TMEM) and half a block to overlap with.
-// Slower at 8192: 16 softmax warps (2379, they spill), two blocks in flight through halves of TMEM (1581), one wait for scores and
+// dS = P (scale dP - scale delta) has its factor before it is rounded (it is no power of two: on the sums it would put every rounding
+// elsewhere), in the statistics and a fused multiply-add; a multiplication of its own took 3 % at 8192 tokens.
+// Slower at 8192 (of 1543 then): 16 softmax warps (2379, they spill), two blocks in flight through halves of TMEM (1581), one wait for scores and
 // statistics together (1912), a share of the exponentials on the fp32 units (1604 with a quarter, 1688 with half).
 //
 // dK, dV keep keys as rows (TMEM lanes): S^T = K Q^T, P^T = exp2(S^T - lse) over S^T, dV += P^T dO, dS^T over dP^T = V dO^T, dK += dS^T Q.
@@ -511,7 +513,7 @@ __global__ void __launch_bounds__(FWD2_THREADS, 2) attn_fwd_pipelined_kernel(con
 // Where the query heads of a kv head are spread over several CTAs these form a cluster, which adds their dK, dV in the order of the
 // ranks through distributed shared memory; all results are the same in every run.
 constexpr int BWD_THREADS = 320;
-constexpr int BWD_STATS = 2 * AB;                              // lse2 | delta of a block, floats
+constexpr int BWD_STATS = 2 * AB;                              // lse2 | scale * delta of a block, floats
 constexpr int BWD_SMEM = 7 * TILE_BYTES + 2 * BWD_STATS * 4 + 256 + 768;   // (768: what alignment to 1024 may take)
 constexpr int MAX_SETS = 8;                                    // CTAs that share a kv head's query heads: a cluster
 static_assert(BWD_SMEM <= 227 * 1024, "attention backward: shared memory of a CTA");
@@ -519,7 +521,7 @@ static_assert(BWD_SMEM <= 227 * 1024, "attention backward: shared memory of a CT
 struct AttnBwdParams {
   CUtensorMap tmQ, tmK, tmV, tmdO;
   const int4* sched;            // by rank: {seq_start, seq_end, block, flat block}; seq_start < 0: none
-  const float* stats;           // [flat block][head][lse2 x 128 | delta x 128]
+  const float* stats;           // [flat block][head][lse2 x 128 | scale * delta x 128]
   bf16* dq; bf16* dk; bf16* dv;
   int heads_q, heads_kv, hpc;   // hpc: query heads per dK, dV CTA
   int tokens, blocks;           // rows of the tensors; entries of the schedule
@@ -528,7 +530,7 @@ struct AttnBwdParams {
 };
 
 __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __restrict__ o, const bf16* __restrict__ dout, const float* __restrict__ lse,
-                                                               const int* __restrict__ cu, int num_seqs, int tokens, int heads, int heads_kv, int4* __restrict__ sched,
+                                                               const int* __restrict__ cu, int num_seqs, int tokens, int heads, int heads_kv, float scale, int4* __restrict__ sched,
                                                                float* __restrict__ stats, bf16* __restrict__ dq, bf16* __restrict__ dk, bf16* __restrict__ dv, int* status) {
   after_predecessor();
   int seq_start, seq_end, blk;
@@ -589,7 +591,7 @@ __global__ void __launch_bounds__(256, 2) attn_bwd_prepare_kernel(const bf16* __
     for (int i = 0; i < 4; ++i) { const float2 x = __bfloat1622float2(pa[i]), y = __bfloat1622float2(pb[i]); s += x.x * y.x + x.y * y.y; }
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (sub == 0) { st[r] = valid ? lse[row * heads + h] * 1.4426950408889634f : 0.f; st[AB + r] = valid ? s : 0.f; }
+    if (sub == 0) { st[r] = valid ? lse[row * heads + h] * 1.4426950408889634f : 0.f; st[AB + r] = valid ? s * scale : 0.f; }
   }
 }
 
@@ -825,7 +827,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
           tmem_ld_32x32(t_row + 128 + c, d);
           tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - dl[x]) * p.scale);
+          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * fmaf(__uint_as_float(d[x]), p.scale, -dl[x]));
           if (masked) {                  // (a branch of its own: tests between the products cost 900 clocks a block)
 #pragma unroll
             for (int x = 0; x < 32; ++x) if (hidden(c + x)) d[x] = 0u;
@@ -990,7 +992,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
           tmem_ld_32x32(t_dp + c, d);
           tmem_ld_wait();
 #pragma unroll
-          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * (__uint_as_float(d[x]) - delta) * p.scale);
+          for (int x = 0; x < 32; ++x) d[x] = __float_as_uint(pr[c + x] * fmaf(__uint_as_float(d[x]), p.scale, -delta));
           if (j == qb) {                 // diagonal: keys to the right of the query
 #pragma unroll
             for (int x = 0; x < 32; ++x) if (half * 64 + c + x > r) d[x] = 0u;
@@ -1154,7 +1156,7 @@ extern "C" int mdt_attention_bwd(const void* q, const void* k, const void* v, co
     configured = true;
   }
   launch_after(attn_bwd_prepare_kernel, dim3((unsigned)b.blocks, heads_q), 256, 0, s, (const bf16*)o, (const bf16*)dout, lse, cu_seqlens, num_seqs,
-               total_tokens, heads_q, heads_kv, reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq, p.dk, p.dv, status);
+               total_tokens, heads_q, heads_kv, scale, reinterpret_cast<int4*>(scratch), scratch + b.off_stats, p.dq, p.dk, p.dv, status);
   ++g_att_launches;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
