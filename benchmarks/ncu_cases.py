@@ -1,6 +1,6 @@
 """Small single-GPU cases for profiler captures: one kernel family per case, a handful of launches.
 
-    python benchmarks/ncu_cases.py gemm|gemm_pair|gemm_cluster|gemm_split|gather_gemm|rs_block|expert_mlp|attention|attention_long|dispatch|gemm_exchange
+    python benchmarks/ncu_cases.py gemm|gemm_pair|gemm_cluster|gemm_split|gather_gemm|rs_block|expert_mlp|expert_rows|adapters|attention|attention_long|dispatch|gemm_exchange
 
 Sizes keep the working set above the 126 MB L2 where DRAM figures matter, but far below a GB of launches.
 """
@@ -69,6 +69,34 @@ def main():
         with torch.no_grad():
             for _ in range(3):
                 C.grouped_swiglu_mlp(xg, w1, w2, w3, plan)
+    elif case == "expert_rows":
+        # products of a micro-batch with the weights as the 256-row operand: 144 rows for each of two experts through gate and up and through
+        # the SwiGLU backward, 300 rows through the head; and one weight gradient, written and added to
+        E, F, H, rows = 2, 14336, 4096, 144
+        plan = C.make_plan(torch.arange(E, device=dev, dtype=torch.int32).repeat_interleave(rows)[:, None], E)
+        xg = C.ext.gather_rows(torch.randn(E * rows, H, device=dev, dtype=bf), plan.src_slot, plan.padded_offsets, E, None, 1)
+        w1, w2, w3 = (torch.randn(E, F, H, device=dev, dtype=bf) * 0.02 for _ in range(3))
+        R = xg.shape[0]
+        h, g, u, dg, du = (torch.empty(R, F, device=dev, dtype=bf) for _ in range(5))
+        dw = torch.empty(E, F, H, device=dev, dtype=bf)
+        y = torch.where((plan.src_slot >= 0)[:, None], torch.randn(R, H, device=dev, dtype=bf), 0.0).to(bf)
+        x, head = torch.randn(300, H, device=dev, dtype=bf), torch.randn(32000, H, device=dev, dtype=bf) * 0.02
+        for _ in range(3):
+            C._g(1, xg, False, w1, False, h, F, H, plan, B2=w3, C2=g, C3=u)
+            C.mm_nt(x, head)
+            C._g(1, y, False, w2, False, dg, F, H, plan, C2=du, swiglu=(g, u))
+            C._g(2, dg, True, xg, True, dw, H, 0, plan)
+            C._g(2, dg, True, xg, True, dw, H, 0, plan, accumulate=True)
+    elif case == "adapters":
+        # one attention block with rank-16 adapters, 576 tokens, forward and backward
+        from moe_distributed_training_b200 import MixtralConfig
+        from moe_distributed_training_b200.train.engine import build_engine
+        cfg = MixtralConfig(vocab_size=512, hidden_size=4096, intermediate_size=1024, num_hidden_layers=1, num_attention_heads=32, num_key_value_heads=8,
+                            head_dim=128, num_local_experts=2, num_experts_per_tok=1)
+        eng = build_engine(cfg, dtype=bf, device_type="cuda", learning_rate=1e-3, seed=0, use_lora="attn-only")
+        ids = torch.randint(0, 512, (576,), device=dev)
+        for _ in range(3):
+            eng.forward_backward({"input_ids": ids, "labels": ids, "cu_seqlens": torch.tensor([0, 576], dtype=torch.int32, device=dev), "max_seqlen": 576}, 1.0)
     elif case in ("attention", "attention_long"):
         T, Hq, Hkv, d = (1024 if case == "attention" else 8192), 32, 8, 128
         q = torch.randn(T, Hq, d, device=dev, dtype=bf, requires_grad=True)
