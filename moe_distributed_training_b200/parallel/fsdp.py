@@ -26,6 +26,7 @@ what passing that mesh to `fully_shard` does in the reference
 from __future__ import annotations
 
 import os
+import sys
 from typing import List, Optional
 
 import torch
@@ -156,15 +157,17 @@ class FlatParamGroup:
 
     def take_places(self, grads: List[Optional[torch.Tensor]]):
         """(buffer for the flat gradient, indices of the weights whose gradient in `grads` is its part already).  A part that was given
-        out and did not come back may be in somebody's hands (a gradient that was asked for by itself, one that a hook
-        kept): then the buffer is left to them and another one taken."""
+        out and did not come back, or that `grads` does not hold alone, is in somebody's hands (a gradient that was asked for by
+        itself, one that a hook or a reader of .grad kept): then the buffer is left to them and another one taken."""
         places, self._places = self._places, None
         if places is not None:
             flat, given = places
             base, size = flat.data_ptr(), flat.element_size()
             there = {i for i in given if grads[i] is not None and grads[i].data_ptr() == base + self.specs[i][4] * size
                      and grads[i].shape == self.specs[i][2] and grads[i].dtype == flat.dtype and grads[i].is_contiguous()}
-            if len(there) == len(given):
+            # tensors on the buffer: it, its storage's handle here and the parts; references to a part: the list and the argument
+            alone = torch._C._storage_Use_Count(flat.untyped_storage()._cdata) == 2 + len(given)
+            if len(there) == len(given) and alone and all(sys.getrefcount(grads[i]) == 2 for i in there):
                 return flat, there
         return torch.empty_like(self.shard.data), set()
 
@@ -295,10 +298,11 @@ class _LayerFn(torch.autograd.Function):
         finally:
             layer._ckpt_mode = 0
             layer._moe_stash = None
-        grads = torch.autograd.grad(y, [xin] + leaves + local, gout, allow_unused=True)
-        dx = grads[0]
-        runner._reduce_unit_grads(unit, list(grads[1:1 + len(leaves)]))
-        for p, g in zip(local, grads[1 + len(leaves):]):
+        grads = list(torch.autograd.grad(y, [xin] + leaves + local, gout, allow_unused=True))
+        dx, of_leaves, of_local = grads[0], grads[1:1 + len(leaves)], grads[1 + len(leaves):]
+        del grads                       # (see take_places)
+        runner._reduce_unit_grads(unit, of_leaves)
+        for p, g in zip(local, of_local):
             if g is not None:
                 p.grad = g if p.grad is None else p.grad.add_(g)
         runner._release(idx)
@@ -809,25 +813,27 @@ class ShardedMixtral:
     def head(self, x, lab, batch, return_logits=False) -> CausalLMOutput:
         return self.model.head(x, lab, batch, return_logits)
 
+    @staticmethod
+    def _take_grads(leaves):
+        """The gradients of the leaves, which keep none (see take_places)."""
+        grads = [leaf.grad for leaf in leaves]
+        for leaf in leaves:
+            leaf.grad = None
+        return grads
+
     def finish_microbatch(self):
         """Collect the root unit's gradients after `loss.backward()`."""
         g = self.root.trainable_group
         if g is not None and self._root_leaves:
-            grads = [leaf.grad for leaf in self._root_leaves]
-            self._reduce_unit_grads(self.root, grads)
-            for leaf in self._root_leaves:
-                leaf.grad = None
+            self._reduce_unit_grads(self.root, self._take_grads(self._root_leaves))
         self._root_leaves = []
         for idx in sorted(self._direct_units, reverse=True):
             unit = self.units[idx]
             tg = unit.trainable_group
             if tg is not None:
-                leaves = tg.installed_leaves()
-                grads = [leaf.grad for leaf in leaves]
+                grads = self._take_grads(tg.installed_leaves())
                 if any(gr is not None for gr in grads):
                     self._reduce_unit_grads(unit, grads)
-                for leaf in leaves:
-                    leaf.grad = None
         self._direct_units.clear()
         for idx in list(self._slot):
             self._release(idx)

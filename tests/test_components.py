@@ -330,10 +330,12 @@ def test_parts_of_the_flat_gradient_are_given_out_once():
             t.copy_(one(i))
         return out
     # all parts come back: no copy
-    a, b = parts(0, 2)
+    grads = parts(0, 2)
+    grads.insert(1, one(1))
     buffer = g._places[0]
-    eng.runner._reduce_unit_grads(unit, [a, one(1), b])
+    eng.runner._reduce_unit_grads(unit, grads)
     assert g.shard.grad is buffer and torch.equal(g.shard.grad, want)
+    del grads
     # there is a flat gradient: no parts, the next gradients are added
     assert g.grad_tensor(0) is None
     eng.runner._reduce_unit_grads(unit, [one(0), one(1), one(2)])
@@ -352,6 +354,17 @@ def test_parts_of_the_flat_gradient_are_given_out_once():
         assert torch.equal(g.shard.grad, expected) and torch.equal(held, one(0))
         g.shard.grad.fill_(7.0)
         assert torch.equal(held, one(0))
+    # a part that came back, but that somebody else has too: the tensor, a view of it, one without its graph
+    for keep in (lambda t: t, lambda t: t.view(-1)[1:], lambda t: t.detach()):
+        eng.optimizer.zero_grad(set_to_none=True)
+        grads = parts(0, 1, 2)
+        kept = keep(grads[1])
+        before = kept.clone()
+        eng.runner._reduce_unit_grads(unit, grads)
+        del grads
+        assert torch.equal(g.shard.grad, want)
+        eng.runner._reduce_unit_grads(unit, [one(0), one(1), one(2)])
+        assert torch.equal(g.shard.grad, 2 * want) and torch.equal(kept, before)
     # a micro-batch that failed
     for drop in (eng.runner.discard_microbatch, eng.runner.zero_grad):
         eng.optimizer.zero_grad(set_to_none=True)

@@ -927,6 +927,27 @@ def test_gradients_of_dense_weights_pass_through_autograd(recompute):
             _close(got[unit][o:o + n], factor * want[unit][o:o + n].float(), 4e-3, g.qualnames[i])
 
 
+@pytest.mark.parametrize("recompute", [True, False])
+def test_gradients_that_somebody_keeps_stay_what_they_were(recompute):
+    """What a hook or a reader of .grad has kept of the first micro-batch is not changed by the second one."""
+    eng, mbs, groups = _small_engine(recompute)
+    with torch.no_grad():
+        _forward(eng, mbs[0])                        # (the weights' views exist from here on)
+    kept = []
+    q = eng.model.model.layers[0].self_attn.q_proj.weight
+    handle = q.register_hook(lambda g: kept.append(g))
+    _forward(eng, mbs[0]).loss.backward()
+    kept += [eng.model.lm_head.weight.grad, eng.model.model.embed_tokens.weight.grad.detach()]
+    handle.remove()
+    want = [t.clone() for t in kept]
+    eng.runner.finish_microbatch()
+    first = _all_grads(eng, groups)
+    _forward(eng, mbs[1]).loss.backward()
+    eng.runner.finish_microbatch()
+    assert len(kept) == 3 and all(torch.equal(a, b) for a, b in zip(kept, want))
+    assert not all(torch.equal(a, b) for a, b in zip(first, _all_grads(eng, groups)))
+
+
 def test_adapter_blocks_store_gate_and_up_only_for_a_graph(ops, monkeypatch):
     """Passes without a graph (evaluation, the first pass of recomputed blocks) leave the inputs of SwiGLU unwritten, trainable adapters or not."""
     from moe_distributed_training_b200 import MixtralConfig
