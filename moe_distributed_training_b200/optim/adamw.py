@@ -22,6 +22,12 @@ class FusedAdamW(torch.optim.Optimizer):
         super().__init__(params, defaults)
         self.state_dtype = state_dtype
         self._grad_scale = 1.0
+        self.also_zero = []          # called by zero_grad: gradients that are on their way to the parameters'
+
+    def zero_grad(self, set_to_none: bool = True) -> None:
+        super().zero_grad(set_to_none=set_to_none)
+        for drop in getattr(self, "also_zero", ()):          # (not there after unpickling)
+            drop()
 
     @property
     def grad_scale(self) -> float:

@@ -838,7 +838,7 @@ class ShardedMixtral:
         for idx in list(self._slot):
             self._release(idx)
 
-    def _drop_microbatch_grads(self):
+    def drop_microbatch_grads(self):
         """Forget the gradients that a micro-batch has left with the weights' views and in parts of flat gradients."""
         for u in self.all_units():
             g = u.trainable_group
@@ -851,7 +851,7 @@ class ShardedMixtral:
     def discard_microbatch(self):
         """After a forward or backward pass that failed: nothing of the micro-batch that has not reached the flat gradients does
         (blocks whose backward pass was over have added theirs; `zero_grad` drops these)."""
-        self._drop_microbatch_grads()
+        self.drop_microbatch_grads()
         self._root_leaves = []
         self._direct_units.clear()
         for idx in list(self._slot):
@@ -860,7 +860,7 @@ class ShardedMixtral:
     def zero_grad(self):
         for p in self.model.parameters():
             p.grad = None
-        self._drop_microbatch_grads()
+        self.drop_microbatch_grads()
 
     # ------------------------------------------------------------------ unsharded views (checkpoint export)
     def full_state(self, unit: FsdpUnit, grads: bool = False):

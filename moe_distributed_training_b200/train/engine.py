@@ -84,6 +84,12 @@ class Engine:
     step_count: int = 0
     last: dict = field(default_factory=dict)
 
+    def __post_init__(self):
+        # a loop of the caller's own whose backward pass failed: what it left with the weights' views goes with the gradients
+        drop = getattr(self.runner, "drop_microbatch_grads", None)
+        if drop is not None and hasattr(self.optimizer, "also_zero"):
+            self.optimizer.also_zero.append(drop)
+
     def to_device(self, mb: dict) -> dict:
         out = {}
         for k, v in mb.items():

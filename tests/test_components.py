@@ -374,6 +374,33 @@ def test_parts_of_the_flat_gradient_are_given_out_once():
         g._places = None
 
 
+@pytest.mark.parametrize("recompute", [True, False])
+@pytest.mark.parametrize("drop", ["optimizer", "runner"])
+def test_zero_grad_drops_what_an_unfinished_micro_batch_left(recompute, drop):
+    """A loop of one's own whose backward pass failed, or that gives a micro-batch up: after zero_grad of the optimizer or of the runner the
+    next micro-batch's gradients are its own."""
+    from moe_distributed_training_b200 import MixtralConfig
+    from moe_distributed_training_b200.data.synthetic import SyntheticInstructionDataset, batches
+    from moe_distributed_training_b200.train.engine import build_engine
+    cfg = MixtralConfig(vocab_size=64, hidden_size=32, intermediate_size=32, num_hidden_layers=2, num_attention_heads=2, num_key_value_heads=1,
+                        num_local_experts=2, num_experts_per_tok=1)
+    first, second = list(batches(SyntheticInstructionDataset(cfg.vocab_size, 2, 10, 20), 1))
+
+    def grads(given_up):
+        eng = build_engine(cfg, dtype=torch.float32, device_type="cpu", learning_rate=1e-3, seed=0, activation_checkpointing=recompute)
+        run = lambda mb: eng.model(mb["input_ids"], labels=mb["labels"], cu_seqlens=mb["cu_seqlens"], max_seqlen=mb["max_seqlen"]).loss.backward()
+        if given_up:
+            run(first)
+            assert eng.model.lm_head.weight.grad is not None
+            (eng.optimizer if drop == "optimizer" else eng.runner).zero_grad()
+            assert eng.model.lm_head.weight.grad is None
+        run(second)
+        eng.runner.finish_microbatch()
+        return [p.grad.clone() for p in eng.model.parameters() if p.grad is not None]
+    for a, b in zip(grads(True), grads(False)):
+        assert torch.equal(a, b)
+
+
 def test_expert_gradient_buffers_become_grad_only_once_they_are_written(monkeypatch):
     """A backward pass that fails before its weight-gradient products are launched leaves `.grad` as it was; one that
     succeeds hands over exactly the buffers that it wrote, and the next one adds to them."""
